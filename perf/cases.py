@@ -55,30 +55,30 @@ WIDE = dict(dim=4096, hidden=11008, layers=2, heads=32, kv_heads=32, vocab=32000
 def listed():
     return [
         # a single user's chat loop on the small model, through the reference's own call (host tokens in, host logits out)
-        dict(STORIES110M, name="decode stories110M f32, 1 slot", kind="decode", weights="f32", seq_len=1024, slots=1, first=211, stride=0, call="logits", paged=False),
+        dict(STORIES110M, name="decode stories110M f32 1 slot", kind="decode", weights="f32", seq_len=1024, slots=1, first=211, stride=0, call="logits", paged=False),
         # the batching driver's default step at its benchmark's batch: tokens in, sampled tokens out (temperature 1, top-p 0.9)
-        dict(STORIES110M, name="decode stories110M f32, 256 slots", kind="decode", weights="f32", seq_len=512, slots=256, first=0, stride=1, call="sample", paged=False),
+        dict(STORIES110M, name="decode stories110M f32 256 slots", kind="decode", weights="f32", seq_len=512, slots=256, first=0, stride=1, call="sample", paged=False),
         # a handful of users on the large model in full precision
-        dict(WIDE, name="decode 7B f32, 6 slots", kind="decode", weights="f32", seq_len=1024, slots=6, first=17, stride=131, call="resident", paged=False),
+        dict(WIDE, name="decode 7B f32 6 slots", kind="decode", weights="f32", seq_len=1024, slots=6, first=17, stride=131, call="resident", paged=False),
         # one user on the quantised large model, well into a conversation
-        dict(WIDE, name="decode 7B q8, 1 slot", kind="decode", weights="q8", seq_len=2048, slots=1, first=1003, stride=0, call="resident", paged=False),
+        dict(WIDE, name="decode 7B q8 1 slot", kind="decode", weights="q8", seq_len=2048, slots=1, first=1003, stride=0, call="resident", paged=False),
         # a full batch on the quantised large model behind the paged cache
-        dict(WIDE, name="decode 7B q8, 64 slots paged", kind="decode", weights="q8", seq_len=2048, slots=64, first=3, stride=9, call="resident", paged=True),
+        dict(WIDE, name="decode 7B q8 64 slots paged", kind="decode", weights="q8", seq_len=2048, slots=64, first=3, stride=9, call="resident", paged=True),
         # a medium batch of long contexts on the bf16 model
-        dict(WIDE, name="decode 7B bf16, 24 slots", kind="decode", weights="bf16", seq_len=2048, slots=24, first=100, stride=61, call="resident", paged=False),
+        dict(WIDE, name="decode 7B bf16 24 slots", kind="decode", weights="bf16", seq_len=2048, slots=24, first=100, stride=61, call="resident", paged=False),
         # many short prompts of the small model at once
-        dict(STORIES110M, name="prefill stories110M f32, 16 prompts", kind="prefill", weights="f32", seq_len=512, seqs=16, shortest=9, longest=201, start=0),
+        dict(STORIES110M, name="prefill stories110M f32 16 prompts", kind="prefill", weights="f32", seq_len=512, seqs=16, shortest=9, longest=201, start=0),
         # one long prompt in full precision
-        dict(WIDE, name="prefill 7B f32, 1024", kind="prefill", weights="f32", seq_len=1024, seqs=1, shortest=1024, longest=1024, start=0),
+        dict(WIDE, name="prefill 7B f32 1024", kind="prefill", weights="f32", seq_len=1024, seqs=1, shortest=1024, longest=1024, start=0),
         # a few prompts on the quantised model
-        dict(WIDE, name="prefill 7B q8, 3 prompts", kind="prefill", weights="q8", seq_len=1024, seqs=3, shortest=37, longest=700, start=0),
+        dict(WIDE, name="prefill 7B q8 3 prompts", kind="prefill", weights="q8", seq_len=1024, seqs=3, shortest=37, longest=700, start=0),
         # long prompts on the bf16 model: what decides the time to the first token of long documents
-        dict(WIDE, name="prefill 7B bf16, 2 prompts", kind="prefill", weights="bf16", seq_len=2048, seqs=2, shortest=777, longest=2048, start=0),
+        dict(WIDE, name="prefill 7B bf16 2 prompts", kind="prefill", weights="bf16", seq_len=2048, seqs=2, shortest=777, longest=2048, start=0),
         # a softmax-attention design in serving: two prompts enter, then both decode
-        dict(name="layered attention, 2 requests", kind="layered", design="gavodra", width=2048, heads=16, kv_heads=4, dim=128, ff=6144, layers=2, vocab=32000,
+        dict(name="layered attention 2 requests", kind="layered", design="gavodra", width=2048, heads=16, kv_heads=4, dim=128, ff=6144, layers=2, vocab=32000,
              dtype="bfloat16", seqs=2, shortest=1100, longest=2900, new=8),
         # a recurrent design (retention, windowed attention, key-value memory) in serving
-        dict(name="layered recurrent, 3 requests", kind="layered", design="logulix", width=1024, heads=8, kv_heads=2, dim=128, ff=4608, layers=4, vocab=32000,
+        dict(name="layered recurrent 3 requests", kind="layered", design="logulix", width=1024, heads=8, kv_heads=2, dim=128, ff=4608, layers=4, vocab=32000,
              dtype="bfloat16", seqs=3, shortest=150, longest=1300, new=8),
     ]
 
