@@ -308,6 +308,154 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant_
   if (threadIdx.x == 0 && *abort_flag && p.error_flag) *((volatile int*)p.error_flag) = 1;
 }
 
+// ---- few output tiles: the K range of a tile dealt to a cluster ------------------------------------------------------------
+// A product of a few rows with a matrix of a few thousand (decoding) has 8 to 100 tiles of 128 outputs: with a CTA per tile most SMs
+// idle and the time is one CTA's walk over K.  Here the CTAs of a cluster take a share of a tile's K range each, leave their
+// partial tiles in their own shared memory and sum each other's through distributed shared memory, ranks in ascending order
+// (bit-reproducible; no partials in global memory, no counters).  Bound by the latency of one share: launch, first loads, MMA chain,
+// exchange.  Cold weights, a launch behind the other, before -> now: [2 rows] x [1024 x 4608] 24.1 -> 7.5 us, [2048 x 6144] 30.9 -> 9.7,
+// [3088 x 2048] 13.0 -> 7.1; [100 rows] x [2048 x 6144] 37.7 -> 14.9.  One tile per cluster, a share's k-blocks are all
+// in flight where the ring holds them; two CTAs fit an SM.
+template <int NT>
+struct BfcSmem {
+  static constexpr int W_BYTES = TC_BM * 128, X_BYTES = NT * 128, STAGE = W_BYTES + X_BYTES;
+  static constexpr int NST = NT <= 32 ? 5 : (NT == 64 ? 4 : 3);
+  static constexpr int TMEM_COLS = NT < 32 ? 32 : NT;
+  static constexpr int TOTAL = NST * STAGE + 1024 + (2 * NST + 1) * 8 + 64;
+  static_assert(NST * STAGE >= NT * TC_BM * 4, "the partial tile reuses the ring");
+  static_assert(2 * (TOTAL + 1024) <= 228 * 1024, "two CTAs per SM");
+};
+
+template <int NT>
+__global__ void __launch_bounds__(BF_THREADS)
+gemm_bf16_cluster_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant__ CUtensorMap mw1,
+                         const __grid_constant__ CUtensorMap mw2, const __grid_constant__ CUtensorMap mx, const BfP p) {
+  using S = BfcSmem<NT>;
+  extern __shared__ unsigned char tc_smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + S::NST * S::STAGE);   // stage landed
+  uint64_t* empty = full + S::NST;                                          // the MMAs that read the stage have completed
+  uint64_t* accum = empty + S::NST;                                         // this share's accumulator complete
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum + 1);
+  int* abort_flag = reinterpret_cast<int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int cl = p.splits, rank = (int)(blockIdx.x % cl);     // cluster = `cl` consecutive CTAs
+  int tile = (int)(blockIdx.x / cl) / p.ny;
+  const int n0 = ((int)(blockIdx.x / cl) - tile * p.ny) * NT;
+  int mat = 0;
+  while (mat + 1 < p.n_mats && tile >= p.tiles[mat]) { tile -= p.tiles[mat]; mat++; }
+  const int row0 = tile * TC_BM;
+  const int kb0 = rank * p.kblocks_per_split;
+  const int nkb = max(0, min(p.kblocks_total - kb0, p.kblocks_per_split));
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S::NST; s++) { tc_mbar_init(&full[s], 1); tc_mbar_init(&empty[s], 1); }
+    tc_mbar_init(accum, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem_u32(tmem_slot)), "r"(S::TMEM_COLS));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem_d = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      const CUtensorMap* mw = (mat == 0 || p.stacked) ? &mw0 : (mat == 1 ? &mw1 : &mw2);
+      const int wrow = p.w_row[mat] + row0, xrow = p.x_row[mat] + n0;
+      uint64_t pol_w;
+      asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol_w));
+      auto load_w = [&](int i, int s) {
+        if (p.ny == 1) tc_tma_2d_hint(smem + s * S::STAGE, mw, (kb0 + i) * BF_BK, wrow, &full[s], pol_w);
+        else tc_tma_2d(smem + s * S::STAGE, mw, (kb0 + i) * BF_BK, wrow, &full[s]);
+      };
+      // the first ring of weights goes out ahead of the dependency wait (bytes may land before the matching expect_tx)
+      const int pre = nkb < S::NST ? nkb : S::NST;
+      for (int i = 0; i < pre; i++) load_w(i, i);
+      pdl_wait();
+      for (int i = 0; i < pre; i++) {
+        tc_mbar_expect_tx(&full[i], S::STAGE);
+        tc_tma_2d(smem + i * S::STAGE + S::W_BYTES, &mx, (kb0 + i) * BF_BK, xrow, &full[i]);
+      }
+      for (int i = pre; i < nkb; i++) {
+        const int s = i % S::NST;
+        if (!tc_mbar_wait(&empty[s], ((i / S::NST) & 1u) ^ 1u, abort_flag)) break;
+        tc_mbar_expect_tx(&full[s], S::STAGE);
+        load_w(i, s);
+        tc_tma_2d(smem + s * S::STAGE + S::W_BYTES, &mx, (kb0 + i) * BF_BK, xrow, &full[s]);
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = bf_idesc(NT);
+      bool ok = true;
+      for (int i = 0; i < nkb; i++) {
+        const int s = i % S::NST;
+        if (!tc_mbar_wait(&full[s], (i / S::NST) & 1u, abort_flag)) { ok = false; break; }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint64_t adesc = tc_smem_desc(tc_smem_u32(smem + s * S::STAGE));
+        const uint64_t bdesc = tc_smem_desc(tc_smem_u32(smem + s * S::STAGE + S::W_BYTES));
+#pragma unroll
+        for (int k = 0; k < BF_BK / 16; k++) bf_mma(tmem_d, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, (uint32_t)((i | k) != 0));
+        tc_commit(&empty[s]);
+      }
+      if (ok && nkb > 0) tc_commit(accum);
+    }
+  }
+  float* part = reinterpret_cast<float*>(smem);   // [NT][128], over the ring once its last MMA has read it
+  if (warp >= 4) {
+    const int r = (warp & 3) * 32 + lane;
+    pdl_trigger();
+    const bool ok = nkb > 0 && tc_mbar_wait(accum, 0u, abort_flag);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+    for (int c = 0; c < NT; c += 16) {
+      uint32_t v[16];
+      if (ok) {
+        tc_tmem_ld16(tmem_d + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c, v);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      }
+#pragma unroll
+      for (int j = 0; j < 16; j++) part[(c + j) * TC_BM + r] = ok ? __uint_as_float(v[j]) : 0.0f;
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  }
+  __syncthreads();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  {
+    // this rank's columns: rank, rank + cl, ... of the tile; half of the threads each take one at a time, a thread a row
+    pdl_wait();   // returns at once (the producer waited): the column scales of the previous kernel are visible here
+    const int r = threadIdx.x & (TC_BM - 1), row = row0 + r;
+    const int n_cols = min(NT, p.N - n0);
+    const uint32_t base = tc_smem_u32(part) + (uint32_t)r * 4u;
+    for (int c = rank + cl * (int)(threadIdx.x >> 7); c < n_cols; c += 2 * cl) {
+      float acc = 0.0f;
+      for (int z = 0; z < cl; z++) {
+        uint32_t a;
+        float v;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(base + (uint32_t)(c * TC_BM * 4)), "r"(z));
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+        acc += v;
+      }
+      if (p.colscale) acc *= p.colscale[n0 + c];
+      if (row < p.M[mat]) p.out[(size_t)(n0 + c) * p.ldo + p.out_off[mat] + row] = acc;
+    }
+  }
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // a CTA's shared memory stays until every rank has read it
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  if (warp == 2) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(S::TMEM_COLS));
+  }
+  if (threadIdx.x == 0 && *abort_flag && p.error_flag) *((volatile int*)p.error_flag) = 1;
+}
+
 // ------------------------------------------------------------------ host side ----
 bool gemm_bf16_ok(const BfArgs& a) {
   if (a.K % 8 || a.ldx % 8 || a.K < BF_BK || a.N < 1 || a.n_mats < 1 || a.n_mats > (a.stacked ? BF_MAX_MATS : 3) || !a.X || !a.out) return false;
@@ -335,6 +483,45 @@ static int bf_mt(int NT, int N) {
   if (forced < 0) { const char* v = getenv("THA_BF16_MT"); forced = (v && *v) ? atoi(v) : 0; }
   if (forced == 1 || forced == 2) return NT == 256 ? forced : 1;
   return (NT == 256 && N >= 512) ? 2 : 1;
+}
+
+template <int NT>
+static cudaLaunchConfig_t bfc_config(cudaLaunchAttribute* attr, int grid, int cl, cudaStream_t st, bool pdl) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid); cfg.blockDim = dim3(BF_THREADS); cfg.dynamicSmemBytes = BfcSmem<NT>::TOTAL; cfg.stream = st;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cl; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr; cfg.numAttrs = pdl ? 2 : 1;
+  return cfg;
+}
+// CTAs per cluster for a product of `items` tiles over kb k-blocks, 1: a CTA per tile.  Two CTAs fit an SM (296 in all), but clusters
+// have to fit a GPC's SMs together: from about 200 CTAs on some clusters wait for others to end.  Measured on both sides of the line,
+// 2 rows, us at 1 / 2 / 4 / 8 ranks: [25 tiles, K 2048] 13.0 / 9.3 / 7.4 / 7.1 (200 CTAs of 8); [36, 1024] 8.7 / 7.2 / 6.5 / 9.5 (288);
+// [49, 1024] 9.0 / 7.5 / 6.9 / 10.1; [96, 2048] 14.8 / 13.2 / 16.4 / 19.0; [250, 2048] 27.7 / 28.7 / 34.1 / 45.0.  A pair of CTAs does not pay
+// for 128-column tiles (100 rows, [36, 1024]: 15.0 / 15.6 / 11.3; [96, 2048]: 21.6 / 22.9).
+static int bfc_ranks(int nt, int items, int kb) {
+  for (int cl = 8; cl > (nt == 128 ? 2 : 1); cl >>= 1)
+    if (kb >= 2 * cl && items * cl <= 200) return cl;
+  return 1;
+}
+// Launches the cluster form where its rule takes it; *taken says whether it did.
+template <int NT>
+static int bfc_try(cudaStream_t st, const CUtensorMap* mw, const CUtensorMap& mx, BfP p, bool pdl, bool* taken) {
+  const int cl = bfc_ranks(NT, p.n_items, p.kblocks_total);
+  *taken = cl > 1;
+  if (cl <= 1) return THA_STATUS_SUCCESS;
+  p.splits = cl;
+  p.kblocks_per_split = ceil_div(p.kblocks_total, cl);
+  auto k = gemm_bf16_cluster_kernel<NT>;
+  THA_CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, BfcSmem<NT>::TOTAL));
+  cudaLaunchAttribute attr[2];
+  const cudaLaunchConfig_t cfg = bfc_config<NT>(attr, p.n_items * cl, cl, st, pdl);
+  count_launch();
+  THA_CUDA_OK(cudaLaunchKernelEx(&cfg, k, mw[0], mw[1], mw[2], mx, p));
+  trace_launch(reinterpret_cast<const void*>(k), st);
+  return THA_STATUS_SUCCESS;
 }
 
 bool gemm_bf16_swiglu_ok(const BfArgs& a) {
@@ -388,6 +575,17 @@ int gemm_bf16_launch(cudaStream_t st, const BfArgs& a, bool pdl) {
   p.ny = ceil_div(a.N, NT);
   p.splits = splits;
   p.n_items = tiles * p.ny * splits;
+  if (splits == 1 && !swiglu && NT <= 128) {   // callers that split K themselves sum the partials in a kernel of theirs
+    bool taken = false;
+    int rc = THA_STATUS_SUCCESS;
+    switch (NT) {
+      case 16: rc = bfc_try<16>(st, mw, mx, p, pdl, &taken); break;
+      case 32: rc = bfc_try<32>(st, mw, mx, p, pdl, &taken); break;
+      case 64: rc = bfc_try<64>(st, mw, mx, p, pdl, &taken); break;
+      default: rc = bfc_try<128>(st, mw, mx, p, pdl, &taken);
+    }
+    if (taken || rc != THA_STATUS_SUCCESS) return rc;
+  }
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   dim3 grid(p.n_items < sms ? p.n_items : sms, 1, 1);
