@@ -856,7 +856,9 @@ __global__ void __launch_bounds__(128, 3) hyb_attn_mma_kernel(tha_attn_t a, tha_
   }
 }
 
-// the splits of a (row, head) in ascending key order: out = sum_s acc_s e^(m_s - M) / sum_s l_s e^(m_s - M); a warp each
+// the splits of a (row, head) in ascending key order: out = sum_s acc_s e^(m_s - M) / sum_s l_s e^(m_s - M); a warp each.  Lane s
+// keeps split s's maximum, sum and factor (at most 32 splits); eight splits' values of a channel are in flight at once (the sums one
+// load after the other took 32 us for 16 splits of 2 rows).
 template <typename T>
 __global__ void hyb_attn_merge_kernel(T* __restrict__ out, const float* __restrict__ partial, int n_rows, int heads, int E, int splits,
                                       tha_attn_t a, const float* __restrict__ gate, long long ldg) {
@@ -864,20 +866,26 @@ __global__ void hyb_attn_merge_kernel(T* __restrict__ out, const float* __restri
   if (idx >= n_rows * heads) return;
   const size_t stride = (size_t)n_rows * heads * (E + 2);
   const float* p0 = partial + (size_t)idx * (E + 2);
-  float M = -INFINITY;
-  for (int s = 0; s < splits; s++) M = fmaxf(M, p0[s * stride + E]);
-  float L = 0.f;
-  for (int s = 0; s < splits; s++) { const float ms = p0[s * stride + E]; if (ms > -INFINITY) L += p0[s * stride + E + 1] * expf(ms - M); }
-  // lane s keeps split s's factor (at most 16 splits); splits that saw nothing have factor 0 and are not read
-  float w = 0.f;
-  if (lane < splits) { const float ms = p0[lane * stride + E]; w = ms > -INFINITY ? expf(ms - M) : 0.f; }
+  const float ms = lane < splits ? p0[lane * stride + E] : -INFINITY, ls = lane < splits ? p0[lane * stride + E + 1] : 0.f;
+  const float M = warp_max(ms);
+  const float w = ms > -INFINITY ? expf(ms - M) : 0.f;   // splits that saw nothing have factor 0 and do not enter the sums
+  const float L = warp_sum(w > 0.f ? ls * w : 0.f);
   const int row = idx / heads, head = idx - row * heads;
   const float fin = hyb_attn_final_factor(a, head, M, L, gate ? gate + (size_t)row * ldg : nullptr);
   // every lane walks every group of 32 channels (the shuffles need the whole warp), also where E is not a multiple of 32
   for (int e0 = 0; e0 < E; e0 += 32) {
     const int e = e0 + lane;
     float o = 0.f;
-    for (int s = 0; s < splits; s++) { const float ws = __shfl_sync(THA_FULL_MASK, w, s); if (ws > 0.f && e < E) o = fmaf(p0[s * stride + e], ws, o); }
+    for (int s0 = 0; s0 < splits; s0 += 8) {
+      float v[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++) v[u] = (s0 + u < splits && e < E) ? p0[(size_t)(s0 + u) * stride + e] : 0.f;
+#pragma unroll
+      for (int u = 0; u < 8; u++) {
+        const float ws = __shfl_sync(THA_FULL_MASK, w, s0 + u);
+        if (ws > 0.f) o = fmaf(v[u], ws, o);
+      }
+    }
     if (e < E) hyb_store(out + (size_t)idx * E + e, o * fin);
   }
 }
@@ -1751,6 +1759,10 @@ namespace tha {
 // hybrid_latent.cu: tensor-core attention for key rows wider than AM_MAXD whose values lie inside the keys
 bool hyb_attn_wide_ok(const tha_attn_t* a);
 int hyb_attn_wide_pairs(const tha_attn_t* a, const tha_rows_t* rows);
+bool hyb_attn_row_ok(const tha_attn_t* a, const tha_rows_t* rows, const tha_kv_t* kv, const float* q);   // hybrid_attn_row.cu
+int hyb_attn_row_splits(const tha_attn_t* a, const tha_rows_t* rows, int max_keys);
+int hyb_attn_row_launch(cudaStream_t s, int dtype, const tha_attn_t* a, const tha_rows_t* rows, const tha_kv_t* kv, const float* q, void* out, int splits,
+                        float* partial, const float* gate, long long ldg);
 int hyb_attn_wide_launch(cudaStream_t s, const tha_attn_t* a, const tha_rows_t* rows, const tha_kv_t* kv, const float* q, __nv_bfloat16* out,
                          dim3 grid, int pairs, int AG, int AP, int splits, float* partial);
 }  // namespace tha
@@ -1786,7 +1798,8 @@ extern "C" int tha_hyb_attn_gated(void* stream, int dtype, const tha_attn_t* a, 
   const size_t smem = tc ? sizeof(__nv_bfloat16) * ((size_t)ATT_KEYS * (a->dim + 8) + (size_t)ATT_KEYS * (a->vdim + 8)) +
                                (a->rel ? sizeof(float) * (size_t)AG * attn_rel_pitch(AP) : 0)
                          : sizeof(float) * ((size_t)ATT_PAIRS * a->dim + (size_t)ATT_KEYS * (a->dim + 4) + (size_t)ATT_KEYS * a->vdim + ATT_PAIRS * ATT_KEYS);
-  if (!wide && smem > 227 * 1024) return THA_STATUS_NOT_SUPPORTED;
+  const bool row_form = hyb_attn_row_ok(a, rows, kv, q);   // one row per sequence
+  if (!wide && !row_form && smem > 227 * 1024) return THA_STATUS_NOT_SUPPORTED;
   // position tiles: at most one ragged tile per sequence beyond rows / AP
   const int tiles = rows->n_rows / AP + rows->n_seqs;
   // few blocks and many keys (decoding at long contexts): deal the key tiles of a block to several
@@ -1794,6 +1807,21 @@ extern "C" int tha_hyb_attn_gated(void* stream, int dtype, const tha_attn_t* a, 
   int max_keys = a->chunk > 0 && a->chunk < seen ? a->chunk : seen;
   if (a->window > 0 && a->window + a->keep_first + 2 * ATT_KEYS < max_keys) max_keys = a->window + a->keep_first + 2 * ATT_KEYS;
   int splits = 1;
+  cudaStream_t s = (cudaStream_t)stream;
+  if (row_form) {
+    splits = split_scratch ? hyb_attn_row_splits(a, rows, max_keys) : 1;
+    while (splits > 1 && (size_t)splits * rows->n_rows * a->heads * (a->vdim + 2) > split_scratch_floats) splits--;
+    const int st = hyb_attn_row_launch(s, dtype, a, rows, kv, q, out, splits, split_scratch, gate, ldg);
+    if (st != THA_STATUS_SUCCESS || splits <= 1) return st;
+    const dim3 mgrid(ceil_div(rows->n_rows * a->heads, 4));
+    if (dtype != THA_DT_BF16 || a->out_f32)
+      THA_CUDA_OK(launch(hyb_attn_merge_kernel<float>, mgrid, dim3(128), 0, s, false, (float*)out, (const float*)split_scratch, rows->n_rows, a->heads, a->vdim,
+                         splits, *a, gate, ldg));
+    else
+      THA_CUDA_OK(launch(hyb_attn_merge_kernel<bf16>, mgrid, dim3(128), 0, s, false, (bf16*)out, (const float*)split_scratch, rows->n_rows, a->heads, a->vdim,
+                         splits, *a, gate, ldg));
+    return THA_STATUS_SUCCESS;
+  }
   const long long blocks = (long long)tiles * a->kv_heads * ceil_div(gsize, AG);
   if (split_scratch && blocks < 4 * 148 && max_keys >= 4 * ATT_KEYS) {
     splits = (int)((6 * 148 + blocks - 1) / blocks);
@@ -1802,7 +1830,6 @@ extern "C" int tha_hyb_attn_gated(void* stream, int dtype, const tha_attn_t* a, 
     while (splits > 1 && (size_t)splits * rows->n_rows * a->heads * (a->vdim + 2) > split_scratch_floats) splits--;
   }
   const dim3 grid(tiles * splits, a->kv_heads, ceil_div(gsize, AG));
-  cudaStream_t s = (cudaStream_t)stream;
   if (dtype == THA_DT_BF16) {
     if (wide) {
       const int st = hyb_attn_wide_launch(s, a, rows, kv, q, (bf16*)out, grid, pairs, AG, AP, splits, split_scratch);
