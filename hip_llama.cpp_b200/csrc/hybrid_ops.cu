@@ -560,7 +560,7 @@ __global__ void __launch_bounds__(128) hyb_attn_kernel(tha_attn_t a, tha_rows_t 
 
 // ------------------------------------------------------------------------------------------------------------------
 // the same attention on the tensor cores, for the bf16 number format and heads of up to 128 channels (multiples of 16 /
-// 8): a block takes 64 (position, query head) pairs of one K/V head, each of its 4 warps 16 of them.  Per tile of 32 keys
+// 8): a block takes 128 (position, query head) pairs of one K/V head, each of its 8 warps 16 of them.  Per tile of 32 keys
 // (aligned to absolute multiples of 32 as above): K rows and V rows go to shared memory as bf16, both row-major; a warp
 // computes its 16 x 32 scores with mma.sync m16n8k16 (q as the A operand from registers), scales and masks them in fp32,
 // keeps the online softmax of its rows among the four lanes that share a row, rounds the weights to bf16 (the row sums
@@ -568,8 +568,12 @@ __global__ void __launch_bounds__(128) hyb_attn_kernel(tha_attn_t a, tha_rows_t 
 // two adjacent 8-key score tiles are one 16-deep A operand.  No exchange between warps; accumulators fp32.
 // With a distance bias (REL) the block's heads x the distances a tile can meet (its positions + 31) are staged beside the keys; a tile
 // that lies wholly where the bias no longer changes adds one register per row instead.
+// The next tile's cache rows travel to registers while this one is computed and are rounded into the other half of a double buffer
+// behind it: one barrier per tile, no load latency between barriers (a block of 64 pairs that loaded, stored and computed a tile
+// one after the other ran at 43 TFLOP/s).  Fragments come by ldmatrix, tiles that every pair sees skip the masks, an accumulator is
+// rescaled only where some row's maximum moved.  Bound by mma.sync issue and the softmax between the two products.
 // ------------------------------------------------------------------------------------------------------------------
-constexpr int AM_PAIRS = 64, AM_MAXD = 128;
+constexpr int AM_WARPS = 8, AM_THREADS = 32 * AM_WARPS, AM_PAIRS = 16 * AM_WARPS, AM_MAXD = 128;
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
@@ -582,19 +586,28 @@ __device__ __forceinline__ float attn_softcap_fast(float s, float cap, float two
   return cap - __fdividef(2.0f * cap, 1.0f + __expf(s * two_over_cap));
 }
 
+__device__ __forceinline__ float attn_ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 __host__ __device__ inline int attn_rel_pitch(int AP) { return (AP + 31 - 8 + 31) / 32 * 32 + 8; }   // 8 banks from one head to the next
+// bytes of one half of the double buffer: [32][D + 8] keys, [32][E + 8] values, [AG][pitch] biases
+__host__ __device__ inline int attn_mma_stage(int D, int E, int AG, int AP, bool rel) {
+  return (int)sizeof(__nv_bfloat16) * ATT_KEYS * (D + 8 + E + 8) + (rel ? (int)sizeof(float) * AG * attn_rel_pitch(AP) : 0);
+}
 
 template <bool EXACT, bool CAP, bool REL>
-__global__ void __launch_bounds__(128, 3) hyb_attn_mma_kernel(tha_attn_t a, tha_rows_t rows, tha_kv_t kv, const float* __restrict__ q,
+__global__ void __launch_bounds__(AM_THREADS, 1) hyb_attn_mma_kernel(tha_attn_t a, tha_rows_t rows, tha_kv_t kv, const float* __restrict__ q,
                                                            __nv_bfloat16* __restrict__ out, int AG, int AP, int splits,
                                                            float* __restrict__ partial, const float* __restrict__ gate, long long ldg) {
   extern __shared__ __align__(16) unsigned char smraw[];
   const int D = a.dim, E = a.vdim, gsize = a.heads / a.kv_heads;
-  const int KS = D + 8, VS = E + 8;                      // padded rows: conflict-free fragment and ldmatrix reads
-  __nv_bfloat16* Ks = reinterpret_cast<__nv_bfloat16*>(smraw);   // [32][KS]
-  __nv_bfloat16* Vs = Ks + ATT_KEYS * KS;                        // [32][VS], row-major like the cache: transposed on the way out
-  const unsigned vs_base = (unsigned)__cvta_generic_to_shared(Vs);
-  float* Bs = REL ? reinterpret_cast<float*>(Vs + ATT_KEYS * VS) : nullptr;   // [AG][BP]: bias at distance (p_first - last key of the tile) + i
+  const int KS = D + 8, VS = E + 8;                      // padded rows: conflict-free ldmatrix reads
+  const int stage = attn_mma_stage(D, E, AG, AP, REL);
+  const unsigned sm_base = (unsigned)__cvta_generic_to_shared(smraw);
+  const int v_off = (int)sizeof(__nv_bfloat16) * ATT_KEYS * KS, b_off = v_off + (int)sizeof(__nv_bfloat16) * ATT_KEYS * VS;   // within a half
   const int BP = REL ? attn_rel_pitch(AP) : 0;
   int seq = -1, r0 = 0, r_end = 0;
   {
@@ -627,7 +640,7 @@ __global__ void __launch_bounds__(128, 3) hyb_attn_mma_kernel(tha_attn_t a, tha_
     row_ok[x] = pp < AP && row_r[x] < r_end && hg < gsize;
     row_pos[x] = p_first + pp;
     row_first[x] = a.chunk > 0 ? (row_pos[x] / a.chunk) * a.chunk : 0;
-    row_scale[x] = (a.head_scale && row_ok[x]) ? a.head_scale[row_h[x]] : 1.0f;
+    row_scale[x] = a.scale * ((a.head_scale && row_ok[x]) ? a.head_scale[row_h[x]] : 1.0f);
   }
   // q fragments: [k step][4]
   uint32_t qf[AM_MAXD / 16][4];
@@ -643,22 +656,23 @@ __global__ void __launch_bounds__(128, 3) hyb_attn_mma_kernel(tha_attn_t a, tha_
   }
   const float two_over_cap = CAP ? 2.0f / a.softcap : 0.f;
   float row_far[2] = {0.f, 0.f};
-  const float* row_bias[2] = {Bs, Bs};   // this row's bias at key 0 of a tile; key i of the tile is i entries before it
+  int row_bias[2] = {0, 0};   // this row's bias at key 0 of a tile (floats from the half's biases); key i of the tile is i entries before it
   if (REL) {
 #pragma unroll
     for (int x = 0; x < 2; x++) {
       const int pr = warp * 16 + lr + 8 * x;
       if (row_ok[x]) row_far[x] = hyb_attn_rel(a, row_h[x], a.rel_n - 1);
-      row_bias[x] = Bs + (pr % AG) * BP + min(pr / AG, AP - 1) + ATT_KEYS - 1 - lc;
+      row_bias[x] = (pr % AG) * BP + min(pr / AG, AP - 1) + ATT_KEYS - 1 - lc;
     }
   }
-  float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
+  float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f}, shift_run[2] = {INFINITY, INFINITY};   // shift: -m log2(e), rounded
   float oacc[AM_MAXD / 8][4];
 #pragma unroll
   for (int n = 0; n < AM_MAXD / 8; n++)
 #pragma unroll
     for (int v = 0; v < 4; v++) oacc[n][v] = 0.f;
   const int key_lo = a.chunk > 0 ? (p_first / a.chunk) * a.chunk : 0;
+  const int last_first = a.chunk > 0 ? (p_last / a.chunk) * a.chunk : 0;   // where the last position's visible keys begin
   const HybTiles tiles = hyb_attn_tiles(a, key_lo, p_first, p_last);
   int ti_begin = 0, ti_end = tiles.n;
   if (splits > 1) {
@@ -666,83 +680,61 @@ __global__ void __launch_bounds__(128, 3) hyb_attn_mma_kernel(tha_attn_t a, tha_
     ti_begin = sp * per;
     ti_end = min(tiles.n, ti_begin + per);
   }
-  // cache rows start on 16-byte boundaries when the pool's row pitch and the heads' offsets are multiples of four floats
-  const bool vec4 = (kv.kv_dim & 3) == 0 && ((D | E) & 3) == 0 && ((reinterpret_cast<size_t>(kv.k_pool) | reinterpret_cast<size_t>(kv.v_pool)) & 15) == 0;
-  for (int ti = ti_begin; ti < ti_end; ti++) {
-    const int kt = ti < tiles.n_a ? tiles.begin + ATT_KEYS * ti : tiles.resume + ATT_KEYS * (ti - tiles.n_a);
-    __syncthreads();
-    // stage the tile: a warp takes 8 keys, four at a time through registers
-    size_t krow[ATT_KEYS / 4];
+  auto tile_key = [&](int ti) { return ti < tiles.n_a ? tiles.begin + ATT_KEYS * ti : tiles.resume + ATT_KEYS * (ti - tiles.n_a); };
+  // cache rows start on 16-byte boundaries when the pool's row pitch is a multiple of four floats (the heads' offsets are)
+  const bool vec4 = (kv.kv_dim & 3) == 0 && ((reinterpret_cast<size_t>(kv.k_pool) | reinterpret_cast<size_t>(kv.v_pool)) & 15) == 0;
+  // a tile on its way: warp w holds keys w, w + 8, .. of it, a lane four channels of K and of V
+  float4 kbuf[ATT_KEYS / AM_WARPS], vbuf[ATT_KEYS / AM_WARPS];
+  auto fetch = [&](const float* pool, size_t row, int width, int head) -> float4 {
+    if (row == (size_t)-1 || 4 * lane >= width) return make_float4(0.f, 0.f, 0.f, 0.f);
+    const float* src = pool + row + (size_t)head * width + 4 * lane;
+    if (vec4) return __ldg(reinterpret_cast<const float4*>(src));
+    return make_float4(__ldg(src), __ldg(src + 1), __ldg(src + 2), __ldg(src + 3));
+  };
+  auto load_tile = [&](int kt) {
+    const int mine = kt + lane;   // a lane looks one key's row up
+    const size_t row = (mine <= p_last && mine >= key_lo) ? hyb_kv_row(kv, slot, mine, a.cache_layer) : (size_t)-1;
 #pragma unroll
-    for (int jj = 0; jj < ATT_KEYS / 4; jj++) {
-      const int t = kt + warp + 4 * jj;
-      krow[jj] = (t <= p_last && t >= key_lo) ? hyb_kv_row(kv, slot, t, a.cache_layer) : (size_t)-1;
+    for (int j = 0; j < ATT_KEYS / AM_WARPS; j++) {
+      const size_t at = __shfl_sync(THA_FULL_MASK, row, warp + AM_WARPS * j);
+      kbuf[j] = fetch(kv.k_pool, at, D, g);
+      vbuf[j] = fetch(kv.v_pool, at, E, gv);
     }
-    if (vec4) {
-      // 16-byte aligned cache rows: a lane takes four channels of a row in one 128-bit load (eight rows in flight) and leaves
-      // them as four bf16 in one 64-bit store
+  };
+  auto store_tile = [&](int kt, int half) {
+    unsigned char* base = smraw + half * stage;
+    __nv_bfloat16 *Ks = reinterpret_cast<__nv_bfloat16*>(base), *Vs = reinterpret_cast<__nv_bfloat16*>(base + v_off);
 #pragma unroll
-      for (int which = 0; which < 2; which++) {
-        const float* pool = which ? kv.v_pool : kv.k_pool;
-        const int width4 = (which ? E : D) >> 2;
-        float4 buf[ATT_KEYS / 4];
-#pragma unroll
-        for (int jj = 0; jj < ATT_KEYS / 4; jj++) {
-          const bool live = krow[jj] != (size_t)-1 && lane < width4;
-          const float4* src = reinterpret_cast<const float4*>(pool + (live ? krow[jj] : 0) + (size_t)(which ? gv : g) * (width4 << 2));
-          buf[jj] = live ? __ldg(src + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-        if (lane < width4) {
-#pragma unroll
-          for (int jj = 0; jj < ATT_KEYS / 4; jj++) {
-            const int j = warp + 4 * jj;
-            uint2 pk;
-            pk.x = pack_bf16(buf[jj].x, buf[jj].y);
-            pk.y = pack_bf16(buf[jj].z, buf[jj].w);
-            *reinterpret_cast<uint2*>((which ? Vs + j * VS : Ks + j * KS) + 4 * lane) = pk;
-          }
-        }
-      }
-    } else {
-#pragma unroll
-    for (int which = 0; which < 2; which++) {
-      const float* pool = which ? kv.v_pool : kv.k_pool;
-      const int width = which ? E : D;
-      const int gh = which ? gv : g;
-#pragma unroll
-      for (int j0 = 0; j0 < ATT_KEYS / 4; j0 += 4) {
-        float buf[4][AM_MAXD / 32];
-#pragma unroll
-        for (int jj = 0; jj < 4; jj++) {
-          const bool live = krow[j0 + jj] != (size_t)-1;
-          const float* src = pool + (live ? krow[j0 + jj] : 0) + (size_t)gh * width;
-#pragma unroll
-          for (int c = 0; c < AM_MAXD / 32; c++) buf[jj][c] = (live && lane + 32 * c < width) ? __ldg(src + lane + 32 * c) : 0.f;
-        }
-#pragma unroll
-        for (int jj = 0; jj < 4; jj++) {
-          const int j = warp + 4 * (j0 + jj);
-#pragma unroll
-          for (int c = 0; c < AM_MAXD / 32; c++) {
-            const int d = lane + 32 * c;
-            if (d < width) {
-              if (which) Vs[j * VS + d] = __float2bfloat16_rn(buf[jj][c]);
-              else Ks[j * KS + d] = __float2bfloat16_rn(buf[jj][c]);
-            }
-          }
-        }
-      }
+    for (int j = 0; j < ATT_KEYS / AM_WARPS; j++) {
+      const int key = warp + AM_WARPS * j;
+      if (4 * lane < D) *reinterpret_cast<uint2*>(Ks + key * KS + 4 * lane) = make_uint2(pack_bf16(kbuf[j].x, kbuf[j].y), pack_bf16(kbuf[j].z, kbuf[j].w));
+      if (4 * lane < E) *reinterpret_cast<uint2*>(Vs + key * VS + 4 * lane) = make_uint2(pack_bf16(vbuf[j].x, vbuf[j].y), pack_bf16(vbuf[j].z, vbuf[j].w));
     }
-    }
-    const bool near = REL && p_first - (kt + ATT_KEYS - 1) < a.rel_n - 1;   // the same for the whole block
-    if (near) {
-      const int d0 = p_first - (kt + ATT_KEYS - 1);
-      for (int i = threadIdx.x; i < AG * (AP + ATT_KEYS - 1); i += blockDim.x) {
+    const int d0 = p_first - (kt + ATT_KEYS - 1);
+    if (REL && d0 < a.rel_n - 1) {
+      float* Bs = reinterpret_cast<float*>(base + b_off);
+      for (int i = threadIdx.x; i < AG * (AP + ATT_KEYS - 1); i += AM_THREADS) {
         const int hl = i / (AP + ATT_KEYS - 1), n = i - hl * (AP + ATT_KEYS - 1), hg = part * AG + hl;
         Bs[hl * BP + n] = hg < gsize ? hyb_attn_rel(a, g * gsize + hg, d0 + n) : 0.f;
       }
     }
-    __syncthreads();
+  };
+  if (ti_begin < ti_end) {
+    const int kt = tile_key(ti_begin);
+    load_tile(kt);
+    store_tile(kt, 0);
+  }
+  __syncthreads();
+  constexpr float LOG2E = 1.4426950408889634f;
+  for (int ti = ti_begin, half = 0; ti < ti_end; ti++, half ^= 1) {
+    const int kt = tile_key(ti);
+    const bool more = ti + 1 < ti_end;
+    if (more) load_tile(tile_key(ti + 1));
+    const unsigned ks_base = sm_base + (unsigned)(half * stage), vs_base = ks_base + (unsigned)v_off;
+    const bool near = REL && p_first - (kt + ATT_KEYS - 1) < a.rel_n - 1;   // the same for the whole block
+    const float* Bs = REL ? reinterpret_cast<const float*>(smraw + half * stage + b_off) : nullptr;
+    // every position of the block sees every key of the tile
+    const bool whole = kt + ATT_KEYS - 1 <= p_first && kt >= last_first && (a.window <= 0 || p_last - kt < a.window || kt + ATT_KEYS <= a.keep_first);
     // scores of this warp's 16 pairs against the 32 keys
     float sacc[4][4];
 #pragma unroll
@@ -753,17 +745,20 @@ __global__ void __launch_bounds__(128, 3) hyb_attn_mma_kernel(tha_attn_t a, tha_
     for (int ks = 0; ks < AM_MAXD / 16; ks++) {
       if (16 * ks < D) {
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-          uint32_t b[2];
-          const __nv_bfloat16* kr = Ks + (8 * j + lr) * KS + 16 * ks + lc;
-          b[0] = *reinterpret_cast<const uint32_t*>(kr);
-          b[1] = *reinterpret_cast<const uint32_t*>(kr + 8);
-          mma_bf16_16816(sacc[j], qf[ks], b);
+        for (int j = 0; j < 4; j += 2) {
+          // lanes 0..7 and 8..15 name the rows of keys 8 j .. at this k step's two halves, lanes 16..31 those of the next eight keys
+          uint32_t b[4];
+          const unsigned addr = ks_base + (unsigned)(((8 * j + (lane & 7) + ((lane & 16) >> 1)) * KS + 16 * ks + (lane & 8)) * sizeof(__nv_bfloat16));
+          asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]) : "r"(addr));
+          const uint32_t b0[2] = {b[0], b[1]}, b1[2] = {b[2], b[3]};
+          mma_bf16_16816(sacc[j], qf[ks], b0);
+          mma_bf16_16816(sacc[j + 1], qf[ks], b1);
         }
       }
     }
     // scale, mask, online softmax of rows A (values 0, 1 of every score tile) and B (values 2, 3)
     uint32_t pa[2][4], pl[2][4];   // the weights as A operands: rounded to bf16, and (EXACT) what the rounding left over
+    float corr[2];
 #pragma unroll
     for (int x = 0; x < 2; x++) {
       float mx = -INFINITY;
@@ -771,24 +766,26 @@ __global__ void __launch_bounds__(128, 3) hyb_attn_mma_kernel(tha_attn_t a, tha_
       for (int j = 0; j < 4; j++)
 #pragma unroll
         for (int y = 0; y < 2; y++) {
-          const int t = kt + 8 * j + lc + y;
-          const bool vis = row_ok[x] && hyb_attn_sees(a, t, row_pos[x], row_first[x]);
-          float sv = sacc[j][2 * x + y] * a.scale * row_scale[x];
+          float sv = sacc[j][2 * x + y] * row_scale[x];
           if (CAP) sv = attn_softcap_fast(sv, a.softcap, two_over_cap);
-          if (REL) sv += near ? row_bias[x][-(8 * j + y)] : row_far[x];
-          if (!vis) sv = -INFINITY;
+          if (REL) sv += near ? Bs[row_bias[x] - (8 * j + y)] : row_far[x];
+          if (!whole) {
+            const int t = kt + 8 * j + lc + y;
+            if (!(row_ok[x] && hyb_attn_sees(a, t, row_pos[x], row_first[x]))) sv = -INFINITY;
+          }
           sacc[j][2 * x + y] = sv;
           mx = fmaxf(mx, sv);
         }
       mx = fmaxf(mx, __shfl_xor_sync(THA_FULL_MASK, mx, 1));
       mx = fmaxf(mx, __shfl_xor_sync(THA_FULL_MASK, mx, 2));
       const float m_new = fmaxf(m_run[x], mx);
-      const float corr = m_new > -INFINITY ? expf(m_run[x] - m_new) : 1.f;
+      const float shift = m_new > -INFINITY ? -m_new * LOG2E : 0.f;   // nothing seen yet: every weight is 2^-inf = 0
+      corr[x] = 1.f;
+      if (m_new > -INFINITY) { corr[x] = attn_ex2(shift - shift_run[x]); shift_run[x] = shift; }   // exactly 1 while the maximum stays
       float sum = 0.f;
 #pragma unroll
       for (int j = 0; j < 4; j++) {
-        float p0 = 0.f, p1 = 0.f;
-        if (m_new > -INFINITY) { p0 = expf(sacc[j][2 * x] - m_new); p1 = expf(sacc[j][2 * x + 1] - m_new); }   // exp(-inf) = 0 for masked keys
+        const float p0 = attn_ex2(fmaf(sacc[j][2 * x], LOG2E, shift)), p1 = attn_ex2(fmaf(sacc[j][2 * x + 1], LOG2E, shift));
         const __nv_bfloat162 pr = __floats2bfloat162_rn(p0, p1);
         if (EXACT) {   // hi + lo carry 16 mantissa bits of the fp32 weight; the sum adds the fp32 weights themselves
           sum += p0 + p1;
@@ -800,10 +797,12 @@ __global__ void __launch_bounds__(128, 3) hyb_attn_mma_kernel(tha_attn_t a, tha_
       }
       sum += __shfl_xor_sync(THA_FULL_MASK, sum, 1);
       sum += __shfl_xor_sync(THA_FULL_MASK, sum, 2);
-      l_run[x] = l_run[x] * corr + sum;
+      l_run[x] = l_run[x] * corr[x] + sum;
       m_run[x] = m_new;
+    }
+    if (__any_sync(THA_FULL_MASK, corr[0] != 1.f || corr[1] != 1.f)) {
 #pragma unroll
-      for (int n = 0; n < AM_MAXD / 8; n++) { oacc[n][2 * x] *= corr; oacc[n][2 * x + 1] *= corr; }
+      for (int n = 0; n < AM_MAXD / 8; n++) { oacc[n][0] *= corr[0]; oacc[n][1] *= corr[0]; oacc[n][2] *= corr[1]; oacc[n][3] *= corr[1]; }
     }
     // weights times values: two k steps of 16 keys, two channel tiles per ldmatrix.  Values [key][channel] row-major,
     // transposed on the way: lanes 0..15 name the rows of keys 16 t2 + (lane & 15) at this channel tile, lanes 16..31 the same
@@ -821,14 +820,16 @@ __global__ void __launch_bounds__(128, 3) hyb_attn_mma_kernel(tha_attn_t a, tha_
                        : "=r"(vf[0]), "=r"(vf[1]), "=r"(vf[2]), "=r"(vf[3]) : "r"(addr));
           const uint32_t v0[2] = {vf[0], vf[1]}, v1[2] = {vf[2], vf[3]};
           mma_bf16_16816(oacc[n], pa[t2], v0);
-          if (EXACT) mma_bf16_16816(oacc[n], pl[t2], v0);
-          if (two) {
-            mma_bf16_16816(oacc[n + 1], pa[t2], v1);
-            if (EXACT) mma_bf16_16816(oacc[n + 1], pl[t2], v1);
+          if (two) mma_bf16_16816(oacc[n + 1], pa[t2], v1);
+          if (EXACT) {
+            mma_bf16_16816(oacc[n], pl[t2], v0);
+            if (two) mma_bf16_16816(oacc[n + 1], pl[t2], v1);
           }
         }
       }
     }
+    if (more) store_tile(tile_key(ti + 1), half ^ 1);   // its last readers passed the barrier of the tile before
+    __syncthreads();
   }
 #pragma unroll
   for (int x = 0; x < 2; x++) {
@@ -1779,6 +1780,15 @@ static bool hyb_tc_attn() {
   return on != 0;
 }
 
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_smem(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, bool pdl, Args... args) {
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  return launch(kernel, grid, block, smem, s, pdl, args...);
+}
+
 extern "C" int tha_hyb_attn_gated(void* stream, int dtype, const tha_attn_t* a, const tha_rows_t* rows, const tha_kv_t* kv, const float* q,
                                   void* out, float* split_scratch, size_t split_scratch_floats, const float* proj, long long ldp) {
   if (rows->n_rows < 1) return THA_STATUS_SUCCESS;
@@ -1795,8 +1805,7 @@ extern "C" int tha_hyb_attn_gated(void* stream, int dtype, const tha_attn_t* a, 
   const bool wide = !tc && !a->rel && !gate && !a->head_scale && a->softcap <= 0.f && !a->out_f32 && a->v_share <= 1 && dtype == THA_DT_BF16 && hyb_tc_linear() && hyb_tc_attn() && hyb_attn_wide_ok(a);
   const int pairs = wide ? hyb_attn_wide_pairs(a, rows) : tc ? AM_PAIRS : ATT_PAIRS;
   const int AG = gsize < pairs ? gsize : pairs, AP = pairs / AG;
-  const size_t smem = tc ? sizeof(__nv_bfloat16) * ((size_t)ATT_KEYS * (a->dim + 8) + (size_t)ATT_KEYS * (a->vdim + 8)) +
-                               (a->rel ? sizeof(float) * (size_t)AG * attn_rel_pitch(AP) : 0)
+  const size_t smem = tc ? 2 * (size_t)attn_mma_stage(a->dim, a->vdim, AG, AP, a->rel != nullptr)
                          : sizeof(float) * ((size_t)ATT_PAIRS * a->dim + (size_t)ATT_KEYS * (a->dim + 4) + (size_t)ATT_KEYS * a->vdim + ATT_PAIRS * ATT_KEYS);
   const bool row_form = hyb_attn_row_ok(a, rows, kv, q);   // one row per sequence
   if (!wide && !row_form && smem > 227 * 1024) return THA_STATUS_NOT_SUPPORTED;
@@ -1823,8 +1832,9 @@ extern "C" int tha_hyb_attn_gated(void* stream, int dtype, const tha_attn_t* a, 
     return THA_STATUS_SUCCESS;
   }
   const long long blocks = (long long)tiles * a->kv_heads * ceil_div(gsize, AG);
-  if (split_scratch && blocks < 4 * 148 && max_keys >= 4 * ATT_KEYS) {
-    splits = (int)((6 * 148 + blocks - 1) / blocks);
+  const int fill = tc ? 2 * 148 : 4 * 148;   // blocks from which the SMs are full without splits (the tensor-core form: one block of 8 warps each)
+  if (split_scratch && blocks < fill && max_keys >= 4 * ATT_KEYS) {
+    splits = (int)((fill + fill / 2 + blocks - 1) / blocks);
     if (splits > max_keys / (2 * ATT_KEYS)) splits = max_keys / (2 * ATT_KEYS);
     if (splits > 16) splits = 16;
     while (splits > 1 && (size_t)splits * rows->n_rows * a->heads * (a->vdim + 2) > split_scratch_floats) splits--;
@@ -1836,13 +1846,13 @@ extern "C" int tha_hyb_attn_gated(void* stream, int dtype, const tha_attn_t* a, 
       if (st != THA_STATUS_SUCCESS) return st;
     } else if (tc) {
       if (a->rel)
-        THA_CUDA_OK(launch(hyb_attn_mma_kernel<true, false, true>, grid, dim3(128), smem, s, false, *a, *rows, *kv, q, (bf16*)out, AG, AP, splits, split_scratch, gate, ldg));
+        THA_CUDA_OK(launch_smem(hyb_attn_mma_kernel<true, false, true>, grid, dim3(AM_THREADS), smem, s, false, *a, *rows, *kv, q, (bf16*)out, AG, AP, splits, split_scratch, gate, ldg));
       else if (a->softcap > 0.f)
-        THA_CUDA_OK(launch(hyb_attn_mma_kernel<true, true, false>, grid, dim3(128), smem, s, false, *a, *rows, *kv, q, (bf16*)out, AG, AP, splits, split_scratch, gate, ldg));
+        THA_CUDA_OK(launch_smem(hyb_attn_mma_kernel<true, true, false>, grid, dim3(AM_THREADS), smem, s, false, *a, *rows, *kv, q, (bf16*)out, AG, AP, splits, split_scratch, gate, ldg));
       else if (a->fp32_scores)
-        THA_CUDA_OK(launch(hyb_attn_mma_kernel<true, false, false>, grid, dim3(128), smem, s, false, *a, *rows, *kv, q, (bf16*)out, AG, AP, splits, split_scratch, gate, ldg));
+        THA_CUDA_OK(launch_smem(hyb_attn_mma_kernel<true, false, false>, grid, dim3(AM_THREADS), smem, s, false, *a, *rows, *kv, q, (bf16*)out, AG, AP, splits, split_scratch, gate, ldg));
       else
-        THA_CUDA_OK(launch(hyb_attn_mma_kernel<false, false, false>, grid, dim3(128), smem, s, false, *a, *rows, *kv, q, (bf16*)out, AG, AP, splits, split_scratch, gate, ldg));
+        THA_CUDA_OK(launch_smem(hyb_attn_mma_kernel<false, false, false>, grid, dim3(AM_THREADS), smem, s, false, *a, *rows, *kv, q, (bf16*)out, AG, AP, splits, split_scratch, gate, ldg));
     } else {
       if (a->vdim <= 256) {
         if (smem > 48 * 1024) THA_CUDA_OK(cudaFuncSetAttribute(hyb_attn_kernel<bf16, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
