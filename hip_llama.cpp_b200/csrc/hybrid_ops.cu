@@ -857,37 +857,33 @@ __global__ void __launch_bounds__(AM_THREADS, 1) hyb_attn_mma_kernel(tha_attn_t 
   }
 }
 
-// the splits of a (row, head) in ascending key order: out = sum_s acc_s e^(m_s - M) / sum_s l_s e^(m_s - M); a warp each.  Lane s
-// keeps split s's maximum, sum and factor (at most 32 splits); eight splits' values of a channel are in flight at once (the sums one
-// load after the other took 32 us for 16 splits of 2 rows).
+// the splits of a (row, head) in ascending key order: out = sum_s acc_s e^(m_s - M) / sum_s l_s e^(m_s - M); a block per (row, head), a warp
+// per 32 channels.  Lane s keeps split s's maximum, sum and factor (at most 32 splits); a channel's values of all splits are in
+// flight at once (one load after the other took 32 us for 16 splits of 2 rows, eight at a time and a warp for all channels 20 us for 32).
+constexpr int AMG_SPLITS = 32;
 template <typename T>
-__global__ void hyb_attn_merge_kernel(T* __restrict__ out, const float* __restrict__ partial, int n_rows, int heads, int E, int splits,
-                                      tha_attn_t a, const float* __restrict__ gate, long long ldg) {
-  const int idx = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (idx >= n_rows * heads) return;
+__global__ void __launch_bounds__(128) hyb_attn_merge_kernel(T* __restrict__ out, const float* __restrict__ partial, int n_rows, int heads, int E, int splits,
+                                                             tha_attn_t a, const float* __restrict__ gate, long long ldg) {
+  const int idx = blockIdx.x, lane = threadIdx.x & 31;
   const size_t stride = (size_t)n_rows * heads * (E + 2);
   const float* p0 = partial + (size_t)idx * (E + 2);
   const float ms = lane < splits ? p0[lane * stride + E] : -INFINITY, ls = lane < splits ? p0[lane * stride + E + 1] : 0.f;
-  const float M = warp_max(ms);
-  const float w = ms > -INFINITY ? expf(ms - M) : 0.f;   // splits that saw nothing have factor 0 and do not enter the sums
-  const float L = warp_sum(w > 0.f ? ls * w : 0.f);
   const int row = idx / heads, head = idx - row * heads;
-  const float fin = hyb_attn_final_factor(a, head, M, L, gate ? gate + (size_t)row * ldg : nullptr);
-  // every lane walks every group of 32 channels (the shuffles need the whole warp), also where E is not a multiple of 32
-  for (int e0 = 0; e0 < E; e0 += 32) {
+  for (int e0 = (threadIdx.x >> 5) * 32; e0 < E; e0 += blockDim.x) {
     const int e = e0 + lane;
+    float v[AMG_SPLITS];
+#pragma unroll
+    for (int u = 0; u < AMG_SPLITS; u++) v[u] = (u < splits && e < E) ? p0[(size_t)u * stride + e] : 0.f;
+    const float M = warp_max(ms);
+    const float w = ms > -INFINITY ? expf(ms - M) : 0.f;   // splits that saw nothing have factor 0 and do not enter the sums
+    const float L = warp_sum(w > 0.f ? ls * w : 0.f);
     float o = 0.f;
-    for (int s0 = 0; s0 < splits; s0 += 8) {
-      float v[8];
 #pragma unroll
-      for (int u = 0; u < 8; u++) v[u] = (s0 + u < splits && e < E) ? p0[(size_t)(s0 + u) * stride + e] : 0.f;
-#pragma unroll
-      for (int u = 0; u < 8; u++) {
-        const float ws = __shfl_sync(THA_FULL_MASK, w, s0 + u);
-        if (ws > 0.f) o = fmaf(v[u], ws, o);
-      }
+    for (int u = 0; u < AMG_SPLITS; u++) {
+      const float ws = __shfl_sync(THA_FULL_MASK, w, u);
+      if (ws > 0.f) o = fmaf(v[u], ws, o);
     }
-    if (e < E) hyb_store(out + (size_t)idx * E + e, o * fin);
+    if (e < E) hyb_store(out + (size_t)idx * E + e, o * hyb_attn_final_factor(a, head, M, L, gate ? gate + (size_t)row * ldg : nullptr));
   }
 }
 
@@ -1822,7 +1818,7 @@ extern "C" int tha_hyb_attn_gated(void* stream, int dtype, const tha_attn_t* a, 
     while (splits > 1 && (size_t)splits * rows->n_rows * a->heads * (a->vdim + 2) > split_scratch_floats) splits--;
     const int st = hyb_attn_row_launch(s, dtype, a, rows, kv, q, out, splits, split_scratch, gate, ldg);
     if (st != THA_STATUS_SUCCESS || splits <= 1) return st;
-    const dim3 mgrid(ceil_div(rows->n_rows * a->heads, 4));
+    const dim3 mgrid(rows->n_rows * a->heads);
     if (dtype != THA_DT_BF16 || a->out_f32)
       THA_CUDA_OK(launch(hyb_attn_merge_kernel<float>, mgrid, dim3(128), 0, s, false, (float*)out, (const float*)split_scratch, rows->n_rows, a->heads, a->vdim,
                          splits, *a, gate, ldg));
@@ -1863,10 +1859,10 @@ extern "C" int tha_hyb_attn_gated(void* stream, int dtype, const tha_attn_t* a, 
       }
     }
     if (splits > 1 && a->out_f32)
-      THA_CUDA_OK(launch(hyb_attn_merge_kernel<float>, dim3(ceil_div(rows->n_rows * a->heads, 4)), dim3(128), 0, s, false, (float*)out,
+      THA_CUDA_OK(launch(hyb_attn_merge_kernel<float>, dim3(rows->n_rows * a->heads), dim3(128), 0, s, false, (float*)out,
                          (const float*)split_scratch, rows->n_rows, a->heads, a->vdim, splits, *a, gate, ldg));
     else if (splits > 1)
-      THA_CUDA_OK(launch(hyb_attn_merge_kernel<bf16>, dim3(ceil_div(rows->n_rows * a->heads, 4)), dim3(128), 0, s, false, (bf16*)out,
+      THA_CUDA_OK(launch(hyb_attn_merge_kernel<bf16>, dim3(rows->n_rows * a->heads), dim3(128), 0, s, false, (bf16*)out,
                          (const float*)split_scratch, rows->n_rows, a->heads, a->vdim, splits, *a, gate, ldg));
   } else {
     if (a->vdim <= 256) {
@@ -1877,7 +1873,7 @@ extern "C" int tha_hyb_attn_gated(void* stream, int dtype, const tha_attn_t* a, 
       THA_CUDA_OK(launch(hyb_attn_kernel<float, 16>, grid, dim3(128), smem, s, false, *a, *rows, *kv, q, (float*)out, AG, AP, splits, split_scratch, gate, ldg));
     }
     if (splits > 1)
-      THA_CUDA_OK(launch(hyb_attn_merge_kernel<float>, dim3(ceil_div(rows->n_rows * a->heads, 4)), dim3(128), 0, s, false, (float*)out,
+      THA_CUDA_OK(launch(hyb_attn_merge_kernel<float>, dim3(rows->n_rows * a->heads), dim3(128), 0, s, false, (float*)out,
                          (const float*)split_scratch, rows->n_rows, a->heads, a->vdim, splits, *a, gate, ldg));
   }
   return THA_STATUS_SUCCESS;
