@@ -3,12 +3,14 @@
 // which is quadratic in traffic for a long prompt).
 //
 // Same arithmetic as the reference's per-position loop (run.cc:288-321: score = q.k / sqrt(hs),
-// softmax over t <= pos, weighted sum of V) evaluated tile by tile with an online softmax:
-//   CTA = 64 consecutive query rows of one (sequence, head); loop over 64-key tiles of the cache
+// softmax over t <= pos, weighted sum of V) evaluated tile by tile with an online softmax, all of it in fp32:
+//   CTA = 16 RI consecutive query rows (64 or 128) of one (sequence, head); loop over 64-key tiles of the cache
 //   (which already holds this layer's K/V rows of the chunk -- tc_rope_scatter_kernel ran first);
-//   S = Q K^T on a 4x4 register micro-tile per thread out of transposed shared-memory tiles
-//   (conflict-free 128-bit reads), running max / sum per row, P staged in shared memory, O += P V.
-// K/V tiles are read once per 64 queries; scores never leave the SM.
+//   S = Q K^T on an RI x 4 register micro-tile per thread (rows ty + 16 i, keys tx + 16 j, four channels per 128-bit
+//   shared-memory read), running max / sum per row, P staged in shared memory, O += P V.
+// K and V tiles arrive by cp.async, whole rows at a time: V of a tile while its scores are computed, K of the next one under P V -- one
+// buffer each and two barriers per tile.  Bound by fp32 FMA (128 per SM and clock; two LDS.128 per 16 FMAs at RI = 8).
+// The longest tiles start first.
 #include "common.cuh"
 #include "workspace.h"
 
@@ -19,28 +21,35 @@ struct AttnPrefillP {
   const float* kc; const float* vc;                           // cache base of the layer
   long long kv_batch_stride; int kv_dim, kv_mul, dim;
   const int* row_slot; const int* row_pos;                    // [rows]
-  const int* tile_row0; const int* tile_n;                    // [tiles]: first row and row count (<= 64) of each query tile
+  const int* tile_row0; const int* tile_n;                    // [tiles]: first row and row count (<= 16 RI) of each query tile
   KvPaged pg;                                                 // pg.table != nullptr: kc / vc are block pools, rows found through the table
 };
 
-constexpr int PF_TQ = 64, PF_TK = 64;
+constexpr int PF_TK = 64, PF_PS = PF_TK + 4;   // keys per tile, row pitch of P
 
 __device__ __forceinline__ float pf_tf32(float v) { return __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xFFFFE000u); }
+__device__ __forceinline__ void pf_cp16(float* dst, const float* src, bool live) {   // 16 bytes, zeros where the key is past the end
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
 
-template <int HS>
+template <int HS, int RI>
+constexpr size_t pf_smem() { return ((size_t)(16 * RI + PF_TK) * (HS + 4) + (size_t)PF_TK * HS + (size_t)16 * RI * PF_PS) * sizeof(float); }
+
+template <int HS, int RI>
 __global__ void __launch_bounds__(256) attn_prefill_kernel(const AttnPrefillP p) {
+  constexpr int TQ = 16 * RI, KS = HS + 4;   // rows pitched by 4 banks: conflict-free 128-bit reads of 16 neighbouring rows
   constexpr int CW = HS / 16;              // output columns per thread
   constexpr int NV = (CW >= 4) ? CW / 4 : 1;
   constexpr int VW = (CW >= 4) ? 4 : CW;   // floats per V read
   extern __shared__ float4 pf_smem4[];
-  float* Qt = reinterpret_cast<float*>(pf_smem4);   // [HS][64]   Qt[k][row]
-  float* Kt = Qt + HS * PF_TQ;                       // [HS][64]   Kt[k][key]
-  float* Vs = Kt + HS * PF_TK;                       // [64][HS]
-  float* Ps = Vs + PF_TK * HS;                       // [64][64]   P[row][key]
+  float* Qs = reinterpret_cast<float*>(pf_smem4);   // [TQ][KS]
+  float* Ks = Qs + TQ * KS;                          // [64][KS]
+  float* Vs = Ks + PF_TK * KS;                       // [64][HS]
+  float* Ps = Vs + PF_TK * HS;                       // [TQ][PF_PS]
 
   pdl_wait();
   pdl_trigger();
-  const int tile = blockIdx.x, h = blockIdx.y;
+  const int heads = p.dim / HS, tile = blockIdx.x / heads, h = blockIdx.x - tile * heads;   // the heads of a tile side by side
   const int row0 = p.tile_row0[tile], n = p.tile_n[tile];
   const int slot = p.row_slot[row0], pos0 = p.row_pos[row0];
   if (pos0 < 0 || n <= 0) return;
@@ -49,101 +58,99 @@ __global__ void __launch_bounds__(256) attn_prefill_kernel(const AttnPrefillP p)
   const float* kbase = (p.pg.table ? p.kc : p.kc + (size_t)slot * p.kv_batch_stride) + kh * HS;
   const float* vbase = (p.pg.table ? p.vc : p.vc + (size_t)slot * p.kv_batch_stride) + kh * HS;
   const int kmax = pos0 + n - 1;   // last key any row of the tile may see
-  const float sqrt_hs = sqrtf((float)HS);
+  const float inv_sqrt_hs = 1.0f / sqrtf((float)HS);
+  constexpr int C4 = HS / 4;       // float4 per row
 
-  // ---- Q tile, transposed: thread = (row, every 4th float4 column) ----
-  {
-    const int r = tid & 63, c0 = tid >> 6;
-    const int rr = (r < n) ? r : n - 1;
-    const float* qrow = p.q + (size_t)(row0 + rr) * p.dim + h * HS;
-    for (int c = c0; c < HS / 4; c += 4) {
-      const float4 v = *reinterpret_cast<const float4*>(qrow + 4 * c);
-      Qt[(4 * c + 0) * PF_TQ + r] = v.x; Qt[(4 * c + 1) * PF_TQ + r] = v.y;
-      Qt[(4 * c + 2) * PF_TQ + r] = v.z; Qt[(4 * c + 3) * PF_TQ + r] = v.w;
-    }
-  }
-
-  float m[4], l[4], o[4][CW];
+  // keys tk0 .. tk0 + 63 -> dst (row pitch `pitch`): consecutive threads take consecutive 16-byte pieces of a row
+  auto load_rows = [&](float* dst, int pitch, const float* base, int tk0) {
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    m[i] = -INFINITY; l[i] = 0.0f;
-#pragma unroll
-    for (int c = 0; c < CW; c++) o[i][c] = 0.0f;
-  }
-  int qpos[4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) { const int r = ty * 4 + i; qpos[i] = pos0 + ((r < n) ? r : n - 1); }
-
-  for (int tk0 = 0; tk0 <= kmax; tk0 += PF_TK) {
-    __syncthreads();   // the previous tile's K/V/P are no longer read (also orders the Q stores the first time)
-    {
-      const int r = tid & 63, c0 = tid >> 6;
+    for (int i0 = 0; i0 < PF_TK * C4; i0 += 256) {
+      const int i = i0 + tid, r = i / C4, c = i - r * C4;
       const int t = tk0 + r;
       const bool live = t <= kmax;
       const int tr = live ? t : kmax;
       const long long roff = p.pg.table ? kv_paged_off(p.pg, slot, tr, p.kv_dim) : (long long)tr * p.kv_dim;
-      const float* krow = kbase + roff;
-      const float* vrow = vbase + roff;
-      for (int c = c0; c < HS / 4; c += 4) {
-        const float4 kv = *reinterpret_cast<const float4*>(krow + 4 * c);
-        Kt[(4 * c + 0) * PF_TK + r] = kv.x; Kt[(4 * c + 1) * PF_TK + r] = kv.y;
-        Kt[(4 * c + 2) * PF_TK + r] = kv.z; Kt[(4 * c + 3) * PF_TK + r] = kv.w;
-        float4 vv = *reinterpret_cast<const float4*>(vrow + 4 * c);
-        if (!live) vv = make_float4(0.f, 0.f, 0.f, 0.f);   // a masked key has weight 0; keep 0 * garbage out of the sum
-        *reinterpret_cast<float4*>(Vs + r * HS + 4 * c) = vv;
-      }
+      pf_cp16(dst + r * pitch + 4 * c, base + roff + 4 * c, live);
     }
-    __syncthreads();
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  static_assert(PF_TK * C4 % 256 == 0, "every thread copies the same number of pieces");
+  load_rows(Ks, KS, kbase, 0);
+  for (int i = tid; i < TQ * C4; i += 256) {
+    const int r = i / C4, c = i - r * C4;
+    *reinterpret_cast<float4*>(Qs + r * KS + 4 * c) = *reinterpret_cast<const float4*>(p.q + (size_t)(row0 + (r < n ? r : n - 1)) * p.dim + h * HS + 4 * c);
+  }
 
-    // ---- S = Q K^T : rows ty*4.., keys tx*4.. ----
-    float s[4][4];
+  float m[RI], l[RI], o[RI][CW];
+  int qpos[RI];
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+  for (int i = 0; i < RI; i++) {
+    m[i] = -INFINITY; l[i] = 0.0f;
+    const int r = ty + 16 * i;
+    qpos[i] = pos0 + ((r < n) ? r : n - 1);
+#pragma unroll
+    for (int c = 0; c < CW; c++) o[i][c] = 0.0f;
+  }
+
+  for (int tk0 = 0; tk0 <= kmax; tk0 += PF_TK) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();   // this tile's K is in place (and Q, the first time); the previous tile's V and P are no longer read
+    load_rows(Vs, HS, vbase, tk0);
+
+    // ---- S = Q K^T : rows ty + 16 i, keys tx + 16 j ----
+    float s[RI][4];
+#pragma unroll
+    for (int i = 0; i < RI; i++)
 #pragma unroll
       for (int j = 0; j < 4; j++) s[i][j] = 0.0f;
-#pragma unroll 8
-    for (int k = 0; k < HS; k++) {
-      const float4 a = *reinterpret_cast<const float4*>(Qt + k * PF_TQ + ty * 4);
-      const float4 b = *reinterpret_cast<const float4*>(Kt + k * PF_TK + tx * 4);
-      const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll 2
+    for (int k = 0; k < HS; k += 4) {
+      float4 b[4];
 #pragma unroll
-      for (int i = 0; i < 4; i++)
+      for (int j = 0; j < 4; j++) b[j] = *reinterpret_cast<const float4*>(Ks + (tx + 16 * j) * KS + k);
 #pragma unroll
-        for (int j = 0; j < 4; j++) s[i][j] = fmaf(av[i], bv[j], s[i][j]);
+      for (int i = 0; i < RI; i++) {
+        const float4 a = *reinterpret_cast<const float4*>(Qs + (ty + 16 * i) * KS + k);
+#pragma unroll
+        for (int j = 0; j < 4; j++) s[i][j] = dot4(a, b[j], s[i][j]);
+      }
     }
     // ---- scale, causal mask, online softmax (row statistics shared by the 16 threads of a row) ----
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
+    for (int i = 0; i < RI; i++) {
       float rmax = -INFINITY;
 #pragma unroll
       for (int j = 0; j < 4; j++) {
-        const int t = tk0 + tx * 4 + j;
-        s[i][j] = (t <= qpos[i]) ? s[i][j] / sqrt_hs : -INFINITY;
+        const int t = tk0 + tx + 16 * j;
+        s[i][j] = (t <= qpos[i]) ? s[i][j] * inv_sqrt_hs : -INFINITY;
         rmax = fmaxf(rmax, s[i][j]);
       }
 #pragma unroll
       for (int off = 8; off > 0; off >>= 1) rmax = fmaxf(rmax, __shfl_xor_sync(THA_FULL_MASK, rmax, off));
       const float mn = fmaxf(m[i], rmax);          // finite: key 0 is visible to every row in the first tile
       const float corr = expf(m[i] - mn);          // exp(-inf) = 0 on the first tile
-      float4 pv;
-      pv.x = expf(s[i][0] - mn); pv.y = expf(s[i][1] - mn); pv.z = expf(s[i][2] - mn); pv.w = expf(s[i][3] - mn);
-      l[i] = l[i] * corr + ((pv.x + pv.y) + (pv.z + pv.w));   // per-thread partial of the row sum; reduced at the end
+      float sum = 0.0f;
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const float pv = expf(s[i][j] - mn);
+        sum += pv;
+        Ps[(ty + 16 * i) * PF_PS + tx + 16 * j] = pv;
+      }
+      l[i] = l[i] * corr + sum;   // per-thread partial of the row sum; reduced at the end
 #pragma unroll
       for (int c = 0; c < CW; c++) o[i][c] *= corr;
       m[i] = mn;
-      *reinterpret_cast<float4*>(Ps + (ty * 4 + i) * PF_TK + tx * 4) = pv;
     }
-    __syncthreads();
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();   // V and P are in place, every score is computed: K's buffer is free
+    if (tk0 + PF_TK <= kmax) load_rows(Ks, KS, kbase, tk0 + PF_TK);
 
-    // ---- O += P V : rows ty*4.., columns tx*VW + 64*v ----
-#pragma unroll 2
+    // ---- O += P V : rows ty + 16 i, columns tx*VW + 64*v ----
+#pragma unroll 1
     for (int t = 0; t < PF_TK; t += 4) {
-      float pr[4][4];
+      float4 pr[RI];
 #pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const float4 a = *reinterpret_cast<const float4*>(Ps + (ty * 4 + i) * PF_TK + t);
-        pr[i][0] = a.x; pr[i][1] = a.y; pr[i][2] = a.z; pr[i][3] = a.w;
-      }
+      for (int i = 0; i < RI; i++) pr[i] = *reinterpret_cast<const float4*>(Ps + (ty + 16 * i) * PF_PS + t);
 #pragma unroll
       for (int tt = 0; tt < 4; tt++) {
         float vv[CW];
@@ -159,31 +166,42 @@ __global__ void __launch_bounds__(256) attn_prefill_kernel(const AttnPrefillP p)
           for (int c = 0; c < CW; c++) vv[c] = vr[tx * CW + c];
         }
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+        for (int i = 0; i < RI; i++) {
+          const float w = tt == 0 ? pr[i].x : (tt == 1 ? pr[i].y : (tt == 2 ? pr[i].z : pr[i].w));
 #pragma unroll
-          for (int c = 0; c < CW; c++) o[i][c] = fmaf(pr[i][tt], vv[c], o[i][c]);
+          for (int c = 0; c < CW; c++) o[i][c] = fmaf(w, vv[c], o[i][c]);
+        }
       }
     }
   }
 
   // ---- normalise and store (fp32 row and its tf32 hi/lo split for the wo matmul) ----
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
+  for (int i = 0; i < RI; i++) {
     float L = l[i];
 #pragma unroll
     for (int off = 8; off > 0; off >>= 1) L += __shfl_xor_sync(THA_FULL_MASK, L, off);
-    const int r = ty * 4 + i;
+    const int r = ty + 16 * i;
     if (r >= n) continue;
     const size_t base = (size_t)(row0 + r) * p.dim + h * HS;
 #pragma unroll
-    for (int c = 0; c < CW; c++) {
-      const int col = (VW == 4) ? (tx * 4 + 64 * (c >> 2) + (c & 3)) : (tx * CW + c);
-      const float v = o[i][c] / L;
-      p.out[base + col] = v;
-      if (p.out_hi) {
-        const float hi = pf_tf32(v);
-        p.out_hi[base + col] = hi;
-        p.out_lo[base + col] = v - hi;
+    for (int v = 0; v < CW / VW; v++) {
+      const int col = (VW == 4) ? tx * 4 + 64 * v : tx * CW;
+      float hi[VW], val[VW];
+#pragma unroll
+      for (int e = 0; e < VW; e++) { val[e] = o[i][v * VW + e] / L; hi[e] = pf_tf32(val[e]); }
+      if constexpr (VW == 4) {
+        *reinterpret_cast<float4*>(p.out + base + col) = make_float4(val[0], val[1], val[2], val[3]);
+        if (p.out_hi) {
+          *reinterpret_cast<float4*>(p.out_hi + base + col) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+          *reinterpret_cast<float4*>(p.out_lo + base + col) = make_float4(val[0] - hi[0], val[1] - hi[1], val[2] - hi[2], val[3] - hi[3]);
+        }
+      } else {
+#pragma unroll
+        for (int e = 0; e < VW; e++) {
+          p.out[base + col + e] = val[e];
+          if (p.out_hi) { p.out_hi[base + col + e] = hi[e]; p.out_lo[base + col + e] = val[e] - hi[e]; }
+        }
       }
     }
   }
@@ -192,28 +210,32 @@ __global__ void __launch_bounds__(256) attn_prefill_kernel(const AttnPrefillP p)
 bool attn_prefill_supported(int head_size, int kv_dim) {
   return (head_size == 16 || head_size == 32 || head_size == 64 || head_size == 128) && kv_dim % 4 == 0;
 }
+// Query rows per tile: 128 where the prompts fill them (two LDS.128 per 16 FMAs, against three for 64 rows), 64 for short ones.
+int attn_prefill_tile_rows(int rows, int n_seqs) { return rows >= 192 * n_seqs ? 128 : 64; }
 
+// tile_row0 / tile_n: tiles of at most tile_rows (64 or 128) query rows, never across sequences, longest contexts first
 int attn_prefill_launch(cudaStream_t stream, int n_tiles, int n_heads, int n_kv_heads, int head_size, const float* q,
                         float* out, float* out_hi, float* out_lo, const float* kc, const float* vc,
                         long long kv_batch_stride, const int* row_slot, const int* row_pos, const int* tile_row0,
-                        const int* tile_n, bool pdl, const KvPaged* pg) {
-  if (!attn_prefill_supported(head_size, n_kv_heads * head_size)) return THA_STATUS_NOT_SUPPORTED;
+                        const int* tile_n, bool pdl, const KvPaged* pg, int tile_rows) {
+  if (!attn_prefill_supported(head_size, n_kv_heads * head_size) || (tile_rows != 64 && tile_rows != 128)) return THA_STATUS_NOT_SUPPORTED;
   AttnPrefillP p;
   p.q = q; p.out = out; p.out_hi = out_hi; p.out_lo = out_lo; p.kc = kc; p.vc = vc;
   if (pg) p.pg = *pg; else p.pg = KvPaged{};
   p.kv_batch_stride = kv_batch_stride; p.kv_dim = n_kv_heads * head_size; p.kv_mul = n_heads / n_kv_heads;
   p.dim = n_heads * head_size;
   p.row_slot = row_slot; p.row_pos = row_pos; p.tile_row0 = tile_row0; p.tile_n = tile_n;
-  const size_t smem = ((size_t)3 * head_size * 64 + 64 * 64) * sizeof(float);
   void (*k)(const AttnPrefillP) = nullptr;
+  size_t smem = 0;
+  const bool big = tile_rows == 128;
   switch (head_size) {
-    case 16: k = attn_prefill_kernel<16>; break;
-    case 32: k = attn_prefill_kernel<32>; break;
-    case 64: k = attn_prefill_kernel<64>; break;
-    default: k = attn_prefill_kernel<128>; break;
+    case 16: k = big ? attn_prefill_kernel<16, 8> : attn_prefill_kernel<16, 4>; smem = big ? pf_smem<16, 8>() : pf_smem<16, 4>(); break;
+    case 32: k = big ? attn_prefill_kernel<32, 8> : attn_prefill_kernel<32, 4>; smem = big ? pf_smem<32, 8>() : pf_smem<32, 4>(); break;
+    case 64: k = big ? attn_prefill_kernel<64, 8> : attn_prefill_kernel<64, 4>; smem = big ? pf_smem<64, 8>() : pf_smem<64, 4>(); break;
+    default: k = big ? attn_prefill_kernel<128, 8> : attn_prefill_kernel<128, 4>; smem = big ? pf_smem<128, 8>() : pf_smem<128, 4>(); break;
   }
   if (smem > 40 * 1024) THA_CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  THA_CUDA_OK(launch(k, dim3(n_tiles, n_heads), dim3(256), smem, stream, pdl, p));
+  THA_CUDA_OK(launch(k, dim3((unsigned)n_tiles * n_heads), dim3(256), smem, stream, pdl, p));
   return THA_STATUS_SUCCESS;
 }
 

@@ -34,7 +34,7 @@ bool attn_prefill_supported(int head_size, int kv_dim);
 int attn_prefill_launch(cudaStream_t stream, int n_tiles, int n_heads, int n_kv_heads, int head_size, const float* q,
                         float* out, float* out_hi, float* out_lo, const float* kc, const float* vc,
                         long long kv_batch_stride, const int* row_slot, const int* row_pos, const int* tile_row0,
-                        const int* tile_n, bool pdl, const KvPaged* pg = nullptr);
+                        const int* tile_n, bool pdl, const KvPaged* pg, int tile_rows);
 bool attn_fused_rope_supported(int n_heads, int n_kv_heads, int head_size);
 int attn_fused_rope_launch(cudaStream_t stream, Workspace* ws, int B, const int* pos_d, int n_heads, int n_kv_heads, float* q_out,
                            float* out, float* kc, float* vc, long long kv_batch_stride, int head_size, int seq_len, bool pdl,
@@ -400,7 +400,7 @@ static int bf_issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, 
       rounded = true;
     } else if (io.n_tiles > 0)
       THA_TRY_RC(attn_prefill_launch(st, io.n_tiles, c.n_heads, c.n_kv_heads, hs, io.q, io.xb, nullptr, nullptr, kcl,
-                                     vcl, kv_bs, io.slot, io.pos, io.tile_row0, io.tile_n, pdl, &pg));
+                                     vcl, kv_bs, io.slot, io.pos, io.tile_row0, io.tile_n, pdl, &pg, 64));
     else if (rope_in_attn) {
       THA_TRY_RC(attn_fused_rope_launch(st, ws, R, io.pos, c.n_heads, c.n_kv_heads, io.q, io.xb, const_cast<float*>(kcl),
                                         const_cast<float*>(vcl), kv_bs, hs, c.seq_len, pdl, nullptr, nullptr, nullptr, nullptr, 0, 0, &pg,

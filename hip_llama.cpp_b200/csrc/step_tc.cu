@@ -20,6 +20,7 @@
 //
 // Split-K partials are summed by their consumer in a fixed order, so the step is bit-reproducible
 // run to run (no floating-point atomics anywhere).
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <vector>
@@ -51,7 +52,8 @@ int attn_fused_rope_launch(cudaStream_t stream, Workspace* ws, int B, const int*
 int attn_prefill_launch(cudaStream_t stream, int n_tiles, int n_heads, int n_kv_heads, int head_size, const float* q,
                         float* out, float* out_hi, float* out_lo, const float* kc, const float* vc,
                         long long kv_batch_stride, const int* row_slot, const int* row_pos, const int* tile_row0,
-                        const int* tile_n, bool pdl, const KvPaged* pg = nullptr);
+                        const int* tile_n, bool pdl, const KvPaged* pg, int tile_rows);
+int attn_prefill_tile_rows(int rows, int n_seqs);
 
 __device__ __forceinline__ float st_tf32(float v) { return __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xFFFFE000u); }
 
@@ -617,6 +619,7 @@ struct RowsIO {
   float *x, *q, *xb;                       // [R, d] residual stream / rotated queries / attention output
   const int *token, *pos, *slot;           // [R]; slot == nullptr: row r lives in cache slab r (decode)
   int n_tiles; const int *tile_row0, *tile_n;   // prefill attention tiles (n_tiles == 0: per-row decode attention)
+  int tile_rows;                           // query rows per tile at most (64 or 128)
   int n_out; const int* out_rows;          // classifier rows (out_rows == nullptr: every row)
   float* logits; int* next;                // [n_out, vocab] (nullable: skip the classifier), [n_out] (nullable)
 };
@@ -863,7 +866,7 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
     } else if (io.n_tiles > 0) {
       THA_TRY_RC(attn_prefill_launch(st, io.n_tiles, c.n_heads, c.n_kv_heads, hs, io.q, io.xb, wq ? nullptr : sc.xh,
                                      wq ? nullptr : sc.xl, kcl, vcl, kv_bs, io.slot, io.pos,
-                                     io.tile_row0, io.tile_n, pdl, &pg));
+                                     io.tile_row0, io.tile_n, pdl, &pg, io.tile_rows));
     } else if (rope_in_attn) {
       THA_TRY_RC(attn_fused_rope_launch(st, ws, R, io.pos, c.n_heads, c.n_kv_heads, io.q, io.xb, const_cast<float*>(kcl),
                                         const_cast<float*>(vcl), kv_bs, hs, c.seq_len, pdl, wq ? nullptr : sc.xh, wq ? nullptr : sc.xl,
@@ -962,15 +965,21 @@ int step_tc_prefill(cudaStream_t st, Workspace* ws, const tha_config_t& c, const
   for (int i = 0; i < n_seqs; i++) {
     if (len[i] < 1 || pos0[i] < 0 || slot[i] < 0 || (long long)pos0[i] + len[i] > c.seq_len) return THA_STATUS_INVALID_ARG;
     R += len[i];
-    T += ceil_div(len[i], 64);
   }
   if (R < 1 || R > (1 << 20)) return THA_STATUS_INVALID_ARG;
+  const int TQ = attn_prefill_tile_rows((int)R, n_seqs);
+  struct Tile { int row0, n, last; };   // `last`: last position the tile's rows see
+  std::vector<Tile> tiles;
+  for (int i = 0, r0 = 0; i < n_seqs; r0 += len[i], i++)
+    for (int j = 0; j < len[i]; j += TQ) { const int n = (len[i] - j < TQ) ? len[i] - j : TQ; tiles.push_back({r0 + j, n, pos0[i] + j + n - 1}); }
+  std::stable_sort(tiles.begin(), tiles.end(), [](const Tile& x, const Tile& y) { return x.last > y.last; });   // the longest start first
+  T = (long long)tiles.size();
   // tables: [slot R | pos R | token R | tile_row0 T | tile_n T | last n_seqs]
   std::vector<int> tab((size_t)3 * R + 2 * T + n_seqs);
   int *h_slot = tab.data(), *h_pos = h_slot + R, *h_tok = h_pos + R, *h_t0 = h_tok + R, *h_tn = h_t0 + T, *h_last = h_tn + T;
-  int r = 0, t = 0;
+  for (long long t = 0; t < T; t++) { h_t0[t] = tiles[t].row0; h_tn[t] = tiles[t].n; }
+  int r = 0;
   for (int i = 0; i < n_seqs; i++) {
-    for (int j = 0; j < len[i]; j += 64) { h_t0[t] = r + j; h_tn[t] = (len[i] - j < 64) ? len[i] - j : 64; t++; }
     for (int j = 0; j < len[i]; j++, r++) {
       h_slot[r] = slot[i]; h_pos[r] = pos0[i] + j; h_tok[r] = tokens[r];
       if (tokens[r] < 0 || tokens[r] >= c.vocab_size) return THA_STATUS_INVALID_ARG;
@@ -988,7 +997,7 @@ int step_tc_prefill(cudaStream_t st, Workspace* ws, const tha_config_t& c, const
   RowsIO io = {};
   io.R = (int)R; io.x = sc.xr; io.q = sc.qr; io.xb = sc.xbr;
   io.slot = sc.tab; io.pos = sc.tab + R; io.token = sc.tab + 2 * R;
-  io.n_tiles = (int)T; io.tile_row0 = sc.tab + 3 * R; io.tile_n = sc.tab + 3 * R + T;
+  io.n_tiles = (int)T; io.tile_rows = TQ; io.tile_row0 = sc.tab + 3 * R; io.tile_n = sc.tab + 3 * R + T;
   io.n_out = n_seqs; io.out_rows = sc.tab + 3 * R + 2 * T; io.logits = logits; io.next = logits ? next_d : nullptr;
   return issue_rows(st, ws, c, w, wq, s, io, rc, rs, pdl_enabled() != 0, tp);
 }

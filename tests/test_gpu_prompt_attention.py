@@ -1,0 +1,48 @@
+"""fp32 prompt attention (csrc/attn_prefill.cu) inside tha_prefill_f32: prompts at the edges of query and key tiles, both tile heights,
+every head size, grouped queries, portions behind a context, against a float64 statement."""
+import numpy as np
+import pytest
+import torch
+
+import llama64
+from pkgload import load_pkg
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return float((a.double() - b).norm() / b.norm())
+
+
+@pytest.mark.parametrize("heads,kv_heads,hs", [(8, 8, 16), (4, 2, 32), (2, 2, 64), (4, 1, 128), (2, 2, 128)])
+@pytest.mark.parametrize("lens,start", [([1], 0), ([64, 63, 65], 0), ([127, 1, 129], 70), ([192], 0), ([193, 383], 0), ([500], 131), ([2, 640, 66], 1)])
+def test_prompts(heads, kv_heads, hs, lens, start):
+    eng, ck = load_pkg("engine"), load_pkg("checkpoint")
+    cfg = ck.Config(heads * hs, 96, 2, heads, kv_heads, 80, start + max(lens) + 3)
+    if not load_pkg("cabi").lib().c.tha_prefill_supported(eng.c_config(cfg)):
+        pytest.skip("the decode attention does not take this head layout")
+    # queries and keys of order one: a score s of magnitude S carries the products' error (1e-6) times S into its weight, and 0.15 here (S up to 60
+    # at 512 channels) gave 4e-5
+    w = eng.device_random_weights(cfg, seed=3, std=cfg.dim ** -0.5)
+    e = eng.Engine(w, len(lens), with_att=False)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    e.state.key_cache.normal_(generator=g)
+    e.state.value_cache.normal_(generator=g)
+    rng = np.random.default_rng(7)
+    seqs = [(i, start, rng.integers(0, cfg.vocab_size, n).astype(np.int32)) for i, n in enumerate(lens)]
+    before = {"k": e.state.key_cache.clone(), "v": e.state.value_cache.clone()}
+    logits = torch.empty(len(lens), cfg.vocab_size, device="cuda")
+    torch.cuda.synchronize()
+    e.prefill(seqs, logits)
+    torch.cuda.synchronize()
+    want, k, v = llama64.forward(cfg, w.t, lambda c, s, l, n: before[c][s, l, :n], seqs)
+    # fp32 sums of up to 640 terms through two layers: a few 1e-6; 3xTF32 products the same
+    assert rel(logits, want) < 3e-5
+    at = 0
+    for i, n in enumerate(lens):
+        for which, got, exact in (("k", e.state.key_cache, k), ("v", e.state.value_cache, v)):
+            assert rel(got[i, :, start:start + n], exact[at:at + n].transpose(0, 1)) < 3e-5
+            other = torch.ones(cfg.seq_len, dtype=torch.bool)
+            other[start:start + n] = False
+            assert torch.equal(got[i][:, other], before[which][i][:, other])    # nothing else was written
+        at += n
