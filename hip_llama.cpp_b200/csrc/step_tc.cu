@@ -170,9 +170,62 @@ __global__ void __launch_bounds__(1024) tc_prep_kernel(float* __restrict__ x, co
   }
 }
 
+// The same for prompt rows (no tensor parallelism): a block of 64 to 256 threads a row, a thread four float4 whose loads are in flight
+// together; several rows per SM.  1024 rows of 4096: 28.5 us with a 1024-thread
+// block a row, 21.3 with this; 1936 rows of 768: 12.5 us (192 threads), 9.5.
+__global__ void __launch_bounds__(256) tc_prep_prompt_kernel(float* __restrict__ x, const float* __restrict__ part, int nz, long long zstride,
+                                                             const float* __restrict__ emb, const int* __restrict__ token, const int* __restrict__ pos,
+                                                             const float* __restrict__ gain, int d, float* __restrict__ xh, float* __restrict__ xl,
+                                                             float* __restrict__ scale) {
+  __shared__ float red[33];
+  pdl_trigger();
+  pdl_wait();
+  const int b = blockIdx.x, d4 = d >> 2;
+  float4* xr = reinterpret_cast<float4*>(x + (size_t)b * d);
+  float4* hr = reinterpret_cast<float4*>(xh + (size_t)b * d);
+  float4* lr = reinterpret_cast<float4*>(xl + (size_t)b * d);
+  const bool live = pos[b] >= 0;
+  const float4* src = emb ? reinterpret_cast<const float4*>(emb + (size_t)token[b] * d) : xr;
+  float ss = 0.0f;
+  for (int i0 = threadIdx.x; i0 < d4; i0 += 4 * blockDim.x) {
+    float4 v[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const int i = i0 + k * (int)blockDim.x;
+      v[k] = i < d4 && live ? src[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    for (int z = 0; z < nz && live; z++) {   // fixed order
+      float4 pz[4];
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const int i = i0 + k * (int)blockDim.x;
+        pz[k] = i < d4 ? ldg_stream(reinterpret_cast<const float4*>(part + (size_t)z * zstride + (size_t)b * d) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; k++) { v[k].x += pz[k].x; v[k].y += pz[k].y; v[k].z += pz[k].z; v[k].w += pz[k].w; }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const int i = i0 + k * (int)blockDim.x;
+      if (i >= d4) break;
+      if (live && (emb || nz)) xr[i] = v[k];
+      ss = dot4(v[k], v[k], ss);
+      const float4 g = reinterpret_cast<const float4*>(gain)[i];
+      v[k].x *= g.x; v[k].y *= g.y; v[k].z *= g.z; v[k].w *= g.w;
+      const float4 h = make_float4(st_tf32(v[k].x), st_tf32(v[k].y), st_tf32(v[k].z), st_tf32(v[k].w));
+      hr[i] = h;
+      lr[i] = make_float4(v[k].x - h.x, v[k].y - h.y, v[k].z - h.z, v[k].w - h.w);
+    }
+  }
+  const float tot = block_sum(ss, red);
+  if (threadIdx.x == 0) scale[b] = live ? 1.0f / sqrtf(tot / d + 1e-5f) : 0.0f;
+}
+
 // q|k|v rows of every slot (sum of nz partials): RoPE on q and k pairs (run.cc:271-286 with the host-built
-// cos/sin tables), q -> state, k/v -> the cache row of pos[b].  A thread takes TWO pairs a block-width apart (two
-// independent chains of loads).  grid (pairs / 512, B).
+// cos/sin tables), q -> state, k/v -> the cache row of pos[b].  A thread takes two pairs per 128-bit load, two loads a block-width apart
+// (the fused attention of these steps takes only head sizes that are powers of two from 4 on, and reads the same rows by 128 bits).
+// Bound by memory: 2825 rows of 12288 (277 MB moved) took 84 us with two 64-bit loads, 64 with these.
+// grid (ld / 2048, rows)
 __global__ void __launch_bounds__(256) tc_rope_scatter_kernel(const float* __restrict__ part, int nz, long long zstride,
                                                               int ld, const int* __restrict__ pos, int d, int kvd, int hs,
                                                               const float* __restrict__ rc, const float* __restrict__ rs,
@@ -188,18 +241,17 @@ __global__ void __launch_bounds__(256) tc_rope_scatter_kernel(const float* __res
   const int sb = slot ? slot[b] : b;   // cache slab of this row
   // where the row of position pb lives: the slot's dense slab, or a block of the pool (BatchManager)
   const long long rowoff = pg.table ? kv_paged_off(pg, sb, pb, kvd) : (long long)sb * kv_bs + loff + (long long)pb * kvd;
-  float2 v[2];
+  float4 v[2];
   int idx[2];
 #pragma unroll
   for (int u = 0; u < 2; u++) {
-    const int pair = (blockIdx.x * 2 + u) * blockDim.x + threadIdx.x;
-    idx[u] = pair * 2;
-    v[u] = make_float2(0.f, 0.f);
+    idx[u] = 4 * ((blockIdx.x * 2 + u) * blockDim.x + threadIdx.x);
+    v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (idx[u] < d + 2 * kvd) {
 #pragma unroll 4
       for (int z = 0; z < nz; z++) {
-        const float2 pz = *reinterpret_cast<const float2*>(part + (size_t)z * zstride + (size_t)b * ld + idx[u]);
-        v[u].x += pz.x; v[u].y += pz.y;
+        const float4 pz = *reinterpret_cast<const float4*>(part + (size_t)z * zstride + (size_t)b * ld + idx[u]);
+        v[u].x += pz.x; v[u].y += pz.y; v[u].z += pz.z; v[u].w += pz.w;
       }
     }
   }
@@ -210,14 +262,15 @@ __global__ void __launch_bounds__(256) tc_rope_scatter_kernel(const float* __res
     if (i < d + kvd) {
       const int li = (i < d) ? i : i - d;
       const int j = (li % hs) >> 1;
-      const float c = rc[(size_t)pb * (hs >> 1) + j], s = rs[(size_t)pb * (hs >> 1) + j];
+      const float2 c = *reinterpret_cast<const float2*>(rc + (size_t)pb * (hs >> 1) + j), s = *reinterpret_cast<const float2*>(rs + (size_t)pb * (hs >> 1) + j);
       // one product rounded, the other fused: the SAME expression as the attention kernel's in-kernel RoPE (attention.cu), so the
       // two forms of the step leave identical bits in the cache
-      const float r0 = fmaf(v[u].x, c, -__fmul_rn(v[u].y, s)), r1 = fmaf(v[u].x, s, __fmul_rn(v[u].y, c));
-      if (i < d) *reinterpret_cast<float2*>(q + (size_t)b * d + li) = make_float2(r0, r1);
-      else *reinterpret_cast<float2*>(kc + rowoff + li) = make_float2(r0, r1);
+      const float4 r = make_float4(fmaf(v[u].x, c.x, -__fmul_rn(v[u].y, s.x)), fmaf(v[u].x, s.x, __fmul_rn(v[u].y, c.x)),
+                                   fmaf(v[u].z, c.y, -__fmul_rn(v[u].w, s.y)), fmaf(v[u].z, s.y, __fmul_rn(v[u].w, c.y)));
+      if (i < d) *reinterpret_cast<float4*>(q + (size_t)b * d + li) = r;
+      else *reinterpret_cast<float4*>(kc + rowoff + li) = r;
     } else {
-      *reinterpret_cast<float2*>(vc + rowoff + (i - d - kvd)) = v[u];
+      *reinterpret_cast<float4*>(vc + rowoff + (i - d - kvd)) = v[u];
     }
   }
   kt_stamp(kt, 6);
@@ -226,7 +279,7 @@ __global__ void __launch_bounds__(256) tc_rope_scatter_kernel(const float* __res
 int rope_scatter_launch(cudaStream_t st, bool pdl, int R, const float* part, int nz, long long zstride, int ld, const int* pos, int d,
                         int kvd, int hs, const float* rc, const float* rs, float* q, float* kc, float* vc, long long kv_bs, int loff,
                         const int* slot, const KvPaged* pg) {
-  THA_CUDA_OK(launch(tc_rope_scatter_kernel, dim3(ceil_div(ld / 2, 512), R), dim3(256), 0, st, pdl, part, nz, zstride, ld, pos, d, kvd, hs,
+  THA_CUDA_OK(launch(tc_rope_scatter_kernel, dim3(ceil_div(ld / 4, 512), R), dim3(256), 0, st, pdl, part, nz, zstride, ld, pos, d, kvd, hs,
                      rc, rs, q, kc, vc, kv_bs, loff, slot, pg ? *pg : KvPaged{}));
   return THA_STATUS_SUCCESS;
 }
@@ -263,6 +316,43 @@ __global__ void __launch_bounds__(256) tc_swiglu_split_kernel(const float* __res
   kt_stamp(kt, 6);
 }
 
+// The same for prompt rows (thousands of blocks whatever a thread takes): two float4 a block-width apart, four 128-bit loads in flight; 1024 rows
+// of 11008 (180 MB moved) took 76 us with two values per thread, 64 with this.  grid (h / 2048, rows)
+__global__ void __launch_bounds__(256) tc_swiglu_split_wide_kernel(const float* __restrict__ part, int nz, long long zstride, int ld,
+                                                                   const int* __restrict__ pos, int h, float* __restrict__ hh, float* __restrict__ hl) {
+  pdl_trigger();
+  pdl_wait();
+  const int b = blockIdx.y;
+  const bool live = pos[b] >= 0;
+  float4 a[2], c[2];
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    const int i = 4 * ((blockIdx.x * 2 + u) * blockDim.x + threadIdx.x);
+    a[u] = c[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < h && live) {
+      for (int z = 0; z < nz; z++) {
+        const float4 az = ldg_stream(reinterpret_cast<const float4*>(part + (size_t)z * zstride + (size_t)b * ld + i));
+        const float4 cz = ldg_stream(reinterpret_cast<const float4*>(part + (size_t)z * zstride + (size_t)b * ld + h + i));
+        a[u].x += az.x; a[u].y += az.y; a[u].z += az.z; a[u].w += az.w;
+        c[u].x += cz.x; c[u].y += cz.y; c[u].z += cz.z; c[u].w += cz.w;
+      }
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    const int i = 4 * ((blockIdx.x * 2 + u) * blockDim.x + threadIdx.x);
+    if (i >= h) continue;
+    float4 r = a[u];
+    r.x *= (1.0f / (1.0f + expf(-r.x))); r.x *= c[u].x;   // run.cc:344-347 operation order
+    r.y *= (1.0f / (1.0f + expf(-r.y))); r.y *= c[u].y;
+    r.z *= (1.0f / (1.0f + expf(-r.z))); r.z *= c[u].z;
+    r.w *= (1.0f / (1.0f + expf(-r.w))); r.w *= c[u].w;
+    const float4 hi = make_float4(st_tf32(r.x), st_tf32(r.y), st_tf32(r.z), st_tf32(r.w));
+    *reinterpret_cast<float4*>(hh + (size_t)b * h + i) = hi;
+    *reinterpret_cast<float4*>(hl + (size_t)b * h + i) = make_float4(r.x - hi.x, r.y - hi.y, r.z - hi.z, r.w - hi.w);
+  }
+}
+
 
 // ---- Q8_0 rows (runq.c:344-481 on the tensor cores) ---------------------------------------------------------------
 // The activation that enters a matmul is quantised exactly as runq.c:145-171 does (scale = max|x| / 127 per group,
@@ -273,6 +363,7 @@ __global__ void __launch_bounds__(256) tc_swiglu_split_kernel(const float* __res
 // One block per output row (up to 1024 threads, one or more float4 per thread, all loads of a thread independent):
 // x row = embedding row or x + sum of partials (written back), RMSNorm in the reference's order w * (ss * x)
 // (run.cc:196-209), group quantisation.  gs in {32, 64, 128}; d % gs == 0.
+constexpr int PROMPT_ROWS = 512;   // rows from which a launch fills the machine whatever a thread takes
 constexpr int PREP_MAX_V = 4;   // float4 per thread kept in registers: d <= 4 * 1024 * 4
 __global__ void __launch_bounds__(1024) tc_prep_q8_kernel(float* __restrict__ x, const float* __restrict__ part, int nz,
                                                           long long zstride, const float* __restrict__ emb,
@@ -339,8 +430,8 @@ __global__ void __launch_bounds__(1024) tc_prep_q8_kernel(float* __restrict__ x,
   kt_stamp(kt, 6);
 }
 
-// One float4 per thread: src row (attention output), or with h > 0 the SwiGLU of the w1|w3 partials (run.cc:344-347
-// order), quantised per group (int8 row + transposed scales).  grid (ceil(K / 4 / 256), rows)
+// Two float4 per thread: src row (attention output), or with h > 0 the SwiGLU of the w1|w3 partials (run.cc:344-347
+// order), quantised per group (int8 row + transposed scales).  grid (ceil(K / 4 / 512), rows)
 __global__ void __launch_bounds__(256) tc_quant_split_kernel(const float* __restrict__ src, long long ld, int nz,
                                                              long long zstride, int h, const int* __restrict__ pos, int K,
                                                              int gs, int8_t* __restrict__ oq, float* __restrict__ osT, int ldxs) {
@@ -349,28 +440,36 @@ __global__ void __launch_bounds__(256) tc_quant_split_kernel(const float* __rest
   pdl_wait();
   kt_stamp(kt, 1);
   const int b = blockIdx.y;
-  const int i4 = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool in = 4 * i4 < K;   // K % gs == 0: a group is never cut, but a warp may be
-  float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (in && pos[b] >= 0) {
-    if (h > 0) {
-      float4 a = make_float4(0.f, 0.f, 0.f, 0.f), c = a;
+  const bool live = pos[b] >= 0;
+  float4 r[2];
+#pragma unroll
+  for (int u = 0; u < 2; u++) {   // two float4 a block-width apart: their loads are in flight together
+    const int i4 = (blockIdx.x * 2 + u) * blockDim.x + threadIdx.x;
+    r[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (4 * i4 < K && live) {
+      if (h > 0) {
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), c = a;
 #pragma unroll 8
-      for (int z = 0; z < nz; z++) {
-        const float4 pa = *reinterpret_cast<const float4*>(src + (size_t)z * zstride + (size_t)b * ld + 4 * i4);
-        const float4 pc = *reinterpret_cast<const float4*>(src + (size_t)z * zstride + (size_t)b * ld + h + 4 * i4);
-        a.x += pa.x; a.y += pa.y; a.z += pa.z; a.w += pa.w;
-        c.x += pc.x; c.y += pc.y; c.z += pc.z; c.w += pc.w;
+        for (int z = 0; z < nz; z++) {
+          const float4 pa = *reinterpret_cast<const float4*>(src + (size_t)z * zstride + (size_t)b * ld + 4 * i4);
+          const float4 pc = *reinterpret_cast<const float4*>(src + (size_t)z * zstride + (size_t)b * ld + h + 4 * i4);
+          a.x += pa.x; a.y += pa.y; a.z += pa.z; a.w += pa.w;
+          c.x += pc.x; c.y += pc.y; c.z += pc.z; c.w += pc.w;
+        }
+        r[u].x = a.x * (1.0f / (1.0f + expf(-a.x))); r[u].x *= c.x;
+        r[u].y = a.y * (1.0f / (1.0f + expf(-a.y))); r[u].y *= c.y;
+        r[u].z = a.z * (1.0f / (1.0f + expf(-a.z))); r[u].z *= c.z;
+        r[u].w = a.w * (1.0f / (1.0f + expf(-a.w))); r[u].w *= c.w;
+      } else {
+        r[u] = *reinterpret_cast<const float4*>(src + (size_t)b * ld + 4 * i4);
       }
-      r.x = a.x * (1.0f / (1.0f + expf(-a.x))); r.x *= c.x;
-      r.y = a.y * (1.0f / (1.0f + expf(-a.y))); r.y *= c.y;
-      r.z = a.z * (1.0f / (1.0f + expf(-a.z))); r.z *= c.z;
-      r.w = a.w * (1.0f / (1.0f + expf(-a.w))); r.w *= c.w;
-    } else {
-      r = *reinterpret_cast<const float4*>(src + (size_t)b * ld + 4 * i4);
     }
   }
-  q8_quant4(r, gs, i4, oq + (size_t)b * K, osT, ldxs, b, in);
+#pragma unroll
+  for (int u = 0; u < 2; u++) {
+    const int i4 = (blockIdx.x * 2 + u) * blockDim.x + threadIdx.x;   // K % gs == 0: a group is never cut, but a warp may be
+    q8_quant4(r[u], gs, i4, oq + (size_t)b * K, osT, ldxs, b, 4 * i4 < K);
+  }
   kt_stamp(kt, 6);
 }
 
@@ -774,6 +873,9 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
   int prep_threads = ceil_div(d / 4, 32) * 32;   // one float4 per thread where the row allows it
   if (prep_threads > 1024) prep_threads = 1024;
   if (prep_threads < 128) prep_threads = 128;
+  // prompt rows: up to four float4 per thread, so that several rows share an SM
+  const int prompt_threads = d <= 1024 ? 64 : (d <= 4096 ? ceil_div(d / 16, 32) * 32 : 256);
+  if (R >= PROMPT_ROWS && q8 && d / 4 <= 256 * PREP_MAX_V) prep_threads = prompt_threads;
   // tensor parallelism: split counts of every rank's w2 (local hidden sizes may differ), exchange bookkeeping
   int z_w2_of[TP_MAX] = {0};
   const bool tpx = tp && tp->tp > 1;
@@ -811,6 +913,8 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
     if (wq) {
       THA_CUDA_OK(launch(tc_prep_q8_kernel, dim3(rows), dim3(prep_threads), 0, st, pdl, io.x, part, nz, zs, emb, io.token,
                          io.pos, gain, d, gs, sc.xq, sc.xsT, ldxs, gather, tpp));
+    } else if (rows >= PROMPT_ROWS && !gather && !tpp.n) {
+      THA_CUDA_OK(launch(tc_prep_prompt_kernel, dim3(rows), dim3(prompt_threads), 0, st, pdl, io.x, part, nz, zs, emb, io.token, io.pos, gain, d, sc.xh, sc.xl, sc.scale));
     } else {
       THA_CUDA_OK(launch(tc_prep_kernel, dim3(rows), dim3(prep_threads), 0, st, pdl, io.x, part, nz, zs, emb, io.token,
                          io.pos, gain, d, sc.xh, sc.xl, sc.scale, gather, tpp));
@@ -855,7 +959,7 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
     const bool rope_in_attn = io.n_tiles == 0 && !(!io.logits && l == L - 1) && !(skip & 2) && rope_fuse_mode() &&
                               attn_fused_rope_supported(c.n_heads, c.n_kv_heads, hs);
     if (!(skip & 8) && !rope_in_attn)
-    THA_CUDA_OK(launch(tc_rope_scatter_kernel, dim3(ceil_div(ld_qkv / 2, 512), R), dim3(256), 0, st, pdl, (const float*)sc.part,
+    THA_CUDA_OK(launch(tc_rope_scatter_kernel, dim3(ceil_div(ld_qkv / 4, 512), R), dim3(256), 0, st, pdl, (const float*)sc.part,
                        pl.z_qkv, (long long)R * ld_qkv, ld_qkv, io.pos, da, kvd, hs, rc, rs, io.q, s.key_cache, s.value_cache,
                        kv_bs, loff, io.slot, pg));
     if (!io.logits && l == L - 1) {   // cache-only ingestion: the last layer's K/V rows are in place
@@ -880,7 +984,7 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
     }
     if ((skip & 16) || (wq && io.n_tiles == 0 && !(skip & 2))) {
     } else if (wq)   // prompt rows: runq.c:437 as its own launch
-      THA_CUDA_OK(launch(tc_quant_split_kernel, dim3(ceil_div(da / 4, 256), R), dim3(256), 0, st, pdl, (const float*)io.xb, (long long)da,
+      THA_CUDA_OK(launch(tc_quant_split_kernel, dim3(ceil_div(da / 4, 512), R), dim3(256), 0, st, pdl, (const float*)io.xb, (long long)da,
                          0, 0LL, 0, io.pos, da, gs, sc.xq, sc.xsT, ldxs));
     {
       const float* W[1] = {wq ? nullptr : w.wo + (size_t)l * d * da};
@@ -897,8 +1001,11 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
     }
     if (skip & 16) {
     } else if (wq)   // runq.c:457-465: SwiGLU, then quantise hb
-      THA_CUDA_OK(launch(tc_quant_split_kernel, dim3(ceil_div(hd / 4, 256), R), dim3(256), 0, st, pdl, (const float*)sc.part,
+      THA_CUDA_OK(launch(tc_quant_split_kernel, dim3(ceil_div(hd / 4, 512), R), dim3(256), 0, st, pdl, (const float*)sc.part,
                          (long long)ld_h, pl.z_w13, (long long)R * ld_h, hd, io.pos, hd, gs, sc.hq, sc.hsT, ldxs));
+    else if (R >= PROMPT_ROWS)
+      THA_CUDA_OK(launch(tc_swiglu_split_wide_kernel, dim3(ceil_div(hd, 2048), R), dim3(256), 0, st, pdl, (const float*)sc.part, pl.z_w13,
+                         (long long)R * ld_h, ld_h, io.pos, hd, sc.hh, sc.hl));
     else
       THA_CUDA_OK(launch(tc_swiglu_split_kernel, dim3(ceil_div(hd, 512), R), dim3(256), 0, st, pdl, (const float*)sc.part, pl.z_w13,
                          (long long)R * ld_h, ld_h, io.pos, hd, sc.hh, sc.hl));

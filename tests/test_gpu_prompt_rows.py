@@ -1,0 +1,56 @@
+"""The row kernels of a step (csrc/step_tc.cu) from 512 prompt rows on: widths around a block's share."""
+import numpy as np
+import pytest
+import torch
+
+import llama64
+from pkgload import load_pkg
+
+pytestmark = pytest.mark.gpu
+
+
+def rel(a, b):
+    return float((a.double() - b.double()).norm() / b.double().norm())
+
+
+def prefill(e, seqs, vocab):
+    out = torch.empty(len(seqs), vocab, device="cuda")
+    torch.cuda.synchronize()
+    e.prefill(seqs, out)
+    torch.cuda.synchronize()
+    return out
+
+
+@pytest.mark.parametrize("heads,hs,hidden", [(8, 16, 36), (16, 64, 2052), (18, 64, 100), (33, 128, 4196)])
+@pytest.mark.parametrize("lens", [[512], [400, 111, 2]])
+def test_fp32_rows(heads, hs, hidden, lens):
+    eng, ck = load_pkg("engine"), load_pkg("checkpoint")
+    cfg = ck.Config(heads * hs, hidden, 1, heads, heads, 96, 520)
+    w = eng.device_random_weights(cfg, seed=2, std=cfg.dim ** -0.5)
+    e = eng.Engine(w, len(lens), with_att=False)
+    rng = np.random.default_rng(3)
+    seqs = [(i, 0, rng.integers(0, 96, n).astype(np.int32)) for i, n in enumerate(lens)]
+    got = prefill(e, seqs, 96)
+    want, k, v = llama64.forward(cfg, w.t, lambda c, s, l, n: e.state.key_cache[s, l, :n], seqs)
+    # 3xTF32 sums of 32 to 4224 terms: 1e-6 to 1e-5 (accumulation in the tensor core), through three products one after the other
+    assert rel(got, want) < 5e-5
+    at = 0
+    for i, n in enumerate(lens):
+        assert rel(e.state.key_cache[i, :, :n], k[at:at + n].transpose(0, 1)) < 3e-5 and rel(e.state.value_cache[i, :, :n], v[at:at + n].transpose(0, 1)) < 3e-5
+        at += n
+
+
+@pytest.mark.parametrize("heads,hs,hidden", [(8, 32, 128), (18, 64, 2112), (33, 128, 4160)])
+def test_q8_rows(heads, hs, hidden):
+    """One call of 512 + 1 rows against calls of 171: the first layer's key rows (rmsnorm, quantiser, product, rotation) differ by the order
+    of partial sums at most, later values by quantiser steps that fall the other way."""
+    eng, ck = load_pkg("engine"), load_pkg("checkpoint")
+    cfg = ck.Config(heads * hs, hidden, 2, heads, heads, 96, 520)
+    w = eng.device_random_weights(cfg, q8=True, seed=4, gs=32)
+    toks = np.random.default_rng(5).integers(0, 96, 513).astype(np.int32)
+    a, b = eng.Engine(w, 1, with_att=False), eng.Engine(w, 1, with_att=False)
+    got = prefill(a, [(0, 0, toks)], 96)
+    for i in range(0, 513, 171):
+        want = prefill(b, [(0, i, toks[i:i + 171])], 96)
+    assert rel(a.state.key_cache[0, 0, :513], b.state.key_cache[0, 0, :513]) < 2e-6
+    assert rel(got, want) < 5e-2
