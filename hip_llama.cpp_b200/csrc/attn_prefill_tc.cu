@@ -260,7 +260,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap mk, const __grid_cons
     }
     __syncthreads();
     // ---- S = Q K^T
-    if (tid == 0) {
+    if (tid < 32 && tc_elect()) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       constexpr uint32_t idesc = ptc_idesc(PTC_TK);
 #pragma unroll
@@ -317,7 +317,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap mk, const __grid_cons
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
     // ---- P V
-    if (tid == 0) {
+    if (tid < 32 && tc_elect()) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       constexpr uint32_t idesc = ptc_idesc(HS);
 #pragma unroll

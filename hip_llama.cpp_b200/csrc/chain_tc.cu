@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) chain_tf32x3_kernel(const __gri
 
   if (warp == 0) {
     // ===== W producer: never waits for anything but ring space -- runs ahead through the phases
-    if (lane == 0) {
+    if (tc_elect()) {
       int gb = 0, n_it = 0;
       bool ok = true;
       for (int it = blockIdx.x; it < P.n_items && ok; it += gridDim.x, n_it++) {
@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) chain_tf32x3_kernel(const __gri
     }
   } else if (warp == 3) {
     // ===== X producer: the activations of a phase exist once the phase before has finished this column tile
-    if (lane == 0) {
+    if (tc_elect()) {
       pdl_wait();
       int gb = 0, n_it = 0;
       bool ok = true;
@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) chain_tf32x3_kernel(const __gri
     }
   } else if (warp == 1) {
     // ===== MMA issuer (as gemm_tf32x3_kernel)
-    if (lane == 0) {
+    if (tc_elect()) {
       constexpr uint32_t idesc = tc_idesc(NT), idesc2 = tc_idesc(2 * NT);
       int gb = 0, n_it = 0;
       bool ok = true;

@@ -131,7 +131,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant_
 
   if (warp == 0) {
     // ===== TMA producer
-    if (lane == 0) {
+    if (tc_elect()) {
       uint64_t pol_w;
       asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol_w));
       const bool stream_w = p.ny == 1;            // every weight tile is read once: do not let it displace the activations in L2
@@ -172,7 +172,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant_
     }
   } else if (warp == 1) {
     // ===== MMA issuer
-    if (lane == 0) {
+    if (tc_elect()) {
       constexpr uint32_t idesc = bf_idesc(NT);
       int gb = 0, n_it = 0;
       bool ok = true;
@@ -365,7 +365,7 @@ gemm_bf16_cluster_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_c
   const uint32_t tmem_d = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (tc_elect()) {
       const CUtensorMap* mw = (mat == 0 || p.stacked) ? &mw0 : (mat == 1 ? &mw1 : &mw2);
       const int wrow = p.w_row[mat] + row0, xrow = p.x_row[mat] + n0;
       uint64_t pol_w;
@@ -391,7 +391,7 @@ gemm_bf16_cluster_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_c
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (tc_elect()) {
       constexpr uint32_t idesc = bf_idesc(NT);
       bool ok = true;
       for (int i = 0; i < nkb; i++) {

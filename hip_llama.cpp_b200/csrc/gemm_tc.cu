@@ -122,7 +122,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constan
   if (warp == 0) {
     // ===== W producer: weights never depend on the previous kernel, so no programmatic-dependency wait here --
     // with PDL the whole ring is already in flight while the predecessor drains.
-    if (lane == 0) {
+    if (tc_elect()) {
       uint64_t pol_w;
       asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol_w));
       int gb = 0;                                 // running stage counter at the start of the item
@@ -144,7 +144,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constan
     }
   } else if (warp == 3) {
     // ===== X producer (activations: written by the previous kernel)
-    if (lane == 0) {
+    if (tc_elect()) {
       pdl_wait();
       kt_stamp(kt, 1);
       int gb = 0;
@@ -168,7 +168,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constan
     }
   } else if (warp == 1) {
     // ===== MMA issuer: A (weights, hi / lo) from TMEM, B (activations, hi / lo) from shared memory
-    if (lane == 0) {
+    if (tc_elect()) {
       constexpr uint32_t idesc = tc_idesc(NT), idesc2 = tc_idesc(2 * NT);
       int gb = 0, n_it = 0;
       bool ok = true;
@@ -189,7 +189,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constan
           const int nk = (w.nkb - i * S::KG) < S::KG ? (w.nkb - i * S::KG) : S::KG;
           // Per K = 8 step TWO MMAs instead of three: the X tile is stored [Xhi rows | Xlo rows], so one
           // descriptor over 2*NT rows gives D[:, 0:NT] += Whi.Xhi and D[:, NT:2NT] += Whi.Xlo in a single
-          // instruction (an MMA of this shape costs ~60 cycles for any N <= 128); Wlo.Xhi then adds into the
+          // instruction (an MMA of this shape costs ~45 cycles up to N = 64, 64 at 128); Wlo.Xhi then adds into the
           // second half.  Columns [NT, 2NT) hold the small correction terms, [0, NT) the main sum.
 #pragma unroll
           for (int kk = 0; kk < S::KG; kk++) {
