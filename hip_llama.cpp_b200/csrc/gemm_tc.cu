@@ -505,11 +505,12 @@ int gemm_tc_check_error() {
 // Every tcgen05 instruction costs its issuing thread a few hundred cycles whatever its size (measured: ~300 per
 // kind::i8 MMA, ~200 per tcgen05.ld, ~450 per wait::ld), so the epilogue reads 128 accumulator columns -- 128/NT
 // consecutive groups, laid out back to back in TMEM -- per round trip.
-// Epilogue warps: four (one per 32-lane TMEM quarter) for narrow column tiles; EIGHT for NT >= 32 -- two per quarter, each with
-// half of the tile's columns.  At NT = 64 a slot of 16 KB of weights leaves 64 KB of int32 group sums in TMEM (read at 64 B per
-// cycle: ~1000 cycles) and costs 640 scaling instructions per row; with one warp per quarter the two are strictly serial
-// (~1650 cycles per slot, 2.0 TB/s of weights); with two, one warp's TMEM read runs under the other's arithmetic.
-__host__ __device__ constexpr int q8i_epi_warps(int nt) { return nt >= 32 ? 8 : 4; }
+// Epilogue warps: four (one per 32-lane TMEM quarter) for narrow column tiles, eight at NT = 32, SIXTEEN at NT = 64 -- four per quarter,
+// each with a quarter of the tile's columns.  A slot of 16 KB of weights leaves 64 KB of int32 group sums in TMEM; a warp's TMEM reads and the
+// wait for them take several hundred cycles (four warps reading: 171 B a cycle, sixteen: 440), and only other warps of the same scheduler can
+// fill them.  930 rows x 12288 x 4096: 317 us with eight warps, 293 with sixteen and two scaling products to an instruction; 64 rows 38.0 -> 36.2.
+// (mma.sync with the sums in registers: 329 us, and 29.8 against 19.4 at one row.)
+__host__ __device__ constexpr int q8i_epi_warps(int nt) { return nt >= 64 ? 16 : (nt >= 32 ? 8 : 4); }
 __host__ __device__ constexpr int q8i_threads(int nt) { return 128 + 32 * q8i_epi_warps(nt); }
 
 struct Q8iP {
@@ -563,6 +564,16 @@ __device__ __forceinline__ void tc_tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
 __device__ __forceinline__ void tc_tmem_ld64(uint32_t taddr, uint32_t* v) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x64.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, %48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%64];"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31]), "=r"(v[32]), "=r"(v[33]), "=r"(v[34]), "=r"(v[35]), "=r"(v[36]), "=r"(v[37]), "=r"(v[38]), "=r"(v[39]), "=r"(v[40]), "=r"(v[41]), "=r"(v[42]), "=r"(v[43]), "=r"(v[44]), "=r"(v[45]), "=r"(v[46]), "=r"(v[47]), "=r"(v[48]), "=r"(v[49]), "=r"(v[50]), "=r"(v[51]), "=r"(v[52]), "=r"(v[53]), "=r"(v[54]), "=r"(v[55]), "=r"(v[56]), "=r"(v[57]), "=r"(v[58]), "=r"(v[59]), "=r"(v[60]), "=r"(v[61]), "=r"(v[62]), "=r"(v[63]) : "r"(taddr));
+}
+
+// (f0 * ws * x0, f1 * ws * x1), each product rounded by itself; two lanes to an instruction save issue slots (the sums stay scalar: a packed add
+// after a packed multiply is contracted)
+__device__ __forceinline__ void q8i_scale2(float f0, float f1, float ws, float x0, float x1, float& p0, float& p1) {
+  asm("{\n\t.reg .b64 f, w, x;\n\t"
+      "mov.b64 f, {%2, %3};\n\tmov.b64 w, {%4, %4};\n\tmov.b64 x, {%5, %6};\n\t"
+      "mul.rn.f32x2 f, f, w;\n\tmul.rn.f32x2 f, f, x;\n\t"
+      "mov.b64 {%0, %1}, f;\n\t}"
+      : "=f"(p0), "=f"(p1) : "f"(f0), "f"(f1), "f"(ws), "f"(x0), "f"(x1));
 }
 
 // Persistent: a CTA walks the work items (weight tile, column tile, K split) blockIdx.x, blockIdx.x + gridDim.x, ...
@@ -796,12 +807,23 @@ gemm_q8i_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant__
             for (int c = 0; c < CH; c += 4) {
               const float4 t = *reinterpret_cast<const float4*>(xs_sm + gi * NT + c0 + c);   // same address in every lane: a broadcast
               const float xs[4] = {t.x, t.y, t.z, t.w};
+              // runq.c:334 in its order, no contraction
+              if (EW == 4) {
 #pragma unroll
-              for (int e = 0; e < 4; e++) {
-                // |group sum| <= 128 * 127 * 127 < 2^22: 1.5 * 2^23 + i is exact in fp32, so this IS (float)i -- two
-                // full-rate instructions instead of a quarter-rate I2F
-                const float f = __int_as_float(0x4B400000 + (int)v[b * CH + c + e]) - 12582912.0f;
-                acc[c + e] = __fadd_rn(acc[c + e], __fmul_rn(__fmul_rn(f, ws), xs[e]));   // runq.c:334, no contraction
+                for (int e = 0; e < 4; e++) {
+                  // |group sum| <= 128 * 127 * 127 < 2^22: 1.5 * 2^23 + i is exact in fp32, so this IS (float)i -- two
+                  // full-rate instructions instead of a half-rate I2F: with one warp per scheduler latency counts, not issue slots
+                  const float f = __int_as_float(0x4B400000 + (int)v[b * CH + c + e]) - 12582912.0f;
+                  acc[c + e] = __fadd_rn(acc[c + e], __fmul_rn(__fmul_rn(f, ws), xs[e]));
+                }
+              } else {
+#pragma unroll
+                for (int e = 0; e < 4; e += 2) {
+                  float p0, p1;
+                  q8i_scale2(__int2float_rn((int)v[b * CH + c + e]), __int2float_rn((int)v[b * CH + c + e + 1]), ws, xs[e], xs[e + 1], p0, p1);
+                  acc[c + e] = __fadd_rn(acc[c + e], p0);
+                  acc[c + e + 1] = __fadd_rn(acc[c + e + 1], p1);
+                }
               }
             }
           }
