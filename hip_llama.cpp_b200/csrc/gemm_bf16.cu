@@ -467,7 +467,6 @@ bool gemm_bf16_ok(const BfArgs& a) {
   return true;
 }
 
-int gemm_bf16_pick_nt(int N) { return N <= 16 ? 16 : (N <= 32 ? 32 : (N <= 64 ? 64 : (N <= 128 ? 128 : 256))); }
 
 template <int NT, int MT = 1, bool SWIGLU = false>
 static int bf_launch_nt(cudaStream_t st, const CUtensorMap* mw, const CUtensorMap& mx, const BfP& p, dim3 grid, bool pdl) {
@@ -477,12 +476,22 @@ static int bf_launch_nt(cudaStream_t st, const CUtensorMap* mw, const CUtensorMa
   THA_CUDA_OK(launch(k, grid, dim3(128 + 128 * MT), (size_t)S::TOTAL, st, pdl, mw[0], mw[1], mw[2], mx, p));
   return THA_STATUS_SUCCESS;
 }
-// 256-row work items for prompt-sized N (THA_BF16_MT=1 keeps 128-row items)
-static int bf_mt(int NT, int N) {
-  static int forced = -1;
-  if (forced < 0) { const char* v = getenv("THA_BF16_MT"); forced = (v && *v) ? atoi(v) : 0; }
-  if (forced == 1 || forced == 2) return NT == 256 ? forced : 1;
-  return (NT == 256 && N >= 512) ? 2 : 1;
+// Output tile (128 mt weight rows x nt activation rows) of a product of `tiles` 128-row weight tiles with N activation rows: the one whose
+// waves over the SMs cost least.  A wave of 256 x 256 / 128 x 256 / 128 x 128 / 128 x 64 tiles takes 50 / 28 / 20.5 / 19.5 us at K = 4096
+// (small tiles pull more through L2 per product), so a large tile pays once it fills the SMs.  Measured, us, in that order: 2100 rows x
+// [4096, 4096] 54 / 59 / 86 / 155; 2825 x [4096, 4096] 92 / 80 / 103 / 190; 2100 x [1024, 4608] 53 / 33 / 30 / 49; 700 x [2048, 2048] 35 / 25 / 19 / 26;
+// 4000 x [12288, 4096] 313 / 312 / 409 / 763.
+BfTile gemm_bf16_tile(int tiles, int N) {
+  if (N <= 128) return {N <= 16 ? 16 : (N <= 32 ? 32 : (N <= 64 ? 64 : 128)), 1};
+  static const struct { BfTile t; int cost; } form[4] = {{{256, 2}, 100}, {{256, 1}, 56}, {{128, 1}, 41}, {{64, 1}, 39}};
+  BfTile best = form[0].t;
+  long long least = 0;
+  for (int i = 0; i < 4; i++) {
+    const long long items = (long long)ceil_div(tiles, form[i].t.mt) * ceil_div(N, form[i].t.nt);
+    const long long c = (items + 147) / 148 * form[i].cost;
+    if (i == 0 || c < least) { least = c; best = form[i].t; }
+  }
+  return best;
 }
 
 template <int NT>
@@ -525,17 +534,17 @@ static int bfc_try(cudaStream_t st, const CUtensorMap* mw, const CUtensorMap& mx
 }
 
 bool gemm_bf16_swiglu_ok(const BfArgs& a) {
-  const int NT = gemm_bf16_pick_nt(a.N);
-  return a.swiglu_out && a.n_mats == 2 && a.M[0] == a.M[1] && a.splits <= 1 && NT == 256 && bf_mt(NT, a.N) == 2 && !a.colscale &&
-         (a.ld_swiglu % 1) == 0;
+  return a.swiglu_out && a.n_mats == 2 && a.M[0] == a.M[1] && a.splits <= 1 && a.N >= 512 && !a.colscale;
 }
 
 int gemm_bf16_launch(cudaStream_t st, const BfArgs& a, bool pdl) {
   if (!gemm_bf16_ok(a)) return THA_STATUS_INVALID_ARG;
-  const int NT = gemm_bf16_pick_nt(a.N);
   const bool swiglu = a.swiglu_out != nullptr;
   if (swiglu && !gemm_bf16_swiglu_ok(a)) return THA_STATUS_NOT_SUPPORTED;
-  const int MT = swiglu ? 1 : bf_mt(NT, a.N);   // SwiGLU: 128-row boxes of each of the two matrices (the kernel itself runs MT = 2)
+  int tiles128 = 0;
+  for (int i = 0; i < a.n_mats; i++) tiles128 += ceil_div(a.M[i], TC_BM);
+  const BfTile tile = swiglu ? BfTile{256, 1} : gemm_bf16_tile(tiles128, a.N);
+  const int NT = tile.nt, MT = tile.mt;   // SwiGLU: 128-row boxes of each of the two matrices (the kernel itself runs MT = 2)
   CUtensorMap mw[3], mx;
   BfP p = {};
   int tiles = 0;

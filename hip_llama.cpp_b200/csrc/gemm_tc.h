@@ -56,7 +56,8 @@ struct BfArgs {
 };
 bool gemm_bf16_swiglu_ok(const BfArgs& a);   // the launch can take the SwiGLU read-out
 bool gemm_bf16_ok(const BfArgs& a);
-int gemm_bf16_pick_nt(int N);
+struct BfTile { int nt, mt; };
+BfTile gemm_bf16_tile(int tiles, int N);   // output tile: 128 mt weight rows (of `tiles` 128-row tiles) x nt activation rows
 int gemm_bf16_launch(cudaStream_t st, const BfArgs& a, bool pdl);
 
 bool gemm_tc_ok(const TcArgs& a);

@@ -1,5 +1,5 @@
-"""bf16 products of few rows, whose tiles are dealt to clusters of CTAs along K (csrc/gemm_bf16.cu): ragged tiles, ragged and empty
-shares of K, every column-tile width, and the sizes on both sides of the rule that picks the cluster."""
+"""bf16 products (csrc/gemm_bf16.cu): few rows, whose tiles are dealt to clusters of CTAs along K, with ragged tiles, ragged and empty shares of
+K, every column-tile width and the sizes on both sides of the rule that picks the cluster; and more rows, with every output tile."""
 import ctypes as C
 
 import pytest
@@ -10,9 +10,9 @@ from pkgload import load_pkg
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("rows", [1, 16, 17, 33, 64, 65, 128])
+@pytest.mark.parametrize("rows", [1, 16, 17, 33, 64, 65, 128, 129, 384, 700, 1100])
 @pytest.mark.parametrize("M,K", [(128, 64), (133, 128), (1024, 256), (1024, 1160), (2048, 1096), (3205, 512), (3208, 1024), (4608, 520), (6401, 256), (12900, 256)])
-def test_few_rows(rows, M, K):
+def test_rows(rows, M, K):
     lib = load_pkg("cabi").lib()
     g = torch.Generator(device="cuda").manual_seed(rows * 1000 + K)
     W = torch.randn(M, K, device="cuda", generator=g).to(torch.bfloat16)
