@@ -19,6 +19,7 @@ __device__ __forceinline__ float4 ar_ld(const float* p) { return ldg_stream(rein
 template <typename T, int GS>
 __global__ void __launch_bounds__(AR_THREADS) hyb_attn_row_kernel(tha_attn_t a, tha_rows_t rows, tha_kv_t kv, const float* __restrict__ q, T* __restrict__ out,
                                                                   int splits, float* __restrict__ partial, const float* __restrict__ gate, long long ldg) {
+  hyb_pdl_enter();
   constexpr int NI = AR_MAXD / 32;                 // float4 per lane of a row of up to 128 channels
   __shared__ float sm_acc[4][GS][AR_MAXD];
   __shared__ float sm_ml[4][GS][2];
@@ -157,9 +158,9 @@ static int row_launch(cudaStream_t s, const tha_attn_t* a, const tha_rows_t* row
                       const float* gate, long long ldg) {
   const int gsize = a->heads / a->kv_heads, gs = gsize >= 3 ? AR_HEADS : gsize;
   const dim3 grid(rows->n_rows * splits, a->kv_heads, ceil_div(gsize, gs));
-  if (gs == 1) THA_CUDA_OK(launch(hyb_attn_row_kernel<T, 1>, grid, dim3(AR_THREADS), 0, s, false, *a, *rows, *kv, q, out, splits, partial, gate, ldg));
-  else if (gs == 2) THA_CUDA_OK(launch(hyb_attn_row_kernel<T, 2>, grid, dim3(AR_THREADS), 0, s, false, *a, *rows, *kv, q, out, splits, partial, gate, ldg));
-  else THA_CUDA_OK(launch(hyb_attn_row_kernel<T, AR_HEADS>, grid, dim3(AR_THREADS), 0, s, false, *a, *rows, *kv, q, out, splits, partial, gate, ldg));
+  if (gs == 1) THA_CUDA_OK(launch(hyb_attn_row_kernel<T, 1>, grid, dim3(AR_THREADS), 0, s, pdl_enabled() != 0, *a, *rows, *kv, q, out, splits, partial, gate, ldg));
+  else if (gs == 2) THA_CUDA_OK(launch(hyb_attn_row_kernel<T, 2>, grid, dim3(AR_THREADS), 0, s, pdl_enabled() != 0, *a, *rows, *kv, q, out, splits, partial, gate, ldg));
+  else THA_CUDA_OK(launch(hyb_attn_row_kernel<T, AR_HEADS>, grid, dim3(AR_THREADS), 0, s, pdl_enabled() != 0, *a, *rows, *kv, q, out, splits, partial, gate, ldg));
   return THA_STATUS_SUCCESS;
 }
 int hyb_attn_row_launch(cudaStream_t s, int dtype, const tha_attn_t* a, const tha_rows_t* rows, const tha_kv_t* kv, const float* q, void* out, int splits,

@@ -24,6 +24,7 @@ template <typename T>
 __global__ void hyb_add_norm_kernel(float* __restrict__ x, const float* __restrict__ left, const float* __restrict__ left_b, float c_left, const float* __restrict__ right,
                                     float c_right, const float* __restrict__ embed_out, const float* __restrict__ vec, tha_norm_t n,
                                     int has_norm, float eps, T* __restrict__ out, long long ldo, int width) {
+  hyb_pdl_enter();
   __shared__ float red[33];
   const int r = blockIdx.x;
   float* xr = x + (size_t)r * width;
@@ -66,6 +67,7 @@ __global__ void hyb_add_norm_kernel(float* __restrict__ x, const float* __restri
 template <typename T>
 __global__ void hyb_side_gate_kernel(T* __restrict__ out, const float* __restrict__ gate_raw, long long ldg, const T* __restrict__ table, int side_cols,
                                      int col0, const int* __restrict__ token, int n_rows, int dim) {
+  hyb_pdl_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_rows * dim) return;
   const int r = i / dim, j = i - r * dim;
@@ -81,6 +83,7 @@ template <typename T>
 __global__ void hyb_block_finish_kernel(float* __restrict__ x, const float* __restrict__ ff, const float* __restrict__ ff_b, const float* __restrict__ y,
                                         float m, const float* __restrict__ w, float eps, float* __restrict__ tap, const float* __restrict__ embed_out,
                                         const float* __restrict__ vec, tha_norm_t n, int has_norm, T* __restrict__ out, long long ldo, int width) {
+  hyb_pdl_enter();
   __shared__ float red[33];
   const int r = blockIdx.x;
   float* xr = x + (size_t)r * width;
@@ -129,6 +132,7 @@ template <typename T, int V>
 __global__ void hyb_post_norm_kernel(float* __restrict__ x, const float* __restrict__ dense, const float* __restrict__ dense_gate, long long ldg, int top,
                                      const float* __restrict__ weight, const int* __restrict__ inv, const float* __restrict__ down, float m, tha_norm_t n,
                                      float eps, float* __restrict__ tap, T* __restrict__ out, int width) {
+  hyb_pdl_enter();
   extern __shared__ __align__(16) float yrow[];
   __shared__ float red[33];
   const size_t r = blockIdx.x;
@@ -188,10 +192,10 @@ extern "C" int tha_hyb_add_norm(void* stream, int dtype, float* x, const float* 
   const tha_norm_t none = {};
   const int nt = block_threads(width);
   if (dtype == THA_DT_BF16)
-    THA_CUDA_OK(launch(hyb_add_norm_kernel<bf16>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, false, x, left, left_b, c_left, right, c_right, embed_out, vec,
+    THA_CUDA_OK(launch(hyb_add_norm_kernel<bf16>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, pdl_enabled() != 0, x, left, left_b, c_left, right, c_right, embed_out, vec,
                        n ? *n : none, n ? 1 : 0, eps, (bf16*)out, ldo > 0 ? ldo : (long long)width, width));
   else
-    THA_CUDA_OK(launch(hyb_add_norm_kernel<float>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, false, x, left, left_b, c_left, right, c_right, embed_out,
+    THA_CUDA_OK(launch(hyb_add_norm_kernel<float>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, pdl_enabled() != 0, x, left, left_b, c_left, right, c_right, embed_out,
                        vec, n ? *n : none, n ? 1 : 0, eps, (float*)out, ldo > 0 ? ldo : (long long)width, width));
   return THA_STATUS_SUCCESS;
 }
@@ -202,10 +206,10 @@ extern "C" int tha_hyb_side_gate(void* stream, int dtype, void* out, const float
   if (!out || !gate_raw || !side_table || !token || side->col0 < 0 || side->col0 + side->dim > side_cols) return THA_STATUS_INVALID_ARG;
   const dim3 grid(ceil_div(n_rows * side->dim, 256));
   if (dtype == THA_DT_BF16)
-    THA_CUDA_OK(launch(hyb_side_gate_kernel<bf16>, grid, dim3(256), 0, (cudaStream_t)stream, false, (bf16*)out, gate_raw, ldg, (const bf16*)side_table,
+    THA_CUDA_OK(launch(hyb_side_gate_kernel<bf16>, grid, dim3(256), 0, (cudaStream_t)stream, pdl_enabled() != 0, (bf16*)out, gate_raw, ldg, (const bf16*)side_table,
                        side_cols, side->col0, token, n_rows, side->dim));
   else
-    THA_CUDA_OK(launch(hyb_side_gate_kernel<float>, grid, dim3(256), 0, (cudaStream_t)stream, false, (float*)out, gate_raw, ldg,
+    THA_CUDA_OK(launch(hyb_side_gate_kernel<float>, grid, dim3(256), 0, (cudaStream_t)stream, pdl_enabled() != 0, (float*)out, gate_raw, ldg,
                        (const float*)side_table, side_cols, side->col0, token, n_rows, side->dim));
   return THA_STATUS_SUCCESS;
 }
@@ -218,10 +222,10 @@ extern "C" int tha_hyb_block_finish(void* stream, int dtype, float* x, const flo
   const tha_norm_t none = {};
   const int nt = block_threads(width);
   if (dtype == THA_DT_BF16)
-    THA_CUDA_OK(launch(hyb_block_finish_kernel<bf16>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, false, x, ff, ff_b, y, m, y_norm, eps, tap, embed_out,
+    THA_CUDA_OK(launch(hyb_block_finish_kernel<bf16>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, pdl_enabled() != 0, x, ff, ff_b, y, m, y_norm, eps, tap, embed_out,
                        vec, next_norm ? *next_norm : none, next_norm ? 1 : 0, (bf16*)out, ldo > 0 ? ldo : (long long)width, width));
   else
-    THA_CUDA_OK(launch(hyb_block_finish_kernel<float>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, false, x, ff, ff_b, y, m, y_norm, eps, tap, embed_out,
+    THA_CUDA_OK(launch(hyb_block_finish_kernel<float>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, pdl_enabled() != 0, x, ff, ff_b, y, m, y_norm, eps, tap, embed_out,
                        vec, next_norm ? *next_norm : none, next_norm ? 1 : 0, (float*)out, ldo > 0 ? ldo : (long long)width, width));
   return THA_STATUS_SUCCESS;
 }
@@ -238,7 +242,7 @@ extern "C" int tha_hyb_post_norm(void* stream, int dtype, float* x, const float*
 #define POST_GO(T, V)                                                                                                                     \
   do {                                                                                                                                    \
     if (smem > 47 * 1024) THA_CUDA_OK(cudaFuncSetAttribute(hyb_post_norm_kernel<T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-    THA_CUDA_OK(launch(hyb_post_norm_kernel<T, V>, grid, block, smem, (cudaStream_t)stream, false, x, dense, dense_gate, ldg, top, weight, inv, down, m, \
+    THA_CUDA_OK(launch(hyb_post_norm_kernel<T, V>, grid, block, smem, (cudaStream_t)stream, pdl_enabled() != 0, x, dense, dense_gate, ldg, top, weight, inv, down, m, \
                        *norm, eps, tap, (T*)out, width));                                                                                 \
   } while (0)
   if (dtype == THA_DT_BF16) { if (vec) POST_GO(bf16, 4); else POST_GO(bf16, 1); }

@@ -25,6 +25,7 @@ namespace tha {
 constexpr int GD_WARPS = 4, GD_COLS = 2;
 
 __global__ void hyb_tanh_cols_kernel(float* __restrict__ proj, long long ldp, int col0, int cols, int n_rows) {
+  hyb_pdl_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_rows * cols) return;
   float* p = proj + (size_t)(i / cols) * ldp + col0 + i % cols;
@@ -33,6 +34,7 @@ __global__ void hyb_tanh_cols_kernel(float* __restrict__ proj, long long ldp, in
 
 __global__ void hyb_gdelta_gates_kernel(float* __restrict__ w, float* __restrict__ proj, long long ldp, int o_a, size_t n, int hd,
                                         const float* __restrict__ w0, const float* __restrict__ a_b) {
+  hyb_pdl_enter();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int c = (int)(i % hd);
@@ -45,6 +47,7 @@ template <int RPL, int AHEAD>
 __global__ void __launch_bounds__(32 * GD_WARPS) hyb_gdelta_scan_kernel(tha_gdelta_t g, tha_rows_t rows, tha_state_store_t st,
                                                                         const float* __restrict__ proj, long long ldp,
                                                                         const float* __restrict__ decay, float* __restrict__ o_raw) {
+  hyb_pdl_enter();
   const int s = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int D = g.dim;
   const int pair = blockIdx.z * GD_WARPS + warp, e0 = pair * GD_COLS;
@@ -151,15 +154,15 @@ extern "C" int tha_hyb_gdelta_scan(void* stream, int dtype, const tha_gdelta_t* 
   if (g->dim > 256) return THA_STATUS_NOT_SUPPORTED;   // 8 key channels per lane is the widest register form
   cudaStream_t s = (cudaStream_t)stream;
   const int R = rows->n_rows, HD = g->heads * g->dim;
-  THA_CUDA_OK(launch(hyb_tanh_cols_kernel, dim3(ceil_div(R * g->rank, 256)), dim3(256), 0, s, false, proj, ldp, g->o_w1, g->rank, R));
+  THA_CUDA_OK(launch(hyb_tanh_cols_kernel, dim3(ceil_div(R * g->rank, 256)), dim3(256), 0, s, pdl_enabled() != 0, proj, ldp, g->o_w1, g->rank, R));
   const int st1 = tha_hyb_linear(stream, dtype, w_raw, HD, proj + g->o_w1, ldp, 1, nullptr, g->w_w2, 0, R, HD, g->rank, nullptr, 0);
   if (st1 != THA_STATUS_SUCCESS) return st1;
   const size_t n = (size_t)R * HD;
-  THA_CUDA_OK(launch(hyb_gdelta_gates_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, s, false, w_raw, proj, ldp, g->o_a, n, HD, g->w0,
+  THA_CUDA_OK(launch(hyb_gdelta_gates_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, s, pdl_enabled() != 0, w_raw, proj, ldp, g->o_a, n, HD, g->w0,
                      g->a_b));
   const dim3 grid(rows->n_seqs, g->heads, ceil_div(g->dim, GD_COLS * GD_WARPS)), block(32 * GD_WARPS);
 #define GD_LAUNCH(RPL, A) \
-  THA_CUDA_OK(launch(hyb_gdelta_scan_kernel<RPL, A>, grid, block, 0, s, false, *g, *rows, *st, (const float*)proj, ldp, (const float*)w_raw, o_raw))
+  THA_CUDA_OK(launch(hyb_gdelta_scan_kernel<RPL, A>, grid, block, 0, s, pdl_enabled() != 0, *g, *rows, *st, (const float*)proj, ldp, (const float*)w_raw, o_raw))
   // tokens fetched ahead: two at 65 .. 128 key channels (measured: four 4 % slower, eight spill), four below
   if (g->dim <= 32) GD_LAUNCH(1, 4);
   else if (g->dim <= 64) GD_LAUNCH(2, 4);

@@ -24,6 +24,7 @@ namespace tha {
 constexpr int GLA_WARPS = 4, GLA_STATE_PAD = 8;   // a head's value columns are padded to a multiple of 8 in the slot
 
 __global__ void hyb_gla_decay_kernel(float* __restrict__ z, size_t n, int hd, const float* __restrict__ bias, float inv_tau) {
+  hyb_pdl_enter();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float v = z[i] + (bias ? bias[i % hd] : 0.f);
@@ -32,6 +33,7 @@ __global__ void hyb_gla_decay_kernel(float* __restrict__ z, size_t n, int hd, co
 
 __global__ void hyb_hgrn_gates_kernel(float* __restrict__ proj, long long ldp, float* __restrict__ decay, size_t n, int hd, int o_q, int o_f,
                                       const float* __restrict__ f_b, const float* __restrict__ lower) {
+  hyb_pdl_enter();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const size_t r = i / hd;
@@ -90,6 +92,7 @@ __global__ void __launch_bounds__(32 * GLA_WARPS) hyb_gla_scan_kernel(tha_gla_t 
                                                                       const float* __restrict__ proj, long long ldp,
                                                                       const float* __restrict__ decay, const float* __restrict__ aux,
                                                                       float* __restrict__ o_raw, float qscale, ScanSegs segs) {
+  hyb_pdl_enter();
   const int h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int D = g.dim, E = g.vdim;
   const int e0 = (blockIdx.z * GLA_WARPS + warp) * GLA_COLS;
@@ -272,6 +275,7 @@ __global__ void __launch_bounds__(32 * GLA_WARPS) hyb_gla_scan_kernel(tha_gla_t 
 
 // end states from zero -> true end states, a thread per state element of a head, the segments in order (eight loads in flight)
 __global__ void hyb_scan_combine_kernel(tha_gla_t g, tha_rows_t rows, ScanSegs segs) {
+  hyb_pdl_enter();
   const int EP = (g.vdim + GLA_STATE_PAD - 1) / GLA_STATE_PAD * GLA_STATE_PAD, n = g.dim * EP;
   const int i = blockIdx.x * blockDim.x + threadIdx.x, h = blockIdx.y, s = blockIdx.z;
   if (i >= n) return;
@@ -341,10 +345,10 @@ static int gla_scan_launch(cudaStream_t s, const tha_gla_t* g, const tha_rows_t*
   const bool decode = !seg && rows->max_seq_rows <= 2 && g->dim <= 128;
   const int cols = wide ? 8 : (seg || decode) && g->dim <= 128 ? 4 : 2;
   const dim3 grid(seg ? rows->n_rows / len + rows->n_seqs : rows->n_seqs, g->heads, ceil_div(g->vdim, cols * GLA_WARPS)), block(32 * GLA_WARPS);
-#define GLA_LAUNCH(R, A, C, F, L, V) THA_CUDA_OK(launch(hyb_gla_scan_kernel<R, A, C, F, L, V>, grid, block, 0, s, false, *g, *rows, *st, proj, ldp, dec, aux, o_raw, qscale, segs))
+#define GLA_LAUNCH(R, A, C, F, L, V) THA_CUDA_OK(launch(hyb_gla_scan_kernel<R, A, C, F, L, V>, grid, block, 0, s, pdl_enabled() != 0, *g, *rows, *st, proj, ldp, dec, aux, o_raw, qscale, segs))
 #define GLA_BOTH(R, A, C, V) do { if (seg) { GLA_LAUNCH(R, A, C, LFORM, true, V); \
     THA_CUDA_OK(launch(hyb_scan_combine_kernel, dim3(ceil_div(g->dim * ((g->vdim + GLA_STATE_PAD - 1) / GLA_STATE_PAD * GLA_STATE_PAD), 256), g->heads, rows->n_seqs), \
-                       dim3(256), 0, s, false, *g, *rows, segs)); } \
+                       dim3(256), 0, s, pdl_enabled() != 0, *g, *rows, segs)); } \
     GLA_LAUNCH(R, A, C, FORM, false, V); } while (0)
   // many warps per scheduler (segments): wide loads, eight columns a warp, two tokens ahead; few: two columns, four tokens ahead
   if (wide) { if (g->dim <= 64) GLA_BOTH(2, 2, 8, 2); else GLA_BOTH(4, 2, 8, 4); }
@@ -385,7 +389,7 @@ extern "C" int tha_hyb_gla_scan(void* stream, int dtype, const tha_gla_t* g, con
   if (g->dim > 512) return THA_STATUS_NOT_SUPPORTED;   // 16 key channels per lane is the widest register form
   cudaStream_t s = (cudaStream_t)stream;
   const size_t n = (size_t)rows->n_rows * g->heads * g->dim;
-  THA_CUDA_OK(launch(hyb_gla_decay_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, s, false, z_raw, n, g->heads * g->dim, g->b_a2,
+  THA_CUDA_OK(launch(hyb_gla_decay_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, s, pdl_enabled() != 0, z_raw, n, g->heads * g->dim, g->b_a2,
                      1.0f / g->tau));
   const int status = hyb_scan_launch(s, SCAN_CHANNEL_DECAY, g, rows, st, proj, ldp, z_raw, nullptr, o_raw, 1.0f / sqrtf((float)g->dim), seg_scratch,
                                      seg_scratch_floats);
@@ -403,7 +407,7 @@ extern "C" int tha_hyb_hgrn_scan(void* stream, int dtype, const tha_hgrn_t* g, c
   if (g->dim > 512) return THA_STATUS_NOT_SUPPORTED;
   cudaStream_t s = (cudaStream_t)stream;
   const size_t n = (size_t)rows->n_rows * g->heads * g->dim;
-  THA_CUDA_OK(launch(hyb_hgrn_gates_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, s, false, proj, ldp, decay, n, g->heads * g->dim,
+  THA_CUDA_OK(launch(hyb_hgrn_gates_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, s, pdl_enabled() != 0, proj, ldp, decay, n, g->heads * g->dim,
                      g->o_q, g->o_f, g->f_b, g->lower));
   tha_gla_t a = {};
   a.heads = g->heads; a.dim = g->dim; a.vdim = g->vdim; a.o_q = g->o_q; a.o_k = g->o_f; a.o_v = g->o_v; a.state_off = g->state_off;

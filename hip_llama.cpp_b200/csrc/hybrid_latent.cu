@@ -18,6 +18,7 @@ namespace tha {
 template <typename T>
 __global__ void hyb_latent_prepare_kernel(tha_latent_t a, tha_rows_t rows, tha_kv_t kv, const float* __restrict__ proj, long long ldp,
                                           const float* __restrict__ cos_t, const float* __restrict__ sin_t, int rot_dims, T* __restrict__ cq) {
+  hyb_pdl_enter();
   __shared__ float red[33];
   const int r = blockIdx.x;
   const float* pr = proj + (size_t)r * ldp;
@@ -47,6 +48,7 @@ __global__ void hyb_latent_prepare_kernel(tha_latent_t a, tha_rows_t rows, tha_k
 template <typename T>
 __global__ void hyb_latent_split_q_kernel(tha_latent_t a, int n_rows, const float* __restrict__ qfull, long long ldq, const float* __restrict__ cos_t,
                                           const float* __restrict__ sin_t, int rot_dims, T* __restrict__ q_plain, float* __restrict__ q_abs) {
+  hyb_pdl_enter();
   const int r = blockIdx.x;
   const int per = a.dim + a.rot_dim, DA = a.kv_rank + a.rot_dim, half = rot_dims / 2;
   const float* q = qfull + (size_t)r * ldq;
@@ -94,6 +96,7 @@ template <int MT>
 __global__ void __launch_bounds__(128 * MT) hyb_attn_wide_kernel(tha_attn_t a, tha_rows_t rows, tha_kv_t kv, const float* __restrict__ q,
                                                                  __nv_bfloat16* __restrict__ out, int AG, int AP, int splits,
                                                                  float* __restrict__ partial) {
+  hyb_pdl_enter();
   constexpr int PAIRS = 16 * MT, NW = 4 * MT;
   extern __shared__ __align__(16) unsigned char smraw[];
   const int D = a.dim, E = a.vdim, gsize = a.heads / a.kv_heads, ES = E / 4;
@@ -349,13 +352,13 @@ int hyb_attn_wide_launch(cudaStream_t s, const tha_attn_t* a, const tha_rows_t* 
   const size_t smem = wide_smem(a, pairs);
   if (pairs == 64) {
     THA_CUDA_OK(cudaFuncSetAttribute(hyb_attn_wide_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    THA_CUDA_OK(launch(hyb_attn_wide_kernel<4>, grid, dim3(512), smem, s, false, *a, *rows, *kv, q, out, AG, AP, splits, partial));
+    THA_CUDA_OK(launch(hyb_attn_wide_kernel<4>, grid, dim3(512), smem, s, pdl_enabled() != 0, *a, *rows, *kv, q, out, AG, AP, splits, partial));
   } else if (pairs == 32) {
     THA_CUDA_OK(cudaFuncSetAttribute(hyb_attn_wide_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    THA_CUDA_OK(launch(hyb_attn_wide_kernel<2>, grid, dim3(256), smem, s, false, *a, *rows, *kv, q, out, AG, AP, splits, partial));
+    THA_CUDA_OK(launch(hyb_attn_wide_kernel<2>, grid, dim3(256), smem, s, pdl_enabled() != 0, *a, *rows, *kv, q, out, AG, AP, splits, partial));
   } else {
     THA_CUDA_OK(cudaFuncSetAttribute(hyb_attn_wide_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    THA_CUDA_OK(launch(hyb_attn_wide_kernel<1>, grid, dim3(128), smem, s, false, *a, *rows, *kv, q, out, AG, AP, splits, partial));
+    THA_CUDA_OK(launch(hyb_attn_wide_kernel<1>, grid, dim3(128), smem, s, pdl_enabled() != 0, *a, *rows, *kv, q, out, AG, AP, splits, partial));
   }
   return THA_STATUS_SUCCESS;
 }
@@ -374,10 +377,10 @@ extern "C" int tha_hyb_latent_prepare(void* stream, int dtype, const tha_latent_
   int nt = 64;
   while (nt < a->kv_rank / 2 && nt < 256) nt += 32;
   if (dtype == THA_DT_BF16)
-    THA_CUDA_OK(launch(hyb_latent_prepare_kernel<bf16>, dim3(rows->n_rows), dim3(nt), 0, (cudaStream_t)stream, false, *a, *rows, *kv, proj, ldp,
+    THA_CUDA_OK(launch(hyb_latent_prepare_kernel<bf16>, dim3(rows->n_rows), dim3(nt), 0, (cudaStream_t)stream, pdl_enabled() != 0, *a, *rows, *kv, proj, ldp,
                        cos_t, sin_t, rot_dims, (bf16*)cq));
   else
-    THA_CUDA_OK(launch(hyb_latent_prepare_kernel<float>, dim3(rows->n_rows), dim3(nt), 0, (cudaStream_t)stream, false, *a, *rows, *kv, proj, ldp,
+    THA_CUDA_OK(launch(hyb_latent_prepare_kernel<float>, dim3(rows->n_rows), dim3(nt), 0, (cudaStream_t)stream, pdl_enabled() != 0, *a, *rows, *kv, proj, ldp,
                        cos_t, sin_t, rot_dims, (float*)cq));
   return THA_STATUS_SUCCESS;
 }
@@ -390,10 +393,10 @@ extern "C" int tha_hyb_latent_split_q(void* stream, int dtype, const tha_latent_
   int nt = 64;
   while (nt < a->heads * a->dim / 2 && nt < 256) nt += 32;
   if (dtype == THA_DT_BF16)
-    THA_CUDA_OK(launch(hyb_latent_split_q_kernel<bf16>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, false, *a, n_rows, qfull, ldq, cos_t, sin_t,
+    THA_CUDA_OK(launch(hyb_latent_split_q_kernel<bf16>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, pdl_enabled() != 0, *a, n_rows, qfull, ldq, cos_t, sin_t,
                        rot_dims, (bf16*)q_plain, q_abs));
   else
-    THA_CUDA_OK(launch(hyb_latent_split_q_kernel<float>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, false, *a, n_rows, qfull, ldq, cos_t, sin_t,
+    THA_CUDA_OK(launch(hyb_latent_split_q_kernel<float>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, pdl_enabled() != 0, *a, n_rows, qfull, ldq, cos_t, sin_t,
                        rot_dims, (float*)q_plain, q_abs));
   return THA_STATUS_SUCCESS;
 }

@@ -24,6 +24,7 @@ namespace tha {
 template <typename T>
 __global__ void hyb_rmsnorm_kernel(T* __restrict__ out, const float* __restrict__ x, const float* __restrict__ w, float w_offset,
                                    float eps, int width, const int* __restrict__ rows_idx) {
+  hyb_pdl_enter();
   __shared__ float red[33];
   const int r = blockIdx.x;
   const float* xr = x + (size_t)(rows_idx ? rows_idx[r] : r) * width;
@@ -38,6 +39,7 @@ __global__ void hyb_rmsnorm_kernel(T* __restrict__ out, const float* __restrict_
 template <typename T>
 __global__ void hyb_dyt_kernel(T* __restrict__ out, const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b,
                                float alpha, int width, const int* __restrict__ rows_idx) {
+  hyb_pdl_enter();
   const int r = blockIdx.x;
   const float* xr = x + (size_t)(rows_idx ? rows_idx[r] : r) * width;
   for (int i = threadIdx.x; i < width; i += blockDim.x) hyb_store(out + (size_t)r * width + i, fmaf(tanhf(alpha * xr[i]), w[i], b ? b[i] : 0.f));
@@ -46,6 +48,7 @@ __global__ void hyb_dyt_kernel(T* __restrict__ out, const float* __restrict__ x,
 // two dynamic-tanh norms of the same row in one pass (the two norms of a parallel block)
 template <typename T>
 __global__ void hyb_dyt2_kernel(T* __restrict__ out1, T* __restrict__ out2, const float* __restrict__ x, tha_norm_t n1, tha_norm_t n2, int width) {
+  hyb_pdl_enter();
   const int r = blockIdx.x;
   const float* xr = x + (size_t)r * width;
   for (int i = threadIdx.x; i < width; i += blockDim.x) {
@@ -60,6 +63,7 @@ __global__ void hyb_dyt2_kernel(T* __restrict__ out1, T* __restrict__ out2, cons
 template <typename T>
 __global__ void hyb_layernorm_kernel(T* __restrict__ out, const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b,
                                      float eps, int width, const int* __restrict__ rows_idx) {
+  hyb_pdl_enter();
   __shared__ float red[33];
   const int r = blockIdx.x;
   const float* xr = x + (size_t)(rows_idx ? rows_idx[r] : r) * width;
@@ -85,6 +89,7 @@ __global__ void __launch_bounds__(256) hyb_linear_kernel(float* __restrict__ C, 
                                                          long long w_group_stride, int M, int N, int K,
                                                          const int* __restrict__ group_off, int n_groups, long long a_zs, long long w_zs,
                                                          long long c_zs) {
+  hyb_pdl_enter();
   __shared__ float As[LK][LT + 4];
   __shared__ float Ws[LK][LT + 4];
   // blockIdx.z: one independent product per head (strides in elements), 0 strides otherwise
@@ -165,6 +170,7 @@ __global__ void __launch_bounds__(128) hyb_linear_mma_kernel(float* __restrict__
                                                              const __nv_bfloat16* __restrict__ W, long long w_group_stride, int M, int N,
                                                              int K, const int* __restrict__ group_off, int n_groups, long long a_zs,
                                                              long long w_zs, long long c_zs) {
+  hyb_pdl_enter();
   __shared__ __align__(16) __nv_bfloat16 As[LT][MKP];
   __shared__ __align__(16) __nv_bfloat16 Ws[LT][MKP];
   A += (size_t)blockIdx.z * a_zs; W += (size_t)blockIdx.z * w_zs; C += (size_t)blockIdx.z * c_zs;
@@ -259,6 +265,7 @@ __global__ void __launch_bounds__(128) hyb_linear_mma_kernel(float* __restrict__
 // ------------------------------------------------------------------------------------------------------------------
 __global__ void hyb_rotary_kernel(const double* __restrict__ inv_freq, int half, float mag, const int* __restrict__ pos, int n_rows,
                                   float* __restrict__ cos_out, float* __restrict__ sin_out) {
+  hyb_pdl_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_rows * half) return;
   const int r = i / half, c = i % half;
@@ -275,6 +282,7 @@ __global__ void hyb_rotary_kernel(const double* __restrict__ inv_freq, int half,
 __global__ void hyb_attn_prepare_kernel(tha_attn_t a, tha_rows_t rows, tha_kv_t kv, const float* __restrict__ proj, long long ldp,
                                         const float* __restrict__ cos_t, const float* __restrict__ sin_t, int rot_dims,
                                         float* __restrict__ q_out) {
+  hyb_pdl_enter();
   const int r = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int slot = rows.seq_slot[rows.row_seq[r]], t = rows.pos[r];
@@ -348,6 +356,7 @@ template <typename T, int VC>
 __global__ void __launch_bounds__(128) hyb_attn_kernel(tha_attn_t a, tha_rows_t rows, tha_kv_t kv, const float* __restrict__ q,
                                                        T* __restrict__ out, int AG, int AP, int splits, float* __restrict__ partial,
                                                        const float* __restrict__ gate, long long ldg) {
+  hyb_pdl_enter();
   extern __shared__ __align__(16) float sm[];
   const int D = a.dim, E = a.vdim, gsize = a.heads / a.kv_heads;
   const bool vec = ((D | E) & 3) == 0;         // 128-bit shared-memory reads: rows padded to keep them aligned and conflict-free
@@ -605,6 +614,7 @@ template <bool EXACT, bool CAP, bool REL, int DT>
 __global__ void __launch_bounds__(AM_THREADS, 1) hyb_attn_mma_kernel(tha_attn_t a, tha_rows_t rows, tha_kv_t kv, const float* __restrict__ q,
                                                            __nv_bfloat16* __restrict__ out, int AG, int AP, int splits,
                                                            float* __restrict__ partial, const float* __restrict__ gate, long long ldg) {
+  hyb_pdl_enter();
   extern __shared__ __align__(16) unsigned char smraw[];
   const int D = DT ? DT : a.dim, E = DT ? DT : a.vdim, gsize = a.heads / a.kv_heads;
   const int KS = D + 8, VS = E + 8;                      // padded rows: conflict-free ldmatrix reads
@@ -873,6 +883,7 @@ constexpr int AMG_SPLITS = 32;
 template <typename T>
 __global__ void __launch_bounds__(128) hyb_attn_merge_kernel(T* __restrict__ out, const float* __restrict__ partial, int n_rows, int heads, int E, int splits,
                                                              tha_attn_t a, const float* __restrict__ gate, long long ldg) {
+  hyb_pdl_enter();
   const int idx = blockIdx.x, lane = threadIdx.x & 31;
   const size_t stride = (size_t)n_rows * heads * (E + 2);
   const float* p0 = partial + (size_t)idx * (E + 2);
@@ -907,6 +918,7 @@ __global__ void __launch_bounds__(128) hyb_attn_merge_kernel(T* __restrict__ out
 // exp(-exp(A_log) * softplus(z + dt_bias)) and the raw write strength becomes sigmoid(z).
 __global__ void hyb_mem_gates_kernel(float* __restrict__ proj, long long ldp, int n_rows, int heads, int o_i, int o_f,
                                      const float* __restrict__ b_i, const float* __restrict__ b_f, float cap) {
+  hyb_pdl_enter();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= n_rows * heads) return;
   const int r = idx / heads, h = idx - r * heads;
@@ -916,6 +928,7 @@ __global__ void hyb_mem_gates_kernel(float* __restrict__ proj, long long ldp, in
 }
 __global__ void hyb_delta_gates_kernel(float* __restrict__ dt, float* __restrict__ proj, long long ldp, int n_rows, int heads, int D, int o_b,
                                        const float* __restrict__ a_log, const float* __restrict__ dt_bias) {
+  hyb_pdl_enter();
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (size_t)n_rows * heads * D) return;
   const int hd = (int)(idx % ((size_t)heads * D)), h = hd / D;
@@ -934,6 +947,7 @@ constexpr int SCAN_THREADS = 256;
 
 __global__ void __launch_bounds__(SCAN_THREADS) hyb_mem_scan_kernel(tha_mem_t m, tha_rows_t rows, tha_state_store_t st,
                                                                     const float* __restrict__ proj, long long ldp, float* __restrict__ o_raw, int SC) {
+  hyb_pdl_enter();
   extern __shared__ float sm[];
   const int s = blockIdx.x, h = blockIdx.y, e0 = blockIdx.z * SC;
   const int D = m.dim, E = m.vdim, nt = SCAN_THREADS;
@@ -1016,6 +1030,7 @@ template <int RPL>
 __global__ void __launch_bounds__(32 * SCAN_WARPS) hyb_mem_scan_warp_kernel(tha_mem_t m, tha_rows_t rows, tha_state_store_t st,
                                                                             const float* __restrict__ proj, long long ldp,
                                                                             float* __restrict__ o_raw) {
+  hyb_pdl_enter();
   const int s = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int D = m.dim, E = m.vdim;
   const int e0 = (blockIdx.z * SCAN_WARPS + warp) * SCW;
@@ -1112,6 +1127,7 @@ __global__ void __launch_bounds__(32 * SCAN_WARPS) hyb_delta_scan_warp_kernel(th
                                                                               const float* __restrict__ qkv, const float* __restrict__ proj,
                                                                               long long ldp, const float* __restrict__ dt_raw,
                                                                               float* __restrict__ o_raw) {
+  hyb_pdl_enter();
   const int s = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int D = dl.dim, E = dl.vdim;
   const int e0 = (blockIdx.z * SCAN_WARPS + warp) * SCW;
@@ -1198,6 +1214,7 @@ template <typename T>
 __global__ void hyb_head_gate_kernel(T* __restrict__ out, const float* __restrict__ o_raw, int n_rows, int heads, int E, float eps,
                                      const float* __restrict__ norm, int norm_per_head, const float* __restrict__ gate, long long ldg,
                                      int do_norm, int gate_act) {
+  hyb_pdl_enter();
   const int idx = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (idx >= n_rows * heads) return;
   const int r = idx / heads, h = idx - r * heads;
@@ -1227,6 +1244,7 @@ template <typename T, int V>
 __global__ void hyb_conv_kernel(tha_rows_t rows, tha_state_store_t st, long long conv_state_off, const float* __restrict__ proj,
                                 long long ldp, int col0, int channels, int taps, const float* __restrict__ w, const float* __restrict__ bias,
                                 int act, int add_input, T* __restrict__ out) {
+  hyb_pdl_enter();
   const int c = V * (blockIdx.x * blockDim.x + threadIdx.x);
   if (c >= channels) return;
   float wr[CONV_MAX_TAPS][V];
@@ -1282,6 +1300,7 @@ template <typename T>
 __global__ void hyb_conv_long_kernel(tha_rows_t rows, tha_state_store_t st, long long conv_state_off, const float* __restrict__ proj,
                                      long long ldp, int col0, int channels, int taps, const float* __restrict__ w,
                                      const float* __restrict__ bias, int act, int add_input, T* __restrict__ out) {
+  hyb_pdl_enter();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= channels) return;
   const float bv = bias ? bias[c] : 0.f;
@@ -1302,6 +1321,7 @@ __global__ void hyb_conv_long_kernel(tha_rows_t rows, tha_state_store_t st, long
 // after the convolution: tail[i] <- the input (taps-1-i) tokens before the end of what the sequence has seen now
 __global__ void hyb_conv_tail_kernel(tha_rows_t rows, tha_state_store_t st, long long conv_state_off, const float* __restrict__ proj,
                                      long long ldp, int col0, int channels, int taps, const float* __restrict__ bias) {
+  hyb_pdl_enter();
   const int c = blockIdx.x * blockDim.x + threadIdx.x, s = blockIdx.y;
   if (c >= channels) return;
   const float bv = bias ? bias[c] : 0.f;
@@ -1321,6 +1341,7 @@ __global__ void hyb_conv_tail_kernel(tha_rows_t rows, tha_state_store_t st, long
 __global__ void __launch_bounds__(SCAN_THREADS) hyb_delta_scan_kernel(tha_delta_t dl, tha_rows_t rows, tha_state_store_t st,
                                                                       const float* __restrict__ qkv, const float* __restrict__ proj, long long ldp,
                                                                       const float* __restrict__ dt_raw, float* __restrict__ o_raw, int SC) {
+  hyb_pdl_enter();
   extern __shared__ float sm[];
   const int s = blockIdx.x, h = blockIdx.y, e0 = blockIdx.z * SC;
   const int D = dl.dim, E = dl.vdim, nt = SCAN_THREADS;
@@ -1401,6 +1422,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) hyb_delta_scan_kernel(tha_delta_
 // ------------------------------------------------------------------------------------------------------------------
 __global__ void hyb_route_kernel(int experts, int top, int o_router, const float* __restrict__ proj, long long ldp, int n_rows,
                                  int* __restrict__ expert_id, float* __restrict__ weight, int* __restrict__ counts) {
+  hyb_pdl_enter();
   const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (r >= n_rows) return;
   const float* z = proj + (size_t)r * ldp + o_router;
@@ -1435,6 +1457,7 @@ template <bool SIGMOID>
 __global__ void hyb_route_groups_kernel(int experts, int top, int groups, int keep, int o_router, const float* __restrict__ correction,
                                         const float* __restrict__ proj, long long ldp, int n_rows, int* __restrict__ expert_id,
                                         float* __restrict__ weight, int* __restrict__ counts, float scale) {
+  hyb_pdl_enter();
   const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (r >= n_rows) return;
   const float* z = proj + (size_t)r * ldp + o_router;
@@ -1520,6 +1543,7 @@ __device__ __forceinline__ float hyb_act_value(int act, float g, float u, float 
 template <typename T>
 __global__ void hyb_ff_act_kernel(T* __restrict__ y, const float* __restrict__ gu, long long ldg, int col_g, int col_u, int n, int ff, int act,
                                   float limit, float alpha) {
+  hyb_pdl_enter();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (size_t)n * ff) return;
   const size_t r = i / ff; const int c = (int)(i - r * ff);
@@ -1530,6 +1554,7 @@ __global__ void hyb_ff_act_kernel(T* __restrict__ y, const float* __restrict__ g
 template <typename T>
 __global__ void hyb_ff_act_vec_kernel(T* __restrict__ y, const float* __restrict__ gu, long long ldg, int col_g, int col_u, int ff, int act,
                                       float limit, float alpha) {
+  hyb_pdl_enter();
   const int c = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
   if (c >= ff) return;
   const size_t r = blockIdx.y;
@@ -1549,6 +1574,7 @@ __global__ void hyb_ff_act_vec_kernel(T* __restrict__ y, const float* __restrict
 __global__ void __launch_bounds__(1024) hyb_route_sort_kernel(int experts, int top, int n_rows, const int* __restrict__ expert_id,
                                                               const int* __restrict__ counts, int* __restrict__ group_off,
                                                               int* __restrict__ sorted_row, int* __restrict__ inv) {
+  hyb_pdl_enter();
   __shared__ int wcount[32];
   __shared__ int s_start;
   const int e = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -1602,9 +1628,9 @@ extern "C" int tha_hyb_rmsnorm(void* stream, int dtype, void* out, const float* 
   if (n_rows < 1) return THA_STATUS_SUCCESS;
   const int nt = pick_threads(width / 4);
   if (dtype == THA_DT_BF16)
-    THA_CUDA_OK(launch(hyb_rmsnorm_kernel<bf16>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, false, (bf16*)out, x, w, w_offset, eps, width, rows_idx));
+    THA_CUDA_OK(launch(hyb_rmsnorm_kernel<bf16>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, pdl_enabled() != 0, (bf16*)out, x, w, w_offset, eps, width, rows_idx));
   else
-    THA_CUDA_OK(launch(hyb_rmsnorm_kernel<float>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, false, (float*)out, x, w, w_offset, eps, width, rows_idx));
+    THA_CUDA_OK(launch(hyb_rmsnorm_kernel<float>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, pdl_enabled() != 0, (float*)out, x, w, w_offset, eps, width, rows_idx));
   return THA_STATUS_SUCCESS;
 }
 
@@ -1616,18 +1642,18 @@ extern "C" int tha_hyb_norm(void* stream, int dtype, void* out, const float* x, 
     if (n_rows < 1) return THA_STATUS_SUCCESS;
     const int nt = pick_threads(width / 4);
     if (dtype == THA_DT_BF16)
-      THA_CUDA_OK(launch(hyb_layernorm_kernel<bf16>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, false, (bf16*)out, x, n->w, n->b, eps, width, rows_idx));
+      THA_CUDA_OK(launch(hyb_layernorm_kernel<bf16>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, pdl_enabled() != 0, (bf16*)out, x, n->w, n->b, eps, width, rows_idx));
     else
-      THA_CUDA_OK(launch(hyb_layernorm_kernel<float>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, false, (float*)out, x, n->w, n->b, eps, width, rows_idx));
+      THA_CUDA_OK(launch(hyb_layernorm_kernel<float>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, pdl_enabled() != 0, (float*)out, x, n->w, n->b, eps, width, rows_idx));
     return THA_STATUS_SUCCESS;
   }
   if (n->kind != THA_NORM_DYT || !n->w) return THA_STATUS_INVALID_ARG;
   if (n_rows < 1) return THA_STATUS_SUCCESS;
   const int nt = pick_threads(width);
   if (dtype == THA_DT_BF16)
-    THA_CUDA_OK(launch(hyb_dyt_kernel<bf16>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, false, (bf16*)out, x, n->w, n->b, n->alpha, width, rows_idx));
+    THA_CUDA_OK(launch(hyb_dyt_kernel<bf16>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, pdl_enabled() != 0, (bf16*)out, x, n->w, n->b, n->alpha, width, rows_idx));
   else
-    THA_CUDA_OK(launch(hyb_dyt_kernel<float>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, false, (float*)out, x, n->w, n->b, n->alpha, width, rows_idx));
+    THA_CUDA_OK(launch(hyb_dyt_kernel<float>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, pdl_enabled() != 0, (float*)out, x, n->w, n->b, n->alpha, width, rows_idx));
   return THA_STATUS_SUCCESS;
 }
 
@@ -1637,9 +1663,9 @@ extern "C" int tha_hyb_norm_pair(void* stream, int dtype, void* out1, void* out2
     if (n_rows < 1) return THA_STATUS_SUCCESS;
     const int nt = pick_threads(width);
     if (dtype == THA_DT_BF16)
-      THA_CUDA_OK(launch(hyb_dyt2_kernel<bf16>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, false, (bf16*)out1, (bf16*)out2, x, *n1, *n2, width));
+      THA_CUDA_OK(launch(hyb_dyt2_kernel<bf16>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, pdl_enabled() != 0, (bf16*)out1, (bf16*)out2, x, *n1, *n2, width));
     else
-      THA_CUDA_OK(launch(hyb_dyt2_kernel<float>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, false, (float*)out1, (float*)out2, x, *n1, *n2, width));
+      THA_CUDA_OK(launch(hyb_dyt2_kernel<float>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, pdl_enabled() != 0, (float*)out1, (float*)out2, x, *n1, *n2, width));
     return THA_STATUS_SUCCESS;
   }
   const int st = tha_hyb_norm(stream, dtype, out1, x, n1, eps, n_rows, width, nullptr);
@@ -1654,18 +1680,18 @@ extern "C" int tha_hyb_linear_heads(void* stream, int dtype, float* C, long long
   const dim3 grid(ceil_div(N, LT), ceil_div(M, LT), heads), block(256);
   const int* none = nullptr;
   if (dtype == THA_DT_BF16 && !a_f32 && hyb_tc_linear() && K % 8 == 0 && lda % 8 == 0 && a_hs % 8 == 0 && w_hs % 8 == 0 && aligned16(A) && aligned16(W)) {
-    THA_CUDA_OK(launch(hyb_linear_mma_kernel, grid, dim3(128), 0, s, false, C, ldc, (const bf16*)A, lda, none, (const bf16*)W, 0ll, M, N, K, none, 0,
+    THA_CUDA_OK(launch(hyb_linear_mma_kernel, grid, dim3(128), 0, s, pdl_enabled() != 0, C, ldc, (const bf16*)A, lda, none, (const bf16*)W, 0ll, M, N, K, none, 0,
                        a_hs, w_hs, c_hs));
     return THA_STATUS_SUCCESS;
   }
   if (dtype == THA_DT_F32)
-    THA_CUDA_OK(launch(hyb_linear_kernel<float, float>, grid, block, 0, s, false, C, ldc, (const float*)A, lda, none, (const float*)W, 0ll, M, N, K,
+    THA_CUDA_OK(launch(hyb_linear_kernel<float, float>, grid, block, 0, s, pdl_enabled() != 0, C, ldc, (const float*)A, lda, none, (const float*)W, 0ll, M, N, K,
                        none, 0, a_hs, w_hs, c_hs));
   else if (a_f32)
-    THA_CUDA_OK(launch(hyb_linear_kernel<float, bf16>, grid, block, 0, s, false, C, ldc, (const float*)A, lda, none, (const bf16*)W, 0ll, M, N, K,
+    THA_CUDA_OK(launch(hyb_linear_kernel<float, bf16>, grid, block, 0, s, pdl_enabled() != 0, C, ldc, (const float*)A, lda, none, (const bf16*)W, 0ll, M, N, K,
                        none, 0, a_hs, w_hs, c_hs));
   else
-    THA_CUDA_OK(launch(hyb_linear_kernel<bf16, bf16>, grid, block, 0, s, false, C, ldc, (const bf16*)A, lda, none, (const bf16*)W, 0ll, M, N, K,
+    THA_CUDA_OK(launch(hyb_linear_kernel<bf16, bf16>, grid, block, 0, s, pdl_enabled() != 0, C, ldc, (const bf16*)A, lda, none, (const bf16*)W, 0ll, M, N, K,
                        none, 0, a_hs, w_hs, c_hs));
   return THA_STATUS_SUCCESS;
 }
@@ -1675,10 +1701,10 @@ extern "C" int tha_hyb_head_gate(void* stream, int dtype, void* out, const float
   if (n_rows < 1) return THA_STATUS_SUCCESS;
   const dim3 grid(ceil_div(n_rows * heads, 4));
   if (dtype == THA_DT_BF16)
-    THA_CUDA_OK(launch(hyb_head_gate_kernel<bf16>, grid, dim3(128), 0, (cudaStream_t)stream, false, (bf16*)out, o_raw, n_rows, heads, E, eps, norm,
+    THA_CUDA_OK(launch(hyb_head_gate_kernel<bf16>, grid, dim3(128), 0, (cudaStream_t)stream, pdl_enabled() != 0, (bf16*)out, o_raw, n_rows, heads, E, eps, norm,
                        norm_per_head, gate, ldg, do_norm, gate_act));
   else
-    THA_CUDA_OK(launch(hyb_head_gate_kernel<float>, grid, dim3(128), 0, (cudaStream_t)stream, false, (float*)out, o_raw, n_rows, heads, E, eps, norm,
+    THA_CUDA_OK(launch(hyb_head_gate_kernel<float>, grid, dim3(128), 0, (cudaStream_t)stream, pdl_enabled() != 0, (float*)out, o_raw, n_rows, heads, E, eps, norm,
                        norm_per_head, gate, ldg, do_norm, gate_act));
   return THA_STATUS_SUCCESS;
 }
@@ -1696,23 +1722,23 @@ extern "C" int tha_hyb_linear(void* stream, int dtype, float* C, long long ldc, 
     b.n_mats = 1; b.W[0] = (const uint16_t*)W; b.M[0] = N; b.out_off[0] = 0; b.K = K;
     b.X = (const uint16_t*)A; b.N = M; b.ldx = lda;
     b.out = C; b.ldo = ldc; b.zstride = 0; b.splits = 1; b.colscale = nullptr;
-    if (hyb_tc_linear() && gemm_bf16_ok(b)) return gemm_bf16_launch(s, b, false);
+    if (hyb_tc_linear() && gemm_bf16_ok(b)) return gemm_bf16_launch(s, b, hyb_gemm_pdl());
   }
   const int mt = ceil_div(M, LT) + (group_off ? n_groups : 0);
   const dim3 grid(ceil_div(N, LT), mt), block(256);
   if (dtype == THA_DT_BF16 && !a_f32 && hyb_tc_linear() && K % 8 == 0 && lda % 8 == 0 && w_group_stride % 8 == 0 && aligned16(A) && aligned16(W)) {
-    THA_CUDA_OK(launch(hyb_linear_mma_kernel, grid, dim3(128), 0, s, false, C, ldc, (const bf16*)A, lda, a_rows, (const bf16*)W, w_group_stride,
+    THA_CUDA_OK(launch(hyb_linear_mma_kernel, grid, dim3(128), 0, s, pdl_enabled() != 0, C, ldc, (const bf16*)A, lda, a_rows, (const bf16*)W, w_group_stride,
                        M, N, K, group_off, n_groups, 0ll, 0ll, 0ll));
     return THA_STATUS_SUCCESS;
   }
   if (dtype == THA_DT_F32)
-    THA_CUDA_OK(launch(hyb_linear_kernel<float, float>, grid, block, 0, s, false, C, ldc, (const float*)A, lda, a_rows, (const float*)W,
+    THA_CUDA_OK(launch(hyb_linear_kernel<float, float>, grid, block, 0, s, pdl_enabled() != 0, C, ldc, (const float*)A, lda, a_rows, (const float*)W,
                        w_group_stride, M, N, K, group_off, n_groups, 0ll, 0ll, 0ll));
   else if (a_f32)
-    THA_CUDA_OK(launch(hyb_linear_kernel<float, bf16>, grid, block, 0, s, false, C, ldc, (const float*)A, lda, a_rows, (const bf16*)W,
+    THA_CUDA_OK(launch(hyb_linear_kernel<float, bf16>, grid, block, 0, s, pdl_enabled() != 0, C, ldc, (const float*)A, lda, a_rows, (const bf16*)W,
                        w_group_stride, M, N, K, group_off, n_groups, 0ll, 0ll, 0ll));
   else
-    THA_CUDA_OK(launch(hyb_linear_kernel<bf16, bf16>, grid, block, 0, s, false, C, ldc, (const bf16*)A, lda, a_rows, (const bf16*)W,
+    THA_CUDA_OK(launch(hyb_linear_kernel<bf16, bf16>, grid, block, 0, s, pdl_enabled() != 0, C, ldc, (const bf16*)A, lda, a_rows, (const bf16*)W,
                        w_group_stride, M, N, K, group_off, n_groups, 0ll, 0ll, 0ll));
   return THA_STATUS_SUCCESS;
 }
@@ -1730,7 +1756,7 @@ extern "C" int tha_hyb_linear_groups(void* stream, int dtype, float* C, long lon
     for (int g = 0, at = 0; g < n_groups; at += group_n_host[g], g++) {
       b.M[g] = group_n_host[g]; b.out_off[g] = at; b.w_row[g] = at; b.x_row[g] = g * M;
     }
-    if (gemm_bf16_ok(b)) return gemm_bf16_launch((cudaStream_t)stream, b, false);
+    if (gemm_bf16_ok(b)) return gemm_bf16_launch((cudaStream_t)stream, b, hyb_gemm_pdl());
   }
   const size_t es = dtype == THA_DT_BF16 ? 2 : 4;
   for (int g = 0, at = 0; g < n_groups; at += group_n_host[g], g++) {
@@ -1744,7 +1770,7 @@ extern "C" int tha_hyb_linear_groups(void* stream, int dtype, float* C, long lon
 extern "C" int tha_hyb_rotary_table(void* stream, const tha_rotary_t* rot, const int* pos, int n_rows, float* cos_out, float* sin_out) {
   const int half = rot->dims / 2;
   if (n_rows < 1 || half < 1) return THA_STATUS_SUCCESS;
-  THA_CUDA_OK(launch(hyb_rotary_kernel, dim3(ceil_div(n_rows * half, 128)), dim3(128), 0, (cudaStream_t)stream, false, rot->inv_freq, half,
+  THA_CUDA_OK(launch(hyb_rotary_kernel, dim3(ceil_div(n_rows * half, 128)), dim3(128), 0, (cudaStream_t)stream, pdl_enabled() != 0, rot->inv_freq, half,
                      rot->mag, pos, n_rows, cos_out, sin_out));
   return THA_STATUS_SUCCESS;
 }
@@ -1756,7 +1782,7 @@ extern "C" int tha_hyb_attn_prepare(void* stream, const tha_attn_t* a, const tha
       a->kv_heads / (a->v_share > 1 ? a->v_share : 1) * a->vdim > kv->kv_dim || (a->v_is_k && a->vdim != a->dim))
     return THA_STATUS_INVALID_ARG;
   const int nt = pick_threads(32 * (a->heads + 2 * a->kv_heads));
-  THA_CUDA_OK(launch(hyb_attn_prepare_kernel, dim3(rows->n_rows), dim3(nt), 0, (cudaStream_t)stream, false, *a, *rows, *kv, proj, ldp, cos_t,
+  THA_CUDA_OK(launch(hyb_attn_prepare_kernel, dim3(rows->n_rows), dim3(nt), 0, (cudaStream_t)stream, pdl_enabled() != 0, *a, *rows, *kv, proj, ldp, cos_t,
                      sin_t, rot_dims, q_out));
   return THA_STATUS_SUCCESS;
 }
@@ -1831,10 +1857,10 @@ extern "C" int tha_hyb_attn_gated(void* stream, int dtype, const tha_attn_t* a, 
     if (st != THA_STATUS_SUCCESS || splits <= 1) return st;
     const dim3 mgrid(rows->n_rows * a->heads);
     if (dtype != THA_DT_BF16 || a->out_f32)
-      THA_CUDA_OK(launch(hyb_attn_merge_kernel<float>, mgrid, dim3(128), 0, s, false, (float*)out, (const float*)split_scratch, rows->n_rows, a->heads, a->vdim,
+      THA_CUDA_OK(launch(hyb_attn_merge_kernel<float>, mgrid, dim3(128), 0, s, pdl_enabled() != 0, (float*)out, (const float*)split_scratch, rows->n_rows, a->heads, a->vdim,
                          splits, *a, gate, ldg));
     else
-      THA_CUDA_OK(launch(hyb_attn_merge_kernel<bf16>, mgrid, dim3(128), 0, s, false, (bf16*)out, (const float*)split_scratch, rows->n_rows, a->heads, a->vdim,
+      THA_CUDA_OK(launch(hyb_attn_merge_kernel<bf16>, mgrid, dim3(128), 0, s, pdl_enabled() != 0, (bf16*)out, (const float*)split_scratch, rows->n_rows, a->heads, a->vdim,
                          splits, *a, gate, ldg));
     return THA_STATUS_SUCCESS;
   }
@@ -1854,32 +1880,32 @@ extern "C" int tha_hyb_attn_gated(void* stream, int dtype, const tha_attn_t* a, 
     } else if (tc) {
       const int dt = a->dim == a->vdim && (a->dim == 64 || a->dim == 128) ? a->dim : 0;
       auto k = a->rel ? mma_of<true, false, true>(dt) : a->softcap > 0.f ? mma_of<true, true, false>(dt) : a->fp32_scores ? mma_of<true, false, false>(dt) : mma_of<false, false, false>(dt);
-      THA_CUDA_OK(launch_smem(k, grid, dim3(AM_THREADS), smem, s, false, *a, *rows, *kv, q, (bf16*)out, AG, AP, splits, split_scratch, gate, ldg));
+      THA_CUDA_OK(launch_smem(k, grid, dim3(AM_THREADS), smem, s, pdl_enabled() != 0, *a, *rows, *kv, q, (bf16*)out, AG, AP, splits, split_scratch, gate, ldg));
     } else {
       if (a->vdim <= 256) {
         if (smem > 48 * 1024) THA_CUDA_OK(cudaFuncSetAttribute(hyb_attn_kernel<bf16, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        THA_CUDA_OK(launch(hyb_attn_kernel<bf16, 8>, grid, dim3(128), smem, s, false, *a, *rows, *kv, q, (bf16*)out, AG, AP, splits, split_scratch, gate, ldg));
+        THA_CUDA_OK(launch(hyb_attn_kernel<bf16, 8>, grid, dim3(128), smem, s, pdl_enabled() != 0, *a, *rows, *kv, q, (bf16*)out, AG, AP, splits, split_scratch, gate, ldg));
       } else {
         if (smem > 48 * 1024) THA_CUDA_OK(cudaFuncSetAttribute(hyb_attn_kernel<bf16, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        THA_CUDA_OK(launch(hyb_attn_kernel<bf16, 16>, grid, dim3(128), smem, s, false, *a, *rows, *kv, q, (bf16*)out, AG, AP, splits, split_scratch, gate, ldg));
+        THA_CUDA_OK(launch(hyb_attn_kernel<bf16, 16>, grid, dim3(128), smem, s, pdl_enabled() != 0, *a, *rows, *kv, q, (bf16*)out, AG, AP, splits, split_scratch, gate, ldg));
       }
     }
     if (splits > 1 && a->out_f32)
-      THA_CUDA_OK(launch(hyb_attn_merge_kernel<float>, dim3(rows->n_rows * a->heads), dim3(128), 0, s, false, (float*)out,
+      THA_CUDA_OK(launch(hyb_attn_merge_kernel<float>, dim3(rows->n_rows * a->heads), dim3(128), 0, s, pdl_enabled() != 0, (float*)out,
                          (const float*)split_scratch, rows->n_rows, a->heads, a->vdim, splits, *a, gate, ldg));
     else if (splits > 1)
-      THA_CUDA_OK(launch(hyb_attn_merge_kernel<bf16>, dim3(rows->n_rows * a->heads), dim3(128), 0, s, false, (bf16*)out,
+      THA_CUDA_OK(launch(hyb_attn_merge_kernel<bf16>, dim3(rows->n_rows * a->heads), dim3(128), 0, s, pdl_enabled() != 0, (bf16*)out,
                          (const float*)split_scratch, rows->n_rows, a->heads, a->vdim, splits, *a, gate, ldg));
   } else {
     if (a->vdim <= 256) {
       if (smem > 48 * 1024) THA_CUDA_OK(cudaFuncSetAttribute(hyb_attn_kernel<float, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      THA_CUDA_OK(launch(hyb_attn_kernel<float, 8>, grid, dim3(128), smem, s, false, *a, *rows, *kv, q, (float*)out, AG, AP, splits, split_scratch, gate, ldg));
+      THA_CUDA_OK(launch(hyb_attn_kernel<float, 8>, grid, dim3(128), smem, s, pdl_enabled() != 0, *a, *rows, *kv, q, (float*)out, AG, AP, splits, split_scratch, gate, ldg));
     } else {
       if (smem > 48 * 1024) THA_CUDA_OK(cudaFuncSetAttribute(hyb_attn_kernel<float, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      THA_CUDA_OK(launch(hyb_attn_kernel<float, 16>, grid, dim3(128), smem, s, false, *a, *rows, *kv, q, (float*)out, AG, AP, splits, split_scratch, gate, ldg));
+      THA_CUDA_OK(launch(hyb_attn_kernel<float, 16>, grid, dim3(128), smem, s, pdl_enabled() != 0, *a, *rows, *kv, q, (float*)out, AG, AP, splits, split_scratch, gate, ldg));
     }
     if (splits > 1)
-      THA_CUDA_OK(launch(hyb_attn_merge_kernel<float>, dim3(rows->n_rows * a->heads), dim3(128), 0, s, false, (float*)out,
+      THA_CUDA_OK(launch(hyb_attn_merge_kernel<float>, dim3(rows->n_rows * a->heads), dim3(128), 0, s, pdl_enabled() != 0, (float*)out,
                          (const float*)split_scratch, rows->n_rows, a->heads, a->vdim, splits, *a, gate, ldg));
   }
   return THA_STATUS_SUCCESS;
@@ -1896,7 +1922,7 @@ static int scan_slice(int vdim) { int sc = 1; while (sc < vdim && sc < 16) sc <<
 template <typename T>
 static int head_gate_launch(cudaStream_t s, T* out, const float* o_raw, int n_rows, int heads, int E, float eps, const float* norm,
                             int norm_per_head, const float* gate, long long ldg) {
-  THA_CUDA_OK(launch(hyb_head_gate_kernel<T>, dim3(ceil_div(n_rows * heads, 4)), dim3(128), 0, s, false, out, o_raw, n_rows, heads, E, eps, norm,
+  THA_CUDA_OK(launch(hyb_head_gate_kernel<T>, dim3(ceil_div(n_rows * heads, 4)), dim3(128), 0, s, pdl_enabled() != 0, out, o_raw, n_rows, heads, E, eps, norm,
                      norm_per_head, gate, ldg, 1, (int)THA_GATE_SIGMOID));
   return THA_STATUS_SUCCESS;
 }
@@ -1905,21 +1931,21 @@ extern "C" int tha_hyb_mem_scan(void* stream, int dtype, const tha_mem_t* m, con
                                 float* proj, long long ldp, float* o_raw, void* out) {
   if (rows->n_seqs < 1) return THA_STATUS_SUCCESS;
   cudaStream_t s = (cudaStream_t)stream;
-  THA_CUDA_OK(launch(hyb_mem_gates_kernel, dim3(ceil_div(rows->n_rows * m->heads, 128)), dim3(128), 0, s, false, proj, ldp, rows->n_rows, m->heads,
+  THA_CUDA_OK(launch(hyb_mem_gates_kernel, dim3(ceil_div(rows->n_rows * m->heads, 128)), dim3(128), 0, s, pdl_enabled() != 0, proj, ldp, rows->n_rows, m->heads,
                      m->o_i, m->o_f, m->b_i, m->b_f, m->gate_cap));
   if (m->dim <= 256 && scan_in_registers()) {
     const dim3 grid(rows->n_seqs, m->heads, ceil_div(m->vdim, SCW * SCAN_WARPS)), block(32 * SCAN_WARPS);
-    if (m->dim <= 32) THA_CUDA_OK(launch(hyb_mem_scan_warp_kernel<1>, grid, block, 0, s, false, *m, *rows, *st, proj, ldp, o_raw));
-    else if (m->dim <= 64) THA_CUDA_OK(launch(hyb_mem_scan_warp_kernel<2>, grid, block, 0, s, false, *m, *rows, *st, proj, ldp, o_raw));
-    else if (m->dim <= 128) THA_CUDA_OK(launch(hyb_mem_scan_warp_kernel<4>, grid, block, 0, s, false, *m, *rows, *st, proj, ldp, o_raw));
-    else THA_CUDA_OK(launch(hyb_mem_scan_warp_kernel<8>, grid, block, 0, s, false, *m, *rows, *st, proj, ldp, o_raw));
+    if (m->dim <= 32) THA_CUDA_OK(launch(hyb_mem_scan_warp_kernel<1>, grid, block, 0, s, pdl_enabled() != 0, *m, *rows, *st, proj, ldp, o_raw));
+    else if (m->dim <= 64) THA_CUDA_OK(launch(hyb_mem_scan_warp_kernel<2>, grid, block, 0, s, pdl_enabled() != 0, *m, *rows, *st, proj, ldp, o_raw));
+    else if (m->dim <= 128) THA_CUDA_OK(launch(hyb_mem_scan_warp_kernel<4>, grid, block, 0, s, pdl_enabled() != 0, *m, *rows, *st, proj, ldp, o_raw));
+    else THA_CUDA_OK(launch(hyb_mem_scan_warp_kernel<8>, grid, block, 0, s, pdl_enabled() != 0, *m, *rows, *st, proj, ldp, o_raw));
   } else {
     const int SC = scan_slice(m->vdim), parts = SCAN_THREADS / SC;
     const size_t smem = sizeof(float) * ((size_t)m->dim * SC + m->dim + 2 * (2 * (size_t)m->dim + SC + 2) + (size_t)parts * SC);
     if (smem > 227 * 1024) return THA_STATUS_NOT_SUPPORTED;
     const dim3 grid(rows->n_seqs, m->heads, ceil_div(m->vdim, SC));
     if (smem > 48 * 1024) THA_CUDA_OK(cudaFuncSetAttribute(hyb_mem_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    THA_CUDA_OK(launch(hyb_mem_scan_kernel, grid, dim3(SCAN_THREADS), smem, s, false, *m, *rows, *st, proj, ldp, o_raw, SC));
+    THA_CUDA_OK(launch(hyb_mem_scan_kernel, grid, dim3(SCAN_THREADS), smem, s, pdl_enabled() != 0, *m, *rows, *st, proj, ldp, o_raw, SC));
   }
   const float* gate = proj + m->o_g;
   if (dtype == THA_DT_BF16) return head_gate_launch(s, (bf16*)out, o_raw, rows->n_rows, m->heads, m->vdim, m->eps, m->norm, 1, gate, ldp);
@@ -1939,9 +1965,9 @@ extern "C" int tha_hyb_conv(void* stream, int dtype, const tha_rows_t* rows, con
     /* about eight blocks per SM: a block walks several rows with its taps in registers */                                               \
     const int gy = min(rows->n_rows, max(1, 148 * 8 / gx));                                                                               \
     const dim3 grid(gx, gy);                                                                                                              \
-    if (f32) THA_CUDA_OK(launch(KF, grid, dim3(128), 0, s, false, *rows, *st, conv_state_off, proj, ldp, col0, channels, taps, w, bias, act, add_input, \
+    if (f32) THA_CUDA_OK(launch(KF, grid, dim3(128), 0, s, pdl_enabled() != 0, *rows, *st, conv_state_off, proj, ldp, col0, channels, taps, w, bias, act, add_input, \
                                 (float*)out));                                                                                            \
-    else THA_CUDA_OK(launch(KB, grid, dim3(128), 0, s, false, *rows, *st, conv_state_off, proj, ldp, col0, channels, taps, w, bias, act, add_input,     \
+    else THA_CUDA_OK(launch(KB, grid, dim3(128), 0, s, pdl_enabled() != 0, *rows, *st, conv_state_off, proj, ldp, col0, channels, taps, w, bias, act, add_input,     \
                             (bf16*)out));                                                                                                 \
   } while (0)
   if (taps > CONV_MAX_TAPS) CONV_GO(hyb_conv_long_kernel<float>, hyb_conv_long_kernel<bf16>, 1);
@@ -1954,7 +1980,7 @@ extern "C" int tha_hyb_conv(void* stream, int dtype, const tha_rows_t* rows, con
 extern "C" int tha_hyb_conv_tail(void* stream, const tha_rows_t* rows, const tha_state_store_t* st, long long conv_state_off,
                                  const float* proj, long long ldp, int col0, int channels, int taps, const float* bias) {
   if (rows->n_rows < 1 || channels < 1 || taps <= 1) return THA_STATUS_SUCCESS;
-  THA_CUDA_OK(launch(hyb_conv_tail_kernel, dim3(ceil_div(channels, 128), rows->n_seqs), dim3(128), 0, (cudaStream_t)stream, false, *rows, *st,
+  THA_CUDA_OK(launch(hyb_conv_tail_kernel, dim3(ceil_div(channels, 128), rows->n_seqs), dim3(128), 0, (cudaStream_t)stream, pdl_enabled() != 0, *rows, *st,
                      conv_state_off, proj, ldp, col0, channels, taps, bias));
   return THA_STATUS_SUCCESS;
 }
@@ -1973,22 +1999,22 @@ extern "C" int tha_hyb_delta_scan(void* stream, int dtype, const tha_delta_t* d,
   cudaStream_t s = (cudaStream_t)stream;
   {
     const size_t n = (size_t)rows->n_rows * d->heads * d->dim;
-    THA_CUDA_OK(launch(hyb_delta_gates_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, s, false, dt_raw, proj, ldp, rows->n_rows, d->heads,
+    THA_CUDA_OK(launch(hyb_delta_gates_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, s, pdl_enabled() != 0, dt_raw, proj, ldp, rows->n_rows, d->heads,
                        d->dim, d->o_b, d->a_log, d->dt_bias));
   }
   if (d->dim <= 256 && scan_in_registers()) {
     const dim3 grid(rows->n_seqs, d->heads, ceil_div(d->vdim, SCW * SCAN_WARPS)), block(32 * SCAN_WARPS);
-    if (d->dim <= 32) THA_CUDA_OK(launch(hyb_delta_scan_warp_kernel<1>, grid, block, 0, s, false, *d, *rows, *st, qkv, proj, ldp, dt_raw, o_raw));
-    else if (d->dim <= 64) THA_CUDA_OK(launch(hyb_delta_scan_warp_kernel<2>, grid, block, 0, s, false, *d, *rows, *st, qkv, proj, ldp, dt_raw, o_raw));
-    else if (d->dim <= 128) THA_CUDA_OK(launch(hyb_delta_scan_warp_kernel<4>, grid, block, 0, s, false, *d, *rows, *st, qkv, proj, ldp, dt_raw, o_raw));
-    else THA_CUDA_OK(launch(hyb_delta_scan_warp_kernel<8>, grid, block, 0, s, false, *d, *rows, *st, qkv, proj, ldp, dt_raw, o_raw));
+    if (d->dim <= 32) THA_CUDA_OK(launch(hyb_delta_scan_warp_kernel<1>, grid, block, 0, s, pdl_enabled() != 0, *d, *rows, *st, qkv, proj, ldp, dt_raw, o_raw));
+    else if (d->dim <= 64) THA_CUDA_OK(launch(hyb_delta_scan_warp_kernel<2>, grid, block, 0, s, pdl_enabled() != 0, *d, *rows, *st, qkv, proj, ldp, dt_raw, o_raw));
+    else if (d->dim <= 128) THA_CUDA_OK(launch(hyb_delta_scan_warp_kernel<4>, grid, block, 0, s, pdl_enabled() != 0, *d, *rows, *st, qkv, proj, ldp, dt_raw, o_raw));
+    else THA_CUDA_OK(launch(hyb_delta_scan_warp_kernel<8>, grid, block, 0, s, pdl_enabled() != 0, *d, *rows, *st, qkv, proj, ldp, dt_raw, o_raw));
   } else {
     const int SC = scan_slice(d->vdim), parts = SCAN_THREADS / SC;
     const size_t smem = sizeof(float) * ((size_t)d->dim * SC + 2 * (3 * (size_t)d->dim + SC + 1) + (size_t)parts * SC + SC);
     if (smem > 227 * 1024) return THA_STATUS_NOT_SUPPORTED;
     const dim3 grid(rows->n_seqs, d->heads, ceil_div(d->vdim, SC));
     if (smem > 48 * 1024) THA_CUDA_OK(cudaFuncSetAttribute(hyb_delta_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    THA_CUDA_OK(launch(hyb_delta_scan_kernel, grid, dim3(SCAN_THREADS), smem, s, false, *d, *rows, *st, qkv, proj, ldp, dt_raw, o_raw, SC));
+    THA_CUDA_OK(launch(hyb_delta_scan_kernel, grid, dim3(SCAN_THREADS), smem, s, pdl_enabled() != 0, *d, *rows, *st, qkv, proj, ldp, dt_raw, o_raw, SC));
   }
   const long long ldg = (long long)d->heads * d->vdim;
   if (dtype == THA_DT_BF16) return head_gate_launch(s, (bf16*)out, o_raw, rows->n_rows, d->heads, d->vdim, d->eps, d->norm, 0, gate_raw, ldg);
@@ -2006,16 +2032,16 @@ extern "C" int tha_hyb_moe_route(void* stream, const tha_moe_t* e, const float* 
     const int groups = e->groups > 1 ? e->groups : 1;
     if (e->experts % groups || e->experts > 4096 || e->keep_groups < 1) return THA_STATUS_INVALID_ARG;
     auto kernel = e->route == THA_ROUTE_SIGMOID_GROUPS ? hyb_route_groups_kernel<true> : hyb_route_groups_kernel<false>;
-    THA_CUDA_OK(launch(kernel, dim3(ceil_div(n_rows, 4)), dim3(128), 0, s, false, e->experts, e->top, groups,
+    THA_CUDA_OK(launch(kernel, dim3(ceil_div(n_rows, 4)), dim3(128), 0, s, pdl_enabled() != 0, e->experts, e->top, groups,
                        e->keep_groups < groups ? e->keep_groups : groups, e->o_router, e->correction, proj, ldp, n_rows, expert_id, weight, counts,
                        e->weight_scale));
   } else {
-    THA_CUDA_OK(launch(hyb_route_kernel, dim3(ceil_div(n_rows, 4)), dim3(128), 0, s, false, e->experts, e->top, e->o_router, proj, ldp, n_rows,
+    THA_CUDA_OK(launch(hyb_route_kernel, dim3(ceil_div(n_rows, 4)), dim3(128), 0, s, pdl_enabled() != 0, e->experts, e->top, e->o_router, proj, ldp, n_rows,
                        expert_id, weight, counts));
   }
   int nt = 64;
   while (nt < 1024 && nt < n_rows * e->top) nt *= 2;
-  THA_CUDA_OK(launch(hyb_route_sort_kernel, dim3(e->experts), dim3(nt), 0, s, false, e->experts, e->top, n_rows, (const int*)expert_id,
+  THA_CUDA_OK(launch(hyb_route_sort_kernel, dim3(e->experts), dim3(nt), 0, s, pdl_enabled() != 0, e->experts, e->top, n_rows, (const int*)expert_id,
                      (const int*)counts, group_off, sorted_row, inv));
   return THA_STATUS_SUCCESS;
 }
@@ -2033,16 +2059,16 @@ extern "C" int tha_hyb_ff_act(void* stream, int dtype, int act, void* y, const f
   if (ff % 4 == 0 && ldg % 4 == 0 && col_u % 4 == 0 && (!gated || col_g % 4 == 0) && aligned16(gu) && n <= 65535) {
     const dim3 grid(ceil_div(ff / 4, 128), n);
     if (dtype == THA_DT_BF16)
-      THA_CUDA_OK(launch(hyb_ff_act_vec_kernel<bf16>, grid, dim3(128), 0, s, false, (bf16*)y, gu, ldg, col_g, col_u, ff, act, limit, alpha));
+      THA_CUDA_OK(launch(hyb_ff_act_vec_kernel<bf16>, grid, dim3(128), 0, s, pdl_enabled() != 0, (bf16*)y, gu, ldg, col_g, col_u, ff, act, limit, alpha));
     else
-      THA_CUDA_OK(launch(hyb_ff_act_vec_kernel<float>, grid, dim3(128), 0, s, false, (float*)y, gu, ldg, col_g, col_u, ff, act, limit, alpha));
+      THA_CUDA_OK(launch(hyb_ff_act_vec_kernel<float>, grid, dim3(128), 0, s, pdl_enabled() != 0, (float*)y, gu, ldg, col_g, col_u, ff, act, limit, alpha));
     return THA_STATUS_SUCCESS;
   }
   const dim3 grid((unsigned)(((size_t)n * ff + 255) / 256));
   if (dtype == THA_DT_BF16)
-    THA_CUDA_OK(launch(hyb_ff_act_kernel<bf16>, grid, dim3(256), 0, s, false, (bf16*)y, gu, ldg, col_g, col_u, n, ff, act, limit, alpha));
+    THA_CUDA_OK(launch(hyb_ff_act_kernel<bf16>, grid, dim3(256), 0, s, pdl_enabled() != 0, (bf16*)y, gu, ldg, col_g, col_u, n, ff, act, limit, alpha));
   else
-    THA_CUDA_OK(launch(hyb_ff_act_kernel<float>, grid, dim3(256), 0, s, false, (float*)y, gu, ldg, col_g, col_u, n, ff, act, limit, alpha));
+    THA_CUDA_OK(launch(hyb_ff_act_kernel<float>, grid, dim3(256), 0, s, pdl_enabled() != 0, (float*)y, gu, ldg, col_g, col_u, n, ff, act, limit, alpha));
   return THA_STATUS_SUCCESS;
 }
 

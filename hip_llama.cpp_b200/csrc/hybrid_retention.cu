@@ -13,6 +13,7 @@ namespace tha {
 // a block per row; work item = one pair of rotated channels, or one channel that passes unchanged, of one head of q or k
 __global__ void hyb_rotate_qk_kernel(float* __restrict__ proj, long long ldp, int o_q, int o_k, int heads, int dim, int rot_dims, int layout,
                                      const float* __restrict__ cos_t, const float* __restrict__ sin_t, float k_scale) {
+  hyb_pdl_enter();
   const int r = blockIdx.x, half = rot_dims >> 1, per = half + (dim - rot_dims);
   float* row = proj + (size_t)r * ldp;
   const float* c = cos_t + (size_t)r * half;
@@ -44,7 +45,7 @@ extern "C" int tha_hyb_retention_scan(void* stream, int dtype, const tha_retenti
   if (g->heads < 1 || g->dim < 1 || g->vdim < 1 || rot_dims > g->dim || (rot_dims & 1)) return THA_STATUS_INVALID_ARG;
   if (g->dim > 512) return THA_STATUS_NOT_SUPPORTED;
   cudaStream_t s = (cudaStream_t)stream;
-  THA_CUDA_OK(launch(hyb_rotate_qk_kernel, dim3(rows->n_rows), dim3(256), 0, s, false, proj, ldp, g->o_q, g->o_k, g->heads, g->dim, rot_dims,
+  THA_CUDA_OK(launch(hyb_rotate_qk_kernel, dim3(rows->n_rows), dim3(256), 0, s, pdl_enabled() != 0, proj, ldp, g->o_q, g->o_k, g->heads, g->dim, rot_dims,
                      g->rot_layout, cos_t, sin_t, 1.0f / sqrtf((float)g->dim)));
   tha_gla_t a = {};
   a.heads = g->heads; a.dim = g->dim; a.vdim = g->vdim; a.o_q = g->o_q; a.o_k = g->o_k; a.o_v = g->o_v; a.state_off = g->state_off;

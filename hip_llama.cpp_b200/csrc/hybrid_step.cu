@@ -21,6 +21,7 @@ template <typename T>
 __global__ void hyb_embed_kernel(float* __restrict__ x, const T* __restrict__ embed, const int* __restrict__ token, int width,
                                  const T* __restrict__ pos_embed, const int* __restrict__ pos, float scale, float* __restrict__ x0,
                                  T* __restrict__ copy, T* __restrict__ join) {
+  hyb_pdl_enter();
   const int r = blockIdx.x;
   const T* e = embed + (size_t)token[r] * width;
   const T* p = pos_embed ? pos_embed + (size_t)pos[r] * width : nullptr;
@@ -42,6 +43,7 @@ __global__ void hyb_finish_kernel(float* __restrict__ x, int width, float eps, c
                                   const float* __restrict__ weight, const int* __restrict__ inv, const float* __restrict__ down,
                                   const float* __restrict__ shared_down, const float* __restrict__ shared_gate, long long ld_shared_gate,
                                   const float* __restrict__ scale_mix, const float* __restrict__ scale_ff, float* __restrict__ tap) {
+  hyb_pdl_enter();
   __shared__ float red[33];
   const int r = blockIdx.x;
   const float* l = left + (size_t)r * width;
@@ -70,6 +72,7 @@ __global__ void hyb_finish_kernel(float* __restrict__ x, int width, float eps, c
 }
 
 __global__ void hyb_softcap_kernel(float* __restrict__ z, size_t n, float cap) {
+  hyb_pdl_enter();
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) z[i] = cap * tanhf(z[i] / cap);
 }
@@ -81,11 +84,15 @@ constexpr int HYB_HOST_INTS = 1024;
 // rows of h in expert-sorted order, so that every expert's rows are one contiguous matrix
 template <typename T>
 __global__ void hyb_gather_rows_kernel(T* __restrict__ dst, const T* __restrict__ src, const int* __restrict__ rows_idx, int width) {
+  hyb_pdl_enter();
   const size_t r = blockIdx.x;
   const T* s = src + (size_t)rows_idx[r] * width;
   for (int i = threadIdx.x; i < width; i += blockDim.x) dst[r * width + i] = s[i];
 }
 static HybScratch g_scratch[64];
+static thread_local bool g_in_step = false;
+struct InStep { InStep() { g_in_step = true; } ~InStep() { g_in_step = false; } };
+bool hyb_gemm_pdl() { return g_in_step && pdl_enabled() != 0; }
 
 struct Carver {
   char* base; size_t at = 0;
@@ -285,7 +292,7 @@ static int hyb_run_experts(void* stream, HybScratch& sc, int dt, int R, int W, c
     // contiguous rows to the TMA-fed tcgen05 matmul of the bf16 path (two launches per expert that has rows)
     if (!sc.host_ints) THA_CUDA_OK(cudaMallocHost((void**)&sc.host_ints, HYB_HOST_INTS * sizeof(int)));
     THA_CUDA_OK(cudaMemcpyAsync(sc.host_ints, b.group_off, (e.experts + 1) * sizeof(int), cudaMemcpyDeviceToHost, s));
-    THA_CUDA_OK(launch(hyb_gather_rows_kernel<bf16>, dim3(R * top), dim3(128), 0, s, false, (bf16*)b.hg, (const bf16*)hf, (const int*)b.sorted_row, W));
+    THA_CUDA_OK(launch(hyb_gather_rows_kernel<bf16>, dim3(R * top), dim3(128), 0, s, pdl_enabled() != 0, (bf16*)b.hg, (const bf16*)hf, (const int*)b.sorted_row, W));
     THA_CUDA_OK(cudaStreamSynchronize(s));
     const int* off = sc.host_ints;
     for (int x = 0; x < e.experts; x++) {
@@ -321,6 +328,7 @@ extern "C" int tha_hyb_step(void* stream, const tha_hyb_model_t* m, const tha_ro
   THA_CUDA_OK(cudaGetDevice(&dev));
   HybScratch& sc = g_scratch[dev & 63];
   std::lock_guard<std::mutex> lock(sc.mu);
+  InStep in_step;
   StepBuffers b;
   const size_t need = carve(m, rows, n_want, nullptr, &b);
   if (need > sc.cap) {   // grow: nothing of an earlier step may still be using the old slab
@@ -337,10 +345,10 @@ extern "C" int tha_hyb_step(void* stream, const tha_hyb_model_t* m, const tha_ro
   bool h_ready = false;   // what ran before already left this layer's first input in b.h (b.hf: see norm_out)
   if (m->n_layers > 0 && m->layers[0].block == THA_BLOCK_POST) h_ready = true;   // the first mixer reads the embedding output itself
   if (dt == THA_DT_BF16)
-    THA_CUDA_OK(launch(hyb_embed_kernel<bf16>, dim3(R), dim3(128), 0, s, false, b.x, (const bf16*)m->embed, rows->token, W, (const bf16*)m->pos_embed,
+    THA_CUDA_OK(launch(hyb_embed_kernel<bf16>, dim3(R), dim3(128), 0, s, pdl_enabled() != 0, b.x, (const bf16*)m->embed, rows->token, W, (const bf16*)m->pos_embed,
                        rows->pos, embed_scale, b.x0, h_ready ? (bf16*)b.h : (bf16*)nullptr, (bf16*)b.join));
   else
-    THA_CUDA_OK(launch(hyb_embed_kernel<float>, dim3(R), dim3(128), 0, s, false, b.x, (const float*)m->embed, rows->token, W,
+    THA_CUDA_OK(launch(hyb_embed_kernel<float>, dim3(R), dim3(128), 0, s, pdl_enabled() != 0, b.x, (const float*)m->embed, rows->token, W,
                        (const float*)m->pos_embed, rows->pos, embed_scale, b.x0, h_ready ? (float*)b.h : (float*)nullptr, (float*)b.join));
   for (int i = 0; i < m->n_rot; i++) HYB_OK(tha_hyb_rotary_table(stream, &m->rot[i], rows->pos, R, b.cos_t[i], b.sin_t[i]));
 
@@ -646,7 +654,7 @@ extern "C" int tha_hyb_step(void* stream, const tha_hyb_model_t* m, const tha_ro
         if (e.shared_scaled) sgate = fproj + e.o_sscale;
       }
     }
-    THA_CUDA_OK(launch(hyb_finish_kernel, dim3(R), dim3(128), 0, s, false, b.x, W, m->eps, (const float*)b.left, right, L.left_out, L.right_out, top,
+    THA_CUDA_OK(launch(hyb_finish_kernel, dim3(R), dim3(128), 0, s, pdl_enabled() != 0, b.x, W, m->eps, (const float*)b.left, right, L.left_out, L.right_out, top,
                        (const float*)b.weight, (const int*)b.inv, (const float*)b.down, sdown, sgate, ldf, L.scale_mix, L.scale_ff,
                        taps ? taps + (size_t)li * R * W : (float*)nullptr));
   }
@@ -655,7 +663,7 @@ extern "C" int tha_hyb_step(void* stream, const tha_hyb_model_t* m, const tha_ro
     HYB_OK(tha_hyb_linear(stream, dt, logits, m->vocab, b.hn, W, 0, nullptr, m->head, 0, n_want, m->vocab, W, nullptr, 0));
     if (m->logit_softcap > 0.f) {
       const size_t n = (size_t)n_want * m->vocab;
-      THA_CUDA_OK(launch(hyb_softcap_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, s, false, logits, n, m->logit_softcap));
+      THA_CUDA_OK(launch(hyb_softcap_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, s, pdl_enabled() != 0, logits, n, m->logit_softcap));
     }
   }
   return THA_STATUS_SUCCESS;

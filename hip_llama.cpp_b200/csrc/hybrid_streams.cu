@@ -51,6 +51,7 @@ template <int V> __device__ __forceinline__ void stv(__nv_bfloat16* p, const flo
 
 template <int NS, typename T, int V>
 __global__ void __launch_bounds__(512) hyb_streams_kernel(StreamsArgs a, T* __restrict__ out) {
+  hyb_pdl_enter();
   extern __shared__ __align__(16) float u_row[];   // [width] when a read follows
   __shared__ float red[33];
   __shared__ float c_mix[NS * NS], c_out[NS], c_in[NS];
@@ -155,6 +156,7 @@ __global__ void __launch_bounds__(512) hyb_streams_kernel(StreamsArgs a, T* __re
 template <typename T, int V>
 __global__ void __launch_bounds__(256) hyb_polynorm_kernel(T* __restrict__ y, const float* __restrict__ gu, long long ldg, int col_u,
                                                            const float* __restrict__ bias, float c0, float c1, float c2, float c3, float eps, int ff) {
+  hyb_pdl_enter();
   __shared__ float red[33];
   const size_t r = blockIdx.x;
   const float* z = gu + r * ldg + col_u;
@@ -192,6 +194,7 @@ __global__ void __launch_bounds__(256) hyb_polynorm_kernel(T* __restrict__ y, co
 template <typename T>
 __global__ void hyb_diff_combine_kernel(T* __restrict__ out, const float* __restrict__ att, int n_rows, int H, int gs, int E, float lambda,
                                         float mult, float eps, const float* __restrict__ gate, long long ldg) {
+  hyb_pdl_enter();
   const int idx = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (idx >= n_rows * H) return;
   const int r = idx / H, h = idx - r * H, g = h / gs, hh = h - g * gs;
@@ -218,7 +221,7 @@ static int streams_launch(cudaStream_t s, const StreamsArgs& a, int out_kind, vo
 #define STREAMS_GO(T, V)                                                                                                               \
   do {                                                                                                                                 \
     if (smem > 48 * 1024) THA_CUDA_OK(cudaFuncSetAttribute(hyb_streams_kernel<NS, T, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-    THA_CUDA_OK(launch(hyb_streams_kernel<NS, T, V>, dim3(n_rows), dim3(nt), smem, s, false, a, (T*)out));                             \
+    THA_CUDA_OK(launch(hyb_streams_kernel<NS, T, V>, dim3(n_rows), dim3(nt), smem, s, pdl_enabled() != 0, a, (T*)out));                             \
   } while (0)
   if (out_kind == 0) { if (vec) STREAMS_GO(float, VV); else STREAMS_GO(float, 1); }
   else { if (vec) STREAMS_GO(__nv_bfloat16, VV); else STREAMS_GO(__nv_bfloat16, 1); }
@@ -265,7 +268,7 @@ extern "C" int tha_hyb_polynorm(void* stream, int dtype, void* y, const float* g
   const bool vec = ff % 4 == 0 && ldg % 4 == 0 && col_u % 4 == 0 && aligned16(gu) && aligned16(bias) && aligned16(y);
   const int nt = ff >= (vec ? 4096 : 1024) ? 256 : 128;
 #define POLY_GO(T, V) \
-  THA_CUDA_OK(launch(hyb_polynorm_kernel<T, V>, dim3(n), dim3(nt), 0, s, false, (T*)y, gu, ldg, col_u, bias, c[0], c[1], c[2], c[3], eps, ff))
+  THA_CUDA_OK(launch(hyb_polynorm_kernel<T, V>, dim3(n), dim3(nt), 0, s, pdl_enabled() != 0, (T*)y, gu, ldg, col_u, bias, c[0], c[1], c[2], c[3], eps, ff))
   if (dtype == THA_DT_BF16) { if (vec) POLY_GO(bf16, 4); else POLY_GO(bf16, 1); }
   else { if (vec) POLY_GO(float, 4); else POLY_GO(float, 1); }
 #undef POLY_GO
@@ -281,10 +284,10 @@ extern "C" int tha_hyb_diff_combine(void* stream, int dtype, const tha_attn_t* a
   cudaStream_t s = (cudaStream_t)stream;
   const dim3 grid(ceil_div(n_rows * H, 4));
   if (dtype == THA_DT_BF16)
-    THA_CUDA_OK(launch(hyb_diff_combine_kernel<bf16>, grid, dim3(128), 0, s, false, (bf16*)out, att, n_rows, H, gs, a->vdim, a->diff_lambda, a->diff_mult,
+    THA_CUDA_OK(launch(hyb_diff_combine_kernel<bf16>, grid, dim3(128), 0, s, pdl_enabled() != 0, (bf16*)out, att, n_rows, H, gs, a->vdim, a->diff_lambda, a->diff_mult,
                        a->eps, gate, ldp));
   else
-    THA_CUDA_OK(launch(hyb_diff_combine_kernel<float>, grid, dim3(128), 0, s, false, (float*)out, att, n_rows, H, gs, a->vdim, a->diff_lambda, a->diff_mult,
+    THA_CUDA_OK(launch(hyb_diff_combine_kernel<float>, grid, dim3(128), 0, s, pdl_enabled() != 0, (float*)out, att, n_rows, H, gs, a->vdim, a->diff_lambda, a->diff_mult,
                        a->eps, gate, ldp));
   return THA_STATUS_SUCCESS;
 }

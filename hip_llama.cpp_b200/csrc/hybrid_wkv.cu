@@ -34,6 +34,7 @@ __device__ __forceinline__ void shift_load(const float* p, float* v) {
 template <typename T, int V>
 __global__ void hyb_token_shift_kernel(tha_rows_t rows, tha_state_store_t st, long long state_off, const float* __restrict__ h, int width,
                                        const float* __restrict__ mu, int n_mix, T* __restrict__ out) {
+  hyb_pdl_enter();
   const int c = V * (blockIdx.y * blockDim.x + threadIdx.x), r = blockIdx.x;
   if (c >= width) return;
   const int s = rows.row_seq[r];
@@ -60,6 +61,7 @@ constexpr int WD_T = 64, WD_K = 16;
 template <typename T>
 __global__ void __launch_bounds__(256) hyb_wkv_decay_kernel(float* __restrict__ decay, const float* __restrict__ z, long long ldz, int rank,
                                                             const T* __restrict__ w2, const float* __restrict__ w0, int n_rows, int n_ch) {
+  hyb_pdl_enter();
   __shared__ float As[WD_K][WD_T + 4];
   __shared__ float Ws[WD_K][WD_T + 4];
   const int c0 = blockIdx.x * WD_T, r0 = blockIdx.y * WD_T;
@@ -110,7 +112,7 @@ extern "C" int tha_hyb_token_shift(void* stream, int dtype, const tha_rows_t* ro
   cudaStream_t s = (cudaStream_t)stream;
   const bool vec = width % 4 == 0 && aligned16(h) && aligned16(mu) && aligned16(out);
   const dim3 grid(rows->n_rows, ceil_div(vec ? width / 4 : width, 128));
-#define SHIFT_GO(T, V) THA_CUDA_OK(launch(hyb_token_shift_kernel<T, V>, grid, dim3(128), 0, s, false, *rows, *st, shift_state_off, h, width, mu, n_mix, (T*)out))
+#define SHIFT_GO(T, V) THA_CUDA_OK(launch(hyb_token_shift_kernel<T, V>, grid, dim3(128), 0, s, pdl_enabled() != 0, *rows, *st, shift_state_off, h, width, mu, n_mix, (T*)out))
   if (dtype == THA_DT_BF16) { if (vec) SHIFT_GO(bf16, 4); else SHIFT_GO(bf16, 1); }
   else { if (vec) SHIFT_GO(float, 4); else SHIFT_GO(float, 1); }
 #undef SHIFT_GO
@@ -126,9 +128,9 @@ extern "C" int tha_hyb_wkv_scan(void* stream, int dtype, const tha_wkv_t* g, con
   const int R = rows->n_rows, HD = g->heads * g->dim;
   const dim3 grid(ceil_div(HD, WD_T), ceil_div(R, WD_T));
   if (dtype == THA_DT_BF16)
-    THA_CUDA_OK(launch(hyb_wkv_decay_kernel<bf16>, grid, dim3(256), 0, s, false, decay, proj + g->o_w1, ldp, g->rank, (const bf16*)g->w_w2, g->w0, R, HD));
+    THA_CUDA_OK(launch(hyb_wkv_decay_kernel<bf16>, grid, dim3(256), 0, s, pdl_enabled() != 0, decay, proj + g->o_w1, ldp, g->rank, (const bf16*)g->w_w2, g->w0, R, HD));
   else
-    THA_CUDA_OK(launch(hyb_wkv_decay_kernel<float>, grid, dim3(256), 0, s, false, decay, proj + g->o_w1, ldp, g->rank, (const float*)g->w_w2, g->w0, R, HD));
+    THA_CUDA_OK(launch(hyb_wkv_decay_kernel<float>, grid, dim3(256), 0, s, pdl_enabled() != 0, decay, proj + g->o_w1, ldp, g->rank, (const float*)g->w_w2, g->w0, R, HD));
   tha_gla_t a = {};
   a.heads = g->heads; a.dim = g->dim; a.vdim = g->dim; a.o_q = g->o_r; a.o_k = g->o_k; a.o_v = g->o_v; a.state_off = g->state_off;
   const int status = hyb_scan_launch(s, SCAN_BONUS, &a, rows, st, proj, ldp, decay, g->u, o_raw, 1.0f, seg_scratch, seg_scratch_floats);
