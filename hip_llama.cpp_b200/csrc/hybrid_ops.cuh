@@ -11,8 +11,9 @@ namespace tha {
 // kernels ahead have completed (no-op in a launch without the programmatic attribute).  A step of a few decoded rows is 20 to 100 kernels of 2
 // to 10 us, and the launches between them were a quarter of it: two layers of attention 286 -> 220 us, four recurrent ones 405 -> 285.
 __device__ __forceinline__ void hyb_pdl_enter() { pdl_trigger(); pdl_wait(); }
-// The bf16 matmul asks for its first weights AHEAD of that wait: only inside tha_hyb_step, where a matrix is the model's own -- in a call
-// of its own it may be what the kernel ahead is writing.
+// The bf16 matmul asks for its first weights AHEAD of that wait: only inside tha_hyb_step, where a matrix is the model's own and no kernel of
+// the step writes it, and whose first kernel is launched behind the completion of all that is ahead of the step on its stream -- in
+// a call of its own a matrix may be what the kernel ahead is writing.
 bool hyb_gemm_pdl();
 __device__ __forceinline__ float hyb_load(const float* p) { return *p; }
 __device__ __forceinline__ float hyb_load(const __nv_bfloat16* p) { return __bfloat162float(*p); }

@@ -344,11 +344,13 @@ extern "C" int tha_hyb_step(void* stream, const tha_hyb_model_t* m, const tha_ro
   const float embed_scale = m->embed_scale != 0.f ? m->embed_scale : 1.0f;
   bool h_ready = false;   // what ran before already left this layer's first input in b.h (b.hf: see norm_out)
   if (m->n_layers > 0 && m->layers[0].block == THA_BLOCK_POST) h_ready = true;   // the first mixer reads the embedding output itself
+  // No programmatic launch here: the step's first kernel starts when everything ahead of the call on this stream has completed, so the
+  // weights that the products ask for ahead of their own wait (hyb_gemm_pdl) may be what a kernel just ahead of the step wrote.
   if (dt == THA_DT_BF16)
-    THA_CUDA_OK(launch(hyb_embed_kernel<bf16>, dim3(R), dim3(128), 0, s, pdl_enabled() != 0, b.x, (const bf16*)m->embed, rows->token, W, (const bf16*)m->pos_embed,
+    THA_CUDA_OK(launch(hyb_embed_kernel<bf16>, dim3(R), dim3(128), 0, s, false, b.x, (const bf16*)m->embed, rows->token, W, (const bf16*)m->pos_embed,
                        rows->pos, embed_scale, b.x0, h_ready ? (bf16*)b.h : (bf16*)nullptr, (bf16*)b.join));
   else
-    THA_CUDA_OK(launch(hyb_embed_kernel<float>, dim3(R), dim3(128), 0, s, pdl_enabled() != 0, b.x, (const float*)m->embed, rows->token, W,
+    THA_CUDA_OK(launch(hyb_embed_kernel<float>, dim3(R), dim3(128), 0, s, false, b.x, (const float*)m->embed, rows->token, W,
                        (const float*)m->pos_embed, rows->pos, embed_scale, b.x0, h_ready ? (float*)b.h : (float*)nullptr, (float*)b.join));
   for (int i = 0; i < m->n_rot; i++) HYB_OK(tha_hyb_rotary_table(stream, &m->rot[i], rows->pos, R, b.cos_t[i], b.sin_t[i]));
 
