@@ -430,8 +430,12 @@ __global__ void __launch_bounds__(1024) tc_prep_q8_kernel(float* __restrict__ x,
   kt_stamp(kt, 6);
 }
 
-// Two float4 per thread: src row (attention output), or with h > 0 the SwiGLU of the w1|w3 partials (run.cc:344-347
-// order), quantised per group (int8 row + transposed scales).  grid (ceil(K / 4 / 512), rows)
+// V float4 per thread, a block-width apart: src row (attention output), or with h > 0 the SwiGLU of the w1|w3 partials (run.cc:344-347
+// order), quantised per group (int8 row + transposed scales).  One for the few rows of a decode step, where twice the blocks count and the
+// second float4's partials come behind the first's: a step of Llama-2-7B at 1 / 8 / 16 slots takes 2.483 / 2.552 / 2.664 ms with one, 2.533 / 2.610 / 2.713
+// with two.  Two from PROMPT_ROWS on, their loads in flight together.
+// grid (ceil(K / 4 / (256 V)), rows)
+template <int V>
 __global__ void __launch_bounds__(256) tc_quant_split_kernel(const float* __restrict__ src, long long ld, int nz,
                                                              long long zstride, int h, const int* __restrict__ pos, int K,
                                                              int gs, int8_t* __restrict__ oq, float* __restrict__ osT, int ldxs) {
@@ -441,10 +445,10 @@ __global__ void __launch_bounds__(256) tc_quant_split_kernel(const float* __rest
   kt_stamp(kt, 1);
   const int b = blockIdx.y;
   const bool live = pos[b] >= 0;
-  float4 r[2];
+  float4 r[V];
 #pragma unroll
-  for (int u = 0; u < 2; u++) {   // two float4 a block-width apart: their loads are in flight together
-    const int i4 = (blockIdx.x * 2 + u) * blockDim.x + threadIdx.x;
+  for (int u = 0; u < V; u++) {
+    const int i4 = (blockIdx.x * V + u) * blockDim.x + threadIdx.x;
     r[u] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (4 * i4 < K && live) {
       if (h > 0) {
@@ -466,11 +470,18 @@ __global__ void __launch_bounds__(256) tc_quant_split_kernel(const float* __rest
     }
   }
 #pragma unroll
-  for (int u = 0; u < 2; u++) {
-    const int i4 = (blockIdx.x * 2 + u) * blockDim.x + threadIdx.x;   // K % gs == 0: a group is never cut, but a warp may be
+  for (int u = 0; u < V; u++) {
+    const int i4 = (blockIdx.x * V + u) * blockDim.x + threadIdx.x;   // K % gs == 0: a group is never cut, but a warp may be
     q8_quant4(r[u], gs, i4, oq + (size_t)b * K, osT, ldxs, b, 4 * i4 < K);
   }
   kt_stamp(kt, 6);
+}
+static int quant_split_launch(cudaStream_t st, bool pdl, int rows, const float* src, long long ld, int nz, long long zstride, int h, const int* pos, int K, int gs,
+                              int8_t* oq, float* osT, int ldxs) {
+  const int v = rows >= PROMPT_ROWS ? 2 : 1;
+  THA_CUDA_OK(launch(v == 2 ? tc_quant_split_kernel<2> : tc_quant_split_kernel<1>, dim3(ceil_div(K / 4, 256 * v), rows), dim3(256), 0, st, pdl, src, ld, nz, zstride, h, pos,
+                     K, gs, oq, osT, ldxs));
+  return THA_STATUS_SUCCESS;
 }
 
 // ---- scratch ----------------------------------------------------------------------------
@@ -984,8 +995,7 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
     }
     if ((skip & 16) || (wq && io.n_tiles == 0 && !(skip & 2))) {
     } else if (wq)   // prompt rows: runq.c:437 as its own launch
-      THA_CUDA_OK(launch(tc_quant_split_kernel, dim3(ceil_div(da / 4, 512), R), dim3(256), 0, st, pdl, (const float*)io.xb, (long long)da,
-                         0, 0LL, 0, io.pos, da, gs, sc.xq, sc.xsT, ldxs));
+      THA_TRY_RC(quant_split_launch(st, pdl, R, io.xb, (long long)da, 0, 0LL, 0, io.pos, da, gs, sc.xq, sc.xsT, ldxs));
     {
       const float* W[1] = {wq ? nullptr : w.wo + (size_t)l * d * da};
       const tha_qtensor_t* Q[1] = {wq ? &wq->wo : nullptr};
@@ -1001,8 +1011,7 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
     }
     if (skip & 16) {
     } else if (wq)   // runq.c:457-465: SwiGLU, then quantise hb
-      THA_CUDA_OK(launch(tc_quant_split_kernel, dim3(ceil_div(hd / 4, 512), R), dim3(256), 0, st, pdl, (const float*)sc.part,
-                         (long long)ld_h, pl.z_w13, (long long)R * ld_h, hd, io.pos, hd, gs, sc.hq, sc.hsT, ldxs));
+      THA_TRY_RC(quant_split_launch(st, pdl, R, sc.part, (long long)ld_h, pl.z_w13, (long long)R * ld_h, hd, io.pos, hd, gs, sc.hq, sc.hsT, ldxs));
     else if (R >= PROMPT_ROWS)
       THA_CUDA_OK(launch(tc_swiglu_split_wide_kernel, dim3(ceil_div(hd, 2048), R), dim3(256), 0, st, pdl, (const float*)sc.part, pl.z_w13,
                          (long long)R * ld_h, ld_h, io.pos, hd, sc.hh, sc.hl));

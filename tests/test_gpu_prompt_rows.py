@@ -54,3 +54,22 @@ def test_q8_rows(heads, hs, hidden):
         want = prefill(b, [(0, i, toks[i:i + 171])], 96)
     assert rel(a.state.key_cache[0, 0, :513], b.state.key_cache[0, 0, :513]) < 2e-6
     assert rel(got, want) < 5e-2
+
+
+@pytest.mark.parametrize("rows", [2, 511, 512])
+@pytest.mark.parametrize("hidden", [32, 1024, 1056, 2080])
+def test_quantiser_on_both_sides_of_its_line(rows, hidden):
+    """The SwiGLU quantiser takes one float4 a thread below 512 rows and two from there on, the same bits either way: the rows of one call
+    against calls of their own (each value differs by the order of partial sums ahead of the quantiser at most)."""
+    eng, ck = load_pkg("engine"), load_pkg("checkpoint")
+    cfg = ck.Config(256, hidden, 2, 8, 8, 96, 520)
+    w = eng.device_random_weights(cfg, q8=True, seed=6, gs=32)
+    toks = np.random.default_rng(8).integers(0, 96, rows).astype(np.int32)
+    a, b = eng.Engine(w, 1, with_att=False), eng.Engine(w, 1, with_att=False)
+    prefill(a, [(0, 0, toks)], 96)
+    half = rows // 2
+    prefill(b, [(0, 0, toks[:half])], 96)
+    prefill(b, [(0, half, toks[half:])], 96)
+    # the second layer's rows have gone through the first one's SwiGLU and its quantiser: a value in a thousand may fall the other way
+    for cache in (lambda e: e.state.key_cache, lambda e: e.state.value_cache):
+        assert rel(cache(a)[0, 1, :rows], cache(b)[0, 1, :rows]) < 1e-2
