@@ -1,5 +1,8 @@
-// Softmax attention of single rows (decoding: one token per sequence) of the layer-program path, in fp32 straight from the cache rows.
+// Softmax attention of single rows (decoding: a sequence with one row in the step) of the layer-program path, in fp32 straight from the cache rows.
 //
+// Which form a row takes depends on its own sequence alone: a decoded token is computed here whether or not another sequence brings a prompt
+// portion to the same step (the tiled kernels, which round to bf16 in that number format, then take the longer portions only).  What still
+// depends on the step is the number of runs a context is cut into, the order of an fp32 sum.
 // The tiled kernels (hybrid_ops.cu) give a block 16 to 128 (position, head) pairs and stage key tiles through shared memory; with
 // one position per sequence most pairs are empty and a block walks its tiles one load latency after the other.  Here a block takes one row,
 // up to four query heads of one key/value head, and a run of 32-key tiles.  Eight lanes share a key (a lane: four channels of every 32), so
@@ -24,10 +27,12 @@ __global__ void __launch_bounds__(AR_THREADS) hyb_attn_row_kernel(tha_attn_t a, 
   __shared__ float sm_acc[4][GS][AR_MAXD];
   __shared__ float sm_ml[4][GS][2];
   const int D = a.dim, E = a.vdim, gsize = a.heads / a.kv_heads;
-  const int r = blockIdx.x / splits, sp = blockIdx.x - r * splits, g = blockIdx.y, h0 = blockIdx.z * GS;
+  const int seq = blockIdx.x / splits, sp = blockIdx.x - seq * splits, g = blockIdx.y, h0 = blockIdx.z * GS;
+  const int r = rows.seq_first[seq];
+  if (rows.seq_first[seq + 1] - r != 1) return;   // a longer portion: the tiled kernels'
   const int gv = a.v_share > 1 ? g / a.v_share : g;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, kq = lane >> 3, c4 = 4 * (lane & 7);
-  const int p = rows.pos[r], slot = rows.seq_slot[rows.row_seq[r]];
+  const int p = rows.pos[r], slot = rows.seq_slot[seq];
   const int first = a.chunk > 0 ? (p / a.chunk) * a.chunk : 0;
   float4 qv[GS][NI], acc[GS][NI];
   float m_run[GS], l_run[GS], hs[GS];
@@ -125,7 +130,7 @@ __global__ void __launch_bounds__(AR_THREADS) hyb_attn_row_kernel(tha_attn_t a, 
 #pragma unroll
     for (int x = 0; x < 4; x++) { w[x] = sm_ml[x][h][0] > -INFINITY ? expf(sm_ml[x][h][0] - M) : 0.f; L += w[x] * sm_ml[x][h][1]; }
     const float inv = splits > 1 ? 1.0f : hyb_attn_final_factor(a, head, M, L, gate ? gate + (size_t)r * ldg : nullptr);
-    float* pd = splits > 1 ? partial + (((size_t)sp * rows.n_rows + r) * a.heads + head) * (E + 2) : nullptr;
+    float* pd = splits > 1 ? partial + (((size_t)sp * rows.n_seqs + seq) * a.heads + head) * (E + 2) : nullptr;
     for (int e = lane; e < E; e += 32) {
       float o = 0.f;
 #pragma unroll
@@ -139,16 +144,16 @@ __global__ void __launch_bounds__(AR_THREADS) hyb_attn_row_kernel(tha_attn_t a, 
   }
 }
 
-// Heads of 32, 64, 96 or 128 channels on 16-byte aligned cache rows, one row per sequence; groups of more than eight query heads fill the
+// Heads of 32, 64, 96 or 128 channels on 16-byte aligned cache rows; groups of more than eight query heads fill the
 // tiled kernels' pairs, and here their key rows would be read a third time.
-bool hyb_attn_row_ok(const tha_attn_t* a, const tha_rows_t* rows, const tha_kv_t* kv, const float* q) {
-  return rows->max_seq_rows == 1 && a->heads <= 2 * AR_HEADS * a->kv_heads && a->dim % 32 == 0 && a->vdim % 32 == 0 && a->dim <= AR_MAXD && a->vdim <= AR_MAXD &&
+bool hyb_attn_row_ok(const tha_attn_t* a, const tha_kv_t* kv, const float* q) {
+  return a->heads <= 2 * AR_HEADS * a->kv_heads && a->dim % 32 == 0 && a->vdim % 32 == 0 && a->dim <= AR_MAXD && a->vdim <= AR_MAXD &&
          kv->kv_dim % 4 == 0 && aligned16(kv->k_pool) && aligned16(kv->v_pool) && aligned16(q);
 }
-// Runs of a row's key tiles: blocks for two to four on an SM, two tiles each at least.
+// Runs of a row's key tiles, were every sequence a single row: blocks for two to four on an SM, two tiles each at least.
 int hyb_attn_row_splits(const tha_attn_t* a, const tha_rows_t* rows, int max_keys) {
   const int gsize = a->heads / a->kv_heads;
-  const long long blocks = (long long)rows->n_rows * a->kv_heads * ceil_div(gsize, AR_HEADS);
+  const long long blocks = (long long)rows->n_seqs * a->kv_heads * ceil_div(gsize, AR_HEADS);
   long long s = ceil_div(4 * 148, (int)(blocks < 4 * 148 ? blocks : 4 * 148));
   if (s > max_keys / 64) s = max_keys / 64;
   return s < 1 ? 1 : (s > 32 ? 32 : (int)s);
@@ -157,7 +162,7 @@ template <typename T>
 static int row_launch(cudaStream_t s, const tha_attn_t* a, const tha_rows_t* rows, const tha_kv_t* kv, const float* q, T* out, int splits, float* partial,
                       const float* gate, long long ldg) {
   const int gsize = a->heads / a->kv_heads, gs = gsize >= 3 ? AR_HEADS : gsize;
-  const dim3 grid(rows->n_rows * splits, a->kv_heads, ceil_div(gsize, gs));
+  const dim3 grid(rows->n_seqs * splits, a->kv_heads, ceil_div(gsize, gs));
   if (gs == 1) THA_CUDA_OK(launch(hyb_attn_row_kernel<T, 1>, grid, dim3(AR_THREADS), 0, s, pdl_enabled() != 0, *a, *rows, *kv, q, out, splits, partial, gate, ldg));
   else if (gs == 2) THA_CUDA_OK(launch(hyb_attn_row_kernel<T, 2>, grid, dim3(AR_THREADS), 0, s, pdl_enabled() != 0, *a, *rows, *kv, q, out, splits, partial, gate, ldg));
   else THA_CUDA_OK(launch(hyb_attn_row_kernel<T, AR_HEADS>, grid, dim3(AR_THREADS), 0, s, pdl_enabled() != 0, *a, *rows, *kv, q, out, splits, partial, gate, ldg));

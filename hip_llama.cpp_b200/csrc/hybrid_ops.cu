@@ -355,7 +355,7 @@ constexpr int ATT_PAIRS = 16, ATT_KEYS = 32, ATT_MAX_VC = 16;   // value channel
 template <typename T, int VC>
 __global__ void __launch_bounds__(128) hyb_attn_kernel(tha_attn_t a, tha_rows_t rows, tha_kv_t kv, const float* __restrict__ q,
                                                        T* __restrict__ out, int AG, int AP, int splits, float* __restrict__ partial,
-                                                       const float* __restrict__ gate, long long ldg) {
+                                                       const float* __restrict__ gate, long long ldg, int min_rows) {
   hyb_pdl_enter();
   extern __shared__ __align__(16) float sm[];
   const int D = a.dim, E = a.vdim, gsize = a.heads / a.kv_heads;
@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(128) hyb_attn_kernel(tha_attn_t a, tha_rows_t 
     int tile = (int)(gridDim.x / splits) - 1 - (int)(blockIdx.x / splits);
     for (int s = 0; s < rows.n_seqs; s++) {
       const int lo = rows.seq_first[s], hi = rows.seq_first[s + 1];
-      const int nt = (hi - lo + AP - 1) / AP;
+      const int nt = hi - lo >= min_rows ? (hi - lo + AP - 1) / AP : 0;
       if (tile < nt) { seq = s; r0 = lo + tile * AP; r_end = min(hi, r0 + AP); break; }
       tile -= nt;
     }
@@ -613,7 +613,7 @@ __host__ __device__ inline int attn_mma_stage(int D, int E, int AG, int AP, bool
 template <bool EXACT, bool CAP, bool REL, int DT>
 __global__ void __launch_bounds__(AM_THREADS, 1) hyb_attn_mma_kernel(tha_attn_t a, tha_rows_t rows, tha_kv_t kv, const float* __restrict__ q,
                                                            __nv_bfloat16* __restrict__ out, int AG, int AP, int splits,
-                                                           float* __restrict__ partial, const float* __restrict__ gate, long long ldg) {
+                                                           float* __restrict__ partial, const float* __restrict__ gate, long long ldg, int min_rows) {
   hyb_pdl_enter();
   extern __shared__ __align__(16) unsigned char smraw[];
   const int D = DT ? DT : a.dim, E = DT ? DT : a.vdim, gsize = a.heads / a.kv_heads;
@@ -628,7 +628,7 @@ __global__ void __launch_bounds__(AM_THREADS, 1) hyb_attn_mma_kernel(tha_attn_t 
     int tile = (int)(gridDim.x / splits) - 1 - (int)(blockIdx.x / splits);
     for (int s = 0; s < rows.n_seqs; s++) {
       const int lo = rows.seq_first[s], hi = rows.seq_first[s + 1];
-      const int nt = (hi - lo + AP - 1) / AP;
+      const int nt = hi - lo >= min_rows ? (hi - lo + AP - 1) / AP : 0;
       if (tile < nt) { seq = s; r0 = lo + tile * AP; r_end = min(hi, r0 + AP); break; }
       tile -= nt;
     }
@@ -879,16 +879,25 @@ __global__ void __launch_bounds__(AM_THREADS, 1) hyb_attn_mma_kernel(tha_attn_t 
 // the splits of a (row, head) in ascending key order: out = sum_s acc_s e^(m_s - M) / sum_s l_s e^(m_s - M); a block per (row, head), a warp
 // per 32 channels.  Lane s keeps split s's maximum, sum and factor (at most 32 splits); a channel's values of all splits are in
 // flight at once (one load after the other took 32 us for 16 splits of 2 rows, eight at a time and a warp for all channels 20 us for 32).
+// What the partials are of: MERGE_ROWS every row of the step, MERGE_LONGER the rows of portions of two and more, MERGE_SINGLE the one row
+// of every sequence that has one (partials by sequence).
 constexpr int AMG_SPLITS = 32;
+enum { MERGE_ROWS = 0, MERGE_LONGER = 1, MERGE_SINGLE = 2 };
 template <typename T>
-__global__ void __launch_bounds__(128) hyb_attn_merge_kernel(T* __restrict__ out, const float* __restrict__ partial, int n_rows, int heads, int E, int splits,
+__global__ void __launch_bounds__(128) hyb_attn_merge_kernel(T* __restrict__ out, const float* __restrict__ partial, tha_rows_t rows, int which, int splits,
                                                              tha_attn_t a, const float* __restrict__ gate, long long ldg) {
   hyb_pdl_enter();
-  const int idx = blockIdx.x, lane = threadIdx.x & 31;
-  const size_t stride = (size_t)n_rows * heads * (E + 2);
+  const int idx = blockIdx.x, lane = threadIdx.x & 31, heads = a.heads, E = a.vdim;
+  const size_t stride = (size_t)(which == MERGE_SINGLE ? rows.n_seqs : rows.n_rows) * heads * (E + 2);
   const float* p0 = partial + (size_t)idx * (E + 2);
   const float ms = lane < splits ? p0[lane * stride + E] : -INFINITY, ls = lane < splits ? p0[lane * stride + E + 1] : 0.f;
-  const int row = idx / heads, head = idx - row * heads;
+  const int at = idx / heads, head = idx - at * heads;
+  int row = at;
+  if (which != MERGE_ROWS) {
+    const int seq = which == MERGE_SINGLE ? at : rows.row_seq[at], first = rows.seq_first[seq];
+    if ((rows.seq_first[seq + 1] - first == 1) != (which == MERGE_SINGLE)) return;
+    if (which == MERGE_SINGLE) row = first;
+  }
   for (int e0 = (threadIdx.x >> 5) * 32; e0 < E; e0 += blockDim.x) {
     const int e = e0 + lane;
     float v[AMG_SPLITS];
@@ -903,7 +912,7 @@ __global__ void __launch_bounds__(128) hyb_attn_merge_kernel(T* __restrict__ out
       const float ws = __shfl_sync(THA_FULL_MASK, w, u);
       if (ws > 0.f) o = fmaf(v[u], ws, o);
     }
-    if (e < E) hyb_store(out + (size_t)idx * E + e, o * hyb_attn_final_factor(a, head, M, L, gate ? gate + (size_t)row * ldg : nullptr));
+    if (e < E) hyb_store(out + ((size_t)row * heads + head) * E + e, o * hyb_attn_final_factor(a, head, M, L, gate ? gate + (size_t)row * ldg : nullptr));
   }
 }
 
@@ -1791,7 +1800,7 @@ namespace tha {
 // hybrid_latent.cu: tensor-core attention for key rows wider than AM_MAXD whose values lie inside the keys
 bool hyb_attn_wide_ok(const tha_attn_t* a);
 int hyb_attn_wide_pairs(const tha_attn_t* a, const tha_rows_t* rows);
-bool hyb_attn_row_ok(const tha_attn_t* a, const tha_rows_t* rows, const tha_kv_t* kv, const float* q);   // hybrid_attn_row.cu
+bool hyb_attn_row_ok(const tha_attn_t* a, const tha_kv_t* kv, const float* q);   // hybrid_attn_row.cu
 int hyb_attn_row_splits(const tha_attn_t* a, const tha_rows_t* rows, int max_keys);
 int hyb_attn_row_launch(cudaStream_t s, int dtype, const tha_attn_t* a, const tha_rows_t* rows, const tha_kv_t* kv, const float* q, void* out, int splits,
                         float* partial, const float* gate, long long ldg);
@@ -1831,7 +1840,7 @@ extern "C" int tha_hyb_attn_gated(void* stream, int dtype, const tha_attn_t* a, 
   if (a->heads % a->kv_heads || a->vdim > 32 * ATT_MAX_VC) return THA_STATUS_NOT_SUPPORTED;
   if (a->v_share > 1 && (a->kv_heads % a->v_share || a->values_in_keys)) return THA_STATUS_INVALID_ARG;
   const int gsize = a->heads / a->kv_heads;
-  // bf16 with heads the tensor-core form covers: 64 pairs per block; else 16 pairs on the fp32 cores
+  // bf16 with heads the tensor-core form covers: 128 pairs per block; else 16 pairs on the fp32 cores
   if (a->rel && a->rel_n < 1) return THA_STATUS_INVALID_ARG;
   const bool tc = !(a->rel && a->softcap > 0.f) && dtype == THA_DT_BF16 && hyb_tc_linear() && hyb_tc_attn() && a->dim % 16 == 0 && a->vdim % 8 == 0 && a->dim <= AM_MAXD && a->vdim <= AM_MAXD &&
                   (a->heads * a->vdim) % 2 == 0;
@@ -1840,7 +1849,7 @@ extern "C" int tha_hyb_attn_gated(void* stream, int dtype, const tha_attn_t* a, 
   const int AG = gsize < pairs ? gsize : pairs, AP = pairs / AG;
   const size_t smem = tc ? 2 * (size_t)attn_mma_stage(a->dim, a->vdim, AG, AP, a->rel != nullptr)
                          : sizeof(float) * ((size_t)ATT_PAIRS * a->dim + (size_t)ATT_KEYS * (a->dim + 4) + (size_t)ATT_KEYS * a->vdim + ATT_PAIRS * ATT_KEYS);
-  const bool row_form = hyb_attn_row_ok(a, rows, kv, q);   // one row per sequence
+  const bool row_form = hyb_attn_row_ok(a, kv, q);   // sequences with one row in the step go to the row kernel (longer portions to the tiled ones)
   if (!wide && !row_form && smem > 227 * 1024) return THA_STATUS_NOT_SUPPORTED;
   // position tiles: at most one ragged tile per sequence beyond rows / AP
   const int tiles = rows->n_rows / AP + rows->n_seqs;
@@ -1850,20 +1859,22 @@ extern "C" int tha_hyb_attn_gated(void* stream, int dtype, const tha_attn_t* a, 
   if (a->window > 0 && a->window + a->keep_first + 2 * ATT_KEYS < max_keys) max_keys = a->window + a->keep_first + 2 * ATT_KEYS;
   int splits = 1;
   cudaStream_t s = (cudaStream_t)stream;
-  if (row_form) {
-    splits = split_scratch ? hyb_attn_row_splits(a, rows, max_keys) : 1;
-    while (splits > 1 && (size_t)splits * rows->n_rows * a->heads * (a->vdim + 2) > split_scratch_floats) splits--;
-    const int st = hyb_attn_row_launch(s, dtype, a, rows, kv, q, out, splits, split_scratch, gate, ldg);
-    if (st != THA_STATUS_SUCCESS || splits <= 1) return st;
-    const dim3 mgrid(rows->n_rows * a->heads);
+  auto merge = [&](int which, int n, int parts) -> int {
+    const dim3 grid(n * a->heads);
     if (dtype != THA_DT_BF16 || a->out_f32)
-      THA_CUDA_OK(launch(hyb_attn_merge_kernel<float>, mgrid, dim3(128), 0, s, pdl_enabled() != 0, (float*)out, (const float*)split_scratch, rows->n_rows, a->heads, a->vdim,
-                         splits, *a, gate, ldg));
+      THA_CUDA_OK(launch(hyb_attn_merge_kernel<float>, grid, dim3(128), 0, s, pdl_enabled() != 0, (float*)out, (const float*)split_scratch, *rows, which, parts, *a, gate, ldg));
     else
-      THA_CUDA_OK(launch(hyb_attn_merge_kernel<bf16>, mgrid, dim3(128), 0, s, pdl_enabled() != 0, (bf16*)out, (const float*)split_scratch, rows->n_rows, a->heads, a->vdim,
-                         splits, *a, gate, ldg));
+      THA_CUDA_OK(launch(hyb_attn_merge_kernel<bf16>, grid, dim3(128), 0, s, pdl_enabled() != 0, (bf16*)out, (const float*)split_scratch, *rows, which, parts, *a, gate, ldg));
     return THA_STATUS_SUCCESS;
+  };
+  if (row_form && (rows->n_seqs > 1 || rows->max_seq_rows == 1)) {
+    int parts = split_scratch ? hyb_attn_row_splits(a, rows, max_keys) : 1;
+    while (parts > 1 && (size_t)parts * rows->n_seqs * a->heads * (a->vdim + 2) > split_scratch_floats) parts--;
+    THA_TRY_RC(hyb_attn_row_launch(s, dtype, a, rows, kv, q, out, parts, split_scratch, gate, ldg));
+    if (parts > 1) THA_TRY_RC(merge(rows->max_seq_rows == 1 ? MERGE_ROWS : MERGE_SINGLE, rows->n_seqs, parts));
+    if (rows->max_seq_rows == 1) return THA_STATUS_SUCCESS;
   }
+  const int min_rows = row_form ? 2 : 1;
   const long long blocks = (long long)tiles * a->kv_heads * ceil_div(gsize, AG);
   const int fill = tc ? 2 * 148 : 4 * 148;   // blocks from which the SMs are full without splits (the tensor-core form: one block of 8 warps each)
   if (split_scratch && blocks < fill && max_keys >= 4 * ATT_KEYS) {
@@ -1880,34 +1891,26 @@ extern "C" int tha_hyb_attn_gated(void* stream, int dtype, const tha_attn_t* a, 
     } else if (tc) {
       const int dt = a->dim == a->vdim && (a->dim == 64 || a->dim == 128) ? a->dim : 0;
       auto k = a->rel ? mma_of<true, false, true>(dt) : a->softcap > 0.f ? mma_of<true, true, false>(dt) : a->fp32_scores ? mma_of<true, false, false>(dt) : mma_of<false, false, false>(dt);
-      THA_CUDA_OK(launch_smem(k, grid, dim3(AM_THREADS), smem, s, pdl_enabled() != 0, *a, *rows, *kv, q, (bf16*)out, AG, AP, splits, split_scratch, gate, ldg));
+      THA_CUDA_OK(launch_smem(k, grid, dim3(AM_THREADS), smem, s, pdl_enabled() != 0, *a, *rows, *kv, q, (bf16*)out, AG, AP, splits, split_scratch, gate, ldg, min_rows));
     } else {
       if (a->vdim <= 256) {
         if (smem > 48 * 1024) THA_CUDA_OK(cudaFuncSetAttribute(hyb_attn_kernel<bf16, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        THA_CUDA_OK(launch(hyb_attn_kernel<bf16, 8>, grid, dim3(128), smem, s, pdl_enabled() != 0, *a, *rows, *kv, q, (bf16*)out, AG, AP, splits, split_scratch, gate, ldg));
+        THA_CUDA_OK(launch(hyb_attn_kernel<bf16, 8>, grid, dim3(128), smem, s, pdl_enabled() != 0, *a, *rows, *kv, q, (bf16*)out, AG, AP, splits, split_scratch, gate, ldg, min_rows));
       } else {
         if (smem > 48 * 1024) THA_CUDA_OK(cudaFuncSetAttribute(hyb_attn_kernel<bf16, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        THA_CUDA_OK(launch(hyb_attn_kernel<bf16, 16>, grid, dim3(128), smem, s, pdl_enabled() != 0, *a, *rows, *kv, q, (bf16*)out, AG, AP, splits, split_scratch, gate, ldg));
+        THA_CUDA_OK(launch(hyb_attn_kernel<bf16, 16>, grid, dim3(128), smem, s, pdl_enabled() != 0, *a, *rows, *kv, q, (bf16*)out, AG, AP, splits, split_scratch, gate, ldg, min_rows));
       }
     }
-    if (splits > 1 && a->out_f32)
-      THA_CUDA_OK(launch(hyb_attn_merge_kernel<float>, dim3(rows->n_rows * a->heads), dim3(128), 0, s, pdl_enabled() != 0, (float*)out,
-                         (const float*)split_scratch, rows->n_rows, a->heads, a->vdim, splits, *a, gate, ldg));
-    else if (splits > 1)
-      THA_CUDA_OK(launch(hyb_attn_merge_kernel<bf16>, dim3(rows->n_rows * a->heads), dim3(128), 0, s, pdl_enabled() != 0, (bf16*)out,
-                         (const float*)split_scratch, rows->n_rows, a->heads, a->vdim, splits, *a, gate, ldg));
   } else {
     if (a->vdim <= 256) {
       if (smem > 48 * 1024) THA_CUDA_OK(cudaFuncSetAttribute(hyb_attn_kernel<float, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      THA_CUDA_OK(launch(hyb_attn_kernel<float, 8>, grid, dim3(128), smem, s, pdl_enabled() != 0, *a, *rows, *kv, q, (float*)out, AG, AP, splits, split_scratch, gate, ldg));
+      THA_CUDA_OK(launch(hyb_attn_kernel<float, 8>, grid, dim3(128), smem, s, pdl_enabled() != 0, *a, *rows, *kv, q, (float*)out, AG, AP, splits, split_scratch, gate, ldg, min_rows));
     } else {
       if (smem > 48 * 1024) THA_CUDA_OK(cudaFuncSetAttribute(hyb_attn_kernel<float, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      THA_CUDA_OK(launch(hyb_attn_kernel<float, 16>, grid, dim3(128), smem, s, pdl_enabled() != 0, *a, *rows, *kv, q, (float*)out, AG, AP, splits, split_scratch, gate, ldg));
+      THA_CUDA_OK(launch(hyb_attn_kernel<float, 16>, grid, dim3(128), smem, s, pdl_enabled() != 0, *a, *rows, *kv, q, (float*)out, AG, AP, splits, split_scratch, gate, ldg, min_rows));
     }
-    if (splits > 1)
-      THA_CUDA_OK(launch(hyb_attn_merge_kernel<float>, dim3(rows->n_rows * a->heads), dim3(128), 0, s, pdl_enabled() != 0, (float*)out,
-                         (const float*)split_scratch, rows->n_rows, a->heads, a->vdim, splits, *a, gate, ldg));
   }
+  if (splits > 1) THA_TRY_RC(merge(row_form ? MERGE_LONGER : MERGE_ROWS, rows->n_rows, splits));
   return THA_STATUS_SUCCESS;
 }
 

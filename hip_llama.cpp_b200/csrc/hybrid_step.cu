@@ -234,8 +234,9 @@ static size_t carve(const tha_hyb_model_t* m, const tha_rows_t* rows, int n_want
   b->abuf = c.take<char>(R * av * es);
   b->mbuf = c.take<char>(R * mv * es);
   b->oraw = c.take<float>(R * mv);
-  // key splits of the attention in small steps: 16 x rows x heads x (vdim + 2) floats at most (2 * heads <= 2 * heads * dim)
-  b->split_floats = R <= 1024 ? (size_t)16 * R * (av + 2 * qd) : 0;
+  // key splits of the attention, of every row in small steps, of the single rows beside a prompt in large ones: 16 x rows x heads x (vdim + 2)
+  // floats and more (2 * heads <= 2 * heads * dim)
+  b->split_floats = (size_t)16 * (R <= 1024 ? R : rows->n_seqs > 1 ? rows->n_seqs : 0) * (av + 2 * qd);
   b->split = c.take<float>(b->split_floats);
   b->scan_floats = scan;
   b->scan = scan ? c.take<float>(scan) : nullptr;

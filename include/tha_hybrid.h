@@ -510,8 +510,11 @@ int tha_hyb_add_norm(void* stream, int dtype, float* x, const float* left, const
                      float c_right, const float* embed_out, const float* vec, const tha_norm_t* n, float eps, void* out, long long ldo,
                      int n_rows, int width);
 /* softmax attention of every row over its visible cache rows; out dtype-typed [n_rows, heads * vdim].
+ * A sequence with ONE row in the step (a decoded token) is computed in fp32 in every number format, whatever the other sequences bring,
+ * where key and value heads have 32, 64, 96 or 128 channels, at most eight query heads share a key head, and pools and q are 16-byte aligned.
  * split_scratch (nullable, fp32): room for the partial results when a step of few rows at long contexts is cut along
- * the keys (splits * n_rows * heads * (vdim + 2) floats are used, as many splits as fit, at most 16) */
+ * the keys (splits * n_rows * heads * (vdim + 2) floats are used, splits * n_seqs for single rows; as many splits as fit, at most 16, 32 for
+ * single rows) */
 int tha_hyb_attn(void* stream, int dtype, const tha_attn_t* a, const tha_rows_t* rows, const tha_kv_t* kv, const float* q,
                  void* out, float* split_scratch, size_t split_scratch_floats);
 /* the matrix memory over the rows of every sequence in order, state read from and written back to the slots;
