@@ -853,6 +853,14 @@ __global__ void __launch_bounds__(AM_THREADS, 1) hyb_attn_mma_kernel(tha_attn_t 
 #pragma unroll
   for (int x = 0; x < 2; x++) {
     if (!row_ok[x]) continue;
+    if (m_run[x] > -INFINITY) {
+      // the weights are 2^(s log2(e) + shift) with shift = -m log2(e) ROUNDED: all of them, and their sum, carry the factor 2^(m log2(e) + shift)
+      // over e^(s - m) (up to 6e-8 |m|; the fma gives the exponent exactly).  It goes out here: the merge of the splits and the sink weigh the sums by m.
+      const float f = attn_ex2(-fmaf(m_run[x], LOG2E, shift_run[x]));
+      l_run[x] *= f;
+#pragma unroll
+      for (int n = 0; n < AM_MAXD / 8; n++) { oacc[n][2 * x] *= f; oacc[n][2 * x + 1] *= f; }
+    }
     if (splits > 1) {
       float* dst = partial + (((size_t)(blockIdx.x % splits) * rows.n_rows + row_r[x]) * a.heads + row_h[x]) * (E + 2);
 #pragma unroll

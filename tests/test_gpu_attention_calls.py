@@ -105,3 +105,29 @@ def test_runs_of_a_single_row(dtype, out_f32, heads, kv_heads, dim, vdim, window
     got = run(dtype, a, cache, q, seqs, runs * heads * (vdim + 2))
     # fp32 throughout; rounded to bf16 at the end where that is asked for: eight significant bits, so half a unit is up to 2^-8 of a value
     assert rel(got, want(a, cache, q, seqs)) < (2e-6 if dtype == H.F32 or out_f32 else 2.0 ** -8)
+
+
+@pytest.mark.parametrize("form", ["runs", "sink"])
+def test_large_scores(form):
+    """Scores around 65536 that differ by whole 64ths, a different largest one in every run of keys: every score, weight exponent and value is
+    exact, so the result carries the 16 bits of the weights (hi + lo) and fp32 sums.  An exponent's offset rounded per run (65536 log2(e)
+    has a spacing of 2^-7) would move the runs, or the keys and the sink,
+    against one another by up to 0.3 %."""
+    heads, dim, p0 = 2, 64, 1023
+    a = H.Attn(heads=heads, kv_heads=1, dim=dim, vdim=dim, rot=-1, scale=1.0, out_f32=1, fp32_scores=1)
+    cache = Cache(1, p0 + 2, 1, dim, dim)
+    rng = np.random.default_rng(7)
+    t = np.arange(cache.k.shape[1])
+    run_of = t // 96
+    x = (rng.integers(0, 96, run_of.max() + 1)[run_of] + t * 37 % 32) / 64.0
+    cache.k.zero_()
+    cache.k[0, :, 0, 0] = 65536.0
+    cache.k[0, :, 0, 1] = torch.from_numpy(x).cuda().float()
+    cache.v[0, :, 0] = torch.from_numpy(rng.choice([-1.0, 1.0], (run_of.max() + 1, dim))[run_of]).cuda().float()
+    q = torch.zeros(2, heads, dim, device="cuda")
+    q[:, :, :2] = 1.0
+    sink = torch.tensor([65543.5, 65544.0 + 5 / 64], device="cuda") if form == "sink" else None
+    a.sink = H.ptr(sink)
+    seqs = [(0, p0, 2)]                     # a portion of two rows: the tensor-core form
+    got = run(H.BF16, a, cache, q, seqs, 0 if form == "sink" else 16 * 2 * heads * (dim + 2))
+    assert rel(got, want(a, cache, q, seqs, sink)) < 5e-5
