@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(256) attn_prefill_kernel(const AttnPrefillP p)
   const float* kbase = (p.pg.table ? p.kc : p.kc + (size_t)slot * p.kv_batch_stride) + kh * HS;
   const float* vbase = (p.pg.table ? p.vc : p.vc + (size_t)slot * p.kv_batch_stride) + kh * HS;
   const int kmax = pos0 + n - 1;   // last key any row of the tile may see
-  const float inv_sqrt_hs = 1.0f / sqrtf((float)HS);
+  const float sqrt_hs = sqrtf((float)HS);
   constexpr int C4 = HS / 4;       // float4 per row
 
   // keys tk0 .. tk0 + 63 -> dst (row pitch `pitch`): consecutive threads take consecutive 16-byte pieces of a row
@@ -122,21 +122,25 @@ __global__ void __launch_bounds__(256) attn_prefill_kernel(const AttnPrefillP p)
 #pragma unroll
       for (int j = 0; j < 4; j++) {
         const int t = tk0 + tx + 16 * j;
-        s[i][j] = (t <= qpos[i]) ? s[i][j] * inv_sqrt_hs : -INFINITY;
+        s[i][j] = (t <= qpos[i]) ? s[i][j] / sqrt_hs : -INFINITY;
         rmax = fmaxf(rmax, s[i][j]);
       }
 #pragma unroll
       for (int off = 8; off > 0; off >>= 1) rmax = fmaxf(rmax, __shfl_xor_sync(THA_FULL_MASK, rmax, off));
       const float mn = fmaxf(m[i], rmax);          // finite: key 0 is visible to every row in the first tile
       const float corr = expf(m[i] - mn);          // exp(-inf) = 0 on the first tile
-      float sum = 0.0f;
 #pragma unroll
       for (int j = 0; j < 4; j++) {
-        const float pv = expf(s[i][j] - mn);
-        sum += pv;
-        Ps[(ty + 16 * i) * PF_PS + tx + 16 * j] = pv;
+        s[i][j] = expf(s[i][j] - mn);
+        Ps[(ty + 16 * i) * PF_PS + tx + 16 * j] = s[i][j];
       }
-      l[i] = l[i] * corr + sum;   // per-thread partial of the row sum; reduced at the end
+      // partial of the row sum, reduced at the end: thread tx adds the four neighbouring keys 4 m .. 4 m + 3, m = 4 (tx & 3) + (tx >> 2), which four
+      // neighbouring threads hold (three exchanges).  The grouping is part of the result's bits: a quantiser behind it turns a last bit into
+      // a step, and with sums in another order 3 of 130 next tokens of quantised prompts changed.
+      const bool b0 = tx & 1, b1 = tx & 2;
+      const float u0 = (b0 ? s[i][1] : s[i][0]) + __shfl_xor_sync(THA_FULL_MASK, b0 ? s[i][0] : s[i][1], 1);   // column j = tx & 1
+      const float u1 = (b0 ? s[i][3] : s[i][2]) + __shfl_xor_sync(THA_FULL_MASK, b0 ? s[i][2] : s[i][3], 1);   // and that plus two
+      l[i] = l[i] * corr + ((b1 ? u1 : u0) + __shfl_xor_sync(THA_FULL_MASK, b1 ? u0 : u1, 2));
 #pragma unroll
       for (int c = 0; c < CW; c++) o[i][c] *= corr;
       m[i] = mn;
@@ -179,8 +183,10 @@ __global__ void __launch_bounds__(256) attn_prefill_kernel(const AttnPrefillP p)
 #pragma unroll
   for (int i = 0; i < RI; i++) {
     float L = l[i];
-#pragma unroll
-    for (int off = 8; off > 0; off >>= 1) L += __shfl_xor_sync(THA_FULL_MASK, L, off);
+    L += __shfl_xor_sync(THA_FULL_MASK, L, 2);   // m ^ 8, m ^ 4, m ^ 2, m ^ 1
+    L += __shfl_xor_sync(THA_FULL_MASK, L, 1);
+    L += __shfl_xor_sync(THA_FULL_MASK, L, 8);
+    L += __shfl_xor_sync(THA_FULL_MASK, L, 4);
     const int r = ty + 16 * i;
     if (r >= n) continue;
     const size_t base = (size_t)(row0 + r) * p.dim + h * HS;
