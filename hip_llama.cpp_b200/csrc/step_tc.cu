@@ -365,6 +365,25 @@ __global__ void __launch_bounds__(256) tc_swiglu_split_wide_kernel(const float* 
 // (run.cc:196-209), group quantisation.  gs in {32, 64, 128}; d % gs == 0.
 constexpr int PROMPT_ROWS = 512;   // rows from which a launch fills the machine whatever a thread takes
 constexpr int PREP_MAX_V = 4;   // float4 per thread kept in registers: d <= 4 * 1024 * 4
+// The sum over a row of up to 1024 float4, ss[k] that of float4 threadIdx.x + k blockDim.x: warps of 32 neighbouring float4, then those sums.  The
+// same tree, and bits, for every block width: what follows is quantised, where a last bit may become a step.
+__device__ __forceinline__ float prep_row_sum(const float (&ss)[PREP_MAX_V], int d4, float* red) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+  for (int k = 0; k < PREP_MAX_V; k++) {
+    if (k * (int)blockDim.x >= d4) break;
+    const float w = warp_sum(ss[k]);
+    if (lane == 0 && 32 * (wid + k * nw) < d4) red[wid + k * nw] = w;
+  }
+  __syncthreads();
+  if (wid == 0) {
+    const float t = warp_sum(32 * lane < d4 ? red[lane] : 0.0f);
+    if (lane == 0) red[32] = t;
+  }
+  __syncthreads();
+  return red[32];
+}
+
 __global__ void __launch_bounds__(1024) tc_prep_q8_kernel(float* __restrict__ x, const float* __restrict__ part, int nz,
                                                           long long zstride, const float* __restrict__ emb,
                                                           const int* __restrict__ token, const int* __restrict__ pos,
@@ -389,7 +408,8 @@ __global__ void __launch_bounds__(1024) tc_prep_q8_kernel(float* __restrict__ x,
   }
   const float* er = emb ? emb + (size_t)token[b] * d : nullptr;
   float4 v[PREP_MAX_V];
-  float ss = 0.0f;
+  const bool one = blockDim.x < 1024;   // at most 1024 float4 a row (the launch's rule)
+  float ss = 0.0f, part_ss[PREP_MAX_V] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
   for (int k = 0; k < PREP_MAX_V; k++) {
     const int i = threadIdx.x + k * blockDim.x;
@@ -408,10 +428,11 @@ __global__ void __launch_bounds__(1024) tc_prep_q8_kernel(float* __restrict__ x,
         }
       }
       if ((er || nz) && !gather) reinterpret_cast<float4*>(xr)[i] = v[k];
-      ss = dot4(v[k], v[k], ss);
+      if (one) part_ss[k] = dot4(v[k], v[k], 0.0f);
+      else ss = dot4(v[k], v[k], ss);
     }
   }
-  ss = block_sum(ss, red);
+  ss = one ? prep_row_sum(part_ss, d4, red) : block_sum(ss, red);
   ss /= d; ss += 1e-5f;
   const float ssn = 1.0f / sqrtf(ss);
 #pragma unroll

@@ -57,7 +57,7 @@ def test_q8_rows(heads, hs, hidden):
 
 
 @pytest.mark.parametrize("rows", [2, 511, 512])
-@pytest.mark.parametrize("hidden", [32, 1024, 1056, 2080])
+@pytest.mark.parametrize("hidden", [128, 1024, 1056, 2080])
 def test_quantiser_on_both_sides_of_its_line(rows, hidden):
     """The SwiGLU quantiser takes one float4 a thread below 512 rows and two from there on, the same bits either way: the rows of one call
     against calls of their own (each value differs by the order of partial sums ahead of the quantiser at most)."""
@@ -73,3 +73,18 @@ def test_quantiser_on_both_sides_of_its_line(rows, hidden):
     # the second layer's rows have gone through the first one's SwiGLU and its quantiser: a value in a thousand may fall the other way
     for cache in (lambda e: e.state.key_cache, lambda e: e.state.value_cache):
         assert rel(cache(a)[0, 1, :rows], cache(b)[0, 1, :rows]) < 1e-2
+
+
+@pytest.mark.parametrize("heads,hs,hidden", [(18, 64, 2112), (9, 128, 1024), (32, 128, 512)])
+def test_q8_rows_are_the_same_bits_in_both_forms(heads, hs, hidden):
+    """A prompt of 512 rows against its first 511: the same products and attention tiles, rmsnorm and quantiser in their prompt form and in the other.
+    Both add in the same order, so that no value falls on the other side of a quantiser step."""
+    eng, ck = load_pkg("engine"), load_pkg("checkpoint")
+    cfg = ck.Config(heads * hs, hidden, 3, heads, heads, 96, 520)
+    w = eng.device_random_weights(cfg, q8=True, seed=9, gs=32)
+    toks = np.random.default_rng(10).integers(0, 96, 512).astype(np.int32)
+    a, b = eng.Engine(w, 1, with_att=False), eng.Engine(w, 1, with_att=False)
+    prefill(a, [(0, 0, toks)], 96)
+    prefill(b, [(0, 0, toks[:511])], 96)
+    assert torch.equal(a.state.key_cache[0, :, :511], b.state.key_cache[0, :, :511])
+    assert torch.equal(a.state.value_cache[0, :, :511], b.state.value_cache[0, :, :511])
