@@ -83,6 +83,10 @@ __global__ void hyb_layernorm_kernel(T* __restrict__ out, const float* __restric
 // ------------------------------------------------------------------------------------------------------------------
 constexpr int LT = 64, LK = 16;
 
+// Launched plainly in the fp32 number format, where it carries the step: started under the kernels ahead, its blocks take the slots that
+// those leave over, several on one SM and none on another, and a product that the FMA pipes bound ends with its busiest SM.  Two layers of
+// attention (width 2048, a prompt of 600 and six tokens) 24.4 ms a request with the programmatic launch, 21.9 without; four recurrent
+// ones (width 2048, three prompts of up to 120) 42.8 / 39.5.  (Triggering behind the loop over K instead: 21.8 / 42.9.)
 template <typename TA, typename TW>
 __global__ void __launch_bounds__(256) hyb_linear_kernel(float* __restrict__ C, long long ldc, const TA* __restrict__ A, long long lda,
                                                          const int* __restrict__ a_rows, const TW* __restrict__ W,
@@ -1702,7 +1706,7 @@ extern "C" int tha_hyb_linear_heads(void* stream, int dtype, float* C, long long
     return THA_STATUS_SUCCESS;
   }
   if (dtype == THA_DT_F32)
-    THA_CUDA_OK(launch(hyb_linear_kernel<float, float>, grid, block, 0, s, pdl_enabled() != 0, C, ldc, (const float*)A, lda, none, (const float*)W, 0ll, M, N, K,
+    THA_CUDA_OK(launch(hyb_linear_kernel<float, float>, grid, block, 0, s, false, C, ldc, (const float*)A, lda, none, (const float*)W, 0ll, M, N, K,
                        none, 0, a_hs, w_hs, c_hs));
   else if (a_f32)
     THA_CUDA_OK(launch(hyb_linear_kernel<float, bf16>, grid, block, 0, s, pdl_enabled() != 0, C, ldc, (const float*)A, lda, none, (const bf16*)W, 0ll, M, N, K,
@@ -1749,7 +1753,7 @@ extern "C" int tha_hyb_linear(void* stream, int dtype, float* C, long long ldc, 
     return THA_STATUS_SUCCESS;
   }
   if (dtype == THA_DT_F32)
-    THA_CUDA_OK(launch(hyb_linear_kernel<float, float>, grid, block, 0, s, pdl_enabled() != 0, C, ldc, (const float*)A, lda, a_rows, (const float*)W,
+    THA_CUDA_OK(launch(hyb_linear_kernel<float, float>, grid, block, 0, s, false, C, ldc, (const float*)A, lda, a_rows, (const float*)W,
                        w_group_stride, M, N, K, group_off, n_groups, 0ll, 0ll, 0ll));
   else if (a_f32)
     THA_CUDA_OK(launch(hyb_linear_kernel<float, bf16>, grid, block, 0, s, pdl_enabled() != 0, C, ldc, (const float*)A, lda, a_rows, (const bf16*)W,
