@@ -510,15 +510,20 @@ static cudaLaunchConfig_t bfc_config(cudaLaunchAttribute* attr, int grid, int cl
 // 2 rows, us at 1 / 2 / 4 / 8 ranks: [25 tiles, K 2048] 13.0 / 9.3 / 7.4 / 7.1 (200 CTAs of 8); [36, 1024] 8.7 / 7.2 / 6.5 / 9.5 (288);
 // [49, 1024] 9.0 / 7.5 / 6.9 / 10.1; [96, 2048] 14.8 / 13.2 / 16.4 / 19.0; [250, 2048] 27.7 / 28.7 / 34.1 / 45.0.  A pair of CTAs does not pay
 // for 128-column tiles (100 rows, [36, 1024]: 15.0 / 15.6 / 11.3; [96, 2048]: 21.6 / 22.9).
-static int bfc_ranks(int nt, int items, int kb) {
-  for (int cl = 8; cl > (nt == 128 ? 2 : 1); cl >>= 1)
+// Prompts (more than 128 rows, whose tile gemm_bf16_tile chose for a CTA each): four and eight ranks, from K = 4096 on.  us without / with:
+// [1024 x 4608] 129 rows 18.9 / 12.6, 384 rows 18.8 / 15.2; [2048 x 6144] 129 rows 23.1 / 16.8; at K = 2048 about even ([1024 x 2048] 129 rows
+// 12.4 / 10.7, 384 rows 11.0 / 12.7); at 1024 slower ([1024 x 1024] 256 rows 8.4 / 10.6); pairs slower throughout ([4096 x 4096] 129 rows
+// 18.8 / 22.6, [3088 x 2048] 192 rows 12.6 / 16.6, [2048 x 6144] 256 rows 22.9 / 25.0).
+static int bfc_ranks(int nt, int rows, int items, int kb) {
+  if (rows > 128 && kb < 4096 / BF_BK) return 1;
+  for (int cl = 8; cl > (nt == 128 || rows > 128 ? 2 : 1); cl >>= 1)
     if (kb >= 2 * cl && items * cl <= 200) return cl;
   return 1;
 }
 // Launches the cluster form where its rule takes it; *taken says whether it did.
 template <int NT>
 static int bfc_try(cudaStream_t st, const CUtensorMap* mw, const CUtensorMap& mx, BfP p, bool pdl, bool* taken) {
-  const int cl = bfc_ranks(NT, p.n_items, p.kblocks_total);
+  const int cl = bfc_ranks(NT, p.N, p.n_items, p.kblocks_total);
   *taken = cl > 1;
   if (cl <= 1) return THA_STATUS_SUCCESS;
   p.splits = cl;

@@ -28,3 +28,10 @@ def test_rows(rows, M, K):
     assert bool(((out[:rows, :M].double() - want).abs() <= bound).all())
     assert bool((out[rows] == 7.0).all()) and bool((out[:, M:] == 7.0).all())       # nothing outside the product
     assert lib.c.tha_gemm_check_error() == 0
+
+
+@pytest.mark.parametrize("rows", [129, 384, 512])
+@pytest.mark.parametrize("M,K", [(1024, 4096), (1024, 4032), (2048, 6144), (1000, 4680)])
+def test_prompt_rows_on_both_sides_of_the_line(rows, M, K):
+    """More than 128 rows: clusters of four and eight from K = 4096 on, a CTA a tile below."""
+    test_rows(rows, M, K)
