@@ -481,13 +481,13 @@ static int bf_launch_nt(cudaStream_t st, const CUtensorMap* mw, const CUtensorMa
 // (small tiles pull more through L2 per product), so a large tile pays once it fills the SMs.  Measured, us, in that order: 2100 rows x
 // [4096, 4096] 54 / 59 / 86 / 155; 2825 x [4096, 4096] 92 / 80 / 103 / 190; 2100 x [1024, 4608] 53 / 33 / 30 / 49; 700 x [2048, 2048] 35 / 25 / 19 / 26;
 // 4000 x [12288, 4096] 313 / 312 / 409 / 763.
-BfTile gemm_bf16_tile(int tiles, int N) {
+BfTile gemm_bf16_tile(int tiles, int N, int splits) {
   if (N <= 128) return {N <= 16 ? 16 : (N <= 32 ? 32 : (N <= 64 ? 64 : 128)), 1};
   static const struct { BfTile t; int cost; } form[4] = {{{256, 2}, 100}, {{256, 1}, 56}, {{128, 1}, 41}, {{64, 1}, 39}};
   BfTile best = form[0].t;
   long long least = 0;
   for (int i = 0; i < 4; i++) {
-    const long long items = (long long)ceil_div(tiles, form[i].t.mt) * ceil_div(N, form[i].t.nt);
+    const long long items = (long long)ceil_div(tiles, form[i].t.mt) * ceil_div(N, form[i].t.nt) * splits;
     const long long c = (items + 147) / 148 * form[i].cost;
     if (i == 0 || c < least) { least = c; best = form[i].t; }
   }
@@ -548,7 +548,7 @@ int gemm_bf16_launch(cudaStream_t st, const BfArgs& a, bool pdl) {
   if (swiglu && !gemm_bf16_swiglu_ok(a)) return THA_STATUS_NOT_SUPPORTED;
   int tiles128 = 0;
   for (int i = 0; i < a.n_mats; i++) tiles128 += ceil_div(a.M[i], TC_BM);
-  const BfTile tile = swiglu ? BfTile{256, 1} : gemm_bf16_tile(tiles128, a.N);
+  const BfTile tile = swiglu ? BfTile{256, 1} : gemm_bf16_tile(tiles128, a.N, a.splits < 1 ? 1 : a.splits);
   const int NT = tile.nt, MT = tile.mt;   // SwiGLU: 128-row boxes of each of the two matrices (the kernel itself runs MT = 2)
   CUtensorMap mw[3], mx;
   BfP p = {};

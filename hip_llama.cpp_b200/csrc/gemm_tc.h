@@ -57,7 +57,7 @@ struct BfArgs {
 bool gemm_bf16_swiglu_ok(const BfArgs& a);   // the launch can take the SwiGLU read-out
 bool gemm_bf16_ok(const BfArgs& a);
 struct BfTile { int nt, mt; };
-BfTile gemm_bf16_tile(int tiles, int N);   // output tile: 128 mt weight rows (of `tiles` 128-row tiles) x nt activation rows
+BfTile gemm_bf16_tile(int tiles, int N, int splits);   // output tile: 128 mt weight rows (of `tiles` 128-row tiles) x nt activation rows; K in `splits` shares
 int gemm_bf16_launch(cudaStream_t st, const BfArgs& a, bool pdl);
 
 bool gemm_tc_ok(const TcArgs& a);

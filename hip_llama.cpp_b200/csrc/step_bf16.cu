@@ -237,15 +237,15 @@ static int bf_grow(T** p, size_t* cap, size_t need, Workspace* ws) {
 }
 
 // Split-K factor of one matmul: whole waves of the 148 persistent CTAs, at least two 64-value k-blocks per split, a
-// charge per split for the partials its consumer sums (as step_tc.cu's planner).  Prompt-sized row counts (>= 512: 256-row
-// work items, gemm_bf16.cu gemm_bf16_tile) are compute-bound, and there a split is expensive: it writes and re-reads R x M fp32
+// charge per split for the partials its consumer sums (as step_tc.cu's planner).  Counted in items of 256 columns (and 256 rows
+// from 512 on) whatever tile the product then takes (gemm_bf16_tile): the number of splits is the order of a sum, which rounding to bf16 turns into
+// other logits and now and then another token; the tile is not.  Prompt-sized row counts (>= 512) are compute-bound, and there a split is expensive: it writes and re-reads R x M fp32
 // partials, 4 F / (K BW) of the matmul's own time (F ~ 1.3 PFLOP/s, BW ~ 6.5 TB/s: 0.2 at K = 4096) -- at 2048 rows the old
 // charge picked three splits for wq|wk|wv and the RoPE kernel read 303 MB per layer.
 static int bf_splits(int tiles, int K, int R) {
   const int kb = ceil_div(K, 64);
   const bool big = R >= 512;
-  const BfTile tile = gemm_bf16_tile(tiles, R);
-  const int items1 = ceil_div(tiles, tile.mt) * ceil_div(R, tile.nt);
+  const int items1 = (big ? ceil_div(tiles, 2) : tiles) * ceil_div(R, R <= 128 ? gemm_bf16_tile(tiles, R, 1).nt : 256);
   int best = 1;
   float best_score = -1.0f;
   const float charge = big ? 800.0f / (float)K : 0.012f + 0.25f * (float)R / (float)K / 16.0f;
