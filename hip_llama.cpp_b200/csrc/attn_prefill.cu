@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(256) attn_prefill_kernel(const AttnPrefillP p)
       }
       // partial of the row sum, reduced at the end: thread tx adds the four neighbouring keys 4 m .. 4 m + 3, m = 4 (tx & 3) + (tx >> 2), which four
       // neighbouring threads hold (three exchanges).  The grouping is part of the result's bits: a quantiser behind it turns a last bit into
-      // a step, and with sums in another order 3 of 130 next tokens of quantised prompts changed.
+      // a step, and with sums in another order 3 of 79 next tokens of quantised prompts changed.
       const bool b0 = tx & 1, b1 = tx & 2;
       const float u0 = (b0 ? s[i][1] : s[i][0]) + __shfl_xor_sync(THA_FULL_MASK, b0 ? s[i][0] : s[i][1], 1);   // column j = tx & 1
       const float u1 = (b0 ? s[i][3] : s[i][2]) + __shfl_xor_sync(THA_FULL_MASK, b0 ? s[i][2] : s[i][3], 1);   // and that plus two
