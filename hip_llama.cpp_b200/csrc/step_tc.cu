@@ -363,7 +363,11 @@ __global__ void __launch_bounds__(256) tc_swiglu_split_wide_kernel(const float* 
 // One block per output row (up to 1024 threads, one or more float4 per thread, all loads of a thread independent):
 // x row = embedding row or x + sum of partials (written back), RMSNorm in the reference's order w * (ss * x)
 // (run.cc:196-209), group quantisation.  gs in {32, 64, 128}; d % gs == 0.
-constexpr int PROMPT_ROWS = 512;   // rows from which a launch fills the machine whatever a thread takes
+// Whether `rows` rows of `width` fill the machine whatever a thread takes, so that the row kernels may take their prompt form (more loads a thread,
+// fewer threads a row).  us a prefill with / without it: width 4096, 256 rows 943 / 932 (Q8_0), 512 rows 1754 / 1763 (Q8_0), 2470 / 2489 (fp32);
+// width 768, 512 rows 1738 / 1674, 800 rows 1641 / 1650, 1536 rows 2457 / 2561.
+constexpr int PROMPT_ROWS = 512;
+static bool prompt_form(int rows, int width) { return rows >= PROMPT_ROWS && (long long)rows * width >= 768 * 768; }
 constexpr int PREP_MAX_V = 4;   // float4 per thread kept in registers: d <= 4 * 1024 * 4
 // The sum over a row of up to 1024 float4, ss[k] that of float4 threadIdx.x + k blockDim.x: warps of 32 neighbouring float4, then those sums.  The
 // same tree, and bits, for every block width: what follows is quantised, where a last bit may become a step.
@@ -454,7 +458,7 @@ __global__ void __launch_bounds__(1024) tc_prep_q8_kernel(float* __restrict__ x,
 // V float4 per thread, a block-width apart: src row (attention output), or with h > 0 the SwiGLU of the w1|w3 partials (run.cc:344-347
 // order), quantised per group (int8 row + transposed scales).  One for the few rows of a decode step, where twice the blocks count and the
 // second float4's partials come behind the first's: a step of Llama-2-7B at 1 / 8 / 16 slots takes 2.483 / 2.552 / 2.664 ms with one, 2.533 / 2.610 / 2.713
-// with two.  Two from PROMPT_ROWS on, their loads in flight together.
+// with two.  Two in the prompt form, their loads in flight together.
 // grid (ceil(K / 4 / (256 V)), rows)
 template <int V>
 __global__ void __launch_bounds__(256) tc_quant_split_kernel(const float* __restrict__ src, long long ld, int nz,
@@ -497,9 +501,9 @@ __global__ void __launch_bounds__(256) tc_quant_split_kernel(const float* __rest
   }
   kt_stamp(kt, 6);
 }
-static int quant_split_launch(cudaStream_t st, bool pdl, int rows, const float* src, long long ld, int nz, long long zstride, int h, const int* pos, int K, int gs,
+static int quant_split_launch(cudaStream_t st, bool pdl, int rows, int width, const float* src, long long ld, int nz, long long zstride, int h, const int* pos, int K, int gs,
                               int8_t* oq, float* osT, int ldxs) {
-  const int v = rows >= PROMPT_ROWS ? 2 : 1;
+  const int v = prompt_form(rows, width) ? 2 : 1;
   THA_CUDA_OK(launch(v == 2 ? tc_quant_split_kernel<2> : tc_quant_split_kernel<1>, dim3(ceil_div(K / 4, 256 * v), rows), dim3(256), 0, st, pdl, src, ld, nz, zstride, h, pos,
                      K, gs, oq, osT, ldxs));
   return THA_STATUS_SUCCESS;
@@ -907,7 +911,7 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
   if (prep_threads < 128) prep_threads = 128;
   // prompt rows: up to four float4 per thread, so that several rows share an SM
   const int prompt_threads = d <= 1024 ? 64 : (d <= 4096 ? ceil_div(d / 16, 32) * 32 : 256);
-  if (R >= PROMPT_ROWS && q8 && d / 4 <= 256 * PREP_MAX_V) prep_threads = prompt_threads;
+  if (prompt_form(R, d) && q8 && d / 4 <= 256 * PREP_MAX_V) prep_threads = prompt_threads;
   // tensor parallelism: split counts of every rank's w2 (local hidden sizes may differ), exchange bookkeeping
   int z_w2_of[TP_MAX] = {0};
   const bool tpx = tp && tp->tp > 1;
@@ -945,7 +949,7 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
     if (wq) {
       THA_CUDA_OK(launch(tc_prep_q8_kernel, dim3(rows), dim3(prep_threads), 0, st, pdl, io.x, part, nz, zs, emb, io.token,
                          io.pos, gain, d, gs, sc.xq, sc.xsT, ldxs, gather, tpp));
-    } else if (rows >= PROMPT_ROWS && !gather && !tpp.n) {
+    } else if (prompt_form(rows, d) && !gather && !tpp.n) {
       THA_CUDA_OK(launch(tc_prep_prompt_kernel, dim3(rows), dim3(prompt_threads), 0, st, pdl, io.x, part, nz, zs, emb, io.token, io.pos, gain, d, sc.xh, sc.xl, sc.scale));
     } else {
       THA_CUDA_OK(launch(tc_prep_kernel, dim3(rows), dim3(prep_threads), 0, st, pdl, io.x, part, nz, zs, emb, io.token,
@@ -1016,7 +1020,7 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
     }
     if ((skip & 16) || (wq && io.n_tiles == 0 && !(skip & 2))) {
     } else if (wq)   // prompt rows: runq.c:437 as its own launch
-      THA_TRY_RC(quant_split_launch(st, pdl, R, io.xb, (long long)da, 0, 0LL, 0, io.pos, da, gs, sc.xq, sc.xsT, ldxs));
+      THA_TRY_RC(quant_split_launch(st, pdl, R, d, io.xb, (long long)da, 0, 0LL, 0, io.pos, da, gs, sc.xq, sc.xsT, ldxs));
     {
       const float* W[1] = {wq ? nullptr : w.wo + (size_t)l * d * da};
       const tha_qtensor_t* Q[1] = {wq ? &wq->wo : nullptr};
@@ -1032,8 +1036,8 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
     }
     if (skip & 16) {
     } else if (wq)   // runq.c:457-465: SwiGLU, then quantise hb
-      THA_TRY_RC(quant_split_launch(st, pdl, R, sc.part, (long long)ld_h, pl.z_w13, (long long)R * ld_h, hd, io.pos, hd, gs, sc.hq, sc.hsT, ldxs));
-    else if (R >= PROMPT_ROWS)
+      THA_TRY_RC(quant_split_launch(st, pdl, R, d, sc.part, (long long)ld_h, pl.z_w13, (long long)R * ld_h, hd, io.pos, hd, gs, sc.hq, sc.hsT, ldxs));
+    else if (prompt_form(R, d))
       THA_CUDA_OK(launch(tc_swiglu_split_wide_kernel, dim3(ceil_div(hd, 2048), R), dim3(256), 0, st, pdl, (const float*)sc.part, pl.z_w13,
                          (long long)R * ld_h, ld_h, io.pos, hd, sc.hh, sc.hl));
     else

@@ -59,10 +59,10 @@ def test_q8_rows(heads, hs, hidden):
 @pytest.mark.parametrize("rows", [2, 511, 512])
 @pytest.mark.parametrize("hidden", [128, 1024, 1056, 2080])
 def test_quantiser_on_both_sides_of_its_line(rows, hidden):
-    """The SwiGLU quantiser takes one float4 a thread below 512 rows and two from there on, the same bits either way: the rows of one call
+    """The SwiGLU quantiser takes one float4 a thread below 512 rows of this width and two from there on, the same bits either way: the rows of one call
     against calls of their own (each value differs by the order of partial sums ahead of the quantiser at most)."""
     eng, ck = load_pkg("engine"), load_pkg("checkpoint")
-    cfg = ck.Config(256, hidden, 2, 8, 8, 96, 520)
+    cfg = ck.Config(1152, hidden, 2, 18, 18, 96, 520)
     w = eng.device_random_weights(cfg, q8=True, seed=6, gs=32)
     toks = np.random.default_rng(8).integers(0, 96, rows).astype(np.int32)
     a, b = eng.Engine(w, 1, with_att=False), eng.Engine(w, 1, with_att=False)
@@ -88,3 +88,21 @@ def test_q8_rows_are_the_same_bits_in_both_forms(heads, hs, hidden):
     prefill(b, [(0, 0, toks[:511])], 96)
     assert torch.equal(a.state.key_cache[0, :, :511], b.state.key_cache[0, :, :511])
     assert torch.equal(a.state.value_cache[0, :, :511], b.state.value_cache[0, :, :511])
+
+
+@pytest.mark.parametrize("heads,hs,hidden,lens", [(8, 16, 36, [4700]), (16, 64, 2052, [300, 280])])
+def test_fp32_rows_of_narrow_models(heads, hs, hidden, lens):
+    """Narrow models reach the prompt form of the row kernels with more rows."""
+    eng, ck = load_pkg("engine"), load_pkg("checkpoint")
+    cfg = ck.Config(heads * hs, hidden, 1, heads, heads, 96, max(lens) + 4)
+    w = eng.device_random_weights(cfg, seed=2, std=cfg.dim ** -0.5)
+    e = eng.Engine(w, len(lens), with_att=False)
+    rng = np.random.default_rng(3)
+    seqs = [(i, 0, rng.integers(0, 96, n).astype(np.int32)) for i, n in enumerate(lens)]
+    got = prefill(e, seqs, 96)
+    want, k, v = llama64.forward(cfg, w.t, lambda c, s, l, n: e.state.key_cache[s, l, :n], seqs)
+    assert rel(got, want) < 5e-5        # as test_fp32_rows
+    at = 0
+    for i, n in enumerate(lens):
+        assert rel(e.state.key_cache[i, :, :n], k[at:at + n].transpose(0, 1)) < 3e-5 and rel(e.state.value_cache[i, :, :n], v[at:at + n].transpose(0, 1)) < 3e-5
+        at += n
