@@ -216,8 +216,11 @@ __global__ void __launch_bounds__(256) attn_prefill_kernel(const AttnPrefillP p)
 bool attn_prefill_supported(int head_size, int kv_dim) {
   return (head_size == 16 || head_size == 32 || head_size == 64 || head_size == 128) && kv_dim % 4 == 0;
 }
-// Query rows per tile: 128 where the prompts fill them (two LDS.128 per 16 FMAs, against three for 64 rows), 64 for short ones.
-int attn_prefill_tile_rows(int rows, int n_seqs) { return rows >= 192 * n_seqs ? 128 : 64; }
+// Query rows per tile (the result's bits do not depend on it): 128, with a quarter to a third fewer shared-memory reads per FMA, where the prompts fill
+// such tiles and these (tiles128 x heads of them) leave no SM without one for long, 64 otherwise.  us a prefill with tiles of 64 / 128: 32 heads of
+// 128, one prompt of 256 890 / 933, of 512 1683 / 1754, of 640 2102 / 2144 (Q8_0; 160 tiles of 128), four of 256 4557 / 4529 (fp32; 256); 12 heads
+// of 64, eight prompts of 192 2315 / 2455 (192), one of 512 1776 / 1738 (48).
+int attn_prefill_tile_rows(int rows, int n_seqs, int tiles128, int heads) { return rows >= 192 * n_seqs && tiles128 * heads >= 256 ? 128 : 64; }
 
 // tile_row0 / tile_n: tiles of at most tile_rows (64 or 128) query rows, never across sequences, longest contexts first
 int attn_prefill_launch(cudaStream_t stream, int n_tiles, int n_heads, int n_kv_heads, int head_size, const float* q,

@@ -53,7 +53,7 @@ int attn_prefill_launch(cudaStream_t stream, int n_tiles, int n_heads, int n_kv_
                         float* out, float* out_hi, float* out_lo, const float* kc, const float* vc,
                         long long kv_batch_stride, const int* row_slot, const int* row_pos, const int* tile_row0,
                         const int* tile_n, bool pdl, const KvPaged* pg, int tile_rows);
-int attn_prefill_tile_rows(int rows, int n_seqs);
+int attn_prefill_tile_rows(int rows, int n_seqs, int tiles128, int heads);
 
 __device__ __forceinline__ float st_tf32(float v) { return __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xFFFFE000u); }
 
@@ -1108,7 +1108,9 @@ int step_tc_prefill(cudaStream_t st, Workspace* ws, const tha_config_t& c, const
     R += len[i];
   }
   if (R < 1 || R > (1 << 20)) return THA_STATUS_INVALID_ARG;
-  const int TQ = attn_prefill_tile_rows((int)R, n_seqs);
+  int tiles128 = 0;
+  for (int i = 0; i < n_seqs; i++) tiles128 += ceil_div(len[i], 128);
+  const int TQ = attn_prefill_tile_rows((int)R, n_seqs, tiles128, c.n_heads);
   struct Tile { int row0, n, last; };   // `last`: last position the tile's rows see
   std::vector<Tile> tiles;
   for (int i = 0, r0 = 0; i < n_seqs; r0 += len[i], i++)

@@ -46,3 +46,17 @@ def test_prompts(heads, kv_heads, hs, lens, start):
             other[start:start + n] = False
             assert torch.equal(got[i][:, other], before[which][i][:, other])    # nothing else was written
         at += n
+
+
+TALL = [(64, 64, 16, [500], 3), (64, 8, 32, [193, 383], 0), (32, 32, 64, [1030], 5), (32, 8, 128, [700, 400], 70)]
+
+
+@pytest.mark.parametrize("heads,kv_heads,hs,lens,start", TALL)
+def test_tall_tiles(heads, kv_heads, hs, lens, start):
+    """Many heads, which is where tiles of 128 rows are taken: ragged last tiles, a context in front."""
+    test_prompts(heads, kv_heads, hs, lens, start)
+
+
+@pytest.mark.parametrize("heads,kv_heads,hs,lens,start", TALL)
+def test_tall_tiles_paged(heads, kv_heads, hs, lens, start):
+    test_paged_prompts(heads, kv_heads, hs, lens, start, 16)
