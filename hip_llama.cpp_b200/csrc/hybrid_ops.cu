@@ -1931,6 +1931,10 @@ static bool scan_in_registers() {
   const char* v = getenv("THA_HYB_SCAN");
   return !(v && !strcmp(v, "shared"));
 }
+// The scans below are serial in a portion's tokens, on a few hundred blocks: started under the kernel ahead, their blocks crowd on the SMs that it
+// leaves free, and a long portion runs at the pace of the most crowded one.  So only short portions (decoding) are launched programmatically:
+// four layers of width 1024 with three matrix memories and a delta rule, a prompt of 4096 tokens: 14.1 ms with all kernels launched programmatically, 11.1 with none.
+static bool scan_pdl(const tha_rows_t* rows) { return rows->max_seq_rows <= 64 && pdl_enabled() != 0; }
 // columns per block of the scans: a power of two that divides the thread count
 static int scan_slice(int vdim) { int sc = 1; while (sc < vdim && sc < 16) sc <<= 1; return sc; }
 
@@ -1950,17 +1954,17 @@ extern "C" int tha_hyb_mem_scan(void* stream, int dtype, const tha_mem_t* m, con
                      m->o_i, m->o_f, m->b_i, m->b_f, m->gate_cap));
   if (m->dim <= 256 && scan_in_registers()) {
     const dim3 grid(rows->n_seqs, m->heads, ceil_div(m->vdim, SCW * SCAN_WARPS)), block(32 * SCAN_WARPS);
-    if (m->dim <= 32) THA_CUDA_OK(launch(hyb_mem_scan_warp_kernel<1>, grid, block, 0, s, pdl_enabled() != 0, *m, *rows, *st, proj, ldp, o_raw));
-    else if (m->dim <= 64) THA_CUDA_OK(launch(hyb_mem_scan_warp_kernel<2>, grid, block, 0, s, pdl_enabled() != 0, *m, *rows, *st, proj, ldp, o_raw));
-    else if (m->dim <= 128) THA_CUDA_OK(launch(hyb_mem_scan_warp_kernel<4>, grid, block, 0, s, pdl_enabled() != 0, *m, *rows, *st, proj, ldp, o_raw));
-    else THA_CUDA_OK(launch(hyb_mem_scan_warp_kernel<8>, grid, block, 0, s, pdl_enabled() != 0, *m, *rows, *st, proj, ldp, o_raw));
+    if (m->dim <= 32) THA_CUDA_OK(launch(hyb_mem_scan_warp_kernel<1>, grid, block, 0, s, scan_pdl(rows), *m, *rows, *st, proj, ldp, o_raw));
+    else if (m->dim <= 64) THA_CUDA_OK(launch(hyb_mem_scan_warp_kernel<2>, grid, block, 0, s, scan_pdl(rows), *m, *rows, *st, proj, ldp, o_raw));
+    else if (m->dim <= 128) THA_CUDA_OK(launch(hyb_mem_scan_warp_kernel<4>, grid, block, 0, s, scan_pdl(rows), *m, *rows, *st, proj, ldp, o_raw));
+    else THA_CUDA_OK(launch(hyb_mem_scan_warp_kernel<8>, grid, block, 0, s, scan_pdl(rows), *m, *rows, *st, proj, ldp, o_raw));
   } else {
     const int SC = scan_slice(m->vdim), parts = SCAN_THREADS / SC;
     const size_t smem = sizeof(float) * ((size_t)m->dim * SC + m->dim + 2 * (2 * (size_t)m->dim + SC + 2) + (size_t)parts * SC);
     if (smem > 227 * 1024) return THA_STATUS_NOT_SUPPORTED;
     const dim3 grid(rows->n_seqs, m->heads, ceil_div(m->vdim, SC));
     if (smem > 48 * 1024) THA_CUDA_OK(cudaFuncSetAttribute(hyb_mem_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    THA_CUDA_OK(launch(hyb_mem_scan_kernel, grid, dim3(SCAN_THREADS), smem, s, pdl_enabled() != 0, *m, *rows, *st, proj, ldp, o_raw, SC));
+    THA_CUDA_OK(launch(hyb_mem_scan_kernel, grid, dim3(SCAN_THREADS), smem, s, scan_pdl(rows), *m, *rows, *st, proj, ldp, o_raw, SC));
   }
   const float* gate = proj + m->o_g;
   if (dtype == THA_DT_BF16) return head_gate_launch(s, (bf16*)out, o_raw, rows->n_rows, m->heads, m->vdim, m->eps, m->norm, 1, gate, ldp);
@@ -2019,17 +2023,17 @@ extern "C" int tha_hyb_delta_scan(void* stream, int dtype, const tha_delta_t* d,
   }
   if (d->dim <= 256 && scan_in_registers()) {
     const dim3 grid(rows->n_seqs, d->heads, ceil_div(d->vdim, SCW * SCAN_WARPS)), block(32 * SCAN_WARPS);
-    if (d->dim <= 32) THA_CUDA_OK(launch(hyb_delta_scan_warp_kernel<1>, grid, block, 0, s, pdl_enabled() != 0, *d, *rows, *st, qkv, proj, ldp, dt_raw, o_raw));
-    else if (d->dim <= 64) THA_CUDA_OK(launch(hyb_delta_scan_warp_kernel<2>, grid, block, 0, s, pdl_enabled() != 0, *d, *rows, *st, qkv, proj, ldp, dt_raw, o_raw));
-    else if (d->dim <= 128) THA_CUDA_OK(launch(hyb_delta_scan_warp_kernel<4>, grid, block, 0, s, pdl_enabled() != 0, *d, *rows, *st, qkv, proj, ldp, dt_raw, o_raw));
-    else THA_CUDA_OK(launch(hyb_delta_scan_warp_kernel<8>, grid, block, 0, s, pdl_enabled() != 0, *d, *rows, *st, qkv, proj, ldp, dt_raw, o_raw));
+    if (d->dim <= 32) THA_CUDA_OK(launch(hyb_delta_scan_warp_kernel<1>, grid, block, 0, s, scan_pdl(rows), *d, *rows, *st, qkv, proj, ldp, dt_raw, o_raw));
+    else if (d->dim <= 64) THA_CUDA_OK(launch(hyb_delta_scan_warp_kernel<2>, grid, block, 0, s, scan_pdl(rows), *d, *rows, *st, qkv, proj, ldp, dt_raw, o_raw));
+    else if (d->dim <= 128) THA_CUDA_OK(launch(hyb_delta_scan_warp_kernel<4>, grid, block, 0, s, scan_pdl(rows), *d, *rows, *st, qkv, proj, ldp, dt_raw, o_raw));
+    else THA_CUDA_OK(launch(hyb_delta_scan_warp_kernel<8>, grid, block, 0, s, scan_pdl(rows), *d, *rows, *st, qkv, proj, ldp, dt_raw, o_raw));
   } else {
     const int SC = scan_slice(d->vdim), parts = SCAN_THREADS / SC;
     const size_t smem = sizeof(float) * ((size_t)d->dim * SC + 2 * (3 * (size_t)d->dim + SC + 1) + (size_t)parts * SC + SC);
     if (smem > 227 * 1024) return THA_STATUS_NOT_SUPPORTED;
     const dim3 grid(rows->n_seqs, d->heads, ceil_div(d->vdim, SC));
     if (smem > 48 * 1024) THA_CUDA_OK(cudaFuncSetAttribute(hyb_delta_scan_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    THA_CUDA_OK(launch(hyb_delta_scan_kernel, grid, dim3(SCAN_THREADS), smem, s, pdl_enabled() != 0, *d, *rows, *st, qkv, proj, ldp, dt_raw, o_raw, SC));
+    THA_CUDA_OK(launch(hyb_delta_scan_kernel, grid, dim3(SCAN_THREADS), smem, s, scan_pdl(rows), *d, *rows, *st, qkv, proj, ldp, dt_raw, o_raw, SC));
   }
   const long long ldg = (long long)d->heads * d->vdim;
   if (dtype == THA_DT_BF16) return head_gate_launch(s, (bf16*)out, o_raw, rows->n_rows, d->heads, d->vdim, d->eps, d->norm, 0, gate_raw, ldg);
