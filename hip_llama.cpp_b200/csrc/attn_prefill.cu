@@ -9,7 +9,8 @@
 //   S = Q K^T on an RI x 4 register micro-tile per thread (rows ty + 16 i, keys tx + 16 j, four channels per 128-bit
 //   shared-memory read), running max / sum per row, P staged in shared memory, O += P V.
 // K and V tiles arrive by cp.async, whole rows at a time: V of a tile while its scores are computed, K of the next one under P V -- one
-// buffer each and two barriers per tile.  Bound by fp32 FMA (128 per SM and clock; two LDS.128 per 16 FMAs at RI = 8).
+// buffer each and two barriers per tile.  Bound by fp32 FMA (128 per SM and clock) and the shared-memory reads beside
+// it: per 16 FMAs 1.5 of 128 bits in Q K^T and 1.0 (heads of 128) or 1.5 (of 64) in P V at RI = 8; 2, 1.5 and 2 at RI = 4.
 // The longest tiles start first.
 #include "common.cuh"
 #include "workspace.h"

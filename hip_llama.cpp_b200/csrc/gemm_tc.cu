@@ -501,14 +501,16 @@ int gemm_tc_check_error() {
 // (compiled without FMA contraction).  TMEM holds a ring of group accumulators so the MMAs of the next groups
 // overlap the scaling of the previous one; shared memory holds a ring of [W 128x128 | X NTx128] int8 slots.
 //   warp 0  TMA producer (weights first: they do not depend on the previous kernel)   warps 1, 3  MMA issuers
-//   warp 2  TMEM allocation     warps 4-7  epilogue: one warp per 32-lane TMEM quarter, thread = weight row
+//   warp 2  TMEM allocation     warps 4 on  epilogue: one, two or four warps per 32-lane TMEM quarter (q8i_epi_warps), thread = weight row x its
+//   warp's share of the columns
 // Every tcgen05 instruction costs its issuing thread a few hundred cycles whatever its size (measured: ~300 per
 // kind::i8 MMA, ~200 per tcgen05.ld, ~450 per wait::ld), so the epilogue reads 128 accumulator columns -- 128/NT
 // consecutive groups, laid out back to back in TMEM -- per round trip.
 // Epilogue warps: four (one per 32-lane TMEM quarter) for narrow column tiles, eight at NT = 32, SIXTEEN at NT = 64 -- four per quarter,
 // each with a quarter of the tile's columns.  A slot of 16 KB of weights leaves 64 KB of int32 group sums in TMEM; a warp's TMEM reads and the
 // wait for them take several hundred cycles (four warps reading: 171 B a cycle, sixteen: 440), and only other warps of the same scheduler can
-// fill them.  930 rows x 12288 x 4096: 317 us with eight warps, 293 with sixteen and two scaling products to an instruction; 64 rows 38.0 -> 36.2.
+// fill them.  930 rows x 12288 x 4096: 317 us with eight warps, 293 with sixteen and two scaling products to an instruction; 64 rows 38.0 -> 36.2.  At 32 columns
+// eight warps stay, with I2F and packed products: 17 to 32 rows x 12288 x 4096 25.4 -> 23.6 us, x 4096 x 11008 49.1 -> 46.1.
 // (mma.sync with the sums in registers: 329 us, and 29.8 against 19.4 at one row.)
 __host__ __device__ constexpr int q8i_epi_warps(int nt) { return nt >= 64 ? 16 : (nt >= 32 ? 8 : 4); }
 __host__ __device__ constexpr int q8i_threads(int nt) { return 128 + 32 * q8i_epi_warps(nt); }
@@ -593,7 +595,7 @@ gemm_q8i_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant__
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::NSLOT * S::SLOT);
   uint64_t* full = bars;                 // slot landed (W + X bytes)
   uint64_t* mdone = full + S::NSLOT;     // the MMAs of a slot have completed: slot reusable, accumulators readable
-  uint64_t* aempty = mdone + S::NMD;     // a slot's accumulators have been read out by the 4 epilogue warps
+  uint64_t* aempty = mdone + S::NMD;     // a slot's accumulators have been read out by all epilogue warps
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(aempty + S::NACC_MAX);
   int* abort_flag = reinterpret_cast<int*>(tmem_slot + 1);
 
@@ -721,7 +723,7 @@ gemm_q8i_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant__
       }
     }
   } else if (warp >= 4) {
-    // ===== epilogue: thread = weight row (TMEM lane) x CH columns (all NT, or one half of them: q8i_epi_warps)
+    // ===== epilogue: thread = weight row (TMEM lane) x CH columns (all NT, a half or a quarter of them: q8i_epi_warps)
     constexpr int EW = q8i_epi_warps(NT), ET = 32 * EW, CH = NT * 4 / EW;
     const int q = warp & 3;
     const int c0 = ((warp - 4) >> 2) * CH;       // first column of this warp's share

@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(1024) tc_prep_q8_kernel(float* __restrict__ x,
 
 // V float4 per thread, a block-width apart: src row (attention output), or with h > 0 the SwiGLU of the w1|w3 partials (run.cc:344-347
 // order), quantised per group (int8 row + transposed scales).  One for the few rows of a decode step, where twice the blocks count and the
-// second float4's partials come behind the first's: a step of Llama-2-7B at 1 / 8 / 16 slots takes 2.483 / 2.552 / 2.664 ms with one, 2.533 / 2.610 / 2.713
+// second float4's partials come behind the first's: a step of Llama-2-7B at 1 / 8 / 16 slots takes 2.476 / 2.547 / 2.656 ms with one, 2.533 / 2.610 / 2.713
 // with two.  Two in the prompt form, their loads in flight together.
 // grid (ceil(K / 4 / (256 V)), rows)
 template <int V>
