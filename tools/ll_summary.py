@@ -1,4 +1,4 @@
-"""Summarise an ncu launch list (long-format csv of tools/gpu_ll*.sh: one row per launch and metric):
+"""Summarise an ncu launch list (long-format csv of ncu --csv: one row per launch and metric):
    python tools/ll_summary.py file.csv [launches_per_step]
 Per kernel (name, grid): launches, average duration, DRAM bytes read / written per launch, share of the summed time."""
 import collections
