@@ -487,439 +487,6 @@ int gemm_tc_check_error() {
   return h;
 }
 
-// =====================================================================================================
-// Q8_0 x Q8_0 on the INT8 tensor cores: runq.c:317-342 evaluated exactly as written.
-//
-//   out[n, m] = sum_g  (float)( sum_{k in g} Wq[m,k] * Xq[n,k] )  *  Ws[m,g]  *  Xs[n,g]        (groups ascending)
-//
-// The inner integer sum of a group is ONE accumulator pass of tcgen05.mma.kind::i8 (int8 x int8 -> int32, exact;
-// K = 32 per instruction, gs/32 instructions per group) with BOTH operands read straight from the TMA-written
-// shared-memory tiles: no conversion warps, weights cross HBM and shared memory as the int8 bytes of the file.
-// Each finished group accumulator [128 rows x NT columns] is pulled out of TMEM by the epilogue warps
-// (thread = weight row), converted exactly, scaled by the row's weight scale and the column's activation scale in
-// the reference's order and added in fp32 -- so without split-K the result is bit-identical to runq.c's loop
-// (compiled without FMA contraction).  TMEM holds a ring of group accumulators so the MMAs of the next groups
-// overlap the scaling of the previous one; shared memory holds a ring of [W 128x128 | X NTx128] int8 slots.
-//   warp 0  TMA producer (weights first: they do not depend on the previous kernel)   warps 1, 3  MMA issuers
-//   warp 2  TMEM allocation     warps 4 on  epilogue: one, two or four warps per 32-lane TMEM quarter (q8i_epi_warps), thread = weight row x its
-//   warp's share of the columns
-// Every tcgen05 instruction costs its issuing thread a few hundred cycles whatever its size (measured: ~300 per
-// kind::i8 MMA, ~200 per tcgen05.ld, ~450 per wait::ld), so the epilogue reads 128 accumulator columns -- 128/NT
-// consecutive groups, laid out back to back in TMEM -- per round trip.
-// Epilogue warps: four (one per 32-lane TMEM quarter) for narrow column tiles, eight at NT = 32, SIXTEEN at NT = 64 -- four per quarter,
-// each with a quarter of the tile's columns.  A slot of 16 KB of weights leaves 64 KB of int32 group sums in TMEM; a warp's TMEM reads and the
-// wait for them take several hundred cycles (four warps reading: 171 B a cycle, sixteen: 440), and only other warps of the same scheduler can
-// fill them.  930 rows x 12288 x 4096: 317 us with eight warps, 293 with sixteen and two scaling products to an instruction; 64 rows 38.0 -> 36.2.  At 32 columns
-// eight warps stay, with I2F and packed products: 17 to 32 rows x 12288 x 4096 25.4 -> 23.6 us, x 4096 x 11008 49.1 -> 46.1.
-// (mma.sync with the sums in registers: 329 us, and 29.8 against 19.4 at one row.)
-__host__ __device__ constexpr int q8i_epi_warps(int nt) { return nt >= 64 ? 16 : (nt >= 32 ? 8 : 4); }
-__host__ __device__ constexpr int q8i_threads(int nt) { return 128 + 32 * q8i_epi_warps(nt); }
-
-struct Q8iP {
-  int M[3]; int tiles[3]; int out_off[3];
-  const float* S[3];                 // weight group scales [M, ngrp]
-  const float* xsT; int ldxs;        // activation group scales, transposed: xsT[g * ldxs + n]
-  int K, N, ny, gs, ngrp;
-  int slots_total, slots_per_split;  // ring slots of 128 values
-  float* out; long long ldo; long long zstride;
-  int* error_flag;
-  int nring;                         // shared-memory ring slots in use
-  int splits, n_items;               // work items = (tiles of all matrices) x column tiles x splits
-};
-
-template <int NT>
-struct Q8iSmem {
-  static constexpr int W_BYTES = TC_BM * 128, X_BYTES = NT * 128, SLOT = W_BYTES + X_BYTES;
-  static constexpr int NSLOT_RAW = (TC_SMEM_LIMIT - 3072) / SLOT;
-  static constexpr int NSLOT = NSLOT_RAW > 10 ? 10 : NSLOT_RAW;
-  // One tcgen05.commit per STAGE of SPC slots (a commit costs the issuing thread a few hundred cycles; the same
-  // barrier releases the stage's shared-memory slots to the producer and hands its accumulators to the epilogue).
-  static constexpr int SPC = 1;
-  // MMA-issuing warps: a tcgen05.mma.kind::i8 costs its issuing thread ~300 cycles whatever its size (measured), so
-  // the slots are dealt round-robin to two issuers (each owns whole groups: accumulation order is untouched).  The number
-  // of accumulator stages is a multiple of the issuers, so a stage is always refilled by the same thread (a waiter
-  // that skipped a phase of the release barrier would read its parity wrongly).
-  static constexpr int NISS = 2;
-  static constexpr int TMEM_COLS = 512;
-  static constexpr int NMD = 64;                  // commit barriers (more than the slots that can be in flight)
-  static constexpr int NACC_MAX = 32;
-  static constexpr int TOTAL = NSLOT * SLOT + 1024 + (NSLOT + NMD + NACC_MAX) * 8 + 64;
-  static_assert(TOTAL <= TC_SMEM_LIMIT, "shared memory overflow");
-  static_assert(NSLOT + NACC_MAX + 1 <= NMD, "commit barrier ring too short");
-};
-
-__host__ __device__ constexpr uint32_t q8i_idesc(int nt) {   // kind::i8: D = S32 (2), A = B = signed 8-bit (1), K-major, M = 128
-  return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nt >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
-}
-__device__ __forceinline__ void q8i_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void tc_tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]) : "r"(taddr));
-}
-
-__device__ __forceinline__ void tc_tmem_ld64(uint32_t taddr, uint32_t* v) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x64.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47, %48, %49, %50, %51, %52, %53, %54, %55, %56, %57, %58, %59, %60, %61, %62, %63}, [%64];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31]), "=r"(v[32]), "=r"(v[33]), "=r"(v[34]), "=r"(v[35]), "=r"(v[36]), "=r"(v[37]), "=r"(v[38]), "=r"(v[39]), "=r"(v[40]), "=r"(v[41]), "=r"(v[42]), "=r"(v[43]), "=r"(v[44]), "=r"(v[45]), "=r"(v[46]), "=r"(v[47]), "=r"(v[48]), "=r"(v[49]), "=r"(v[50]), "=r"(v[51]), "=r"(v[52]), "=r"(v[53]), "=r"(v[54]), "=r"(v[55]), "=r"(v[56]), "=r"(v[57]), "=r"(v[58]), "=r"(v[59]), "=r"(v[60]), "=r"(v[61]), "=r"(v[62]), "=r"(v[63]) : "r"(taddr));
-}
-
-// (f0 * ws * x0, f1 * ws * x1), each product rounded by itself; two lanes to an instruction save issue slots (the sums stay scalar: a packed add
-// after a packed multiply is contracted)
-__device__ __forceinline__ void q8i_scale2(float f0, float f1, float ws, float x0, float x1, float& p0, float& p1) {
-  asm("{\n\t.reg .b64 f, w, x;\n\t"
-      "mov.b64 f, {%2, %3};\n\tmov.b64 w, {%4, %4};\n\tmov.b64 x, {%5, %6};\n\t"
-      "mul.rn.f32x2 f, f, w;\n\tmul.rn.f32x2 f, f, x;\n\t"
-      "mov.b64 {%0, %1}, f;\n\t}"
-      : "=f"(p0), "=f"(p1) : "f"(f0), "f"(f1), "f"(ws), "f"(x0), "f"(x1));
-}
-
-// Persistent: a CTA walks the work items (weight tile, column tile, K split) blockIdx.x, blockIdx.x + gridDim.x, ...
-// with ONE running slot counter, so the TMA ring, the MMA issuers and the epilogue flow from one item into the next
-// without draining (a fresh CTA per item paid ~3 us of ramp for ~6 us of streaming).  Every item is padded to a whole
-// number of TMEM read batches with slots past the end of K: TMA zero-fills them, their integer sums are 0 and the
-// epilogue skips their groups.
-template <int NT>
-__global__ void __launch_bounds__(q8i_threads(NT), 1)
-gemm_q8i_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant__ CUtensorMap mw1,
-                const __grid_constant__ CUtensorMap mw2, const __grid_constant__ CUtensorMap mx, const Q8iP p) {
-  using S = Q8iSmem<NT>;
-  extern __shared__ unsigned char tc_smem_raw[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
-  const int nring = p.nring;             // ring slots actually used (the activation scales take the rest)
-  float* xs_sm = reinterpret_cast<float*>(smem + nring * S::SLOT);   // [groups of one item][NT]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::NSLOT * S::SLOT);
-  uint64_t* full = bars;                 // slot landed (W + X bytes)
-  uint64_t* mdone = full + S::NSLOT;     // the MMAs of a slot have completed: slot reusable, accumulators readable
-  uint64_t* aempty = mdone + S::NMD;     // a slot's accumulators have been read out by all epilogue warps
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(aempty + S::NACC_MAX);
-  int* abort_flag = reinterpret_cast<int*>(tmem_slot + 1);
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int mpg = p.gs >> 5;                     // MMAs per group
-  const int gps = 128 / p.gs;                    // groups per slot
-  const int nacc = S::TMEM_COLS / (gps * NT);    // accumulator stages (slots) in TMEM: 4 .. 32, a power of two
-  const int nacc_sh = 31 - __clz(nacc);
-  constexpr int LG = 128 / NT;                   // groups per TMEM read (128 columns)
-  const int sb = LG / gps;                       // slots per TMEM read batch (NT <= gs: at least 1)
-  const int tiles01 = p.tiles[0] + p.tiles[1];
-  __shared__ int kt_q8_s;
-
-  // work item -> (matrix, row0, n0, first slot, real slots, padded slots, real groups)
-  struct Item { int mat, row0, n0, slot0, nslots, npad, ng; };
-  auto item_of = [&](int it) -> Item {
-    Item w;
-    const int z = it % p.splits;
-    const int t = it / p.splits;
-    int tile = t / p.ny;
-    w.n0 = (t - tile * p.ny) * NT;
-    w.mat = 0;
-    if (tile >= p.tiles[0]) { w.mat = 1; if (tile >= tiles01) { w.mat = 2; tile -= tiles01; } else tile -= p.tiles[0]; }
-    w.row0 = tile * TC_BM;
-    w.slot0 = z * p.slots_per_split;
-    w.nslots = p.slots_total - w.slot0;
-    if (w.nslots > p.slots_per_split) w.nslots = p.slots_per_split;
-    w.npad = ((w.nslots + sb - 1) / sb) * sb;
-    const int g0 = w.slot0 * gps;
-    w.ng = p.ngrp - g0;
-    if (w.ng > w.nslots * gps) w.ng = w.nslots * gps;
-    return w;
-  };
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < S::NSLOT; s++) tc_mbar_init(&full[s], 1);
-    for (int b = 0; b < S::NMD; b++) tc_mbar_init(&mdone[b], 1);
-    for (int b = 0; b < S::NACC_MAX; b++) tc_mbar_init(&aempty[b], q8i_epi_warps(NT));
-    *abort_flag = 0;
-    kt_q8_s = kt_begin((unsigned long long)KT_GEMM_Q8 | ((unsigned long long)p.splits << 16) | ((unsigned long long)p.n_items << 32));
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  }
-  if (warp == 0 && lane == 0) {
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&mw0) : "memory");
-    if (p.tiles[1]) asm volatile("prefetch.tensormap [%0];" ::"l"(&mw1) : "memory");
-    if (p.tiles[2]) asm volatile("prefetch.tensormap [%0];" ::"l"(&mw2) : "memory");
-    asm volatile("prefetch.tensormap [%0];" ::"l"(&mx) : "memory");
-  }
-  if (warp == 2) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem_u32(tmem_slot)), "r"(S::TMEM_COLS));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = *tmem_slot;
-  const int kt = kt_q8_s;
-
-  if (warp == 0) {
-    // ===== TMA producer
-    if (lane == 0) {
-      uint64_t pol_w;
-      asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol_w));
-      int jb = 0;                                   // running slot counter at the start of the item
-      bool ok = true;
-      for (int it = blockIdx.x; it < p.n_items && ok; it += gridDim.x) {
-        const Item w = item_of(it);
-        const CUtensorMap* mw = (w.mat == 0) ? &mw0 : (w.mat == 1 ? &mw1 : &mw2);
-        int j = 0;
-        if (jb == 0) {
-          // the first ring of weight tiles goes out before the dependency wait (transaction bytes may land before
-          // the matching expect_tx: the phase cannot complete until the arrival below)
-          const int pre = w.npad < nring ? w.npad : nring;
-          for (; j < pre; j++) tc_tma_2d_hint(smem + j * S::SLOT, mw, (w.slot0 + j) * 32, w.row0, &full[j], pol_w);
-          pdl_wait();
-          kt_stamp(kt, 1);
-          for (j = 0; j < pre; j++) {
-            tc_mbar_expect_tx(&full[j], S::SLOT);
-            tc_tma_2d(smem + j * S::SLOT + S::W_BYTES, &mx, (w.slot0 + j) * 32, w.n0, &full[j]);
-          }
-        }
-        for (; j < w.npad; j++) {
-          const int jg = jb + j, s = jg % nring;
-          if (jg >= nring) {
-            const int st = jg - nring;              // the slot use whose MMAs must have completed
-            if (!tc_mbar_wait(&mdone[st % S::NMD], (st / S::NMD) & 1u, abort_flag)) { ok = false; break; }
-          }
-          tc_mbar_expect_tx(&full[s], S::SLOT);
-          tc_tma_2d_hint(smem + s * S::SLOT, mw, (w.slot0 + j) * 32, w.row0, &full[s], pol_w);
-          tc_tma_2d(smem + s * S::SLOT + S::W_BYTES, &mx, (w.slot0 + j) * 32, w.n0, &full[s]);
-        }
-        jb += w.npad;
-      }
-    }
-  } else if (warp == 1 || warp == 3) {
-    // ===== MMA issuers (warps 1 and 3): issuer i takes the slots with running index = i (mod 2)
-    if (lane == 0) {
-      constexpr uint32_t idesc = q8i_idesc(NT);
-      const int mpg_sh = 31 - __clz(mpg), gps_sh = 31 - __clz(gps), nacc_mask = nacc - 1;   // all powers of two
-      const int me = warp >> 1;
-      int jb = 0;
-      bool ok = true;
-      for (int it = blockIdx.x; it < p.n_items && ok; it += gridDim.x) {
-        const Item w = item_of(it);
-        for (int j = (jb + me) & 1; j < w.npad; j += 2) {
-          const int jg = jb + j, s = jg % nring;
-          if (jg >= nacc) {                         // the accumulator stage must have been drained
-            if (!tc_mbar_wait(&aempty[jg & nacc_mask], ((jg >> nacc_sh) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
-          }
-          if (!tc_mbar_wait(&full[s], (jg / nring) & 1u, abort_flag)) { ok = false; break; }
-          if (jg == 0) kt_stamp(kt, 2);
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint64_t adesc = tc_smem_desc(tc_smem_u32(smem + s * S::SLOT));
-          const uint64_t bdesc = tc_smem_desc(tc_smem_u32(smem + s * S::SLOT + S::W_BYTES));
-          const uint32_t acc0 = tmem_base + (uint32_t)(((jg & nacc_mask) << gps_sh) * NT);
-#pragma unroll
-          for (int sub = 0; sub < 4; sub++)       // past the end of K the tiles are zero-filled: always four MMAs
-            q8i_mma(acc0 + (uint32_t)((sub >> mpg_sh) * NT), adesc + (uint64_t)(sub * 2), bdesc + (uint64_t)(sub * 2), idesc,
-                    (uint32_t)((sub & (mpg - 1)) != 0));
-          tc_commit(&mdone[jg % S::NMD]);
-        }
-        if (jb == 0 && warp == 1) kt_stamp(kt, 3);
-        jb += w.npad;
-      }
-    }
-  } else if (warp >= 4) {
-    // ===== epilogue: thread = weight row (TMEM lane) x CH columns (all NT, a half or a quarter of them: q8i_epi_warps)
-    constexpr int EW = q8i_epi_warps(NT), ET = 32 * EW, CH = NT * 4 / EW;
-    const int q = warp & 3;
-    const int c0 = ((warp - 4) >> 2) * CH;       // first column of this warp's share
-    const int r = q * 32 + lane;
-    const uint32_t tq = tmem_base + ((uint32_t)(q * 32) << 16);
-    const int gps_sh = 31 - __clz(gps);
-    pdl_trigger();
-    pdl_wait();                                     // the activation scales come from the previous kernel
-    int jb = 0;
-    bool ok = true;
-    uint32_t v[LG * CH];
-    for (int it = blockIdx.x; it < p.n_items && ok; it += gridDim.x) {
-      const Item w = item_of(it);
-      const int ng = w.ng;
-      const int row = w.row0 + r;
-      const bool row_ok = row < p.M[w.mat];
-      const int g0 = w.slot0 * gps;
-      const float* srow = p.S[w.mat] + (size_t)(row_ok ? row : p.M[w.mat] - 1) * p.ngrp + g0;
-      float acc[CH];
-#pragma unroll
-      for (int c = 0; c < CH; c++) acc[c] = 0.0f;
-      // Weight scales: this thread's row, four groups per 128-bit load, requested two to three chunks (8-12 groups,
-      // well over a thousand cycles) before their use -- with ~200 KB of the SM's memory carved out as shared, L1
-      // keeps next to nothing and every one of these loads is an L2 round trip.
-      const bool ws_vec = ((reinterpret_cast<uintptr_t>(srow) & 15u) == 0) && (p.ngrp % 4 == 0);
-      auto load_ws4 = [&](int chunk) -> float4 {
-        const int g = 4 * chunk;
-        float4 r4 = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (g + 3 < ng && ws_vec) return __ldg(reinterpret_cast<const float4*>(srow + g));
-        if (g < ng) r4.x = __ldg(srow + g);
-        if (g + 1 < ng) r4.y = __ldg(srow + g + 1);
-        if (g + 2 < ng) r4.z = __ldg(srow + g + 2);
-        if (g + 3 < ng) r4.w = __ldg(srow + g + 3);
-        return r4;
-      };
-      float4 ws_cur = load_ws4(0), ws_n1 = load_ws4(1), ws_n2 = load_ws4(2);
-      {  // the activation scales of this item's K range -> shared memory (NT floats per group)
-        asm volatile("bar.sync 1, %0;" ::"n"(ET) : "memory");   // the epilogue warps: everybody is done with the previous item's
-        const float* src = p.xsT + (size_t)g0 * p.ldxs + w.n0;
-        const int t = threadIdx.x - 128;            // 0..ET-1
-        for (int i = t; i < ng * (NT / 4); i += ET) {
-          const int g = i / (NT / 4), c4 = i - g * (NT / 4);
-          reinterpret_cast<float4*>(xs_sm)[i] = __ldg(reinterpret_cast<const float4*>(src + (size_t)g * p.ldxs) + c4);
-        }
-        asm volatile("bar.sync 1, %0;" ::"n"(ET) : "memory");
-      }
-      for (int bi = 0; bi * sb < w.npad && ok; bi++) {
-        // the batch's slots: the last slot of each issuer covers the earlier ones (an issuer's commits complete in order)
-        const int s_first = jb + bi * sb, s_last = s_first + sb - 1;
-        int wok = 1;
-        if (lane == 0) {
-          wok = tc_mbar_wait(&mdone[s_last % S::NMD], (s_last / S::NMD) & 1u, abort_flag) ? 1 : 0;
-          if (wok && sb > 1) wok = tc_mbar_wait(&mdone[(s_last - 1) % S::NMD], ((s_last - 1) / S::NMD) & 1u, abort_flag) ? 1 : 0;
-        }
-        ok = __shfl_sync(THA_FULL_MASK, wok, 0) != 0;
-        if (!ok) break;
-        if (jb == 0 && bi == 0 && threadIdx.x == 128) kt_stamp(kt, 4);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t ta = tq + (uint32_t)(((s_first & (nacc - 1)) << gps_sh) * NT);
-        if (EW == 4) {
-          tc_tmem_ld64(ta, v);
-          tc_tmem_ld64(ta + 64, v + 64);
-        } else {   // this warp's CH columns of each of the LG groups, 16 at a time
-#pragma unroll
-          for (int b = 0; b < LG; b++)
-#pragma unroll
-            for (int c = 0; c < CH; c += 16)
-              tc_tmem_ld16(ta + (uint32_t)(b * NT + c0 + c), *reinterpret_cast<uint32_t(*)[16]>(v + b * CH + c));
-        }
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        __syncwarp();
-        if (lane == 0)
-          for (int sl = s_first; sl <= s_last; sl++) tc_mbar_arrive(&aempty[sl & (nacc - 1)]);
-#pragma unroll
-        for (int b = 0; b < LG; b++) {
-          const int gi = bi * LG + b;
-          if (gi < ng) {
-            if ((gi & 3) == 0 && gi > 0) { ws_cur = ws_n1; ws_n1 = ws_n2; ws_n2 = load_ws4((gi >> 2) + 2); }
-            const int wi = gi & 3;
-            const float ws = wi == 0 ? ws_cur.x : (wi == 1 ? ws_cur.y : (wi == 2 ? ws_cur.z : ws_cur.w));
-#pragma unroll
-            for (int c = 0; c < CH; c += 4) {
-              const float4 t = *reinterpret_cast<const float4*>(xs_sm + gi * NT + c0 + c);   // same address in every lane: a broadcast
-              const float xs[4] = {t.x, t.y, t.z, t.w};
-              // runq.c:334 in its order, no contraction
-              if (EW == 4) {
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                  // |group sum| <= 128 * 127 * 127 < 2^22: 1.5 * 2^23 + i is exact in fp32, so this IS (float)i -- two
-                  // full-rate instructions instead of a half-rate I2F: with one warp per scheduler latency counts, not issue slots
-                  const float f = __int_as_float(0x4B400000 + (int)v[b * CH + c + e]) - 12582912.0f;
-                  acc[c + e] = __fadd_rn(acc[c + e], __fmul_rn(__fmul_rn(f, ws), xs[e]));
-                }
-              } else {
-#pragma unroll
-                for (int e = 0; e < 4; e += 2) {
-                  float p0, p1;
-                  q8i_scale2(__int2float_rn((int)v[b * CH + c + e]), __int2float_rn((int)v[b * CH + c + e + 1]), ws, xs[e], xs[e + 1], p0, p1);
-                  acc[c + e] = __fadd_rn(acc[c + e], p0);
-                  acc[c + e + 1] = __fadd_rn(acc[c + e + 1], p1);
-                }
-              }
-            }
-          }
-        }
-      }
-      float* outz = p.out + (size_t)(it % p.splits) * p.zstride + p.out_off[w.mat] + row;
-      if (ok && row_ok) {
-#pragma unroll
-        for (int c = 0; c < CH; c++) {
-          const int n = w.n0 + c0 + c;
-          if (n < p.N) outz[(size_t)n * p.ldo] = acc[c];
-        }
-      }
-      if (jb == 0 && threadIdx.x == 128) kt_stamp(kt, 5);
-      jb += w.npad;
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) kt_stamp(kt, 6);
-  if (warp == 2) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(S::TMEM_COLS));
-  }
-  if (threadIdx.x == 0 && *abort_flag && p.error_flag) *((volatile int*)p.error_flag) = 1;
-}
-
-bool gemm_q8i_ok(const Q8iArgs& a) {
-  if (a.gs != 32 && a.gs != 64 && a.gs != 128) return false;
-  if (a.K % a.gs || a.K < 128 || a.K % 16 || a.N < 1 || a.n_mats < 1 || a.n_mats > 3 || !a.Xq || !a.xsT || !a.out) return false;
-  if ((reinterpret_cast<uintptr_t>(a.Xq) & 15u) || (reinterpret_cast<uintptr_t>(a.xsT) & 15u) || a.ldxs % 4) return false;
-  for (int i = 0; i < a.n_mats; i++)
-    if (!a.Wq[i] || !a.Ws[i] || (reinterpret_cast<uintptr_t>(a.Wq[i]) & 15u) || a.M[i] < 1) return false;
-  return true;
-}
-
-int gemm_q8i_pick_nt(int N, int gs) {   // a slot's groups must fit one 128-column TMEM read: NT <= gs
-  const int nt = N <= 16 ? 16 : (N <= 32 ? 32 : 64);
-  return nt > gs ? gs : nt;
-}
-
-template <int NT>
-static int q8i_launch_nt(cudaStream_t st, const CUtensorMap* mw, const CUtensorMap& mx, const Q8iP& p, dim3 grid, bool pdl) {
-  using S = Q8iSmem<NT>;
-  auto k = gemm_q8i_kernel<NT>;
-  THA_CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL));
-  THA_CUDA_OK(launch(k, grid, dim3(q8i_threads(NT)), (size_t)S::TOTAL, st, pdl, mw[0], mw[1], mw[2], mx, p));
-  return THA_STATUS_SUCCESS;
-}
-
-int gemm_q8i_launch(cudaStream_t st, const Q8iArgs& a, bool pdl) {
-  if (!gemm_q8i_ok(a)) return THA_STATUS_INVALID_ARG;
-  const int NT = gemm_q8i_pick_nt(a.N, a.gs);
-  if (a.ldxs < ceil_div(a.N, NT) * NT) return THA_STATUS_INVALID_ARG;   // a column tile reads NT scales per group
-  CUtensorMap mw[3], mx;
-  Q8iP p = {};
-  int tiles = 0;
-  for (int i = 0; i < 3; i++) {
-    if (i < a.n_mats) {
-      THA_TRY_RC(tc_map(a.Wq[i], a.M[i], a.K, a.K, TC_BM, &mw[i], 1));
-      p.M[i] = a.M[i]; p.tiles[i] = ceil_div(a.M[i], TC_BM); p.out_off[i] = a.out_off[i]; p.S[i] = a.Ws[i];
-    } else {
-      mw[i] = mw[0];
-    }
-    tiles += p.tiles[i];
-  }
-  THA_TRY_RC(tc_map(a.Xq, a.N, a.K, a.K, NT, &mx, 1));
-  p.xsT = a.xsT; p.ldxs = a.ldxs; p.K = a.K; p.N = a.N; p.gs = a.gs; p.ngrp = a.K / a.gs;
-  p.slots_total = ceil_div(a.K, 128);
-  const int splits = a.splits < 1 ? 1 : a.splits;
-  p.slots_per_split = ceil_div(p.slots_total, splits);
-  if (ceil_div(p.slots_total, p.slots_per_split) != splits) return THA_STATUS_INVALID_ARG;
-  p.out = a.out; p.ldo = a.ldo; p.zstride = a.zstride;
-  THA_TRY_RC(gemm_tc_init(&p.error_flag));
-  {  // the activation scales of one item sit behind the ring: [groups per (padded) split][NT] floats
-    const int slot_bytes = TC_BM * 128 + NT * 128;
-    const int nslot_max = (TC_SMEM_LIMIT - 3072) / slot_bytes > 10 ? 10 : (TC_SMEM_LIMIT - 3072) / slot_bytes;
-    const int sb = a.gs / NT;
-    const int xs_bytes = ceil_div(p.slots_per_split, sb) * sb * (128 / a.gs) * NT * 4;
-    p.nring = nslot_max - ceil_div(xs_bytes, slot_bytes);
-    if (p.nring < 3) return THA_STATUS_NOT_SUPPORTED;
-  }
-  p.ny = ceil_div(a.N, NT);
-  p.splits = splits;
-  p.n_items = tiles * p.ny * splits;
-  const int sms = sm_budget();
-  dim3 grid(p.n_items < sms ? p.n_items : sms, 1, 1);
-  switch (NT) {
-    case 16: return q8i_launch_nt<16>(st, mw, mx, p, grid, pdl);
-    case 32: return q8i_launch_nt<32>(st, mw, mx, p, grid, pdl);
-    default: return q8i_launch_nt<64>(st, mw, mx, p, grid, pdl);
-  }
-}
-
 static std::map<int, std::pair<float*, size_t>> g_split_scratch;   // per device: scratch of the C-ABI matmuls ([hi | lo], [Bt | hi | lo])
 
 // Forget tensor maps (call when buffers they describe are freed and their addresses may be reused

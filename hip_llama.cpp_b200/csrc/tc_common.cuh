@@ -44,8 +44,7 @@ __device__ __forceinline__ bool tc_mbar_wait(uint64_t* bar, unsigned parity, int
 // One lane of a converged warp, in a form that the compiler knows to be one: the descriptors of tcgen05 and TMA instructions go through uniform
 // registers, and under `lane == 0` each such instruction is wrapped in a loop over the lanes that might take part.  A stage of barrier wait,
 // fence, four MMAs of 128 x 64 x 8 (tf32) or x 32 (int8) and commit took its issuer 500 cycles that way, 214 with this.
-// Per step of two Llama-2-7B layers at 6 slots (fp32) 640 -> 517 us, prefill of 1024 tokens 5131 -> 4877, 16 prompts of stories110M 2909 -> 2765; the Q8_0
-// kernel, bound by its epilogue, was slower with it (1 slot 207 -> 220 us) and keeps lane 0.
+// Per step of two Llama-2-7B layers at 6 slots (fp32) 640 -> 517 us, prefill of 1024 tokens 5131 -> 4877, 16 prompts of stories110M 2909 -> 2765.
 __device__ __forceinline__ bool tc_elect() {
   uint32_t one;
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
