@@ -100,6 +100,7 @@ struct AttnP {
   const float* kc; const float* vc;         // already offset by loff
   long long kv_batch_stride; int kv_dim, head_size, kv_mul, dim;
   int nseg, nsplit;
+  int sorted;                               // attn_stream_kernel: slots by context, longest first
   float4* part_acc; float2* part_ml; int* counters;
   float* out_hi; float* out_lo;             // nullable: the tf32 hi/lo split of `out` for the tensor-core wo matmul
   int8_t* out_q; float* out_sT; int ldxs, gs;   // nullable: `out` quantised per group (runq.c:145-171) for the int8 wo matmul
@@ -132,8 +133,10 @@ __device__ __forceinline__ void attn_store(const AttnP& p, float* outp, float4 r
 }
 
 // J = float4 slots per lane; a CTA covers a segment of 128*J query floats (whole heads).
-template <int J, bool ROPE = false>
-__global__ void __launch_bounds__(256) attn_fused_kernel(const AttnP p) {
+// DEEP (J = 1, few CTAs): the rows of a warp's next step are on their way while this one's are folded in -- twice the bytes in flight for twice the registers
+// (116 .. 124: two CTAs of eight warps an SM, so only for grids that fit in one wave of those).  Same sums.
+template <int J, bool ROPE = false, bool DEEP = false>
+__global__ void __launch_bounds__(256, DEEP ? 2 : 0) attn_fused_kernel(const AttnP p) {
   constexpr int F = 32 * J;  // slots per segment
   extern __shared__ float4 sm_acc[];                 // [warps][F]
   float2* sm_ml = reinterpret_cast<float2*>(sm_acc + (blockDim.x >> 5) * F);  // [warps][F]
@@ -231,6 +234,65 @@ __global__ void __launch_bounds__(256) attn_fused_kernel(const AttnP p) {
   constexpr int RW = (J <= 2) ? 4 : 2;
   const float inv_sqrt_hs = 1.0f / sqrt_hs;
   const int nw = blockDim.x >> 5;   // warps of this CTA: 8, or fewer when the grid would not fit one wave (attn_pick_warps)
+  if constexpr (DEEP) {
+    const int step = nw * RW;
+    auto load = [&](int t, float4 (&kr)[RW][J], float4 (&vr)[RW][J]) {
+      long long roff[RW];
+#pragma unroll
+      for (int r = 0; r < RW; r++) {
+        const int tr = (t + nw * r) < t1 ? t + nw * r : t;
+        roff[r] = p.pg.table ? kv_paged_off(p.pg, b, tr, p.kv_dim) : (long long)tr * p.kv_dim;
+        const float* ka = kb + roff[r];
+#pragma unroll
+        for (int j = 0; j < J; j++) kr[r][j] = ldg_stream(reinterpret_cast<const float4*>(ka + koff[j]));
+      }
+#pragma unroll
+      for (int r = 0; r < RW; r++) {
+        const float* va = vb + roff[r];
+#pragma unroll
+        for (int j = 0; j < J; j++) vr[r][j] = ldg_stream(reinterpret_cast<const float4*>(va + koff[j]));
+      }
+    };
+    auto fold = [&](int t, const float4 (&kr)[RW][J], const float4 (&vr)[RW][J]) {
+#pragma unroll
+      for (int j = 0; j < J; j++) {
+        float sc[RW];
+#pragma unroll
+        for (int r = 0; r < RW; r++) sc[r] = dot4(qv[j], kr[r][j], 0.0f);
+        for (int o = LH >> 1; o > 0; o >>= 1) {
+#pragma unroll
+          for (int r = 0; r < RW; r++) sc[r] += __shfl_xor_sync(THA_FULL_MASK, sc[r], o);
+        }
+        float mn = m[j];
+#pragma unroll
+        for (int r = 0; r < RW; r++) {
+          sc[r] = (t + nw * r) < t1 ? sc[r] * inv_sqrt_hs : -INFINITY;
+          mn = fmaxf(mn, sc[r]);
+        }
+        const float corr = __expf(m[j] - mn);   // exp(-inf) = 0 on the first step
+        float ls = l[j] * corr;
+        float4 a = make_float4(acc[j].x * corr, acc[j].y * corr, acc[j].z * corr, acc[j].w * corr);
+#pragma unroll
+        for (int r = 0; r < RW; r++) {
+          const float pr = __expf(sc[r] - mn);  // dead rows: exp(-inf) = 0
+          ls += pr;
+          a.x = fmaf(pr, vr[r][j].x, a.x); a.y = fmaf(pr, vr[r][j].y, a.y);
+          a.z = fmaf(pr, vr[r][j].z, a.z); a.w = fmaf(pr, vr[r][j].w, a.w);
+        }
+        l[j] = ls; acc[j] = a; m[j] = mn;
+      }
+    };
+    float4 k0[RW][J], v0[RW][J], k1[RW][J], v1[RW][J];
+    int t = t0 + warp;
+    if (t < t1) load(t, k0, v0);
+    for (; t < t1; t += 2 * step) {
+      if (t + step < t1) load(t + step, k1, v1);
+      fold(t, k0, v0);
+      if (t + step >= t1) break;
+      if (t + 2 * step < t1) load(t + 2 * step, k0, v0);
+      fold(t + step, k1, v1);
+    }
+  } else {
   for (int t = t0 + warp; t < t1; t += nw * RW) {
     float4 kr[RW][J], vr[RW][J];
     bool live[RW];
@@ -277,6 +339,7 @@ __global__ void __launch_bounds__(256) attn_fused_kernel(const AttnP p) {
       }
       l[j] = ls; acc[j] = a; m[j] = mn;
     }
+  }
   }
 
   if (ROPE && own_new) {   // ---- the new position, from registers
@@ -355,12 +418,205 @@ __global__ void __launch_bounds__(256) attn_fused_kernel(const AttnP p) {
   if (threadIdx.x == 0) p.counters[b * p.nseg + seg] = 0;  // self-reset for the next launch
 }
 
+// The same attention for steps whose (slot, segment) pairs outnumber the SMs (no split of the time axis), one segment float4 a lane: a persistent CTA per
+// SM whose groups of nw warps take a pair at a time, longest contexts first, there and back over the groups.  Warp w of a group folds the rows
+// t = w (mod nw) as warp w of attn_fused_kernel's CTA does, in its order and with its sums: the same bits.  A lane's shares of the next rows travel to shared
+// memory by cp.async (each lane reads only what it copied itself: no barrier in the loop), two steps of four rows ahead.
+// Bound: HBM.  attn_fused_kernel has one step in flight per warp and, with all CTAs on the machine at once, the longest of ragged contexts
+// run on alone at a step per round trip to memory.  Two Llama-2-7B layers, us a step: Q8_0, 64 slots at positions 3 .. 570 660 -> 482; bf16, 24 slots at
+// 100 .. 1503 555 -> 446; fp32, 6 slots at 17 .. 672 511 -> 449; Q8_0, 40 slots at 1800 1558 -> 980.
+constexpr int AS_WARPS = 24, AS_STAGES = 2, AS_ROWS = 4, AS_MAX_SLOTS = 256;
+constexpr int AS_RING_F4 = AS_WARPS * AS_STAGES * 2 * AS_ROWS * 32;                                        // 196608 bytes
+constexpr int AS_SMEM = AS_RING_F4 * (int)sizeof(float4) + AS_WARPS * 32 * (int)(sizeof(float4) + sizeof(float2));   // and the warps' sums
+
+__device__ __forceinline__ void attn_cp16(uint32_t dst, const float* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+
+__device__ __forceinline__ float4 attn_lds16(uint32_t src) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(src) : "memory");
+  return v;
+}
+
+__global__ void __launch_bounds__(32 * AS_WARPS, 1) attn_stream_kernel(const AttnP p, int B, int nw) {
+  extern __shared__ float4 as_ring[];                  // [warps][stages][K rows | V rows][lane]
+  __shared__ int s_pos[AS_MAX_SLOTS], s_order[AS_MAX_SLOTS];
+  const int kt = threadIdx.x == 0 ? kt_begin(KT_ATTN) : -1;
+  pdl_trigger();
+  pdl_wait();
+  kt_stamp(kt, 1);
+  if (p.sorted) {
+    for (int i = threadIdx.x; i < B; i += blockDim.x) s_pos[i] = p.pos[i];
+    __syncthreads();
+    for (int i = threadIdx.x; i < B; i += blockDim.x) {   // longest context first
+      const int mine = s_pos[i];
+      int rank = 0;
+      for (int j = 0; j < B; j++) rank += (s_pos[j] > mine || (s_pos[j] == mine && j < i)) ? 1 : 0;
+      s_order[rank] = i;
+    }
+    __syncthreads();
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int hs = p.head_size, LH = hs >> 2;
+  const float inv_sqrt_hs = 1.0f / sqrtf((float)hs);
+  const uint32_t ring = (uint32_t)__cvta_generic_to_shared(as_ring + (size_t)warp * AS_STAGES * 2 * AS_ROWS * 32 + lane);
+  const int grp = warp / nw, w = warp - grp * nw, ngrp = AS_WARPS / nw;
+  float4* sm_acc = as_ring + AS_RING_F4 + grp * nw * 32;
+  float2* sm_ml = reinterpret_cast<float2*>(as_ring + AS_RING_F4 + AS_WARPS * 32) + grp * nw * 32;
+  auto group_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "r"(32 * nw) : "memory"); };
+  const int total = B * p.nseg, G = gridDim.x * ngrp, mine = grp * gridDim.x + blockIdx.x;
+  for (int base = 0, back = 0; base < total; base += G, back ^= 1) {
+    const int i = base + (back ? G - 1 - mine : mine);
+    if (i >= total) continue;
+    const int seg = i % p.nseg, b = p.sorted ? s_order[i / p.nseg] : i / p.nseg;
+    const int pb = p.sorted ? s_pos[b] : p.pos[b];
+    const int qo = seg * 128 + 4 * lane;
+    float* outp = p.out + (size_t)b * p.dim + qo;
+    if (pb < 0) {   // idle slot: zeros into the matmul that follows, as attn_fused_kernel
+      if (w == 0 && p.rp.out_b16) *reinterpret_cast<uint2*>(p.rp.out_b16 + (size_t)b * p.dim + qo) = make_uint2(0u, 0u);
+      if (w == 0 && p.out_q)
+        q8_quant4(make_float4(0.f, 0.f, 0.f, 0.f), p.gs, qo >> 2, p.out_q + (size_t)b * p.dim, p.out_sT, p.ldxs, b, true);
+      continue;
+    }
+    const int koff = ((qo / hs) / p.kv_mul) * hs + (qo % hs);
+    const float* kb = (p.pg.table ? p.kc : p.kc + (size_t)b * p.kv_batch_stride) + koff;
+    const float* vb = (p.pg.table ? p.vc : p.vc + (size_t)b * p.kv_batch_stride) + koff;
+    const int t1 = pb;                                  // cached rows; the new one comes from the matmul's partials
+    int ahead = w;                                      // first row of the next step to ask for
+    uint32_t put = ring;
+    auto ask = [&]() {
+      if (ahead < t1) {
+#pragma unroll
+        for (int r = 0; r < AS_ROWS; r++) {
+          const int tr = ahead + nw * r < t1 ? ahead + nw * r : ahead;
+          const long long off = p.pg.table ? kv_paged_off(p.pg, b, tr, p.kv_dim) : (long long)tr * p.kv_dim;
+          attn_cp16(put + r * 512, kb + off);
+          attn_cp16(put + (AS_ROWS + r) * 512, vb + off);
+        }
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      ahead += nw * AS_ROWS;
+      put = put == ring + (AS_STAGES - 1) * 2 * AS_ROWS * 512 ? ring : put + 2 * AS_ROWS * 512;
+    };
+#pragma unroll
+    for (int s = 0; s < AS_STAGES; s++) ask();
+    // ---- q (rotated) of this segment, and in stream 0 the new position's k and v, as attn_fused_kernel<1, true>
+    const bool own_new = w == 0;
+    float4 qv, knew, vnew;
+    {
+      const float* pr = p.rp.part + (size_t)b * p.rp.ld;
+      float4 a = make_float4(0.f, 0.f, 0.f, 0.f), kk = a, vv = a;
+      for (int z = 0; z < p.rp.nz; z++) {
+        const float4 t = *reinterpret_cast<const float4*>(pr + (size_t)z * p.rp.zstride + qo);
+        a.x += t.x; a.y += t.y; a.z += t.z; a.w += t.w;
+        if (own_new) {
+          const float4 tk = *reinterpret_cast<const float4*>(pr + (size_t)z * p.rp.zstride + p.dim + koff);
+          const float4 tv = *reinterpret_cast<const float4*>(pr + (size_t)z * p.rp.zstride + p.dim + p.kv_dim + koff);
+          kk.x += tk.x; kk.y += tk.y; kk.z += tk.z; kk.w += tk.w;
+          vv.x += tv.x; vv.y += tv.y; vv.z += tv.z; vv.w += tv.w;
+        }
+      }
+      const int jj = (qo % hs) >> 1;
+      const float2 c2 = *reinterpret_cast<const float2*>(p.rp.rc + (size_t)pb * (hs >> 1) + jj);
+      const float2 s2 = *reinterpret_cast<const float2*>(p.rp.rs + (size_t)pb * (hs >> 1) + jj);
+      auto rot = [](float x, float y, float c, float sn, float& o0, float& o1) {
+        o0 = fmaf(x, c, -__fmul_rn(y, sn));
+        o1 = fmaf(x, sn, __fmul_rn(y, c));
+      };
+      rot(a.x, a.y, c2.x, s2.x, qv.x, qv.y);
+      rot(a.z, a.w, c2.y, s2.y, qv.z, qv.w);
+      if (p.rp.q_out && own_new) *reinterpret_cast<float4*>(p.rp.q_out + (size_t)b * p.dim + qo) = qv;
+      if (own_new) {
+        rot(kk.x, kk.y, c2.x, s2.x, knew.x, knew.y);
+        rot(kk.z, kk.w, c2.y, s2.y, knew.z, knew.w);
+        vnew = vv;
+        const long long ro = p.pg.table ? kv_paged_off(p.pg, b, pb, p.kv_dim) : (long long)b * p.kv_batch_stride + (long long)pb * p.kv_dim;
+        *reinterpret_cast<float4*>(p.rp.kc_w + ro + koff) = knew;
+        *reinterpret_cast<float4*>(p.rp.vc_w + ro + koff) = vnew;
+      }
+    }
+    float m = -INFINITY, l = 0.0f;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    uint32_t get = ring;
+    for (int t = w; t < t1; t += nw * AS_ROWS) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(AS_STAGES - 1) : "memory");
+      float4 kr[AS_ROWS], vr[AS_ROWS];
+#pragma unroll
+      for (int r = 0; r < AS_ROWS; r++) vr[r] = attn_lds16(get + (AS_ROWS + r) * 512);
+#pragma unroll
+      for (int r = 0; r < AS_ROWS; r++) kr[r] = attn_lds16(get + r * 512);
+      get = get == ring + (AS_STAGES - 1) * 2 * AS_ROWS * 512 ? ring : get + 2 * AS_ROWS * 512;
+      float sc[AS_ROWS];
+#pragma unroll
+      for (int r = 0; r < AS_ROWS; r++) sc[r] = dot4(qv, kr[r], 0.0f);
+      for (int o = LH >> 1; o > 0; o >>= 1) {
+#pragma unroll
+        for (int r = 0; r < AS_ROWS; r++) sc[r] += __shfl_xor_sync(THA_FULL_MASK, sc[r], o);
+      }
+      ask();                                            // into the stage just read: the scores have used what was read last
+      float mn = m;
+#pragma unroll
+      for (int r = 0; r < AS_ROWS; r++) {
+        sc[r] = (t + nw * r) < t1 ? sc[r] * inv_sqrt_hs : -INFINITY;
+        mn = fmaxf(mn, sc[r]);
+      }
+      const float corr = __expf(m - mn);
+      float ls = l * corr;
+      float4 a = make_float4(acc.x * corr, acc.y * corr, acc.z * corr, acc.w * corr);
+#pragma unroll
+      for (int r = 0; r < AS_ROWS; r++) {
+        const float pr = __expf(sc[r] - mn);
+        ls += pr;
+        a.x = fmaf(pr, vr[r].x, a.x); a.y = fmaf(pr, vr[r].y, a.y);
+        a.z = fmaf(pr, vr[r].z, a.z); a.w = fmaf(pr, vr[r].w, a.w);
+      }
+      l = ls; acc = a; m = mn;
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");   // the ring is the next stream's
+    if (own_new) {   // ---- the new position, from registers
+      float sc = dot4(qv, knew, 0.0f);
+      for (int o = LH >> 1; o > 0; o >>= 1) sc += __shfl_xor_sync(THA_FULL_MASK, sc, o);
+      sc *= inv_sqrt_hs;
+      const float mn = fmaxf(m, sc);
+      const float corr = __expf(m - mn);
+      const float pr = __expf(sc - mn);
+      l = l * corr + pr;
+      acc = make_float4(fmaf(pr, vnew.x, acc.x * corr), fmaf(pr, vnew.y, acc.y * corr), fmaf(pr, vnew.z, acc.z * corr), fmaf(pr, vnew.w, acc.w * corr));
+      m = mn;
+    }
+    group_sync();                                       // the merge before this one is done
+    sm_acc[w * 32 + lane] = acc;
+    sm_ml[w * 32 + lane] = make_float2(m, l);
+    group_sync();
+    if (w != 0) continue;
+    float M = -INFINITY, L = 0.0f;
+    float4 A = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int x = 0; x < nw; x++) M = fmaxf(M, sm_ml[x * 32 + lane].x);
+    for (int x = 0; x < nw; x++) {
+      const float2 ml = sm_ml[x * 32 + lane];
+      const float e = (ml.x == -INFINITY) ? 0.0f : expf(ml.x - M);
+      const float4 pa = sm_acc[x * 32 + lane];
+      L += ml.y * e;
+      A.x += pa.x * e; A.y += pa.y * e; A.z += pa.z * e; A.w += pa.w * e;
+    }
+    attn_store(p, outp, make_float4(A.x / L, A.y / L, A.z / L, A.w / L), b);
+  }
+  kt_stamp(kt, 6);
+}
+
 }  // namespace tha
 
 // ------------------------------------------------------------------ launchers -------
 namespace tha {
 
 int attn_fused_nsplit(int B, int nseg, int seq_len);
+
+static int attn_sms() {
+  static int sms = 0;
+  if (!sms) { int dev = 0, n = 148; if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev); sms = n; }
+  return sms;
+}
 
 // Segment choice for the fused kernel: a CTA covers G whole heads with G*hs = 128*J floats, J in 1..8.
 // Returns J (0 = shape not supported by the fused kernel).  The NARROWEST segment wins: J = 1 needs 48 registers per
@@ -410,14 +666,22 @@ int attn_fused_nsplit(int B, int nseg, int seq_len) {
   return target;
 }
 
+// attn_stream_kernel or attn_fused_kernel: both give the same bits.  The persistent CTAs hold 24 warps; where attn_fused_kernel would have more on an SM at once
+// (25 .. 32: as many as its registers allow), uniform contexts keep it at the bandwidth of HBM and the persistent kernel, which then needs a second
+// round, loses (16 slots at 500: 244 -> 273 us a step; 158 slots of stories110M at 106: 934 -> 1049), while ragged long ones gain (64 slots at 357 .. 1239: 1132 -> 806;
+// 15 at 27 .. 965: 332 -> 309).  Positions are on the device; the length of the cache stands for them.  Below 25 warps an SM it gains or is even: 44 drawn steps,
+// ratio 0.96 to 1.40, 1.05 on average.
+static bool attn_stream_ok(int B, int nseg, int nsplit, int nw, int seq_len) {
+  return nsplit == 1 && B <= AS_MAX_SLOTS && nw >= 2 && AS_WARPS % nw == 0 && sm_budget() >= attn_sms() && (B * nseg <= AS_WARPS / nw * attn_sms() || seq_len >= 1024);
+}
+
 // Warps per CTA.  Eight, unless the grid (one CTA per slot and segment, unsplit) would then need more than one wave of
 // the machine: 256 slots x 6 segments of stories110M are 1536 CTAs against 740 resident ones (five per SM at 48 registers), i.e.
 // three rounds of a latency-bound kernel (12 us per layer at position 10).  Warps per SM are what the register file allows either
 // way, so narrower CTAs cost no bandwidth at long contexts; they put every (slot, segment) on the machine at once.
 // A CTA needs one thread per float4 of its segment for the merge: warps >= J.
 static int attn_pick_warps(void (*k)(const AttnP), int J, long long ctas) {
-  static int sms = 0;
-  if (!sms) { int dev = 0; sms = 148; if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
+  const int sms = attn_sms();
   static int forced = -1;
   if (forced < 0) { const char* v = getenv("THA_ATTN_WARPS"); forced = (v && *v) ? atoi(v) : 0; }
   if (forced >= J && forced <= 8 && forced > 0) return forced;
@@ -467,6 +731,15 @@ static int attn_fused_launch_impl(cudaStream_t stream, Workspace* ws, int B, con
     case 7: k = attn_fused_kernel<7>; break; case 8: k = attn_fused_kernel<8>; break;
   }
   const int nw = attn_pick_warps(k, J, (long long)B * p.nseg * p.nsplit);
+  if (rp && J == 1 && attn_stream_ok(B, p.nseg, p.nsplit, nw, seq_len)) {
+    const int pairs = B * p.nseg, sms = attn_sms();
+    p.sorted = pairs > AS_WARPS / nw * sms;   // one round: the order does not matter
+    THA_CUDA_OK(cudaFuncSetAttribute(attn_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AS_SMEM));
+    THA_CUDA_OK(launch(attn_stream_kernel, dim3(pairs < sms ? pairs : sms), dim3(32 * AS_WARPS), (size_t)AS_SMEM, stream, pdl, p, B, nw));
+    return THA_STATUS_SUCCESS;
+  }
+  // few CTAs (nw is then 8): the deep form, in one wave of two an SM
+  if (rp && J == 1 && nw == 8 && B * p.nseg * p.nsplit <= 2 * attn_sms()) k = attn_fused_kernel<1, true, true>;
   dim3 grid(B, p.nseg, p.nsplit), block(32 * nw);
   const size_t smem = (size_t)nw * F * (sizeof(float4) + sizeof(float2));
   if (smem > 40 * 1024) THA_CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
