@@ -5,14 +5,18 @@
 #include <cuda_bf16.h>
 
 #include <stdlib.h>
+#include <string.h>
 
 #include <mutex>
+#include <new>
+#include <vector>
 
 #include "common.cuh"
 #include "hybrid_ops.cuh"
 #include "tha_hybrid.h"
 
 namespace tha {
+int launches_get();   // forward.cu
 
 // x = embed[token] * scale (+ the learned vector of the row's position when the model has a position table); x0, when given,
 // keeps a copy of it for the layers that add the embedding output again; copy (nullable) gets it in the products' number format; join [rows, 2 width], when given, gets both halves of the
@@ -318,21 +322,11 @@ static int hyb_run_experts(void* stream, HybScratch& sc, int dt, int R, int W, c
   return THA_STATUS_SUCCESS;
 }
 
-extern "C" int tha_hyb_step(void* stream, const tha_hyb_model_t* m, const tha_rows_t* rows, const tha_kv_t* kv,
-                            const tha_state_store_t* st, int n_want, const int* want_rows, float* logits, float* taps) {
-  if (!m || !rows || !kv || !st || m->n_rot > 64) return THA_STATUS_INVALID_ARG;
-  const int R = rows->n_rows;
-  if (R < 1) return THA_STATUS_SUCCESS;
-  cudaStream_t s = (cudaStream_t)stream;
-  const int dt = m->dtype, W = m->width;
-  int dev = 0;
-  THA_CUDA_OK(cudaGetDevice(&dev));
-  HybScratch& sc = g_scratch[dev & 63];
-  std::lock_guard<std::mutex> lock(sc.mu);
-  InStep in_step;
+// The scratch of a step, grown where it has to be (under the scratch's lock).
+static int hyb_grow(HybScratch& sc, const tha_hyb_model_t* m, const tha_rows_t* rows, int n_want) {
   StepBuffers b;
   const size_t need = carve(m, rows, n_want, nullptr, &b);
-  if (need > sc.cap) {   // grow: nothing of an earlier step may still be using the old slab
+  if (need > sc.cap) {   // nothing of an earlier step may still be using the old slab
     THA_CUDA_OK(cudaDeviceSynchronize());
     if (sc.base) THA_CUDA_OK(cudaFree(sc.base));
     sc.base = nullptr; sc.cap = 0;
@@ -340,6 +334,17 @@ extern "C" int tha_hyb_step(void* stream, const tha_hyb_model_t* m, const tha_ro
     THA_CUDA_OK(cudaMalloc((void**)&sc.base, want));
     sc.cap = want;
   }
+  return THA_STATUS_SUCCESS;
+}
+
+// The step's launches, over scratch that is large enough (under its lock).
+static int hyb_issue(void* stream, HybScratch& sc, const tha_hyb_model_t* m, const tha_rows_t* rows, const tha_kv_t* kv, const tha_state_store_t* st, int n_want,
+                     const int* want_rows, float* logits, float* taps) {
+  const int R = rows->n_rows;
+  cudaStream_t s = (cudaStream_t)stream;
+  const int dt = m->dtype, W = m->width;
+  InStep in_step;
+  StepBuffers b;
   carve(m, rows, n_want, sc.base, &b);
 
   const float embed_scale = m->embed_scale != 0.f ? m->embed_scale : 1.0f;
@@ -670,4 +675,103 @@ extern "C" int tha_hyb_step(void* stream, const tha_hyb_model_t* m, const tha_ro
     }
   }
   return THA_STATUS_SUCCESS;
+}
+
+static HybScratch* hyb_scratch_of_device() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  return &g_scratch[dev & 63];
+}
+
+extern "C" int tha_hyb_step(void* stream, const tha_hyb_model_t* m, const tha_rows_t* rows, const tha_kv_t* kv,
+                            const tha_state_store_t* st, int n_want, const int* want_rows, float* logits, float* taps) {
+  if (!m || !rows || !kv || !st || m->n_rot > 64) return THA_STATUS_INVALID_ARG;
+  if (rows->n_rows < 1) return THA_STATUS_SUCCESS;
+  HybScratch* sc = hyb_scratch_of_device();
+  if (!sc) return THA_STATUS_EXECUTION_FAILED;
+  std::lock_guard<std::mutex> lock(sc->mu);
+  HYB_OK(hyb_grow(*sc, m, rows, n_want));
+  return hyb_issue(stream, *sc, m, rows, kv, st, n_want, want_rows, logits, taps);
+}
+
+// ---- decode-sized steps as executable graphs ---------------------------------------------------------------------------
+// A step of one row per sequence is 24 to 60 kernels of 2 to 10 us, and issuing one takes the host 2 to 3 us.  As a graph, us a step of ServingEngine.step
+// with its copies: four layers of retention, windowed attention and key-value memory (width 1024, 3 requests, 52 kernels) 277 -> 242; two attention
+// layers of width 2048 (2 requests, 24 kernels) 216 -> 195.  A step is captured when it comes a second time in the same form (15 us more, once).
+struct HybGraph { std::vector<unsigned char> key; cudaGraphExec_t exec; int launches; unsigned long long last_use; };
+constexpr size_t HYB_MAX_GRAPHS = 8;
+struct tha_hyb_plan {
+  std::vector<HybGraph> graphs;
+  std::vector<unsigned char> last;   // the form of the last step that was issued kernel by kernel
+  unsigned long long clock = 0;
+};
+
+extern "C" int tha_hyb_plan_create(tha_hyb_plan_t** plan) {
+  if (!plan) return THA_STATUS_INVALID_ARG;
+  *plan = new (std::nothrow) tha_hyb_plan;
+  return *plan ? THA_STATUS_SUCCESS : THA_STATUS_EXECUTION_FAILED;
+}
+extern "C" void tha_hyb_plan_destroy(tha_hyb_plan_t* plan) {
+  if (!plan) return;
+  for (HybGraph& g : plan->graphs) cudaGraphExecDestroy(g.exec);
+  delete plan;
+}
+
+extern "C" int tha_hyb_step_planned(void* stream, tha_hyb_plan_t* plan, const tha_hyb_model_t* m, const tha_rows_t* rows, const tha_kv_t* kv,
+                                    const tha_state_store_t* st, int n_want, const int* want_rows, float* logits) {
+  if (!m || !rows || !kv || !st || m->n_rot > 64) return THA_STATUS_INVALID_ARG;
+  cudaStream_t s = (cudaStream_t)stream;
+  if (!plan || !graph_enabled() || !s || s == cudaStreamLegacy || rows->n_rows < 1 || rows->max_seq_rows != 1)
+    return tha_hyb_step(stream, m, rows, kv, st, n_want, want_rows, logits, nullptr);
+  // The longest context sizes the attention's splits only: a step stands for all of up to the next multiple of 256.
+  tha_rows_t r = *rows;
+  r.max_pos |= 255;
+  HybScratch* sc = hyb_scratch_of_device();
+  if (!sc) return THA_STATUS_EXECUTION_FAILED;
+  std::lock_guard<std::mutex> lock(sc->mu);
+  HYB_OK(hyb_grow(*sc, m, &r, n_want));
+  std::vector<unsigned char> key;   // every value that the launches depend on, field by field
+  key.reserve(256);
+  auto put = [&](auto v) { const unsigned char* b = reinterpret_cast<const unsigned char*>(&v); key.insert(key.end(), b, b + sizeof(v)); };
+  put(m); put(stream); put(sc->base); put(want_rows); put(logits); put(n_want); put(pdl_enabled());
+  put(r.n_rows); put(r.n_seqs); put(r.token); put(r.pos); put(r.row_seq); put(r.seq_first); put(r.seq_slot); put(r.max_pos);
+  put(kv->k_pool); put(kv->v_pool); put(kv->table); put(kv->table_stride); put(kv->block_size); put(kv->n_cache_layers); put(kv->kv_dim);
+  put(st->base); put(st->slot_floats);
+  HybGraph* hit = nullptr;
+  for (HybGraph& g : plan->graphs)
+    if (g.key == key) hit = &g;
+  if (!hit && plan->last == key) {
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    const int before = launches_get();
+    if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+      const int rc = hyb_issue(stream, *sc, m, &r, kv, st, n_want, want_rows, logits, nullptr);
+      const cudaError_t e = cudaStreamEndCapture(s, &graph);
+      if (rc != THA_STATUS_SUCCESS || e != cudaSuccess || cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) exec = nullptr;
+      if (graph) cudaGraphDestroy(graph);
+    }
+    const int launches = launches_get() - before;
+    count_launch(-launches);
+    if (exec) {
+      if (plan->graphs.size() >= HYB_MAX_GRAPHS) {
+        size_t old = 0;
+        for (size_t i = 1; i < plan->graphs.size(); i++)
+          if (plan->graphs[i].last_use < plan->graphs[old].last_use) old = i;
+        cudaGraphExecDestroy(plan->graphs[old].exec);
+        plan->graphs.erase(plan->graphs.begin() + old);
+      }
+      plan->graphs.push_back({key, exec, launches, 0});
+      hit = &plan->graphs.back();
+    } else {
+      cudaGetLastError();   // not capturable after all: kernel by kernel
+    }
+  }
+  if (hit) {
+    hit->last_use = ++plan->clock;
+    count_launch(hit->launches);
+    THA_CUDA_OK(cudaGraphLaunch(hit->exec, s));
+    return THA_STATUS_SUCCESS;
+  }
+  plan->last = key;
+  return hyb_issue(stream, *sc, m, &r, kv, st, n_want, want_rows, logits, nullptr);
 }

@@ -19,13 +19,15 @@ SequenceEngine::SequenceEngine(LayerModel* model, int max_tokens, int max_seqs)
   const size_t blocks = bm_.blocks_for(round_up(max_tokens, 64));
   if (!bm_.create_pool(blocks, model->separate_values())) { err_ = std::string("cannot allocate the cache pool: ") + tha_last_error(); return; }
   if (!bm_.create_state_slots((size_t)model->state_floats())) { err_ = std::string("cannot allocate the state slots: ") + tha_last_error(); return; }
-  if (tha_stream_create(&stream_) != 0) { err_ = tha_last_error(); return; }
+  if (tha_stream_create(&stream_) != 0 || tha_hyb_plan_create(&plan_) != 0) { err_ = tha_last_error(); return; }
   filled_.assign(max_seqs, 0);
   ok_ = true;
 }
 
 SequenceEngine::~SequenceEngine() {
-  if (stream_) { tha_stream_sync(stream_); tha_stream_destroy(stream_); }
+  if (stream_) tha_stream_sync(stream_);
+  tha_hyb_plan_destroy(plan_);
+  if (stream_) tha_stream_destroy(stream_);
   if (stage_h_) tha_host_free(stage_h_);
   if (logits_h_) tha_host_free(logits_h_);
   for (void* p : {(void*)stage_d_, (void*)logits_d_, (void*)taps_d_, (void*)rng_d_, (void*)next_d_, (void*)samp_pos_d_, (void*)reseed_d_})
@@ -159,8 +161,8 @@ bool SequenceEngine::run(const std::vector<StepEntry>& entries, bool to_host, st
     taps_cap_ = n_taps;
     if (tha_malloc((void**)&taps_d_, taps_cap_ * sizeof(float)) != 0) return fail(tha_last_error());
   }
-  const int status = tha_hyb_step(stream_, model_->device_model(), &rows, &kv, &st, (int)n_want, want_d, n_want ? logits_d_ : nullptr,
-                                  taps ? taps_d_ : nullptr);
+  const int status = taps ? tha_hyb_step(stream_, model_->device_model(), &rows, &kv, &st, (int)n_want, want_d, n_want ? logits_d_ : nullptr, taps_d_)
+                          : tha_hyb_step_planned(stream_, plan_, model_->device_model(), &rows, &kv, &st, (int)n_want, want_d, n_want ? logits_d_ : nullptr);
   if (status != 0) return fail(std::string("step failed (status ") + std::to_string(status) + "): " + tha_last_error());
   if (to_host && n_want) {
     if (n_want * (size_t)vocab > logits_h_cap_) {

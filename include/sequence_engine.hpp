@@ -69,6 +69,7 @@ class SequenceEngine {
   bool ok_ = false;
   std::string err_;
   void* stream_ = nullptr;
+  tha_hyb_plan_t* plan_ = nullptr;        // decode steps as executable graphs
   std::map<std::string, int> slot_of_;
   std::vector<int> filled_;               // per slot: positions fed
   int next_request_id_ = 0;

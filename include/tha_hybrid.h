@@ -448,6 +448,16 @@ typedef struct {
 int tha_hyb_step(void* stream, const tha_hyb_model_t* m, const tha_rows_t* rows, const tha_kv_t* kv,
                  const tha_state_store_t* st, int n_want, const int* want_rows, float* logits, float* taps);
 
+/* The same step for a serving loop, which repeats steps of one row per sequence: a plan keeps such steps as executable graphs (a step of
+ * another size, a context past another 256 positions or regrown scratch makes another; eight at most) and replays them; every other
+ * step is tha_hyb_step.  All arrays and the cache may hold new values in every call.  A plan belongs to one model, whose
+ * descriptions do not change while it lives, to one device and to one thread at a time; plan == NULL: tha_hyb_step. */
+typedef struct tha_hyb_plan tha_hyb_plan_t;
+int tha_hyb_plan_create(tha_hyb_plan_t** plan);
+void tha_hyb_plan_destroy(tha_hyb_plan_t* plan);   /* behind the last step that was issued with it */
+int tha_hyb_step_planned(void* stream, tha_hyb_plan_t* plan, const tha_hyb_model_t* m, const tha_rows_t* rows, const tha_kv_t* kv,
+                         const tha_state_store_t* st, int n_want, const int* want_rows, float* logits);
+
 /* ---- the mechanisms, one call each (also what tha_hyb_step is made of) ------------------------------------------- */
 /* out[r, :] = x[r, :] / sqrt(mean(x[r]^2) + eps) * (w_offset + w), rows picked through `rows_idx` when not NULL;
  * out is dtype-typed (bf16 / fp32) */
