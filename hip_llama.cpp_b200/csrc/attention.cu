@@ -402,16 +402,38 @@ __global__ void __launch_bounds__(256, DEEP ? 2 : 0) attn_fused_kernel(const Att
   if (!is_last) return;
   __threadfence();
   if (f < F) {
+    // Fixed order: independent of arrival.  Eight splits' partials are asked for before the first is used: one round trip to L2 for up to eight splits
+    // in place of two a split.  Steps of stories110M at 16 fp32 slots 454 -> 434 us, 8 bf16 slots 395 -> 383.
+    constexpr int MB = J > 1 || DEEP ? 8 : 1;   // (one at a time where the registers are counted; launches of that form with splits are the deep one's)
     float GM = -INFINITY;
-    for (int s = 0; s < nsp; s++) GM = fmaxf(GM, __ldcg(&p.part_ml[pbase + (size_t)s * F + f]).x);
+    float2 ml[MB];
+    float4 pa[MB];
+    auto fetch = [&](int s0, bool sums) {
+#pragma unroll
+      for (int u = 0; u < MB; u++)
+        if (s0 + u < nsp) {
+          ml[u] = __ldcg(&p.part_ml[pbase + (size_t)(s0 + u) * F + f]);
+          if (sums) pa[u] = __ldcg(&p.part_acc[pbase + (size_t)(s0 + u) * F + f]);
+        }
+    };
+    fetch(0, nsp <= MB);
+    for (int s0 = 0; s0 < nsp; s0 += MB) {
+      if (s0) fetch(s0, false);
+#pragma unroll
+      for (int u = 0; u < MB; u++)
+        if (s0 + u < nsp) GM = fmaxf(GM, ml[u].x);
+    }
     float GL = 0.0f;
     float4 GA = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s = 0; s < nsp; s++) {   // fixed order: result independent of arrival order
-      const float2 ml = __ldcg(&p.part_ml[pbase + (size_t)s * F + f]);
-      const float e = (ml.x == -INFINITY) ? 0.0f : expf(ml.x - GM);
-      const float4 a = __ldcg(&p.part_acc[pbase + (size_t)s * F + f]);
-      GL += ml.y * e;
-      GA.x += a.x * e; GA.y += a.y * e; GA.z += a.z * e; GA.w += a.w * e;
+    for (int s0 = 0; s0 < nsp; s0 += MB) {
+      if (nsp > MB) fetch(s0, true);
+#pragma unroll
+      for (int u = 0; u < MB; u++)
+        if (s0 + u < nsp) {
+          const float e = (ml[u].x == -INFINITY) ? 0.0f : expf(ml[u].x - GM);
+          GL += ml[u].y * e;
+          GA.x += pa[u].x * e; GA.y += pa[u].y * e; GA.z += pa[u].z * e; GA.w += pa[u].w * e;
+        }
     }
     attn_store(p, outp, make_float4(GA.x / GL, GA.y / GL, GA.z / GL, GA.w / GL), b);
   }
