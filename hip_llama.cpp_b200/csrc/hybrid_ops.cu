@@ -1812,6 +1812,9 @@ namespace tha {
 // hybrid_latent.cu: tensor-core attention for key rows wider than AM_MAXD whose values lie inside the keys
 bool hyb_attn_wide_ok(const tha_attn_t* a);
 int hyb_attn_wide_pairs(const tha_attn_t* a, const tha_rows_t* rows);
+// hybrid_attn_tc.cu: prompt portions on tcgen05
+int hyb_attn_tc_launch(cudaStream_t s, const tha_attn_t* a, const tha_rows_t* rows, const tha_kv_t* kv, const float* q, __nv_bfloat16* out, const float* gate,
+                       long long ldg, int min_rows, float* scratch, size_t scratch_floats);
 bool hyb_attn_row_ok(const tha_attn_t* a, const tha_kv_t* kv, const float* q);   // hybrid_attn_row.cu
 int hyb_attn_row_splits(const tha_attn_t* a, const tha_rows_t* rows, int max_keys);
 int hyb_attn_row_launch(cudaStream_t s, int dtype, const tha_attn_t* a, const tha_rows_t* rows, const tha_kv_t* kv, const float* q, void* out, int splits,
@@ -1887,6 +1890,10 @@ extern "C" int tha_hyb_attn_gated(void* stream, int dtype, const tha_attn_t* a, 
     if (rows->max_seq_rows == 1) return THA_STATUS_SUCCESS;
   }
   const int min_rows = row_form ? 2 : 1;
+  if (tc) {
+    const int st = hyb_attn_tc_launch(s, a, rows, kv, q, (bf16*)out, gate, ldg, min_rows, split_scratch, split_scratch_floats);
+    if (st != THA_STATUS_NOT_SUPPORTED) return st;
+  }
   const long long blocks = (long long)tiles * a->kv_heads * ceil_div(gsize, AG);
   const int fill = tc ? 2 * 148 : 4 * 148;   // blocks from which the SMs are full without splits (the tensor-core form: one block of 8 warps each)
   if (split_scratch && blocks < fill && max_keys >= 4 * ATT_KEYS) {

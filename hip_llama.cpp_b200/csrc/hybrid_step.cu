@@ -17,6 +17,7 @@
 
 namespace tha {
 int launches_get();   // forward.cu
+size_t hyb_attn_tc_scratch(const tha_attn_t* a, const tha_rows_t* rows);   // hybrid_attn_tc.cu
 
 // x = embed[token] * scale (+ the learned vector of the row's position when the model has a position table); x0, when given,
 // keeps a copy of it for the layers that add the embedding output again; copy (nullable) gets it in the products' number format; join [rows, 2 width], when given, gets both halves of the
@@ -148,7 +149,7 @@ static size_t carve(const tha_hyb_model_t* m, const tha_rows_t* rows, int n_want
   size_t n_in = 0, qd = 0, av = 0, mv = 0, cc = 0, dd = 0, dg = 0, gu = 0, ff = 0, sff = 0, top = 0, ne = 0;
   size_t n_in2 = 0, qr = 0, qf = 0, qp = 0;
   bool norm2 = false, keep_embed = false, join = false, shift = false;
-  size_t sd = 0, n_str = 0, hfw = 0, attf = 0, scan = 0;
+  size_t sd = 0, n_str = 0, hfw = 0, attf = 0, scan = 0, staged = 0;
   auto scan_scratch = [&](int heads, int dim, int vdim) {
     scan = max(scan, tha_hyb_scan_scratch_floats(heads, dim, vdim, rows->n_rows, rows->n_seqs, rows->max_seq_rows));
   };
@@ -163,6 +164,7 @@ static size_t carve(const tha_hyb_model_t* m, const tha_rows_t* rows, int n_want
     if (L.mixer == THA_MIX_ATTN || L.mixer == THA_MIX_ATTN_GDELTA) {
       qd = max(qd, (size_t)L.attn.heads * L.attn.dim);
       av = max(av, (size_t)L.attn.heads * L.attn.vdim);
+      if (m->dtype == THA_DT_BF16) staged = max(staged, hyb_attn_tc_scratch(&L.attn, rows));
       if (L.attn.diff) attf = max(attf, (size_t)L.attn.heads * L.attn.vdim);
       if (L.attn.conv_taps > 0) cc = max(cc, hyb_attn_conv_channels(L.attn));
     }
@@ -190,6 +192,7 @@ static size_t carve(const tha_hyb_model_t* m, const tha_rows_t* rows, int n_want
       qd = max(qd, (size_t)L.attn.heads * L.attn.dim);
       av = max(av, (size_t)L.attn.heads * L.attn.vdim);
       mv = max(mv, (size_t)L.mem.heads * L.mem.vdim);
+      if (m->dtype == THA_DT_BF16) staged = max(staged, hyb_attn_tc_scratch(&L.attn, rows));
     } else if (L.mixer == THA_MIX_DELTA) {
       cc = max(cc, (size_t)2 * L.delta.kv_heads * L.delta.dim + (size_t)L.delta.heads * L.delta.vdim);
       dd = max(dd, (size_t)L.delta.heads * L.delta.dim);
@@ -241,6 +244,8 @@ static size_t carve(const tha_hyb_model_t* m, const tha_rows_t* rows, int n_want
   // key splits of the attention, of every row in small steps, of the single rows beside a prompt in large ones: 16 x rows x heads x (vdim + 2)
   // floats and more (2 * heads <= 2 * heads * dim)
   b->split_floats = (size_t)16 * (R <= 1024 ? R : rows->n_seqs > 1 ? rows->n_seqs : 0) * (av + 2 * qd);
+  // prompt portions on tcgen05: their sequences' keys and values as bf16, ahead of the merge of single rows on the same stream
+  b->split_floats = max(b->split_floats, staged);
   b->split = c.take<float>(b->split_floats);
   b->scan_floats = scan;
   b->scan = scan ? c.take<float>(scan) : nullptr;

@@ -1,0 +1,84 @@
+"""Prompt portions on tcgen05 (csrc/hybrid_attn_tc.cu) through tha_hyb_attn_gated: every form of scores, both head sizes, groups that fill a block evenly and not,
+ragged ends of blocks, of key tiles and of halves of them, portions behind a context, several sequences with short ones among them, against a
+float64 statement on inputs that are exact in bf16."""
+import ctypes as C
+
+import pytest
+import torch
+
+import hyb_cabi as H
+from test_gpu_attention_calls import Cache, rel
+
+pytestmark = pytest.mark.gpu
+LONG = [(0, 0, 1)], [(0, 0, 2065)], [(1, 0, 1300), (0, 77, 900), (2, 5, 1), (3, 0, 33)], [(0, 1000, 1100), (1, 31, 1025)]
+
+
+def want(a, cache, q, seqs, t):
+    out, at, group = [], 0, a.heads // a.kv_heads
+    for slot, p0, n in seqs:
+        K, V = (x[slot, :p0 + n].double().repeat_interleave(group, 1) for x in (cache.k, cache.v))
+        s = torch.einsum("nhd,thd->hnt", q[at:at + n].double(), K) * a.scale
+        if a.softcap:
+            s = a.softcap * torch.tanh(s / a.softcap)
+        k, p = torch.arange(p0 + n, device="cuda"), torch.arange(p0, p0 + n, device="cuda")[:, None]
+        if "rel" in t:
+            s = s + t["rel"].double()[:, (p - k).clamp(0, a.rel_n - 1)]
+        hidden = k > p
+        if a.window:
+            hidden = hidden | ((p - k >= a.window) & (k >= a.keep_first))
+        if a.chunk:
+            hidden = hidden | (k < p // a.chunk * a.chunk)
+        s = s.masked_fill(hidden, float("-inf"))
+        if "sink" in t:
+            s = torch.cat([s, t["sink"].double()[:, None, None].expand(-1, n, 1)], -1)
+            V = torch.cat([V, torch.zeros_like(V[:1])])
+        o = torch.einsum("hnt,the->nhe", torch.softmax(s, -1), V)
+        if "gate" in t:
+            o = o * torch.sigmoid(t["gate"][at:at + n].double())[:, :, None]
+        out.append(o)
+        at += n
+    return torch.cat(out)
+
+
+@pytest.mark.parametrize("seqs", LONG)
+@pytest.mark.parametrize("heads,kv_heads,dim", [(16, 4, 128), (6, 2, 128), (16, 16, 64), (8, 1, 64)])
+@pytest.mark.parametrize("form", [dict(), dict(fp32_scores=1), dict(softcap=7.0, window=300), dict(rel=2048), dict(rel=40, window=500, keep_first=70),
+                                  dict(fp32_scores=1, chunk=333, sink=1), dict(window=50, keep_first=10, gate=1)])
+def test_portions(heads, kv_heads, dim, seqs, form):
+    a = H.Attn()
+    a.heads, a.kv_heads, a.dim, a.vdim, a.rot, a.scale, a.out_f32 = heads, kv_heads, dim, dim, -1, dim ** -0.5, 1
+    for k in ("fp32_scores", "softcap", "window", "keep_first", "chunk"):
+        setattr(a, k, form.get(k, 0))
+    g = torch.Generator(device="cuda").manual_seed(heads + dim)
+    R, longest = sum(n for _, _, n in seqs), max(p + n for _, p, n in seqs)
+    cache = Cache(max(s for s, _, _ in seqs) + 1, longest, kv_heads, dim, dim)
+    cache.k, cache.v = cache.k.bfloat16().float(), cache.v.bfloat16().float()
+    q = torch.randn(R, heads, dim, device="cuda", generator=g).bfloat16().float()
+    t = {}
+    if "rel" in form:
+        t["rel"] = torch.randn(heads, form["rel"], device="cuda", generator=g)
+        a.rel, a.rel_n = t["rel"].data_ptr(), form["rel"]
+    if "sink" in form:
+        t["sink"] = torch.randn(heads, device="cuda", generator=g)
+        a.sink = t["sink"].data_ptr()
+    if "gate" in form:
+        t["gate"] = torch.randn(R, heads, device="cuda", generator=g)
+        a.head_gate, a.o_g = 1, 0
+    lib = H.lib()
+    lib.c.tha_hyb_attn_gated.argtypes = [H.P, H.I, C.POINTER(H.Attn), C.POINTER(H.Rows), C.POINTER(H.Kv), H.P, H.P, H.P, C.c_size_t, H.P, H.L]
+    rows, keep = H.rows_of(seqs)
+    kv = cache.struct()
+    out = torch.full((R + 1, heads, dim), 7.0, device="cuda")
+    floats = len(seqs) * (longest + 32) * kv_heads * dim + 64
+    scratch = torch.full((floats + 1024,), float("nan"), device="cuda")     # what is not staged may hold anything
+    exact = want(a, cache, q, seqs, t)
+    # weights as two bf16 (2^-17 of themselves) or one (2^-9), random over hundreds of keys; the scores' fp32 sums below that
+    tol = 1e-5 if a.fp32_scores or a.softcap or "rel" in form else 3e-3
+    for given in (floats, 0):       # without scratch the step takes the other kernel
+        out.fill_(7.0)
+        torch.cuda.synchronize()
+        lib.check(lib.c.tha_hyb_attn_gated(None, H.BF16, a, rows, kv, H.ptr(q), H.ptr(out), H.ptr(scratch) if given else None, given, H.ptr(t.get("gate")), heads))
+        torch.cuda.synchronize()
+        assert bool(torch.isnan(scratch[floats:]).all()) and bool((out[R] == 7.0).all())
+        assert rel(out[:R], exact) < tol
+    assert lib.c.tha_gemm_check_error() == 0
