@@ -38,6 +38,11 @@ bool gemm_q8i_ok(const Q8iArgs& a);
 int gemm_q8i_pick_nt(int N, int gs);
 int gemm_q8i_launch(cudaStream_t st, const Q8iArgs& a, bool pdl);
 
+// What the kernel that rotates prompt rows leaves for the tensor-core attention besides the cache: q [rows][dim], k / v
+// [staged row][kv_dim] in bf16; row: the staged row of every row; pad: staged rows behind it that are zeroed in v (non-zero
+// for a sequence's last row only).  All null: none of it.
+struct RopeBf16 { uint16_t *q, *k, *v; const int *row, *pad; };
+
 // bf16 weights x bf16 activations (gemm_bf16.cu): both operands straight from TMA-written shared memory
 constexpr int BF_MAX_MATS = 8;
 struct BfArgs {

@@ -221,17 +221,25 @@ __global__ void __launch_bounds__(256) tc_prep_prompt_kernel(float* __restrict__
   if (threadIdx.x == 0) scale[b] = live ? 1.0f / sqrtf(tot / d + 1e-5f) : 0.0f;
 }
 
+// four values to bf16, nearest even
+__device__ __forceinline__ uint2 rope_bf16x4(float4 v) {
+  uint2 r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r.x) : "f"(v.y), "f"(v.x));
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r.y) : "f"(v.w), "f"(v.z));
+  return r;
+}
 // q|k|v rows of every slot (sum of nz partials): RoPE on q and k pairs (run.cc:271-286 with the host-built
 // cos/sin tables), q -> state, k/v -> the cache row of pos[b].  A thread takes two pairs per 128-bit load, two loads a block-width apart
 // (the fused attention of these steps takes only head sizes that are powers of two from 4 on, and reads the same rows by 128 bits).
 // Bound by memory: 2825 rows of 12288 (277 MB moved) took 84 us with two 64-bit loads, 64 with these.
+// b16 (bf16 prompts): q as bf16 rows in place of fp32 ones, K and V as bf16 rows besides (gemm_tc.h).
 // grid (ld / 2048, rows)
 __global__ void __launch_bounds__(256) tc_rope_scatter_kernel(const float* __restrict__ part, int nz, long long zstride,
                                                               int ld, const int* __restrict__ pos, int d, int kvd, int hs,
                                                               const float* __restrict__ rc, const float* __restrict__ rs,
                                                               float* __restrict__ q, float* __restrict__ kc,
                                                               float* __restrict__ vc, long long kv_bs, int loff,
-                                                              const int* __restrict__ slot, const KvPaged pg) {
+                                                              const int* __restrict__ slot, const KvPaged pg, const RopeBf16 b16) {
   const int kt = threadIdx.x == 0 ? kt_begin(KT_ROPE) : -1;
   pdl_trigger();   // the next kernel may start its launch (it waits for this grid to complete before touching memory)
   pdl_wait();
@@ -267,10 +275,23 @@ __global__ void __launch_bounds__(256) tc_rope_scatter_kernel(const float* __res
       // two forms of the step leave identical bits in the cache
       const float4 r = make_float4(fmaf(v[u].x, c.x, -__fmul_rn(v[u].y, s.x)), fmaf(v[u].x, s.x, __fmul_rn(v[u].y, c.x)),
                                    fmaf(v[u].z, c.y, -__fmul_rn(v[u].w, s.y)), fmaf(v[u].z, s.y, __fmul_rn(v[u].w, c.y)));
-      if (i < d) *reinterpret_cast<float4*>(q + (size_t)b * d + li) = r;
-      else *reinterpret_cast<float4*>(kc + rowoff + li) = r;
+      if (i >= d) {
+        *reinterpret_cast<float4*>(kc + rowoff + li) = r;
+        if (b16.k) *reinterpret_cast<uint2*>(b16.k + (size_t)b16.row[b] * kvd + li) = rope_bf16x4(r);
+      } else if (b16.q) {
+        *reinterpret_cast<uint2*>(b16.q + (size_t)b * d + li) = rope_bf16x4(r);
+      } else {
+        *reinterpret_cast<float4*>(q + (size_t)b * d + li) = r;
+      }
     } else {
-      *reinterpret_cast<float4*>(vc + rowoff + (i - d - kvd)) = v[u];
+      const int li = i - d - kvd;
+      *reinterpret_cast<float4*>(vc + rowoff + li) = v[u];
+      if (b16.v) {
+        const size_t at = (size_t)b16.row[b] * kvd + li;
+        *reinterpret_cast<uint2*>(b16.v + at) = rope_bf16x4(v[u]);
+        // behind a sequence's last row zeros to the end of its group of 16 keys: weights of 0 meet them there
+        for (int z = 1; z <= b16.pad[b]; z++) *reinterpret_cast<uint2*>(b16.v + at + (size_t)z * kvd) = make_uint2(0u, 0u);
+      }
     }
   }
   kt_stamp(kt, 6);
@@ -278,9 +299,9 @@ __global__ void __launch_bounds__(256) tc_rope_scatter_kernel(const float* __res
 
 int rope_scatter_launch(cudaStream_t st, bool pdl, int R, const float* part, int nz, long long zstride, int ld, const int* pos, int d,
                         int kvd, int hs, const float* rc, const float* rs, float* q, float* kc, float* vc, long long kv_bs, int loff,
-                        const int* slot, const KvPaged* pg) {
+                        const int* slot, const KvPaged* pg, const RopeBf16* b16) {
   THA_CUDA_OK(launch(tc_rope_scatter_kernel, dim3(ceil_div(ld / 4, 512), R), dim3(256), 0, st, pdl, part, nz, zstride, ld, pos, d, kvd, hs,
-                     rc, rs, q, kc, vc, kv_bs, loff, slot, pg ? *pg : KvPaged{}));
+                     rc, rs, q, kc, vc, kv_bs, loff, slot, pg ? *pg : KvPaged{}, b16 ? *b16 : RopeBf16{}));
   return THA_STATUS_SUCCESS;
 }
 
@@ -997,7 +1018,7 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
     if (!(skip & 8) && !rope_in_attn)
     THA_CUDA_OK(launch(tc_rope_scatter_kernel, dim3(ceil_div(ld_qkv / 4, 512), R), dim3(256), 0, st, pdl, (const float*)sc.part,
                        pl.z_qkv, (long long)R * ld_qkv, ld_qkv, io.pos, da, kvd, hs, rc, rs, io.q, s.key_cache, s.value_cache,
-                       kv_bs, loff, io.slot, pg));
+                       kv_bs, loff, io.slot, pg, RopeBf16{}));
     if (!io.logits && l == L - 1) {   // cache-only ingestion: the last layer's K/V rows are in place
       if (tpx) THA_CUDA_OK(launch(tp_epoch_kernel, dim3(1), dim3(32), 0, st, pdl, tp->epoch()));
       return THA_STATUS_SUCCESS;

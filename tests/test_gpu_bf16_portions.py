@@ -1,0 +1,48 @@
+"""Prompts of the bf16 model in portions (csrc/attn_prefill_tc.cu; the rows ahead of a portion by bf_kv_context_kernel): cuts and ends on both sides of the
+groups of 16 keys and the tiles of 128, plain and paged caches, with NaN in scratch from a call before.  Same statement and bound as
+tests/test_gpu_bf16.py: a rounding that falls on the other side moves a logit by a few 1e-3 of the largest, three such steps are allowed."""
+import numpy as np
+import pytest
+
+from gpu_util import assert_close_scaled
+from pkgload import load_pkg
+from test_gpu_bf16 import BF16_EPS, MODELS, bf16_model
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("name,cuts,lens", [("hs64", (16, 127, 1), (33, 128, 17)), ("hs64", (128, 15, 100), (129, 16, 190)),
+                                            ("hs128", (127, 129, 255), (130, 257, 257)), ("hs128", (17, 128, 383), (400, 144, 385))])
+def test_portions_vs_oracle(oracle, tmp_path, name, cuts, lens):
+    import torch
+    eng = load_pkg("engine")
+    cfg, wb, path = bf16_model(tmp_path, name, MODELS[name])
+    m = oracle.open(path, bf16=True)
+    m.set_bf16_attention(True)
+    rng = np.random.default_rng(lens[0])
+    prompts = [rng.integers(0, cfg.vocab_size, n).astype(np.int32) for n in lens]
+    want = []
+    for b in range(3):
+        seq = m.new_seq()
+        for i, t in enumerate(prompts[b]):
+            lg = seq.forward(int(t), i)
+        want.append(lg.copy())
+    w = eng.DeviceWeightsBF16(cfg, wb)
+    per = -(-cfg.seq_len // 16)
+    pages = eng.PagedKV(cfg, 4, 4 * per, 16)
+    pages.set_table(rng.permutation(4 * per).reshape(4, per).astype(np.int32))
+    bits = []
+    for e in (eng.Engine(w, 4), eng.Engine(w, 4, paged=pages)):
+        logits, nxt = torch.empty(3, cfg.vocab_size, device="cuda"), torch.empty(3, dtype=torch.int32, device="cuda")
+        e.state.key_cache.fill_(float("nan"))
+        e.state.value_cache.fill_(float("nan"))
+        e.prefill([(3, cfg.seq_len - 7, prompts[0][:5])] * 3, logits, nxt)     # a context of NaN: staged rows of it stay in scratch
+        e.prefill([(b, 0, prompts[b][:cuts[b]]) for b in range(3)])
+        e.prefill([(b, cuts[b], prompts[b][cuts[b]:]) for b in range(3)], logits, nxt)
+        torch.cuda.synchronize()
+        assert load_pkg("cabi").lib().c.tha_gemm_check_error() == 0
+        for b in range(3):
+            assert_close_scaled(logits[b].cpu().numpy(), want[b], BF16_EPS, f"slot {b}, {cuts[b]} + {lens[b] - cuts[b]}")
+        bits.append(logits.clone())
+    pages.close()
+    assert torch.equal(bits[0], bits[1])
