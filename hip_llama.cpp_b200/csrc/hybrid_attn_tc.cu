@@ -140,7 +140,6 @@ template <bool EXACT, bool CAP, bool REL, int DT>
 __global__ void __launch_bounds__(AT_THREADS, 1) hyb_attn_tc_kernel(const __grid_constant__ CUtensorMap mk, const __grid_constant__ CUtensorMap mv, tha_attn_t a, tha_rows_t rows, const float* __restrict__ q,
                                                                     __nv_bfloat16* __restrict__ out, int AG, int AP, const float* __restrict__ gate,
                                                                     long long ldg, int min_rows, int* error_flag) {
-  hyb_pdl_enter();
   constexpr int KB = DT / 64;                        // 64-channel blocks
   constexpr int Q_GROUP = KB * AT_ROWS * 128, K_STAGE = AT_KEYS * DT * 2, KV_STAGE = 2 * K_STAGE;
   constexpr float LOG2E = 1.4426950408889634f;
@@ -154,6 +153,29 @@ __global__ void __launch_bounds__(AT_THREADS, 1) hyb_attn_tc_kernel(const __grid
   __shared__ int abort_s;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < AT_STAGES; i++) { tc_mbar_init(&kv_full[i], 1); tc_mbar_init(&kv_empty[i], 1); }
+    for (int w = 0; w < 2; w++)
+      for (int b = 0; b < 2; b++) { tc_mbar_init(&s_full[w][b], 1); tc_mbar_init(&p_full[w][b], 4); tc_mbar_init(&pv_done[w][b], 1); }
+    abort_s = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  // All of the SM's TMEM, ahead of the trigger: the product behind this kernel may start on this SM once every block has triggered, allocates its own columns
+  // at once and keeps them until this grid has completed.  A block that came to its allocation after that would wait for ever (with heads of
+  // 64 both fit an SM).
+  if (warp == 9) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem_u32(&tmem_slot)), "r"(512));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+  }
+  at_fence_before();
+  __syncthreads();
+  at_fence_after();
+  const uint32_t tmem = tmem_slot;
+  hyb_pdl_enter();
+  auto release = [&]() {
+    if (warp == 9) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
+  };
   int seq = -1, r0 = 0, r_end = 0;
   {
     // the last tiles of a prompt see the most keys: tile numbers in descending order over all sequences, so that the grid ends on short ones
@@ -176,7 +198,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) hyb_attn_tc_kernel(const __grid
         i -= nt;
       }
     }
-    if (seq < 0) return;
+    if (seq < 0) { release(); return; }   // the same for the whole block
     r0 = rows.seq_first[seq] + tile * AP;
     r_end = min(rows.seq_first[seq + 1], r0 + AP);
   }
@@ -191,18 +213,6 @@ __global__ void __launch_bounds__(AT_THREADS, 1) hyb_attn_tc_kernel(const __grid
   auto half_key = [&](int ti) { return ti < tiles.n_a ? tiles.begin + 32 * ti : tiles.resume + 32 * (ti - tiles.n_a); };
   const int BP = REL ? at_rel_pitch(AP, a.rel_n) : 0, pad = at_rel_pad(AP);
 
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < AT_STAGES; i++) { tc_mbar_init(&kv_full[i], 1); tc_mbar_init(&kv_empty[i], 1); }
-    for (int w = 0; w < 2; w++)
-      for (int b = 0; b < 2; b++) { tc_mbar_init(&s_full[w][b], 1); tc_mbar_init(&p_full[w][b], 4); tc_mbar_init(&pv_done[w][b], 1); }
-    abort_s = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  }
-  if (warp == 9) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc_smem_u32(&tmem_slot)), "r"(512));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
-  }
   // q, rounded: warp w takes rows w, w + 13, ..; pairs past the block's positions are zeros
   for (int pr = warp; pr < 2 * AT_ROWS; pr += AT_THREADS / 32) {
     const int pp = pr / AG, hg = pr - pp * AG;
@@ -221,10 +231,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) hyb_attn_tc_kernel(const __grid
       for (int i = threadIdx.x; i < count; i += AT_THREADS) Bs[hl * BP + i] = hyb_attn_rel(a, g * gsize + hl, i - pad) * LOG2E;
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  at_fence_before();
   __syncthreads();
-  at_fence_after();
-  const uint32_t tmem = tmem_slot;
   int* abort_flag = &abort_s;
 
   if (warp < 8) {
@@ -420,10 +427,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) hyb_attn_tc_kernel(const __grid
   }
   __syncwarp();
   __syncthreads();
-  if (warp == 9) {
-    at_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512));
-  }
+  at_fence_after();
+  release();
   if (threadIdx.x == 0 && abort_s && error_flag) *((volatile int*)error_flag) = 1;
 }
 

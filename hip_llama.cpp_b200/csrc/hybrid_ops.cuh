@@ -7,9 +7,10 @@
 #include "tha_hybrid.h"
 
 namespace tha {
-// First statement of every kernel of this path: the next kernel of the stream may start its launch now, and nothing is read before the
+// First statement of every kernel of this path (but see below): the next kernel of the stream may start its launch now, and nothing is read before the
 // kernels ahead have completed (no-op in a launch without the programmatic attribute).  A step of a few decoded rows is 20 to 100 kernels of 2
 // to 10 us, and the launches between them were a quarter of it: two layers of attention 286 -> 220 us, four recurrent ones 405 -> 285.
+// A kernel that allocates TMEM does so ahead of this: a product started behind its trigger allocates its own at once and holds it until that kernel is done.
 __device__ __forceinline__ void hyb_pdl_enter() { pdl_trigger(); pdl_wait(); }
 // The bf16 matmul asks for its first weights AHEAD of that wait: only inside tha_hyb_step, where a matrix is the model's own and no kernel of
 // the step writes it, and whose first kernel is launched behind the completion of all that is ahead of the step on its stream -- in

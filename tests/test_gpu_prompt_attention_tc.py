@@ -3,10 +3,12 @@ ragged ends of blocks, of key tiles and of halves of them, portions behind a con
 float64 statement on inputs that are exact in bf16."""
 import ctypes as C
 
+import numpy as np
 import pytest
 import torch
 
 import hyb_cabi as H
+import test_gpu_gavodra as G
 from test_gpu_attention_calls import Cache, rel
 
 pytestmark = pytest.mark.gpu
@@ -82,3 +84,17 @@ def test_portions(heads, kv_heads, dim, seqs, form):
         assert bool(torch.isnan(scratch[floats:]).all()) and bool((out[R] == 7.0).all())
         assert rel(out[:R], exact) < tol
     assert lib.c.tha_gemm_check_error() == 0
+
+
+@pytest.mark.parametrize("lengths", [[64], [100, 128, 64]])
+def test_the_output_product_behind_it(tmp_path, lengths):
+    """Whole steps with heads of 64: a block of the attention and one of the product behind it, both of which allocate TMEM, fit an SM side by side."""
+    b = G.one_layer(tmp_path, G.attention(heads=64, kv_heads=8, dim=64, vdim=64, scale=0.125), width=4096)
+    prompts = [G.tokens_for(b, n, n) for n in lengths]
+    e = b.engine("bfloat16")
+    for turn in range(3):
+        names = ["%d.%d" % (turn, i) for i in range(len(lengths))]
+        got = e.step([(r, t, list(range(len(t)))) for r, t in zip(names, prompts)])
+        for r in names:
+            e.finish(r)
+        assert G.rel_err(got, np.concatenate([b.ref(t)[0] for t in prompts])) < G.BF16_TOL
