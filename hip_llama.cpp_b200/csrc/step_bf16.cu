@@ -10,7 +10,6 @@
 //   prep  x += partials | embedding row; RMSNorm in the reference's order g * (ss * x); round -> bf16 row
 //   gemm  wq|wk|wv -> partials;  rope_scatter (step_tc.cu);  attention (fp32);  round -> bf16
 //   gemm  wo -> partials;  prep(ffn);  gemm w1|w3;  SwiGLU + round;  gemm w2 -> partials;  ... prep(final); gemm wcls
-#include <limits.h>
 #include <stdlib.h>
 
 #include <map>
@@ -182,18 +181,18 @@ __global__ void bf_convert_kernel(const float* __restrict__ src, uint16_t* __res
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) dst[i] = f32_to_bf16(src[i]);
 }
 
-// Cache rows ahead of a portion (positions 0 .. pos0[i] - 1 of sequence i) -> bf16 (nearest even) staged rows base[i] + t:
-// 8 rows x 512 columns a block, a thread's eight loads ahead of its stores (a warp a row, load by load: 8 us more for 77 rows of 4096).
-// grid (kvd / 512, longest of them / 8, sequences)
+// Cache rows of positions 0 .. upto[i] - 1 of sequence i -> bf16 (nearest even) staged rows base[i] + t; with `pad` zeros in v16 behind them to the end
+// of their group of 16 (weights of 0 meet them there).  8 rows x 512 columns a block, a thread's eight loads ahead of its stores (a warp a row,
+// load by load: 8 us more for 77 rows of 4096).  grid (longest of them and its zeros / 8, kvd / 512, sequences)
 __global__ void __launch_bounds__(256) bf_kv_context_kernel(const float* __restrict__ kc, const float* __restrict__ vc, long long kv_bs,
-                                                            const int* __restrict__ seq_slot, const int* __restrict__ pos0,
-                                                            const int* __restrict__ base, const KvPaged pg, int kvd,
+                                                            const int* __restrict__ seq_slot, const int* __restrict__ upto,
+                                                            const int* __restrict__ base, int pad, const KvPaged pg, int kvd,
                                                             uint16_t* __restrict__ k16, uint16_t* __restrict__ v16) {
   pdl_trigger();
   pdl_wait();
-  const int i = blockIdx.z, n = pos0[i], slot = seq_slot[i];
-  const int t0 = blockIdx.y * 8 + (threadIdx.x >> 7), c = blockIdx.x * 512 + 4 * (threadIdx.x & 127);
-  if (t0 >= n || c >= kvd) return;
+  const int i = blockIdx.z, n = upto[i], end = pad ? (n + 15) & ~15 : n, slot = seq_slot[i];
+  const int t0 = blockIdx.x * 8 + (threadIdx.x >> 7), c = blockIdx.y * 512 + 4 * (threadIdx.x & 127);
+  if (t0 >= end || c >= kvd) return;
   float4 k[4], v[4];
 #pragma unroll
   for (int u = 0; u < 4; u++) {
@@ -206,12 +205,12 @@ __global__ void __launch_bounds__(256) bf_kv_context_kernel(const float* __restr
     return make_uint2(f32_to_bf16(x.x) | (uint32_t)f32_to_bf16(x.y) << 16, f32_to_bf16(x.z) | (uint32_t)f32_to_bf16(x.w) << 16);
   };
 #pragma unroll
-  for (int u = 0; u < 4; u++)
-    if (t0 + 2 * u < n) {
-      const size_t to = (size_t)(base[i] + t0 + 2 * u) * kvd + c;
-      *reinterpret_cast<uint2*>(k16 + to) = pack(k[u]);
-      *reinterpret_cast<uint2*>(v16 + to) = pack(v[u]);
-    }
+  for (int u = 0; u < 4; u++) {
+    const int t = t0 + 2 * u;
+    const size_t to = (size_t)(base[i] + t) * kvd + c;
+    if (t < n) *reinterpret_cast<uint2*>(k16 + to) = pack(k[u]);
+    if (t < end) *reinterpret_cast<uint2*>(v16 + to) = t < n ? pack(v[u]) : make_uint2(0u, 0u);
+  }
 }
 
 // ---- scratch (per workspace) ---------------------------------------------------------------------------------------
@@ -283,7 +282,15 @@ bool step_bf16_supported(const tha_config_t* c) {
   return attn_fused_supported(c->n_heads, hs, d, kvd);
 }
 
-static int bf_prepare(Workspace* ws, const tha_config_t& c, int R, bool prefill, int n_tab, int Rs = 0) {
+// Staged rows of K and V that a call may hold at once: 256 MB of them, or twice the rows that it brings (its other scratch is ten times that); one sequence,
+// whatever its context, always fits by itself.
+constexpr long long BF_STAGE_BYTES = 256ll << 20;
+static long long bf_stage_rows(int kvd, long long rows) {
+  const long long budget = BF_STAGE_BYTES / (4ll * kvd);
+  return 2 * rows > budget ? 2 * rows : budget;
+}
+
+static int bf_prepare(Workspace* ws, const tha_config_t& c, int R, bool prefill, int n_tab, long long Rs = 0, long long keep = 0) {
   THA_TRY_RC(gemm_tc_init(nullptr));
   std::lock_guard<std::mutex> lk(g_bf_mu);
   BfScratch& s = g_bf_scratch[ws];
@@ -298,8 +305,10 @@ static int bf_prepare(Workspace* ws, const tha_config_t& c, int R, bool prefill,
     THA_TRY_RC(bf_grow(&s.tab, &s.n_tab, (size_t)n_tab, ws));
     const int kvd_ = c.dim / c.n_heads * c.n_kv_heads;
     if (Rs > 0) {
-      THA_TRY_RC(bf_grow(&s.k16, &s.n_k16, (size_t)Rs * kvd_, ws));
-      THA_TRY_RC(bf_grow(&s.v16, &s.n_v16, (size_t)Rs * kvd_, ws));
+      const size_t need = (size_t)Rs * kvd_;
+      const size_t get = keep > Rs && need > s.n_k16 ? (size_t)keep * kvd_ : need;
+      THA_TRY_RC(bf_grow(&s.k16, &s.n_k16, get, ws));
+      THA_TRY_RC(bf_grow(&s.v16, &s.n_v16, get, ws));
     }
     return THA_STATUS_SUCCESS;
   }
@@ -308,13 +317,17 @@ static int bf_prepare(Workspace* ws, const tha_config_t& c, int R, bool prefill,
 }
 int step_bf16_prepare(Workspace* ws, const tha_config_t* c, int B) { return bf_prepare(ws, *c, B, false, 0); }
 
+// Sequences whose attention runs at once, staged side by side.  A call is one group, unless its contexts are more than the staging scratch
+// may hold (BF_STAGE_BYTES): then one group after the other, layer by layer, in the same scratch.
+struct BfGroup { int seq0, n_seqs, tile0, n_tiles, longest; };   // longest: the most rows staged from the cache for one of its sequences
 struct BfRows {
   int R;
   float *x, *q, *xb;
   const int *token, *pos, *slot;
   int n_tiles; const int *tile_row0, *tile_n; int tile_rows;   // prefill attention tiles (rows per tile: 64 CUDA cores, 128 tensor cores)
-  const int *srow, *spad; int Rs;                              // tensor cores: staged row of every row, rows to zero behind it (gemm_tc.h RopeBf16), staged rows in all
-  const int *seq_slot, *seq_pos0, *seq_base; int n_seqs, longest_context;   // and what the cache holds ahead of the call: positions below seq_pos0, staged from seq_base on
+  const int *srow, *spad; int Rs;                              // tensor cores: staged row of every row, rows to zero behind it (gemm_tc.h RopeBf16), staged rows of the largest group
+  const int *seq_slot, *seq_upto, *seq_base;                   // and what is staged from the cache: positions below seq_upto, from seq_base on
+  const std::vector<BfGroup>* groups;
   int n_out; const int* out_rows;
   float* logits; int* next;
 };
@@ -377,18 +390,22 @@ static int bf_issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, 
     const bool rope_in_attn = io.n_tiles == 0 && !(!io.logits && l == L - 1) && rope_fuse_mode() &&
                               attn_fused_rope_supported(c.n_heads, c.n_kv_heads, hs);
     const bool tc_attn = io.n_tiles > 0 && io.tile_rows == 128;   // prompt rows, head size 64 / 128: Q K^T and P V on the tensor cores (attn_prefill_tc.cu)
-    const RopeBf16 b16 = {reinterpret_cast<uint16_t*>(io.q), sc.k16, sc.v16, io.srow, io.spad};
+    RopeBf16 b16 = {reinterpret_cast<uint16_t*>(io.q), sc.k16, sc.v16, io.srow, io.spad};
+    const bool one_group = tc_attn && io.groups->size() == 1;
+    if (tc_attn && !one_group) b16 = RopeBf16{b16.q, nullptr, nullptr, nullptr, nullptr};   // K and V by the groups, from the cache
     if (!rope_in_attn)
     THA_TRY_RC(rope_scatter_launch(st, pdl, R, sc.part, pl.z_qkv, (long long)R * ld_qkv, ld_qkv, io.pos, d, kvd, hs, rc, rs, io.q,
                                    s.key_cache, s.value_cache, kv_bs, loff, io.slot, &pg, tc_attn ? &b16 : nullptr));
     if (!io.logits && l == L - 1) return THA_STATUS_SUCCESS;   // cache-only ingestion: the last layer's K/V rows are in place
     bool rounded = false;   // the attention kernel already left its output as bf16 rows in sc.xb
     if (tc_attn) {
-      if (io.longest_context > 0)
-        THA_CUDA_OK(launch(bf_kv_context_kernel, dim3(ceil_div(kvd, 512), ceil_div(io.longest_context, 8), io.n_seqs), dim3(256), 0, st, pdl,
-                           kcl, vcl, kv_bs, io.seq_slot, io.seq_pos0, io.seq_base, pg, kvd, sc.k16, sc.v16));
-      THA_TRY_RC(attn_prefill_tc_launch(st, io.n_tiles, R, c.n_heads, c.n_kv_heads, hs, b16.q, sc.xb, io.pos, io.tile_row0, io.tile_n, pdl,
-                                        sc.k16, sc.v16, io.Rs, io.srow));
+      for (const BfGroup& g : *io.groups) {
+        if (g.longest > 0)
+          THA_CUDA_OK(launch(bf_kv_context_kernel, dim3(ceil_div(g.longest, 8), ceil_div(kvd, 512), g.n_seqs), dim3(256), 0, st, pdl, kcl, vcl, kv_bs,
+                             io.seq_slot + g.seq0, io.seq_upto + g.seq0, io.seq_base + g.seq0, (int)!one_group, pg, kvd, sc.k16, sc.v16));
+        THA_TRY_RC(attn_prefill_tc_launch(st, g.n_tiles, R, c.n_heads, c.n_kv_heads, hs, b16.q, sc.xb, io.pos, io.tile_row0 + g.tile0, io.tile_n + g.tile0,
+                                          pdl, sc.k16, sc.v16, io.Rs, io.srow));
+      }
       rounded = true;
     } else if (io.n_tiles > 0)
       THA_TRY_RC(attn_prefill_launch(st, io.n_tiles, c.n_heads, c.n_kv_heads, hs, io.q, io.xb, nullptr, nullptr, kcl,
@@ -470,24 +487,43 @@ int step_bf16_prefill(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
   std::vector<int> tab((size_t)5 * R + 2 * T + 4 * n_seqs);
   int *h_slot = tab.data(), *h_pos = h_slot + R, *h_tok = h_pos + R, *h_t0 = h_tok + R, *h_tn = h_t0 + T, *h_last = h_tn + T;
   int *h_srow = h_last + n_seqs, *h_spad = h_srow + R;   // staged row of every row: a sequence's positions from 0 on, at a multiple of 128
-  int *h_sslot = h_spad + R, *h_spos = h_sslot + n_seqs, *h_sbase = h_spos + n_seqs;
-  int r = 0, t = 0, longest = 0;
-  long long Rs = 0;
+  int *h_sslot = h_spad + R, *h_upto = h_sslot + n_seqs, *h_sbase = h_upto + n_seqs;
+  const long long most = bf_stage_rows(hs * c.n_kv_heads, R);
+  std::vector<BfGroup> groups;
+  int r = 0, t = 0;
+  long long Rs = 0, at = 0;   // staged rows of the largest group, and of the last one so far
+  bool behind = false;        // a portion behind a context
   for (int i = 0; i < n_seqs; i++) {
-    const int end = pos0[i] + len[i];
-    for (int j = 0; j < len[i]; j++) { h_srow[r + j] = (int)Rs + pos0[i] + j; h_spad[r + j] = j + 1 < len[i] ? 0 : -end & 15; }
-    h_sslot[i] = slot[i]; h_spos[i] = pos0[i]; h_sbase[i] = (int)Rs;
-    if (pos0[i] > longest) longest = pos0[i];
-    Rs += ceil_div(end, 128) * 128;
-    if (Rs > INT_MAX) return THA_STATUS_INVALID_ARG;
+    const int end = pos0[i] + len[i], rows = ceil_div(end, 128) * 128;
+    if (i == 0 || at + rows > most) { groups.push_back({i, 0, t, 0, 0}); at = 0; }
+    BfGroup& g = groups.back();
+    g.n_seqs++;
+    if (pos0[i] > g.longest) g.longest = pos0[i];
+    behind = behind || pos0[i] > 0;
+    for (int j = 0; j < len[i]; j++) { h_srow[r + j] = (int)at + pos0[i] + j; h_spad[r + j] = j + 1 < len[i] ? 0 : -end & 15; }
+    h_sslot[i] = slot[i]; h_upto[i] = pos0[i]; h_sbase[i] = (int)at;
+    at += rows;
+    if (at > Rs) Rs = at;
     for (int j = 0; j < len[i]; j += TQ) { h_t0[t] = r + j; h_tn[t] = (len[i] - j < TQ) ? len[i] - j : TQ; t++; }
+    g.n_tiles = t - g.tile0;
     for (int j = 0; j < len[i]; j++, r++) {
       h_slot[r] = slot[i]; h_pos[r] = pos0[i] + j; h_tok[r] = tokens[r];
       if (tokens[r] < 0 || tokens[r] >= c.vocab_size) return THA_STATUS_INVALID_ARG;
     }
     h_last[i] = r - 1;
   }
-  THA_TRY_RC(bf_prepare(ws, c, (int)R, true, (int)tab.size(), TQ == 128 ? (int)Rs : 0));
+  if (groups.size() > 1)   // everything from the cache, with the zeros behind it: the rows that this call brings lie there by then
+    for (BfGroup& g : groups) {
+      g.longest = 0;
+      for (int i = g.seq0; i < g.seq0 + g.n_seqs; i++) {
+        h_upto[i] = pos0[i] + len[i];
+        if (((h_upto[i] + 15) & ~15) > g.longest) g.longest = (h_upto[i] + 15) & ~15;
+      }
+    }
+  // Scratch that grows frees and drops the workspace's graphs: a prompt in portions, which asks for more with each, gets room for whole contexts.
+  long long keep = behind ? (long long)n_seqs * (ceil_div(c.seq_len, 128) * 128) : 0;
+  if (keep > most) keep = most;
+  THA_TRY_RC(bf_prepare(ws, c, (int)R, true, (int)tab.size(), TQ == 128 ? Rs : 0, keep));
   BfScratch sc;
   {
     std::lock_guard<std::mutex> lk(g_bf_mu);
@@ -498,8 +534,8 @@ int step_bf16_prefill(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
   io.R = (int)R; io.x = sc.xr; io.q = sc.qr; io.xb = sc.xbr;
   io.slot = sc.tab; io.pos = sc.tab + R; io.token = sc.tab + 2 * R;
   io.n_tiles = (int)T; io.tile_row0 = sc.tab + 3 * R; io.tile_n = sc.tab + 3 * R + T; io.tile_rows = TQ;
-  io.srow = sc.tab + 3 * R + 2 * T + n_seqs; io.spad = io.srow + R; io.Rs = (int)Rs;
-  io.seq_slot = io.spad + R; io.seq_pos0 = io.seq_slot + n_seqs; io.seq_base = io.seq_pos0 + n_seqs; io.n_seqs = n_seqs; io.longest_context = longest;
+  io.srow = sc.tab + 3 * R + 2 * T + n_seqs; io.spad = io.srow + R; io.Rs = (int)Rs; io.groups = &groups;
+  io.seq_slot = io.spad + R; io.seq_upto = io.seq_slot + n_seqs; io.seq_base = io.seq_upto + n_seqs;
   io.n_out = n_seqs; io.out_rows = sc.tab + 3 * R + 2 * T; io.logits = logits; io.next = logits ? next_d : nullptr;
   return bf_issue_rows(st, ws, c, w, s, io, rc, rs, pdl_enabled() != 0);
 }

@@ -46,3 +46,52 @@ def test_portions_vs_oracle(oracle, tmp_path, name, cuts, lens):
         bits.append(logits.clone())
     pages.close()
     assert torch.equal(bits[0], bits[1])
+
+
+def free():
+    import torch
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+def engine(slots, seq_len, layers):
+    eng, ck = load_pkg("engine"), load_pkg("checkpoint")
+    w = eng.DeviceWeightsBF16.random(ck.Config(512, 768, layers, 4, 4, 96, seq_len), seed=3)
+    e = eng.Engine(w, slots)
+    e.state.key_cache.normal_()
+    e.state.value_cache.normal_()
+    return e
+
+
+def test_scratch_of_many_short_portions_behind_long_contexts_is_bounded():
+    """160 contexts of about 2000 rows are 670 MB of staged rows: they are taken in groups, with the results of calls of 40, which are one group each."""
+    import torch
+    e = engine(160, 2064, 2)
+    rng = np.random.default_rng(0)
+    seqs = [(i, int(rng.integers(1900, 2040)), rng.integers(0, 96, int(rng.integers(1, 20))).astype(np.int32)) for i in range(160)]
+    before = e.state.key_cache.clone(), e.state.value_cache.clone()
+    want, nxt = torch.empty(160, 96, device="cuda"), torch.empty(160, dtype=torch.int32, device="cuda")
+    for i in range(0, 160, 40):
+        e.prefill(seqs[i:i + 40], want[i:i + 40], nxt[i:i + 40])
+    rows = [c.clone() for c in (e.state.key_cache, e.state.value_cache)]
+    e.state.key_cache.copy_(before[0])
+    e.state.value_cache.copy_(before[1])
+    got, had = torch.empty_like(want), free()
+    e.prefill(seqs, got, nxt)
+    assert had - free() < 300 << 20
+    assert load_pkg("cabi").lib().c.tha_gemm_check_error() == 0
+    for i in range(160):
+        assert_close_scaled(got[i].cpu().numpy(), want[i].cpu().numpy(), BF16_EPS, f"sequence {i}")
+    for a, b in zip(rows, (e.state.key_cache, e.state.value_cache)):
+        assert float((a - b).abs().max()) <= BF16_EPS * float(a.abs().max())
+
+
+def test_portions_of_a_prompt_grow_the_scratch_once():
+    """Growing frees, allocates and drops the workspace's graphs."""
+    e = engine(1, 32768, 1)
+    rng = np.random.default_rng(1)
+    left = []
+    for at in range(0, 32768, 4096):
+        e.prefill([(0, at, rng.integers(0, 96, 4096).astype(np.int32))])
+        left.append(free())
+    assert len(set(left[1:])) == 1
