@@ -16,6 +16,7 @@ void set_last_error(const char* where, cudaError_t e);
 int pdl_enabled();     // programmatic dependent launch between the step's kernels
 int graph_enabled();   // capture the decode step into a CUDA graph
 
+#define THA_TRY_RC(expr) do { int _st = (expr); if (_st != THA_STATUS_SUCCESS) return _st; } while (0)
 #define THA_CUDA_OK(expr)                                  \
   do {                                                     \
     cudaError_t _e = (expr);                               \

@@ -515,8 +515,8 @@ extern "C" int tha_gemm_tf32x3(void* stream, float* out, long long ldo, const fl
     auto& e = g_split_scratch[dev];
     const size_t need = (size_t)2 * N * K;
     if (need > e.second) {
-      if (e.first) THA_CUDA_OK(cudaFree(e.first));
-      THA_CUDA_OK(cudaMalloc(&e.first, need * sizeof(float)));
+      e.second = 0;
+      THA_TRY_RC(scratch_replace(&e.first, need));
       e.second = need;
     }
     scratch = e.first;
@@ -565,8 +565,8 @@ int matmul_tc_route(cudaStream_t st, int m, int n, int k, const float* A, const 
     auto& e = g_split_scratch[dev];
     const size_t need = (size_t)n * k + (size_t)2 * m * k;
     if (need > e.second) {
-      if (e.first) THA_CUDA_OK(cudaFree(e.first));
-      THA_CUDA_OK(cudaMalloc(&e.first, need * sizeof(float)));
+      e.second = 0;
+      THA_TRY_RC(scratch_replace(&e.first, need));
       e.second = need;
     }
     scratch = e.first;

@@ -5,8 +5,6 @@
 
 namespace tha {
 
-#define THA_TRY_RC(expr) do { int _st = (expr); if (_st != THA_STATUS_SUCCESS) return _st; } while (0)
-
 struct TcArgs {
   int n_mats;                 // 1..3 stacked weight matrices with the same K
   const float* W[3]; int M[3]; int out_off[3];   // rows of matrix i land at out[n*ldo + out_off[i] + row]

@@ -797,14 +797,14 @@ int mega_step_launch(cudaStream_t st, Workspace* ws, int B, const tha_config_t* 
   if (smax < 1) smax = 1;
   const size_t items = (size_t)B * cfg->n_heads * smax;
   if (items * hs > sc.att_floats || items > sc.att_items || B * cfg->n_heads > sc.cnt_cap) {
-    if (sc.att_acc) { cudaFree(sc.att_acc); cudaFree(sc.att_ml); cudaFree(sc.att_cnt); }
-    sc.att_floats = items * hs; sc.att_items = items; sc.cnt_cap = B * cfg->n_heads;
-    THA_CUDA_OK(cudaMalloc(&sc.att_acc, sc.att_floats * sizeof(float)));
-    THA_CUDA_OK(cudaMalloc(&sc.att_ml, sc.att_items * sizeof(float2)));
-    THA_CUDA_OK(cudaMalloc(&sc.att_cnt, sc.cnt_cap * sizeof(int)));
-    THA_CUDA_OK(cudaMemset(sc.att_cnt, 0, sc.cnt_cap * sizeof(int)));
-    THA_CUDA_OK(cudaDeviceSynchronize());
     ws_drop_graphs(ws);
+    sc.att_floats = sc.att_items = sc.cnt_cap = 0;
+    THA_TRY_RC(scratch_replace(&sc.att_acc, items * hs));
+    THA_TRY_RC(scratch_replace(&sc.att_ml, items));
+    THA_TRY_RC(scratch_replace(&sc.att_cnt, (size_t)B * cfg->n_heads));
+    THA_CUDA_OK(cudaMemset(sc.att_cnt, 0, (size_t)B * cfg->n_heads * sizeof(int)));
+    THA_CUDA_OK(cudaDeviceSynchronize());
+    sc.att_floats = items * hs; sc.att_items = items; sc.cnt_cap = B * cfg->n_heads;
   }
   if (prepare_only) return THA_STATUS_SUCCESS;
 

@@ -227,11 +227,11 @@ static std::mutex g_bf_mu;
 template <typename T>
 static int bf_grow(T** p, size_t* cap, size_t need, Workspace* ws) {
   if (need <= *cap) return THA_STATUS_SUCCESS;
-  if (*p) THA_CUDA_OK(cudaFree(*p));
-  THA_CUDA_OK(cudaMalloc(p, need * sizeof(T)));
-  *cap = need;
   ws_drop_graphs(ws);
   gemm_tc_forget();
+  *cap = 0;
+  THA_TRY_RC(scratch_replace(p, need));
+  *cap = need;
   return THA_STATUS_SUCCESS;
 }
 

@@ -561,11 +561,11 @@ void step_tc_release(Workspace* ws) {
 
 static int grow(float** p, size_t* cap, size_t need, Workspace* ws) {
   if (need <= *cap) return THA_STATUS_SUCCESS;
-  if (*p) THA_CUDA_OK(cudaFree(*p));
-  THA_CUDA_OK(cudaMalloc(p, need * sizeof(float)));
-  *cap = need;
   ws_drop_graphs(ws);   // cached graphs captured the old pointers
   gemm_tc_forget();
+  *cap = 0;
+  THA_TRY_RC(scratch_replace(p, need));
+  *cap = need;
   return THA_STATUS_SUCCESS;
 }
 
@@ -704,28 +704,28 @@ static int prepare_rows(Workspace* ws, const tha_config_t* c, int R, bool prefil
     THA_TRY_RC(grow(&s.ss, &s.n_ss, sf, ws));
     const int stride = ceil_div(ci, 32) * 32, blocks = c->n_layers + 1;
     if (stride > s.ctr_stride || blocks > s.n_ctr_blocks) {
-      if (s.ctr) THA_CUDA_OK(cudaFree(s.ctr));
-      s.ctr_stride = stride > s.ctr_stride ? stride : s.ctr_stride;
-      s.n_ctr_blocks = blocks > s.n_ctr_blocks ? blocks : s.n_ctr_blocks;
-      THA_CUDA_OK(cudaMalloc(&s.ctr, (size_t)s.ctr_stride * s.n_ctr_blocks * sizeof(int)));
-      THA_CUDA_OK(cudaMemset(s.ctr, 0, (size_t)s.ctr_stride * s.n_ctr_blocks * sizeof(int)));   // every launch leaves its block zero again
+      const int new_stride = stride > s.ctr_stride ? stride : s.ctr_stride, new_blocks = blocks > s.n_ctr_blocks ? blocks : s.n_ctr_blocks;
       ws_drop_graphs(ws);
+      s.ctr_stride = s.n_ctr_blocks = 0;
+      THA_TRY_RC(scratch_replace(&s.ctr, (size_t)new_stride * new_blocks));
+      THA_CUDA_OK(cudaMemset(s.ctr, 0, (size_t)new_stride * new_blocks * sizeof(int)));   // every launch leaves its block zero again
+      s.ctr_stride = new_stride; s.n_ctr_blocks = new_blocks;
     }
   }
   THA_TRY_RC(grow(&s.part, &s.n_part, part_need, ws));
   if (R > s.n_b) {
-    if (s.scale) cudaFree(s.scale);
-    THA_CUDA_OK(cudaMalloc(&s.scale, (size_t)R * sizeof(float)));
-    s.n_b = R;
     ws_drop_graphs(ws);
+    s.n_b = 0;
+    THA_TRY_RC(scratch_replace(&s.scale, (size_t)R));
+    s.n_b = R;
   }
   if (prefill) {
     THA_TRY_RC(grow(&s.xr, &s.n_xr, (size_t)R * c->dim, ws));
     THA_TRY_RC(grow(&s.qr, &s.n_qr, (size_t)R * c->dim, ws));
     THA_TRY_RC(grow(&s.xbr, &s.n_xbr, (size_t)R * c->dim, ws));
     if ((size_t)n_tab > s.n_tab) {
-      if (s.tab) THA_CUDA_OK(cudaFree(s.tab));
-      THA_CUDA_OK(cudaMalloc(&s.tab, (size_t)n_tab * sizeof(int)));
+      s.n_tab = 0;
+      THA_TRY_RC(scratch_replace(&s.tab, (size_t)n_tab));
       s.n_tab = n_tab;
     }
     return THA_STATUS_SUCCESS;

@@ -176,31 +176,33 @@ int ws_ensure_dual(Workspace* ws) {
 
 int ws_ensure_attn(Workspace* ws, size_t part_slots, int n_counters) {
   if (part_slots > ws->part_cap) {
-    if (ws->part_acc) { cudaFree(ws->part_acc); cudaFree(ws->part_ml); }
     size_t cap = part_slots + part_slots / 4;
-    THA_CUDA_OK(cudaMalloc(&ws->part_acc, cap * sizeof(float4)));
-    THA_CUDA_OK(cudaMalloc(&ws->part_ml, cap * sizeof(float2)));
-    ws->part_cap = cap;
     ws_drop_graphs(ws);  // cached graphs captured the old pointers
+    ws->part_cap = 0;
+    THA_TRY_RC(scratch_replace(&ws->part_acc, cap));
+    THA_TRY_RC(scratch_replace(&ws->part_ml, cap));
+    ws->part_cap = cap;
   }
   if (n_counters > ws->counters_cap) {
-    if (ws->counters) cudaFree(ws->counters);
     int cap = n_counters * 2;
-    THA_CUDA_OK(cudaMalloc(&ws->counters, cap * sizeof(int)));
+    ws_drop_graphs(ws);
+    ws->counters_cap = 0;
+    THA_TRY_RC(scratch_replace(&ws->counters, (size_t)cap));
     THA_CUDA_OK(cudaMemset(ws->counters, 0, cap * sizeof(int)));
     ws->counters_cap = cap;
-    ws_drop_graphs(ws);
   }
   return THA_STATUS_SUCCESS;
 }
 
 int ws_ensure_tokpos(Workspace* ws, int n_batches) {
   if (n_batches <= ws->tokpos_cap) return THA_STATUS_SUCCESS;
-  if (ws->tok_d) { cudaFree(ws->tok_d); cudaFreeHost(ws->tokpos_h); }
   int cap = n_batches < 64 ? 64 : n_batches * 2;
+  ws_drop_graphs(ws);
+  ws->tokpos_cap = 0;
+  if (ws->tokpos_h) { cudaFreeHost(ws->tokpos_h); ws->tokpos_h = nullptr; }
   // device: [tok | pos | force | reseed (u64) | next | rng (u64)]; the pinned mirror has the same first five blocks, so ONE
   // copy of 5 * cap ints stages everything a sampled step takes from the host (greedy steps copy the first two)
-  THA_CUDA_OK(cudaMalloc(&ws->tok_d, 8 * cap * sizeof(int)));
+  THA_TRY_RC(scratch_replace(&ws->tok_d, (size_t)8 * cap));
   THA_CUDA_OK(cudaMemset(ws->tok_d, 0, 8 * cap * sizeof(int)));
   ws->pos_d = ws->tok_d + cap;
   ws->force_d = ws->tok_d + 2 * cap;
@@ -210,19 +212,18 @@ int ws_ensure_tokpos(Workspace* ws, int n_batches) {
   THA_CUDA_OK(cudaMallocHost(&ws->tokpos_h, 6 * cap * sizeof(int)));
   ws->next_h = ws->tokpos_h + 5 * cap;
   ws->tokpos_cap = cap;
-  ws_drop_graphs(ws);
   return THA_STATUS_SUCCESS;
 }
 
 int ws_ensure_q8(Workspace* ws, int n_batches, int kmax, int gs) {
   const size_t need = (size_t)n_batches * kmax;
   if (need <= ws->q8_cap) return THA_STATUS_SUCCESS;
-  if (ws->q8_xq) { cudaFree(ws->q8_xq); cudaFree(ws->q8_xs); }
-  THA_CUDA_OK(cudaMalloc(&ws->q8_xq, need));
-  (void)gs;   // groups are at least 16 values (the kernel's requirement): need / 16 scales always suffice
-  THA_CUDA_OK(cudaMalloc(&ws->q8_xs, (need / 16 + 1) * sizeof(float)));
-  ws->q8_cap = need;
   ws_drop_graphs(ws);
+  ws->q8_cap = 0;
+  THA_TRY_RC(scratch_replace(&ws->q8_xq, need));
+  (void)gs;   // groups are at least 16 values (the kernel's requirement): need / 16 scales always suffice
+  THA_TRY_RC(scratch_replace(&ws->q8_xs, need / 16 + 1));
+  ws->q8_cap = need;
   return THA_STATUS_SUCCESS;
 }
 

@@ -75,6 +75,22 @@ inline void ws_drop_graphs(Workspace* ws) {
     w->graphs.clear();
   }
 }
+// A scratch array of n elements in place of *p.  The caller has dropped the graphs that hold the old pointer and set the size it knows to 0: when
+// the new array cannot be had, *p is null, and the next call asks again.
+template <typename T>
+int scratch_replace(T** p, size_t n) {
+  T* old = *p;
+  *p = nullptr;
+  if (old) THA_CUDA_OK(cudaFree(old));
+  const cudaError_t e = cudaMalloc((void**)p, n * sizeof(T));
+  if (e != cudaSuccess) {
+    cudaGetLastError();   // not the next launch's error
+    *p = nullptr;
+    set_last_error("scratch allocation", e);
+    return THA_STATUS_EXECUTION_FAILED;
+  }
+  return THA_STATUS_SUCCESS;
+}
 void ws_release(Workspace* ws);        // free everything a (tensor-parallel rank's) workspace owns
 void step_tc_release(Workspace* ws);   // ... and the row pipeline's scratch keyed by it
 int skip_mode();       // bit mask of kernel classes left out of the row pipeline (live-share measurements): 1 layer matmuls, 2 attention,

@@ -95,3 +95,35 @@ def test_portions_of_a_prompt_grow_the_scratch_once():
         e.prefill([(0, at, rng.integers(0, 96, 4096).astype(np.int32))])
         left.append(free())
     assert len(set(left[1:])) == 1
+
+
+def test_a_call_that_finds_no_room_leaves_the_workspace_usable():
+    """Scratch that cannot grow: an error, and the calls behind it allocate again instead of using what was given back."""
+    import torch
+    e = engine(2, 40000, 2)
+    rng = np.random.default_rng(2)
+    small = [(0, 0, rng.integers(0, 96, 40).astype(np.int32)), (1, 3, rng.integers(0, 96, 9).astype(np.int32))]
+    tok, pos = torch.tensor([5, 6], dtype=torch.int32, device="cuda"), torch.tensor([41, 12], dtype=torch.int32, device="cuda")
+
+    def calls():
+        logits, nxt = torch.empty(2, 96, device="cuda"), torch.empty(2, dtype=torch.int32, device="cuda")
+        e.prefill(small, logits, nxt)
+        step = torch.empty(2, 96, device="cuda")
+        e.decode_step(tok, pos, step, nxt, stream=stream)
+        e.decode_step(tok, pos, step, nxt, stream=stream)
+        torch.cuda.synchronize()
+        return torch.stack([logits, step])
+
+    stream = torch.cuda.Stream()
+    want = calls()
+    held = []
+    try:
+        for leave in (600 << 20, 100 << 20):      # some of its arrays fit, then none
+            held.append(torch.empty(max(0, free() - leave), dtype=torch.uint8, device="cuda"))
+            with pytest.raises(Exception):
+                e.prefill([(0, 0, rng.integers(0, 96, 39990).astype(np.int32))] * 4, torch.empty(4, 96, device="cuda"), torch.empty(4, dtype=torch.int32, device="cuda"))
+            torch.cuda.synchronize()
+    finally:
+        held.clear()
+        torch.cuda.empty_cache()
+    assert torch.equal(calls(), want)
