@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) hyb_attn_tc_kernel(const __grid
   auto half_key = [&](int ti) { return ti < tiles.n_a ? tiles.begin + 32 * ti : tiles.resume + 32 * (ti - tiles.n_a); };
   const int BP = REL ? at_rel_pitch(AP, a.rel_n) : 0, pad = at_rel_pad(AP);
 
-  // q, rounded: warp w takes rows w, w + 13, ..; pairs past the block's positions are zeros
+  // q, rounded: warp w takes rows w, w + 10, ..; pairs past the block's positions are zeros
   for (int pr = warp; pr < 2 * AT_ROWS; pr += AT_THREADS / 32) {
     const int pp = pr / AG, hg = pr - pp * AG;
     const bool ok = pp < AP && r0 + pp < r_end;
@@ -258,8 +258,9 @@ __global__ void __launch_bounds__(AT_THREADS, 1) hyb_attn_tc_kernel(const __grid
       for (int hf = 0; hf < 2; hf++) {
         uint32_t s[32];
         at_ld32(t_s + (uint32_t)(b * AT_KEYS + 32 * hf), s);
-        const int ti = 2 * j + hf, kt = half_key(ti);
+        const int ti = 2 * j + hf;
         const bool there = ti < tiles.n;
+        const int kt = half_key(there ? ti : tiles.n - 1);   // behind the last half its own keys again, as fetched: the biases end there
         // every position of the block sees every key of this half
         const bool whole = there && kt + 31 <= p_first && kt >= last_first && (a.window <= 0 || p_last - kt < a.window || kt + 32 <= a.keep_first);
         const bool near = REL && p_first - (kt + 31) < a.rel_n - 1;   // the same for the whole block
