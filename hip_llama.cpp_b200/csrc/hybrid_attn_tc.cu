@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) hyb_attn_tc_kernel(const __grid
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(at_raw) + 1023) & ~(uintptr_t)1023);
   unsigned char* Qs = smem;                          // [group][block][row][128 bytes]
   unsigned char* KVs = Qs + 2 * Q_GROUP;             // [stage][K | V][block][key][128 bytes]
-  float* Bs = reinterpret_cast<float*>(KVs + AT_STAGES * KV_STAGE);   // biases [head][pitch], times log2(e)
+  float* Bs = reinterpret_cast<float*>(KVs + AT_STAGES * KV_STAGE);   // biases [head][pitch]
   __shared__ uint64_t kv_full[AT_STAGES], kv_empty[AT_STAGES], s_full[2][2], p_full[2][2], pv_done[2][2];
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_s;
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) hyb_attn_tc_kernel(const __grid
   if (REL) {
     const int count = min(a.rel_n, p_last + 1) + 2 * pad;   // distances past the block's farthest key are not asked for
     for (int hl = 0; hl < AG; hl++)
-      for (int i = threadIdx.x; i < count; i += AT_THREADS) Bs[hl * BP + i] = hyb_attn_rel(a, g * gsize + hl, i - pad) * LOG2E;
+      for (int i = threadIdx.x; i < count; i += AT_THREADS) Bs[hl * BP + i] = hyb_attn_rel(a, g * gsize + hl, i - pad);
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   __syncthreads();
@@ -241,11 +241,11 @@ __global__ void __launch_bounds__(AT_THREADS, 1) hyb_attn_tc_kernel(const __grid
     const bool row_ok = pp < AP && r0 + pp < r_end;
     const int pos = p_first + pp, first = a.chunk > 0 ? (pos / a.chunk) * a.chunk : 0;
     const float scale = a.scale * ((a.head_scale && row_ok) ? a.head_scale[h] : 1.0f);
-    const float scale2 = scale * LOG2E, two_over_cap = CAP ? 2.0f / a.softcap : 0.f;
-    const float far2 = REL && row_ok ? hyb_attn_rel(a, h, a.rel_n - 1) * LOG2E : 0.f;
+    const float two_over_cap = CAP ? 2.0f / a.softcap : 0.f;
+    const float far = REL && row_ok ? hyb_attn_rel(a, h, a.rel_n - 1) : 0.f;
     const uint32_t lanes = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t t_s = tmem + lanes + (uint32_t)(w * 2 * AT_KEYS), t_o = tmem + lanes + (uint32_t)(4 * AT_KEYS + w * DT);
-    float m = -INFINITY, l = 0.f;
+    float m = -INFINITY, l = 0.f, shift = 0.f;       // weights: 2^(score log2(e) + shift), shift = -m log2(e) rounded; 0 while nothing was seen
     bool ok = true;
     for (int j = 0; j < n && ok; j++) {
       const int b = j & 1;
@@ -270,9 +270,9 @@ __global__ void __launch_bounds__(AT_THREADS, 1) hyb_attn_tc_kernel(const __grid
         for (int i = 0; i < 32; i++) {
           const float sv = __uint_as_float(s[i]);
           float x;
-          if (CAP) x = (a.softcap - __fdividef(2.0f * a.softcap, 1.0f + __expf(sv * scale * two_over_cap))) * LOG2E;
-          else if (REL) x = fmaf(sv, scale2, near ? bias[-i] : far2);
-          else x = sv * scale2;
+          if (CAP) x = a.softcap - __fdividef(2.0f * a.softcap, 1.0f + __expf(sv * scale * two_over_cap));
+          else if (REL) x = fmaf(sv, scale, near ? bias[-i] : far);
+          else x = sv * scale;
           t[32 * hf + i] = x;
         }
         if (!whole) {
@@ -285,8 +285,10 @@ __global__ void __launch_bounds__(AT_THREADS, 1) hyb_attn_tc_kernel(const __grid
       }
       const bool grow = mx > m;                       // also from -inf, where nothing was seen before
       if (__any_sync(THA_FULL_MASK, grow)) {
-        const float m_new = grow ? mx : m, corr = grow ? at_ex2(m - m_new) : 1.0f;
-        m = m_new;
+        const float to = grow ? -mx * LOG2E : shift;
+        const float corr = m > -INFINITY ? at_ex2(to - shift) : grow ? 0.f : 1.f;
+        m = grow ? mx : m;
+        shift = to;
         l *= corr;
         if (j > 0) {   // all products of earlier tiles are in the accumulator
           ok = __all_sync(THA_FULL_MASK, tc_mbar_wait(&pv_done[w][b ^ 1], (unsigned)((j - 1) >> 1) & 1u, abort_flag) && ok);
@@ -302,14 +304,13 @@ __global__ void __launch_bounds__(AT_THREADS, 1) hyb_attn_tc_kernel(const __grid
           }
         }
       }
-      const float shift = m > -INFINITY ? m : 0.f;    // nothing seen yet: every weight is 2^-inf = 0
       float sum = 0.f;
 #pragma unroll
       for (int c = 0; c < AT_KEYS / 2; c += 16) {
         uint32_t hi[16], lo[16];
 #pragma unroll
         for (int i = 0; i < 16; i++) {
-          const float p0 = at_ex2(t[2 * (c + i)] - shift), p1 = at_ex2(t[2 * (c + i) + 1] - shift);
+          const float p0 = at_ex2(fmaf(t[2 * (c + i)], LOG2E, shift)), p1 = at_ex2(fmaf(t[2 * (c + i) + 1], LOG2E, shift));
           hi[i] = at_bf16x2(p0, p1);
           const float h0 = __uint_as_float(hi[i] << 16), h1 = __uint_as_float(hi[i] & 0xFFFF0000u);
           if (EXACT) {   // hi + lo carry 16 mantissa bits of the fp32 weight; the sum adds the fp32 weights themselves
@@ -331,12 +332,12 @@ __global__ void __launch_bounds__(AT_THREADS, 1) hyb_attn_tc_kernel(const __grid
     if (ok) ok = tc_mbar_wait(&pv_done[w][(n - 1) & 1], (unsigned)((n - 1) >> 1) & 1u, abort_flag);
     at_fence_after();
     ok = __all_sync(THA_FULL_MASK, ok);
-    float inv = 1.0f / l;
-    if (a.sink && row_ok) {   // 1 / (l + 2^(sink log2(e) - m)) in a form that cannot overflow
-      const float sk = a.sink[h] * LOG2E, M = fmaxf(m, sk), e = at_ex2(m - M);
-      inv = e / (l * e + at_ex2(sk - M));
+    float inv = 0.f;
+    if (row_ok) {
+      // all weights and their sum carry the factor 2^(m log2(e) + shift) of the rounded shift; the sink is weighed by m itself
+      const float f = m > -INFINITY ? at_ex2(-fmaf(m, LOG2E, shift)) : 1.f;
+      inv = f * hyb_attn_final_factor(a, h, m, l * f, gate ? gate + (size_t)(r0 + pp) * ldg : nullptr);
     }
-    if (gate && row_ok) inv *= hyb_sigmoid(gate[(size_t)(r0 + pp) * ldg + h]);
 #pragma unroll
     for (int c = 0; c < DT; c += 32) {
       uint32_t o[32];

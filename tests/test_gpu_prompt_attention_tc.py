@@ -86,6 +86,36 @@ def test_portions(heads, kv_heads, dim, seqs, form):
     assert lib.c.tha_gemm_check_error() == 0
 
 
+@pytest.mark.parametrize("dim", [64, 128])
+@pytest.mark.parametrize("sink", [False, True])
+def test_large_common_scores(dim, sink):
+    """Scores of 4096 or 8192 and a few units apart, exact in fp32: what is left of the error is the weights' (two bf16, 2^-17 of themselves, over hundreds of
+    keys).  Rounded in other units, as powers of two, such scores would be off by 1e-4 each."""
+    a = H.Attn()
+    a.heads, a.kv_heads, a.dim, a.vdim, a.rot, a.scale, a.out_f32, a.fp32_scores = 16, 16 * 64 // dim, dim, dim, -1, 2.0 ** -5, 1, 1
+    R, g = 1100, torch.Generator(device="cuda").manual_seed(dim)
+    cache = Cache(1, R, a.kv_heads, dim, dim)
+    cache.v = cache.v.bfloat16().float()
+    q = torch.randint(-3, 4, (R, a.heads, dim), device="cuda", generator=g).float()
+    cache.k.copy_(torch.randint(-3, 4, cache.k.shape, device="cuda", generator=g).float())
+    q[..., :dim // 2] = cache.k[..., :dim // 2] = 64.0
+    t = {}
+    if sink:
+        t["sink"] = 64.0 * dim + torch.randint(-2, 6, (a.heads,), device="cuda", generator=g).float()
+        a.sink = t["sink"].data_ptr()
+    seqs = [(0, 0, R)]
+    rows, keep = H.rows_of(seqs)
+    lib = H.lib()
+    lib.c.tha_hyb_attn_gated.argtypes = [H.P, H.I, C.POINTER(H.Attn), C.POINTER(H.Rows), C.POINTER(H.Kv), H.P, H.P, H.P, C.c_size_t, H.P, H.L]
+    out, scratch = torch.empty(R, a.heads, dim, device="cuda"), torch.empty((R + 32) * a.kv_heads * dim + 64, device="cuda")
+    exact = want(a, cache, q, seqs, t)
+    for given in (scratch.numel(), 0):
+        torch.cuda.synchronize()
+        lib.check(lib.c.tha_hyb_attn_gated(None, H.BF16, a, rows, cache.struct(), H.ptr(q), H.ptr(out), H.ptr(scratch) if given else None, given, None, 0))
+        torch.cuda.synchronize()
+        assert rel(out, exact) < 1e-5
+
+
 @pytest.mark.parametrize("lengths", [[64], [100, 128, 64]])
 def test_the_output_product_behind_it(tmp_path, lengths):
     """Whole steps with heads of 64: a block of the attention and one of the product behind it, both of which allocate TMEM, fit an SM side by side."""
