@@ -1846,6 +1846,19 @@ static cudaError_t launch_smem(void (*kernel)(KArgs...), dim3 grid, dim3 block, 
   return launch(kernel, grid, block, smem, s, pdl, args...);
 }
 
+// Keys that the row of the longest context sees at most.
+static int attn_max_keys(const tha_attn_t* a, int max_pos) {
+  const int seen = max_pos + 1;
+  int max_keys = a->chunk > 0 && a->chunk < seen ? a->chunk : seen;
+  if (a->window > 0 && a->window + a->keep_first + 2 * ATT_KEYS < max_keys) max_keys = a->window + a->keep_first + 2 * ATT_KEYS;
+  return max_keys;
+}
+// All that the runs of keys below depend on of max_pos: two tiles each at least, never more than 32 of them.
+int tha::hyb_attn_run_limit(const tha_attn_t* a, int max_pos) {
+  const int n = attn_max_keys(a, max_pos) / (2 * ATT_KEYS);
+  return n < 32 ? n : 32;
+}
+
 extern "C" int tha_hyb_attn_gated(void* stream, int dtype, const tha_attn_t* a, const tha_rows_t* rows, const tha_kv_t* kv, const float* q,
                                   void* out, float* split_scratch, size_t split_scratch_floats, const float* proj, long long ldp) {
   if (rows->n_rows < 1) return THA_STATUS_SUCCESS;
@@ -1869,9 +1882,7 @@ extern "C" int tha_hyb_attn_gated(void* stream, int dtype, const tha_attn_t* a, 
   // position tiles: at most one ragged tile per sequence beyond rows / AP
   const int tiles = rows->n_rows / AP + rows->n_seqs;
   // few blocks and many keys (decoding at long contexts): deal the key tiles of a block to several
-  const int seen = rows->max_pos + 1;
-  int max_keys = a->chunk > 0 && a->chunk < seen ? a->chunk : seen;
-  if (a->window > 0 && a->window + a->keep_first + 2 * ATT_KEYS < max_keys) max_keys = a->window + a->keep_first + 2 * ATT_KEYS;
+  const int max_keys = attn_max_keys(a, rows->max_pos);
   int splits = 1;
   cudaStream_t s = (cudaStream_t)stream;
   auto merge = [&](int which, int n, int parts) -> int {
@@ -1934,7 +1945,7 @@ extern "C" int tha_hyb_attn_gated(void* stream, int dtype, const tha_attn_t* a, 
 }
 
 // THA_HYB_SCAN=shared keeps the shared-memory scans at every head size (A/B aid and the test of that form)
-static bool scan_in_registers() {
+bool tha::hyb_scan_in_registers() {
   const char* v = getenv("THA_HYB_SCAN");
   return !(v && !strcmp(v, "shared"));
 }
@@ -1960,7 +1971,7 @@ extern "C" int tha_hyb_mem_scan(void* stream, int dtype, const tha_mem_t* m, con
   cudaStream_t s = (cudaStream_t)stream;
   THA_CUDA_OK(launch(hyb_mem_gates_kernel, dim3(ceil_div(rows->n_rows * m->heads, 128)), dim3(128), 0, s, pdl_enabled() != 0, proj, ldp, rows->n_rows, m->heads,
                      m->o_i, m->o_f, m->b_i, m->b_f, m->gate_cap));
-  if (m->dim <= 256 && scan_in_registers()) {
+  if (m->dim <= 256 && hyb_scan_in_registers()) {
     const dim3 grid(rows->n_seqs, m->heads, ceil_div(m->vdim, SCW * SCAN_WARPS)), block(32 * SCAN_WARPS);
     if (m->dim <= 32) THA_CUDA_OK(launch(hyb_mem_scan_warp_kernel<1>, grid, block, 0, s, scan_pdl(rows), *m, *rows, *st, proj, ldp, o_raw));
     else if (m->dim <= 64) THA_CUDA_OK(launch(hyb_mem_scan_warp_kernel<2>, grid, block, 0, s, scan_pdl(rows), *m, *rows, *st, proj, ldp, o_raw));
@@ -2029,7 +2040,7 @@ extern "C" int tha_hyb_delta_scan(void* stream, int dtype, const tha_delta_t* d,
     THA_CUDA_OK(launch(hyb_delta_gates_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), 0, s, pdl_enabled() != 0, dt_raw, proj, ldp, rows->n_rows, d->heads,
                        d->dim, d->o_b, d->a_log, d->dt_bias));
   }
-  if (d->dim <= 256 && scan_in_registers()) {
+  if (d->dim <= 256 && hyb_scan_in_registers()) {
     const dim3 grid(rows->n_seqs, d->heads, ceil_div(d->vdim, SCW * SCAN_WARPS)), block(32 * SCAN_WARPS);
     if (d->dim <= 32) THA_CUDA_OK(launch(hyb_delta_scan_warp_kernel<1>, grid, block, 0, s, scan_pdl(rows), *d, *rows, *st, qkv, proj, ldp, dt_raw, o_raw));
     else if (d->dim <= 64) THA_CUDA_OK(launch(hyb_delta_scan_warp_kernel<2>, grid, block, 0, s, scan_pdl(rows), *d, *rows, *st, qkv, proj, ldp, dt_raw, o_raw));

@@ -342,6 +342,15 @@ static int hyb_grow(HybScratch& sc, const tha_hyb_model_t* m, const tha_rows_t* 
   return THA_STATUS_SUCCESS;
 }
 
+// The attention of a latent layer: one key/value head over the cached rows [latent | rotated part]; the values are the latent itself.
+static tha_attn_t latent_attn(const tha_latent_t& a) {
+  tha_attn_t at = {};
+  at.heads = a.heads; at.kv_heads = 1; at.dim = a.kv_rank + a.rot_dim; at.vdim = a.kv_rank; at.rot = -1; at.unit_rms = 0; at.eps = a.eps;
+  at.scale = a.scale; at.chunk = 0; at.cache_layer = a.cache_layer; at.values_in_keys = 1;
+  at.window = a.window; at.sink = a.sink; at.fp32_scores = a.fp32_scores;
+  return at;
+}
+
 // The step's launches, over scratch that is large enough (under its lock).
 static int hyb_issue(void* stream, HybScratch& sc, const tha_hyb_model_t* m, const tha_rows_t* rows, const tha_kv_t* kv, const tha_state_store_t* st, int n_want,
                      const int* want_rows, float* logits, float* taps) {
@@ -505,11 +514,7 @@ static int hyb_issue(void* stream, HybScratch& sc, const tha_hyb_model_t* m, con
       // keys absorbed into the queries: q_abs[h, 0:kv_rank] = W_uk[h]^T q_plain[h]
       HYB_OK(tha_hyb_linear_heads(stream, dt, b.q, (long long)a.heads * DA, DA, b.qplain, (long long)a.heads * a.dim, a.dim, 0, a.w_uk_t,
                                   (long long)a.kv_rank * a.dim, R, a.kv_rank, a.dim, a.heads));
-      // one key/value head over the cached rows [latent | rotated part]; the values are the latent itself
-      tha_attn_t at = {};
-      at.heads = a.heads; at.kv_heads = 1; at.dim = DA; at.vdim = a.kv_rank; at.rot = -1; at.unit_rms = 0; at.eps = a.eps;
-      at.scale = a.scale; at.chunk = 0; at.cache_layer = a.cache_layer; at.values_in_keys = 1;
-      at.window = a.window; at.sink = a.sink; at.fp32_scores = a.fp32_scores;
+      const tha_attn_t at = latent_attn(a);
       tha_kv_t lkv = *kv;
       lkv.v_pool = kv->k_pool;
       HYB_OK(tha_hyb_attn(stream, dt, &at, rows, &lkv, b.q, b.abuf, b.split_floats ? b.split : nullptr, b.split_floats));
@@ -701,14 +706,23 @@ extern "C" int tha_hyb_step(void* stream, const tha_hyb_model_t* m, const tha_ro
 
 // ---- decode-sized steps as executable graphs ---------------------------------------------------------------------------
 // A step of one row per sequence is 24 to 60 kernels of 2 to 10 us, and issuing one takes the host 2 to 3 us.  As a graph, us a step of ServingEngine.step
-// with its copies: four layers of retention, windowed attention and key-value memory (width 1024, 3 requests, 52 kernels) 277 -> 242; two attention
-// layers of width 2048 (2 requests, 24 kernels) 216 -> 195.  A step is captured when it comes a second time in the same form (15 us more, once).
-struct HybGraph { std::vector<unsigned char> key; cudaGraphExec_t exec; int launches; unsigned long long last_use; };
-constexpr size_t HYB_MAX_GRAPHS = 8;
+// with its copies: four layers of retention, windowed attention and key-value memory (width 1024, 3 requests, 52 kernels) 284 -> 242; two attention
+// layers of width 2048 (3 requests, 24 kernels) 226 -> 204.  Capturing, instantiating and uploading take 350 us for the first and 190 for the second, as
+// much as nine replays save: a form is captured when it has been issued ten times, so that requests of a few tokens, and batches that keep changing,
+// do not pay for graphs that they do not use.
+struct HybForm {
+  std::vector<unsigned char> key;
+  cudaGraphExec_t exec;
+  int launches, issued;
+  bool refused;               // its capture failed: always issued
+  unsigned long long last_use;
+};
+constexpr size_t HYB_MAX_FORMS = 64;
+constexpr int HYB_CAPTURE_AFTER = 10;
 struct tha_hyb_plan {
-  std::vector<HybGraph> graphs;
-  std::vector<unsigned char> last;   // the form of the last step that was issued kernel by kernel
+  std::vector<HybForm> forms;   // the least recently used one goes first
   unsigned long long clock = 0;
+  long long captured = 0, replayed = 0;
 };
 
 extern "C" int tha_hyb_plan_create(tha_hyb_plan_t** plan) {
@@ -718,65 +732,87 @@ extern "C" int tha_hyb_plan_create(tha_hyb_plan_t** plan) {
 }
 extern "C" void tha_hyb_plan_destroy(tha_hyb_plan_t* plan) {
   if (!plan) return;
-  for (HybGraph& g : plan->graphs) cudaGraphExecDestroy(g.exec);
+  for (HybForm& f : plan->forms)
+    if (f.exec) cudaGraphExecDestroy(f.exec);
   delete plan;
+}
+extern "C" void tha_hyb_plan_counts(const tha_hyb_plan_t* plan, long long* captured, long long* replayed) {
+  if (captured) *captured = plan ? plan->captured : 0;
+  if (replayed) *replayed = plan ? plan->replayed : 0;
 }
 
 extern "C" int tha_hyb_step_planned(void* stream, tha_hyb_plan_t* plan, const tha_hyb_model_t* m, const tha_rows_t* rows, const tha_kv_t* kv,
                                     const tha_state_store_t* st, int n_want, const int* want_rows, float* logits) {
   if (!m || !rows || !kv || !st || m->n_rot > 64) return THA_STATUS_INVALID_ARG;
   cudaStream_t s = (cudaStream_t)stream;
-  if (!plan || !graph_enabled() || !s || s == cudaStreamLegacy || rows->n_rows < 1 || rows->max_seq_rows != 1)
-    return tha_hyb_step(stream, m, rows, kv, st, n_want, want_rows, logits, nullptr);
-  // The longest context sizes the attention's splits only: a step stands for all of up to the next multiple of 256.
-  tha_rows_t r = *rows;
-  r.max_pos |= 255;
+  bool plain = !plan || !graph_enabled() || !s || s == cudaStreamLegacy || rows->n_rows < 1 || rows->max_seq_rows != 1;
+  if (!plain) {   // nor within a capture of the caller's
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    THA_CUDA_OK(cudaStreamIsCapturing(s, &cap));
+    plain = cap != cudaStreamCaptureStatusNone;
+  }
+  if (plain) return tha_hyb_step(stream, m, rows, kv, st, n_want, want_rows, logits, nullptr);
   HybScratch* sc = hyb_scratch_of_device();
   if (!sc) return THA_STATUS_EXECUTION_FAILED;
   std::lock_guard<std::mutex> lock(sc->mu);
-  HYB_OK(hyb_grow(*sc, m, &r, n_want));
-  std::vector<unsigned char> key;   // every value that the launches depend on, field by field
-  key.reserve(256);
+  HYB_OK(hyb_grow(*sc, m, rows, n_want));
+  // Every value that the launches depend on, field by field; the arrays' contents are read on the device.  Of the longest context: the runs of keys that the
+  // attention is cut into and the rows that it stages.
+  std::vector<unsigned char> key;
+  key.reserve(512);
   auto put = [&](auto v) { const unsigned char* b = reinterpret_cast<const unsigned char*>(&v); key.insert(key.end(), b, b + sizeof(v)); };
-  put(m); put(stream); put(sc->base); put(want_rows); put(logits); put(n_want); put(pdl_enabled());
-  put(r.n_rows); put(r.n_seqs); put(r.token); put(r.pos); put(r.row_seq); put(r.seq_first); put(r.seq_slot); put(r.max_pos);
+  put(m); put(stream); put(sc->base); put(want_rows); put(logits); put(n_want); put(pdl_enabled()); put(hyb_scan_in_registers()); put(hyb_expert_rows());
+  put(rows->n_rows); put(rows->n_seqs); put(rows->token); put(rows->pos); put(rows->row_seq); put(rows->seq_first); put(rows->seq_slot);
   put(kv->k_pool); put(kv->v_pool); put(kv->table); put(kv->table_stride); put(kv->block_size); put(kv->n_cache_layers); put(kv->kv_dim);
   put(st->base); put(st->slot_floats);
-  HybGraph* hit = nullptr;
-  for (HybGraph& g : plan->graphs)
-    if (g.key == key) hit = &g;
-  if (!hit && plan->last == key) {
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    const int before = launches_get();
-    if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-      const int rc = hyb_issue(stream, *sc, m, &r, kv, st, n_want, want_rows, logits, nullptr);
-      const cudaError_t e = cudaStreamEndCapture(s, &graph);
-      if (rc != THA_STATUS_SUCCESS || e != cudaSuccess || cudaGraphInstantiate(&exec, graph, 0) != cudaSuccess) exec = nullptr;
-      if (graph) cudaGraphDestroy(graph);
-    }
-    const int launches = launches_get() - before;
-    count_launch(-launches);
-    if (exec) {
-      if (plan->graphs.size() >= HYB_MAX_GRAPHS) {
-        size_t old = 0;
-        for (size_t i = 1; i < plan->graphs.size(); i++)
-          if (plan->graphs[i].last_use < plan->graphs[old].last_use) old = i;
-        cudaGraphExecDestroy(plan->graphs[old].exec);
-        plan->graphs.erase(plan->graphs.begin() + old);
-      }
-      plan->graphs.push_back({key, exec, launches, 0});
-      hit = &plan->graphs.back();
-    } else {
-      cudaGetLastError();   // not capturable after all: kernel by kernel
-    }
+  for (int li = 0; li < m->n_layers; li++) {
+    const tha_hyb_layer_t& L = m->layers[li];
+    tha_attn_t at = L.attn;
+    if (L.mixer == THA_MIX_LATENT) at = latent_attn(L.latent);
+    else if (L.mixer != THA_MIX_ATTN && L.mixer != THA_MIX_ATTN_GDELTA && L.mixer != THA_MIX_PARALLEL) continue;
+    put(hyb_attn_run_limit(&at, rows->max_pos));
+    put(hyb_attn_tc_scratch(&at, rows));
   }
-  if (hit) {
-    hit->last_use = ++plan->clock;
-    count_launch(hit->launches);
-    THA_CUDA_OK(cudaGraphLaunch(hit->exec, s));
+  HybForm* f = nullptr;
+  for (HybForm& x : plan->forms)
+    if (x.key == key) f = &x;
+  if (!f) {
+    if (plan->forms.size() >= HYB_MAX_FORMS) {
+      size_t old = 0;
+      for (size_t i = 1; i < plan->forms.size(); i++)
+        if (plan->forms[i].last_use < plan->forms[old].last_use) old = i;
+      if (plan->forms[old].exec) cudaGraphExecDestroy(plan->forms[old].exec);
+      plan->forms.erase(plan->forms.begin() + old);
+    }
+    plan->forms.push_back({std::move(key), nullptr, 0, 0, false, 0});
+    f = &plan->forms.back();
+  }
+  f->last_use = ++plan->clock;
+  if (f->exec) {
+    count_launch(f->launches);
+    plan->replayed++;
+    THA_CUDA_OK(cudaGraphLaunch(f->exec, s));
     return THA_STATUS_SUCCESS;
   }
-  plan->last = key;
-  return hyb_issue(stream, *sc, m, &r, kv, st, n_want, want_rows, logits, nullptr);
+  HYB_OK(hyb_issue(stream, *sc, m, rows, kv, st, n_want, want_rows, logits, nullptr));
+  if (f->refused || ++f->issued < HYB_CAPTURE_AFTER) return THA_STATUS_SUCCESS;
+  // captured for the next time while the device works on this one
+  cudaGraph_t graph = nullptr;
+  const int before = launches_get();
+  if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+    const int rc = hyb_issue(stream, *sc, m, rows, kv, st, n_want, want_rows, logits, nullptr);
+    const cudaError_t e = cudaStreamEndCapture(s, &graph);
+    if (rc != THA_STATUS_SUCCESS || e != cudaSuccess || cudaGraphInstantiate(&f->exec, graph, 0) != cudaSuccess) f->exec = nullptr;
+    if (graph) cudaGraphDestroy(graph);
+  }
+  f->launches = launches_get() - before;
+  count_launch(-f->launches);
+  if (f->exec) {
+    plan->captured++;
+    if (cudaGraphUpload(f->exec, s) != cudaSuccess) cudaGetLastError();   // the first launch does it then
+  } else {
+    f->refused = true;      // not capturable after all
+    cudaGetLastError();
+  }
+  return THA_STATUS_SUCCESS;
 }

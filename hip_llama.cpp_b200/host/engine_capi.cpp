@@ -41,6 +41,7 @@ extern "C" int thaEngineVocab(tha_engine_t* e) { return e->model->vocab(); }
 extern "C" int thaEngineWidth(tha_engine_t* e) { return e->model->device_model()->width; }
 extern "C" int thaEngineLayers(tha_engine_t* e) { return e->model->device_model()->n_layers; }
 extern "C" long long thaEngineFreeBlocks(tha_engine_t* e) { return (long long)e->engine->free_blocks(); }
+extern "C" long long thaEngineReplayedSteps(tha_engine_t* e) { return e->engine->replayed_steps(); }
 extern "C" int thaEngineSlot(tha_engine_t* e, const char* id) { return e->engine->slot(id); }
 extern "C" long long thaEngineSteps(tha_engine_t* e) { return e->engine->steps_run(); }
 

@@ -43,6 +43,8 @@ def host_lib():
         lib.thaEngineFreeBlocks.restype = C.c_longlong
         lib.thaEngineSteps.argtypes = [vp]
         lib.thaEngineSteps.restype = C.c_longlong
+        lib.thaEngineReplayedSteps.argtypes = [vp]
+        lib.thaEngineReplayedSteps.restype = C.c_longlong
         lib.thaEngineSlot.argtypes = [vp, C.c_char_p]
         lib.thaEngineStep.argtypes = [vp, I, C.POINTER(C.c_char_p), vp, vp, vp, vp, vp, vp]
         lib.thaEngineFinish.argtypes = [vp, C.c_char_p]
@@ -119,6 +121,10 @@ class ServingEngine:
 
     def steps_run(self) -> int:
         return int(self.lib.thaEngineSteps(self.h))
+
+    def replayed_steps(self) -> int:
+        """Decode steps that ran as executable graphs."""
+        return int(self.lib.thaEngineReplayedSteps(self.h))
 
     def generate(self, prompts, max_new, temperature: float = 0.0, topp: float = 0.9, seed: int = 1, portion: int = 256):
         lens = np.array([len(p) for p in prompts], np.int32)

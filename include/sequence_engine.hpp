@@ -53,6 +53,7 @@ class SequenceEngine {
   void finish(const std::string& id);
   int live() const { return (int)slot_of_.size(); }
   int position(const std::string& id) const;   // tokens the request has been fed so far, -1 if unknown
+  long long replayed_steps() const { long long n = 0; tha_hyb_plan_counts(plan_, nullptr, &n); return n; }   // decode steps that ran as graphs
   size_t free_blocks() const { return bm_.free_blocks(); }
   int slot(const std::string& id) const;       // -1 if not live
 

@@ -35,6 +35,7 @@ int thaEngineFinish(tha_engine_t* e, const char* id);
 int thaEngineGenerate(tha_engine_t* e, int n_requests, const int* prompt_lens, const int* prompts, const int* max_new,
                       float temperature, float topp, unsigned long long seed, int portion, int* out_tokens);
 long long thaEngineSteps(tha_engine_t* e);
+long long thaEngineReplayedSteps(tha_engine_t* e);   /* decode steps that ran as executable graphs */
 
 #ifdef __cplusplus
 }

@@ -449,12 +449,13 @@ int tha_hyb_step(void* stream, const tha_hyb_model_t* m, const tha_rows_t* rows,
                  const tha_state_store_t* st, int n_want, const int* want_rows, float* logits, float* taps);
 
 /* The same step for a serving loop, which repeats steps of one row per sequence: a plan keeps such steps as executable graphs (a step of
- * another size, a context past another 256 positions or regrown scratch makes another; eight at most) and replays them; every other
- * step is tha_hyb_step.  All arrays and the cache may hold new values in every call.  A plan belongs to one model, whose
+ * another size, a context that its attention cuts into more runs of keys or regrown scratch makes another; 64 forms at most) and replays them once a
+ * form has been issued a few times; every other step is tha_hyb_step.  The launches are the same, and so are the results.  All arrays and the cache may hold new values in every call.  A plan belongs to one model, whose
  * descriptions do not change while it lives, to one device and to one thread at a time; plan == NULL: tha_hyb_step. */
 typedef struct tha_hyb_plan tha_hyb_plan_t;
 int tha_hyb_plan_create(tha_hyb_plan_t** plan);
 void tha_hyb_plan_destroy(tha_hyb_plan_t* plan);   /* behind the last step that was issued with it */
+void tha_hyb_plan_counts(const tha_hyb_plan_t* plan, long long* captured, long long* replayed);   /* graphs made and steps replayed so far */
 int tha_hyb_step_planned(void* stream, tha_hyb_plan_t* plan, const tha_hyb_model_t* m, const tha_rows_t* rows, const tha_kv_t* kv,
                          const tha_state_store_t* st, int n_want, const int* want_rows, float* logits);
 
