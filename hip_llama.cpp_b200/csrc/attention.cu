@@ -634,6 +634,9 @@ namespace tha {
 
 int attn_fused_nsplit(int B, int nseg, int seq_len);
 
+static int attn_sms();
+// the deep form: one wave of two CTAs of eight warps an SM
+static bool attn_deep_ok(int ctas, int nw) { return nw == 8 && ctas <= 2 * attn_sms(); }
 static int attn_sms() {
   static int sms = 0;
   if (!sms) { int dev = 0, n = 148; if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev); sms = n; }
@@ -688,13 +691,40 @@ int attn_fused_nsplit(int B, int nseg, int seq_len) {
   return target;
 }
 
-// attn_stream_kernel or attn_fused_kernel: both give the same bits.  The persistent CTAs hold 24 warps; where attn_fused_kernel would have more on an SM at once
-// (25 .. 32: as many as its registers allow), uniform contexts keep it at the bandwidth of HBM and the persistent kernel, which then needs a second
-// round, loses (16 slots at 500: 244 -> 273 us a step; 158 slots of stories110M at 106: 934 -> 1049), while ragged long ones gain (64 slots at 357 .. 1239: 1132 -> 806;
-// 15 at 27 .. 965: 332 -> 309).  Positions are on the device; the length of the cache stands for them.  Below 25 warps an SM it gains or is even: 44 drawn steps,
-// ratio 0.96 to 1.40, 1.05 on average.
-static bool attn_stream_ok(int B, int nseg, int nsplit, int nw, int seq_len) {
-  return nsplit == 1 && B <= AS_MAX_SLOTS && nw >= 2 && AS_WARPS % nw == 0 && sm_budget() >= attn_sms() && (B * nseg <= AS_WARPS / nw * attn_sms() || seq_len >= 1024);
+// attn_stream_kernel or attn_fused_kernel (either form): all give the same bits.  Where the line lies depends on the contexts: the persistent kernel
+// evens out ragged ones, but its 210 KB an SM keep the next product's blocks, and the weights that they ask for ahead, off the SM until it is done, and a
+// last round of few pairs over its 24 warps an SM costs a whole one.  Measured on 1451 steps (two layers of Llama-2-7B, stories110M, stories42M;
+// fp32, Q8_0, bf16; 5 .. 200 slots at uniform and ragged contexts of 5 .. 2000), time of the fused one over the persistent one's: 0.85 .. 2.05, 1.039 on
+// average; this rule takes the persistent one where that is 0.98 .. 2.05 and gains 1.055 on average, of 1.064 if each step took the better.  The classes:
+//   Q8_0, and bf16 at narrow rows, in groups of less than eight warps (the products' rings leave the fused kernel's loads little L1): 0.98 .. 2.05 from 200
+//     positions on average on
+//   else where the pairs fill less than two thirds of their rounds: 0.86 .. 1.06 at uniform contexts, 0.91 .. 1.14 with some spread, 1.00 .. 1.36 with the
+//     longest half the mean above it, and 200 positions
+//   Q8_0 at narrow rows, and fp32 at wide ones where the alternative is the deep form: 0.97 .. 1.05 below 100 positions, 1.00 .. 1.47 above
+//   else against the deep form: 0.85 .. 1.09 with less than 450 positions between mean and longest, 0.99 .. 1.12 with more
+//   otherwise: 0.93 .. 1.17 below, 0.99 .. 1.55 above a mean of 1500, to which each position between mean and longest adds twelve
+// A step whose positions are on the device goes by what the last one of as many slots reported (1 us a step), and the first by the fused kernel.
+int context_class(int longest, long long sum, int slots) {
+  const long long mean = slots > 0 ? sum / slots : 0, spread = longest - mean;
+  return (longest >= 100 ? CTX_LONG : 0) | (mean >= 200 ? CTX_FILLED : 0) | (mean + 12 * spread >= 1500 ? CTX_RAGGED : 0) | (spread >= 450 ? CTX_SPREAD : 0) |
+         (spread >= 200 && 2 * longest >= 3 * mean ? CTX_SKEWED : 0);
+}
+static bool attn_stream_ok(const AttnP& p, int B, int nw, int contexts) {
+  if (p.nsplit != 1 || B > AS_MAX_SLOTS || nw < 2 || AS_WARPS % nw || sm_budget() < attn_sms()) return false;
+  const int pairs = B * p.nseg, at_once = AS_WARPS / nw * attn_sms();
+  const bool q8 = p.out_q, b16 = p.rp.out_b16, wide = p.kv_dim >= 2048, deep = attn_deep_ok(pairs, nw);
+  if (nw < 8 && (q8 || (b16 && !wide)) && (contexts & CTX_FILLED)) return true;
+  if (!deep && 3 * pairs < 2 * ceil_div(pairs, at_once) * at_once) return contexts & CTX_SKEWED;
+  if (q8 ? !wide : wide && deep && !b16) return contexts & CTX_LONG;
+  return contexts & (deep ? CTX_SPREAD : CTX_RAGGED);
+}
+
+// Where a step of B slots tells its contexts; nullptr: it does not, or has no such choice.
+unsigned long long* attn_report_to(Workspace* ws, int B, int n_heads, int n_kv_heads, int head_size, int seq_len) {
+  const int dim = n_heads * head_size;
+  const bool choice = (ws->step_contexts & CTX_REPORT) && fused_J(n_heads, head_size, dim, n_heads / n_kv_heads) == 1 &&
+                      attn_fused_nsplit(B, dim / 128, seq_len) == 1 && sm_budget() >= attn_sms();
+  return choice ? ws->contexts_h + B : nullptr;
 }
 
 // Warps per CTA.  Eight, unless the grid (one CTA per slot and segment, unsplit) would then need more than one wave of
@@ -753,15 +783,19 @@ static int attn_fused_launch_impl(cudaStream_t stream, Workspace* ws, int B, con
     case 7: k = attn_fused_kernel<7>; break; case 8: k = attn_fused_kernel<8>; break;
   }
   const int nw = attn_pick_warps(k, J, (long long)B * p.nseg * p.nsplit);
-  if (rp && J == 1 && attn_stream_ok(B, p.nseg, p.nsplit, nw, seq_len)) {
+  ws->attn_form = ATTN_FUSED;
+  if (rp && J == 1 && attn_stream_ok(p, B, nw, ws->step_contexts)) {
+    ws->attn_form = ATTN_STREAM;
     const int pairs = B * p.nseg, sms = attn_sms();
     p.sorted = pairs > AS_WARPS / nw * sms;   // one round: the order does not matter
     THA_CUDA_OK(cudaFuncSetAttribute(attn_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, AS_SMEM));
     THA_CUDA_OK(launch(attn_stream_kernel, dim3(pairs < sms ? pairs : sms), dim3(32 * AS_WARPS), (size_t)AS_SMEM, stream, pdl, p, B, nw));
     return THA_STATUS_SUCCESS;
   }
-  // few CTAs (nw is then 8): the deep form, in one wave of two an SM
-  if (rp && J == 1 && nw == 8 && B * p.nseg * p.nsplit <= 2 * attn_sms()) k = attn_fused_kernel<1, true, true>;
+  if (rp && J == 1 && attn_deep_ok(B * p.nseg * p.nsplit, nw)) {
+    k = attn_fused_kernel<1, true, true>;
+    ws->attn_form = ATTN_DEEP;
+  }
   dim3 grid(B, p.nseg, p.nsplit), block(32 * nw);
   const size_t smem = (size_t)nw * F * (sizeof(float4) + sizeof(float2));
   if (smem > 40 * 1024) THA_CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));

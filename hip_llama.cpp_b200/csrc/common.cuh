@@ -92,6 +92,18 @@ __device__ __forceinline__ long long kv_paged_off(const KvPaged& g, int slot, in
 
 // Wait until the kernels this launch depends on have completed and their writes are
 // visible (no-op when the launch carried no programmatic attribute).
+// Longest and mean of n contexts to the host (workspace.h contexts_h), by one warp
+__device__ __forceinline__ void report_contexts(const int* pos, int n, unsigned long long* out) {
+  int longest = 0, sum = 0;
+  for (int i = threadIdx.x & 31; i < n; i += 32) {
+    const int t = max(pos[i], 0);
+    longest = max(longest, t);
+    sum += t;
+  }
+  longest = __reduce_max_sync(THA_FULL_MASK, longest);
+  sum = __reduce_add_sync(THA_FULL_MASK, sum);
+  if ((threadIdx.x & 31) == 0) *reinterpret_cast<volatile unsigned long long*>(out) = (unsigned long long)longest << 32 | (unsigned)(sum / n);
+}
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Allow the next kernel in the stream to start launching.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }

@@ -68,6 +68,20 @@ int sample_launch(cudaStream_t st, int B, float* logits, int vocab, float temper
                   const unsigned long long* reseed, const int* force, const int* pos, int* next, bool pdl);
 
 static thread_local int g_last_step_launches = 0;
+static thread_local int g_last_step_attention = 0;   // ATTN_*
+// CTX_* of the step that this thread is about to take, where the caller gave host positions; -1: they are on the device
+static thread_local int g_host_contexts = -1;
+struct HostContexts {
+  HostContexts(const int* pos, int B) {
+    int longest = 0;
+    long long sum = 0;
+    for (int b = 0; b < B; b++)
+      if (pos[b] > 0) { sum += pos[b]; if (pos[b] > longest) longest = pos[b]; }
+    g_host_contexts = context_class(longest, sum, B);
+  }
+  ~HostContexts() { g_host_contexts = -1; }
+};
+static int step_contexts(Workspace* ws, int B) { return g_host_contexts >= 0 ? g_host_contexts : ws_reported_contexts(ws, B); }
 #define THA_TRY_RC2(expr) do { int _st = (expr); if (_st != THA_STATUS_SUCCESS) return _st; } while (0)
 
 // A step of R >= dual_min_rows() rows is issued as TWO concurrent branches of half the rows each (fork / join inside the
@@ -104,7 +118,7 @@ static tha_state_t state_rows(const tha_state_t& s, const tha_config_t& c, int r
 
 struct StepArgs {
   int B; tha_config_t cfg; tha_weights_f32_t w; tha_state_t s;
-  const int* token_d; const int* pos_d; float* logits_d; int* next_d; int pdl; int mega; int advance;
+  const int* token_d; const int* pos_d; float* logits_d; int* next_d; int pdl; int mega; int advance; int contexts;
 };
 
 static unsigned long long fnv1a(const void* data, size_t n, unsigned long long h = 1469598103934665603ull) {
@@ -119,8 +133,10 @@ static unsigned long long fnv1a(const void* data, size_t n, unsigned long long h
 // Issue the step directly, or (default) capture it once per distinct argument set into a
 // CUDA graph and replay it.  `key`/`key_len`: every value the launches depend on.
 template <typename IssueFn>
-static int run_step(cudaStream_t st, Workspace* ws, const void* key_data, size_t key_len, IssueFn issue, bool do_launch = true) {
+static int run_step(cudaStream_t st, Workspace* ws, const void* key_data, size_t key_len, IssueFn issue, bool do_launch = true, int contexts = 0) {
   std::lock_guard<std::mutex> guard(ws->mu);
+  ws->step_contexts = contexts;
+  ws->attn_form = 0;
   if (!ws->step_done) THA_CUDA_OK(cudaEventCreateWithFlags(&ws->step_done, cudaEventDisableTiming));
   else if (ws->last_stream != st) THA_CUDA_OK(cudaStreamWaitEvent(st, ws->step_done, 0));   // the previous step (another stream) still owns the scratch
   ws->last_stream = st;
@@ -134,6 +150,7 @@ static int run_step(cudaStream_t st, Workspace* ws, const void* key_data, size_t
     if (!do_launch) return THA_STATUS_SUCCESS;
     int rc2 = issue();
     g_last_step_launches = launches_get();
+    g_last_step_attention = ws->attn_form;
     return rc2;
   }
   // The cache is keyed by a hash of the argument bytes; a hit is only trusted after comparing the bytes themselves (the
@@ -162,6 +179,7 @@ static int run_step(cudaStream_t st, Workspace* ws, const void* key_data, size_t
     if (e != cudaSuccess) { set_last_error("cudaStreamEndCapture", e); return THA_STATUS_EXECUTION_FAILED; }
     StepGraph sg;
     sg.launches = launches_get();
+    sg.attn_form = ws->attn_form;
     sg.key.assign(static_cast<const unsigned char*>(key_data), static_cast<const unsigned char*>(key_data) + key_len);
     e = cudaGraphInstantiate(&sg.exec, graph, 0);
     cudaGraphDestroy(graph);
@@ -172,6 +190,7 @@ static int run_step(cudaStream_t st, Workspace* ws, const void* key_data, size_t
   if (do_launch) THA_CUDA_OK(cudaGraphLaunch(it->second.exec, st));
   else if (fresh) THA_CUDA_OK(cudaGraphUpload(it->second.exec, st));   // prepare only: the executable graph is resident, nothing runs
   g_last_step_launches = it->second.launches;
+  g_last_step_attention = it->second.attn_form;
   return THA_STATUS_SUCCESS;
 }
 
@@ -283,6 +302,7 @@ int decode_step_f32(cudaStream_t st, int B, const tha_config_t* cfg, const tha_w
     THA_TRY(step_tc_prepare(ws, cfg, dp.B0));
     if (dp.on) THA_TRY(step_tc_prepare(dp.ws2, cfg, dp.B1));
     a.mega = dp.on ? 3 : 2;   // part of the graph key
+    a.contexts = dp.on ? 0 : step_contexts(ws, B);   // so is this
     float* lg = logits_d ? logits_d : s->logits;
     return run_step(st, ws, &a, sizeof(a), [&]() {
       const bool pdl = a.pdl != 0;
@@ -300,7 +320,7 @@ int decode_step_f32(cudaStream_t st, int B, const tha_config_t* cfg, const tha_w
       if (advance) THA_TRY(advance_launch(st, dp.B0, const_cast<int*>(token_d), const_cast<int*>(pos_d), next_d, cfg->seq_len, pdl));
       if (dp.on) THA_CUDA_OK(cudaStreamWaitEvent(st, ws->ev_join, 0));
       return (int)THA_STATUS_SUCCESS;
-    });
+    }, true, a.contexts);
   }
   const bool fused = attn_fused_supported(cfg->n_heads, hs, cfg->dim, kvd);
   if (!fused && !s->att) return THA_STATUS_INVALID_ARG;
@@ -319,7 +339,7 @@ int q8_prep_launch(cudaStream_t st, int B, const float* X, int x_stride, const f
 
 struct StepArgsQ8 {
   int B; tha_config_t cfg; tha_weights_q8_t w; tha_state_t s;
-  const int* token_d; const int* pos_d; float* logits_d; int* next_d; int pdl; int tc;
+  const int* token_d; const int* pos_d; float* logits_d; int* next_d; int pdl; int tc; int contexts;
 };
 
 // runq.c:344-481 with the same 5-kernels-per-layer structure; every matmul kernel
@@ -426,6 +446,7 @@ int decode_step_q8(cudaStream_t st, int B, const tha_config_t* cfg, const tha_we
     THA_TRY(step_tc_q8_prepare(ws, cfg, dp.B0, gs));
     if (dp.on) THA_TRY(step_tc_q8_prepare(dp.ws2, cfg, dp.B1, gs));
     a.tc = dp.on ? 2 : 1;   // part of the graph key
+    a.contexts = dp.on ? 0 : step_contexts(ws, B);   // so is this
     float* lg = logits_d ? logits_d : s->logits;
     if (!lg) return THA_STATUS_INVALID_ARG;
     return run_step(st, ws, &a, sizeof(a), [&]() {
@@ -441,7 +462,7 @@ int decode_step_q8(cudaStream_t st, int B, const tha_config_t* cfg, const tha_we
       THA_TRY(step_tc_q8_issue(st, ws, dp.B0, *cfg, *w, *s, token_d, pos_d, lg, next_d, rc, rs, pdl));
       if (dp.on) THA_CUDA_OK(cudaStreamWaitEvent(st, ws->ev_join, 0));
       return (int)THA_STATUS_SUCCESS;
-    });
+    }, true, a.contexts);
   }
   if (kv_pool_find(s->key_cache, nullptr)) return THA_STATUS_NOT_SUPPORTED;   // paged KV: tensor-core row pipeline only
   const bool fused = attn_fused_supported(cfg->n_heads, hs, cfg->dim, kvd);
@@ -466,7 +487,7 @@ int gemv_bf16_launch(cudaStream_t stream, int mode, const GemvP& p, bool pdl);
 
 struct StepArgsBf16 {
   int B; tha_config_t cfg; tha_weights_bf16_t w; tha_state_t s;
-  const int* token_d; const int* pos_d; float* logits_d; int* next_d; int pdl; int gemv;
+  const int* token_d; const int* pos_d; float* logits_d; int* next_d; int pdl; int gemv; int contexts;
 };
 
 // 1-8 slots: the five fused kernels per layer of issue_step_f32 over bf16 weights (gemv_bf16.cu)
@@ -550,9 +571,10 @@ int decode_step_bf16(cudaStream_t st, int B, const tha_config_t* cfg, const tha_
     return run_step(st, ws, &a, sizeof(a), [&]() { return issue_step_bf16_gemv(st, ws, a, lg, rc, rs); });
   }
   THA_TRY(step_bf16_prepare(ws, cfg, B));
+  a.contexts = step_contexts(ws, B);   // part of the graph key
   return run_step(st, ws, &a, sizeof(a), [&]() {
     return step_bf16_issue(st, ws, B, *cfg, *w, *s, token_d, pos_d, lg, next_d, rc, rs, a.pdl != 0);
-  });
+  }, true, a.contexts);
 }
 
 int last_step_launches_get() { return g_last_step_launches; }
@@ -581,6 +603,7 @@ static int forward_host(cudaStream_t st, int B, int vocab, int seq_len, float* s
   if (!ws) return THA_STATUS_EXECUTION_FAILED;
   THA_TRY(ws_ensure_tokpos(ws, B));
   const int cap = ws->tokpos_cap;
+  const HostContexts contexts(pos_host, B);
   memcpy(ws->tokpos_h, token_host, B * sizeof(int));
   memcpy(ws->tokpos_h + cap, pos_host, B * sizeof(int));
   THA_CUDA_OK(cudaMemcpyAsync(ws->tok_d, ws->tokpos_h, 2 * cap * sizeof(int), cudaMemcpyHostToDevice, st));
@@ -636,6 +659,7 @@ static int forward_host_greedy(cudaStream_t st, int B, const tha_config_t* cfg, 
   if (!ws) return THA_STATUS_EXECUTION_FAILED;
   THA_TRY(ws_ensure_tokpos(ws, B));
   const int cap = ws->tokpos_cap;
+  const HostContexts contexts(pos_host, B);
   memcpy(ws->tokpos_h, token_host, B * sizeof(int));
   memcpy(ws->tokpos_h + cap, pos_host, B * sizeof(int));
   THA_CUDA_OK(cudaMemcpyAsync(ws->tok_d, ws->tokpos_h, 2 * cap * sizeof(int), cudaMemcpyHostToDevice, st));
@@ -667,6 +691,7 @@ static int forward_host_sample(cudaStream_t st, int B, const tha_config_t* cfg, 
   if (!ws) return THA_STATUS_EXECUTION_FAILED;
   THA_TRY(ws_ensure_tokpos(ws, B));
   const int cap = ws->tokpos_cap;
+  const HostContexts contexts(pos_host, B);
   int* h = ws->tokpos_h;
   memcpy(h, token_host, B * sizeof(int));
   memcpy(h + cap, pos_host, B * sizeof(int));
@@ -834,6 +859,7 @@ extern "C" int tha_prefill_q8(void* stream, const tha_config_t* cfg, const tha_w
 extern "C" int tha_prefill_supported(const tha_config_t* cfg) { return (cfg && prefill_tc_supported(cfg)) ? 1 : 0; }
 
 extern "C" int tha_last_step_launches(void) { return last_step_launches_get(); }
+extern "C" int tha_last_step_attention(void) { return g_last_step_attention; }
 
 extern "C" int tha_step_needs_att_scratch(const tha_config_t* cfg) {
   if (!cfg || cfg->n_heads <= 0 || cfg->dim % cfg->n_heads) return 1;

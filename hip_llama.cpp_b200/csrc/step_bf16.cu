@@ -67,14 +67,19 @@ constexpr int BPREP_MAX_V = 4;   // float4 per thread kept in registers: d <= 4 
 // One block per output row: x row = embedding row (bf16 table) or x + sum of nz partials (written back), RMSNorm
 // g * (ss * x) (run.cc:196-209 operation order), rounded to bf16.  With `gather`, output row r comes from source row
 // gather[r] and x is left untouched (classifier input of a prefill chunk).
+template <bool REPORT>
 __global__ void __launch_bounds__(1024) bf_prep_kernel(float* __restrict__ x, const float* __restrict__ part, int nz,
                                                        long long zstride, const uint16_t* __restrict__ emb,
                                                        const int* __restrict__ token, const int* __restrict__ pos,
                                                        const float* __restrict__ gain, int d, uint16_t* __restrict__ xb,
-                                                       const int* __restrict__ gather) {
+                                                       const int* __restrict__ gather, unsigned long long* report) {
   __shared__ float red[33];
   pdl_wait();
   pdl_trigger();
+  if (REPORT && blockIdx.x == gridDim.x - 1) {   // one block more than rows
+    if (threadIdx.x < 32) report_contexts(pos, (int)gridDim.x - 1, report);
+    return;
+  }
   const int ob = blockIdx.x;
   const int b = gather ? gather[ob] : ob;
   const int d4 = d >> 2;
@@ -357,9 +362,12 @@ static int bf_issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, 
   // thread hide the L2 latency that a 1024-thread CTA per row (lowest latency for a handful of decode rows) leaves exposed
   if (R >= 512 && d / 4 <= 256 * BPREP_MAX_V && prep_threads > 256) prep_threads = 256;
   const int* nogather = nullptr;
+  // a decode step's first one tells the host about its contexts, where that is asked for: one block more
+  unsigned long long* const report = io.n_tiles == 0 ? attn_report_to(ws, R, c.n_heads, c.n_kv_heads, hs, c.seq_len) : nullptr;
   auto prep = [&](int rows, int nz, long long zs, const uint16_t* emb, const float* gain, const int* gather) -> int {
-    THA_CUDA_OK(launch(bf_prep_kernel, dim3(rows), dim3(prep_threads), 0, st, pdl, io.x, (const float*)sc.part, nz, zs, emb, io.token,
-                       io.pos, gain, d, sc.xb, gather));
+    const bool tell = emb && report;
+    THA_CUDA_OK(launch(tell ? bf_prep_kernel<true> : bf_prep_kernel<false>, dim3(rows + tell), dim3(prep_threads), 0, st, pdl, io.x, (const float*)sc.part, nz,
+                       zs, emb, io.token, io.pos, gain, d, sc.xb, gather, report));
     return THA_STATUS_SUCCESS;
   };
   auto mm = [&](int n, const uint16_t* const* W, const int* M, const int* off, int K, const uint16_t* X, int N, float* out,

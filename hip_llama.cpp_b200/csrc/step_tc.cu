@@ -107,17 +107,22 @@ __global__ void tp_epoch_kernel(unsigned* epoch) {
 // One block per output row.  x row: embedding row (emb != nullptr) or x + sum of nz partials.  With `gather`
 // output row r is computed from source row gather[r] (the classifier input of a prefill chunk: the last
 // row of every sequence) and x is left untouched.
+template <bool REPORT>
 __global__ void __launch_bounds__(1024) tc_prep_kernel(float* __restrict__ x, const float* __restrict__ part, int nz,
                                                       long long zstride, const float* __restrict__ emb,
                                                       const int* __restrict__ token, const int* __restrict__ pos,
                                                       const float* __restrict__ gain, int d, float* __restrict__ xh,
                                                       float* __restrict__ xl, float* __restrict__ scale,
-                                                      const int* __restrict__ gather, const TpPeers tp) {
+                                                      const int* __restrict__ gather, const TpPeers tp, unsigned long long* report) {
   __shared__ float red[33];
   const int kt = threadIdx.x == 0 ? kt_begin(KT_PREP) : -1;
   pdl_trigger();   // the next kernel may start its launch (it waits for this grid to complete before touching memory)
   pdl_wait();
   kt_stamp(kt, 1);
+  if (REPORT && blockIdx.x == gridDim.x - 1) {   // one block more than rows
+    if (threadIdx.x < 32) report_contexts(pos, (int)gridDim.x - 1, report);
+    return;
+  }
   if (tp.n && !emb) tp_wait_peers(tp);
   const int ob = blockIdx.x;
   const int b = gather ? gather[ob] : ob;
@@ -412,17 +417,22 @@ __device__ __forceinline__ float prep_row_sum(const float (&ss)[PREP_MAX_V], int
   return red[32];
 }
 
+template <bool REPORT>
 __global__ void __launch_bounds__(1024) tc_prep_q8_kernel(float* __restrict__ x, const float* __restrict__ part, int nz,
                                                           long long zstride, const float* __restrict__ emb,
                                                           const int* __restrict__ token, const int* __restrict__ pos,
                                                           const float* __restrict__ gain, int d, int gs,
                                                           int8_t* __restrict__ xq, float* __restrict__ xsT, int ldxs,
-                                                          const int* __restrict__ gather, const TpPeers tp) {
+                                                          const int* __restrict__ gather, const TpPeers tp, unsigned long long* report) {
   __shared__ float red[33];
   const int kt = threadIdx.x == 0 ? kt_begin(KT_PREP) : -1;
   pdl_trigger();   // the next kernel may start its launch (it waits for this grid to complete before touching memory)
   pdl_wait();
   kt_stamp(kt, 1);
+  if (REPORT && blockIdx.x == gridDim.x - 1) {   // one block more than rows
+    if (threadIdx.x < 32) report_contexts(pos, (int)gridDim.x - 1, report);
+    return;
+  }
   if (tp.n && !emb) tp_wait_peers(tp);
   const int ob = blockIdx.x;
   const int b = gather ? gather[ob] : ob;
@@ -888,8 +898,8 @@ static int issue_rows_chain(cudaStream_t st, Workspace* ws, const tha_config_t& 
   const TpPeers none = {};
   const int* nogather = nullptr;
   // embedding gather + RMSNorm(att, layer 0) folded + split (src/thaDNN.cpp:31-36, run.cc:196-209)
-  THA_CUDA_OK(launch(tc_prep_kernel, dim3(R), dim3(prep_threads), 0, st, pdl, io.x, (const float*)nullptr, 0, 0LL,
-                     w.token_embedding_table, io.token, io.pos, w.rms_att_weight, d, sc.xh, sc.xl, sc.scale, nogather, none));
+  THA_CUDA_OK(launch(tc_prep_kernel<false>, dim3(R), dim3(prep_threads), 0, st, pdl, io.x, (const float*)nullptr, 0, 0LL,
+                     w.token_embedding_table, io.token, io.pos, w.rms_att_weight, d, sc.xh, sc.xl, sc.scale, nogather, none, (unsigned long long*)nullptr));
   for (int k = 0; k <= L; k++) {
     ChainArgs a = chain_of_launch(k, c, w, s, sc, io, rc, rs);
     a.part = sc.part; a.part_floats = sc.n_part; a.ss_part = sc.ss; a.ss_floats = sc.n_ss;
@@ -967,17 +977,20 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
   float* out_wo = tpx ? tp->xchg(tp->rank, 0) : sc.part;
   float* out_w2 = tpx ? tp->xchg(tp->rank, 1) : sc.part;
   // the (fused RMSNorm +) split that feeds a matmul whose input is the residual stream
+  // a decode step's first one tells the host about its contexts, where that is asked for: one block more
+  unsigned long long* const report = io.n_tiles == 0 && !tp ? attn_report_to(ws, R, c.n_heads, c.n_kv_heads, hs, c.seq_len) : nullptr;
   auto prep = [&](int rows, const float* part, int nz, long long zs, const float* emb, const float* gain, const int* gather,
                   const TpPeers& tpp) -> int {
     if (skip & 4) return THA_STATUS_SUCCESS;
+    const bool tell = emb && report;
     if (wq) {
-      THA_CUDA_OK(launch(tc_prep_q8_kernel, dim3(rows), dim3(prep_threads), 0, st, pdl, io.x, part, nz, zs, emb, io.token,
-                         io.pos, gain, d, gs, sc.xq, sc.xsT, ldxs, gather, tpp));
+      THA_CUDA_OK(launch(tell ? tc_prep_q8_kernel<true> : tc_prep_q8_kernel<false>, dim3(rows + tell), dim3(prep_threads), 0, st, pdl, io.x, part, nz, zs,
+                         emb, io.token, io.pos, gain, d, gs, sc.xq, sc.xsT, ldxs, gather, tpp, report));
     } else if (prompt_form(rows, d) && !gather && !tpp.n) {
       THA_CUDA_OK(launch(tc_prep_prompt_kernel, dim3(rows), dim3(prompt_threads), 0, st, pdl, io.x, part, nz, zs, emb, io.token, io.pos, gain, d, sc.xh, sc.xl, sc.scale));
     } else {
-      THA_CUDA_OK(launch(tc_prep_kernel, dim3(rows), dim3(prep_threads), 0, st, pdl, io.x, part, nz, zs, emb, io.token,
-                         io.pos, gain, d, sc.xh, sc.xl, sc.scale, gather, tpp));
+      THA_CUDA_OK(launch(tell ? tc_prep_kernel<true> : tc_prep_kernel<false>, dim3(rows + tell), dim3(prep_threads), 0, st, pdl, io.x, part, nz, zs, emb,
+                         io.token, io.pos, gain, d, sc.xh, sc.xl, sc.scale, gather, tpp, report));
     }
     return THA_STATUS_SUCCESS;
   };

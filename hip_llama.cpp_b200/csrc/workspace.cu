@@ -147,6 +147,12 @@ Workspace* workspace() {
   if (it != g_ws.end()) return it->second;
   Workspace* ws = new Workspace();
   ws->device = dev;
+  if (cudaMallocHost((void**)&ws->contexts_h, (CTX_MAX_SLOTS + 1) * sizeof(unsigned long long)) == cudaSuccess)
+    memset(ws->contexts_h, 0, (CTX_MAX_SLOTS + 1) * sizeof(unsigned long long));
+  else {
+    cudaGetLastError();
+    ws->contexts_h = nullptr;   // no reports
+  }
   g_ws[dev] = ws;
   return ws;
 }
@@ -160,6 +166,12 @@ void ws_release(Workspace* ws) {
   if (ws->q8_xq) { cudaFree(ws->q8_xq); cudaFree(ws->q8_xs); ws->q8_xq = nullptr; ws->q8_cap = 0; }
   for (auto& r : ws->rope) { cudaFree(r.second.cos_d); cudaFree(r.second.sin_d); }
   ws->rope.clear();
+}
+
+int ws_reported_contexts(Workspace* ws, int slots) {
+  if (!ws->contexts_h || slots > CTX_MAX_SLOTS) return 0;
+  const unsigned long long v = *static_cast<volatile unsigned long long*>(ws->contexts_h + slots);
+  return CTX_REPORT | context_class((int)(v >> 32), (long long)(v & 0xffffffffu) * slots, slots);
 }
 
 int ws_ensure_dual(Workspace* ws) {

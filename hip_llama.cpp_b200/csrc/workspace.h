@@ -18,10 +18,17 @@ struct RopeTable { float* cos_d = nullptr; float* sin_d = nullptr; };
 
 struct StepGraph {
   cudaGraphExec_t exec = nullptr;
-  int launches = 0;
+  int launches = 0, attn_form = 0;
   std::vector<unsigned char> key;        // the argument bytes the graph was captured for (the map key is only their hash)
   unsigned long long last_use = 0;       // for eviction: ws->graph_clock at the last replay
 };
+// What a step's contexts are like, as far as the choice of its attention kernel asks (attention.cu): some of CTX_*.  CTX_REPORT: they are not
+// known to the host; the step tells what it finds, for the next one of as many slots.
+enum { CTX_LONG = 1, CTX_FILLED = 2, CTX_RAGGED = 4, CTX_SPREAD = 8, CTX_SKEWED = 16, CTX_REPORT = 32 };
+constexpr int CTX_MAX_SLOTS = 256;
+int context_class(int longest, long long sum, int slots);
+enum { ATTN_FUSED = 1, ATTN_DEEP = 2, ATTN_STREAM = 3 };   // which decode attention kernel a step launched
+
 constexpr size_t WS_MAX_GRAPHS = 64;     // cached executable graphs per workspace; the least recently used one goes first
 
 struct Workspace {
@@ -48,6 +55,11 @@ struct Workspace {
   // when the stream differs from the previous step's, makes the new stream wait for that event first -- two streams never have
   // steps in flight over the same scratch.  (last_stream is only compared, never dereferenced: it may have been destroyed.)
   std::mutex mu;
+  int step_contexts = 0;                  // CTX_* of the step being issued (under mu)
+  int attn_form = 0;                      // ATTN_* of the step being issued
+  // pinned, by number of slots: longest << 32 | mean of the contexts that the last reporting step found; 0: none yet.  A hint: every form of
+  // the attention gives the same bits, so a stale or foreign value costs time at most.
+  unsigned long long* contexts_h = nullptr;
   cudaStream_t last_stream = nullptr;
   cudaEvent_t step_done = nullptr;
   // two half-batches of a step as two concurrent branches of the graph (forward.cu, "dual"): the second branch's
@@ -66,6 +78,8 @@ KvPaged kv_paged_of(const KvPool& pool, int n_layers, int kv_dim, int layer);
 Workspace* workspace();   // for the current device (thread-safe)
 int ws_ensure_attn(Workspace* ws, size_t part_slots, int n_counters);
 int ws_ensure_tokpos(Workspace* ws, int n_batches);
+unsigned long long* attn_report_to(Workspace* ws, int B, int n_heads, int n_kv_heads, int head_size, int seq_len);   // attention.cu
+int ws_reported_contexts(Workspace* ws, int slots);   // CTX_* for a step whose positions are on the device
 int ws_ensure_q8(Workspace* ws, int n_batches, int kmax, int gs);
 int ws_ensure_dual(Workspace* ws);
 // cached graphs captured pointers that are about to change

@@ -390,3 +390,6 @@ class Engine:
 
     def last_step_launches(self) -> int:
         return self.lib.c.tha_last_step_launches()
+
+    def last_step_attention(self) -> int:
+        return self.lib.c.tha_last_step_attention()

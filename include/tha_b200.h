@@ -354,6 +354,9 @@ int tha_trace_dump(int skip);   /* development aid: THA_TRACE=1 + graphs off -> 
 int tha_step_needs_att_scratch(const tha_config_t* cfg);
 /* number of kernels the last tha_decode_step_* call on this thread launched */
 int tha_last_step_launches(void);
+/* and its decode attention kernel: 0 another path's, 1 a block per (slot, segment), 2 the same with twice the loads in flight, 3 persistent blocks;
+ * all give the same bits */
+int tha_last_step_attention(void);
 
 #ifdef __cplusplus
 }
