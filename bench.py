@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """Headline benchmark: batched greedy decode tok/s of the stories110M architecture (fp32) on
-N B200s, sequences sharded over GPUs (replicated weights, no collective)
-configs[1] -- with the HBM roofline of the decode step and the reference's CPU path beside it.
+N B200s, sequences sharded over GPUs (replicated weights, no collective) -- the reference's headline
+workload -- with the HBM roofline of the decode step and the reference's CPU path beside it.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--batch B] [--model s110m|7b] [--quant f32|q8]
     python bench.py --impl reference ...     # the reference's own CPU code (oracle/_ref) on the host cores
@@ -14,7 +14,7 @@ thaDNN_s_forward_batch in the reference, src/thaDNN.cpp:13-81).
   e2e        tokens/s through the reference-facing call (tha_forward_batch_*: HOST token[] /
              pos[] in, [B, vocab] logits into pinned HOST memory, host argmax), copies inside
              the timed region.
-  roofline   algorithmic bytes of a decode step (SURVEY.md 8d: weights once + KV rows read +
+  roofline   algorithmic bytes of a decode step (weights once + KV rows read +
              KV rows written + embedding rows + logits) / measured step time, against the
              measured HBM copy bandwidth in MEASURED_PEAKS.json.
   cpu_baseline  oracle/_ref (the reference's run.cc / runq.c compiled unmodified) on the
@@ -66,7 +66,7 @@ def parse_args():
                     "decode step (slower: an event after every launch) and skip the llama2 arm")
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-e2e", action="store_true")
-    ap.add_argument("--no-extra", action="store_true", help="skip the bounded sub-records of the other BASELINE configs (extra.*)")
+    ap.add_argument("--no-extra", action="store_true", help="skip the bounded sub-records of the other configurations (extra.*)")
     ap.add_argument("--no-shares", action="store_true", help="skip the live-share measurement (roofline.live_shares_us)")
     ap.add_argument("--cpu-seconds", type=float, default=12.0, help="budget of the cpu_baseline sample")
     return ap.parse_args()
@@ -104,7 +104,7 @@ def measured_traffic(args):
 
 
 def step_bytes(cfg, weight_bytes, pos, B, elem_bytes_emb=4, write_logits=True):
-    """ALGORITHMIC bytes of one decode step with every slot at position `pos` (SURVEY.md 8d)."""
+    """ALGORITHMIC bytes of one decode step with every slot at position `pos`."""
     kv = 2 * cfg.n_layers * cfg.kv_dim * 4
     b = weight_bytes + B * (kv * (pos + 1) + kv) + B * cfg.dim * elem_bytes_emb
     if write_logits:
@@ -489,7 +489,7 @@ def resident_tok_s(e, cfg, B, W, K, device, pos0=0, seed=1):
 
 
 def extra_records(args, device, peak):
-    """Bounded sub-records of the BASELINE configurations the headline line does not cover (configs[2], [3], [4]); a few
+    """Bounded sub-records of the configurations the headline line does not cover; a few
     seconds each, rank 0 of a data-parallel run, random-init weights generated on the device."""
     import dataclasses
     import gc
@@ -512,7 +512,7 @@ def extra_records(args, device, peak):
         free()
         return rec
 
-    try:   # configs[2]: stories110M Q8_0
+    try:   # stories110M Q8_0
         cfg = ck.STORIES110M
         dw = eng.device_random_weights(cfg, q8=True, seed=1337, device=device)
         out["s110m_q8_B256"] = decode_record(cfg, dw, 256, 5, 20, "stories110M Q8_0 batched greedy decode, 256 slots, positions 5..24")
@@ -521,7 +521,7 @@ def extra_records(args, device, peak):
         free()
     except Exception as ex:
         out["s110m_q8"] = {"error": str(ex)}
-    try:   # configs[4]: Llama-2-7B Q8_0 at 1 / 8 / 64 slots
+    try:   # Llama-2-7B Q8_0 at 1 / 8 / 64 slots
         cfg = ck.LLAMA2_7B
         dw = eng.device_random_weights(cfg, q8=True, seed=1337, device=device)
         for B in (1, 8, 64):
@@ -547,7 +547,7 @@ def extra_records(args, device, peak):
         free()
     except Exception as ex:
         out["7b_q8"] = {"error": str(ex)}
-    try:   # configs[3]: Llama-2-7B fp32, prompt of 2048 positions in one pass + first decode steps
+    try:   # Llama-2-7B fp32, prompt of 2048 positions in one pass + first decode steps
         cfg = dataclasses.replace(ck.LLAMA2_7B, seq_len=2304)   # room for decode positions behind the 2048-position prompt
         dw = eng.device_random_weights(cfg, q8=False, seed=1337, device=device)
         e = eng.Engine(dw, 1, device=device, with_att=False)
@@ -594,7 +594,7 @@ def extra_records(args, device, peak):
         free()
     except Exception as ex:
         out["prefill_7b_f32_2048"] = {"error": str(ex)}
-    try:   # configs[3], bf16: prompt of 2048 positions (tensor-core matmuls AND attention), decode at 1 and 64 slots
+    try:   # Llama-2-7B bf16: prompt of 2048 positions (tensor-core matmuls AND attention), decode at 1 and 64 slots
         cfg = dataclasses.replace(ck.LLAMA2_7B, seq_len=2304)
         dw = eng.DeviceWeightsBF16.random(cfg, seed=1337, device=device)
         e = eng.Engine(dw, 1, device=device, with_att=False)
@@ -695,7 +695,7 @@ def cpu_reference(args, cfg, host_w, n_seqs, n_threads, max_steps, warmup, budge
     kindname = "q8" if q8 else "fp32"
     fast = cpu_has_avx2_fma() and ref_available(kindname, fast=True)
     if not ref_available(kindname, fast=fast):
-        raise RuntimeError("oracle/_ref is not built (run __graft_entry__.build() where /root/reference exists)")
+        raise RuntimeError("oracle/_ref is not built (run __graft_entry__.build() where the reference's sources are)")
     if host_w is None:
         host_w = ck.random_weights(cfg, seed=1337, std=0.02)
     with tempfile.TemporaryDirectory() as td:
@@ -807,7 +807,7 @@ def main():
     r = run_ours(args, rank, world, local_rank)
     tp_rec = None
     if world > 1 and args.tp == 1 and not args.no_extra and args.model == "s110m" and args.quant == "f32":
-        # the optional tensor-parallel split (north_star: Llama-2-7B 2/4/8-way), one replica over all ranks of this run
+        # the optional tensor-parallel split (Llama-2-7B 2/4/8-way), one replica over all ranks of this run
         try:
             tp_rec = tp_extra(args, rank, world, local_rank)
         except Exception as ex:

@@ -1,9 +1,9 @@
 """llama2.c checkpoint files: the two on-disk formats the reference reads.
 
-* legacy v0 (fp32): reader `/root/reference/src/utils.cpp:119-170` (== run.cc:110-161),
-  writer `/root/reference/train/export.py:75-127`.
-* version 2 (Q8_0): reader `/root/reference/runq.c:174-251`, writer
-  `/root/reference/train/export.py:182-260`, group quantiser `export.py:45-70`.
+* legacy v0 (fp32): reader `src/utils.cpp:119-170` (== run.cc:110-161),
+  writer `train/export.py:75-127`.
+* version 2 (Q8_0): reader `runq.c:174-251`, writer
+  `train/export.py:182-260`, group quantiser `export.py:45-70`.
 
 The reference's exporter expands every tensor through `struct.pack(*d)`
 (`export.py:34-38`), which is unusable at 7B scale; this module writes the
@@ -11,7 +11,7 @@ identical byte layout with numpy.  `tests/test_checkpoint.py` checks byte
 identity against files produced by the reference exporter (fixtures made by
 `tests/golden/make_golden.py`).
 
-Random-init follows `/root/reference/train/model.py:232-247`: N(0, 0.02) for
+Random-init follows `train/model.py:232-247`: N(0, 0.02) for
 embeddings and linear layers, N(0, 0.02/sqrt(2*n_layers)) for wo and w3, ones
 for the norms, classifier tied to the embedding.
 """

@@ -901,7 +901,7 @@ extern "C" int tha_mha_fused_v1_f32(void* stream, int n_batches, const int* pos_
 
 // ------------------------------------------------------------------ no-allocation variant -------
 // tha_mha_fused_v1_f32_static: the fused attention above for callers that may not allocate (CUDA graph capture, serving
-// loops, harnesses that forbid cudaMalloc).  No counterpart in the reference; added at the request of the run's operators.
+// loops, harnesses that forbid cudaMalloc).  No counterpart in the reference.
 // The split scratch (per-split accumulators, maxima / sums, arrival counters) lives in ONE file-scope device array of a fixed
 // size instead of the Workspace's growable buffers.  Every GPU that loads the library holds the array until exit; every
 // call on a device shares it, so two calls that overlap on that GPU (different streams) race -- serialise them.

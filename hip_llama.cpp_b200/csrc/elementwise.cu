@@ -1,7 +1,7 @@
 // Standalone element-wise / reduction ops of the thaBLAS + thaDNN surface.
 // In the fused decode step these are folded into the GEMV kernels (gemv.cu); the
 // stand-alone forms exist because every reference entry point must exist
-//  and they are what the per-op parity tests call.
+// and they are what the per-op parity tests call.
 #include "common.cuh"
 
 namespace tha {

@@ -59,7 +59,7 @@ int step_tc_q8_issue(cudaStream_t st, Workspace* ws, int B, const tha_config_t& 
 TpCtx* tp_ctx(tha_tp_t* t);
 int gemm_tc_check_error();
 int tc_mode();   // -1 auto (more than TC_MIN_SLOTS slots), 0 never, 1 whenever the shape allows
-// From five slots on the tensor-core row pipeline wins over both small-batch paths (measured after the round-2 read-out fixes):
+// From five slots on the tensor-core row pipeline wins over both small-batch paths (measured):
 // stories110M fp32 at 5 / 8 slots 0.476 / 0.485 ms per step against the persistent step kernel's 0.537 / 0.559; Llama-2-7B fp32 at
 // 8 slots 6.83 ms against the fused GEMV step's 10.71 (0.60 vs 0.38 of HBM); at 4 slots the two are level, below the GEMV / mega paths win.
 constexpr int TC_MIN_SLOTS = 4;
@@ -816,7 +816,7 @@ extern "C" int tha_forward_greedy_q8(void* stream, int n_batches, const tha_conf
                              });
 }
 
-// Batched prompt ingestion (SURVEY.md 8(f) rank 2): what the reference does one forced-prompt step at a time
+// Batched prompt ingestion: what the reference does one forced-prompt step at a time
 // (src/llama.cpp:1029-1030) in one pass of tensor-core matmuls over all prompt positions.
 extern "C" int tha_prefill_f32(void* stream, const tha_config_t* cfg, const tha_weights_f32_t* w, const tha_state_t* s,
                                int n_seqs, const int* slot_host, const int* pos0_host, const int* len_host,
@@ -885,7 +885,7 @@ extern "C" int tha_forward_batch_q8(void* stream, int n_batches, const tha_confi
 }
 
 // ---------------------------------------------------------------------------- tensor parallel ----
-// One rank's share of the decode step / prompt ingestion of a model split tp ways (tp.h; SURVEY.md 8e).  cfg is the
+// One rank's share of the decode step / prompt ingestion of a model split tp ways (tp.h).  cfg is the
 // LOCAL config (n_heads, n_kv_heads, hidden_dim = this rank's share; dim = full width), w / s hold the local shards:
 // wq [L, da, dim], wk/wv [L, kvd, dim], wo [L, dim, da], w1/w3 [L, hd, dim], w2 [L, dim, hd]; embedding, norms and
 // classifier replicated; KV cache [B][L][S][kvd] of the local heads.  Every rank must make the same sequence of calls.

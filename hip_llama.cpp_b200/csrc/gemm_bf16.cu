@@ -5,7 +5,7 @@
 //   out[n, row] = sum_k W[row, k] * X[n, k]      W: [M, K] row-major bf16, X: [N, K] row-major bf16 (rows = slots or
 //                                                prompt positions, already rounded to bf16 by the producing kernel)
 //
-// This is the matmul of the bf16 model path (BASELINE.json configs[3] "fp32/bf16"; the reference declares the 16-bit
+// This is the matmul of the bf16 model path (the reference declares the 16-bit
 // weight structs at include/models.hpp:77-117 and never fills them) for more than 8 rows and for prompt ingestion, where
 // the fp32 path's 3xTF32 scheme spends three tensor-core passes and a converter stage per useful one.
 //

@@ -1,4 +1,4 @@
-// The bf16 model path (BASELINE.json configs[3] "fp32/bf16"; the reference declares 16-bit weight structs at
+// The bf16 model path (the reference declares 16-bit weight structs at
 // include/models.hpp:77-117 and never uses them): weights stored as bf16, the residual stream, RMSNorm, RoPE, attention,
 // SwiGLU and the KV cache in fp32 exactly as run.cc:244-374, and every vector that ENTERS a weight matmul rounded to bf16
 // (round to nearest even) -- which is what the tensor cores consume.  The oracle restates the same rule on the CPU

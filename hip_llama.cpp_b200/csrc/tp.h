@@ -1,5 +1,5 @@
 // Tensor-parallel context of the row pipeline (step_tc.cu): Llama-2-7B split 2/4/8 ways over the GPUs of one NVLink /
-// NVSwitch box (SURVEY.md 8e "Optional TP").  wq/wk/wv/w1/w3 are split by output rows (heads, hidden units), wo/w2 by
+// NVSwitch box.  wq/wk/wv/w1/w3 are split by output rows (heads, hidden units), wo/w2 by
 // input columns; each rank's wo / w2 matmul therefore yields PARTIAL sums of the residual update.  Those partials are
 // never all-reduced by a separate collective: every rank's matmul writes its split-K partials into an exchange buffer
 // in its own HBM that its peers have mapped (cudaIpc / peer access), and the kernel that consumes them anyway

@@ -111,7 +111,7 @@ int skip_mode();       // bit mask of kernel classes left out of the row pipelin
                        // 4 prep, 8 RoPE / scatter, 16 SwiGLU / quantise, 32 classifier, 64 argmax
 int sample_resident_mode();   // 1: the device sampler keeps a slot's row in shared memory
 int rope_fuse_mode();  // 1: a decode step's RoPE + KV scatter run inside the attention kernel
-int chain_mode();      // 1: matmul chains with fused epilogues (chain_tc.cu), 0: one launch per matmul (the round-1 pipeline)
+int chain_mode();      // 1: matmul chains with fused epilogues (chain_tc.cu), 0: one launch per matmul
 int sm_budget();            // SMs one matmul launch may occupy: all of them, or a branch's share while a dual step is planned / issued
 void set_sm_budget(int n);  // 0 = all
 int dual_min_rows();   // rows from which a step is issued as two concurrent half-batches (0 = never)

@@ -160,7 +160,7 @@ void free_weight_on_device_q8(TransformerWeightsQ8* w, int shared_classifier) {
   free(w);
 }
 
-// ---- tensor-parallel shards (DESIGN.md section 5; the slicing hip_llama.cpp_b200/tp.py does with numpy) ------------------
+// ---- tensor-parallel shards (the slicing hip_llama.cpp_b200/tp.py does with numpy) ------------------
 // Local hidden_dim of every rank: whole groups of `unit` values, the first (groups % tp) ranks get one more.
 int tp_split_hidden(int hidden, int tp, int unit, int* out) {
   if (tp < 1 || unit < 1 || hidden % unit) return -1;

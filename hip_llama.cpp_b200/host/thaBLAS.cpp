@@ -81,7 +81,7 @@ thablasStatus_t thaBLAS_s_matmul_reduction(thablasHandle_t* handle, float* A, fl
   if (!handle) return THABLAS_STATUS_HANDLE_IS_NULLPTR;
   return st(tha_matmul_reduction_f32(calc(handle), A, B, C, M, N, K));
 }
-// The reference's MFMA kernel stores D inside its K loop and hard-wires N = 16 (SURVEY.md 0);
+// The reference's MFMA kernel stores D inside its K loop and hard-wires N = 16;
 // the contract its caller relies on is that of thaBLAS_s_matmul_reduction, which this keeps.
 thablasStatus_t thaBLAS_s_sgemm_Mx16xK(thablasHandle_t* handle, float* d_A, float* d_B, float* d_D, int M, int N, int K) {
   return thaBLAS_s_matmul_reduction(handle, d_A, d_B, d_D, M, N, K);

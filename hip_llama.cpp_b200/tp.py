@@ -1,5 +1,4 @@
-"""Tensor-parallel split of a llama2 model over the GPUs of one box (SURVEY.md 8e "Optional TP"; north_star:
-Llama-2-7B 2/4/8-way over NVLink), over the C-ABI's tha_tp_* entry points (include/tha_b200.h).
+"""Tensor-parallel split of a llama2 model over the GPUs of one box (Llama-2-7B 2/4/8-way over NVLink), over the C-ABI's tha_tp_* entry points (include/tha_b200.h).
 
 Megatron-style shards of the reference's weight tensors (layout of include/models.hpp:25-36):
   wq/wk/wv, w1/w3   split by OUTPUT rows  (heads H/tp, kv heads KV/tp, hidden units)

@@ -2,7 +2,7 @@
 //
 // The reference's class of this name (include/BatchManager.hpp:11-52, src/BatchManager.cpp) is
 // a stub that live code never instantiates (uninitialised members, a function without a
-// return, by-value mutation; SURVEY.md 0).  The names and members below are kept; the
+// return, by-value mutation).  The names and members below are kept; the
 // behaviour is the working version of what it gestures at:
 //   * the KV cache of a GPU is one slab [batch_size][n_layers][seq_len][kv_dim] x {K, V} (the
 //     layout thaDNN_s_forward_batch reads), cut into BLOCKS of `block_size` positions;

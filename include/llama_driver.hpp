@@ -95,7 +95,7 @@ int test_data_parallelism(Transformer* transformer, Tokenizer* tokenizer, const 
                           int batch_size);
 int run_data_parallel(Transformer* t32, TransformerQ8* tq8, const char* tokenizer_path, Requests* requests,
                       const DriverOptions& opt, DriverStats* stats);
-// One replica, tensor parallel (DESIGN.md section 5): same slot state machine, the step is tha_tp_forward_greedy.
+// One replica, tensor parallel: same slot state machine, the step is tha_tp_forward_greedy.
 int run_tensor_parallel(Transformer* t32, TransformerQ8* tq8, const char* tokenizer_path, Requests* requests,
                         const DriverOptions& opt, DriverStats* stats);
 long time_in_ms();

@@ -53,7 +53,7 @@ thablasStatus_t thaBLAS_s_vecaddvec(thablasHandle_t* handle, float* a, float* b,
 thablasStatus_t thaBLAS_s_matmulvec(thablasHandle_t handle, float* C, float* B, float* A, int K, int M);
 thablasStatus_t thaDNN_s_matmulvec_v2(thablasHandle_t handle, float* C, float* B, float* A, int K, int M);
 // the header of the reference declares the by-value form and its .cpp defines a by-pointer
-// overload (SURVEY.md 2.5); both exist here
+// overload; both exist here
 thablasStatus_t thaDNN_s_matmulvec_v2(thablasHandle_t* handle, float* C, float* B, float* A, int K, int M);
 
 // ---- level 3 ---------------------------------------------------------------------------

@@ -29,7 +29,7 @@ typedef enum {
 // (src/llama.cpp:935-936).  Only handle1 is used, as in the reference (:40).  Returns after
 // the logits have landed (the reference ends with hipDeviceSynchronize, :78).
 // Differences, all on the safe side: a slot with pos[b] < 0 is idle and skipped (the reference
-// computes garbage rows for idle slots, SURVEY.md 2.5); nothing is allocated per call.
+// computes garbage rows for idle slots); nothing is allocated per call.
 thablasStatus_t thaDNN_s_forward_batch(thablasHandle_t handle1, thablasHandle_t handle2, thablasHandle_t handle3,
                                        int n_batches, Config* p, TransformerWeights* w, RunState* s_batch,
                                        int token[], int pos[], float* logits_host);
@@ -38,7 +38,7 @@ thablasStatus_t thaDNN_s_forward_batch(thablasHandle_t handle1, thablasHandle_t 
 thablasStatus_t thaDNN_q8_forward_batch(thablasHandle_t handle, int n_batches, Config* p, TransformerWeightsQ8* w,
                                         RunState* s_batch, int token[], int pos[], float* logits_host);
 
-// Batched prompt ingestion (additive; SURVEY.md 8(f) rank 2).  HOST arrays: sequence i lives in cache slab slot[i];
+// Batched prompt ingestion (additive).  HOST arrays: sequence i lives in cache slab slot[i];
 // its len[i] tokens (concatenated in tokens[]) go to positions pos0[i]..pos0[i]+len[i]-1 in one pass of tensor-core
 // matmuls, leaving the cache as len[i] forced-prompt steps of thaDNN_s_forward_batch would (src/llama.cpp:1029-1030).
 // logits_d / next_d (DEVICE, nullable): last-position logits [n_seqs, vocab] and their argmax.  Asynchronous.
@@ -54,7 +54,7 @@ thablasStatus_t thaDNN_s_decode_greedy_batch(thablasHandle_t* handle, int n_batc
                                              RunState* s_batch, int* token_d, int* pos_d, int* next_d,
                                              float* logits_d, int advance);
 
-// Tensor-parallel step (additive; SURVEY.md 8e "Optional TP"): ONE replica of a model split over the GPUs of a box,
+// Tensor-parallel step (additive): ONE replica of a model split over the GPUs of a box,
 // one rank per GPU (one host thread per device as in src/llama.cpp:913, or one process per device).  p / w / s_batch
 // are the rank's LOCAL config, weight shards and state (include/tha_b200.h, "tensor parallelism"); the all-reduce after
 // the wo and w2 matmuls is fused into the kernel that consumes it, over NVLink peer memory.  Every rank makes the same

@@ -4,6 +4,6 @@
 
 // In-place softmax of one device vector (max-subtract, expf, divide).  size <= 0 or a null
 // pointer -> ALLOC_FAILED after "THABLAS ERROR: INVALID ARGUMENT" (:103-106).  The reference's
-// header takes the handle by pointer and its .cpp by value (SURVEY.md 2.5): both exist.
+// header takes the handle by pointer and its .cpp by value: both exist.
 thablasStatus_t thaDNN_s_softmax_v2(thablasHandle_t* handle, float* x, int size);
 thablasStatus_t thaDNN_s_softmax_v2(thablasHandle_t handle, float* x, int size);

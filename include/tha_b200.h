@@ -8,7 +8,7 @@
  * symbols; a Python / cgo / JNI caller binds the same symbols directly
  * (see INTEGRATION.md).
  *
- * Citations are to the reference tree (/root/reference): each entry point names
+ * Citations are to the reference tree: each entry point names
  * the reference interface it replaces.
  *
  * Return value: a thablasStatus_t value (include/thaBLAS.hpp:5-19 in the
@@ -69,8 +69,8 @@ typedef struct {
   int group_size;
 } tha_weights_q8_t;
 
-/* bf16 weights (the reference declares 16-bit weight structs at include/models.hpp:77-117 and never fills them;
- * BASELINE.json configs[3] "fp32/bf16"): the tensors of tha_weights_f32_t, matrices and embedding table as raw bf16 bit
+/* bf16 weights (the reference declares 16-bit weight structs at include/models.hpp:77-117 and never fills them):
+ * the tensors of tha_weights_f32_t, matrices and embedding table as raw bf16 bit
  * patterns (round-to-nearest-even of the fp32 checkpoint, tha_convert_bf16), norm gains fp32.  Residual stream, KV cache,
  * attention and logits stay fp32; every vector entering a weight matmul is rounded to bf16. */
 typedef struct {
@@ -87,7 +87,7 @@ int tha_set_option(const char* name, int value); /* "pdl", "graph", "mega" (0/1)
                                                     "dual": slots from which a step runs as two concurrent half-batch
                                                     branches (default 256, 0 never); "ropefuse" (RoPE + KV write inside
                                                     the attention kernel), "sample_resident", "chain", "skip": A/B and
-                                                    diagnostic switches, see DESIGN.md section 4 */
+                                                    diagnostic switches */
 
 /* ---- runtime shim: the only way the C++ host layer touches the CUDA runtime ---------
  * (reference: hipSetDevice / hipMalloc / hipMemcpy / hipHostMalloc / hipStreamCreate /
@@ -181,8 +181,8 @@ int tha_mha_weighted_v2_f32(void* stream, int n_batches, const int* pos_d, int n
 int tha_mha_fused_v1_f32(void* stream, int n_batches, const int* pos_d, int n_heads, int n_kv_heads,
                          int n_layers, const float* q, float* xb, const float* key_cache,
                          const float* value_cache, int head_size, int seq_len, int loff);
-/* The same kernel and arguments for callers that may not allocate.  No counterpart in the reference: added at the
- * request of the run's operators, for code under CUDA graph capture, tight serving loops and harnesses that forbid
+/* The same kernel and arguments for callers that may not allocate.  No counterpart in the reference: for
+ * code under CUDA graph capture, tight serving loops and harnesses that forbid
  * cudaMalloc.  The call allocates nothing (no cudaMalloc / cudaFree, no allocating library routine): the split
  * scratch is a file-scope device array of 787,456 bytes (32768 partial slots of 24 bytes + 256 arrival counters)
  * that every GPU loading the library holds until exit.  A launch whose time split needs more
@@ -239,7 +239,7 @@ int tha_forward_greedy_f32(void* stream, int n_batches, const tha_config_t* cfg,
 int tha_forward_greedy_q8(void* stream, int n_batches, const tha_config_t* cfg, const tha_weights_q8_t* w,
                           const tha_state_t* s, const int* token_host, const int* pos_host, int* next_host);
 /* The driver's sampler on the device (replaces sample() / sample_topp() / sample_mult() / random_f32() of
- * src/llama.cpp:262-411 for B slots at once; SURVEY.md 8(f) rank 1).  logits_d [B, vocab] is overwritten with the
+ * src/llama.cpp:262-411 for B slots at once).  logits_d [B, vocab] is overwritten with the
  * probabilities (as the reference's sample() does).  rng_d [B]: xorshift* state of the request in each slot, advanced once
  * per SAMPLED token; reseed_d (nullable) [B]: non-zero = start the slot's stream from this seed first; force_d (nullable)
  * [B]: >= 0 = the next token is this prompt token, no coin is drawn (src/llama.cpp:1029-1030); pos_d [B]: < 0 = idle.
@@ -269,7 +269,7 @@ int tha_forward_sample_bf16(void* stream, int n_batches, const tha_config_t* cfg
 int tha_prefill_bf16(void* stream, const tha_config_t* cfg, const tha_weights_bf16_t* w, const tha_state_t* s, int n_seqs,
                      const int* slot_host, const int* pos0_host, const int* len_host, const int* tokens_host,
                      float* logits_d, int* next_d);
-/* Paged KV cache (SURVEY.md 8(f) rank 3; fills in include/BatchManager.hpp:11-52 of the reference, whose alloc_new_block /
+/* Paged KV cache (fills in include/BatchManager.hpp:11-52 of the reference, whose alloc_new_block /
  * convert_block_ids_to_block_addrs / push_kv_data_to_kv_cache are stubs).  key_pool / value_pool: device arrays
  * [n_blocks][n_layers][block_size][kv_dim] fp32 owned by the caller; block_table_d: device array [slots][table_stride] of
  * block ids, row s listing in order the blocks that hold slot s's positions (block_size, a power of two, positions each).
@@ -287,7 +287,7 @@ int tha_argmax_batch_f32(void* stream, int n_batches, const float* logits, int v
 int tha_advance_slots(void* stream, int n_batches, int* token_d, int* pos_d, const int* next_d, int seq_len);
 /* 1 when the step for this shape falls back to the three attention stages and therefore needs
  * tha_state_t.att ([B, n_heads, seq_len]); 0 when the fused attention kernel covers it */
-/* Batched prompt ingestion ("prefill"; SURVEY.md 8(f) rank 2).  The reference feeds a prompt one forced token per
+/* Batched prompt ingestion ("prefill").  The reference feeds a prompt one forced token per
  * decode step (src/llama.cpp:1029-1030); this runs all prompt positions of n_seqs sequences through the tcgen05
  * matmuls in one pass.  HOST arrays: sequence i lives in cache slab slot_host[i]; its len_host[i] tokens (concatenated
  * in tokens_host, sequence after sequence) go to positions pos0_host[i] .. pos0_host[i]+len_host[i]-1.  Every row's K/V
@@ -303,7 +303,7 @@ int tha_prefill_q8(void* stream, const tha_config_t* cfg, const tha_weights_q8_t
                    float* logits_d, int* next_d);
 int tha_prefill_supported(const tha_config_t* cfg); /* 1 when tha_prefill_f32 handles this architecture */
 
-/* ---- tensor parallelism (Llama-2-7B split 2/4/8 ways over NVLink; SURVEY.md 8e "Optional TP") ------------------
+/* ---- tensor parallelism (Llama-2-7B split 2/4/8 ways over NVLink) ------------------
  * One tha_tp_t per rank (= per GPU; one process per GPU, or one host thread per GPU in one process as the reference's
  * driver runs, src/llama.cpp:913).  wq/wk/wv/w1/w3 are split by output rows (heads, hidden units), wo/w2 by input
  * columns (the reference has no TP; its closest relative is the pipeline split of src/thaDNN.cpp:83-427).  The

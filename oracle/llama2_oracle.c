@@ -4,8 +4,8 @@
  *
  * CPU restatement (plain C, scalar, sequential sums) of the llama2 forward pass
  * that the reference runs on the host:
- *   fp32 : /root/reference/run.cc:196-374  (== src/seq.cpp:3-183)
- *   Q8_0 : /root/reference/runq.c:139-171, 317-481
+ *   fp32 : run.cc:196-374  (== src/seq.cpp:3-183)
+ *   Q8_0 : runq.c:139-171, 317-481
  *   files: run.cc:110-161 (legacy v0), runq.c:174-251 (v2), writer train/export.py
  * Parity pinned: tests/test_oracle_vs_ref.py compares every function here
  * bit-for-bit with oracle/_ref (the reference sources compiled unmodified) and

@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""BASELINE.json configs[0]: stories110M (fp32, seeded random-init of that architecture -- no checkpoint on the box) greedy
+"""stories110M (fp32, seeded random-init of that architecture -- no checkpoint on the box) greedy
 decode of the 128 prompts of assets/in/gen_in_128.txt through the shipped driver (./build/apps/llama -m test -t 0), with the
 app's own throughput line (the reference's definition: sum(pos - 1) / wall, weight upload included, src/llama.cpp:1596-1615)
 and a parity sample: the first positions of a few requests against the oracle's greedy loop.
