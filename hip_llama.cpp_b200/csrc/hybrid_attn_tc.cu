@@ -476,7 +476,8 @@ static int at_form(cudaStream_t s, const tha_attn_t* a, const tha_rows_t* rows, 
 int hyb_attn_tc_launch(cudaStream_t s, const tha_attn_t* a, const tha_rows_t* rows, const tha_kv_t* kv, const float* q, __nv_bfloat16* out, const float* gate,
                        long long ldg, int min_rows, float* scratch, size_t scratch_floats) {
   const size_t need = hyb_attn_tc_scratch(a, rows);
-  if (!need || !scratch || scratch_floats < need || kv->kv_dim % 4 || !aligned16(kv->k_pool) || !aligned16(kv->v_pool) || !aligned16(q)) return THA_STATUS_NOT_SUPPORTED;
+  if (!need || !scratch || scratch_floats < need || kv->kv_dim % 4 || !aligned16(kv->k_pool) || !aligned16(kv->v_pool) || !aligned16(q) || !aligned16(out))
+    return THA_STATUS_NOT_SUPPORTED;   // 128-bit loads and stores
   const int staged = rows->n_seqs * ((rows->max_pos + 32) / 32 * 32);
   const int kw = a->kv_heads * a->dim, vw = a->kv_heads / (a->v_share > 1 ? a->v_share : 1) * a->dim;
   __nv_bfloat16* k16 = reinterpret_cast<__nv_bfloat16*>((reinterpret_cast<uintptr_t>(scratch) + 127) & ~(uintptr_t)127);

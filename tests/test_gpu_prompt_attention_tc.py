@@ -116,6 +116,30 @@ def test_large_common_scores(dim, sink):
         assert rel(out, exact) < 1e-5
 
 
+@pytest.mark.parametrize("out_f32", [0, 1])
+def test_results_on_an_8_byte_boundary(out_f32):
+    """Its stores are of 16 bytes: such a call takes the other kernel, whose are of 4 and 8."""
+    a = H.Attn()
+    a.heads, a.kv_heads, a.dim, a.vdim, a.rot, a.scale, a.out_f32 = 16, 4, 64, 64, -1, 0.125, out_f32
+    R, g = 1100, torch.Generator(device="cuda").manual_seed(1)
+    cache = Cache(1, R, a.kv_heads, a.dim, a.dim)
+    cache.k, cache.v = cache.k.bfloat16().float(), cache.v.bfloat16().float()
+    q = torch.randn(R, a.heads, a.dim, device="cuda", generator=g).bfloat16().float()
+    seqs = [(0, 0, R)]
+    rows, keep = H.rows_of(seqs)
+    lib = H.lib()
+    lib.c.tha_hyb_attn_gated.argtypes = [H.P, H.I, C.POINTER(H.Attn), C.POINTER(H.Rows), C.POINTER(H.Kv), H.P, H.P, H.P, C.c_size_t, H.P, H.L]
+    scratch = torch.empty((R + 32) * a.kv_heads * a.dim + 64, device="cuda")
+    exact, n = want(a, cache, q, seqs, {}), q.numel()
+    buf = torch.full((n + 8,), 7.0, device="cuda", dtype=torch.float32 if out_f32 else torch.bfloat16)
+    for skip in (0, 2 if out_f32 else 4):
+        out = buf[skip:skip + n]
+        torch.cuda.synchronize()
+        lib.check(lib.c.tha_hyb_attn_gated(None, H.BF16, a, rows, cache.struct(), H.ptr(q), H.ptr(out), H.ptr(scratch), scratch.numel(), None, 0))
+        torch.cuda.synchronize()
+        assert rel(out.view(R, a.heads, a.dim).float(), exact) < (3e-3 if out_f32 else 4e-3)
+
+
 @pytest.mark.parametrize("lengths", [[64], [100, 128, 64]])
 def test_the_output_product_behind_it(tmp_path, lengths):
     """Whole steps with heads of 64: a block of the attention and one of the product behind it, both of which allocate TMEM, fit an SM side by side."""
