@@ -445,6 +445,7 @@ size_t hyb_attn_tc_scratch(const tha_attn_t* a, const tha_rows_t* rows) {
   const int AP = 2 * AT_ROWS / gsize;
   if ((long long)(rows->n_rows / AP) * a->kv_heads < (AP <= 85 ? 16 : 3 * AP / 16)) return 0;
   if (at_smem(a->dim, gsize, AP, a->rel ? a->rel_n : 0) > TC_SMEM_LIMIT - 1024) return 0;
+  if (rows->n_rows / AP + rows->n_seqs > 65535) return 0;   // position tiles are the grid's second dimension
   const long long staged = (long long)rows->n_seqs * ((rows->max_pos + 32) / 32 * 32);
   if (staged > 4ll * rows->n_rows + 4096) return 0;
   return (size_t)staged * a->kv_heads * a->dim + 64;

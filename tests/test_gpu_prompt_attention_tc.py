@@ -116,6 +116,27 @@ def test_large_common_scores(dim, sink):
         assert rel(out, exact) < 1e-5
 
 
+def test_more_position_tiles_than_a_grid_holds():
+    """256 query heads to a key head: a tile of one position; 66000 of them take the other kernel."""
+    a = H.Attn()
+    a.heads, a.kv_heads, a.dim, a.vdim, a.rot, a.scale, a.window = 256, 1, 64, 64, -1, 0.125, 40
+    R, g = 66000, torch.Generator(device="cuda").manual_seed(1)
+    cache = Cache(1, R, 1, 64, 64)
+    cache.k, cache.v = cache.k.bfloat16().float(), cache.v.bfloat16().float()
+    q = torch.randn(R, 256, 64, device="cuda", generator=g)
+    rows, keep = H.rows_of([(0, 0, R)])
+    lib = H.lib()
+    lib.c.tha_hyb_attn_gated.argtypes = [H.P, H.I, C.POINTER(H.Attn), C.POINTER(H.Rows), C.POINTER(H.Kv), H.P, H.P, H.P, C.c_size_t, H.P, H.L]
+    out, scratch = torch.empty(R, 256, 64, device="cuda", dtype=torch.bfloat16), torch.empty((R + 32) * 64 + 64, device="cuda")
+    torch.cuda.synchronize()
+    lib.check(lib.c.tha_hyb_attn_gated(None, H.BF16, a, rows, cache.struct(), H.ptr(q), H.ptr(out), H.ptr(scratch), scratch.numel(), None, 0))
+    torch.cuda.synchronize()
+    for p in (0, 39, 31000, R - 1):
+        K, V = (c[0, max(0, p - 39):p + 1, 0].double() for c in (cache.k, cache.v))
+        exact = torch.softmax(q[p].bfloat16().double() @ K.T * a.scale, -1) @ V
+        assert rel(out[p].float(), exact) < 6e-3       # weights and results rounded to bf16: 2^-9 each
+
+
 @pytest.mark.parametrize("out_f32", [0, 1])
 def test_results_on_an_8_byte_boundary(out_f32):
     """Its stores are of 16 bytes: such a call takes the other kernel, whose are of 4 and 8."""
