@@ -695,26 +695,27 @@ int attn_fused_nsplit(int B, int nseg, int seq_len) {
 // evens out ragged ones, but its 210 KB an SM keep the next product's blocks, and the weights that they ask for ahead, off the SM until it is done, and a
 // last round of few pairs over its 24 warps an SM costs a whole one.  Measured on 1451 steps (two layers of Llama-2-7B, stories110M, stories42M;
 // fp32, Q8_0, bf16; 5 .. 200 slots at uniform and ragged contexts of 5 .. 2000), time of the fused one over the persistent one's: 0.85 .. 2.05, 1.039 on
-// average; this rule takes the persistent one where that is 0.98 .. 2.05 and gains 1.055 on average, of 1.064 if each step took the better.  The classes:
-//   Q8_0, and bf16 at narrow rows, in groups of less than eight warps (the products' rings leave the fused kernel's loads little L1): 0.98 .. 2.05 from 200
-//     positions on average on
-//   else where the pairs fill less than two thirds of their rounds: 0.86 .. 1.06 at uniform contexts, 0.91 .. 1.14 with some spread, 1.00 .. 1.36 with the
-//     longest half the mean above it, and 200 positions
-//   Q8_0 at narrow rows, and fp32 at wide ones where the alternative is the deep form: 0.97 .. 1.05 below 100 positions, 1.00 .. 1.47 above
+// average; this rule takes the persistent one where that is 0.98 .. 2.05 and gains 1.057 on average, of 1.064 if each step took the better.  The classes:
+//   Q8_0, and bf16 at narrow rows, in groups of less than eight warps (the products' rings leave the fused kernel's loads little L1): 0.99 .. 2.05 from a
+//     longest context of 60 on; 0.98 .. 1.41 from 200 on average on where the pairs fill less than two thirds of their rounds
+//   else with such rounds: 0.86 .. 1.06 at uniform contexts, 0.91 .. 1.14 with some spread, 1.00 .. 1.36 with the longest half the mean above it, and 200
+//   Q8_0 at narrow rows, and fp32 at wide ones where the alternative is the deep form: 0.97 .. 1.04 below a longest of 60, 0.98 .. 1.47 above
 //   else against the deep form: 0.85 .. 1.09 with less than 450 positions between mean and longest, 0.99 .. 1.12 with more
 //   otherwise: 0.93 .. 1.17 below, 0.99 .. 1.55 above a mean of 1500, to which each position between mean and longest adds twelve
-// A step whose positions are on the device goes by what the last one of as many slots reported (1 us a step), and the first by the fused kernel.
+// A step whose positions are on the device goes by what the last one of as many slots reported (1 us a step), the first by ragged contexts that end at half
+// the cache.
 int context_class(int longest, long long sum, int slots) {
   const long long mean = slots > 0 ? sum / slots : 0, spread = longest - mean;
-  return (longest >= 100 ? CTX_LONG : 0) | (mean >= 200 ? CTX_FILLED : 0) | (mean + 12 * spread >= 1500 ? CTX_RAGGED : 0) | (spread >= 450 ? CTX_SPREAD : 0) |
+  return (longest >= 60 ? CTX_LONG : 0) | (mean >= 200 ? CTX_FILLED : 0) | (mean + 12 * spread >= 1500 ? CTX_RAGGED : 0) | (spread >= 450 ? CTX_SPREAD : 0) |
          (spread >= 200 && 2 * longest >= 3 * mean ? CTX_SKEWED : 0);
 }
 static bool attn_stream_ok(const AttnP& p, int B, int nw, int contexts) {
   if (p.nsplit != 1 || B > AS_MAX_SLOTS || nw < 2 || AS_WARPS % nw || sm_budget() < attn_sms()) return false;
   const int pairs = B * p.nseg, at_once = AS_WARPS / nw * attn_sms();
   const bool q8 = p.out_q, b16 = p.rp.out_b16, wide = p.kv_dim >= 2048, deep = attn_deep_ok(pairs, nw);
-  if (nw < 8 && (q8 || (b16 && !wide)) && (contexts & CTX_FILLED)) return true;
-  if (!deep && 3 * pairs < 2 * ceil_div(pairs, at_once) * at_once) return contexts & CTX_SKEWED;
+  const bool full = deep || 3 * pairs >= 2 * ceil_div(pairs, at_once) * at_once;
+  if (nw < 8 && (q8 || (b16 && !wide))) return contexts & (full ? CTX_LONG : CTX_FILLED | CTX_SKEWED);
+  if (!full) return contexts & CTX_SKEWED;
   if (q8 ? !wide : wide && deep && !b16) return contexts & CTX_LONG;
   return contexts & (deep ? CTX_SPREAD : CTX_RAGGED);
 }

@@ -102,7 +102,7 @@ __device__ __forceinline__ void report_contexts(const int* pos, int n, unsigned 
   }
   longest = __reduce_max_sync(THA_FULL_MASK, longest);
   sum = __reduce_add_sync(THA_FULL_MASK, sum);
-  if ((threadIdx.x & 31) == 0) *reinterpret_cast<volatile unsigned long long*>(out) = (unsigned long long)longest << 32 | (unsigned)(sum / n);
+  if ((threadIdx.x & 31) == 0) *reinterpret_cast<volatile unsigned long long*>(out) = (unsigned long long)(longest + 1) << 32 | (unsigned)(sum / n);
 }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Allow the next kernel in the stream to start launching.

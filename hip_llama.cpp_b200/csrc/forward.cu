@@ -81,7 +81,7 @@ struct HostContexts {
   }
   ~HostContexts() { g_host_contexts = -1; }
 };
-static int step_contexts(Workspace* ws, int B) { return g_host_contexts >= 0 ? g_host_contexts : ws_reported_contexts(ws, B); }
+static int step_contexts(Workspace* ws, int B, int seq_len) { return g_host_contexts >= 0 ? g_host_contexts : ws_reported_contexts(ws, B, seq_len); }
 #define THA_TRY_RC2(expr) do { int _st = (expr); if (_st != THA_STATUS_SUCCESS) return _st; } while (0)
 
 // A step of R >= dual_min_rows() rows is issued as TWO concurrent branches of half the rows each (fork / join inside the
@@ -302,7 +302,7 @@ int decode_step_f32(cudaStream_t st, int B, const tha_config_t* cfg, const tha_w
     THA_TRY(step_tc_prepare(ws, cfg, dp.B0));
     if (dp.on) THA_TRY(step_tc_prepare(dp.ws2, cfg, dp.B1));
     a.mega = dp.on ? 3 : 2;   // part of the graph key
-    a.contexts = dp.on ? 0 : step_contexts(ws, B);   // so is this
+    a.contexts = dp.on ? 0 : step_contexts(ws, B, cfg->seq_len);   // so is this
     float* lg = logits_d ? logits_d : s->logits;
     return run_step(st, ws, &a, sizeof(a), [&]() {
       const bool pdl = a.pdl != 0;
@@ -446,7 +446,7 @@ int decode_step_q8(cudaStream_t st, int B, const tha_config_t* cfg, const tha_we
     THA_TRY(step_tc_q8_prepare(ws, cfg, dp.B0, gs));
     if (dp.on) THA_TRY(step_tc_q8_prepare(dp.ws2, cfg, dp.B1, gs));
     a.tc = dp.on ? 2 : 1;   // part of the graph key
-    a.contexts = dp.on ? 0 : step_contexts(ws, B);   // so is this
+    a.contexts = dp.on ? 0 : step_contexts(ws, B, cfg->seq_len);   // so is this
     float* lg = logits_d ? logits_d : s->logits;
     if (!lg) return THA_STATUS_INVALID_ARG;
     return run_step(st, ws, &a, sizeof(a), [&]() {
@@ -571,7 +571,7 @@ int decode_step_bf16(cudaStream_t st, int B, const tha_config_t* cfg, const tha_
     return run_step(st, ws, &a, sizeof(a), [&]() { return issue_step_bf16_gemv(st, ws, a, lg, rc, rs); });
   }
   THA_TRY(step_bf16_prepare(ws, cfg, B));
-  a.contexts = step_contexts(ws, B);   // part of the graph key
+  a.contexts = step_contexts(ws, B, cfg->seq_len);   // part of the graph key
   return run_step(st, ws, &a, sizeof(a), [&]() {
     return step_bf16_issue(st, ws, B, *cfg, *w, *s, token_d, pos_d, lg, next_d, rc, rs, a.pdl != 0);
   }, true, a.contexts);

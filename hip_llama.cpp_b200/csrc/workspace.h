@@ -57,7 +57,7 @@ struct Workspace {
   std::mutex mu;
   int step_contexts = 0;                  // CTX_* of the step being issued (under mu)
   int attn_form = 0;                      // ATTN_* of the step being issued
-  // pinned, by number of slots: longest << 32 | mean of the contexts that the last reporting step found; 0: none yet.  A hint: every form of
+  // pinned, by number of slots: (longest + 1) << 32 | mean of the contexts that the last reporting step found; 0: none yet.  A hint: every form of
   // the attention gives the same bits, so a stale or foreign value costs time at most.
   unsigned long long* contexts_h = nullptr;
   cudaStream_t last_stream = nullptr;
@@ -79,7 +79,7 @@ Workspace* workspace();   // for the current device (thread-safe)
 int ws_ensure_attn(Workspace* ws, size_t part_slots, int n_counters);
 int ws_ensure_tokpos(Workspace* ws, int n_batches);
 unsigned long long* attn_report_to(Workspace* ws, int B, int n_heads, int n_kv_heads, int head_size, int seq_len);   // attention.cu
-int ws_reported_contexts(Workspace* ws, int slots);   // CTX_* for a step whose positions are on the device
+int ws_reported_contexts(Workspace* ws, int slots, int seq_len);   // CTX_* for a step whose positions are on the device
 int ws_ensure_q8(Workspace* ws, int n_batches, int kmax, int gs);
 int ws_ensure_dual(Workspace* ws);
 // cached graphs captured pointers that are about to change
