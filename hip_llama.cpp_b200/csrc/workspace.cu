@@ -169,7 +169,7 @@ void ws_release(Workspace* ws) {
 }
 
 int ws_reported_contexts(Workspace* ws, int slots, int seq_len) {
-  const int guess = context_class(seq_len / 2, (long long)slots * (seq_len / 4), slots);
+  const int guess = context_class(seq_len / 2, (long long)slots * (seq_len / 4), slots) & (CTX_FILLED | CTX_RAGGED | CTX_SKEWED);
   if (!ws->contexts_h || slots > CTX_MAX_SLOTS) return guess;
   const unsigned long long v = *static_cast<volatile unsigned long long*>(ws->contexts_h + slots);
   return CTX_REPORT | (v ? context_class((int)(v >> 32) - 1, (long long)(v & 0xffffffffu) * slots, slots) : guess);
