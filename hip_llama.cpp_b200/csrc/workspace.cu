@@ -147,12 +147,6 @@ Workspace* workspace() {
   if (it != g_ws.end()) return it->second;
   Workspace* ws = new Workspace();
   ws->device = dev;
-  if (cudaMallocHost((void**)&ws->contexts_h, (CTX_MAX_SLOTS + 1) * sizeof(unsigned long long)) == cudaSuccess)
-    memset(ws->contexts_h, 0, (CTX_MAX_SLOTS + 1) * sizeof(unsigned long long));
-  else {
-    cudaGetLastError();
-    ws->contexts_h = nullptr;   // no reports
-  }
   g_ws[dev] = ws;
   return ws;
 }
@@ -170,7 +164,17 @@ void ws_release(Workspace* ws) {
 
 int ws_reported_contexts(Workspace* ws, int slots, int seq_len) {
   const int guess = context_class(seq_len / 2, (long long)slots * (seq_len / 4), slots) & (CTX_FILLED | CTX_RAGGED | CTX_SKEWED);
-  if (!ws->contexts_h || slots > CTX_MAX_SLOTS) return guess;
+  if (slots > CTX_MAX_SLOTS) return guess;
+  {
+    std::lock_guard<std::mutex> lk(g_mu);
+    if (!ws->contexts_tried) {   // with the first decode step, as all scratch of one: an operation by itself may be under the caller's capture
+      ws->contexts_tried = true;
+      const size_t bytes = (CTX_MAX_SLOTS + 1) * sizeof(unsigned long long);
+      if (cudaMallocHost((void**)&ws->contexts_h, bytes) == cudaSuccess) memset(ws->contexts_h, 0, bytes);
+      else { cudaGetLastError(); ws->contexts_h = nullptr; }   // no reports
+    }
+  }
+  if (!ws->contexts_h) return guess;
   const unsigned long long v = *static_cast<volatile unsigned long long*>(ws->contexts_h + slots);
   return CTX_REPORT | (v ? context_class((int)(v >> 32) - 1, (long long)(v & 0xffffffffu) * slots, slots) : guess);
 }

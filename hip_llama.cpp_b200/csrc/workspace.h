@@ -60,6 +60,7 @@ struct Workspace {
   // pinned, by number of slots: (longest + 1) << 32 | mean of the contexts that the last reporting step found; 0: none yet.  A hint: every form of
   // the attention gives the same bits, so a stale or foreign value costs time at most.
   unsigned long long* contexts_h = nullptr;
+  bool contexts_tried = false;
   cudaStream_t last_stream = nullptr;
   cudaEvent_t step_done = nullptr;
   // two half-batches of a step as two concurrent branches of the graph (forward.cu, "dual"): the second branch's
