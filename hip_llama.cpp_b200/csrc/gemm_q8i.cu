@@ -18,7 +18,7 @@
 // has to stay below that, so the issuer and the producer are one elected thread each that counts instead of dividing.  Many columns: the epilogue,
 // 16384 sums per slot of 64 columns to convert, scale twice and add (1700 instructions a slot besides what the hand-over of a slot takes,
 // which is paid per warp: hence few warps with many columns, and U columns of one group at a time with the next U already on their way out of TMEM).
-// Two or three epilogue warps a scheduler leave 40 % of the issue slots empty.  At 4096 of K and 64 values a group, us, before (two issuers, 16 warps with
+// Two or three epilogue warps a scheduler leave a third of the issue slots empty.  At 4096 of K and 64 values a group, us, before (two issuers, 16 warps with
 // all of a slot in registers, the item's scales staged between two barriers) and now: 930 rows x 12288 293 -> 171, 64 x 32000 66.5 -> 43.7,
 // 32 x 32000 41.5 -> 33.5, 1 x 12288 19.6 -> 17.6; 930 x 4096 x 11008 290 -> 158.  64 columns by 16 warps instead of 8: 253 for the first of these.
 // mma.sync instead, with the sums in registers: 329, and 29.8 for one row.
@@ -462,7 +462,8 @@ int gemm_q8i_launch(cudaStream_t st, const Q8iArgs& a, bool pdl) {
   const int splits = a.splits < 1 ? 1 : a.splits;
   p.slots_per_split = ceil_div(p.slots_total, splits);
   if (ceil_div(p.slots_total, p.slots_per_split) != splits) return THA_STATUS_INVALID_ARG;
-  {  // the longest split: an item's scales ([groups][planned tile] floats) beside three slots of the planned tile in 220 KB
+  {  // The longest split that is served: an item's scales ([groups][planned tile] floats) beside three slots of the planned tile in 220 KB.  The scales
+     // travel with their slots now and set no limit; what calls are refused is as it was.
     const int slot = TC_BM * 128 + plan_nt * 128, sb = a.gs / plan_nt;
     const int fit = (TC_SMEM_LIMIT - 3072) / slot > 10 ? 10 : (TC_SMEM_LIMIT - 3072) / slot;
     if (fit - ceil_div(ceil_div(p.slots_per_split, sb) * sb * (128 / a.gs) * plan_nt * 4, slot) < 3) return THA_STATUS_NOT_SUPPORTED;
