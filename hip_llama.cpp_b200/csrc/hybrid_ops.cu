@@ -1853,9 +1853,12 @@ static int attn_max_keys(const tha_attn_t* a, int max_pos) {
   if (a->window > 0 && a->window + a->keep_first + 2 * ATT_KEYS < max_keys) max_keys = a->window + a->keep_first + 2 * ATT_KEYS;
   return max_keys;
 }
-// All that the runs of keys below depend on of max_pos: two tiles each at least, never more than 32 of them.
-int tha::hyb_attn_run_limit(const tha_attn_t* a, int max_pos) {
-  const int n = attn_max_keys(a, max_pos) / (2 * ATT_KEYS);
+// All that the launches below depend on of max_pos in a step of one row a sequence: the runs of the row kernel; in the tiled forms two tiles each at
+// least, never more than 32 runs.
+int tha::hyb_attn_single_runs(const tha_attn_t* a, const tha_rows_t* rows, const tha_kv_t* kv) {
+  const int max_keys = attn_max_keys(a, rows->max_pos);
+  if (hyb_attn_row_ok(a, kv, nullptr)) return hyb_attn_row_splits(a, rows, max_keys);
+  const int n = max_keys / (2 * ATT_KEYS);
   return n < 32 ? n : 32;
 }
 

@@ -16,8 +16,9 @@ __device__ __forceinline__ void hyb_pdl_enter() { pdl_trigger(); pdl_wait(); }
 // the step writes it, and whose first kernel is launched behind the completion of all that is ahead of the step on its stream -- in
 // a call of its own a matrix may be what the kernel ahead is writing.
 bool hyb_gemm_pdl();
-int hyb_attn_run_limit(const tha_attn_t* a, int max_pos);   // hybrid_ops.cu: what the attention's launches depend on of the longest context
-bool hyb_scan_in_registers();                               // hybrid_ops.cu: THA_HYB_SCAN
+// hybrid_ops.cu: what the attention's launches depend on of the longest context, single rows; THA_HYB_SCAN
+int hyb_attn_single_runs(const tha_attn_t* a, const tha_rows_t* rows, const tha_kv_t* kv);
+bool hyb_scan_in_registers();
 __device__ __forceinline__ float hyb_load(const float* p) { return *p; }
 __device__ __forceinline__ float hyb_load(const __nv_bfloat16* p) { return __bfloat162float(*p); }
 __device__ __forceinline__ void hyb_store(float* p, float v) { *p = v; }

@@ -768,9 +768,10 @@ extern "C" int tha_hyb_step_planned(void* stream, tha_hyb_plan_t* plan, const th
   for (int li = 0; li < m->n_layers; li++) {
     const tha_hyb_layer_t& L = m->layers[li];
     tha_attn_t at = L.attn;
-    if (L.mixer == THA_MIX_LATENT) at = latent_attn(L.latent);
+    tha_kv_t akv = *kv;
+    if (L.mixer == THA_MIX_LATENT) { at = latent_attn(L.latent); akv.v_pool = akv.k_pool; }
     else if (L.mixer != THA_MIX_ATTN && L.mixer != THA_MIX_ATTN_GDELTA && L.mixer != THA_MIX_PARALLEL) continue;
-    put(hyb_attn_run_limit(&at, rows->max_pos));
+    put(hyb_attn_single_runs(&at, rows, &akv));
     put(hyb_attn_tc_scratch(&at, rows));
   }
   HybForm* f = nullptr;
