@@ -496,42 +496,54 @@ int step_bf16_prefill(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
   int *h_slot = tab.data(), *h_pos = h_slot + R, *h_tok = h_pos + R, *h_t0 = h_tok + R, *h_tn = h_t0 + T, *h_last = h_tn + T;
   int *h_srow = h_last + n_seqs, *h_spad = h_srow + R;   // staged row of every row: a sequence's positions from 0 on, at a multiple of 128
   int *h_sslot = h_spad + R, *h_upto = h_sslot + n_seqs, *h_sbase = h_upto + n_seqs;
-  const long long most = bf_stage_rows(hs * c.n_kv_heads, R);
-  std::vector<BfGroup> groups;
-  int r = 0, t = 0;
-  long long Rs = 0, at = 0;   // staged rows of the largest group, and of the last one so far
-  bool behind = false;        // a portion behind a context
-  for (int i = 0; i < n_seqs; i++) {
-    const int end = pos0[i] + len[i], rows = ceil_div(end, 128) * 128;
-    if (i == 0 || at + rows > most) { groups.push_back({i, 0, t, 0, 0}); at = 0; }
-    BfGroup& g = groups.back();
-    g.n_seqs++;
-    if (pos0[i] > g.longest) g.longest = pos0[i];
-    behind = behind || pos0[i] > 0;
-    for (int j = 0; j < len[i]; j++) { h_srow[r + j] = (int)at + pos0[i] + j; h_spad[r + j] = j + 1 < len[i] ? 0 : -end & 15; }
-    h_sslot[i] = slot[i]; h_upto[i] = pos0[i]; h_sbase[i] = (int)at;
-    at += rows;
-    if (at > Rs) Rs = at;
-    for (int j = 0; j < len[i]; j += TQ) { h_t0[t] = r + j; h_tn[t] = (len[i] - j < TQ) ? len[i] - j : TQ; t++; }
-    g.n_tiles = t - g.tile0;
+  for (int i = 0, r = 0; i < n_seqs; i++) {
     for (int j = 0; j < len[i]; j++, r++) {
       h_slot[r] = slot[i]; h_pos[r] = pos0[i] + j; h_tok[r] = tokens[r];
       if (tokens[r] < 0 || tokens[r] >= c.vocab_size) return THA_STATUS_INVALID_ARG;
     }
-    h_last[i] = r - 1;
+    h_sslot[i] = slot[i]; h_last[i] = r - 1;
   }
-  if (groups.size() > 1)   // everything from the cache, with the zeros behind it: the rows that this call brings lie there by then
-    for (BfGroup& g : groups) {
-      g.longest = 0;
-      for (int i = g.seq0; i < g.seq0 + g.n_seqs; i++) {
-        h_upto[i] = pos0[i] + len[i];
-        if (((h_upto[i] + 15) & ~15) > g.longest) g.longest = (h_upto[i] + 15) & ~15;
-      }
+  std::vector<BfGroup> groups;
+  long long Rs = 0;           // staged rows of the largest group
+  bool behind = false;        // a portion behind a context
+  auto lay_out = [&](long long most) {   // groups of at most so many staged rows, or of one sequence
+    groups.clear();
+    Rs = 0;
+    long long at = 0;
+    for (int i = 0, r = 0, t = 0; i < n_seqs; r += len[i], i++) {
+      const int end = pos0[i] + len[i], rows = ceil_div(end, 128) * 128;
+      if (i == 0 || at + rows > most) { groups.push_back({i, 0, t, 0, 0}); at = 0; }
+      BfGroup& g = groups.back();
+      g.n_seqs++;
+      if (pos0[i] > g.longest) g.longest = pos0[i];
+      behind = behind || pos0[i] > 0;
+      for (int j = 0; j < len[i]; j++) { h_srow[r + j] = (int)at + pos0[i] + j; h_spad[r + j] = j + 1 < len[i] ? 0 : -end & 15; }
+      h_upto[i] = pos0[i]; h_sbase[i] = (int)at;
+      at += rows;
+      if (at > Rs) Rs = at;
+      for (int j = 0; j < len[i]; j += TQ) { h_t0[t] = r + j; h_tn[t] = (len[i] - j < TQ) ? len[i] - j : TQ; t++; }
+      g.n_tiles = t - g.tile0;
     }
+    if (groups.size() > 1)   // everything from the cache, with the zeros behind it: the rows that this call brings lie there by then
+      for (BfGroup& g : groups) {
+        g.longest = 0;
+        for (int i = g.seq0; i < g.seq0 + g.n_seqs; i++) {
+          h_upto[i] = pos0[i] + len[i];
+          if (((h_upto[i] + 15) & ~15) > g.longest) g.longest = (h_upto[i] + 15) & ~15;
+        }
+      }
+  };
+  const long long most = bf_stage_rows(hs * c.n_kv_heads, R);
+  lay_out(most);
   // Scratch that grows frees and drops the workspace's graphs: a prompt in portions, which asks for more with each, gets room for whole contexts.
   long long keep = behind ? (long long)n_seqs * (ceil_div(c.seq_len, 128) * 128) : 0;
   if (keep > most) keep = most;
-  THA_TRY_RC(bf_prepare(ws, c, (int)R, true, (int)tab.size(), TQ == 128 ? Rs : 0, keep));
+  int rc_prep = bf_prepare(ws, c, (int)R, true, (int)tab.size(), TQ == 128 ? Rs : 0, keep);
+  if (rc_prep != THA_STATUS_SUCCESS && behind && TQ == 128) {   // no room for that: one sequence at a time
+    lay_out(0);
+    rc_prep = bf_prepare(ws, c, (int)R, true, (int)tab.size(), Rs, 0);
+  }
+  THA_TRY_RC(rc_prep);
   BfScratch sc;
   {
     std::lock_guard<std::mutex> lk(g_bf_mu);

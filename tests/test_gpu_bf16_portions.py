@@ -1,6 +1,10 @@
 """Prompts of the bf16 model in portions (csrc/attn_prefill_tc.cu; the rows ahead of a portion by bf_kv_context_kernel): cuts and ends on both sides of the
 groups of 16 keys and the tiles of 128, plain and paged caches, with NaN in scratch from a call before.  Same statement and bound as
 tests/test_gpu_bf16.py: a rounding that falls on the other side moves a logit by a few 1e-3 of the largest, three such steps are allowed."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -84,6 +88,42 @@ def test_scratch_of_many_short_portions_behind_long_contexts_is_bounded():
         assert_close_scaled(got[i].cpu().numpy(), want[i].cpu().numpy(), BF16_EPS, f"sequence {i}")
     for a, b in zip(rows, (e.state.key_cache, e.state.value_cache)):
         assert float((a - b).abs().max()) <= BF16_EPS * float(a.abs().max())
+
+
+def test_contexts_that_do_not_fit_side_by_side_are_taken_one_by_one():
+    """With room for one context of them, not for 256 MB: the results of the call that had it, to the bit.  In a process of its own, whose scratch is
+    not there yet."""
+    code = "import test_gpu_bf16_portions as t; t.one_by_one()"
+    r = subprocess.run([sys.executable, "-c", code], cwd=os.path.dirname(os.path.abspath(__file__)), capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "one by one: the same" in r.stdout, r.stdout + r.stderr
+
+
+def one_by_one():
+    import torch
+    rng = np.random.default_rng(4)
+    seqs = [(i, int(rng.integers(1900, 2040)), rng.integers(0, 96, int(rng.integers(1, 20))).astype(np.int32)) for i in range(100)]
+    big = engine(100, 2064, 2)              # its cache is what the second call holds the memory with
+    before = big.state.key_cache.clone(), big.state.value_cache.clone()
+    got = []
+    cabi = load_pkg("cabi").lib()
+    for tight in (True, False):
+        big.state.key_cache.copy_(before[0])
+        big.state.value_cache.copy_(before[1])
+        held = None
+        logits, nxt = torch.empty(100, 96, device="cuda"), torch.empty(100, dtype=torch.int32, device="cuda")
+        if tight:
+            big.prefill([(0, 0, np.zeros(1200, np.int32))])       # the scratch of the rows themselves
+            big.state.key_cache.copy_(before[0])
+            big.state.value_cache.copy_(before[1])
+            held = torch.empty(max(0, free() - (120 << 20)), dtype=torch.uint8, device="cuda")
+        big.prefill(seqs, logits, nxt)
+        torch.cuda.synchronize()
+        assert cabi.c.tha_gemm_check_error() == 0
+        got.append(logits)
+        del held
+        torch.cuda.empty_cache()
+    assert torch.equal(got[0], got[1])
+    print("one by one: the same")
 
 
 def test_portions_of_a_prompt_grow_the_scratch_once():
