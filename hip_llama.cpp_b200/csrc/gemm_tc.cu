@@ -47,11 +47,13 @@ namespace tha {
 
 // Persistent: a CTA walks the work items (weight tile, column tile, K split) blockIdx.x, blockIdx.x + gridDim.x, ...
 // with running stage counters, so the weight ring keeps streaming while the previous item's accumulator is read out.
+// p stays where the launch put it: its arrays are indexed by matrix, and without __grid_constant__ every thread first copied it to local memory (a step of
+// stories110M at 256 slots 1313 -> 1278 us, of two Llama-2-7B layers at 6 slots 465 -> 449).
 template <int NT>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant__ CUtensorMap mw1,
                    const __grid_constant__ CUtensorMap mw2, const __grid_constant__ CUtensorMap mxh,
-                   const __grid_constant__ CUtensorMap mxl, const TcP p) {
+                   const __grid_constant__ CUtensorMap mxl, const __grid_constant__ TcP p) {
   using S = TcSmem<NT>;
   extern __shared__ unsigned char tc_smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
