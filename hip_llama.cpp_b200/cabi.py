@@ -99,6 +99,7 @@ class Lib:
             "tha_forward_batch_q8": [vp, I, C.POINTER(Config), C.POINTER(WeightsQ8), C.POINTER(State), vp, vp, vp],
             "tha_decode_step_q8": [vp, I, C.POINTER(Config), C.POINTER(WeightsQ8), C.POINTER(State), vp, vp, vp, vp],
             "tha_gemm_tf32x3": [vp, vp, C.c_longlong, vp, I, I, vp, I, C.c_longlong],
+            "tha_gemm_f16x3": [vp, vp, C.c_longlong, vp, I, I, vp, I, C.c_longlong, I, vp, vp, vp],
             "tha_gemm_bf16": [vp, vp, C.c_longlong, vp, I, I, vp, I, C.c_longlong],
             "tha_convert_bf16": [vp, vp, vp, C.c_size_t],
             "tha_forward_batch_bf16": [vp, I, C.POINTER(Config), C.POINTER(WeightsBF16), C.POINTER(State), vp, vp, vp],

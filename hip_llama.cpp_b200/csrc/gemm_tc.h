@@ -25,6 +25,28 @@ struct TcP {                  // kernel parameter block
   long long* trace;           // development aid (tha_gemm_trace)
 };
 
+// fp32 weights x activations split into fp16 hi and lo (gemm_f16x3.cu)
+struct X3Args {
+  int n_mats; const float* W[3]; int M[3]; int out_off[3];
+  int K;
+  const uint16_t* Xhi; const uint16_t* Xlo; int N;             // planes [N, K]
+  const float* colscale;                                       // [N], 16-byte aligned: what a product with row n is multiplied by
+  float* out; long long ldo; long long zstride; int splits;
+};
+bool gemm_f16x3_width_ok(int K);
+int gemm_f16x3_splits(int tiles256, int rows_out, int K, int N);   // tiles256: 256-row weight tiles of all matrices, rows_out: their rows
+int gemm_f16x3_launch(cudaStream_t st, const X3Args& a, bool pdl);
+struct X3RowsP {                                               // rows -> planes
+  float* x; long long ld;                                      // rows to be split [rows, ld] (the norm: ld = n); SwiGLU: ld of the partials
+  const float* part; int nz; long long zstride;
+  const float* emb; const int* token; const int* pos; const float* gain;
+  int n;                                                       // values a row
+  uint16_t *hi, *lo; float* scale;
+};
+int x3_norm_launch(cudaStream_t st, bool pdl, int rows, const X3RowsP& p);
+int x3_swiglu_launch(cudaStream_t st, bool pdl, int rows, const X3RowsP& p);
+int x3_split_launch(cudaStream_t st, bool pdl, int rows, const X3RowsP& p);
+
 // Q8_0 weights x Q8_0 activations on the int8 tensor cores (gemm_q8i_kernel)
 struct Q8iArgs {
   int n_mats; const int8_t* Wq[3]; const float* Ws[3]; int M[3]; int out_off[3];

@@ -554,6 +554,8 @@ struct TcScratch {
   // chained matmuls (chain_tc.cu): attention output hi/lo, sums of squares per row tile, counter blocks (one per launch of a step)
   float *ah = nullptr, *al = nullptr, *ss = nullptr; int* ctr = nullptr;
   size_t n_ah = 0, n_al = 0, n_ss = 0; int ctr_stride = 0, n_ctr_blocks = 0;
+  float* scale2 = nullptr;                              // fp16 planes: scales of the rows that are not norms (gemm_f16x3.cu)
+  size_t n_scale2 = 0;
   size_t n_x = 0, n_xl = 0, n_h = 0, n_hl = 0, n_part = 0, n_xr = 0, n_qr = 0, n_xbr = 0, n_tab = 0; int n_b = 0;
 };
 static std::map<Workspace*, TcScratch> g_tc_scratch;   // per workspace (= per device, or per tensor-parallel rank)
@@ -564,7 +566,7 @@ void step_tc_release(Workspace* ws) {
   auto it = g_tc_scratch.find(ws);
   if (it == g_tc_scratch.end()) return;
   TcScratch& s = it->second;
-  void* ptrs[] = {s.xh, s.xl, s.hh, s.hl, s.scale, s.part, s.xr, s.qr, s.xbr, s.tab, s.xq, s.hq, s.xsT, s.hsT, s.ah, s.al, s.ss, s.ctr};
+  void* ptrs[] = {s.xh, s.xl, s.hh, s.hl, s.scale, s.part, s.xr, s.qr, s.xbr, s.tab, s.xq, s.hq, s.xsT, s.hsT, s.ah, s.al, s.ss, s.ctr, s.scale2};
   for (void* p : ptrs) if (p) cudaFree(p);
   g_tc_scratch.erase(it);
 }
@@ -632,18 +634,33 @@ static Dims dims_of(const tha_config_t& c, const TpCtx* tp) {
   return m;
 }
 
+// Whether fp32 prompt rows go through gemm_f16x3.cu: its pairs of CTAs have 256 x 128 outputs, want a kernel more a layer (the attention's rows split by
+// themselves) and a while to fill.  us a prompt, 3xTF32 / this: width 4096, 2 layers, 50 rows 556 / 544, 65 rows 673 / 559, 128 rows 675 / 597, 600 rows 3012 / 1884;
+// 2048, 4 layers, 65 rows 555 / 562, 128 rows 530 / 569, 130 rows 753 / 640; 1024, 6 layers, 384 rows 570 / 610, 512 rows 1162 / 1065; 768, 12 layers, 384 rows
+// 982 / 1076, 460 rows 1392 / 1431, 600 rows 2460 / 2043; 512, 8 layers, 384 rows 524 / 599, 600 rows 1302 / 1101.
+static bool rows_f16x3(const Dims& m, int R, bool prefill, bool q8, bool tp) {
+  return prefill && !q8 && !tp && (R >= PROMPT_ROWS || (m.d >= 2048 && (long long)R * m.d > 1 << 18)) && gemm_f16x3_width_ok(m.d) && gemm_f16x3_width_ok(m.da) && gemm_f16x3_width_ok(m.hd);
+}
+
 static int plan_z(int tiles, int K, int R, bool q8, int gs) {
   if (q8) return pick_splits_q8(tiles, K, R, gs);
   return pick_splits(tiles * ceil_div(R, gemm_tc_pick_nt(R)), K, R, 1);
 }
 
-static TcPlan make_plan(const Dims& m, int R, bool q8, int gs = 64) {
+static TcPlan make_plan(const Dims& m, int R, bool q8, int gs = 64, bool f16x3 = false) {
   const int d = m.d, da = m.da, hd = m.hd, kvd = m.kvd;
   TcPlan p;
+  if (f16x3) {
+    p.z_qkv = gemm_f16x3_splits(ceil_div(da, 256) + 2 * ceil_div(kvd, 256), da + 2 * kvd, d, R);
+    p.z_wo = gemm_f16x3_splits(ceil_div(d, 256), d, da, R);
+    p.z_w13 = gemm_f16x3_splits(2 * ceil_div(hd, 256), 2 * hd, d, R);
+    p.z_w2 = gemm_f16x3_splits(ceil_div(d, 256), d, hd, R);
+  } else {
   p.z_qkv = plan_z(ceil_div(da, 128) + 2 * ceil_div(kvd, 128), d, R, q8, gs);
   p.z_wo = plan_z(ceil_div(d, 128), da, R, q8, gs);
   p.z_w13 = plan_z(2 * ceil_div(hd, 128), d, R, q8, gs);
   p.z_w2 = plan_z(ceil_div(d, 128), hd, R, q8, gs);
+  }
   {   // development aid: THA_TC_Z="qkv,wo,w13,w2" overrides the planner (0 keeps its choice)
     static int ov[4] = {-1, 0, 0, 0};
     if (ov[0] < 0) {
@@ -690,7 +707,9 @@ static int prepare_rows(Workspace* ws, const tha_config_t* c, int R, bool prefil
   std::lock_guard<std::mutex> lk(g_tc_scratch_mu);
   TcScratch& s = g_tc_scratch[ws];
   const Dims dm = dims_of(*c, tp);
-  const TcPlan pl = make_plan(dm, R, q8, gs);
+  const bool f16x3 = rows_f16x3(dm, R, prefill, q8, tp != nullptr);
+  const TcPlan pl = make_plan(dm, R, q8, gs, f16x3);
+  if (f16x3) THA_TRY_RC(grow(&s.scale2, &s.n_scale2, (size_t)R, ws));
   if (q8) {   // int8 rows (sized in floats: bytes / 4) and transposed scales (rows padded to the widest column tile)
     const size_t ldxs = (size_t)ceil_div(R, 64) * 64;
     THA_TRY_RC(grow(reinterpret_cast<float**>(&s.xq), &s.n_xq, ((size_t)R * c->dim + 3) / 4, ws));
@@ -934,7 +953,8 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
     return issue_rows_chain(st, ws, c, w, s, sc, io, rc, rs, pdl);
   const int gs = wq ? wq->group_size : 0;
   const Dims dm = dims_of(c, tp);
-  const TcPlan pl = make_plan(dm, R, q8, q8 ? gs : 64);
+  const bool f16x3 = rows_f16x3(dm, R, io.n_tiles > 0, q8, tp != nullptr);
+  const TcPlan pl = make_plan(dm, R, q8, q8 ? gs : 64, f16x3);
   const int d = dm.d, da = dm.da, hd = dm.hd, hs = dm.hs, kvd = dm.kvd, L = c.n_layers;
   const long long kv_bs = (long long)L * c.seq_len * kvd;
   const int ld_qkv = da + 2 * kvd, ld_h = 2 * hd;
@@ -957,6 +977,9 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
     }
     if (need > tp->xchg_floats || !tp->connected || tp->hidden_of[tp->rank] != hd) return THA_STATUS_INVALID_ARG;
   }
+  // fp16 planes in the place of the tf32 ones (half their bytes)
+  uint16_t *const xh16 = reinterpret_cast<uint16_t*>(sc.xh), *const xl16 = reinterpret_cast<uint16_t*>(sc.xl);
+  uint16_t *const hh16 = reinterpret_cast<uint16_t*>(sc.hh), *const hl16 = reinterpret_cast<uint16_t*>(sc.hl);
   const int skip = skip_mask();
   KvPool pool;
   const bool paged = kv_pool_find(s.key_cache, &pool);
@@ -986,6 +1009,11 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
     if (wq) {
       THA_CUDA_OK(launch(tell ? tc_prep_q8_kernel<true> : tc_prep_q8_kernel<false>, dim3(rows + tell), dim3(prep_threads), 0, st, pdl, io.x, part, nz, zs,
                          emb, io.token, io.pos, gain, d, gs, sc.xq, sc.xsT, ldxs, gather, tpp, report));
+    } else if (f16x3 && !gather) {
+      X3RowsP a = {};
+      a.x = io.x; a.ld = d; a.part = part; a.nz = nz; a.zstride = zs; a.emb = emb; a.token = io.token; a.pos = io.pos; a.gain = gain;
+      a.n = d; a.hi = xh16; a.lo = xl16; a.scale = sc.scale;
+      THA_TRY_RC(x3_norm_launch(st, pdl, rows, a));
     } else if (prompt_form(rows, d) && !gather && !tpp.n) {
       THA_CUDA_OK(launch(tc_prep_prompt_kernel, dim3(rows), dim3(prompt_threads), 0, st, pdl, io.x, part, nz, zs, emb, io.token, io.pos, gain, d, sc.xh, sc.xl, sc.scale));
     } else {
@@ -1001,6 +1029,14 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
                 const float* colscale) -> int {
     if ((skip & 1) && out != io.logits) return THA_STATUS_SUCCESS;
     if ((skip & 32) && out == io.logits) return THA_STATUS_SUCCESS;
+    if (f16x3 && out != io.logits) {
+      X3Args a = {};
+      a.n_mats = n;
+      for (int i = 0; i < n; i++) { a.W[i] = W[i]; a.M[i] = M[i]; a.out_off[i] = off[i]; }
+      a.K = K; a.Xhi = reinterpret_cast<const uint16_t*>(xh); a.Xlo = reinterpret_cast<const uint16_t*>(xl); a.N = N;
+      a.colscale = colscale ? colscale : sc.scale2; a.out = out; a.ldo = ldo; a.zstride = zs; a.splits = z;
+      return gemm_f16x3_launch(st, a, pdl);
+    }
     if (!wq) return gemm(st, pdl, n, W, M, off, K, xh, xl, N, out, ldo, zs, z, colscale);
     const int8_t* q[3]; const float* sc3[3];
     for (int i = 0; i < n; i++) {
@@ -1041,8 +1077,8 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
     }
     if (skip & 2) {
     } else if (io.n_tiles > 0) {
-      THA_TRY_RC(attn_prefill_launch(st, io.n_tiles, c.n_heads, c.n_kv_heads, hs, io.q, io.xb, wq ? nullptr : sc.xh,
-                                     wq ? nullptr : sc.xl, kcl, vcl, kv_bs, io.slot, io.pos,
+      THA_TRY_RC(attn_prefill_launch(st, io.n_tiles, c.n_heads, c.n_kv_heads, hs, io.q, io.xb, wq || f16x3 ? nullptr : sc.xh,
+                                     wq || f16x3 ? nullptr : sc.xl, kcl, vcl, kv_bs, io.slot, io.pos,
                                      io.tile_row0, io.tile_n, pdl, &pg, io.tile_rows));
     } else if (rope_in_attn) {
       THA_TRY_RC(attn_fused_rope_launch(st, ws, R, io.pos, c.n_heads, c.n_kv_heads, io.q, io.xb, const_cast<float*>(kcl),
@@ -1056,6 +1092,10 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
                                    wq ? sc.xq : nullptr, wq ? sc.xsT : nullptr, ldxs, gs, &pg));
     }
     if ((skip & 16) || (wq && io.n_tiles == 0 && !(skip & 2))) {
+    } else if (f16x3) {
+      X3RowsP a = {};
+      a.x = io.xb; a.ld = da; a.pos = io.pos; a.n = da; a.hi = xh16; a.lo = xl16; a.scale = sc.scale2;
+      THA_TRY_RC(x3_split_launch(st, pdl, R, a));
     } else if (wq)   // prompt rows: runq.c:437 as its own launch
       THA_TRY_RC(quant_split_launch(st, pdl, R, d, io.xb, (long long)da, 0, 0LL, 0, io.pos, da, gs, sc.xq, sc.xsT, ldxs));
     {
@@ -1074,7 +1114,11 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
     if (skip & 16) {
     } else if (wq)   // runq.c:457-465: SwiGLU, then quantise hb
       THA_TRY_RC(quant_split_launch(st, pdl, R, d, sc.part, (long long)ld_h, pl.z_w13, (long long)R * ld_h, hd, io.pos, hd, gs, sc.hq, sc.hsT, ldxs));
-    else if (prompt_form(R, d))
+    else if (f16x3) {
+      X3RowsP a = {};
+      a.part = sc.part; a.ld = ld_h; a.nz = pl.z_w13; a.zstride = (long long)R * ld_h; a.pos = io.pos; a.n = hd; a.hi = hh16; a.lo = hl16; a.scale = sc.scale2;
+      THA_TRY_RC(x3_swiglu_launch(st, pdl, R, a));
+    } else if (prompt_form(R, d))
       THA_CUDA_OK(launch(tc_swiglu_split_wide_kernel, dim3(ceil_div(hd, 2048), R), dim3(256), 0, st, pdl, (const float*)sc.part, pl.z_w13,
                          (long long)R * ld_h, ld_h, io.pos, hd, sc.hh, sc.hl));
     else

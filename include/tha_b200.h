@@ -137,6 +137,10 @@ int tha_gemm_tf32x3(void* stream, float* out, long long ldo, const float* W, int
                     long long ldx);
 /* 1 if a tensor-core matmul on the current device gave up on a pipeline barrier since the last call */
 int tha_gemm_check_error(void);
+/* The fp32 matmul of prompts: operands split into fp16 hi and lo under a power of two a row, three products.  hi, lo [N, K] (raw fp16) and scale [N] are
+ * scratch of the caller's; the z-th of `splits` shares of K lands in out + z * N * ldo.  K % 8 == 0, 64 <= K <= 16384, ldx % 4 == 0, 16-byte aligned pointers. */
+int tha_gemm_f16x3(void* stream, float* out, long long ldo, const float* W, int M, int K, const float* X, int N, long long ldx, int splits,
+                   uint16_t* hi, uint16_t* lo, float* scale);
 /* bf16 weights x bf16 activations on the tensor cores (tcgen05.mma.kind::f16, fp32 accumulate), fp32 out:
  * out[n*ldo + row] = sum_k W[row,k] X[n,k]; W [M,K], X [N,ldx] as raw bf16 bit patterns; K % 8 == 0, K >= 64.
  * The matmul of the bf16 model path (tha_*_bf16 below). */

@@ -1,0 +1,107 @@
+"""The fp32 matmul of prompts (csrc/gemm_f16x3.cu): three fp16 products of split operands, against float64."""
+import numpy as np
+import pytest
+import torch
+
+import llama64
+from gpu_util import P, stream_ptr
+from pkgload import load_pkg
+
+pytestmark = pytest.mark.gpu
+RUN = 16 * 64      # values of K that the tensor core sums up before they leave it
+
+
+def product(W, X, splits=1, ldo=None):
+    lib = load_pkg("cabi").lib()
+    (M, K), (N, ldx) = W.shape, X.shape
+    ldo = ldo or M
+    out = torch.full((splits, N, ldo), float("nan"), device="cuda")
+    planes = [torch.empty(N, K, dtype=torch.int16, device="cuda") for _ in range(2)]
+    scale = torch.empty(N, device="cuda")
+    lib.check(lib.c.tha_gemm_f16x3(stream_ptr(), P(out), ldo, P(W), M, K, P(X), N, ldx, splits, P(planes[0]), P(planes[1]), P(scale)), "tha_gemm_f16x3")
+    torch.cuda.synchronize()
+    assert lib.c.tha_gemm_check_error() == 0
+    return out
+
+
+def check(W, X, splits=1, ldo=None):
+    (M, K) = W.shape
+    out = product(W, X, splits, ldo)
+    if ldo:
+        assert torch.isnan(out[:, :, M:]).all()
+    got = out[:, :, :M].double().sum(0)
+    w, x = W.double(), X[:, :K].double()
+    want, size = x @ w.T, x.abs() @ w.abs().T
+    # hi + lo holds 22 bits and lo.lo is left out: 3 2^-22 of a product; an addition in the tensor core drops less than 2^-23 of the running sum, K / 16 of them a run
+    # (and two for the corrections), then a rounding for each run and three to scale
+    bound = 3 * 2.0 ** -22 + (min(K, RUN) / 16 + 4 + K / RUN + 3) * 2.0 ** -23
+    assert ((got - want).abs() <= bound * size).all()
+    return got, want
+
+
+@pytest.mark.parametrize("M,K,N,splits", [(1, 64, 1, 1), (127, 72, 63, 1), (128, 128, 64, 1), (129, 136, 65, 1), (256, 1024, 127, 1), (257, 1032, 128, 1),
+                                          (600, 2056, 129, 2), (513, 4096, 200, 5), (19072, 192, 257, 1), (300, 16384, 3, 1)])
+def test_product(M, K, N, splits):
+    g = torch.Generator(device="cuda").manual_seed(M + K + N)
+    W, X = (torch.randn(s, device="cuda", generator=g) for s in ((M, K), (N, K + 8)))
+    check(W, X, splits, ldo=M + 5)
+
+
+@pytest.mark.parametrize("splits", [1, 2])
+def test_rows_beyond_their_first_values(splits):
+    """Weight rows whose first values say nothing of the others: the pair of CTAs that has one goes over its items again."""
+    g = torch.Generator(device="cuda").manual_seed(3)
+    W, X = torch.randn(700, 1024, device="cuda", generator=g) * 0.02, torch.randn(200, 1024, device="cuda", generator=g)
+    W[3, 200:] *= 1e4
+    W[5, :128] = 0
+    W[130, :1000] = 0
+    W[300] = 0
+    W[301, 700] = 1e7
+    W[302] *= 1e-20
+    W[303] *= 1e20
+    W[600, :128] *= 1e-30
+    X[7] *= 1e-15
+    X[8, 5] = 1e6
+    X[9] = 0
+    X[199] *= 1e15
+    check(W, X, splits)                             # every output against the sizes of its own row and column
+
+
+def test_values_that_are_not_finite_stay_in_their_rows():
+    g = torch.Generator(device="cuda").manual_seed(4)
+    W, X = torch.randn(300, 256, device="cuda", generator=g), torch.randn(70, 256, device="cuda", generator=g)
+    W[20, 50], W[21, 200], X[30, 3], X[31, 3] = float("inf"), float("nan"), float("-inf"), float("nan")
+    bad = ~torch.isfinite(product(W, X)[0])
+    want = torch.zeros_like(bad)
+    want[30:32] = True
+    want[:, 20:22] = True
+    assert torch.equal(bad, want)
+
+
+@pytest.mark.parametrize("heads,hs,kv_heads,hidden,lens", [(16, 128, 16, 4104, [64]), (16, 128, 4, 4104, [65]), (16, 128, 16, 5000, [100, 1, 28]), (32, 64, 32, 264, [129]), (16, 128, 16, 264, [128]), (32, 128, 8, 264, [64]), (32, 128, 8, 264, [40, 25]),
+                                                           (8, 64, 8, 1376, [511]), (8, 64, 2, 1376, [500, 12])])
+def test_prompts(heads, hs, kv_heads, hidden, lens):
+    """Both sides of the rule by rows and width, two layers, behind a context."""
+    eng, ck = load_pkg("engine"), load_pkg("checkpoint")
+    cfg = ck.Config(heads * hs, hidden, 2, heads, kv_heads, 96, 540)
+    w = eng.device_random_weights(cfg, seed=2, std=cfg.dim ** -0.5)
+    e = eng.Engine(w, len(lens), with_att=False)
+    rng = np.random.default_rng(3)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    e.state.key_cache.normal_(0.0, 1.0, generator=g)
+    e.state.value_cache.normal_(0.0, 1.0, generator=g)
+    seqs = [(i, 7, rng.integers(0, 96, n).astype(np.int32)) for i, n in enumerate(lens)]
+    keys = e.state.key_cache.clone()
+    values = e.state.value_cache.clone()
+    got = torch.empty(len(seqs), 96, device="cuda")
+    torch.cuda.synchronize()
+    e.prefill(seqs, got)
+    torch.cuda.synchronize()
+    want, k, v = llama64.forward(cfg, w.t, lambda c, s, l, n: (keys if c == "k" else values)[s, l, :n], seqs)
+    rel = lambda a, b: float((a.double() - b.double()).norm() / b.double().norm())
+    assert rel(got, want) < 5e-5                    # as test_fp32_rows
+    at = 0
+    for i, n in enumerate(lens):
+        assert rel(e.state.key_cache[i, :, 7:7 + n], k[at:at + n].transpose(0, 1)) < 3e-5
+        assert rel(e.state.value_cache[i, :, 7:7 + n], v[at:at + n].transpose(0, 1)) < 3e-5
+        at += n
