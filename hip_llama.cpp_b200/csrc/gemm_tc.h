@@ -47,6 +47,10 @@ int x3_norm_launch(cudaStream_t st, bool pdl, int rows, const X3RowsP& p);
 int x3_swiglu_launch(cudaStream_t st, bool pdl, int rows, const X3RowsP& p);
 int x3_split_launch(cudaStream_t st, bool pdl, int rows, const X3RowsP& p);
 
+// What the attention of such prompts reads (attn_prefill_x3.cu): q [rows][dim], k / v [rows staged][kv_dim] as planes, inverse scales [rows][heads] and
+// [kv head][rows staged].  row: the staged row of every row; pad: staged rows behind it that are zeroed in v (non-zero for a sequence's last row only).
+struct X3Staged { uint16_t *qh, *ql, *kh, *kl, *vh, *vl; float *qs, *ks, *vs; const int *row, *pad; int rows; };
+
 // Q8_0 weights x Q8_0 activations on the int8 tensor cores (gemm_q8i_kernel)
 struct Q8iArgs {
   int n_mats; const int8_t* Wq[3]; const float* Ws[3]; int M[3]; int out_off[3];

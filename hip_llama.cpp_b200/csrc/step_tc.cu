@@ -54,6 +54,13 @@ int attn_prefill_launch(cudaStream_t stream, int n_tiles, int n_heads, int n_kv_
                         long long kv_batch_stride, const int* row_slot, const int* row_pos, const int* tile_row0,
                         const int* tile_n, bool pdl, const KvPaged* pg, int tile_rows);
 int attn_prefill_tile_rows(int rows, int n_seqs, int tiles128, int heads);
+bool attn_prefill_x3_supported(int head_size);
+int x3_rope_launch(cudaStream_t st, bool pdl, int R, const float* part, int nz, long long zstride, int ld, const int* pos, int d, int kvd, int hs, const float* rc,
+                   const float* rs, float* kc, float* vc, long long kv_bs, int loff, const int* slot, const KvPaged& pg, const X3Staged& staged);
+int x3_context_launch(cudaStream_t st, bool pdl, int n_seqs, int longest, const float* kc, const float* vc, long long kv_bs, const int* seq_slot, const int* upto,
+                      const int* base, const KvPaged& pg, int kvd, int hs, const X3Staged& staged);
+int attn_prefill_x3_launch(cudaStream_t st, bool pdl, int n_tiles, int rows, int n_heads, int n_kv_heads, int head_size, float* out, const int* row_pos,
+                           const int* tile_row0, const int* tile_n, const X3Staged& s);
 
 __device__ __forceinline__ float st_tf32(float v) { return __uint_as_float((__float_as_uint(v) + 0x1000u) & 0xFFFFE000u); }
 
@@ -555,7 +562,8 @@ struct TcScratch {
   float *ah = nullptr, *al = nullptr, *ss = nullptr; int* ctr = nullptr;
   size_t n_ah = 0, n_al = 0, n_ss = 0; int ctr_stride = 0, n_ctr_blocks = 0;
   float* scale2 = nullptr;                              // fp16 planes: scales of the rows that are not norms (gemm_f16x3.cu)
-  size_t n_scale2 = 0;
+  float* stage = nullptr;                               // ... k and v planes and inverse scales (attn_prefill_x3.cu)
+  size_t n_scale2 = 0, n_stage = 0;
   size_t n_x = 0, n_xl = 0, n_h = 0, n_hl = 0, n_part = 0, n_xr = 0, n_qr = 0, n_xbr = 0, n_tab = 0; int n_b = 0;
 };
 static std::map<Workspace*, TcScratch> g_tc_scratch;   // per workspace (= per device, or per tensor-parallel rank)
@@ -566,7 +574,7 @@ void step_tc_release(Workspace* ws) {
   auto it = g_tc_scratch.find(ws);
   if (it == g_tc_scratch.end()) return;
   TcScratch& s = it->second;
-  void* ptrs[] = {s.xh, s.xl, s.hh, s.hl, s.scale, s.part, s.xr, s.qr, s.xbr, s.tab, s.xq, s.hq, s.xsT, s.hsT, s.ah, s.al, s.ss, s.ctr, s.scale2};
+  void* ptrs[] = {s.xh, s.xl, s.hh, s.hl, s.scale, s.part, s.xr, s.qr, s.xbr, s.tab, s.xq, s.hq, s.xsT, s.hsT, s.ah, s.al, s.ss, s.ctr, s.scale2, s.stage};
   for (void* p : ptrs) if (p) cudaFree(p);
   g_tc_scratch.erase(it);
 }
@@ -702,7 +710,7 @@ static void chain_needs(const tha_config_t& c, int R, size_t* part_floats, size_
 
 // Allocate / grow everything R rows need (never inside a stream capture).
 static int prepare_rows(Workspace* ws, const tha_config_t* c, int R, bool prefill, int n_tab, bool q8, int gs = 64,
-                        const TpCtx* tp = nullptr) {
+                        const TpCtx* tp = nullptr, int n_out = 0) {
   THA_TRY_RC(gemm_tc_init(nullptr));
   std::lock_guard<std::mutex> lk(g_tc_scratch_mu);
   TcScratch& s = g_tc_scratch[ws];
@@ -717,10 +725,12 @@ static int prepare_rows(Workspace* ws, const tha_config_t* c, int R, bool prefil
     THA_TRY_RC(grow(&s.xsT, &s.n_xsT, ldxs * (c->dim / 32), ws));
     THA_TRY_RC(grow(&s.hsT, &s.n_hsT, ldxs * (c->hidden_dim / 32), ws));
   } else {
-    THA_TRY_RC(grow(&s.xh, &s.n_x, (size_t)R * c->dim, ws));
-    THA_TRY_RC(grow(&s.xl, &s.n_xl, (size_t)R * c->dim, ws));
-    THA_TRY_RC(grow(&s.hh, &s.n_h, (size_t)R * c->hidden_dim, ws));
-    THA_TRY_RC(grow(&s.hl, &s.n_hl, (size_t)R * c->hidden_dim, ws));
+    const int per = f16x3 ? 2 : 1;   // planes of two bytes a value (the classifier's few rows are of four)
+    const size_t out_rows = f16x3 ? (size_t)n_out : 0;
+    THA_TRY_RC(grow(&s.xh, &s.n_x, std::max((size_t)R / per + 1, out_rows) * c->dim, ws));
+    THA_TRY_RC(grow(&s.xl, &s.n_xl, std::max((size_t)R / per + 1, out_rows) * c->dim, ws));
+    THA_TRY_RC(grow(&s.hh, &s.n_h, ((size_t)R / per + 1) * c->hidden_dim, ws));
+    THA_TRY_RC(grow(&s.hl, &s.n_hl, ((size_t)R / per + 1) * c->hidden_dim, ws));
   }
   size_t part_need = pl.part_floats;
   if (!q8 && !prefill && !tp && chain_mode() != 0) {   // the chained step (chain_tc.cu)
@@ -808,6 +818,8 @@ struct RowsIO {
   const int *token, *pos, *slot;           // [R]; slot == nullptr: row r lives in cache slab r (decode)
   int n_tiles; const int *tile_row0, *tile_n;   // prefill attention tiles (n_tiles == 0: per-row decode attention)
   int tile_rows;                           // query rows per tile at most (64 or 128)
+  const X3Staged* staged;                  // fp32 prompts whose attention runs on the tensor cores
+  int n_ctx, longest_ctx; const int *seq_slot, *seq_upto, *seq_base;   // ... and their contexts (n_ctx == 0: none)
   int n_out; const int* out_rows;          // classifier rows (out_rows == nullptr: every row)
   float* logits; int* next;                // [n_out, vocab] (nullable: skip the classifier), [n_out] (nullable)
 };
@@ -1067,7 +1079,12 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
     // decode rows: RoPE + KV scatter ride in the attention kernel (one launch and one dependency less per layer)
     const bool rope_in_attn = io.n_tiles == 0 && !(!io.logits && l == L - 1) && !(skip & 2) && rope_fuse_mode() &&
                               attn_fused_rope_supported(c.n_heads, c.n_kv_heads, hs);
-    if (!(skip & 8) && !rope_in_attn)
+    if (io.staged && !(skip & 8)) {
+      if (io.n_ctx)
+        THA_TRY_RC(x3_context_launch(st, pdl, io.n_ctx, io.longest_ctx, kcl, vcl, kv_bs, io.seq_slot, io.seq_upto, io.seq_base, pg, kvd, hs, *io.staged));
+      THA_TRY_RC(x3_rope_launch(st, pdl, R, sc.part, pl.z_qkv, (long long)R * ld_qkv, ld_qkv, io.pos, da, kvd, hs, rc, rs, s.key_cache, s.value_cache, kv_bs, loff, io.slot,
+                                pg, *io.staged));
+    } else if (!(skip & 8) && !rope_in_attn)
     THA_CUDA_OK(launch(tc_rope_scatter_kernel, dim3(ceil_div(ld_qkv / 4, 512), R), dim3(256), 0, st, pdl, (const float*)sc.part,
                        pl.z_qkv, (long long)R * ld_qkv, ld_qkv, io.pos, da, kvd, hs, rc, rs, io.q, s.key_cache, s.value_cache,
                        kv_bs, loff, io.slot, pg, RopeBf16{}));
@@ -1076,6 +1093,8 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
       return THA_STATUS_SUCCESS;
     }
     if (skip & 2) {
+    } else if (io.staged) {
+      THA_TRY_RC(attn_prefill_x3_launch(st, pdl, io.n_tiles, R, c.n_heads, c.n_kv_heads, hs, io.xb, io.pos, io.tile_row0, io.tile_n, *io.staged));
     } else if (io.n_tiles > 0) {
       THA_TRY_RC(attn_prefill_launch(st, io.n_tiles, c.n_heads, c.n_kv_heads, hs, io.q, io.xb, wq || f16x3 ? nullptr : sc.xh,
                                      wq || f16x3 ? nullptr : sc.xl, kcl, vcl, kv_bs, io.slot, io.pos,
@@ -1189,28 +1208,62 @@ int step_tc_prefill(cudaStream_t st, Workspace* ws, const tha_config_t& c, const
     R += len[i];
   }
   if (R < 1 || R > (1 << 20)) return THA_STATUS_INVALID_ARG;
-  int tiles128 = 0;
-  for (int i = 0; i < n_seqs; i++) tiles128 += ceil_div(len[i], 128);
-  const int TQ = attn_prefill_tile_rows((int)R, n_seqs, tiles128, c.n_heads);
+  for (long long i = 0; i < R; i++)
+    if (tokens[i] < 0 || tokens[i] >= c.vocab_size) return THA_STATUS_INVALID_ARG;
+  int tiles128 = 0, longest_ctx = 0;
+  long long ctx = 0, Rs = 0;   // rows of contexts; staged rows: a sequence's positions from 0 on, at a multiple of 128
+  for (int i = 0; i < n_seqs; i++) {
+    tiles128 += ceil_div(len[i], 128);
+    ctx += pos0[i];
+    longest_ctx = std::max(longest_ctx, pos0[i]);
+    Rs += (long long)ceil_div(pos0[i] + len[i], 128) * 128;
+  }
+  const Dims dm = dims_of(c, tp);
+  const int G = c.n_kv_heads;
+  // Attention of fp32 prompts on the tensor cores, whose tiles are of 128 rows and keys and whose keys are staged as planes, contexts too.  us a prompt without /
+  // with, Llama-2-7B's width (2 layers): 16 sequences of 5 rows 660 / 695, of 33 1614 / 1660, 3 of 30 586 / 595, one of 100 596 / 580, of 512 1412 / 1322; behind a
+  // context of 200, 16 of 10 rows 1034 / 943, 4 of 100 1506 / 1318; 100 rows behind 800 867 / 754.  768 wide (12 layers), 8 of 65 1269 / 1238, one of 520 1953 / 1473,
+  // behind 800 3386 / 1872.  Contexts are staged up to 20 times the call's rows and, past 256 MB, up to as many as these.
+  bool x3 = rows_f16x3(dm, (int)R, true, wq != nullptr, tp != nullptr) && attn_prefill_x3_supported(dm.hs) && R + ctx >= 64ll * n_seqs && ctx <= 20 * R &&
+            (ctx <= R || 8ll * dm.kvd * Rs <= 256ll << 20);
   struct Tile { int row0, n, last; };   // `last`: last position the tile's rows see
   std::vector<Tile> tiles;
-  for (int i = 0, r0 = 0; i < n_seqs; r0 += len[i], i++)
-    for (int j = 0; j < len[i]; j += TQ) { const int n = (len[i] - j < TQ) ? len[i] - j : TQ; tiles.push_back({r0 + j, n, pos0[i] + j + n - 1}); }
-  std::stable_sort(tiles.begin(), tiles.end(), [](const Tile& x, const Tile& y) { return x.last > y.last; });   // the longest start first
-  T = (long long)tiles.size();
-  // tables: [slot R | pos R | token R | tile_row0 T | tile_n T | last n_seqs]
-  std::vector<int> tab((size_t)3 * R + 2 * T + n_seqs);
+  std::vector<int> tab;
+  int TQ = 0, rc_rows = 0;
+  for (;;) {
+    TQ = x3 ? 128 : attn_prefill_tile_rows((int)R, n_seqs, tiles128, c.n_heads);
+    tiles.clear();
+    for (int i = 0, r0 = 0; i < n_seqs; r0 += len[i], i++)
+      for (int j = 0; j < len[i]; j += TQ) { const int n = (len[i] - j < TQ) ? len[i] - j : TQ; tiles.push_back({r0 + j, n, pos0[i] + j + n - 1}); }
+    std::stable_sort(tiles.begin(), tiles.end(), [](const Tile& x, const Tile& y) { return x.last > y.last; });   // the longest start first
+    T = (long long)tiles.size();
+    // tables: [slot R | pos R | token R | tile_row0 T | tile_n T | last n_seqs], then [staged row R | pad R | slot, upto, base n_seqs]
+    tab.assign((size_t)3 * R + 2 * T + n_seqs + (x3 ? 2 * R + 3 * n_seqs : 0), 0);
+    rc_rows = prepare_rows(ws, &c, (int)R, true, (int)tab.size(), wq != nullptr, wq ? wq->group_size : 64, tp, n_seqs);
+    if (!x3) break;
+    std::lock_guard<std::mutex> lk(g_tc_scratch_mu);
+    TcScratch& s2 = g_tc_scratch[ws];
+    const size_t need = (size_t)2 * Rs * dm.kvd + (size_t)R * c.n_heads + (size_t)2 * G * Rs;
+    if (rc_rows == THA_STATUS_SUCCESS && grow(&s2.stage, &s2.n_stage, need, ws) == THA_STATUS_SUCCESS) break;
+    // no room for the planes: the attention that needs none
+    cudaFree(s2.stage);
+    s2.stage = nullptr; s2.n_stage = 0;
+    x3 = false;
+  }
+  THA_TRY_RC(rc_rows);
   int *h_slot = tab.data(), *h_pos = h_slot + R, *h_tok = h_pos + R, *h_t0 = h_tok + R, *h_tn = h_t0 + T, *h_last = h_tn + T;
+  int *h_stage = h_last + n_seqs, *h_pad = h_stage + R, *h_sslot = h_pad + R, *h_upto = h_sslot + n_seqs, *h_base = h_upto + n_seqs;
   for (long long t = 0; t < T; t++) { h_t0[t] = tiles[t].row0; h_tn[t] = tiles[t].n; }
-  int r = 0;
+  int r = 0, at = 0;
   for (int i = 0; i < n_seqs; i++) {
+    const int end = pos0[i] + len[i];
     for (int j = 0; j < len[i]; j++, r++) {
       h_slot[r] = slot[i]; h_pos[r] = pos0[i] + j; h_tok[r] = tokens[r];
-      if (tokens[r] < 0 || tokens[r] >= c.vocab_size) return THA_STATUS_INVALID_ARG;
+      if (x3) { h_stage[r] = at + pos0[i] + j; h_pad[r] = j + 1 < len[i] ? 0 : -end & 15; }
     }
     h_last[i] = r - 1;
+    if (x3) { h_sslot[i] = slot[i]; h_upto[i] = pos0[i]; h_base[i] = at; at += ceil_div(end, 128) * 128; }
   }
-  THA_TRY_RC(prepare_rows(ws, &c, (int)R, true, (int)tab.size(), wq != nullptr, wq ? wq->group_size : 64, tp));
   TcScratch sc;
   {
     std::lock_guard<std::mutex> lk(g_tc_scratch_mu);
@@ -1223,6 +1276,17 @@ int step_tc_prefill(cudaStream_t st, Workspace* ws, const tha_config_t& c, const
   io.slot = sc.tab; io.pos = sc.tab + R; io.token = sc.tab + 2 * R;
   io.n_tiles = (int)T; io.tile_rows = TQ; io.tile_row0 = sc.tab + 3 * R; io.tile_n = sc.tab + 3 * R + T;
   io.n_out = n_seqs; io.out_rows = sc.tab + 3 * R + 2 * T; io.logits = logits; io.next = logits ? next_d : nullptr;
+  X3Staged g = {};
+  if (x3) {
+    const size_t plane = (size_t)Rs * dm.kvd;
+    g.qh = reinterpret_cast<uint16_t*>(sc.qr); g.ql = g.qh + (size_t)R * dm.da;
+    g.kh = reinterpret_cast<uint16_t*>(sc.stage); g.kl = g.kh + plane; g.vh = g.kl + plane; g.vl = g.vh + plane;
+    g.ks = sc.stage + 2 * plane; g.vs = g.ks + (size_t)G * Rs; g.qs = g.vs + (size_t)G * Rs;
+    g.row = io.out_rows + n_seqs; g.pad = g.row + R; g.rows = (int)Rs;
+    io.staged = &g;
+    io.n_ctx = ctx ? n_seqs : 0; io.longest_ctx = longest_ctx;
+    io.seq_slot = g.pad + R; io.seq_upto = io.seq_slot + n_seqs; io.seq_base = io.seq_upto + n_seqs;
+  }
   return issue_rows(st, ws, c, w, wq, s, io, rc, rs, pdl_enabled() != 0, tp);
 }
 

@@ -105,3 +105,39 @@ def test_prompts(heads, hs, kv_heads, hidden, lens):
         assert rel(e.state.key_cache[i, :, 7:7 + n], k[at:at + n].transpose(0, 1)) < 3e-5
         assert rel(e.state.value_cache[i, :, 7:7 + n], v[at:at + n].transpose(0, 1)) < 3e-5
         at += n
+
+
+@pytest.mark.parametrize("heads,hs,kv_heads", [(16, 128, 16), (16, 128, 4), (32, 64, 32), (32, 64, 8)])
+@pytest.mark.parametrize("pos0,lens,paged", [(0, [128, 1, 100], False), (1, [127, 129], False), (127, [130], True), (128, [16, 64, 60], True), (0, [257, 15], True), (300, [20, 130], False)])
+def test_prompt_attention(heads, hs, kv_heads, pos0, lens, paged):
+    """Prompt attention on the tensor cores (csrc/attn_prefill_x3.cu): tiles of 128 rows and keys, portions behind contexts, block tables; keys and values of very
+    different sizes, so that each has a scale of its own."""
+    eng, ck = load_pkg("engine"), load_pkg("checkpoint")
+    cfg = ck.Config(heads * hs, 264, 1, heads, kv_heads, 96, 512)
+    w = eng.device_random_weights(cfg, seed=2, std=cfg.dim ** -0.5)
+    pages = None
+    if paged:
+        per = 512 // 16
+        pages = eng.PagedKV(cfg, len(lens), per * len(lens), 16)
+        pages.set_table(np.random.default_rng(6).permutation(per * len(lens)).astype(np.int32).reshape(len(lens), per))
+    e = eng.Engine(w, len(lens), with_att=False, paged=pages)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    for cache in (e.state.key_cache, e.state.value_cache):
+        cache.normal_(0.0, 1.0, generator=g)
+        cache.mul_(torch.exp2(torch.randint(-12, 2, cache.shape[:-1], device="cuda", generator=g).float())[..., None])
+    rng = np.random.default_rng(3)
+    seqs = [(i, pos0, rng.integers(0, 96, n).astype(np.int32)) for i, n in enumerate(lens)]
+    kept = {"k": e.state.key_cache.clone(), "v": e.state.value_cache.clone()}
+
+    def rows(c, s, l, n):
+        if not paged:
+            return kept[c][s, l, :n]
+        return kept[c][pages.table[s].long(), l].reshape(-1, kept[c].shape[-1])[:n]
+
+    got = torch.empty(len(seqs), 96, device="cuda")
+    torch.cuda.synchronize()
+    e.prefill(seqs, got)
+    torch.cuda.synchronize()
+    want, _, _ = llama64.forward(cfg, w.t, rows, seqs)
+    # sums of 32 to 2048 terms at 1e-6 to 2e-6 each (test_product), through three products and the attention one after the other
+    assert float((got.double() - want).norm() / want.norm()) < 1e-5
