@@ -346,6 +346,93 @@ __global__ void hyb_attn_prepare_kernel(tha_attn_t a, tha_rows_t rows, tha_kv_t 
   }
 }
 
+// The same for heads of up to 128 channels whose places are multiples of four floats (hyb_attn_prepare_ok): a lane has four neighbouring channels, 128-bit loads and stores.
+// Where a row's cache line lies -- three dependent loads -- is looked up ahead of the wait for the projections inside tha_hyb_step (`early`), where rows and table are
+// in place before the step's first kernel starts.  Bound by bytes for prompts, by the chain of loads when decoding.
+__device__ __forceinline__ float4 hyb_scale4(float4 v, float f) { return make_float4(v.x * f, v.y * f, v.z * f, v.w * f); }
+__device__ __forceinline__ float4 hyb_ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+template <int THREADS>   // at most
+__global__ void __launch_bounds__(THREADS, 1280 / THREADS) hyb_attn_prepare4_kernel(tha_attn_t a, tha_rows_t rows, tha_kv_t kv, const float* __restrict__ proj, long long ldp,
+                                                                 const float* __restrict__ cos_t, const float* __restrict__ sin_t, int rot_dims,
+                                                                 float* __restrict__ q_out, int early) {
+  pdl_trigger();
+  if (!early) pdl_wait();
+  const int r = blockIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5, c = 4 * lane;
+  const int t = rows.pos[r], slot = rows.seq_slot[rows.row_seq[r]];
+  const size_t krow = hyb_kv_row(kv, slot, t, a.cache_layer);
+  const size_t mrow = a.v_mix ? hyb_kv_row(kv, slot, t, a.v_mix_layer) : 0;
+  if (early) pdl_wait();
+  const float* pr = proj + (size_t)r * ldp;
+  const int half = rot_dims / 2;
+  const int n_k = a.kv_shared ? 0 : a.kv_heads, n_v = a.kv_shared ? 0 : a.kv_heads / (a.v_share > 1 ? a.v_share : 1);
+  const float q_mult = a.q_temp_every > 0 ? 1.0f + a.q_temp_coef * logf((float)((t + 1) / a.q_temp_every + 1)) : 1.0f;
+  float row_q = 1.0f, row_k = 1.0f;
+  if (!a.head_norm && (a.q_norm || a.k_norm)) {
+    __shared__ float red[33];
+    if (a.q_norm) {
+      float ss = 0.f;
+      for (int i = 4 * threadIdx.x; i < a.heads * a.dim; i += 4 * blockDim.x) { const float4 v = hyb_ld4(pr + a.o_q + i); ss = dot4(v, v, ss); }
+      row_q = 1.0f / sqrtf(block_sum(ss, red) / (float)(a.heads * a.dim) + a.eps);
+    }
+    if (a.k_norm && n_k) {
+      float ss = 0.f;
+      for (int i = 4 * threadIdx.x; i < a.kv_heads * a.dim; i += 4 * blockDim.x) { const float4 v = hyb_ld4(pr + a.o_k + i); ss = dot4(v, v, ss); }
+      row_k = 1.0f / sqrtf(block_sum(ss, red) / (float)(a.kv_heads * a.dim) + a.eps);
+    }
+  }
+  for (int h = warp; h < a.heads + n_k + n_v; h += nwarps) {
+    if (h >= a.heads + n_k) {   // a value head: plain copy, or blended with an earlier layer's values of the token
+      if (c >= a.vdim) continue;
+      const int g = h - a.heads - n_k;
+      float4 v = hyb_ld4(pr + a.o_v + g * a.vdim + c);
+      if (a.v_mix) {
+        const float4 first = hyb_ld4(kv.v_pool + mrow + (size_t)g * a.vdim + c);
+        const float lam = a.v_mix_lambda, rest = 1.0f - lam;
+        v = make_float4(fmaf(lam, first.x, rest * v.x), fmaf(lam, first.y, rest * v.y), fmaf(lam, first.z, rest * v.z), fmaf(lam, first.w, rest * v.w));
+      }
+      *reinterpret_cast<float4*>(kv.v_pool + krow + (size_t)g * a.vdim + c) = v;
+      continue;
+    }
+    const bool is_q = h < a.heads, in = c < a.dim, turn = c < rot_dims;
+    const float* src = pr + (is_q ? a.o_q + h * a.dim : a.o_k + (h - a.heads) * a.dim);
+    float* dst = is_q ? q_out + (size_t)r * a.heads * a.dim + (size_t)h * a.dim : kv.k_pool + krow + (size_t)(h - a.heads) * a.dim;
+    const float* wn = is_q ? a.q_norm : a.k_norm;   // per-channel weights sit inside the rotation, the row's factor outside
+    if (wn && !a.head_norm) wn += is_q ? h * a.dim : (h - a.heads) * a.dim;
+    const bool halves = a.rot_layout == THA_ROT_HALVES, first = c < half;
+    const int pc = halves && turn ? (first ? c + half : c - half) : c;     // where the partners of these channels lie
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
+    if (in) { x = hyb_ld4(src + c); y = hyb_ld4(src + pc); }
+    float ss = dot4(x, x, 0.f);
+    if (in && wn) {
+      const float4 wx = make_float4(wn[c], wn[c + 1], wn[c + 2], wn[c + 3]), wy = make_float4(wn[pc], wn[pc + 1], wn[pc + 2], wn[pc + 3]);
+      x = make_float4(x.x * wx.x, x.y * wx.y, x.z * wx.z, x.w * wx.w);
+      y = make_float4(y.x * wy.x, y.y * wy.y, y.z * wy.z, y.w * wy.w);
+    }
+    float4 v = x;
+    if (turn) {
+      const float *cr = cos_t + (size_t)r * half, *sr = sin_t + (size_t)r * half;
+      if (halves) {
+        const int i = first ? c : c - half;
+        const float s = first ? -1.0f : 1.0f;
+        v = make_float4(x.x * cr[i] + s * (y.x * sr[i]), x.y * cr[i + 1] + s * (y.y * sr[i + 1]), x.z * cr[i + 2] + s * (y.z * sr[i + 2]), x.w * cr[i + 3] + s * (y.w * sr[i + 3]));
+      } else {
+        const int i = c >> 1;
+        v = make_float4(x.x * cr[i] - x.y * sr[i], x.y * cr[i] + x.x * sr[i], x.z * cr[i + 1] - x.w * sr[i + 1], x.w * cr[i + 1] + x.z * sr[i + 1]);
+      }
+    }
+    if (a.unit_rms && !a.head_norm) ss = dot4(v, v, 0.f);
+    float inv = is_q ? q_mult * row_q : row_k;
+    if (a.unit_rms || a.head_norm) inv = 1.0f / sqrtf(warp_sum(ss) / (float)a.dim + a.eps) * inv;
+    if (in) *reinterpret_cast<float4*>(dst + c) = hyb_scale4(v, inv);
+  }
+}
+static bool hyb_attn_prepare_ok(const tha_attn_t* a, const tha_kv_t* kv, const float* proj, long long ldp, int rot_dims, const float* q_out) {
+  return a->dim <= 128 && a->vdim <= 128 && a->dim % 4 == 0 && a->vdim % 4 == 0 && rot_dims % (a->rot_layout == THA_ROT_HALVES ? 8 : 4) == 0 && ldp % 4 == 0 &&
+         a->o_q % 4 == 0 && a->o_k % 4 == 0 && a->o_v % 4 == 0 && kv->kv_dim % 4 == 0 && aligned16(proj) && aligned16(q_out) && aligned16(kv->k_pool) &&
+         aligned16(kv->v_pool);
+}
+
 // ------------------------------------------------------------------------------------------------------------------
 // attention, prompts and decoding alike.  A block takes 16 (position, query head) pairs that share one key/value head:
 // AP consecutive positions of one sequence x AG heads of the group (AG = min(group size, 16), AP = 16 / AG), so a key
@@ -1802,6 +1889,14 @@ extern "C" int tha_hyb_attn_prepare(void* stream, const tha_attn_t* a, const tha
   if (a->heads % a->kv_heads || rot_dims > a->dim || (rot_dims & 1) || a->kv_heads * a->dim > kv->kv_dim ||
       a->kv_heads / (a->v_share > 1 ? a->v_share : 1) * a->vdim > kv->kv_dim || (a->v_is_k && a->vdim != a->dim))
     return THA_STATUS_INVALID_ARG;
+  if (hyb_attn_prepare_ok(a, kv, proj, ldp, rot_dims, q_out)) {
+    // a warp a head where rows are few (a decode step's 6.5 -> 2.2 us), blocks of eight warps for portions, several an SM (4000 rows of 3072 columns 46 -> 31 us)
+    const bool few = rows->n_rows <= 148;
+    const int warps = a->heads + 2 * a->kv_heads, most = few ? 32 : 8;
+    THA_CUDA_OK(launch(few ? hyb_attn_prepare4_kernel<1024> : hyb_attn_prepare4_kernel<256>, dim3(rows->n_rows), dim3(32 * (warps < most ? warps : most)), 0,
+                       (cudaStream_t)stream, pdl_enabled() != 0, *a, *rows, *kv, proj, ldp, cos_t, sin_t, rot_dims, q_out, (int)hyb_gemm_pdl()));
+    return THA_STATUS_SUCCESS;
+  }
   const int nt = pick_threads(32 * (a->heads + 2 * a->kv_heads));
   THA_CUDA_OK(launch(hyb_attn_prepare_kernel, dim3(rows->n_rows), dim3(nt), 0, (cudaStream_t)stream, pdl_enabled() != 0, *a, *rows, *kv, proj, ldp, cos_t,
                      sin_t, rot_dims, q_out));
