@@ -23,6 +23,7 @@
 #include <stdlib.h>
 
 #include "gemm_tc.h"
+#include "hybrid_ops.cuh"
 #include "tc_common.cuh"
 
 namespace tha {
@@ -38,8 +39,11 @@ struct BfP {
   const float* colscale;
   int* error_flag;
   int splits, n_items;
-  uint16_t* swiglu_out; long long ld_swiglu;   // SWIGLU kernels
+  uint16_t* act_out; long long ld_act;         // kernels with an activation in the read-out
+  int act; float act_limit, act_alpha;         // BF_GATED, BF_UNGATED: THA_ACT_*
 };
+// what a work item's read-out does with its accumulators
+enum { BF_PLAIN = 0, BF_SWIGLU = 1, BF_GATED = 2, BF_UNGATED = 3 };
 
 // MT = weight tiles of 128 rows per work item.  MT = 2 (prompt-sized N only): a CTA multiplies 256 weight rows by the
 // same 256 activation columns -- per 64-value k-block it pulls 32 + 32 KB through L2 for twice the flops of the 16 + 32 KB
@@ -70,14 +74,37 @@ __device__ __forceinline__ void bf_mma(uint32_t tmem_d, uint64_t adesc, uint64_t
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
-// SWIGLU (MT = 2): the two 128-row halves of a work item are the SAME rows of two matrices (mw0 = w1, mw1 = w3); the read-out
-// combines the two accumulators of a row into silu(a) * c (run.cc:344-347 order) and stores it as bf16.
-template <int NT, int MT = 1, bool SWIGLU = false>
+// Sixteen columns of a row through an activation (THA_ACT_*) and out as bf16: the branch on the activation is taken once per sixteen.
+template <int ACT>
+__device__ __forceinline__ void bf_act16_of(const uint32_t (&vg)[16], const uint32_t (&vu)[16], float limit, float alpha, __nv_bfloat16* o, long long ld, int n) {
+#pragma unroll
+  for (int j = 0; j < 16; j++) {
+    if (j < n) hyb_store(o, hyb_act_value(ACT, __uint_as_float(vg[j]), __uint_as_float(vu[j]), limit, alpha));
+    o += ld;
+  }
+}
+template <bool GATED>
+__device__ __forceinline__ void bf_act16(int act, const uint32_t (&vg)[16], const uint32_t (&vu)[16], float limit, float alpha, __nv_bfloat16* o,
+                                         long long ld, int n) {
+  if (!GATED) bf_act16_of<THA_ACT_RELU2>(vg, vu, limit, alpha, o, ld, n);
+  else if (act == THA_ACT_SILU_GLU) bf_act16_of<THA_ACT_SILU_GLU>(vg, vu, limit, alpha, o, ld, n);
+  else if (act == THA_ACT_GELU_TANH_GLU) bf_act16_of<THA_ACT_GELU_TANH_GLU>(vg, vu, limit, alpha, o, ld, n);
+  else bf_act16_of<THA_ACT_GLU_CLAMPED>(vg, vu, limit, alpha, o, ld, n);
+}
+
+// BF_SWIGLU, BF_GATED (MT = 2): the two 128-row halves of a work item are the SAME rows of two matrices (mw0 = w1, mw1 = w3); the
+// read-out combines the two accumulators of a row into silu(a) * c (run.cc:344-347 order) or a layer program's gated activation and
+// stores it as bf16.  BF_UNGATED: the tiles of BF_PLAIN, an activation of the accumulator stored as bf16.
+// A pair's tile has 128 columns: its two accumulators leave room for a second pair, so the read-out (an exponential and a division per
+// element) runs behind the next item's products.  256 columns pull a quarter less through L2 but nothing hides their read-out: 4000 rows x
+// [2 x 6144, 2048] 234 us against 154, 2825 x [2 x 11008, 4096] 499 against 385; two prompts of a 7B bf16 model 2.64 -> 2.59 ms.
+template <int NT, int MT = 1, int READ = BF_PLAIN>
 __global__ void __launch_bounds__(128 + 128 * MT, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant__ CUtensorMap mw1,
                  const __grid_constant__ CUtensorMap mw2, const __grid_constant__ CUtensorMap mx, const BfP p) {
   using S = BfSmem<NT, MT>;
   constexpr int NBUF = S::NBUF;
+  constexpr bool PAIR = READ == BF_SWIGLU || READ == BF_GATED;
   extern __shared__ unsigned char tc_smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::NST * S::STAGE);
@@ -98,7 +125,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant_
     w.n0 = (t - tile * p.ny) * NT;
     w.mat = 0;
     while (w.mat + 1 < p.n_mats && tile >= p.tiles[w.mat]) { tile -= p.tiles[w.mat]; w.mat++; }
-    w.row0 = tile * (SWIGLU ? TC_BM : TC_BM * MT);
+    w.row0 = tile * (PAIR ? TC_BM : TC_BM * MT);
     w.wrow = p.w_row[w.mat] + w.row0;   // where the tile lies in its tensor maps
     w.xrow = p.x_row[w.mat] + w.n0;
     w.kb0 = z * p.kblocks_per_split;
@@ -138,7 +165,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant_
       int gb = 0;
       bool ok = true, first = true;
       auto load_w = [&](unsigned char* dst, const CUtensorMap* mw, int kcol, int row0, uint64_t* bar) {
-        if (SWIGLU) {   // 128 rows of w1, then the same 128 rows of w3
+        if (PAIR) {   // 128 rows of w1, then the same 128 rows of w3
           tc_tma_2d(dst, &mw0, kcol, row0, bar);
           tc_tma_2d(dst + TC_BM * 128, &mw1, kcol, row0, bar);
         } else if (stream_w) tc_tma_2d_hint(dst, mw, kcol, row0, bar, pol_w);
@@ -214,12 +241,35 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant_
       const int buf = n_it % NBUF, use = n_it / NBUF;
       if (ok) ok = tc_mbar_wait(&accum[buf], (unsigned)(use & 1), abort_flag);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (SWIGLU) {
+      if (READ == BF_GATED || READ == BF_UNGATED) {
+        // the row's accumulators (gate and up, or one) through the activation; warps 4-7 and 8-11 share the columns of a pair
+        const int arow = w.row0 + (PAIR ? 0 : mt * TC_BM) + r;
+        constexpr int C1 = PAIR ? NT / 2 : NT;
+        const int c0 = PAIR ? mt * C1 : 0;
+        const uint32_t ta = tmem_base + (uint32_t)(buf * MT * NT + (PAIR ? 0 : mt * NT)) + ((uint32_t)(q * 32) << 16);
+        __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.act_out) + (size_t)(w.n0 + c0) * p.ld_act + arow;
+        const int left = arow < p.M[0] ? p.N - w.n0 - c0 : 0;   // columns of this thread's row that are stored
+        if (ok) {
+#pragma unroll 1
+          for (int c = 0; c < C1; c += 16, o += 16 * p.ld_act) {
+            uint32_t vg[16], vu[16];
+            tc_tmem_ld16(ta + (uint32_t)(c0 + c), vg);
+            if (PAIR) tc_tmem_ld16(ta + (uint32_t)(NT + c0 + c), vu);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            bf_act16<PAIR>(p.act, vg, PAIR ? vu : vg, p.act_limit, p.act_alpha, o, p.ld_act, left - c);
+          }
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) tc_mbar_arrive(&accfree[buf]);
+        continue;
+      }
+      if (READ == BF_SWIGLU) {
         // both accumulators of this thread's row; warps 4-7 take the first half of the columns, 8-11 the second
         const int srow = w.row0 + r;
         const uint32_t ta = tmem_base + (uint32_t)(buf * MT * NT) + ((uint32_t)(q * 32) << 16);
         if (ok && srow < p.M[0]) {
-          uint16_t* o = p.swiglu_out + (size_t)(w.n0 + mt * (NT / 2)) * p.ld_swiglu + srow;
+          uint16_t* o = p.act_out + (size_t)(w.n0 + mt * (NT / 2)) * p.ld_act + srow;
 #pragma unroll 1
           for (int c = mt * (NT / 2); c < (mt + 1) * (NT / 2); c += 16) {
             uint32_t va[16], vc[16];
@@ -235,7 +285,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant_
                 const uint32_t u = __float_as_uint(h);   // round to nearest even, NaN stays NaN (step_bf16.cu f32_to_bf16)
                 *o = ((u & 0x7FFFFFFFu) > 0x7F800000u) ? (uint16_t)((u >> 16) | 0x40u) : (uint16_t)((u + 0x7FFFu + ((u >> 16) & 1u)) >> 16);
               }
-              o += p.ld_swiglu;
+              o += p.ld_act;
             }
           }
         }
@@ -468,10 +518,10 @@ bool gemm_bf16_ok(const BfArgs& a) {
 }
 
 
-template <int NT, int MT = 1, bool SWIGLU = false>
+template <int NT, int MT = 1, int READ = BF_PLAIN>
 static int bf_launch_nt(cudaStream_t st, const CUtensorMap* mw, const CUtensorMap& mx, const BfP& p, dim3 grid, bool pdl) {
   using S = BfSmem<NT, MT>;
-  auto k = gemm_bf16_kernel<NT, MT, SWIGLU>;
+  auto k = gemm_bf16_kernel<NT, MT, READ>;
   THA_CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL));
   THA_CUDA_OK(launch(k, grid, dim3(128 + 128 * MT), (size_t)S::TOTAL, st, pdl, mw[0], mw[1], mw[2], mx, p));
   return THA_STATUS_SUCCESS;
@@ -538,25 +588,35 @@ static int bfc_try(cudaStream_t st, const CUtensorMap* mw, const CUtensorMap& mx
   return THA_STATUS_SUCCESS;
 }
 
-bool gemm_bf16_swiglu_ok(const BfArgs& a) {
-  return a.swiglu_out && a.n_mats == 2 && a.M[0] == a.M[1] && a.splits <= 1 && a.N >= 512 && !a.colscale;
+static bool bf_act_pair(const BfArgs& a) { return a.ff_act == 0 || hyb_act_gated(a.ff_act - 1); }
+
+// Where the activation in the read-out is the faster way.  us as product and activation / in one, by rows:
+//   gated    [2 x 4608, 1024]  256: 12.5 / 16.5  400: 25.0 / 17.1  1000: 41 / 26  4000: 118 / 78
+//            [2 x 6144, 2048]  256: 22.7 / 22.7  400: 41.3 / 32.9  1000: 76 / 43  4000: 258 / 154
+//            [2 x 11008, 4096] 256: 57.6 / 63.6  400: 99.6 / 83.2  1000: 189 / 153  4000: 777 / 544
+//   RELU2    [4608, 1024]  160: 12.5 / 8.8  256: 12.4 / 9.5  1000: 35 / 16.5  4000: 84 / 37
+//            [11008, 4096]  160: 50 / 37  1000: 117 / 81  4000: 421 / 289
+// expm1f outweighs the pass that it saves: XIELU [6144, 2048]  160: 19.5 / 20.6  1000: 55 / 59  4000: 140 / 162, so it keeps its own.
+bool gemm_bf16_act_ok(const BfArgs& a) {
+  if (!a.act_out || a.splits > 1 || a.stacked || a.colscale || a.ff_act == 1 + THA_ACT_XIELU) return false;
+  if (!bf_act_pair(a)) return a.n_mats == 1 && a.N > 128;
+  return a.n_mats == 2 && a.M[0] == a.M[1] && a.N >= (a.ff_act ? 257 : 512);
 }
 
 int gemm_bf16_launch(cudaStream_t st, const BfArgs& a, bool pdl) {
   if (!gemm_bf16_ok(a)) return THA_STATUS_INVALID_ARG;
-  const bool swiglu = a.swiglu_out != nullptr;
-  if (swiglu && !gemm_bf16_swiglu_ok(a)) return THA_STATUS_NOT_SUPPORTED;
+  const bool act = a.act_out != nullptr, pair = act && bf_act_pair(a);
+  if (act && !gemm_bf16_act_ok(a)) return THA_STATUS_NOT_SUPPORTED;
   int tiles128 = 0;
   for (int i = 0; i < a.n_mats; i++) tiles128 += ceil_div(a.M[i], TC_BM);
-  const BfTile tile = swiglu ? BfTile{256, 1} : gemm_bf16_tile(tiles128, a.N, a.splits < 1 ? 1 : a.splits);
-  const int NT = tile.nt, MT = tile.mt;   // SwiGLU: 128-row boxes of each of the two matrices (the kernel itself runs MT = 2)
+  const BfTile tile = pair ? BfTile{128, 1} : gemm_bf16_tile(tiles128, a.N, a.splits < 1 ? 1 : a.splits);
+  const int NT = tile.nt, MT = tile.mt;   // pairs: 128-row boxes of each of the two matrices (the kernel itself runs MT = 2)
   CUtensorMap mw[3], mx;
   BfP p = {};
   int tiles = 0;
   p.n_mats = a.n_mats; p.stacked = a.stacked;
   int x_rows = a.N;
   if (a.stacked) {
-    if (swiglu) return THA_STATUS_NOT_SUPPORTED;
     int w_rows = 0;
     for (int i = 0; i < a.n_mats; i++) {
       p.M[i] = a.M[i]; p.tiles[i] = ceil_div(a.M[i], TC_BM * MT); p.out_off[i] = a.out_off[i];
@@ -577,7 +637,9 @@ int gemm_bf16_launch(cudaStream_t st, const BfArgs& a, bool pdl) {
     }
     tiles += p.tiles[i];
   }
-  if (swiglu) { tiles = p.tiles[0]; p.tiles[1] = 0; p.swiglu_out = a.swiglu_out; p.ld_swiglu = a.ld_swiglu; }   // an item = a pair of tiles
+  if (pair) { tiles = p.tiles[0]; p.tiles[1] = 0; p.n_mats = 1; }   // an item = a pair of tiles
+  p.act_out = a.act_out; p.ld_act = a.ld_act;
+  p.act = a.ff_act - 1; p.act_limit = a.act_limit; p.act_alpha = a.act_alpha;
   THA_TRY_RC(tc_map(a.X, x_rows, a.K, a.ldx, NT, &mx, 2));
   p.K = a.K; p.N = a.N;
   p.kblocks_total = ceil_div(a.K, BF_BK);
@@ -589,7 +651,7 @@ int gemm_bf16_launch(cudaStream_t st, const BfArgs& a, bool pdl) {
   p.ny = ceil_div(a.N, NT);
   p.splits = splits;
   p.n_items = tiles * p.ny * splits;
-  if (splits == 1 && !swiglu && NT <= 128) {   // callers that split K themselves sum the partials in a kernel of theirs
+  if (splits == 1 && !act && NT <= 128) {   // callers that split K themselves sum the partials in a kernel of theirs
     bool taken = false;
     int rc = THA_STATUS_SUCCESS;
     switch (NT) {
@@ -606,10 +668,13 @@ int gemm_bf16_launch(cudaStream_t st, const BfArgs& a, bool pdl) {
   switch (NT) {
     case 16: return bf_launch_nt<16>(st, mw, mx, p, grid, pdl);
     case 32: return bf_launch_nt<32>(st, mw, mx, p, grid, pdl);
-    case 64: return bf_launch_nt<64>(st, mw, mx, p, grid, pdl);
-    case 128: return bf_launch_nt<128>(st, mw, mx, p, grid, pdl);
-    default: return swiglu ? bf_launch_nt<256, 2, true>(st, mw, mx, p, grid, pdl)
-                           : (MT == 2 ? bf_launch_nt<256, 2>(st, mw, mx, p, grid, pdl) : bf_launch_nt<256>(st, mw, mx, p, grid, pdl));
+    case 64: return act ? bf_launch_nt<64, 1, BF_UNGATED>(st, mw, mx, p, grid, pdl) : bf_launch_nt<64>(st, mw, mx, p, grid, pdl);
+    case 128:
+      if (pair) return a.ff_act ? bf_launch_nt<128, 2, BF_GATED>(st, mw, mx, p, grid, pdl) : bf_launch_nt<128, 2, BF_SWIGLU>(st, mw, mx, p, grid, pdl);
+      return act ? bf_launch_nt<128, 1, BF_UNGATED>(st, mw, mx, p, grid, pdl) : bf_launch_nt<128>(st, mw, mx, p, grid, pdl);
+    default:
+      if (MT == 2) return act ? bf_launch_nt<256, 2, BF_UNGATED>(st, mw, mx, p, grid, pdl) : bf_launch_nt<256, 2>(st, mw, mx, p, grid, pdl);
+      return act ? bf_launch_nt<256, 1, BF_UNGATED>(st, mw, mx, p, grid, pdl) : bf_launch_nt<256>(st, mw, mx, p, grid, pdl);
   }
 }
 

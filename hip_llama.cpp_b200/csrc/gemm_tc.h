@@ -75,15 +75,17 @@ struct BfArgs {
   const uint16_t* X; int N; long long ldx;       // activations [N, ldx] bf16
   float* out; long long ldo; long long zstride; int splits;
   const float* colscale;
-  // SwiGLU in the read-out (prompt-sized N, two matrices w1 | w3 of equal height, no split-K): a work item multiplies 128 rows
-  // of w1 AND the same 128 rows of w3; its read-out writes silu(w1 x) * (w3 x), rounded to bf16, to swiglu_out[n * ld_swiglu + row]
-  // (the input of the w2 matmul) and `out` is not written at all.
-  uint16_t* swiglu_out; long long ld_swiglu;
+  // A feed-forward's activation in the read-out (prompt-sized N, no split-K); its result, rounded to bf16, goes to act_out[n * ld_act + row]
+  // (the input of the down product) and `out` is not written at all.  ff_act 0: SwiGLU of the llama block, silu(w1 x) * (w3 x); else
+  // 1 + THA_ACT_* of a layer program.  Gated ones (SwiGLU too) take two matrices of equal height, w1 = gate and w3 = up: a work item
+  // multiplies 128 rows of the one AND the same 128 rows of the other.  Ungated ones take one matrix.
+  uint16_t* act_out; long long ld_act;
+  int ff_act; float act_limit, act_alpha;
   // stacked: up to BF_MAX_MATS matrices that are row ranges of ONE matrix W[0], each with activation rows of its own: matrix i =
   // rows w_row[i] .. + M[i] of W[0], its activations rows x_row[i] .. + N of X
   int stacked; int w_row[BF_MAX_MATS]; int x_row[BF_MAX_MATS];
 };
-bool gemm_bf16_swiglu_ok(const BfArgs& a);   // the launch can take the SwiGLU read-out
+bool gemm_bf16_act_ok(const BfArgs& a);   // the launch can take the activation into its read-out, and that is the faster way
 bool gemm_bf16_ok(const BfArgs& a);
 struct BfTile { int nt, mt; };
 BfTile gemm_bf16_tile(int tiles, int N, int splits);   // output tile: 128 mt weight rows (of `tiles` 128-row tiles) x nt activation rows; K in `splits` shares

@@ -1635,19 +1635,6 @@ __global__ void hyb_route_groups_kernel(int experts, int top, int groups, int ke
   if (lane < top) weight[(size_t)r * top + lane] = SIGMOID ? mine * scale : mine / (sum + 1e-20f);
 }
 
-// any of the feed-forward activations (THA_ACT_*): gated ones read a gate value g and an up value u, ungated ones u only.
-// THA_ACT_XIELU arrives with (limit, alpha) = (softplus(p), 1/2 + softplus(q)) of its two stored numbers.
-__device__ __forceinline__ float hyb_act_value(int act, float g, float u, float limit, float alpha) {
-  if (act == THA_ACT_RELU2) {
-    const float p = fmaxf(u, 0.f);
-    return p * p;
-  }
-  if (act == THA_ACT_XIELU) return u > 0.f ? fmaf(limit * u, u, 0.5f * u) : fmaf(alpha, expm1f(u) - u, 0.5f * u);
-  if (act == THA_ACT_SILU_GLU) return g * hyb_sigmoid(g) * u;
-  if (act == THA_ACT_GELU_TANH_GLU) return 0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) * u;
-  const float gc = fminf(g, limit);
-  return gc * hyb_sigmoid(alpha * gc) * (fminf(fmaxf(u, -limit), limit) + 1.0f);
-}
 template <typename T>
 __global__ void hyb_ff_act_kernel(T* __restrict__ y, const float* __restrict__ gu, long long ldg, int col_g, int col_u, int n, int ff, int act,
                                   float limit, float alpha) {
@@ -1655,7 +1642,7 @@ __global__ void hyb_ff_act_kernel(T* __restrict__ y, const float* __restrict__ g
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (size_t)n * ff) return;
   const size_t r = i / ff; const int c = (int)(i - r * ff);
-  const bool gated = act != THA_ACT_RELU2 && act != THA_ACT_XIELU;
+  const bool gated = hyb_act_gated(act);
   hyb_store(y + i, hyb_act_value(act, gated ? gu[r * ldg + col_g + c] : 0.f, gu[r * ldg + col_u + c], limit, alpha));
 }
 // the same with four columns per thread and a row per blockIdx.y (sizes and offsets that are multiples of four)
@@ -1666,7 +1653,7 @@ __global__ void hyb_ff_act_vec_kernel(T* __restrict__ y, const float* __restrict
   const int c = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
   if (c >= ff) return;
   const size_t r = blockIdx.y;
-  const bool gated = act != THA_ACT_RELU2 && act != THA_ACT_XIELU;
+  const bool gated = hyb_act_gated(act);
   const float4 u = *reinterpret_cast<const float4*>(gu + r * ldg + col_u + c);
   const float4 g = gated ? *reinterpret_cast<const float4*>(gu + r * ldg + col_g + c) : make_float4(0.f, 0.f, 0.f, 0.f);
   const float v0 = hyb_act_value(act, g.x, u.x, limit, alpha), v1 = hyb_act_value(act, g.y, u.y, limit, alpha);
@@ -1817,6 +1804,14 @@ extern "C" int tha_hyb_head_gate(void* stream, int dtype, void* out, const float
   return THA_STATUS_SUCCESS;
 }
 
+// THA_ACT_XIELU: the two stored numbers p, q -> the factors the kernels multiply with
+static void hyb_act_factors(int act, float& limit, float& alpha) {
+  if (act != THA_ACT_XIELU) return;
+  const float p = limit, q = alpha;
+  limit = fmaxf(p, 0.f) + log1pf(expf(-fabsf(p)));
+  alpha = 0.5f + fmaxf(q, 0.f) + log1pf(expf(-fabsf(q)));
+}
+
 extern "C" int tha_hyb_linear(void* stream, int dtype, float* C, long long ldc, const void* A, long long lda, int a_f32,
                               const int* a_rows, const void* W, long long w_group_stride, int M, int N, int K,
                               const int* group_off, int n_groups) {
@@ -1849,6 +1844,31 @@ extern "C" int tha_hyb_linear(void* stream, int dtype, float* C, long long ldc, 
     THA_CUDA_OK(launch(hyb_linear_kernel<bf16, bf16>, grid, block, 0, s, pdl_enabled() != 0, C, ldc, (const bf16*)A, lda, a_rows, (const bf16*)W,
                        w_group_stride, M, N, K, group_off, n_groups, 0ll, 0ll, 0ll));
   return THA_STATUS_SUCCESS;
+}
+
+extern "C" int tha_hyb_linear_act(void* stream, int dtype, int act, void* y, float* gu, long long ldg, const void* A, const void* W, int M, int N, int K,
+                                  int col_g, int col_u, int ff, float limit, float alpha) {
+  if (M < 1 || N < 1) return THA_STATUS_SUCCESS;
+  if (K < 1 || ff < 1 || !y || !gu || !A || !W) return THA_STATUS_INVALID_ARG;
+  const bool gated = hyb_act_gated(act);
+  if (dtype == THA_DT_BF16 && hyb_tc_linear() && act >= THA_ACT_GLU_CLAMPED && act <= THA_ACT_SILU_GLU && col_u >= 0 && col_u + ff <= N &&
+      (!gated || (col_g >= 0 && col_g + ff <= N))) {
+    BfArgs b = {};
+    b.n_mats = gated ? 2 : 1; b.K = K;
+    const uint16_t* w = (const uint16_t*)W;
+    if (gated) { b.W[0] = w + (size_t)col_g * K; b.W[1] = w + (size_t)col_u * K; b.M[1] = ff; }
+    else b.W[0] = w + (size_t)col_u * K;
+    b.M[0] = ff;
+    b.X = (const uint16_t*)A; b.N = M; b.ldx = K;
+    b.out = gu; b.ldo = ldg; b.splits = 1;
+    b.act_out = (uint16_t*)y; b.ld_act = ff;
+    b.ff_act = 1 + act; b.act_limit = limit; b.act_alpha = alpha;
+    hyb_act_factors(act, b.act_limit, b.act_alpha);
+    if (gemm_bf16_ok(b) && gemm_bf16_act_ok(b)) return gemm_bf16_launch((cudaStream_t)stream, b, hyb_gemm_pdl());
+  }
+  const int rc = tha_hyb_linear(stream, dtype, gu, ldg, A, K, 0, nullptr, W, 0, M, N, K, nullptr, 0);
+  if (rc != THA_STATUS_SUCCESS) return rc;
+  return tha_hyb_ff_act(stream, dtype, act, y, gu, ldg, col_g, col_u, M, ff, limit, alpha);
 }
 
 extern "C" int tha_hyb_linear_groups(void* stream, int dtype, float* C, long long ldc, const void* A, const void* W, int M, int K, int n_groups,
@@ -2185,13 +2205,9 @@ extern "C" int tha_hyb_moe_route(void* stream, const tha_moe_t* e, const float* 
 extern "C" int tha_hyb_ff_act(void* stream, int dtype, int act, void* y, const float* gu, long long ldg, int col_g, int col_u, int n,
                               int ff, float limit, float alpha) {
   if (n < 1 || ff < 1) return THA_STATUS_SUCCESS;
-  if (act == THA_ACT_XIELU) {   // the two stored numbers p, q -> the factors the kernel multiplies with
-    const float p = limit, q = alpha;
-    limit = fmaxf(p, 0.f) + log1pf(expf(-fabsf(p)));
-    alpha = 0.5f + fmaxf(q, 0.f) + log1pf(expf(-fabsf(q)));
-  }
+  hyb_act_factors(act, limit, alpha);
   cudaStream_t s = (cudaStream_t)stream;
-  const bool gated = act != THA_ACT_RELU2 && act != THA_ACT_XIELU;
+  const bool gated = hyb_act_gated(act);
   if (ff % 4 == 0 && ldg % 4 == 0 && col_u % 4 == 0 && (!gated || col_g % 4 == 0) && aligned16(gu) && n <= 65535) {
     const dim3 grid(ceil_div(ff / 4, 128), n);
     if (dtype == THA_DT_BF16)

@@ -45,6 +45,21 @@ __device__ __forceinline__ float hyb_logsigmoid(float z) { return fminf(z, 0.f) 
 __device__ __forceinline__ float hyb_sigmoid(float z) { return 1.0f / (1.0f + expf(-z)); }
 __device__ __forceinline__ float hyb_softplus(float z) { return fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))); }
 
+// any of the feed-forward activations (THA_ACT_*): gated ones read a gate value g and an up value u, ungated ones u only.
+// THA_ACT_XIELU arrives with (limit, alpha) = (softplus(p), 1/2 + softplus(q)) of its two stored numbers.
+__host__ __device__ __forceinline__ bool hyb_act_gated(int act) { return act != THA_ACT_RELU2 && act != THA_ACT_XIELU; }
+__device__ __forceinline__ float hyb_act_value(int act, float g, float u, float limit, float alpha) {
+  if (act == THA_ACT_RELU2) {
+    const float p = fmaxf(u, 0.f);
+    return p * p;
+  }
+  if (act == THA_ACT_XIELU) return u > 0.f ? fmaf(limit * u, u, 0.5f * u) : fmaf(alpha, expm1f(u) - u, 0.5f * u);
+  if (act == THA_ACT_SILU_GLU) return g * hyb_sigmoid(g) * u;
+  if (act == THA_ACT_GELU_TANH_GLU) return 0.5f * g * (1.0f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))) * u;
+  const float gc = fminf(g, limit);
+  return gc * hyb_sigmoid(alpha * gc) * (fminf(fmaxf(u, -limit), limit) + 1.0f);
+}
+
 // Element d of a vector whose first rot_dims entries are rotated by the row's angles (c, s: cos and sin of its rot_dims / 2
 // pairs): the pair (first, second) becomes (first c - second s, second c + first s).  THA_ROT_INTERLEAVED pairs (2i, 2i + 1),
 // THA_ROT_HALVES pairs (i, i + rot_dims / 2); entries from rot_dims on pass unchanged.  w (nullable): per-entry weights applied first.

@@ -541,12 +541,13 @@ static int hyb_issue(void* stream, HybScratch& sc, const tha_hyb_model_t* m, con
         // the mixer's write and the feed-forward's read in one pass over the streams
         HYB_OK(tha_hyb_streams(stream, dt, b.xs, n_str, nullptr, &L.streams1, b.left, nullptr, 0, nullptr, nullptr, nullptr, nullptr, nullptr,
                                &L.streams2, &L.norm2, m->eps, 0, b.h2, R, W));
-        HYB_OK(tha_hyb_linear(stream, dt, b.proj2, ldp2, b.h2, W, 0, nullptr, L.w_in2, 0, R, L.n_in2, W, nullptr, 0));
+        const tha_dense_ff_t& d = L.dense;
+        const bool in_one = L.has_ff == THA_FF_DENSE && d.act != THA_ACT_POLYNORM && !d.b_up;
+        if (!in_one) HYB_OK(tha_hyb_linear(stream, dt, b.proj2, ldp2, b.h2, W, 0, nullptr, L.w_in2, 0, R, L.n_in2, W, nullptr, 0));
         if (L.has_ff == THA_FF_DENSE) {
-          const tha_dense_ff_t& d = L.dense;
           if (d.act == THA_ACT_POLYNORM) HYB_OK(tha_hyb_polynorm(stream, dt, b.sy, b.proj2, ldp2, d.o_up, d.b_up, d.act_c, m->eps, R, d.ff));
           else if (d.b_up) return THA_STATUS_NOT_SUPPORTED;
-          else HYB_OK(tha_hyb_ff_act(stream, dt, d.act, b.sy, b.proj2, ldp2, d.o_gate, d.o_up, R, d.ff, d.act_p, d.act_q));
+          else HYB_OK(tha_hyb_linear_act(stream, dt, d.act, b.sy, b.proj2, ldp2, b.h2, L.w_in2, R, L.n_in2, W, d.o_gate, d.o_up, d.ff, d.act_p, d.act_q));
           HYB_OK(tha_hyb_linear(stream, dt, b.sdown, W, b.sy, d.ff, 0, nullptr, d.w_down, 0, R, W, d.ff, nullptr, 0));
           HYB_OK(tha_hyb_streams(stream, dt, b.xs, n_str, nullptr, &L.streams2, b.sdown, d.b_down, 0, nullptr, nullptr, nullptr, tap, sum_out,
                                  next ? &next->streams1 : nullptr, next ? &next->norm1 : nullptr, m->eps, nconv, nout, R, W));
@@ -573,8 +574,7 @@ static int hyb_issue(void* stream, HybScratch& sc, const tha_hyb_model_t* m, con
       if (L.has_ff == THA_FF_DENSE) {
         const tha_dense_ff_t& d = L.dense;
         HYB_OK(tha_hyb_add_norm(stream, dt, b.x, b.left, left_b, cl, right, cr, nullptr, nullptr, &L.norm2, m->eps, b.h2, 0, R, W));
-        HYB_OK(tha_hyb_linear(stream, dt, b.proj2, ldp2, b.h2, W, 0, nullptr, L.w_in2, 0, R, L.n_in2, W, nullptr, 0));
-        HYB_OK(tha_hyb_ff_act(stream, dt, d.act, b.sy, b.proj2, ldp2, d.o_gate, d.o_up, R, d.ff, d.act_p, d.act_q));
+        HYB_OK(tha_hyb_linear_act(stream, dt, d.act, b.sy, b.proj2, ldp2, b.h2, L.w_in2, R, L.n_in2, W, d.o_gate, d.o_up, d.ff, d.act_p, d.act_q));
         HYB_OK(tha_hyb_linear(stream, dt, b.sdown, W, b.sy, d.ff, 0, nullptr, d.w_down, 0, R, W, d.ff, nullptr, 0));
         ffo = b.sdown;
       } else if (L.has_ff == THA_FF_NONE && !right) {
@@ -620,13 +620,13 @@ static int hyb_issue(void* stream, HybScratch& sc, const tha_hyb_model_t* m, con
       HYB_OK(tha_hyb_post_norm(stream, dt, b.x, b.left, nullptr, 0, 0, nullptr, nullptr, nullptr, L.res_mult, &L.norm1, m->eps, ff ? nullptr : tap,
                                ff ? b.h : hand_on, R, W));
       if (ff) {
-        HYB_OK(tha_hyb_linear(stream, dt, b.proj2, ldp2, b.h, W, 0, nullptr, L.w_in2, 0, R, L.n_in2, W, nullptr, 0));
+        if (L.has_ff != THA_FF_DENSE) HYB_OK(tha_hyb_linear(stream, dt, b.proj2, ldp2, b.h, W, 0, nullptr, L.w_in2, 0, R, L.n_in2, W, nullptr, 0));
         const float* dense = nullptr;
         const float* dense_gate = nullptr;
         int top = 0;
         if (L.has_ff == THA_FF_DENSE) {
           const tha_dense_ff_t& d = L.dense;
-          HYB_OK(tha_hyb_ff_act(stream, dt, d.act, b.sy, b.proj2, ldp2, d.o_gate, d.o_up, R, d.ff, d.act_p, d.act_q));
+          HYB_OK(tha_hyb_linear_act(stream, dt, d.act, b.sy, b.proj2, ldp2, b.h, L.w_in2, R, L.n_in2, W, d.o_gate, d.o_up, d.ff, d.act_p, d.act_q));
           HYB_OK(tha_hyb_linear(stream, dt, b.sdown, W, b.sy, d.ff, 0, nullptr, d.w_down, 0, R, W, d.ff, nullptr, 0));
           dense = b.sdown;
         } else {
@@ -650,7 +650,7 @@ static int hyb_issue(void* stream, HybScratch& sc, const tha_hyb_model_t* m, con
     const float* fproj = b.proj;
     long long ldf = ldp;
     if (two_norms) {
-      HYB_OK(tha_hyb_linear(stream, dt, b.proj2, ldp2, b.h2, W, 0, nullptr, L.w_in2, 0, R, L.n_in2, W, nullptr, 0));
+      if (L.has_ff != THA_FF_DENSE) HYB_OK(tha_hyb_linear(stream, dt, b.proj2, ldp2, b.h2, W, 0, nullptr, L.w_in2, 0, R, L.n_in2, W, nullptr, 0));
       hf = b.h2; fproj = b.proj2; ldf = ldp2;
     }
     int top = 0;
@@ -658,7 +658,8 @@ static int hyb_issue(void* stream, HybScratch& sc, const tha_hyb_model_t* m, con
     const float* sgate = nullptr;
     if (L.has_ff == THA_FF_DENSE) {
       const tha_dense_ff_t& d = L.dense;
-      HYB_OK(tha_hyb_ff_act(stream, dt, d.act, b.sy, fproj, ldf, d.o_gate, d.o_up, R, d.ff, d.act_p, d.act_q));
+      if (two_norms) HYB_OK(tha_hyb_linear_act(stream, dt, d.act, b.sy, b.proj2, ldp2, b.h2, L.w_in2, R, L.n_in2, W, d.o_gate, d.o_up, d.ff, d.act_p, d.act_q));
+      else HYB_OK(tha_hyb_ff_act(stream, dt, d.act, b.sy, fproj, ldf, d.o_gate, d.o_up, R, d.ff, d.act_p, d.act_q));
       HYB_OK(tha_hyb_linear(stream, dt, b.sdown, W, b.sy, d.ff, 0, nullptr, d.w_down, 0, R, W, d.ff, nullptr, 0));
       sdown = b.sdown;
     } else if (L.has_ff == THA_FF_MOE) {

@@ -444,8 +444,8 @@ static int bf_issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, 
       BfArgs a = {};
       a.n_mats = 2; a.W[0] = W[0]; a.W[1] = W[1]; a.M[0] = hd; a.M[1] = hd; a.out_off[0] = 0; a.out_off[1] = hd;
       a.K = d; a.X = sc.xb; a.N = R; a.ldx = d; a.out = sc.part; a.ldo = ld_h; a.zstride = (long long)R * ld_h; a.splits = pl.z_w13;
-      a.swiglu_out = sc.hb; a.ld_swiglu = hd;
-      swiglu_fused = bf_swiglu_mode() && gemm_bf16_swiglu_ok(a);
+      a.act_out = sc.hb; a.ld_act = hd;
+      swiglu_fused = bf_swiglu_mode() && gemm_bf16_act_ok(a);
       if (swiglu_fused) THA_TRY_RC(gemm_bf16_launch(st, a, pdl));
       else THA_TRY_RC(mm(2, W, M, off, d, sc.xb, R, sc.part, ld_h, (long long)R * ld_h, pl.z_w13));
     }

@@ -574,6 +574,12 @@ int tha_hyb_glu_clamped(void* stream, int dtype, void* y, const float* gu, long 
 int tha_hyb_ff_act(void* stream, int dtype, int act, void* y, const float* gu, long long ldg, int col_g, int col_u, int n,
                    int ff, float limit, float alpha);
 
+/* tha_hyb_linear of M rows [M, K] with a matrix W [N, K] and tha_hyb_ff_act of its columns: y [M, ff] (dtype-typed) = act of the
+ * products with W's rows col_g .. (gated activations) and col_u ...  gu [M, ldg] is room for the products, its contents
+ * afterwards are undefined: bf16 prompts apply the activation where the products are read out. */
+int tha_hyb_linear_act(void* stream, int dtype, int act, void* y, float* gu, long long ldg, const void* A, const void* W, int M, int N,
+                       int K, int col_g, int col_u, int ff, float limit, float alpha);
+
 /* causal convolution over `channels` adjacent columns of proj starting at col0, continuing from the slot's tail (the last
  * taps - 1 inputs of every channel): out[r, c] = act(sum_j w[c, j] in(r - taps + 1 + j, c)) (+ in(r, c) with add_input);
  * bias ([channels], NULL: none) is added to the step's rows before they meet the taps; the tail holds rows with it.
