@@ -5,35 +5,84 @@
 // depends on the step is the number of runs a context is cut into, the order of an fp32 sum.
 // The tiled kernels (hybrid_ops.cu) give a block 16 to 128 (position, head) pairs and stage key tiles through shared memory; with
 // one position per sequence most pairs are empty and a block walks its tiles one load latency after the other.  Here a block takes one row,
-// up to four query heads of one key/value head, and a run of 32-key tiles.  Eight lanes share a key (a lane: four channels of every 32), so
-// a warp's load instruction covers four keys' rows; of a tile each of the four warps takes eight keys, all of whose K and V loads are in
-// flight at once; the running maximum, sum and accumulator live in registers per group of eight lanes and meet only at the end of
+// up to four query heads of one key/value head, and a run of 32-key tiles.  Of a tile each of the four warps takes eight keys and copies their
+// rows to a ring of three tiles in shared memory of its own (cp.async), so that a usual run is in flight at once; eight lanes share a key (a lane:
+// four channels of every 32); the running maximum, sum and accumulator live in registers per group of eight lanes and meet only at the end of
 // the run.  Nothing is rounded: q, keys, values and weights stay fp32 in both number formats.
-// Bound by the latency of a run's loads, and by the cache rows it reads where there are many.
+// Inside a step the rows of all keys but the newest are there before the kernel ahead is done (it writes the newest), so they are asked for
+// ahead of the wait for it; the distance bias is asked for with a tile and not score by score.
+// Bound by the latency of what follows that wait (q, the newest key, three tiles' arithmetic, the meeting of the warps), and by the cache rows it
+// reads where there are many.  16 heads on 4 of 128 channels, 2 rows at 1100 .. 2900, behind the kernel ahead: tiles loaded to registers one by
+// one 15.2 us; the ring, ahead of the wait 11.4; the bias with the tile 9.0; all heads' scores before their sums 8.4.
 #include "common.cuh"
 #include "hybrid_ops.cuh"
 
 namespace tha {
 
 constexpr int AR_HEADS = 4, AR_MAXD = 128, AR_THREADS = 128;
+constexpr int AR_STAGES = 3;   // tiles of a run in flight
 
-__device__ __forceinline__ float4 ar_ld(const float* p) { return ldg_stream(reinterpret_cast<const float4*>(p)); }
+// sixteen bytes from global to shared memory behind the thread's back; bytes 0: zeros, src is not read
+__device__ __forceinline__ void ar_copy16(void* dst, const float* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void ar_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void ar_await() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 template <typename T, int GS>
 __global__ void __launch_bounds__(AR_THREADS) hyb_attn_row_kernel(tha_attn_t a, tha_rows_t rows, tha_kv_t kv, const float* __restrict__ q, T* __restrict__ out,
-                                                                  int splits, float* __restrict__ partial, const float* __restrict__ gate, long long ldg) {
-  hyb_pdl_enter();
+                                                                  int splits, float* __restrict__ partial, const float* __restrict__ gate, long long ldg, int early) {
+  pdl_trigger();
+  if (!early) pdl_wait();
   constexpr int NI = AR_MAXD / 32;                 // float4 per lane of a row of up to 128 channels
+  extern __shared__ __align__(16) float ar_ring[];
   __shared__ float sm_acc[4][GS][AR_MAXD];
   __shared__ float sm_ml[4][GS][2];
   const int D = a.dim, E = a.vdim, gsize = a.heads / a.kv_heads;
   const int seq = blockIdx.x / splits, sp = blockIdx.x - seq * splits, g = blockIdx.y, h0 = blockIdx.z * GS;
   const int r = rows.seq_first[seq];
-  if (rows.seq_first[seq + 1] - r != 1) return;   // a longer portion: the tiled kernels'
+  if (rows.seq_first[seq + 1] - r != 1) {         // a longer portion: the tiled kernels'
+    if (early) pdl_wait();                         // no kernel ends ahead of the one before it
+    return;
+  }
   const int gv = a.v_share > 1 ? g / a.v_share : g;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, kq = lane >> 3, c4 = 4 * (lane & 7);
   const int p = rows.pos[r], slot = rows.seq_slot[seq];
   const int first = a.chunk > 0 ? (p / a.chunk) * a.chunk : 0;
+  const HybTiles tiles = hyb_attn_tiles(a, first, p, p);
+  const int per = (tiles.n + splits - 1) / splits, ti0 = sp * per, ti_end = min(tiles.n, ti0 + per);
+  auto tile_key = [&](int ti) { return (ti < tiles.n_a ? tiles.begin + 32 * ti : tiles.resume + 32 * (ti - tiles.n_a)) + 8 * warp; };
+  // the warp's eight keys of a tile on their way to its place in the ring: lanes 0..7 look their rows up, key 4 j + kq then goes to lanes
+  // kq * 8 ..; `newest`: key p, whose row the kernel ahead writes, or all the others
+  float* ring = ar_ring + (size_t)warp * AR_STAGES * 8 * (D + E);
+  auto fetch = [&](int ti, bool others, bool newest) {
+    const int kt = tile_key(ti), mine = kt + (lane & 7);
+    if (newest && !others && (p < kt || p >= kt + 8)) return;
+    const size_t row = (mine <= p && mine >= first) ? hyb_kv_row(kv, slot, mine, a.cache_layer) : (size_t)-1;
+    float* st = ring + (size_t)((ti - ti0) % AR_STAGES) * 8 * (D + E);
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+      const int key = kt + 4 * j + kq;
+      const size_t at = __shfl_sync(THA_FULL_MASK, row, 4 * j + kq);
+      if (!(key == p ? newest : others)) continue;
+      const bool vis = at != (size_t)-1 && hyb_attn_sees(a, key, p, first);
+      const float *kp = kv.k_pool + (vis ? at : 0) + (size_t)g * D + c4, *vp = kv.v_pool + (vis ? at : 0) + (size_t)gv * E + c4;
+      float* dst = st + (4 * j + kq) * (D + E) + c4;
+#pragma unroll
+      for (int i = 0; i < NI; i++) {
+        if (32 * i < D) ar_copy16(dst + 32 * i, kp + 32 * i, vis ? 16 : 0);
+        if (32 * i < E) ar_copy16(dst + D + 32 * i, vp + 32 * i, vis ? 16 : 0);
+      }
+    }
+  };
+  const int ti_ring = min(ti_end, ti0 + AR_STAGES);
+  for (int ti = ti0; ti < ti_ring; ti++) fetch(ti, true, !early);
+  if (early) {
+    pdl_wait();
+    for (int ti = ti0; ti < ti_ring; ti++) fetch(ti, false, true);
+  }
+  ar_commit();
   float4 qv[GS][NI], acc[GS][NI];
   float m_run[GS], l_run[GS], hs[GS];
 #pragma unroll
@@ -48,55 +97,70 @@ __global__ void __launch_bounds__(AR_THREADS) hyb_attn_row_kernel(tha_attn_t a, 
       qv[h][i] = 32 * i < D ? *reinterpret_cast<const float4*>(qr + 32 * i + c4) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
-  const HybTiles tiles = hyb_attn_tiles(a, first, p, p);
-  const int per = (tiles.n + splits - 1) / splits, ti_end = min(tiles.n, (sp + 1) * per);
-  for (int ti = sp * per; ti < ti_end; ti++) {
-    const int kt = (ti < tiles.n_a ? tiles.begin + 32 * ti : tiles.resume + 32 * (ti - tiles.n_a)) + 8 * warp;
-    // this warp's eight keys: lanes 0..7 look their rows up, key 4 j + kq then goes to lanes kq * 8 ..
-    const int mine = kt + (lane & 7);
-    const size_t row = (mine <= p && mine >= first) ? hyb_kv_row(kv, slot, mine, a.cache_layer) : (size_t)-1;
-    float4 kr[2][NI], vr[2][NI];
+  for (int ti = ti0; ti < ti_end; ti++) {
+    const int kt = tile_key(ti);
+    float bias[GS][2];                                     // the distance's bias: asked for ahead of the tile, all at once
+    if (a.rel) {
+#pragma unroll
+      for (int h = 0; h < GS; h++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) bias[h][j] = hyb_attn_rel(a, g * gsize + min(h0 + h, gsize - 1), max(p - (kt + 4 * j + kq), 0));
+    }
+    if (ti == ti0) ar_await<0>();                          // the first round of the ring is one group, then a group a tile
+    else if (ti >= ti0 + AR_STAGES) ar_await<AR_STAGES - 1>();
+    __syncwarp();
+    const float* st = ring + (size_t)((ti - ti0) % AR_STAGES) * 8 * (D + E);
+    float s[GS][2];                                        // the scores of all heads, then their sums: nothing of one waits for another
     bool vis[2];
 #pragma unroll
     for (int j = 0; j < 2; j++) {
-      const size_t at = __shfl_sync(THA_FULL_MASK, row, 4 * j + kq);
-      vis[j] = at != (size_t)-1 && hyb_attn_sees(a, kt + 4 * j + kq, p, first);
-      const float *kp = kv.k_pool + (vis[j] ? at : 0) + (size_t)g * D + c4, *vp = kv.v_pool + (vis[j] ? at : 0) + (size_t)gv * E + c4;
+      const int key = kt + 4 * j + kq;
+      vis[j] = key <= p && key >= first && hyb_attn_sees(a, key, p, first);
+      const float* src = st + (4 * j + kq) * (D + E) + c4;
+      float4 kr[NI];
 #pragma unroll
-      for (int i = 0; i < NI; i++) kr[j][i] = vis[j] && 32 * i < D ? ar_ld(kp + 32 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int i = 0; i < NI; i++) kr[i] = 32 * i < D ? *reinterpret_cast<const float4*>(src + 32 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int i = 0; i < NI; i++) vr[j][i] = vis[j] && 32 * i < E ? ar_ld(vp + 32 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-#pragma unroll
-    for (int h = 0; h < GS; h++) {
-      float s[2];
-#pragma unroll
-      for (int j = 0; j < 2; j++) {
+      for (int h = 0; h < GS; h++) {
         float d = 0.f;
 #pragma unroll
-        for (int i = 0; i < NI; i++) d = dot4(qv[h][i], kr[j][i], d);
+        for (int i = 0; i < NI; i++) d = dot4(qv[h][i], kr[i], d);
         d += __shfl_xor_sync(THA_FULL_MASK, d, 1);
         d += __shfl_xor_sync(THA_FULL_MASK, d, 2);
         d += __shfl_xor_sync(THA_FULL_MASK, d, 4);
         d = d * a.scale * hs[h];
         if (a.softcap > 0.f) d = hyb_softcap(d, a.softcap);
-        if (a.rel && vis[j] && h0 + h < gsize) d += hyb_attn_rel(a, g * gsize + h0 + h, p - (kt + 4 * j + kq));
-        s[j] = vis[j] ? d : -INFINITY;
-      }
-      const float m_new = fmaxf(m_run[h], fmaxf(s[0], s[1]));
-      if (m_new > -INFINITY) {
-        const float corr = expf(m_run[h] - m_new), w0 = expf(s[0] - m_new), w1 = expf(s[1] - m_new);
-        l_run[h] = l_run[h] * corr + (w0 + w1);
-        m_run[h] = m_new;
-#pragma unroll
-        for (int i = 0; i < NI; i++) {
-          acc[h][i].x = fmaf(w1, vr[1][i].x, fmaf(w0, vr[0][i].x, acc[h][i].x * corr));
-          acc[h][i].y = fmaf(w1, vr[1][i].y, fmaf(w0, vr[0][i].y, acc[h][i].y * corr));
-          acc[h][i].z = fmaf(w1, vr[1][i].z, fmaf(w0, vr[0][i].z, acc[h][i].z * corr));
-          acc[h][i].w = fmaf(w1, vr[1][i].w, fmaf(w0, vr[0][i].w, acc[h][i].w * corr));
-        }
+        if (a.rel) d += bias[h][j];
+        s[h][j] = vis[j] ? d : -INFINITY;
       }
     }
+    float corr[GS];
+#pragma unroll
+    for (int h = 0; h < GS; h++) {
+      const float m_new = fmaxf(m_run[h], fmaxf(s[h][0], s[h][1]));
+      const bool any = m_new > -INFINITY;                  // else nothing was seen so far, and what there is stays
+      corr[h] = any ? expf(m_run[h] - m_new) : 1.f;
+      s[h][0] = any ? expf(s[h][0] - m_new) : 0.f;
+      s[h][1] = any ? expf(s[h][1] - m_new) : 0.f;
+      l_run[h] = l_run[h] * corr[h] + (s[h][0] + s[h][1]);
+      m_run[h] = m_new;
+    }
+    const float *v0 = st + kq * (D + E) + D + c4, *v1 = v0 + 4 * (D + E);
+#pragma unroll
+    for (int i = 0; i < NI; i++) {
+      const float4 x = 32 * i < E ? *reinterpret_cast<const float4*>(v0 + 32 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 y = 32 * i < E ? *reinterpret_cast<const float4*>(v1 + 32 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int h = 0; h < GS; h++) {
+        acc[h][i].x = fmaf(s[h][1], y.x, fmaf(s[h][0], x.x, acc[h][i].x * corr[h]));
+        acc[h][i].y = fmaf(s[h][1], y.y, fmaf(s[h][0], x.y, acc[h][i].y * corr[h]));
+        acc[h][i].z = fmaf(s[h][1], y.z, fmaf(s[h][0], x.z, acc[h][i].z * corr[h]));
+        acc[h][i].w = fmaf(s[h][1], y.w, fmaf(s[h][0], x.w, acc[h][i].w * corr[h]));
+      }
+    }
+    __syncwarp();
+    if (ti + AR_STAGES < ti_end) fetch(ti + AR_STAGES, true, true);
+    ar_commit();
   }
   // the four key groups of a warp, then the four warps
 #pragma unroll
@@ -160,15 +224,23 @@ int hyb_attn_row_splits(const tha_attn_t* a, const tha_rows_t* rows, int max_key
   if (s > most) s = most;
   return s < 1 ? 1 : (s > 32 ? 32 : (int)s);
 }
+template <typename T, int GS>
+static int row_launch_heads(cudaStream_t s, const tha_attn_t* a, const tha_rows_t* rows, const tha_kv_t* kv, const float* q, T* out, int splits, float* partial,
+                            const float* gate, long long ldg, int groups) {
+  auto k = hyb_attn_row_kernel<T, GS>;
+  const int ring = 4 * AR_STAGES * 8 * (a->dim + a->vdim) * (int)sizeof(float);
+  THA_CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, ring));
+  THA_CUDA_OK(launch(k, dim3(rows->n_seqs * splits, a->kv_heads, groups), dim3(AR_THREADS), ring, s, pdl_enabled() != 0, *a, *rows, *kv, q, out, splits, partial,
+                     gate, ldg, (int)hyb_gemm_pdl()));
+  return THA_STATUS_SUCCESS;
+}
 template <typename T>
 static int row_launch(cudaStream_t s, const tha_attn_t* a, const tha_rows_t* rows, const tha_kv_t* kv, const float* q, T* out, int splits, float* partial,
                       const float* gate, long long ldg) {
-  const int gsize = a->heads / a->kv_heads, gs = gsize >= 3 ? AR_HEADS : gsize;
-  const dim3 grid(rows->n_seqs * splits, a->kv_heads, ceil_div(gsize, gs));
-  if (gs == 1) THA_CUDA_OK(launch(hyb_attn_row_kernel<T, 1>, grid, dim3(AR_THREADS), 0, s, pdl_enabled() != 0, *a, *rows, *kv, q, out, splits, partial, gate, ldg));
-  else if (gs == 2) THA_CUDA_OK(launch(hyb_attn_row_kernel<T, 2>, grid, dim3(AR_THREADS), 0, s, pdl_enabled() != 0, *a, *rows, *kv, q, out, splits, partial, gate, ldg));
-  else THA_CUDA_OK(launch(hyb_attn_row_kernel<T, AR_HEADS>, grid, dim3(AR_THREADS), 0, s, pdl_enabled() != 0, *a, *rows, *kv, q, out, splits, partial, gate, ldg));
-  return THA_STATUS_SUCCESS;
+  const int gsize = a->heads / a->kv_heads, gs = gsize >= 3 ? AR_HEADS : gsize, groups = ceil_div(gsize, gs);
+  if (gs == 1) return row_launch_heads<T, 1>(s, a, rows, kv, q, out, splits, partial, gate, ldg, groups);
+  if (gs == 2) return row_launch_heads<T, 2>(s, a, rows, kv, q, out, splits, partial, gate, ldg, groups);
+  return row_launch_heads<T, AR_HEADS>(s, a, rows, kv, q, out, splits, partial, gate, ldg, groups);
 }
 int hyb_attn_row_launch(cudaStream_t s, int dtype, const tha_attn_t* a, const tha_rows_t* rows, const tha_kv_t* kv, const float* q, void* out, int splits,
                         float* partial, const float* gate, long long ldg) {
