@@ -59,9 +59,9 @@ __device__ __forceinline__ float ax_head_max(float4 v, int hs) {
 
 // tc_rope_scatter_kernel (step_tc.cu) for this attention: the same cache rows, to the bit, and the planes.  hs 64 or 128.
 // Bound by memory as that one is; 16 bytes a value of q|k|v with one share of K.  grid (ld / 2048, rows)
-__global__ void __launch_bounds__(256) x3_rope_kernel(const float* __restrict__ part, int nz, long long zstride, int ld, const int* __restrict__ pos, int d, int kvd, int hs,
-                                                      const float* __restrict__ rc, const float* __restrict__ rs, float* __restrict__ kc, float* __restrict__ vc,
-                                                      long long kv_bs, int loff, const int* __restrict__ slot, const KvPaged pg, const X3Staged st) {
+__global__ void __launch_bounds__(256) x3_rope_kernel(const float* part, int nz, long long zstride, int ld, const int* pos, int d, int kvd, int hs,
+                                                      const float* rc, const float* rs, float* kc, float* vc,
+                                                      long long kv_bs, int loff, const int* slot, const KvPaged pg, const X3Staged st) {
   pdl_trigger();
   pdl_wait();
   const int b = blockIdx.y, pb = pos[b], sb = slot[b], staged = st.row[b];
@@ -115,8 +115,8 @@ __global__ void __launch_bounds__(256) x3_rope_kernel(const float* __restrict__ 
 }
 
 // Cache rows of positions 0 .. upto[i] - 1 of sequence i -> planes and scales of staged rows base[i] + t.  grid (kvd / 1024, positions, sequences)
-__global__ void __launch_bounds__(256) x3_context_kernel(const float* __restrict__ kc, const float* __restrict__ vc, long long kv_bs, const int* __restrict__ seq_slot,
-                                                         const int* __restrict__ upto, const int* __restrict__ base, const KvPaged pg, int kvd, int hs, const X3Staged st) {
+__global__ void __launch_bounds__(256) x3_context_kernel(const float* kc, const float* vc, long long kv_bs, const int* seq_slot,
+                                                         const int* upto, const int* base, const KvPaged pg, int kvd, int hs, const X3Staged st) {
   pdl_trigger();
   pdl_wait();                                        // the planes of the layer before have been read
   const int i = blockIdx.z, n = upto[i], slot = seq_slot[i], li = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
@@ -255,7 +255,7 @@ attn_prefill_x3_kernel(const __grid_constant__ CUtensorMap mqh, const __grid_con
   }
   // inverse scales of the tile from key t0 on: threads 0 .. 127 K's, the others V's; 0 behind the last key
   const float* scales = (tid < AX_T ? p.ks : p.vs) + (size_t)kh * p.staged_rows + key_row0 + (tid & (AX_T - 1));
-  auto scale_of = [&](int t0) { return t0 + (tid & (AX_T - 1)) <= kmax ? __ldg(scales + t0) : 0.0f; };
+  auto scale_of = [&](int t0) { return t0 + (tid & (AX_T - 1)) <= kmax ? scales[t0] : 0.0f; };
   auto keep_scale = [&](float v, int buf) {
     if (tid < AX_T) {
       s_ks[buf][tid] = v;

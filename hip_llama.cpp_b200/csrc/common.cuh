@@ -104,6 +104,9 @@ __device__ __forceinline__ void report_contexts(const int* pos, int n, unsigned 
   sum = __reduce_add_sync(THA_FULL_MASK, sum);
   if ((threadIdx.x & 31) == 0) *reinterpret_cast<volatile unsigned long long*>(out) = (unsigned long long)(longest + 1) << 32 | (unsigned)(sum / n);
 }
+// Loads through `const __restrict__` pointers and __ldg are loads of constants to the compiler, which may move them ahead of this statement, and does
+// where little else lies between (a pass over rows that asks for all its operands at once read them before they were there).  A kernel like
+// that reads what the kernels ahead wrote through plain pointers; ldg_stream is volatile and stays.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Allow the next kernel in the stream to start launching.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }

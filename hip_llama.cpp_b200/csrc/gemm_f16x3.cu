@@ -383,7 +383,7 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
           if (n + X3_NT / 2 <= p.N) {
   #pragma unroll
             for (int j = 0; j < X3_NT / 2; j += 4) {
-              const float4 s4 = __ldg(reinterpret_cast<const float4*>(p.colscale + n + j));
+              const float4 s4 = *reinterpret_cast<const float4*>(p.colscale + n + j);
               const float sc[4] = {s4.x, s4.y, s4.z, s4.w};
   #pragma unroll
               for (int e = 0; e < 4; e++) {

@@ -31,8 +31,8 @@ template <int N>
 __device__ __forceinline__ void ar_await() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 template <typename T, int GS>
-__global__ void __launch_bounds__(AR_THREADS) hyb_attn_row_kernel(tha_attn_t a, tha_rows_t rows, tha_kv_t kv, const float* __restrict__ q, T* __restrict__ out,
-                                                                  int splits, float* __restrict__ partial, const float* __restrict__ gate, long long ldg, int early) {
+__global__ void __launch_bounds__(AR_THREADS) hyb_attn_row_kernel(tha_attn_t a, tha_rows_t rows, tha_kv_t kv, const float* q, T* __restrict__ out,
+                                                                  int splits, float* __restrict__ partial, const float* gate, long long ldg, int early) {
   pdl_trigger();
   if (!early) pdl_wait();
   constexpr int NI = AR_MAXD / 32;                 // float4 per lane of a row of up to 128 channels

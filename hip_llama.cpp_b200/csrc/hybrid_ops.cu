@@ -352,8 +352,8 @@ __global__ void hyb_attn_prepare_kernel(tha_attn_t a, tha_rows_t rows, tha_kv_t 
 __device__ __forceinline__ float4 hyb_scale4(float4 v, float f) { return make_float4(v.x * f, v.y * f, v.z * f, v.w * f); }
 __device__ __forceinline__ float4 hyb_ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 template <int THREADS>   // at most
-__global__ void __launch_bounds__(THREADS, 1280 / THREADS) hyb_attn_prepare4_kernel(tha_attn_t a, tha_rows_t rows, tha_kv_t kv, const float* __restrict__ proj, long long ldp,
-                                                                 const float* __restrict__ cos_t, const float* __restrict__ sin_t, int rot_dims,
+__global__ void __launch_bounds__(THREADS, 1280 / THREADS) hyb_attn_prepare4_kernel(tha_attn_t a, tha_rows_t rows, tha_kv_t kv, const float* proj, long long ldp,
+                                                                 const float* cos_t, const float* sin_t, int rot_dims,
                                                                  float* __restrict__ q_out, int early) {
   pdl_trigger();
   if (!early) pdl_wait();
