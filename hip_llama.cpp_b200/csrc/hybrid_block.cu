@@ -133,38 +133,6 @@ __global__ void hyb_block_finish_kernel(float* __restrict__ x, const float* __re
 // P float4 a thread.  The kernels above write x and read it back for each sum; here all that a thread needs of the row and of the norm is asked
 // for at once.  Bound by the latency of one load, two block sums and a store where there are few rows (decoding: 20 to 100 such kernels a
 // step).  3 rows of 1024, behind the kernel ahead: 4.2 -> 1.5 us and 3.5 -> 1.4; 2000 rows: 13 -> 7.7.
-template <int P>
-struct HybRow { float v[P][4]; };
-template <int P>
-__device__ __forceinline__ HybRow<P> row_load(const float* p, int width) {   // p nullable: zeros
-  HybRow<P> r;
-#pragma unroll
-  for (int i = 0; i < P; i++) {
-    const int c = 4 * (threadIdx.x + i * blockDim.x);
-    if (p && c < width) hyb_load_vec(p + c, r.v[i]);
-    else r.v[i][0] = r.v[i][1] = r.v[i][2] = r.v[i][3] = 0.f;
-  }
-  return r;
-}
-template <int P, typename T>
-__device__ __forceinline__ void row_store(T* p, const HybRow<P>& r, int width) {
-#pragma unroll
-  for (int i = 0; i < P; i++) {
-    const int c = 4 * (threadIdx.x + i * blockDim.x);
-    if (c < width) hyb_store_vec(p + c, r.v[i]);
-  }
-}
-// the sum over the block of f of every element inside the row
-template <int P, typename F>
-__device__ __forceinline__ float row_sum(const HybRow<P>& r, int width, float* red, F f) {
-  float s = 0.f;
-#pragma unroll
-  for (int i = 0; i < P; i++)
-    if (4 * (threadIdx.x + i * blockDim.x) < width)
-#pragma unroll
-      for (int e = 0; e < 4; e++) s = f(s, r.v[i][e]);
-  return block_sum(s, red);
-}
 template <int P, typename T>
 __device__ __forceinline__ void row_norm(const HybRow<P>& x, const HybRow<P>& w, const HybRow<P>& b, const tha_norm_t& n, float eps, T* out, int width, float* red) {
   HybRow<P> y;
@@ -292,6 +260,35 @@ __global__ void hyb_post_norm_kernel(float* __restrict__ x, const float* __restr
   }
 }
 
+// the same with the row in registers and what the second pass reads asked for beside the first: 2 rows of 2048, behind the kernel ahead, 2.7 -> 1.8 us
+template <typename T, int P>
+__global__ void __launch_bounds__(256) hyb_post_norm_row_kernel(float* x, const float* dense, const float* dense_gate, long long ldg, int top, const float* weight,
+                                                                const int* inv, const float* down, float m, tha_norm_t n, float eps, float* tap, T* out, int width) {
+  hyb_pdl_enter();
+  __shared__ float red[33];
+  const size_t r = blockIdx.x, at = r * width;
+  HybRow<P> v = row_load<P>(x + at, width), y = row_load<P>(dense ? dense + at : nullptr, width);
+  const HybRow<P> nw = row_load<P>(n.w, width);
+  if (dense) {
+    const float sg = dense_gate ? hyb_sigmoid(dense_gate[r * ldg]) : 1.0f;
+#pragma unroll
+    for (int i = 0; i < 4 * P; i++) y.v[i >> 2][i & 3] *= sg;
+  }
+#pragma unroll 2
+  for (int j = 0; j < top; j++) {
+    const float w = weight[r * top + j];
+    const HybRow<P> d = row_load<P>(down + (size_t)inv[r * top + j] * width, width);
+#pragma unroll
+    for (int i = 0; i < 4 * P; i++) y.v[i >> 2][i & 3] = fmaf(w, d.v[i >> 2][i & 3], y.v[i >> 2][i & 3]);
+  }
+  const float f = m / sqrtf(row_sum(y, width, red, [](float s, float a) { return fmaf(a, a, s); }) / (float)width + eps);
+#pragma unroll
+  for (int i = 0; i < 4 * P; i++) v.v[i >> 2][i & 3] = fmaf(y.v[i >> 2][i & 3] * f, n.w_offset + nw.v[i >> 2][i & 3], v.v[i >> 2][i & 3]);
+  row_store(x + at, v, width);
+  if (tap) row_store(tap + at, v, width);
+  if (out) row_store(out + at, v, width);
+}
+
 }  // namespace tha
 
 using namespace tha;
@@ -385,6 +382,15 @@ extern "C" int tha_hyb_post_norm(void* stream, int dtype, float* x, const float*
     THA_CUDA_OK(launch(hyb_post_norm_kernel<T, V>, grid, block, smem, (cudaStream_t)stream, pdl_enabled() != 0, x, dense, dense_gate, ldg, top, weight, inv, down, m, \
                        *norm, eps, tap, (T*)out, width));                                                                                 \
   } while (0)
+  if (const int parts = vec ? row_parts(width, (int)block.x, 0, {}) : 0) {
+#define POST_ROW(T, P)                                                                                                                                            \
+  THA_CUDA_OK(launch(hyb_post_norm_row_kernel<T, P>, grid, block, 0, (cudaStream_t)stream, pdl_enabled() != 0, x, dense, dense_gate, ldg, top, weight, inv, down, m, \
+                     *norm, eps, tap, (T*)out, width))
+    if (dtype == THA_DT_BF16) { if (parts == 1) POST_ROW(bf16, 1); else if (parts == 2) POST_ROW(bf16, 2); else POST_ROW(bf16, 4); }
+    else { if (parts == 1) POST_ROW(float, 1); else if (parts == 2) POST_ROW(float, 2); else POST_ROW(float, 4); }
+#undef POST_ROW
+    return THA_STATUS_SUCCESS;
+  }
   if (dtype == THA_DT_BF16) { if (vec) POST_GO(bf16, 4); else POST_GO(bf16, 1); }
   else { if (vec) POST_GO(float, 4); else POST_GO(float, 1); }
 #undef POST_GO

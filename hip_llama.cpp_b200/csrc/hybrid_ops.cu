@@ -35,6 +35,21 @@ __global__ void hyb_rmsnorm_kernel(T* __restrict__ out, const float* __restrict_
   for (int i = threadIdx.x; i < width; i += blockDim.x) hyb_store(out + (size_t)r * width + i, xr[i] * inv * (w_offset + (w ? w[i] : 0.f)));
 }
 
+// the same with the row in registers: widths of up to 4096 that are a multiple of four, 16-byte aligned.  Bound by latency: 3 rows of 1024, behind the kernel
+// ahead, 2.9 -> 1.8 us
+template <typename T, int P>
+__global__ void __launch_bounds__(256) hyb_rmsnorm_row_kernel(T* out, const float* x, const float* w, float w_offset, float eps, int width, const int* rows_idx) {
+  hyb_pdl_enter();
+  __shared__ float red[33];
+  const int r = blockIdx.x;
+  const HybRow<P> nw = row_load<P>(w, width);
+  HybRow<P> v = row_load<P>(x + (size_t)(rows_idx ? rows_idx[r] : r) * width, width);
+  const float inv = 1.0f / sqrtf(row_sum(v, width, red, [](float s, float a) { return fmaf(a, a, s); }) / (float)width + eps);
+#pragma unroll
+  for (int i = 0; i < 4 * P; i++) v.v[i >> 2][i & 3] = v.v[i >> 2][i & 3] * inv * (w_offset + nw.v[i >> 2][i & 3]);
+  row_store(out + (size_t)r * width, v, width);
+}
+
 // dynamic tanh: tanh(alpha x) w + b, element by element (no mean, no variance)
 template <typename T>
 __global__ void hyb_dyt_kernel(T* __restrict__ out, const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ b,
@@ -1342,6 +1357,54 @@ __global__ void hyb_head_gate_kernel(T* __restrict__ out, const float* __restric
   }
 }
 
+// the same with a head's columns in registers, four of every 128 a lane: heads of up to 512 columns, a multiple of four, everything 16-byte aligned.
+// 3 rows of 8 heads of 128, behind the kernel ahead: 4.5 -> 2.0 us
+template <typename T, int P>
+__global__ void __launch_bounds__(128) hyb_head_gate4_kernel(T* out, const float* o_raw, int n_rows, int heads, int E, float eps, const float* norm, int norm_per_head,
+                                                             const float* gate, long long ldg, int do_norm, int gate_act) {
+  hyb_pdl_enter();
+  const int idx = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (idx >= n_rows * heads) return;
+  const int r = idx / heads, h = idx - r * heads;
+  float o[P][4], z[P][4], w[P][4];
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < P; i++) {
+    const int e = 4 * lane + 128 * i;
+    const bool in = e < E;
+#pragma unroll
+    for (int k = 0; k < 4; k++) { o[i][k] = z[i][k] = 0.f; w[i][k] = 1.0f; }
+    if (in) hyb_load_vec(o_raw + (size_t)idx * E + e, o[i]);
+    if (in && gate) hyb_load_vec(gate + (size_t)r * ldg + h * E + e, z[i]);
+    if (in && do_norm && norm) hyb_load_vec(norm + (norm_per_head ? h * E + e : e), w[i]);
+  }
+  float inv = 1.0f;
+  if (do_norm) {
+#pragma unroll
+    for (int i = 0; i < 4 * P; i++) ss = fmaf(o[i >> 2][i & 3], o[i >> 2][i & 3], ss);
+    inv = 1.0f / sqrtf(warp_sum(ss) / (float)E + eps);
+  }
+#pragma unroll
+  for (int i = 0; i < P; i++) {
+    const int e = 4 * lane + 128 * i;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const float g = !gate ? 1.0f : gate_act == THA_GATE_SILU ? z[i][k] * hyb_sigmoid(z[i][k]) : hyb_sigmoid(z[i][k]);
+      o[i][k] = (do_norm ? o[i][k] * inv * w[i][k] : o[i][k]) * g;
+    }
+    if (e < E) hyb_store_vec(out + (size_t)idx * E + e, o[i]);
+  }
+}
+template <typename T>
+static int head_gate_launch(cudaStream_t s, T* out, const float* o_raw, int n_rows, int heads, int E, float eps, const float* norm, int norm_per_head, const float* gate,
+                            long long ldg, int do_norm = 1, int gate_act = THA_GATE_SIGMOID) {
+  const bool vec = E % 4 == 0 && E <= 512 && ldg % 4 == 0 && aligned16(out) && aligned16(o_raw) && aligned16(norm) && aligned16(gate);
+  auto k = !vec ? hyb_head_gate_kernel<T> : E <= 128 ? hyb_head_gate4_kernel<T, 1> : E <= 256 ? hyb_head_gate4_kernel<T, 2> : hyb_head_gate4_kernel<T, 4>;
+  THA_CUDA_OK(launch(k, dim3(ceil_div(n_rows * heads, 4)), dim3(128), 0, s, pdl_enabled() != 0, out, o_raw, n_rows, heads, E, eps, norm, norm_per_head, gate, ldg, do_norm,
+                     gate_act));
+  return THA_STATUS_SUCCESS;
+}
+
 // ------------------------------------------------------------------------------------------------------------------
 // short causal convolution + silu; the slot keeps the last taps-1 inputs of every channel (oldest first)
 // ------------------------------------------------------------------------------------------------------------------
@@ -1722,6 +1785,14 @@ extern "C" int tha_hyb_rmsnorm(void* stream, int dtype, void* out, const float* 
                                int n_rows, int width, const int* rows_idx) {
   if (n_rows < 1) return THA_STATUS_SUCCESS;
   const int nt = pick_threads(width / 4);
+  if (width % 4 == 0 && width <= 4096 && aligned16(x) && aligned16(w) && aligned16(out)) {
+    const int parts = ceil_div(width, 4 * nt);
+#define RMS_ROW(T, P) THA_CUDA_OK(launch(hyb_rmsnorm_row_kernel<T, P>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, pdl_enabled() != 0, (T*)out, x, w, w_offset, eps, width, rows_idx))
+    if (dtype == THA_DT_BF16) { if (parts <= 1) RMS_ROW(bf16, 1); else if (parts == 2) RMS_ROW(bf16, 2); else RMS_ROW(bf16, 4); }
+    else { if (parts <= 1) RMS_ROW(float, 1); else if (parts == 2) RMS_ROW(float, 2); else RMS_ROW(float, 4); }
+#undef RMS_ROW
+    return THA_STATUS_SUCCESS;
+  }
   if (dtype == THA_DT_BF16)
     THA_CUDA_OK(launch(hyb_rmsnorm_kernel<bf16>, dim3(n_rows), dim3(nt), 0, (cudaStream_t)stream, pdl_enabled() != 0, (bf16*)out, x, w, w_offset, eps, width, rows_idx));
   else
@@ -1794,14 +1865,9 @@ extern "C" int tha_hyb_linear_heads(void* stream, int dtype, float* C, long long
 extern "C" int tha_hyb_head_gate(void* stream, int dtype, void* out, const float* o_raw, int n_rows, int heads, int E, int do_norm,
                                  float eps, const float* norm, int norm_per_head, const float* gate, long long ldg, int gate_act) {
   if (n_rows < 1) return THA_STATUS_SUCCESS;
-  const dim3 grid(ceil_div(n_rows * heads, 4));
-  if (dtype == THA_DT_BF16)
-    THA_CUDA_OK(launch(hyb_head_gate_kernel<bf16>, grid, dim3(128), 0, (cudaStream_t)stream, pdl_enabled() != 0, (bf16*)out, o_raw, n_rows, heads, E, eps, norm,
-                       norm_per_head, gate, ldg, do_norm, gate_act));
-  else
-    THA_CUDA_OK(launch(hyb_head_gate_kernel<float>, grid, dim3(128), 0, (cudaStream_t)stream, pdl_enabled() != 0, (float*)out, o_raw, n_rows, heads, E, eps, norm,
-                       norm_per_head, gate, ldg, do_norm, gate_act));
-  return THA_STATUS_SUCCESS;
+  cudaStream_t s = (cudaStream_t)stream;
+  return dtype == THA_DT_BF16 ? head_gate_launch(s, (bf16*)out, o_raw, n_rows, heads, E, eps, norm, norm_per_head, gate, ldg, do_norm, gate_act)
+                              : head_gate_launch(s, (float*)out, o_raw, n_rows, heads, E, eps, norm, norm_per_head, gate, ldg, do_norm, gate_act);
 }
 
 // THA_ACT_XIELU: the two stored numbers p, q -> the factors the kernels multiply with
@@ -2074,14 +2140,6 @@ bool tha::hyb_scan_in_registers() {
 static bool scan_pdl(const tha_rows_t* rows) { return rows->max_seq_rows <= 64 && pdl_enabled() != 0; }
 // columns per block of the scans: a power of two that divides the thread count
 static int scan_slice(int vdim) { int sc = 1; while (sc < vdim && sc < 16) sc <<= 1; return sc; }
-
-template <typename T>
-static int head_gate_launch(cudaStream_t s, T* out, const float* o_raw, int n_rows, int heads, int E, float eps, const float* norm,
-                            int norm_per_head, const float* gate, long long ldg) {
-  THA_CUDA_OK(launch(hyb_head_gate_kernel<T>, dim3(ceil_div(n_rows * heads, 4)), dim3(128), 0, s, pdl_enabled() != 0, out, o_raw, n_rows, heads, E, eps, norm,
-                     norm_per_head, gate, ldg, 1, (int)THA_GATE_SIGMOID));
-  return THA_STATUS_SUCCESS;
-}
 
 extern "C" int tha_hyb_mem_scan(void* stream, int dtype, const tha_mem_t* m, const tha_rows_t* rows, const tha_state_store_t* st,
                                 float* proj, long long ldp, float* o_raw, void* out) {

@@ -40,6 +40,39 @@ __device__ __forceinline__ void hyb_store_vec(__nv_bfloat16* p, const float (&v)
   *reinterpret_cast<uint2*>(p) = t;
 }
 
+// A row of a block in registers: P float4 a thread, a block-width apart; elements outside the row are 0
+template <int P>
+struct HybRow { float v[P][4]; };
+template <int P>
+__device__ __forceinline__ HybRow<P> row_load(const float* p, int width) {   // p nullable: zeros
+  HybRow<P> r;
+#pragma unroll
+  for (int i = 0; i < P; i++) {
+    const int c = 4 * (threadIdx.x + i * blockDim.x);
+    if (p && c < width) hyb_load_vec(p + c, r.v[i]);
+    else r.v[i][0] = r.v[i][1] = r.v[i][2] = r.v[i][3] = 0.f;
+  }
+  return r;
+}
+template <int P, typename T>
+__device__ __forceinline__ void row_store(T* p, const HybRow<P>& r, int width) {
+#pragma unroll
+  for (int i = 0; i < P; i++) {
+    const int c = 4 * (threadIdx.x + i * blockDim.x);
+    if (c < width) hyb_store_vec(p + c, r.v[i]);
+  }
+}
+// the sum over the block of f of every element inside the row
+template <int P, typename F>
+__device__ __forceinline__ float row_sum(const HybRow<P>& r, int width, float* red, F f) {
+  float s = 0.f;
+#pragma unroll
+  for (int i = 0; i < P; i++)
+    if (4 * (threadIdx.x + i * blockDim.x) < width)
+#pragma unroll
+      for (int e = 0; e < 4; e++) s = f(s, r.v[i][e]);
+  return block_sum(s, red);
+}
 __device__ __forceinline__ float hyb_softcap(float z, float cap) { return cap * tanhf(z / cap); }
 __device__ __forceinline__ float hyb_logsigmoid(float z) { return fminf(z, 0.f) - log1pf(expf(-fabsf(z))); }
 __device__ __forceinline__ float hyb_sigmoid(float z) { return 1.0f / (1.0f + expf(-z)); }

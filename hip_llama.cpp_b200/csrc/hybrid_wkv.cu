@@ -2,7 +2,7 @@
 //   hyb_token_shift_kernel   every row's mixes with its predecessor, h + (h' - h) * mu, n of them in one pass: the inputs of the grouped
 //                            product (tha_hyb_linear_groups).  The predecessor of a portion's first row is the slot's stored row.
 //   hyb_wkv_decay_kernel     the low-rank decay from end to end: tanh of the W_w1 columns on the way into shared memory, the product with
-//                            W_w2 (fp32 FMA, k ascending), and exp(-exp(. + w0)) on the way out
+//                            W_w2 (fp32 FMA), and exp(-exp(. + w0)) on the way out; hyb_wkv_decay_few_kernel for up to eight rows
 //   the recurrence           hybrid_gla.cu, SCAN_BONUS
 // Mixes are formed from the fp32 norm and rounded once, to the product's number format; decays, state and read-out are fp32 in both
 // number formats.  The head norm, its weight and the silu gate follow in tha_hyb_head_gate.
@@ -100,6 +100,59 @@ __global__ void __launch_bounds__(256) hyb_wkv_decay_kernel(float* __restrict__ 
   }
 }
 
+// The same for few rows: four threads share a channel, sixteen bytes of every 64 of its W2 row each, all asked for before the rows' tanh; R rows at a
+// time.  The tiles above take a barrier and a load latency for every 16 of the rank and fill 1/16 of themselves with 3 rows: rank 64, 1024 channels, 3
+// rows, behind the kernel ahead, 8.3 -> 2.7 us
+constexpr int WD_FEW = 8, WD_RANK = 256;
+__device__ __forceinline__ void wd_load8(const float* p, float (&v)[8]) {
+  const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+__device__ __forceinline__ void wd_load8(const __nv_bfloat16* p, float (&v)[8]) {
+  const uint4 a = *reinterpret_cast<const uint4*>(p);
+  const uint32_t u[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+  for (int i = 0; i < 4; i++) { v[2 * i] = __uint_as_float(u[i] << 16); v[2 * i + 1] = __uint_as_float(u[i] & 0xFFFF0000u); }
+}
+template <typename T>
+__global__ void __launch_bounds__(256) hyb_wkv_decay_few_kernel(float* decay, const float* z, long long ldz, int rank, const T* w2, const float* w0, int n_rows, int n_ch) {
+  hyb_pdl_enter();
+  __shared__ __align__(16) float t[WD_FEW][WD_RANK];
+  const int c = blockIdx.x * 64 + (threadIdx.x >> 2), part = threadIdx.x & 3;
+  constexpr int NI = WD_RANK / 32;
+  float w[NI][8];
+#pragma unroll
+  for (int i = 0; i < NI; i++) {
+    const int k = 32 * i + 8 * part;
+    if (c < n_ch && k < rank) wd_load8(w2 + (size_t)c * rank + k, w[i]);
+    else
+#pragma unroll
+      for (int e = 0; e < 8; e++) w[i][e] = 0.f;
+  }
+  const float bias = c < n_ch ? w0[c] : 0.f;
+  for (int i = threadIdx.x; i < n_rows * rank; i += blockDim.x) {
+    const int r = i / rank;
+    t[r][i - r * rank] = tanhf(z[(size_t)r * ldz + (i - r * rank)]);
+  }
+  __syncthreads();
+  for (int r = 0; r < n_rows; r++) {
+    float acc = 0.f;
+#pragma unroll
+    for (int i = 0; i < NI; i++) {
+      const int k = 32 * i + 8 * part;
+      if (k < rank) {
+        float v[8];
+        wd_load8(&t[r][k], v);
+#pragma unroll
+        for (int e = 0; e < 8; e++) acc = fmaf(v[e], w[i][e], acc);
+      }
+    }
+    acc += __shfl_xor_sync(THA_FULL_MASK, acc, 1);
+    acc += __shfl_xor_sync(THA_FULL_MASK, acc, 2);
+    if (part == 0 && c < n_ch) decay[(size_t)r * n_ch + c] = expf(-expf(acc + bias));
+  }
+}
+
 }  // namespace tha
 
 using namespace tha;
@@ -127,7 +180,14 @@ extern "C" int tha_hyb_wkv_scan(void* stream, int dtype, const tha_wkv_t* g, con
   cudaStream_t s = (cudaStream_t)stream;
   const int R = rows->n_rows, HD = g->heads * g->dim;
   const dim3 grid(ceil_div(HD, WD_T), ceil_div(R, WD_T));
-  if (dtype == THA_DT_BF16)
+  if (R <= WD_FEW && g->rank <= WD_RANK && g->rank % 8 == 0 && aligned16(g->w_w2)) {
+    if (dtype == THA_DT_BF16)
+      THA_CUDA_OK(launch(hyb_wkv_decay_few_kernel<bf16>, dim3(ceil_div(HD, 64)), dim3(256), 0, s, pdl_enabled() != 0, decay, proj + g->o_w1, ldp, g->rank, (const bf16*)g->w_w2,
+                         g->w0, R, HD));
+    else
+      THA_CUDA_OK(launch(hyb_wkv_decay_few_kernel<float>, dim3(ceil_div(HD, 64)), dim3(256), 0, s, pdl_enabled() != 0, decay, proj + g->o_w1, ldp, g->rank, (const float*)g->w_w2,
+                         g->w0, R, HD));
+  } else if (dtype == THA_DT_BF16)
     THA_CUDA_OK(launch(hyb_wkv_decay_kernel<bf16>, grid, dim3(256), 0, s, pdl_enabled() != 0, decay, proj + g->o_w1, ldp, g->rank, (const bf16*)g->w_w2, g->w0, R, HD));
   else
     THA_CUDA_OK(launch(hyb_wkv_decay_kernel<float>, grid, dim3(256), 0, s, pdl_enabled() != 0, decay, proj + g->o_w1, ldp, g->rank, (const float*)g->w_w2, g->w0, R, HD));
