@@ -11,7 +11,7 @@
 // K and V tiles arrive by cp.async, whole rows at a time: V of a tile while its scores are computed, K of the next one under P V -- one
 // buffer each and two barriers per tile.  Bound by fp32 FMA (128 per SM and clock) and the shared-memory reads beside
 // it: per 16 FMAs 1.5 of 128 bits in Q K^T and 1.0 (heads of 128) or 1.5 (of 64) in P V at RI = 8; 2, 1.5 and 2 at RI = 4.
-// The longest tiles start first.
+// The longest tiles start first.  Q8_0 prompts, and fp32 ones that attn_prefill_x3.cu's rule leaves or whose planes get no scratch.
 #include "common.cuh"
 #include "workspace.h"
 

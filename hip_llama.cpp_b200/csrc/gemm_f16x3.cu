@@ -245,7 +245,7 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint64_t xh = tc_smem_desc(tc_smem_u32(xring + s * S::X_STAGE)), xl = xh + (uint64_t)(S::X_PLANE >> 4);
                 const uint32_t ah = tmem + S::COL_A + sa * 64, al = ah + 32;
-  #pragma unroll
+#pragma unroll
                 for (int k = 0; k < X3_BK / 16; k++) {   // K = 16: 8 TMEM columns of A, 32 bytes (2 descriptor units) of B
                   x3_mma(dc, al + 8 * k, xh + (uint64_t)(2 * k), (uint32_t)((i - i0 | k) != 0));
                   x3_mma(dc, ah + 8 * k, xl + (uint64_t)(2 * k), 1u);
@@ -265,141 +265,141 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
   } else if (warp < 4 + X3_CONV_WARPS) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
     for (int pass = 0; pass < 2; pass++) {
-        // ===== converters: every thread takes part in every item's exchange of maxima, whatever became of its waits
-        const int q = warp & 3, r = q * 32 + lane, grp = (warp >> 2) - 1;
-        for (int it = pair; it < p.n_items; it += n_pairs, n_it++) {
-          const Item w = item_of(it);
-          const int i0 = (grp ^ gb) & 1, par = n_it & 3;
-          float m = 0.0f;
-          if (pass == 0) {
-            if (i0 < w.nkb) {
-              const int sw = (gb + i0) % S::SW;
-              if (ok) ok = tc_mbar_wait(&wfull[sw], ((gb + i0) / S::SW) & 1u, abort_flag);
-              if (ok) {
-                const unsigned char* wrow = wring + sw * S::W_STAGE + r * 128;
-  #pragma unroll
-                for (int j = 0; j < 16; j++) {
-                  const float4 v = *reinterpret_cast<const float4*>(wrow + (j >> 3) * (TC_BM * 128) + (((j & 7) ^ (r & 7)) << 4));
-                  m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-                }
+      // ===== converters: every thread takes part in every item's exchange of maxima, whatever became of its waits
+      const int q = warp & 3, r = q * 32 + lane, grp = (warp >> 2) - 1;
+      for (int it = pair; it < p.n_items; it += n_pairs, n_it++) {
+        const Item w = item_of(it);
+        const int i0 = (grp ^ gb) & 1, par = n_it & 3;
+        float m = 0.0f;
+        if (pass == 0) {
+          if (i0 < w.nkb) {
+            const int sw = (gb + i0) % S::SW;
+            if (ok) ok = tc_mbar_wait(&wfull[sw], ((gb + i0) / S::SW) & 1u, abort_flag);
+            if (ok) {
+              const unsigned char* wrow = wring + sw * S::W_STAGE + r * 128;
+#pragma unroll
+              for (int j = 0; j < 16; j++) {
+                const float4 v = *reinterpret_cast<const float4*>(wrow + (j >> 3) * (TC_BM * 128) + (((j & 7) ^ (r & 7)) << 4));
+                m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
               }
             }
-          } else if (w.row0 + r < p.M[w.mat]) {        // the item's share of the whole row
-            const float* wr = p.W[w.mat] + (size_t)(w.row0 + r) * p.K;
-            const int end = min(p.K, (w.kb0 + w.nkb) * X3_BK);
-            for (int k = w.kb0 * X3_BK + 4 * grp; k < end; k += 8) {
-              const float4 v = *reinterpret_cast<const float4*>(wr + k);
-              m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
-            }
           }
-          smax[par][grp][r] = m;
-          asm volatile("bar.sync 1, 256;" ::: "memory");
-          float inverse;
-          const float sc = x3_scale_to(fmaxf(smax[par][0][r], smax[par][1][r]), pass ? 14 : 7, &inverse);
-          if (grp == 0) {
-            rowf[par][r] = inverse;
-            __syncwarp();
-            if (lane == 0) tc_mbar_arrive(&rowready[par]);
+        } else if (w.row0 + r < p.M[w.mat]) {        // the item's share of the whole row
+          const float* wr = p.W[w.mat] + (size_t)(w.row0 + r) * p.K;
+          const int end = min(p.K, (w.kb0 + w.nkb) * X3_BK);
+          for (int k = w.kb0 * X3_BK + 4 * grp; k < end; k += 8) {
+            const float4 v = *reinterpret_cast<const float4*>(wr + k);
+            m = fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
           }
-          __half2 top = __half2half2(__ushort_as_half(0));
-          for (int i = i0; i < w.nkb && ok; i += 2) {
-            const int g = gb + i, sw = g % S::SW, sa = g & 1;
-            ok = tc_mbar_wait(&wfull[sw], (g / S::SW) & 1u, abort_flag);
-            const uint32_t ta = tmem + S::COL_A + sa * 64 + ((uint32_t)(q * 32) << 16);
-  #pragma unroll
-            for (int half = 0; half < 2; half++) {
-              uint32_t hi[16], lo[16];
-              const unsigned char* wrow = wring + sw * S::W_STAGE + half * (TC_BM * 128) + r * 128;
-  #pragma unroll
-              for (int j = 0; j < 8; j++) {            // logical 16-byte chunk j lives at j ^ (row & 7) (SWIZZLE_128B)
-                float4 v = *reinterpret_cast<const float4*>(wrow + ((j ^ (r & 7)) << 4));
-                v.x *= sc; v.y *= sc; v.z *= sc; v.w *= sc;
-                hi[2 * j] = x3_h2(v.x, v.y);
-                hi[2 * j + 1] = x3_h2(v.z, v.w);
-                const __half2 h0 = *reinterpret_cast<__half2*>(&hi[2 * j]), h1 = *reinterpret_cast<__half2*>(&hi[2 * j + 1]);
-                top = __hmax2(top, __hmax2(__habs2(h0), __habs2(h1)));
-                const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
-                lo[2 * j] = x3_h2(v.x - f0.x, v.y - f0.y);
-                lo[2 * j + 1] = x3_h2(v.z - f1.x, v.w - f1.y);
-              }
-              if (half == 0) {
-                if (g >= 2 && ok) ok = tc_mbar_wait(&aempty[sa], ((g >> 1) & 1u) ^ 1u, abort_flag);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-              }
-              x3_tmem_st16(ta + (uint32_t)(16 * half), hi);
-              x3_tmem_st16(ta + (uint32_t)(32 + 16 * half), lo);
-            }
-            __syncwarp();
-            if (lane == 0) tc_mbar_arrive(&wfree[sw]);  // every value has been read and converted
-            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) x3_arrive_leader(&aready[sa]);
-          }
-          if (pass == 0 && (__hisinf(__low2half(top)) || __hisinf(__high2half(top)))) *bad_rows = 1;
-          gb += w.nkb;
         }
+        smax[par][grp][r] = m;
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        float inverse;
+        const float sc = x3_scale_to(fmaxf(smax[par][0][r], smax[par][1][r]), pass ? 14 : 7, &inverse);
+        if (grp == 0) {
+          rowf[par][r] = inverse;
+          __syncwarp();
+          if (lane == 0) tc_mbar_arrive(&rowready[par]);
+        }
+        __half2 top = __half2half2(__ushort_as_half(0));
+        for (int i = i0; i < w.nkb && ok; i += 2) {
+          const int g = gb + i, sw = g % S::SW, sa = g & 1;
+          ok = tc_mbar_wait(&wfull[sw], (g / S::SW) & 1u, abort_flag);
+          const uint32_t ta = tmem + S::COL_A + sa * 64 + ((uint32_t)(q * 32) << 16);
+#pragma unroll
+          for (int half = 0; half < 2; half++) {
+            uint32_t hi[16], lo[16];
+            const unsigned char* wrow = wring + sw * S::W_STAGE + half * (TC_BM * 128) + r * 128;
+#pragma unroll
+            for (int j = 0; j < 8; j++) {            // logical 16-byte chunk j lives at j ^ (row & 7) (SWIZZLE_128B)
+              float4 v = *reinterpret_cast<const float4*>(wrow + ((j ^ (r & 7)) << 4));
+              v.x *= sc; v.y *= sc; v.z *= sc; v.w *= sc;
+              hi[2 * j] = x3_h2(v.x, v.y);
+              hi[2 * j + 1] = x3_h2(v.z, v.w);
+              const __half2 h0 = *reinterpret_cast<__half2*>(&hi[2 * j]), h1 = *reinterpret_cast<__half2*>(&hi[2 * j + 1]);
+              top = __hmax2(top, __hmax2(__habs2(h0), __habs2(h1)));
+              const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
+              lo[2 * j] = x3_h2(v.x - f0.x, v.y - f0.y);
+              lo[2 * j + 1] = x3_h2(v.z - f1.x, v.w - f1.y);
+            }
+            if (half == 0) {
+              if (g >= 2 && ok) ok = tc_mbar_wait(&aempty[sa], ((g >> 1) & 1u) ^ 1u, abort_flag);
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            }
+            x3_tmem_st16(ta + (uint32_t)(16 * half), hi);
+            x3_tmem_st16(ta + (uint32_t)(32 + 16 * half), lo);
+          }
+          __syncwarp();
+          if (lane == 0) tc_mbar_arrive(&wfree[sw]);  // every value has been read and converted
+          asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) x3_arrive_leader(&aready[sa]);
+        }
+        if (pass == 0 && (__hisinf(__low2half(top)) || __hisinf(__high2half(top)))) *bad_rows = 1;
+        gb += w.nkb;
+      }
       if (!again()) break;
     }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
     for (int pass = 0; pass < 2; pass++) {
-        const int q = warp & 3, r = q * 32 + lane, c0 = (X3_NT / 2) * ((warp >> 2) - 1 - X3_CONV_WARPS / 4);
-        pdl_trigger();
-        pdl_wait();                                    // the column scales come from the previous kernel
-        for (int it = pair; it < p.n_items; it += n_pairs, n_it++) {
-          const Item w = item_of(it);
-          const int par = n_it & 3;
-          const uint32_t lanes = (uint32_t)(q * 32) << 16;
-          float sum[X3_NT / 2];
-  #pragma unroll
-          for (int j = 0; j < X3_NT / 2; j++) sum[j] = 0.0f;
-          for (int i0 = 0; i0 < w.nkb; i0 += X3_RUN, n_run++) {
-            const int buf = n_run & 1;
-            if (ok) ok = tc_mbar_wait(&accum[buf], (unsigned)(n_run >> 1) & 1u, abort_flag);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  #pragma unroll
-            for (int part = 0; part < 2; part++) {     // corrections, then the main sum
-              const uint32_t tm = tmem + lanes + (uint32_t)(c0 + (part == 0 ? S::COL_CORR : (buf ? S::COL_MAIN1 : 0)));
-  #pragma unroll
-              for (int c = 0; c < X3_NT / 2; c += 16) {
-                uint32_t v[16];
-                tc_tmem_ld16(tm + (uint32_t)c, v);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-  #pragma unroll
-                for (int j = 0; j < 16; j++) sum[c + j] += __uint_as_float(v[j]);
-              }
-              asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-              __syncwarp();
-              if (lane == 0) x3_arrive_leader(part == 0 ? corrfree : &mainfree[buf]);
+      const int q = warp & 3, r = q * 32 + lane, c0 = (X3_NT / 2) * ((warp >> 2) - 1 - X3_CONV_WARPS / 4);
+      pdl_trigger();
+      pdl_wait();                                    // the column scales come from the previous kernel
+      for (int it = pair; it < p.n_items; it += n_pairs, n_it++) {
+        const Item w = item_of(it);
+        const int par = n_it & 3;
+        const uint32_t lanes = (uint32_t)(q * 32) << 16;
+        float sum[X3_NT / 2];
+#pragma unroll
+        for (int j = 0; j < X3_NT / 2; j++) sum[j] = 0.0f;
+        for (int i0 = 0; i0 < w.nkb; i0 += X3_RUN, n_run++) {
+          const int buf = n_run & 1;
+          if (ok) ok = tc_mbar_wait(&accum[buf], (unsigned)(n_run >> 1) & 1u, abort_flag);
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+          for (int part = 0; part < 2; part++) {     // corrections, then the main sum
+            const uint32_t tm = tmem + lanes + (uint32_t)(c0 + (part == 0 ? S::COL_CORR : (buf ? S::COL_MAIN1 : 0)));
+#pragma unroll
+            for (int c = 0; c < X3_NT / 2; c += 16) {
+              uint32_t v[16];
+              tc_tmem_ld16(tm + (uint32_t)c, v);
+              asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+              for (int j = 0; j < 16; j++) sum[c + j] += __uint_as_float(v[j]);
             }
-          }
-          if (ok) ok = tc_mbar_wait(&rowready[par], (unsigned)(n_it >> 2) & 1u, abort_flag);
-          const float rf = rowf[par][r];
-          const int row = w.row0 + r;
-          if (!ok || row >= p.M[w.mat]) continue;
-          float* o = p.out + (size_t)(it % p.splits) * p.zstride + p.out_off[w.mat] + row + (size_t)(w.n0 + c0) * p.ldo;
-          const int n = w.n0 + c0;
-          if (n + X3_NT / 2 <= p.N) {
-  #pragma unroll
-            for (int j = 0; j < X3_NT / 2; j += 4) {
-              const float4 s4 = *reinterpret_cast<const float4*>(p.colscale + n + j);
-              const float sc[4] = {s4.x, s4.y, s4.z, s4.w};
-  #pragma unroll
-              for (int e = 0; e < 4; e++) {
-                *o = (sum[j + e] * rf) * sc[e];
-                o += p.ldo;
-              }
-            }
-          } else {
-  #pragma unroll
-            for (int j = 0; j < X3_NT / 2; j++)
-              if (n + j < p.N) {
-                *o = (sum[j] * rf) * p.colscale[n + j];
-                o += p.ldo;
-              }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) x3_arrive_leader(part == 0 ? corrfree : &mainfree[buf]);
           }
         }
+        if (ok) ok = tc_mbar_wait(&rowready[par], (unsigned)(n_it >> 2) & 1u, abort_flag);
+        const float rf = rowf[par][r];
+        const int row = w.row0 + r;
+        if (!ok || row >= p.M[w.mat]) continue;
+        float* o = p.out + (size_t)(it % p.splits) * p.zstride + p.out_off[w.mat] + row + (size_t)(w.n0 + c0) * p.ldo;
+        const int n = w.n0 + c0;
+        if (n + X3_NT / 2 <= p.N) {
+#pragma unroll
+          for (int j = 0; j < X3_NT / 2; j += 4) {
+            const float4 s4 = *reinterpret_cast<const float4*>(p.colscale + n + j);
+            const float sc[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+              *o = (sum[j + e] * rf) * sc[e];
+              o += p.ldo;
+            }
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < X3_NT / 2; j++)
+            if (n + j < p.N) {
+              *o = (sum[j] * rf) * p.colscale[n + j];
+              o += p.ldo;
+            }
+        }
+      }
       if (!again()) break;
     }
   }

@@ -4,7 +4,7 @@
 //                                                    X: [N, K] row-major fp32 (N = batch slots or prompt tokens)
 //
 // Used where the GEMV family stops being HBM-bound on CUDA cores: multi-sequence decode with more
-// than 8 slots and batched prefill (replaces thaBLAS_s_matmul_batch,
+// than 4 slots and prefill whose rows or width do not pay for gemm_f16x3.cu (replaces thaBLAS_s_matmul_batch,
 // src/thaBLAS.cpp:191-228, whose grid re-reads every weight row once per slot).
 //
 // Precision: tcgen05 has no fp32 kind.  kind::tf32 reads 32-bit operands and uses 10 mantissa

@@ -16,7 +16,9 @@
 //   gemm          w2  -> partials                                             (src/thaDNN.cpp:69-72)
 // then prep(final norm) -> gemm(wcls) -> logits (-> argmax); prefill runs the classifier only on the last
 // row of each sequence (gathered by the final prep), and its attention is attn_prefill.cu (one pass over the
-// cache per 64 query rows) instead of the per-row decode kernel.
+// cache per 64 query rows) or, fp32 where the step fills it, attn_prefill_x3.cu, instead of the per-row decode kernel.
+// fp32 prompts whose sizes pay for it (rows_f16x3) take the products of gemm_f16x3.cu and its row kernels in the place of gemm, prep and
+// swiglu_split.
 //
 // Split-K partials are summed by their consumer in a fixed order, so the step is bit-reproducible
 // run to run (no floating-point atomics anywhere).
