@@ -332,15 +332,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant_
               *o = x;
               o += p.ldo;
             }
-          } else {
+          } else {   // the last column tile, most prompts': 2000 rows x [2048, 2048] 30.1 -> 26.9 us, 4000 x [1024, 1024] 21.6 -> 18.7 against a multiply an address
+            float* o = outz + (size_t)(w.n0 + c) * p.ldo;
+            const int left = row_ok ? p.N - w.n0 - c : 0;
 #pragma unroll
             for (int j = 0; j < NC; j++) {
-              const int n = w.n0 + c + j;
-              if (n < p.N && row_ok) {
+              if (j < left) {
                 float x = __uint_as_float(v[j]);
-                if (p.colscale) x *= p.colscale[n];
-                outz[(size_t)n * p.ldo] = x;
+                if (p.colscale) x *= p.colscale[w.n0 + c + j];
+                *o = x;
               }
+              o += p.ldo;
             }
           }
         }
