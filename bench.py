@@ -578,7 +578,7 @@ def extra_records(args, device, peak):
         out["prefill_7b_f32_2048"] = {"workload": "Llama-2-7B fp32, one prompt of 2048 positions through tha_prefill_f32 (3xTF32 tensor-core matmuls)",
                                       "ms": ms, "prompt_tok_per_s": T / ms * 1e3, "useful_tflops": flops / ms / 1e9,
                                       "tensor_frac_of_sustained_bf16": flops / ms / 1e9 / tf_peak,
-                                      "note": "useful flops = 2 * T * weights + causal attention; 3xTF32 issues three tf32 MMAs per useful one"}
+                                      "note": "useful flops = 2 * T * weights + causal attention; three fp16 MMAs of split operands per useful one"}
         v, msd = resident_tok_s(e, cfg, 1, 2, 8, device, pos0=T)
         nb = step_bytes(cfg, dw.nbytes(), T + 5, 1)
         out["decode_7b_f32_B1_after_prefill"] = {"workload": "Llama-2-7B fp32 greedy decode, 1 slot, positions 2050..2057", "value": v, "unit": UNIT,
