@@ -575,7 +575,7 @@ def extra_records(args, device, peak):
             tf_peak = float(json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))["bf16_tflops_sustained"])
         except Exception:
             tf_peak = 1381.0
-        out["prefill_7b_f32_2048"] = {"workload": "Llama-2-7B fp32, one prompt of 2048 positions through tha_prefill_f32 (3xTF32 tensor-core matmuls)",
+        out["prefill_7b_f32_2048"] = {"workload": "Llama-2-7B fp32, one prompt of 2048 positions through tha_prefill_f32 (tensor-core matmuls: three fp16 products of split operands)",
                                       "ms": ms, "prompt_tok_per_s": T / ms * 1e3, "useful_tflops": flops / ms / 1e9,
                                       "tensor_frac_of_sustained_bf16": flops / ms / 1e9 / tf_peak,
                                       "note": "useful flops = 2 * T * weights + causal attention; three fp16 MMAs of split operands per useful one"}
