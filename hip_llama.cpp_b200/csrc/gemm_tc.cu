@@ -47,13 +47,14 @@ namespace tha {
 
 // Persistent: a CTA walks the work items (weight tile, column tile, K split) blockIdx.x, blockIdx.x + gridDim.x, ...
 // with running stage counters, so the weight ring keeps streaming while the previous item's accumulator is read out.
-// p stays where the launch put it: its arrays are indexed by matrix, and without __grid_constant__ every thread first copied it to local memory (a step of
-// stories110M at 256 slots 1313 -> 1278 us, of two Llama-2-7B layers at 6 slots 465 -> 449).
+// p's arrays are indexed by constants only: an index at run time made every thread copy p to local memory first (a step of stories110M at 256 slots 1221 us,
+// 1186 now; of two Llama-2-7B layers at 6 slots 455, 432), and __grid_constant__, which spares the copy too, costs launches outside a graph
+// (two prompts of 25 rows, 512 wide, 8 layers: 396 us, 368 without).
 template <int NT>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant__ CUtensorMap mw1,
                    const __grid_constant__ CUtensorMap mw2, const __grid_constant__ CUtensorMap mxh,
-                   const __grid_constant__ CUtensorMap mxl, const __grid_constant__ TcP p) {
+                   const __grid_constant__ CUtensorMap mxl, const TcP p) {
   using S = TcSmem<NT>;
   extern __shared__ unsigned char tc_smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -268,8 +269,8 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constan
       if (n_it == 0 && threadIdx.x == 128) kt_stamp(kt, 4);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int row = w.row0 + r;
-      const bool row_ok = row < p.M[w.mat];
-      float* outz = p.out + (size_t)(it % p.splits) * p.zstride + p.out_off[w.mat] + row;
+      const bool row_ok = row < (w.mat == 0 ? p.M[0] : w.mat == 1 ? p.M[1] : p.M[2]);
+      float* outz = p.out + (size_t)(it % p.splits) * p.zstride + (w.mat == 0 ? p.out_off[0] : w.mat == 1 ? p.out_off[1] : p.out_off[2]) + row;
       if (ok) {
         // Whole tile inside the output (every tile of the model shapes): no per-element bounds checks, the 16 column
         // scales as four 128-bit read-only loads, the store address advanced by one 64-bit add per column.  (The
