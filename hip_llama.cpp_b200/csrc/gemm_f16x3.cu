@@ -57,7 +57,7 @@ struct X3Smem {
   static constexpr int X_PLANE = (X3_NT / 2) * 128;     // 64 rows of 64 halves
   static constexpr int X_STAGE = 2 * X_PLANE;           // hi | lo
   static constexpr int SW = 4, SX = 5;
-  static constexpr int NBARS = 2 * SW + 3 * SX + 2 + 2 + 2 + 2 + 1 + 4;
+  static constexpr int NBARS = 2 * SW + 3 * SX + 2 + 2 + 2 + 2 + 1 + 4 + 4;
   static constexpr int TOTAL = SW * W_STAGE + SX * X_STAGE + 1024 + NBARS * 8 + 64;
   // TMEM columns: main sum 0 | corrections | main sum 1 | two operand slots of 32 (hi) + 32 (lo)
   static constexpr int COL_CORR = 128, COL_MAIN1 = 256, COL_A = 384;
@@ -119,7 +119,8 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
   uint64_t* mainfree = accum + 2;        // [2] rank 0: main sum read out in both CTAs
   uint64_t* corrfree = mainfree + 2;     // rank 0: corrections read out in both CTAs
   uint64_t* rowready = corrfree + 1;     // [4] scales of the weight rows of an item
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(rowready + 4);
+  uint64_t* rowfree = rowready + 4;      // [4] ... and taken by the read-out
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(rowfree + 4);
   int* abort_flag = reinterpret_cast<int*>(tmem_slot + 1);
   int* bad_rows = abort_flag + 1;        // a weight row of this CTA went beyond the scale of its first values
   __shared__ float smax[4][2][TC_BM];    // largest of the first values of a weight row, by converter group; item mod 4
@@ -146,7 +147,7 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
     for (int s = 0; s < S::SX; s++) { tc_mbar_init(&xfull[s], 1); tc_mbar_init(&xpeer[s], 1); tc_mbar_init(&xempty[s], 1); }
     for (int s = 0; s < 2; s++) { tc_mbar_init(&aready[s], 8); tc_mbar_init(&aempty[s], 1); tc_mbar_init(&accum[s], 1); tc_mbar_init(&mainfree[s], 16); }
     tc_mbar_init(corrfree, 16);
-    for (int s = 0; s < 4; s++) tc_mbar_init(&rowready[s], 4);
+    for (int s = 0; s < 4; s++) { tc_mbar_init(&rowready[s], 4); tc_mbar_init(&rowfree[s], 8); }
     *abort_flag = 0;
     *bad_rows = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -297,6 +298,8 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
         float inverse;
         const float sc = x3_scale_to(fmaxf(smax[par][0][r], smax[par][1][r]), pass ? 14 : 7, &inverse);
         if (grp == 0) {
+          // what the MMAs have completed says nothing of the read-out's last step: with a k-block an item these warps are four items ahead of it
+          if (n_it >= 4 && ok) ok = tc_mbar_wait(&rowfree[par], (unsigned)((n_it >> 2) & 1) ^ 1u, abort_flag);
           rowf[par][r] = inverse;
           __syncwarp();
           if (lane == 0) tc_mbar_arrive(&rowready[par]);
@@ -376,6 +379,8 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
         }
         if (ok) ok = tc_mbar_wait(&rowready[par], (unsigned)(n_it >> 2) & 1u, abort_flag);
         const float rf = rowf[par][r];
+        __syncwarp();
+        if (lane == 0) tc_mbar_arrive(&rowfree[par]);
         const int row = w.row0 + r;
         if (!ok || row >= p.M[w.mat]) continue;
         float* o = p.out + (size_t)(it % p.splits) * p.zstride + p.out_off[w.mat] + row + (size_t)(w.n0 + c0) * p.ldo;

@@ -40,8 +40,10 @@ def check(W, X, splits=1, ldo=None):
 
 
 @pytest.mark.parametrize("M,K,N,splits", [(1, 64, 1, 1), (127, 72, 63, 1), (128, 128, 64, 1), (129, 136, 65, 1), (256, 1024, 127, 1), (257, 1032, 128, 1),
-                                          (600, 2056, 129, 2), (513, 4096, 200, 5), (19072, 192, 257, 1), (300, 16384, 3, 1)])
+                                          (600, 2056, 129, 2), (513, 4096, 200, 5), (19072, 192, 257, 1), (300, 16384, 3, 1),
+                                          (32000, 64, 300, 1), (9000, 256, 300, 4), (20000, 72, 600, 1), (20000, 72, 600, 2)])
 def test_product(M, K, N, splits):
+    """Among them shares of one k-block, and more than four items a pair of CTAs: a ring of four scales of weight rows is used again and again."""
     g = torch.Generator(device="cuda").manual_seed(M + K + N)
     W, X = (torch.randn(s, device="cuda", generator=g) for s in ((M, K), (N, K + 8)))
     check(W, X, splits, ldo=M + 5)
