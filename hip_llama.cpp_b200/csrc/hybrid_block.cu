@@ -134,17 +134,17 @@ __global__ void hyb_block_finish_kernel(float* __restrict__ x, const float* __re
 // for at once.  Bound by the latency of one load, two block sums and a store where there are few rows (decoding: 20 to 100 such kernels a
 // step).  3 rows of 1024, behind the kernel ahead: 4.2 -> 1.5 us and 3.5 -> 1.4; 2000 rows: 13 -> 7.7.
 template <int P, typename T>
-__device__ __forceinline__ void row_norm(const HybRow<P>& x, const HybRow<P>& w, const HybRow<P>& b, const tha_norm_t& n, float eps, T* out, int width, float* red) {
+__device__ __forceinline__ void row_norm(const HybRow<P>& x, const HybRow<P>& w, const HybRow<P>& b, const tha_norm_t& n, float eps, T* out, int width, HybRowSum<P>& sm) {
   HybRow<P> y;
   const auto squares = [](float s, float v) { return fmaf(v, v, s); };
   if (n.kind == THA_NORM_LAYER) {
-    const float mean = row_sum(x, width, red, [](float s, float v) { return s + v; }) / (float)width;
-    const float ss = row_sum(x, width, red, [mean](float s, float v) { const float d = v - mean; return fmaf(d, d, s); });
+    const float mean = row_sum(x, width, sm, [](float s, float v) { return s + v; }) / (float)width;
+    const float ss = row_sum(x, width, sm, [mean](float s, float v) { const float d = v - mean; return fmaf(d, d, s); });
     const float inv = 1.0f / sqrtf(ss / (float)width + eps);
 #pragma unroll
     for (int i = 0; i < 4 * P; i++) y.v[i >> 2][i & 3] = fmaf((x.v[i >> 2][i & 3] - mean) * inv, w.v[i >> 2][i & 3], b.v[i >> 2][i & 3]);
   } else if (n.kind == THA_NORM_RMS) {
-    const float inv = 1.0f / sqrtf(row_sum(x, width, red, squares) / (float)width + eps);
+    const float inv = 1.0f / sqrtf(row_sum(x, width, sm, squares) / (float)width + eps);
 #pragma unroll
     for (int i = 0; i < 4 * P; i++) y.v[i >> 2][i & 3] = x.v[i >> 2][i & 3] * inv * (n.w_offset + w.v[i >> 2][i & 3]);
   } else if (n.kind == THA_NORM_DYT) {
@@ -158,12 +158,12 @@ __device__ __forceinline__ void row_norm(const HybRow<P>& x, const HybRow<P>& w,
 
 // no __restrict__: the loads stay behind the wait for the kernel before (pdl_wait)
 template <typename T, int P>
-__global__ void __launch_bounds__(256) hyb_add_norm_row_kernel(float* x, const float* left, const float* left_b, float c_left,
+__global__ void __launch_bounds__(ROW_THREADS) hyb_add_norm_row_kernel(float* x, const float* left, const float* left_b, float c_left,
                                                                const float* right, float c_right, const float* embed_out,
                                                                const float* vec, tha_norm_t n, int has_norm, float eps, T* out,
                                                                long long ldo, int width) {
   hyb_pdl_enter();
-  __shared__ float red[33];
+  __shared__ HybRowSum<P> sm;
   const size_t r = blockIdx.x, at = r * width;
   HybRow<P> v = row_load<P>(x + at, width);
   const HybRow<P> l = row_load<P>(left ? left + at : nullptr, width), lb = row_load<P>(left ? left_b : nullptr, width);
@@ -181,23 +181,23 @@ __global__ void __launch_bounds__(256) hyb_add_norm_row_kernel(float* x, const f
     if (vec) o += pv.v[i >> 2][i & 3];
   }
   row_store(x + at, v, width);
-  if (has_norm) row_norm(v, nw, nb, n, eps, out + r * ldo, width, red);
+  if (has_norm) row_norm(v, nw, nb, n, eps, out + r * ldo, width, sm);
 }
 
 template <typename T, int P>
-__global__ void __launch_bounds__(256) hyb_block_finish_row_kernel(float* x, const float* ff, const float* ff_b,
+__global__ void __launch_bounds__(ROW_THREADS) hyb_block_finish_row_kernel(float* x, const float* ff, const float* ff_b,
                                                                    const float* y, float m, const float* w, float eps,
                                                                    float* tap, const float* embed_out, const float* vec,
                                                                    tha_norm_t n, int has_norm, T* out, long long ldo, int width) {
   hyb_pdl_enter();
-  __shared__ float red[33];
+  __shared__ HybRowSum<P> sm;
   const size_t r = blockIdx.x, at = r * width;
   HybRow<P> v = row_load<P>(x + at, width);
   const HybRow<P> f = row_load<P>(ff ? ff + at : nullptr, width), fb = row_load<P>(ff ? ff_b : nullptr, width);
   const HybRow<P> s = row_load<P>(y ? y + at : nullptr, width), sw = row_load<P>(y ? w : nullptr, width), e = row_load<P>(embed_out ? embed_out + at : nullptr, width);
   const HybRow<P> pv = row_load<P>(vec, width), nw = row_load<P>(has_norm ? n.w : nullptr, width), nb = row_load<P>(has_norm ? n.b : nullptr, width);
   float inv = 0.f;
-  if (y) inv = m / sqrtf(row_sum(s, width, red, [](float a, float b) { return fmaf(b, b, a); }) / (float)width + eps);
+  if (y) inv = m / sqrtf(row_sum(s, width, sm, [](float a, float b) { return fmaf(b, b, a); }) / (float)width + eps);
 #pragma unroll
   for (int i = 0; i < 4 * P; i++) {
     float& o = v.v[i >> 2][i & 3];
@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(256) hyb_block_finish_row_kernel(float* x, con
     if (vec) v.v[i >> 2][i & 3] += pv.v[i >> 2][i & 3];
   }
   row_store(x + at, v, width);
-  if (has_norm) row_norm(v, nw, nb, n, eps, out + r * ldo, width, red);
+  if (has_norm) row_norm(v, nw, nb, n, eps, out + r * ldo, width, sm);
 }
 
 // V channels per thread and step (4: width a multiple of four); the row of y waits in shared memory for its root mean square
@@ -281,7 +281,13 @@ __global__ void __launch_bounds__(256) hyb_post_norm_row_kernel(float* x, const 
 #pragma unroll
     for (int i = 0; i < 4 * P; i++) y.v[i >> 2][i & 3] = fmaf(w, d.v[i >> 2][i & 3], y.v[i >> 2][i & 3]);
   }
-  const float f = m / sqrtf(row_sum(y, width, red, [](float s, float a) { return fmaf(a, a, s); }) / (float)width + eps);
+  float ss = 0.f;                                     // four neighbouring channels after another, as above
+#pragma unroll
+  for (int i = 0; i < P; i++)
+    if (4 * (threadIdx.x + i * blockDim.x) < width)
+#pragma unroll
+      for (int e = 0; e < 4; e++) ss = fmaf(y.v[i][e], y.v[i][e], ss);
+  const float f = m / sqrtf(block_sum(ss, red) / (float)width + eps);
 #pragma unroll
   for (int i = 0; i < 4 * P; i++) v.v[i >> 2][i & 3] = fmaf(y.v[i >> 2][i & 3] * f, n.w_offset + nw.v[i >> 2][i & 3], v.v[i >> 2][i & 3]);
   row_store(x + at, v, width);

@@ -38,13 +38,13 @@ __global__ void hyb_rmsnorm_kernel(T* __restrict__ out, const float* __restrict_
 // the same with the row in registers: widths of up to 4096 that are a multiple of four, 16-byte aligned.  Bound by latency: 3 rows of 1024, behind the kernel
 // ahead, 2.9 -> 1.8 us
 template <typename T, int P>
-__global__ void __launch_bounds__(256) hyb_rmsnorm_row_kernel(T* out, const float* x, const float* w, float w_offset, float eps, int width, const int* rows_idx) {
+__global__ void __launch_bounds__(ROW_THREADS) hyb_rmsnorm_row_kernel(T* out, const float* x, const float* w, float w_offset, float eps, int width, const int* rows_idx) {
   hyb_pdl_enter();
-  __shared__ float red[33];
+  __shared__ HybRowSum<P> sm;
   const int r = blockIdx.x;
   const HybRow<P> nw = row_load<P>(w, width);
   HybRow<P> v = row_load<P>(x + (size_t)(rows_idx ? rows_idx[r] : r) * width, width);
-  const float inv = 1.0f / sqrtf(row_sum(v, width, red, [](float s, float a) { return fmaf(a, a, s); }) / (float)width + eps);
+  const float inv = 1.0f / sqrtf(row_sum(v, width, sm, [](float s, float a) { return fmaf(a, a, s); }) / (float)width + eps);
 #pragma unroll
   for (int i = 0; i < 4 * P; i++) v.v[i >> 2][i & 3] = v.v[i >> 2][i & 3] * inv * (w_offset + nw.v[i >> 2][i & 3]);
   row_store(out + (size_t)r * width, v, width);
@@ -363,7 +363,8 @@ __global__ void hyb_attn_prepare_kernel(tha_attn_t a, tha_rows_t rows, tha_kv_t 
 
 // The same for heads of up to 128 channels whose places are multiples of four floats (hyb_attn_prepare_ok): a lane has four neighbouring channels, 128-bit loads and stores.
 // Where a row's cache line lies -- three dependent loads -- is looked up ahead of the wait for the projections inside tha_hyb_step (`early`), where rows and table are
-// in place before the step's first kernel starts.  Bound by bytes for prompts, by the chain of loads when decoding.
+// in place before the step's first kernel starts.  Bound by bytes for prompts, by the chain of loads when decoding.  Squares are added in the order of the kernel
+// above: a head's by the lanes that would have its channels there, a row's by as many threads.
 __device__ __forceinline__ float4 hyb_scale4(float4 v, float f) { return make_float4(v.x * f, v.y * f, v.z * f, v.w * f); }
 __device__ __forceinline__ float4 hyb_ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 template <int THREADS>   // at most
@@ -375,6 +376,7 @@ __global__ void __launch_bounds__(THREADS, 1280 / THREADS) hyb_attn_prepare4_ker
   const int r = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5, c = 4 * lane;
   const int t = rows.pos[r], slot = rows.seq_slot[rows.row_seq[r]];
+  __shared__ __align__(16) float head[THREADS / 32][128];
   const size_t krow = hyb_kv_row(kv, slot, t, a.cache_layer);
   const size_t mrow = a.v_mix ? hyb_kv_row(kv, slot, t, a.v_mix_layer) : 0;
   if (early) pdl_wait();
@@ -385,14 +387,15 @@ __global__ void __launch_bounds__(THREADS, 1280 / THREADS) hyb_attn_prepare4_ker
   float row_q = 1.0f, row_k = 1.0f;
   if (!a.head_norm && (a.q_norm || a.k_norm)) {
     __shared__ float red[33];
+    const int nt = min((int)blockDim.x, 256);
     if (a.q_norm) {
       float ss = 0.f;
-      for (int i = 4 * threadIdx.x; i < a.heads * a.dim; i += 4 * blockDim.x) { const float4 v = hyb_ld4(pr + a.o_q + i); ss = dot4(v, v, ss); }
+      for (int i = threadIdx.x; i < a.heads * a.dim && (int)threadIdx.x < nt; i += nt) { const float v = pr[a.o_q + i]; ss = fmaf(v, v, ss); }
       row_q = 1.0f / sqrtf(block_sum(ss, red) / (float)(a.heads * a.dim) + a.eps);
     }
     if (a.k_norm && n_k) {
       float ss = 0.f;
-      for (int i = 4 * threadIdx.x; i < a.kv_heads * a.dim; i += 4 * blockDim.x) { const float4 v = hyb_ld4(pr + a.o_k + i); ss = dot4(v, v, ss); }
+      for (int i = threadIdx.x; i < a.kv_heads * a.dim && (int)threadIdx.x < nt; i += nt) { const float v = pr[a.o_k + i]; ss = fmaf(v, v, ss); }
       row_k = 1.0f / sqrtf(block_sum(ss, red) / (float)(a.kv_heads * a.dim) + a.eps);
     }
   }
@@ -418,7 +421,7 @@ __global__ void __launch_bounds__(THREADS, 1280 / THREADS) hyb_attn_prepare4_ker
     const int pc = halves && turn ? (first ? c + half : c - half) : c;     // where the partners of these channels lie
     float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
     if (in) { x = hyb_ld4(src + c); y = hyb_ld4(src + pc); }
-    float ss = dot4(x, x, 0.f);
+    float4 sq = x;                                   // whose squares are the head's norm
     if (in && wn) {
       const float4 wx = make_float4(wn[c], wn[c + 1], wn[c + 2], wn[c + 3]), wy = make_float4(wn[pc], wn[pc + 1], wn[pc + 2], wn[pc + 3]);
       x = make_float4(x.x * wx.x, x.y * wx.y, x.z * wx.z, x.w * wx.w);
@@ -429,16 +432,25 @@ __global__ void __launch_bounds__(THREADS, 1280 / THREADS) hyb_attn_prepare4_ker
       const float *cr = cos_t + (size_t)r * half, *sr = sin_t + (size_t)r * half;
       if (halves) {
         const int i = first ? c : c - half;
-        const float s = first ? -1.0f : 1.0f;
-        v = make_float4(x.x * cr[i] + s * (y.x * sr[i]), x.y * cr[i + 1] + s * (y.y * sr[i + 1]), x.z * cr[i + 2] + s * (y.z * sr[i + 2]), x.w * cr[i + 3] + s * (y.w * sr[i + 3]));
+        if (first) v = make_float4(x.x * cr[i] - y.x * sr[i], x.y * cr[i + 1] - y.y * sr[i + 1], x.z * cr[i + 2] - y.z * sr[i + 2], x.w * cr[i + 3] - y.w * sr[i + 3]);
+        else v = make_float4(x.x * cr[i] + y.x * sr[i], x.y * cr[i + 1] + y.y * sr[i + 1], x.z * cr[i + 2] + y.z * sr[i + 2], x.w * cr[i + 3] + y.w * sr[i + 3]);
       } else {
         const int i = c >> 1;
         v = make_float4(x.x * cr[i] - x.y * sr[i], x.y * cr[i] + x.x * sr[i], x.z * cr[i + 1] - x.w * sr[i + 1], x.w * cr[i + 1] + x.z * sr[i + 1]);
       }
     }
-    if (a.unit_rms && !a.head_norm) ss = dot4(v, v, 0.f);
     float inv = is_q ? q_mult * row_q : row_k;
-    if (a.unit_rms || a.head_norm) inv = 1.0f / sqrtf(warp_sum(ss) / (float)a.dim + a.eps) * inv;
+    if (a.unit_rms || a.head_norm) {
+      if (!a.head_norm) sq = v;
+      if (in) *reinterpret_cast<float4*>(&head[warp][c]) = sq;
+      __syncwarp();
+      float ss = 0.f;
+#pragma unroll
+      for (int d = lane; d < 128; d += 32)
+        if (d < a.dim) ss = fmaf(head[warp][d], head[warp][d], ss);
+      inv = 1.0f / sqrtf(warp_sum(ss) / (float)a.dim + a.eps) * inv;
+      __syncwarp();                                  // read, before the next head
+    }
     if (in) *reinterpret_cast<float4*>(dst + c) = hyb_scale4(v, inv);
   }
 }
@@ -1357,8 +1369,8 @@ __global__ void hyb_head_gate_kernel(T* __restrict__ out, const float* __restric
   }
 }
 
-// the same with a head's columns in registers, four of every 128 a lane: heads of up to 512 columns, a multiple of four, everything 16-byte aligned.
-// 3 rows of 8 heads of 128, behind the kernel ahead: 4.5 -> 2.0 us
+// the same with a head's columns in registers, four of every 128 a lane: heads of up to 512 columns, a multiple of four, everything 16-byte aligned.  The squares
+// change hands to be added in the same order.  3 rows of 8 heads of 128, behind the kernel ahead: 4.5 -> 2.0 us
 template <typename T, int P>
 __global__ void __launch_bounds__(128) hyb_head_gate4_kernel(T* out, const float* o_raw, int n_rows, int heads, int E, float eps, const float* norm, int norm_per_head,
                                                              const float* gate, long long ldg, int do_norm, int gate_act) {
@@ -1366,8 +1378,8 @@ __global__ void __launch_bounds__(128) hyb_head_gate4_kernel(T* out, const float
   const int idx = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (idx >= n_rows * heads) return;
   const int r = idx / heads, h = idx - r * heads;
+  __shared__ __align__(16) float head[4][128 * P];
   float o[P][4], z[P][4], w[P][4];
-  float ss = 0.f;
 #pragma unroll
   for (int i = 0; i < P; i++) {
     const int e = 4 * lane + 128 * i;
@@ -1380,8 +1392,15 @@ __global__ void __launch_bounds__(128) hyb_head_gate4_kernel(T* out, const float
   }
   float inv = 1.0f;
   if (do_norm) {
+    float* hv = head[threadIdx.x >> 5];
 #pragma unroll
-    for (int i = 0; i < 4 * P; i++) ss = fmaf(o[i >> 2][i & 3], o[i >> 2][i & 3], ss);
+    for (int i = 0; i < P; i++)
+      if (4 * lane + 128 * i < E) hyb_store_vec(hv + 4 * lane + 128 * i, o[i]);
+    __syncwarp();
+    float ss = 0.f;
+#pragma unroll
+    for (int e = lane; e < 128 * P; e += 32)
+      if (e < E) ss = fmaf(hv[e], hv[e], ss);
     inv = 1.0f / sqrtf(warp_sum(ss) / (float)E + eps);
   }
 #pragma unroll

@@ -62,16 +62,22 @@ __device__ __forceinline__ void row_store(T* p, const HybRow<P>& r, int width) {
     if (c < width) hyb_store_vec(p + c, r.v[i]);
   }
 }
-// the sum over the block of f of every element inside the row
+// The sum over the block of f of every element inside the row, in the order of the kernels that take a row element by element (a thread's are a block-width
+// apart), so that a row has the same bits whichever form its width and alignment choose.  The row changes hands through shared memory; up to 256 threads.
+constexpr int ROW_THREADS = 256;
+template <int P>
+struct HybRowSum { alignas(16) float row[4 * P * ROW_THREADS]; float red[33]; };
 template <int P, typename F>
-__device__ __forceinline__ float row_sum(const HybRow<P>& r, int width, float* red, F f) {
+__device__ __forceinline__ float row_sum(const HybRow<P>& r, int width, HybRowSum<P>& sm, F f) {
+  row_store(sm.row, r, width);
+  __syncthreads();
   float s = 0.f;
 #pragma unroll
-  for (int i = 0; i < P; i++)
-    if (4 * (threadIdx.x + i * blockDim.x) < width)
-#pragma unroll
-      for (int e = 0; e < 4; e++) s = f(s, r.v[i][e]);
-  return block_sum(s, red);
+  for (int k = 0; k < 4 * P; k++) {
+    const int i = threadIdx.x + k * blockDim.x;
+    if (i < width) s = f(s, sm.row[i]);
+  }
+  return block_sum(s, sm.red);                        // its first barrier ends the reading of the row
 }
 __device__ __forceinline__ float hyb_softcap(float z, float cap) { return cap * tanhf(z / cap); }
 __device__ __forceinline__ float hyb_logsigmoid(float z) { return fminf(z, 0.f) - log1pf(expf(-fabsf(z))); }
