@@ -268,7 +268,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant_
         // both accumulators of this thread's row; warps 4-7 take the first half of the columns, 8-11 the second
         const int srow = w.row0 + r;
         const uint32_t ta = tmem_base + (uint32_t)(buf * MT * NT) + ((uint32_t)(q * 32) << 16);
-        if (ok && srow < p.M[0]) {
+        const int cols = srow < p.M[0] ? p.N - w.n0 : 0;        // of this row that are stored; the loads are the whole warp's
+        if (ok) {
           uint16_t* o = p.act_out + (size_t)(w.n0 + mt * (NT / 2)) * p.ld_act + srow;
 #pragma unroll 1
           for (int c = mt * (NT / 2); c < (mt + 1) * (NT / 2); c += 16) {
@@ -278,7 +279,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant_
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
             for (int j = 0; j < 16; j++) {
-              if (w.n0 + c + j < p.N) {
+              if (c + j < cols) {
                 float h = __uint_as_float(va[j]);
                 h *= (1.0f / (1.0f + expf(-h)));
                 h *= __uint_as_float(vc[j]);

@@ -13,6 +13,7 @@ earlier layer's K/V rows carry a flip forward, most rows agree to fp32 noise; th
 moved by -1 / 0 / +1 ulp: it produces the same 3e-3 .. 7e-3 jumps) is printed beside each result."""
 import numpy as np
 import pytest
+import torch
 
 from gpu_util import assert_close_scaled, small_model_files
 from pkgload import load_pkg
@@ -196,3 +197,22 @@ def test_bf16_stories110m_shape(oracle, tmp_path):
                                  sample=list(range(min(B, 6))))
         check_ratios(r, fl, f"bf16 stories110M shape B={B}")
         del e
+
+
+@pytest.mark.parametrize("hidden", [96, 1000, 1016, 1024])
+def test_prompt_feed_forward_of_a_ragged_width(hidden):
+    """SwiGLU in the read-out of the first product (512 rows on) where the last warp has rows behind the matrix: the second layer's cache rows, to the bit, against a
+    prompt of the first 400 rows, whose product and activation are two kernels."""
+    eng, ck = load_pkg("engine"), load_pkg("checkpoint")
+    cfg = ck.Config(128, hidden, 2, 2, 2, 96, 640)
+    w = eng.DeviceWeightsBF16.random(cfg, seed=7)
+    toks = np.random.default_rng(8).integers(0, 96, 600).astype(np.int32)
+    rows = []
+    for n in (600, 400):
+        e = eng.Engine(w, 1, with_att=False)
+        out = torch.empty(1, 96, device="cuda")
+        torch.cuda.synchronize()
+        e.prefill([(0, 0, toks[:n])], out)
+        torch.cuda.synchronize()
+        rows.append(torch.stack([e.state.key_cache[0, 1, :384], e.state.value_cache[0, 1, :384]]).clone())
+    assert torch.isfinite(rows[0]).all() and torch.equal(*rows)
