@@ -118,7 +118,7 @@ __global__ void __launch_bounds__(256) x3_rope_kernel(const float* part, int nz,
 __global__ void __launch_bounds__(256) x3_context_kernel(const float* kc, const float* vc, long long kv_bs, const int* seq_slot,
                                                          const int* upto, const int* base, const KvPaged pg, int kvd, int hs, const X3Staged st) {
   pdl_trigger();
-  pdl_wait();                                        // the planes of the layer before have been read
+  pdl_wait();                                        // the call's own rows are in the cache
   const int i = blockIdx.z, n = upto[i], slot = seq_slot[i], li = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
   for (int t = blockIdx.y; t < n; t += gridDim.y) {
     const long long off = pg.table ? kv_paged_off(pg, slot, t, kvd) : (long long)slot * kv_bs + (long long)t * kvd;

@@ -1082,10 +1082,11 @@ static int issue_rows(cudaStream_t st, Workspace* ws, const tha_config_t& c, con
     const bool rope_in_attn = io.n_tiles == 0 && !(!io.logits && l == L - 1) && !(skip & 2) && rope_fuse_mode() &&
                               attn_fused_rope_supported(c.n_heads, c.n_kv_heads, hs);
     if (io.staged && !(skip & 8)) {
-      if (io.n_ctx)
-        THA_TRY_RC(x3_context_launch(st, pdl, io.n_ctx, io.longest_ctx, kcl, vcl, kv_bs, io.seq_slot, io.seq_upto, io.seq_base, pg, kvd, hs, *io.staged));
+      // contexts behind the call's own rows: one portion's may hold another's (two portions of a slot, block tables that share a block)
       THA_TRY_RC(x3_rope_launch(st, pdl, R, sc.part, pl.z_qkv, (long long)R * ld_qkv, ld_qkv, io.pos, da, kvd, hs, rc, rs, s.key_cache, s.value_cache, kv_bs, loff, io.slot,
                                 pg, *io.staged));
+      if (io.n_ctx)
+        THA_TRY_RC(x3_context_launch(st, pdl, io.n_ctx, io.longest_ctx, kcl, vcl, kv_bs, io.seq_slot, io.seq_upto, io.seq_base, pg, kvd, hs, *io.staged));
     } else if (!(skip & 8) && !rope_in_attn)
     THA_CUDA_OK(launch(tc_rope_scatter_kernel, dim3(ceil_div(ld_qkv / 4, 512), R), dim3(256), 0, st, pdl, (const float*)sc.part,
                        pl.z_qkv, (long long)R * ld_qkv, ld_qkv, io.pos, da, kvd, hs, rc, rs, io.q, s.key_cache, s.value_cache,
