@@ -9,8 +9,9 @@
 // rows to a ring of three tiles in shared memory of its own (cp.async), so that a usual run is in flight at once; eight lanes share a key (a lane:
 // four channels of every 32); the running maximum, sum and accumulator live in registers per group of eight lanes and meet only at the end of
 // the run.  Nothing is rounded: q, keys, values and weights stay fp32 in both number formats.
-// Inside a step the rows of all keys but the newest are there before the kernel ahead is done (it writes the newest), so they are asked for
-// ahead of the wait for it; the distance bias is asked for with a tile and not score by score.
+// Inside a step of single rows all keys but those that the step itself writes are there before the kernel ahead is done, so they are asked for ahead of
+// the wait for it.  What the step writes is one row a sequence: the row's own key, and the key of another sequence where a caller gives two of them one slot or one
+// block.  The distance bias is asked for with a tile and not score by score.
 // Bound by the latency of what follows that wait (q, the newest key, three tiles' arithmetic, the meeting of the warps), and by the cache rows it
 // reads where there are many.  16 heads on 4 of 128 channels, 2 rows at 1100 .. 2900, behind the kernel ahead: tiles loaded to registers one by
 // one 15.2 us; the ring, ahead of the wait 11.4; the bias with the tile 9.0; all heads' scores before their sums 8.4.
@@ -53,19 +54,21 @@ __global__ void __launch_bounds__(AR_THREADS) hyb_attn_row_kernel(tha_attn_t a, 
   const HybTiles tiles = hyb_attn_tiles(a, first, p, p);
   const int per = (tiles.n + splits - 1) / splits, ti0 = sp * per, ti_end = min(tiles.n, ti0 + per);
   auto tile_key = [&](int ti) { return (ti < tiles.n_a ? tiles.begin + 32 * ti : tiles.resume + 32 * (ti - tiles.n_a)) + 8 * warp; };
-  // the warp's eight keys of a tile on their way to its place in the ring: lanes 0..7 look their rows up, key 4 j + kq then goes to lanes
-  // kq * 8 ..; `newest`: key p, whose row the kernel ahead writes, or all the others
+  // cache row of this lane's key (lane & 7) of the warp's eight of a tile
+  auto row_of = [&](int ti) {
+    const int mine = tile_key(ti) + (lane & 7);
+    return (mine <= p && mine >= first) ? hyb_kv_row(kv, slot, mine, a.cache_layer) : (size_t)-1;
+  };
+  // those keys that `take` has a bit of on their way to the tile's place in the ring: key 4 j + kq goes to lanes kq * 8 ..
   float* ring = ar_ring + (size_t)warp * AR_STAGES * 8 * (D + E);
-  auto fetch = [&](int ti, bool others, bool newest) {
-    const int kt = tile_key(ti), mine = kt + (lane & 7);
-    if (newest && !others && (p < kt || p >= kt + 8)) return;
-    const size_t row = (mine <= p && mine >= first) ? hyb_kv_row(kv, slot, mine, a.cache_layer) : (size_t)-1;
+  auto fetch = [&](int ti, size_t row, unsigned take) {
+    const int kt = tile_key(ti);
     float* st = ring + (size_t)((ti - ti0) % AR_STAGES) * 8 * (D + E);
 #pragma unroll
     for (int j = 0; j < 2; j++) {
       const int key = kt + 4 * j + kq;
       const size_t at = __shfl_sync(THA_FULL_MASK, row, 4 * j + kq);
-      if (!(key == p ? newest : others)) continue;
+      if (!(take >> (4 * j + kq) & 1u)) continue;
       const bool vis = at != (size_t)-1 && hyb_attn_sees(a, key, p, first);
       const float *kp = kv.k_pool + (vis ? at : 0) + (size_t)g * D + c4, *vp = kv.v_pool + (vis ? at : 0) + (size_t)gv * E + c4;
       float* dst = st + (4 * j + kq) * (D + E) + c4;
@@ -76,11 +79,35 @@ __global__ void __launch_bounds__(AR_THREADS) hyb_attn_row_kernel(tha_attn_t a, 
       }
     }
   };
-  const int ti_ring = min(ti_end, ti0 + AR_STAGES);
-  for (int ti = ti0; ti < ti_ring; ti++) fetch(ti, true, !early);
+  size_t row[AR_STAGES];
+  unsigned late[AR_STAGES];                        // of the tile's eight keys those whose rows this step writes
+#pragma unroll
+  for (int i = 0; i < AR_STAGES; i++) row[i] = ti0 + i < ti_end ? row_of(ti0 + i) : (size_t)-1;
+  if (early) {
+    bool mine[AR_STAGES] = {};
+    for (int r0 = 0; r0 < rows.n_rows; r0 += 32) {
+      const int o = min(r0 + lane, rows.n_rows - 1);
+      const size_t written = hyb_kv_row(kv, rows.seq_slot[rows.row_seq[o]], rows.pos[o], a.cache_layer);
+      for (int j = 0; j < min(32, rows.n_rows - r0); j++) {
+        const size_t w = __shfl_sync(THA_FULL_MASK, written, j);
+#pragma unroll
+        for (int i = 0; i < AR_STAGES; i++) mine[i] |= w == row[i];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < AR_STAGES; i++) late[i] = __ballot_sync(THA_FULL_MASK, mine[i]) & 0xFFu;
+  } else {
+#pragma unroll
+    for (int i = 0; i < AR_STAGES; i++) late[i] = 0u;
+  }
+#pragma unroll
+  for (int i = 0; i < AR_STAGES; i++)
+    if (ti0 + i < ti_end) fetch(ti0 + i, row[i], ~late[i]);
   if (early) {
     pdl_wait();
-    for (int ti = ti0; ti < ti_ring; ti++) fetch(ti, false, true);
+#pragma unroll
+    for (int i = 0; i < AR_STAGES; i++)
+      if (late[i]) fetch(ti0 + i, row[i], late[i]);
   }
   ar_commit();
   float4 qv[GS][NI], acc[GS][NI];
@@ -159,7 +186,7 @@ __global__ void __launch_bounds__(AR_THREADS) hyb_attn_row_kernel(tha_attn_t a, 
       }
     }
     __syncwarp();
-    if (ti + AR_STAGES < ti_end) fetch(ti + AR_STAGES, true, true);
+    if (ti + AR_STAGES < ti_end) fetch(ti + AR_STAGES, row_of(ti + AR_STAGES), ~0u);
     ar_commit();
   }
   // the four key groups of a warp, then the four warps
@@ -231,7 +258,7 @@ static int row_launch_heads(cudaStream_t s, const tha_attn_t* a, const tha_rows_
   const int ring = 4 * AR_STAGES * 8 * (a->dim + a->vdim) * (int)sizeof(float);
   THA_CUDA_OK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, ring));
   THA_CUDA_OK(launch(k, dim3(rows->n_seqs * splits, a->kv_heads, groups), dim3(AR_THREADS), ring, s, pdl_enabled() != 0, *a, *rows, *kv, q, out, splits, partial,
-                     gate, ldg, (int)hyb_gemm_pdl()));
+                     gate, ldg, (int)(hyb_gemm_pdl() && rows->max_seq_rows == 1)));
   return THA_STATUS_SUCCESS;
 }
 template <typename T>
