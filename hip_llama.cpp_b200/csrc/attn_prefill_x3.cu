@@ -1,19 +1,19 @@
-// Causal attention of fp32 prompts on the tensor cores: Q K^T and P V as three fp16 products each of operands split in two (gemm_f16x3.cu has the
-// scheme), softmax in fp32 between them, one pass over the keys as in attn_prefill.cu.
+// Causal attention of fp32 prompts on the tensor cores: Q K^T and P V as three fp16 products each of operands split in two (split_f16.cuh), softmax in fp32 between them, one pass over the keys as in attn_prefill.cu.
 //
 // x3_rope_kernel, which rotates q and k and fills the cache, leaves q, k and v of the call's rows as two fp16 planes besides, each (row, head) brought
 // to [2^14, 2^15) by a power of two of its own; x3_context_kernel those of earlier positions.  A score is the product times the two inverse scales.  V's belong to
-// the keys, so they go into the weights: a weight p becomes p vs / c, c the largest inverse scale of the tile, before it is split, and the tile's P V is multiplied
-// by c where it joins the accumulator in registers.  The corrections (hi.lo, lo.hi) of a product are summed ahead of hi.hi, while the sum is small.
+// the keys, so they go into the weights: a weight p becomes p vs / c, c the largest inverse scale of the tile's keys that the row sees, before it is split, and the row's P V
+// of the tile is multiplied by c where it joins the accumulator in registers.  The corrections (hi.lo, lo.hi) of a product are summed ahead of hi.hi, which takes their sum
+// over times 2^-11 (the MMA's scale of its input D).
 //
 // CTA = 128 consecutive query rows of one (sequence, head), 256 threads, two a row (attn_prefill_tc.cu); tiles of 128 keys.  A chain
 // of S, softmax, P V and accumulator, in which the next tile's loads and its S run ahead; heads of 64 have two CTAs an SM (96 KB), of 128 one (192 KB).  Bound by the
 // softmax threads (some 20 instructions a score) and, at one CTA an SM, by the chain.
 #include <cuda.h>
-#include <cuda_fp16.h>
 
 #include "common.cuh"
 #include "gemm_tc.h"
+#include "split_f16.cuh"
 #include "tc_common.cuh"
 #include "workspace.h"
 
@@ -29,26 +29,10 @@ struct AttnX3P {
   int* error_flag;
 };
 
-__device__ __forceinline__ uint32_t ax_h2(float a, float b) {   // a in the low half, nearest even
-  uint32_t r;
-  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
-  return r;
-}
-__device__ __forceinline__ float2 ax_f2(uint32_t h) { return __half22float2(*reinterpret_cast<const __half2*>(&h)); }
 // The power of two that brings |v| to [2^14, 2^15) and its inverse.  At most 2^100: the ratio of two inverse scales stays finite.
-__device__ __forceinline__ float ax_scale(float v, float* inverse) {
-  const int s = min(268 - (int)(__float_as_uint(v) >> 23), 227);
-  *inverse = __uint_as_float((uint32_t)(254 - s) << 23);
-  return __uint_as_float((uint32_t)s << 23);
-}
+__device__ __forceinline__ float ax_scale(float v, float* inverse) { return split_scale<100>(v, 14, inverse); }
 __device__ __forceinline__ void ax_planes(float4 v, float s, uint16_t* hi, uint16_t* lo) {
-  v.x *= s; v.y *= s; v.z *= s; v.w *= s;
-  uint2 h, l;
-  h.x = ax_h2(v.x, v.y); h.y = ax_h2(v.z, v.w);
-  const float2 a = ax_f2(h.x), b = ax_f2(h.y);
-  l.x = ax_h2(v.x - a.x, v.y - a.y); l.y = ax_h2(v.z - b.x, v.w - b.y);
-  *reinterpret_cast<uint2*>(hi) = h;
-  *reinterpret_cast<uint2*>(lo) = l;
+  split_f16x4(v, s, *reinterpret_cast<uint2*>(hi), *reinterpret_cast<uint2*>(lo));
 }
 // Largest |value| of the head that this lane's four values belong to: hs / 4 neighbouring lanes
 __device__ __forceinline__ float ax_head_max(float4 v, int hs) {
@@ -163,12 +147,27 @@ __device__ __forceinline__ void ax_mma(uint32_t tmem_d, uint64_t adesc, uint64_t
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
+// D = A B + D 2^-11
+__device__ __forceinline__ void ax_mma_over(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.eq.b32 p, 0, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p, %4;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "n"(SPLIT_LO) : "memory");
+}
 __device__ __forceinline__ void ax_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
       ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void ax_mma_ts_over(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.eq.b32 p, 0, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p, %4;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "n"(SPLIT_LO) : "memory");
 }
 // MN-major B, SWIZZLE_128B: blocks of 64 columns x 8 rows of K; K groups 1024 bytes apart, column blocks 16 KB
 __device__ __forceinline__ uint64_t ax_desc_mn(uint32_t saddr) {
@@ -186,7 +185,7 @@ attn_prefill_x3_kernel(const __grid_constant__ CUtensorMap mqh, const __grid_con
   extern __shared__ unsigned char ax_raw[];
   __shared__ float s_max[2][AX_T];                   // row maxima / sums of the two column halves
   __shared__ float s_ks[2][AX_T], s_vs[2][AX_T];     // inverse scales of a tile's keys, of this tile and the next
-  __shared__ float s_vm[2][4];                       // largest of s_vs, by warps
+  __shared__ float s_vp[2][AX_T], s_vm[2][4];        // largest of s_vs up to a key of the warp's 32, of all 32
   __shared__ uint64_t qbar, kbar, vbar, sbar, pbar;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_s;
@@ -238,7 +237,10 @@ attn_prefill_x3_kernel(const __grid_constant__ CUtensorMap mqh, const __grid_con
       for (int kb = 0; kb < KBH; kb++) {
         const uint64_t a = tc_smem_desc(tc_smem_u32(Qs + (part == 0 ? TILE : 0) + kb * (128 * 128))), b = tc_smem_desc(tc_smem_u32(Ks + (part == 1 ? TILE : 0) + kb * (128 * 128)));
 #pragma unroll
-        for (int k = 0; k < 4; k++) ax_mma(tmem_s, a + (uint64_t)(2 * k), b + (uint64_t)(2 * k), idesc, (uint32_t)((part | kb | k) != 0));
+        for (int k = 0; k < 4; k++) {
+          if (part == 2 && (kb | k) == 0) ax_mma_over(tmem_s, a, b, idesc);
+          else ax_mma(tmem_s, a + (uint64_t)(2 * k), b + (uint64_t)(2 * k), idesc, (uint32_t)((part | kb | k) != 0));
+        }
       }
     }
     tc_commit(&sbar);
@@ -261,8 +263,14 @@ attn_prefill_x3_kernel(const __grid_constant__ CUtensorMap mqh, const __grid_con
       s_ks[buf][tid] = v;
     } else {
       s_vs[buf][tid - AX_T] = v;
-      const float m = warp_max(v);
-      if (lane == 0) s_vm[buf][qd] = m;
+      float m = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float up = __shfl_up_sync(THA_FULL_MASK, m, o);
+        if (lane >= o) m = fmaxf(m, up);
+      }
+      s_vp[buf][tid - AX_T] = m;
+      if (lane == 31) s_vm[buf][qd] = m;
     }
   };
   keep_scale(scale_of(0), 0);
@@ -280,8 +288,14 @@ attn_prefill_x3_kernel(const __grid_constant__ CUtensorMap mqh, const __grid_con
   for (int t0 = 0; t0 <= kmax; t0 += AX_T, ph ^= 1u) {
     const bool more = t0 + AX_T <= kmax, whole = t0 + AX_T - 1 <= pos0;   // whole: every row sees every key
     const float ahead = more ? scale_of(t0 + AX_T) : 0.0f;
-    const float c = fmaxf(fmaxf(s_vm[ph][0], s_vm[ph][1]), fmaxf(s_vm[ph][2], s_vm[ph][3]));   // a power of two from 2^-100 on
-    if (tid >= AX_T) s_vs[ph][tid - AX_T] *= 16384.0f / c;
+    float c = 1.0f;                                  // a power of two from 2^-100 on; 1 for a row that sees no key of the tile
+    if (const int seen = min(qpos - t0, AX_T - 1); seen >= 0) {
+      c = s_vp[ph][seen];
+#pragma unroll
+      for (int x = 0; x < 3; x++)
+        if (x < seen >> 5) c = fmaxf(c, s_vm[ph][x]);
+    }
+    const float up = 16384.0f / c;
     if (ok) ok = tc_mbar_wait(&sbar, ph, abort_flag);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (warp == 0) {
@@ -326,13 +340,10 @@ attn_prefill_x3_kernel(const __grid_constant__ CUtensorMap mqh, const __grid_con
           float pe = exp2f(fmaf(__uint_as_float(s[j + e]) * ks[e], qf, -m_new));
           if (!whole && tk + 16 * x + j + e > qpos) pe = 0.0f;
           lsum += pe;
-          w[e] = pe * vs[e];
+          w[e] = pe;
         }
-        hi[j >> 1] = ax_h2(w[0], w[1]);
-        hi[(j >> 1) + 1] = ax_h2(w[2], w[3]);
-        const float2 f0 = ax_f2(hi[j >> 1]), f1 = ax_f2(hi[(j >> 1) + 1]);
-        lo[j >> 1] = ax_h2(w[0] - f0.x, w[1] - f0.y);
-        lo[(j >> 1) + 1] = ax_h2(w[2] - f1.x, w[3] - f1.y);
+#pragma unroll
+        for (int e = 0; e < 4; e += 2) split_f16x2(f32x2_mul(make_float2(w[e], w[e + 1]), make_float2(vs[e], vs[e + 1])), up, hi[(j + e) >> 1], lo[(j + e) >> 1]);
       }
       ax_tmem_st8(ts + (uint32_t)(16 * x), hi);
       ax_tmem_st8(ts + (uint32_t)(16 * x + 8), lo);
@@ -355,7 +366,8 @@ attn_prefill_x3_kernel(const __grid_constant__ CUtensorMap mqh, const __grid_con
           ax_mma_ts(tmem_pv, a + 8, vh + (uint64_t)(x * (2048 >> 4)), idesc, (uint32_t)(x != 0));
           ax_mma_ts(tmem_pv, a, vl + (uint64_t)(x * (2048 >> 4)), idesc, 1u);
         }
-        for (int x = 0; x < groups; x++) ax_mma_ts(tmem_pv, tmem_s + (uint32_t)(16 * x), vh + (uint64_t)(x * (2048 >> 4)), idesc, 1u);
+        ax_mma_ts_over(tmem_pv, tmem_s, vh, idesc);
+        for (int x = 1; x < groups; x++) ax_mma_ts(tmem_pv, tmem_s + (uint32_t)(16 * x), vh + (uint64_t)(x * (2048 >> 4)), idesc, 1u);
         tc_commit(&pbar);
       }
       __syncwarp();

@@ -2,14 +2,12 @@
 //
 //   out[n, row] = sum_k W[row, k] * X[n, k]          W: [M, K] row-major fp32, X: [N, K] as two fp16 planes and a power of two a row
 //
-// A value times a power of two of its row is hi + lo, hi = fp16(v), lo = fp16(v - hi): 22 bits of significand, as tf32 hi and lo keep, at twice the
-// MMA rate and half the bytes (the scheme of Ootomo and Yokota, "Recovering single precision accuracy from Tensor Cores while surpassing the
-// FP32 theoretical peak performance", 2022, with a scale of each row in the place of their fixed one).  fp16 ends at 65504 and 2^-24, so
-// the largest value of a row of X is brought to [2^14, 2^15): what is lost of any value is below 2^-39 of the row's largest.  The scale of
-// a weight row comes from its first values: the largest of up to 128 is brought to [2^7, 2^8), which leaves a factor of 256 above it and loses less than 2^-32 of
-// it.  A row that goes further than that, or whose first values are all zero, shows as an infinity in hi: the CTA pair then goes over its items once more with
-// scales of the whole rows.  lo.lo is left out; Whi.Xhi and the two corrections have accumulators of their own, so that the large
-// sum takes K / 16 additions (3xTF32: K / 8).
+// A value times a power of two of its row is hi + lo 2^-11 (split_f16.cuh): 22 bits of significand, as tf32 hi and lo keep, at twice the MMA rate and half the
+// bytes.  The largest value of a row of X is brought to [2^14, 2^15): values down to 2^-28 of it keep their 22 bits, none loses more than 2^-50 of it.  The scale of
+// a weight row comes from its first values: the largest of up to 128 (of a share of K) is brought to [2^7, 2^8), which leaves a factor of 256 above it; values down to 2^-21 of
+// it keep their 22 bits, none loses more than 2^-43 of it.  A row that goes further up than that, or whose first values are all zero, shows as an infinity in hi: the CTA pair
+// then goes over its items once more with scales of the whole rows.  Whi.Xhi and the two corrections have accumulators of their own, so that the large
+// sum takes K / 16 additions (3xTF32: K / 8); the corrections join it in the read-out, times 2^-11.
 //
 // A pair of CTAs (cta_group::2) takes 256 weight rows x 128 activation rows: each has 128 of the weight rows, in TMEM, and 64 of the activation rows, in shared
 // memory, that both halves of the MMA read.  Bound by the tensor pipe under the power limit and by the last, partly filled round over the 74 pairs; the tf32 kernel was
@@ -27,10 +25,10 @@
 //   warps 12-19 read-out: thread = weight row x 64 activation rows.  The corrections leave TMEM first, since the next item's MMAs write
 //               them again; the main sum has two buffers.
 #include <cuda.h>
-#include <cuda_fp16.h>
 
 #include "common.cuh"
 #include "gemm_tc.h"
+#include "split_f16.cuh"
 #include "tc_common.cuh"
 
 namespace tha {
@@ -81,24 +79,13 @@ __device__ __forceinline__ void x3_mma(uint32_t tmem_d, uint32_t tmem_a, uint64_
       "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
       ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(X3_IDESC), "r"(accumulate) : "memory");
 }
-__device__ __forceinline__ uint32_t x3_h2(float a, float b) {   // a in the low half, nearest even, infinity beyond the range
-  uint32_t r;
-  asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
-  return r;
-}
 __device__ __forceinline__ void x3_tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
       ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
         "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]) : "memory");
 }
-// The power of two that brings |v| to [2^e, 2^(e+1)), and its inverse; within what fp32 holds
-__device__ __forceinline__ float x3_scale_to(float v, int e, float* inverse) {
-  int s = 254 + e - (int)(__float_as_uint(v) >> 23);
-  s = s > 253 ? 253 : s;
-  *inverse = __uint_as_float((uint32_t)(254 - s) << 23);
-  return __uint_as_float((uint32_t)s << 23);
-}
+constexpr int X3_SCALE_MOST = 115;       // powers of two of a row's scale at most
 
 __global__ void __launch_bounds__(X3_BOUND, 1)
 gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant__ CUtensorMap mw1, const __grid_constant__ CUtensorMap mw2,
@@ -296,7 +283,7 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
         smax[par][grp][r] = m;
         asm volatile("bar.sync 1, 256;" ::: "memory");
         float inverse;
-        const float sc = x3_scale_to(fmaxf(smax[par][0][r], smax[par][1][r]), pass ? 14 : 7, &inverse);
+        const float sc = split_scale<X3_SCALE_MOST>(fmaxf(smax[par][0][r], smax[par][1][r]), pass ? 14 : 7, &inverse);
         if (grp == 0) {
           // what the MMAs have completed says nothing of the read-out's last step: with a k-block an item these warps are four items ahead of it
           if (n_it >= 4 && ok) ok = tc_mbar_wait(&rowfree[par], (unsigned)((n_it >> 2) & 1) ^ 1u, abort_flag);
@@ -315,15 +302,10 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
             const unsigned char* wrow = wring + sw * S::W_STAGE + half * (TC_BM * 128) + r * 128;
 #pragma unroll
             for (int j = 0; j < 8; j++) {            // logical 16-byte chunk j lives at j ^ (row & 7) (SWIZZLE_128B)
-              float4 v = *reinterpret_cast<const float4*>(wrow + ((j ^ (r & 7)) << 4));
-              v.x *= sc; v.y *= sc; v.z *= sc; v.w *= sc;
-              hi[2 * j] = x3_h2(v.x, v.y);
-              hi[2 * j + 1] = x3_h2(v.z, v.w);
-              const __half2 h0 = *reinterpret_cast<__half2*>(&hi[2 * j]), h1 = *reinterpret_cast<__half2*>(&hi[2 * j + 1]);
-              top = __hmax2(top, __hmax2(__habs2(h0), __habs2(h1)));
-              const float2 f0 = __half22float2(h0), f1 = __half22float2(h1);
-              lo[2 * j] = x3_h2(v.x - f0.x, v.y - f0.y);
-              lo[2 * j + 1] = x3_h2(v.z - f1.x, v.w - f1.y);
+              const float4 v = *reinterpret_cast<const float4*>(wrow + ((j ^ (r & 7)) << 4));
+              split_f16x2(make_float2(v.x, v.y), sc, hi[2 * j], lo[2 * j]);
+              split_f16x2(make_float2(v.z, v.w), sc, hi[2 * j + 1], lo[2 * j + 1]);
+              top = __hmax2(top, __hmax2(__habs2(*reinterpret_cast<__half2*>(&hi[2 * j])), __habs2(*reinterpret_cast<__half2*>(&hi[2 * j + 1]))));
             }
             if (half == 0) {
               if (g >= 2 && ok) ok = tc_mbar_wait(&aempty[sa], ((g >> 1) & 1u) ^ 1u, abort_flag);
@@ -370,7 +352,7 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
               tc_tmem_ld16(tm + (uint32_t)c, v);
               asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-              for (int j = 0; j < 16; j++) sum[c + j] += __uint_as_float(v[j]);
+              for (int j = 0; j < 16; j++) sum[c + j] = part == 0 ? fmaf(__uint_as_float(v[j]), SPLIT_DOWN, sum[c + j]) : sum[c + j] + __uint_as_float(v[j]);
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
@@ -429,15 +411,6 @@ __device__ __forceinline__ void x3_block_sum_max(float& s, float& m, float* red)
   m = warp_max(lane < nw ? red[33 + lane] : 0.0f);
 }
 __device__ __forceinline__ float x3_abs_max(float4 v, float m) { return fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)))); }
-__device__ __forceinline__ void x3_store4(float4 v, float s, uint16_t* hi, uint16_t* lo, int i) {
-  v.x *= s; v.y *= s; v.z *= s; v.w *= s;
-  uint2 h, l;
-  h.x = x3_h2(v.x, v.y); h.y = x3_h2(v.z, v.w);
-  const float2 a = __half22float2(*reinterpret_cast<__half2*>(&h.x)), b = __half22float2(*reinterpret_cast<__half2*>(&h.y));
-  l.x = x3_h2(v.x - a.x, v.y - a.y); l.y = x3_h2(v.z - b.x, v.w - b.y);
-  reinterpret_cast<uint2*>(hi)[i] = h;
-  reinterpret_cast<uint2*>(lo)[i] = l;
-}
 
 // A block a row, a thread up to four float4 a block-width apart, kept in registers between the row's maximum and its planes.  scale[row]: what a product
 // with the row is multiplied by.
@@ -510,11 +483,11 @@ __global__ void __launch_bounds__(1024) x3_rows_kernel(X3RowsP p) {
   }
   x3_block_sum_max(ss, m, red);
   float inverse;
-  const float s = x3_scale_to(m, 14, &inverse);
+  const float s = split_scale<X3_SCALE_MOST>(m, 14, &inverse);
 #pragma unroll
   for (int k = 0; k < 4; k++) {
     const int i = threadIdx.x + k * (int)blockDim.x;
-    if (i < n4) x3_store4(v[k], s, p.hi + (size_t)b * p.n, p.lo + (size_t)b * p.n, i);
+    if (i < n4) split_f16x4(v[k], s, reinterpret_cast<uint2*>(p.hi + (size_t)b * p.n)[i], reinterpret_cast<uint2*>(p.lo + (size_t)b * p.n)[i]);
   }
   if (threadIdx.x == 0) p.scale[b] = !live ? 0.0f : (MODE == X3_NORM ? inverse * (1.0f / sqrtf(ss / p.n + 1e-5f)) : inverse);
 }

@@ -69,6 +69,21 @@ def test_rows_beyond_their_first_values(splits):
     check(W, X, splits)                             # every output against the sizes of its own row and column
 
 
+@pytest.mark.parametrize("down", [2.0 ** -12, 2.0 ** -20, 1e-6])
+@pytest.mark.parametrize("splits", [1, 2])
+def test_rows_that_shrink_behind_their_first_values(splits, down):
+    """Weight rows (and activation rows) of whose values all but a few large ones are small, where only the small ones meet anything but zeros: they keep their 22 bits."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    W, X = torch.randn(300, 1024, device="cuda", generator=g), torch.randn(130, 1024, device="cuda", generator=g)
+    large = torch.zeros(1024, dtype=torch.bool, device="cuda")
+    large[:128] = True
+    large[512:640] = True                            # ahead in each share of K
+    W[:, ~large] *= down
+    X[:100, large] = 0                               # the other rows meet the large values
+    check(W, X, splits)
+    check(X, W, splits)
+
+
 def test_values_that_are_not_finite_stay_in_their_rows():
     g = torch.Generator(device="cuda").manual_seed(4)
     W, X = torch.randn(300, 256, device="cuda", generator=g), torch.randn(70, 256, device="cuda", generator=g)
@@ -143,3 +158,33 @@ def test_prompt_attention(heads, hs, kv_heads, pos0, lens, paged):
     want, _, _ = llama64.forward(cfg, w.t, rows, seqs)
     # sums of 32 to 2048 terms at 1e-6 to 2e-6 each (test_product), through three products and the attention one after the other
     assert float((got.double() - want).norm() / want.norm()) < 1e-5
+
+
+@pytest.mark.parametrize("heads,hs,kv_heads", [(16, 128, 16), (32, 64, 8)])
+@pytest.mark.parametrize("size", [20, 40, 60])
+@pytest.mark.parametrize("at", [45, 100, 200])
+def test_prompt_attention_ahead_of_a_large_value(heads, hs, kv_heads, at, size):
+    """Rows that do not see a key are as exact as without it, whatever the size of its values (2^size times the others'): the weights of a row are scaled by the keys that it sees.
+    The token at `at` is the only one with the channel whose gain is 2^size."""
+    eng, ck = load_pkg("engine"), load_pkg("checkpoint")
+    cfg = ck.Config(heads * hs, 264, 2, heads, kv_heads, 96, 512)
+    w = eng.device_random_weights(cfg, seed=2, std=cfg.dim ** -0.5)
+    w.t["tok_emb"][:, 0] = 0
+    w.t["tok_emb"][95] = 0
+    w.t["tok_emb"][95, 0] = 1
+    w.t["rms_att"][0, 0] = 2.0 ** (size - 0.5 * np.log2(cfg.dim))
+    w.t["wq"][0, :, 0] = 0
+    w.t["wk"][0, :, 0] = 0
+    e = eng.Engine(w, 1, with_att=False)
+    toks = np.random.default_rng(3).integers(0, 95, 230).astype(np.int32)
+    toks[at] = 95
+    got = torch.empty(1, 96, device="cuda")
+    torch.cuda.synchronize()
+    e.prefill([(0, 0, toks)], got)
+    torch.cuda.synchronize()
+    _, k, v = llama64.forward(cfg, w.t, lambda c, s, l, n: e.state.key_cache[0, l, :0], [(0, 0, toks[:at])])
+    assert float(v[:, 0].abs().max()) < 100
+    for cache, want in ((e.state.key_cache, k), (e.state.value_cache, v)):
+        # the second layer's rows: through the attention and four products, as test_prompt_attention
+        assert float((cache[0, 1, :at].double() - want[:, 1]).norm() / want[:, 1].norm()) < 1e-5
+    assert float(e.state.value_cache[0, 0, at].abs().max()) > 2.0 ** (size - 6)
