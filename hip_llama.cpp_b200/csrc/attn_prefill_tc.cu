@@ -265,6 +265,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_cons
       *reinterpret_cast<uint4*>(orow + c) = make_uint4(ptc_bf16x2(acc[c] * inv, acc[c + 1] * inv), ptc_bf16x2(acc[c + 2] * inv, acc[c + 3] * inv),
                                                        ptc_bf16x2(acc[c + 4] * inv, acc[c + 5] * inv), ptc_bf16x2(acc[c + 6] * inv, acc[c + 7] * inv));
   }
+  if (warp == 0 && live_tile && *((volatile int*)abort_flag) && tc_elect()) {   // a tile of K and of V for every tile of keys
+    tc_drain(&qbar, 1, 1);
+    tc_drain(&kbar, 1, kmax / PTC_TK + 1);
+    tc_drain(&vbar, 1, kmax / PTC_TK + 1);
+  }
   __syncthreads();
   if (warp == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

@@ -403,6 +403,11 @@ attn_prefill_x3_kernel(const __grid_constant__ CUtensorMap mqh, const __grid_con
 #pragma unroll
     for (int c = 0; c < HH; c += 4) *reinterpret_cast<float4*>(orow + c) = make_float4(acc[c] / l, acc[c + 1] / l, acc[c + 2] / l, acc[c + 3] / l);
   }
+  if (warp == 0 && live_tile && *((volatile int*)abort_flag) && tc_elect()) {   // a tile of K and of V for every tile of keys
+    tc_drain(&qbar, 1, 1);
+    tc_drain(&kbar, 1, kmax / AX_T + 1);
+    tc_drain(&vbar, 1, kmax / AX_T + 1);
+  }
   __syncthreads();
   if (warp == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

@@ -209,6 +209,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) chain_tf32x3_kernel(const __gri
     if (tc_elect()) {
       int gb = 0, n_it = 0;
       bool ok = true;
+      int sent = 0;
       for (int it = blockIdx.x; it < P.n_items && ok; it += gridDim.x, n_it++) {
         const Item w = item_of(it);
         const ChainPhase& f = P.ph[w.ph];
@@ -218,6 +219,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) chain_tf32x3_kernel(const __gri
           if (g >= S::SW && !tc_mbar_wait(&wfree[s], ((g / S::SW) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
           const int nk = (w.nkb - i * S::KG) < S::KG ? (w.nkb - i * S::KG) : S::KG;
           tc_mbar_expect_tx(&wfull[s], nk * S::W_BYTES);
+          sent = g + 1;
           for (int kk = 0; kk < nk; kk++) {
             unsigned char* dst = wring + s * S::W_STAGE + kk * S::W_BYTES;
             const int kc = (w.kb0 + i * S::KG + kk) * TC_BK;
@@ -234,6 +236,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) chain_tf32x3_kernel(const __gri
         }
         gb += w.nst;
       }
+      if (!ok) tc_drain(wfull, S::SW, sent);
     }
   } else if (warp == 3) {
     // ===== X producer: the activations of a phase exist once the phase before has finished this column tile
@@ -241,6 +244,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) chain_tf32x3_kernel(const __gri
       pdl_wait();
       int gb = 0, n_it = 0;
       bool ok = true;
+      int sent = 0;
       for (int it = blockIdx.x; it < P.n_items && ok; it += gridDim.x, n_it++) {
         const Item w = item_of(it);
         const ChainPhase& f = P.ph[w.ph];
@@ -264,6 +268,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) chain_tf32x3_kernel(const __gri
           if (g >= S::SX && !tc_mbar_wait(&aempty[s], ((g / S::SX) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
           const int nk = (w.nkb - i * S::KG) < S::KG ? (w.nkb - i * S::KG) : S::KG;
           tc_mbar_expect_tx(&ready[s], nk * S::XS_BYTES);
+          sent = g + 1;
           for (int kk = 0; kk < nk; kk++) {
             unsigned char* st = xring + s * S::XS_STAGE + kk * S::XS_BYTES;
             tc_tma_2d(st, mxh, (w.kb0 + i * S::KG + kk) * TC_BK, w.n0, &ready[s]);
@@ -273,6 +278,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) chain_tf32x3_kernel(const __gri
         CH_TRACE(1, n_it);
         gb += w.nst;
       }
+      if (!ok) tc_drain(ready, S::SX, sent);
     }
   } else if (warp == 1) {
     // ===== MMA issuer (as gemm_tf32x3_kernel)
@@ -330,7 +336,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) chain_tf32x3_kernel(const __gri
       for (int i = i0; i < w.nst && ok; i += TC_CGROUPS) {
         const int g = gb + i, sw = g % S::SW, sa = g % S::SA;
         const int nk = (w.nkb - i * S::KG) < S::KG ? (w.nkb - i * S::KG) : S::KG;
-        ok = tc_mbar_wait(&wfull[sw], (g / S::SW) & 1u, abort_flag);
+        ok = tc_mbar_wait_warp(&wfull[sw], (g / S::SW) & 1u, abort_flag);
 #pragma unroll
         for (int kk = 0; kk < S::KG; kk++) {
           if (kk < nk && ok) {
@@ -345,7 +351,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) chain_tf32x3_kernel(const __gri
               lo[4 * j + 0] = __float_as_uint(v.x - h0); lo[4 * j + 1] = __float_as_uint(v.y - h1);
               lo[4 * j + 2] = __float_as_uint(v.z - h2); lo[4 * j + 3] = __float_as_uint(v.w - h3);
             }
-            if (kk == 0 && g >= S::SA && ok) ok = tc_mbar_wait(&aempty[sa], ((g / S::SA) & 1u) ^ 1u, abort_flag);
+            if (kk == 0 && g >= S::SA && ok) ok = tc_mbar_wait_warp(&aempty[sa], ((g / S::SA) & 1u) ^ 1u, abort_flag);
             const uint32_t ta = tmem_a + sa * S::A_STAGE + kk * S::A_COLS + ((uint32_t)(q * 32) << 16);
             tc_tmem_st32(ta, hi);
             tc_tmem_st32(ta + TC_BK, lo);
@@ -363,7 +369,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) chain_tf32x3_kernel(const __gri
         pdl_trigger();
         pdl_wait();
       }
-      if (ok) ok = tc_mbar_wait(accum, n_it & 1u, abort_flag);
+      if (ok) ok = tc_mbar_wait_warp(accum, n_it & 1u, abort_flag);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (et == 0) CH_TRACE(4, n_it);
       const int mode = f.mode;

@@ -164,6 +164,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant_
       const bool stream_w = p.ny == 1;            // every weight tile is read once: do not let it displace the activations in L2
       int gb = 0;
       bool ok = true, first = true;
+      int sent = 0;
       auto load_w = [&](unsigned char* dst, const CUtensorMap* mw, int kcol, int row0, uint64_t* bar) {
         if (PAIR) {   // 128 rows of w1, then the same 128 rows of w3
           tc_tma_2d(dst, &mw0, kcol, row0, bar);
@@ -183,6 +184,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant_
           pdl_wait();
           for (int j = 0; j < pre; j++) {
             tc_mbar_expect_tx(&full[j], S::STAGE);
+            sent = j + 1;
             tc_tma_2d(smem + j * S::STAGE + S::W_BYTES, &mx, (w.kb0 + j) * BF_BK, w.xrow, &full[j]);
           }
           first = false;
@@ -191,11 +193,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant_
           const int g = gb + i, s = g % S::NST;
           if (g >= S::NST && !tc_mbar_wait(&empty[s], ((g / S::NST) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
           tc_mbar_expect_tx(&full[s], S::STAGE);
+          sent = g + 1;
           load_w(smem + s * S::STAGE, mw, (w.kb0 + i) * BF_BK, w.wrow, &full[s]);
           tc_tma_2d(smem + s * S::STAGE + S::W_BYTES, &mx, (w.kb0 + i) * BF_BK, w.xrow, &full[s]);
         }
         gb += w.nkb;
       }
+      if (!ok) tc_drain(full, S::NST, sent);
     }
   } else if (warp == 1) {
     // ===== MMA issuer
@@ -239,7 +243,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant_
     for (int it = blockIdx.x; it < p.n_items; it += gridDim.x, n_it++) {
       const Item w = item_of(it);
       const int buf = n_it % NBUF, use = n_it / NBUF;
-      if (ok) ok = tc_mbar_wait(&accum[buf], (unsigned)(use & 1), abort_flag);
+      if (ok) ok = tc_mbar_wait_warp(&accum[buf], (unsigned)(use & 1), abort_flag);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (READ == BF_GATED || READ == BF_UNGATED) {
         // the row's accumulators (gate and up, or one) through the activation; warps 4-7 and 8-11 share the columns of a pair
@@ -435,13 +439,17 @@ gemm_bf16_cluster_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_c
         tc_mbar_expect_tx(&full[i], S::STAGE);
         tc_tma_2d(smem + i * S::STAGE + S::W_BYTES, &mx, (kb0 + i) * BF_BK, xrow, &full[i]);
       }
-      for (int i = pre; i < nkb; i++) {
+      int sent = pre;
+      bool ok = true;
+      for (int i = pre; i < nkb && ok; i++) {
         const int s = i % S::NST;
-        if (!tc_mbar_wait(&empty[s], ((i / S::NST) & 1u) ^ 1u, abort_flag)) break;
+        if (!tc_mbar_wait(&empty[s], ((i / S::NST) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
         tc_mbar_expect_tx(&full[s], S::STAGE);
         load_w(i, s);
         tc_tma_2d(smem + s * S::STAGE + S::W_BYTES, &mx, (kb0 + i) * BF_BK, xrow, &full[s]);
+        sent = i + 1;
       }
+      if (!ok) tc_drain(full, S::NST, sent);
     }
   } else if (warp == 1) {
     if (tc_elect()) {

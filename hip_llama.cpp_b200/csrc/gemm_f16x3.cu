@@ -55,7 +55,7 @@ struct X3Smem {
   static constexpr int X_PLANE = (X3_NT / 2) * 128;     // 64 rows of 64 halves
   static constexpr int X_STAGE = 2 * X_PLANE;           // hi | lo
   static constexpr int SW = 4, SX = 5;
-  static constexpr int NBARS = 2 * SW + 3 * SX + 2 + 2 + 2 + 2 + 1 + 4 + 4;
+  static constexpr int NBARS = 2 * SW + 3 * SX + 2 + 2 + 2 + 2 + 1 + 4 + 4 + 1;
   static constexpr int TOTAL = SW * W_STAGE + SX * X_STAGE + 1024 + NBARS * 8 + 64;
   // TMEM columns: main sum 0 | corrections | main sum 1 | two operand slots of 32 (hi) + 32 (lo)
   static constexpr int COL_CORR = 128, COL_MAIN1 = 256, COL_A = 384;
@@ -107,7 +107,8 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
   uint64_t* corrfree = mainfree + 2;     // rank 0: corrections read out in both CTAs
   uint64_t* rowready = corrfree + 1;     // [4] scales of the weight rows of an item
   uint64_t* rowfree = rowready + 4;      // [4] ... and taken by the read-out
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(rowfree + 4);
+  uint64_t* mmadone = rowfree + 4;       // all MMAs complete
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mmadone + 1);
   int* abort_flag = reinterpret_cast<int*>(tmem_slot + 1);
   int* bad_rows = abort_flag + 1;        // a weight row of this CTA went beyond the scale of its first values
   __shared__ float smax[4][2][TC_BM];    // largest of the first values of a weight row, by converter group; item mod 4
@@ -134,6 +135,7 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
     for (int s = 0; s < S::SX; s++) { tc_mbar_init(&xfull[s], 1); tc_mbar_init(&xpeer[s], 1); tc_mbar_init(&xempty[s], 1); }
     for (int s = 0; s < 2; s++) { tc_mbar_init(&aready[s], 8); tc_mbar_init(&aempty[s], 1); tc_mbar_init(&accum[s], 1); tc_mbar_init(&mainfree[s], 16); }
     tc_mbar_init(corrfree, 16);
+    tc_mbar_init(mmadone, 1);
     for (int s = 0; s < 4; s++) { tc_mbar_init(&rowready[s], 4); tc_mbar_init(&rowfree[s], 8); }
     *abort_flag = 0;
     *bad_rows = 0;
@@ -160,7 +162,9 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
 
   int gb = 0, n_it = 0, n_run = 0;      // k-blocks, items and runs so far, of both passes
   bool ok = true;
-  // the end of a pass: whether there is another one, the same answer in both CTAs
+  int sent = 0;                         // stages that a producer has asked for
+  // The end of a pass: whether there is another one, the same answer in both CTAs.  Every thread comes here, whatever became of its waits, and each of these is
+  // bounded: so are the two CTAs' waits for each other.
   auto again = [&]() -> bool {
     __syncwarp();
     __syncthreads();
@@ -187,6 +191,7 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
               unsigned char* dst = wring + s * S::W_STAGE;
               tc_tma_2d(dst, mw, (w.kb0 + i) * X3_BK, w.row0, &wfull[s]);
               tc_tma_2d(dst + TC_BM * 128, mw, (w.kb0 + i) * X3_BK + 32, w.row0, &wfull[s]);
+              sent = g + 1;
             }
             gb += w.nkb;
           }
@@ -203,6 +208,7 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
               unsigned char* dst = xring + s * S::X_STAGE;
               tc_tma_2d(dst, &mxh, (w.kb0 + i) * X3_BK, w.n0 + rank * (X3_NT / 2), &xfull[s]);
               tc_tma_2d(dst + S::X_PLANE, &mxl, (w.kb0 + i) * X3_BK, w.n0 + rank * (X3_NT / 2), &xfull[s]);
+              sent = g + 1;
             }
             gb += w.nkb;
           }
@@ -250,6 +256,15 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
       }
       if (!again()) break;
     }
+    if (*((volatile int*)abort_flag)) {                // copies and MMAs end ahead of the blocks
+      if (warp == 0 && tc_elect()) tc_drain(wfull, S::SW, sent);
+      if (warp == 3 && tc_elect()) tc_drain(xfull, S::SX, sent);
+      if (warp == 1 && rank == 0 && tc_elect()) {
+        x3_commit(mmadone);
+        tc_drain(mmadone, 1, 1);
+      }
+    }
+    __syncwarp();
   } else if (warp < 4 + X3_CONV_WARPS) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
     for (int pass = 0; pass < 2; pass++) {
@@ -262,7 +277,7 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
         if (pass == 0) {
           if (i0 < w.nkb) {
             const int sw = (gb + i0) % S::SW;
-            if (ok) ok = tc_mbar_wait(&wfull[sw], ((gb + i0) / S::SW) & 1u, abort_flag);
+            if (ok) ok = tc_mbar_wait_warp(&wfull[sw], ((gb + i0) / S::SW) & 1u, abort_flag);
             if (ok) {
               const unsigned char* wrow = wring + sw * S::W_STAGE + r * 128;
 #pragma unroll
@@ -286,7 +301,7 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
         const float sc = split_scale<X3_SCALE_MOST>(fmaxf(smax[par][0][r], smax[par][1][r]), pass ? 14 : 7, &inverse);
         if (grp == 0) {
           // what the MMAs have completed says nothing of the read-out's last step: with a k-block an item these warps are four items ahead of it
-          if (n_it >= 4 && ok) ok = tc_mbar_wait(&rowfree[par], (unsigned)((n_it >> 2) & 1) ^ 1u, abort_flag);
+          if (n_it >= 4 && ok) ok = tc_mbar_wait_warp(&rowfree[par], (unsigned)((n_it >> 2) & 1) ^ 1u, abort_flag);
           rowf[par][r] = inverse;
           __syncwarp();
           if (lane == 0) tc_mbar_arrive(&rowready[par]);
@@ -294,7 +309,7 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
         __half2 top = __half2half2(__ushort_as_half(0));
         for (int i = i0; i < w.nkb && ok; i += 2) {
           const int g = gb + i, sw = g % S::SW, sa = g & 1;
-          ok = tc_mbar_wait(&wfull[sw], (g / S::SW) & 1u, abort_flag);
+          ok = tc_mbar_wait_warp(&wfull[sw], (g / S::SW) & 1u, abort_flag);
           const uint32_t ta = tmem + S::COL_A + sa * 64 + ((uint32_t)(q * 32) << 16);
 #pragma unroll
           for (int half = 0; half < 2; half++) {
@@ -308,7 +323,7 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
               top = __hmax2(top, __hmax2(__habs2(*reinterpret_cast<__half2*>(&hi[2 * j])), __habs2(*reinterpret_cast<__half2*>(&hi[2 * j + 1]))));
             }
             if (half == 0) {
-              if (g >= 2 && ok) ok = tc_mbar_wait(&aempty[sa], ((g >> 1) & 1u) ^ 1u, abort_flag);
+              if (g >= 2 && ok) ok = tc_mbar_wait_warp(&aempty[sa], ((g >> 1) & 1u) ^ 1u, abort_flag);
               asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             }
             x3_tmem_st16(ta + (uint32_t)(16 * half), hi);
@@ -341,7 +356,7 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
         for (int j = 0; j < X3_NT / 2; j++) sum[j] = 0.0f;
         for (int i0 = 0; i0 < w.nkb; i0 += X3_RUN, n_run++) {
           const int buf = n_run & 1;
-          if (ok) ok = tc_mbar_wait(&accum[buf], (unsigned)(n_run >> 1) & 1u, abort_flag);
+          if (ok) ok = tc_mbar_wait_warp(&accum[buf], (unsigned)(n_run >> 1) & 1u, abort_flag);
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
           for (int part = 0; part < 2; part++) {     // corrections, then the main sum
@@ -359,7 +374,7 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
             if (lane == 0) x3_arrive_leader(part == 0 ? corrfree : &mainfree[buf]);
           }
         }
-        if (ok) ok = tc_mbar_wait(&rowready[par], (unsigned)(n_it >> 2) & 1u, abort_flag);
+        if (ok) ok = tc_mbar_wait_warp(&rowready[par], (unsigned)(n_it >> 2) & 1u, abort_flag);
         const float rf = rowf[par][r];
         __syncwarp();
         if (lane == 0) tc_mbar_arrive(&rowfree[par]);

@@ -194,6 +194,7 @@ gemm_q8i_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant__
       asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol_w));
       int jb = 0;                                   // running slot counter at the start of the item
       int xr = 0, s = 0;                            // running scale buffer and ring slot
+      int sent = 0;
       bool ok = true;
       for (int it = blockIdx.x; it < p.n_items && ok; it += gridDim.x) {
         const Item w = item_of(it);
@@ -210,6 +211,7 @@ gemm_q8i_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant__
           for (int g = 0; g < n; g++) q8i_bulk(xs_sm + ((xr << gps_sh) + g) * NT, src + (size_t)g * p.ldxs, xbytes, &xfull[xr]);
           if (++xr == nxs) xr = 0;
           if (++s == nring) s = 0;
+          sent++;
         };
         int j = 0;
         if (jb == 0) {
@@ -233,6 +235,10 @@ gemm_q8i_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant__
           activations(j);
         }
         jb += w.nslots;
+      }
+      if (!ok) {
+        tc_drain(full, nring, sent);
+        tc_drain(xfull, nxs, sent);
       }
     }
     __syncwarp();

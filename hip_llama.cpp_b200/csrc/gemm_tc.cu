@@ -130,6 +130,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constan
       asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol_w));
       int gb = 0;                                 // running stage counter at the start of the item
       bool ok = true;
+      int sent = 0;
       for (int it = blockIdx.x; it < p.n_items && ok; it += gridDim.x) {
         const Item w = item_of(it);
         const CUtensorMap* mw = (w.mat == 0) ? &mw0 : (w.mat == 1 ? &mw1 : &mw2);
@@ -138,12 +139,14 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constan
           if (g >= S::SW && !tc_mbar_wait(&wfree[s], ((g / S::SW) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
           const int nk = (w.nkb - i * S::KG) < S::KG ? (w.nkb - i * S::KG) : S::KG;
           tc_mbar_expect_tx(&wfull[s], nk * S::W_BYTES);
+          sent = g + 1;
           TC_TRACE(0, i);
           for (int kk = 0; kk < nk; kk++)
             tc_tma_2d_hint(wring + s * S::W_STAGE + kk * S::W_BYTES, mw, (w.kb0 + i * S::KG + kk) * TC_BK, w.row0, &wfull[s], pol_w);
         }
         gb += w.nst;
       }
+      if (!ok) tc_drain(wfull, S::SW, sent);
     }
   } else if (warp == 3) {
     // ===== X producer (activations: written by the previous kernel)
@@ -152,6 +155,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constan
       kt_stamp(kt, 1);
       int gb = 0;
       bool ok = true;
+      int sent = 0;
       for (int it = blockIdx.x; it < p.n_items && ok; it += gridDim.x) {
         const Item w = item_of(it);
         for (int i = 0; i < w.nst; i++) {
@@ -160,6 +164,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constan
           const int nk = (w.nkb - i * S::KG) < S::KG ? (w.nkb - i * S::KG) : S::KG;
           TC_TRACE(1, i);
           tc_mbar_expect_tx(&ready[s], nk * S::XS_BYTES);
+          sent = g + 1;
           for (int kk = 0; kk < nk; kk++) {
             unsigned char* st = xring + s * S::XS_STAGE + kk * S::XS_BYTES;
             tc_tma_2d(st, &mxh, (w.kb0 + i * S::KG + kk) * TC_BK, w.n0, &ready[s]);
@@ -168,6 +173,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constan
         }
         gb += w.nst;
       }
+      if (!ok) tc_drain(ready, S::SX, sent);
     }
   } else if (warp == 1) {
     // ===== MMA issuer: A (weights, hi / lo) from TMEM, B (activations, hi / lo) from shared memory
@@ -229,7 +235,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constan
       for (int i = i0; i < w.nst && ok; i += TC_CGROUPS) {
         const int g = gb + i, sw = g % S::SW, sa = g % S::SA;
         const int nk = (w.nkb - i * S::KG) < S::KG ? (w.nkb - i * S::KG) : S::KG;
-        ok = tc_mbar_wait(&wfull[sw], (g / S::SW) & 1u, abort_flag);
+        ok = tc_mbar_wait_warp(&wfull[sw], (g / S::SW) & 1u, abort_flag);
         if (threadIdx.x == 128 + 128 * grp) TC_TRACE(2, i);
 #pragma unroll
         for (int kk = 0; kk < S::KG; kk++) {
@@ -245,7 +251,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constan
               lo[4 * j + 0] = __float_as_uint(v.x - h0); lo[4 * j + 1] = __float_as_uint(v.y - h1);
               lo[4 * j + 2] = __float_as_uint(v.z - h2); lo[4 * j + 3] = __float_as_uint(v.w - h3);
             }
-            if (kk == 0 && g >= S::SA && ok) ok = tc_mbar_wait(&aempty[sa], ((g / S::SA) & 1u) ^ 1u, abort_flag);
+            if (kk == 0 && g >= S::SA && ok) ok = tc_mbar_wait_warp(&aempty[sa], ((g / S::SA) & 1u) ^ 1u, abort_flag);
             if (kk == 0 && threadIdx.x == 128 + 128 * grp) TC_TRACE(3, i);
             const uint32_t ta = tmem_a + sa * S::A_STAGE + kk * S::A_COLS + ((uint32_t)(q * 32) << 16);
             tc_tmem_st32(ta, hi);                          // consumes every loaded value: the shared-memory reads are complete
@@ -265,7 +271,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constan
         pdl_trigger();
         pdl_wait();   // returns at once (the X producer already waited); makes the predecessor's writes visible to these threads
       }
-      if (ok) ok = tc_mbar_wait(accum, n_it & 1u, abort_flag);
+      if (ok) ok = tc_mbar_wait_warp(accum, n_it & 1u, abort_flag);
       if (n_it == 0 && threadIdx.x == 128) kt_stamp(kt, 4);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int row = w.row0 + r;

@@ -33,13 +33,26 @@ __device__ __forceinline__ bool tc_mbar_try(uint64_t* bar, unsigned parity) {
       : "=r"(ok) : "r"(tc_smem_u32(bar)), "r"(parity) : "memory");
   return ok != 0;
 }
-// Bounded wait: a broken pipeline must end the kernel (and fail the parity test), never hang the GPU.
+// Bounded wait: a broken pipeline must end the kernel (and fail the parity test), never hang the GPU.  A try that finds the phase incomplete comes back after 4 us: 17 s.
 __device__ __forceinline__ bool tc_mbar_wait(uint64_t* bar, unsigned parity, int* abort_flag) {
   for (unsigned n = 0; !tc_mbar_try(bar, parity); n++) {
     if (n > (1u << 22)) { *abort_flag = 1; return false; }
     if ((n & 1023u) == 1023u && *((volatile int*)abort_flag)) return false;
   }
   return true;
+}
+// The same answer for the whole warp, for waits whose outcome decides on instructions that a warp executes together (tcgen05.ld, .st)
+__device__ __forceinline__ bool tc_mbar_wait_warp(uint64_t* bar, unsigned parity, int* abort_flag) {
+  return __all_sync(THA_FULL_MASK, tc_mbar_wait(bar, parity, abort_flag));
+}
+// The end of a TMA producer that has given up: `sent` copies have been asked for, in turn into a ring of n stages with barriers full[n], and some may still be under way, into
+// shared memory that the next block will use: until they have landed, or a second has passed.  (Copies of a producer that came to its end land long before another
+// thread's wait runs out.)  Not on the usual way: a loop over the ring took the int8 product of one row 3 us.
+__device__ __forceinline__ void tc_drain(uint64_t* full, int n, int sent) {
+  unsigned tries = 0;
+  for (int g = sent > n ? sent - n : 0; g < sent; g++)
+    while (!tc_mbar_try(&full[g % n], (unsigned)(g / n) & 1u))
+      if (++tries > (1u << 18)) return;
 }
 // One lane of a converged warp, in a form that the compiler knows to be one: the descriptors of tcgen05 and TMA instructions go through uniform
 // registers, and under `lane == 0` each such instruction is wrapped in a loop over the lanes that might take part.  A stage of barrier wait,
