@@ -1889,14 +1889,6 @@ extern "C" int tha_hyb_head_gate(void* stream, int dtype, void* out, const float
                               : head_gate_launch(s, (float*)out, o_raw, n_rows, heads, E, eps, norm, norm_per_head, gate, ldg, do_norm, gate_act);
 }
 
-// THA_ACT_XIELU: the two stored numbers p, q -> the factors the kernels multiply with
-static void hyb_act_factors(int act, float& limit, float& alpha) {
-  if (act != THA_ACT_XIELU) return;
-  const float p = limit, q = alpha;
-  limit = fmaxf(p, 0.f) + log1pf(expf(-fabsf(p)));
-  alpha = 0.5f + fmaxf(q, 0.f) + log1pf(expf(-fabsf(q)));
-}
-
 extern "C" int tha_hyb_linear(void* stream, int dtype, float* C, long long ldc, const void* A, long long lda, int a_f32,
                               const int* a_rows, const void* W, long long w_group_stride, int M, int N, int K,
                               const int* group_off, int n_groups) {
@@ -1936,7 +1928,7 @@ extern "C" int tha_hyb_linear_act(void* stream, int dtype, int act, void* y, flo
   if (M < 1 || N < 1) return THA_STATUS_SUCCESS;
   if (K < 1 || ff < 1 || !y || !gu || !A || !W) return THA_STATUS_INVALID_ARG;
   const bool gated = hyb_act_gated(act);
-  if (dtype == THA_DT_BF16 && hyb_tc_linear() && act >= THA_ACT_GLU_CLAMPED && act <= THA_ACT_SILU_GLU && col_u >= 0 && col_u + ff <= N &&
+  if (dtype == THA_DT_BF16 && hyb_tc_linear() && act >= THA_ACT_GLU_CLAMPED && act <= THA_ACT_SILU_GLU && act != THA_ACT_XIELU && col_u >= 0 && col_u + ff <= N &&
       (!gated || (col_g >= 0 && col_g + ff <= N))) {
     BfArgs b = {};
     b.n_mats = gated ? 2 : 1; b.K = K;
@@ -1948,7 +1940,6 @@ extern "C" int tha_hyb_linear_act(void* stream, int dtype, int act, void* y, flo
     b.out = gu; b.ldo = ldg; b.splits = 1;
     b.act_out = (uint16_t*)y; b.ld_act = ff;
     b.ff_act = 1 + act; b.act_limit = limit; b.act_alpha = alpha;
-    hyb_act_factors(act, b.act_limit, b.act_alpha);
     if (gemm_bf16_ok(b) && gemm_bf16_act_ok(b)) return gemm_bf16_launch((cudaStream_t)stream, b, hyb_gemm_pdl());
   }
   const int rc = tha_hyb_linear(stream, dtype, gu, ldg, A, K, 0, nullptr, W, 0, M, N, K, nullptr, 0);
@@ -2282,7 +2273,11 @@ extern "C" int tha_hyb_moe_route(void* stream, const tha_moe_t* e, const float* 
 extern "C" int tha_hyb_ff_act(void* stream, int dtype, int act, void* y, const float* gu, long long ldg, int col_g, int col_u, int n,
                               int ff, float limit, float alpha) {
   if (n < 1 || ff < 1) return THA_STATUS_SUCCESS;
-  hyb_act_factors(act, limit, alpha);
+  if (act == THA_ACT_XIELU) {   // the two stored numbers p, q -> the factors the kernel multiplies with
+    const float p = limit, q = alpha;
+    limit = fmaxf(p, 0.f) + log1pf(expf(-fabsf(p)));
+    alpha = 0.5f + fmaxf(q, 0.f) + log1pf(expf(-fabsf(q)));
+  }
   cudaStream_t s = (cudaStream_t)stream;
   const bool gated = hyb_act_gated(act);
   if (ff % 4 == 0 && ldg % 4 == 0 && col_u % 4 == 0 && (!gated || col_g % 4 == 0) && aligned16(gu) && n <= 65535) {

@@ -76,9 +76,6 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
   unsigned ok;
   asm volatile(
@@ -139,7 +136,7 @@ struct PhaseW {      // a CTA's weight side of a GEMV phase
   int u0, u1;        // its units
   int K;             // row length (floats)
   int upr;           // rows per unit (2: QKV pair, W13 w1+w3; 1: others)
-  int nmax;          // units per full chunk (power of two; nmax * upr <= 2 rows)
+  int nmax;          // units per full chunk: 1 or 2 (nmax * upr <= 2 rows)
   int full, n;       // full chunks, all chunks
 };
 struct AttItem { int b, h, s, t0, t1, at; };   // split s of (slot b, head h): positions t0 .. t1 - 1; place of its partial
@@ -157,13 +154,11 @@ __device__ __forceinline__ PhaseW phase_weights(const tha_config_t& c, int kind,
   }
   const int fit = slot_bytes / (w.upr * w.K * (int)sizeof(float));   // host guarantees >= 1
   const int cap = 2 / w.upr;
-  const int n = fit < cap ? fit : cap;
-  w.nmax = n >= 4 ? 4 : (n >= 2 ? 2 : 1);
+  w.nmax = fit < cap ? fit : cap;
   w.u0 = (int)((long long)blockIdx.x * P / gridDim.x);
   w.u1 = (int)((long long)(blockIdx.x + 1) * P / gridDim.x);
   w.full = (w.u1 - w.u0) / w.nmax;
-  const int rem = (w.u1 - w.u0) % w.nmax;
-  w.n = w.full + (rem == 3 ? 2 : (rem ? 1 : 0));
+  w.n = w.full + (w.u1 - w.u0) % w.nmax;
   return w;
 }
 
@@ -173,7 +168,6 @@ struct MegaShared {
   AttItem item;                 // this CTA's first attention item
   int splits[MG_MAX_B];         // of a slot's context
   float red[MG_NW * MG_MAX_B];
-  float scale[MG_MAX_B];
   int pos[MG_MAX_B];
   int tok[MG_MAX_B];
   float amax_v[MG_NW * MG_MAX_B];
@@ -247,15 +241,10 @@ __device__ __forceinline__ Chunk chunk_after(Chunk q, int steps, const MegaShare
   }
   return q;
 }
-// First unit and units of chunk j: full ones, then what is left as 2 and 1
+// First unit and units of chunk j: full ones, then what is left
 __device__ __forceinline__ int chunk_units(const PhaseW& w, int j, int* u) {
-  *u = w.u0 + min(j, w.full) * w.nmax;
-  if (j < w.full) return w.nmax;
-  const int rem = w.u1 - *u;
-  if (rem < 3) return rem;
-  if (j == w.full) return 2;
-  *u += 2;
-  return 1;
+  *u = w.u0 + j * w.nmax;
+  return min(w.nmax, w.u1 - *u);
 }
 // One lane: chunk q into the warp's slot.
 __device__ __forceinline__ void load_chunk(const MegaP& p, MegaShared* sh, Chunk q, unsigned char* dst, uint64_t* bar, uint64_t pol) {
@@ -678,7 +667,6 @@ __global__ void __launch_bounds__(MG_THREADS, 1) mega_step_kernel(const MegaP p)
   if (tid < MG_MAX_B) {
     sh->pos[tid] = (tid < p.B) ? p.pos[tid] : -1;
     sh->tok[tid] = (tid < p.B) ? p.token[tid] : 0;
-    sh->scale[tid] = 1.0f;
   }
   if (tid >= 32 && tid < 38) sh->tab[tid - 32] = phase_weights(c, tid - 32, p.slot_bytes);
   if (tid < MG_NW * MG_MAX_B) { sh->amax_v[tid] = -INFINITY; sh->amax_i[tid] = 0x7fffffff; }
@@ -745,8 +733,7 @@ __global__ void __launch_bounds__(MG_THREADS, 1) mega_step_kernel(const MegaP p)
         const int nr = chunk_units(w, cur.j, &u) * w.upr;
         mbar_wait(&sh->full[warp], loads & 1u, p.bar, sh, 1000u + ph);
         const float4* ws4 = reinterpret_cast<const float4*>(slot);
-        if (nr == 4) consume_chunk<BT, 4, HS>(p, sh, kind, layer, u, ws4, xs4, K, scale_l, tag);
-        else if (nr == 2) consume_chunk<BT, 2, HS>(p, sh, kind, layer, u, ws4, xs4, K, scale_l, tag);
+        if (nr == 2) consume_chunk<BT, 2, HS>(p, sh, kind, layer, u, ws4, xs4, K, scale_l, tag);
         else consume_chunk<BT, 1, HS>(p, sh, kind, layer, u, ws4, xs4, K, scale_l, tag);
         loads++;
         cur = chunk_after(cur, MG_NW, sh, L);

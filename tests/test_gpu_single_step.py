@@ -53,6 +53,17 @@ def test_models_in_turn(slots):
             step(*m, pos, rng)
 
 
+@pytest.mark.parametrize("slots", [5, 6, 7, 8])
+def test_models_in_turn_of_up_to_eight_slots(slots):
+    """Two warps a staged row in place of four to sixteen; with the row pipeline, which takes these sizes from five slots on, switched off."""
+    lib = load_pkg("cabi").lib()
+    lib.check(lib.c.tha_set_option(b"tc", 0))
+    try:
+        test_models_in_turn(slots)
+    finally:
+        lib.check(lib.c.tha_set_option(b"tc", -1))
+
+
 def test_graph_replays_and_steps_in_a_row():
     cfg, w, e = model(12, 64, 12, 2048, 2, 2, 9)
     rng = np.random.default_rng(5)
