@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) chain_tf32x3_kernel(const __gri
       for (int i = i0; i < w.nst && ok; i += TC_CGROUPS) {
         const int g = gb + i, sw = g % S::SW, sa = g % S::SA;
         const int nk = (w.nkb - i * S::KG) < S::KG ? (w.nkb - i * S::KG) : S::KG;
-        ok = tc_mbar_wait_warp(&wfull[sw], (g / S::SW) & 1u, abort_flag);
+        ok = tc_mbar_wait(&wfull[sw], (g / S::SW) & 1u, abort_flag);
 #pragma unroll
         for (int kk = 0; kk < S::KG; kk++) {
           if (kk < nk && ok) {
@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) chain_tf32x3_kernel(const __gri
               lo[4 * j + 0] = __float_as_uint(v.x - h0); lo[4 * j + 1] = __float_as_uint(v.y - h1);
               lo[4 * j + 2] = __float_as_uint(v.z - h2); lo[4 * j + 3] = __float_as_uint(v.w - h3);
             }
-            if (kk == 0 && g >= S::SA && ok) ok = tc_mbar_wait_warp(&aempty[sa], ((g / S::SA) & 1u) ^ 1u, abort_flag);
+            if (kk == 0 && g >= S::SA && ok) ok = tc_mbar_wait(&aempty[sa], ((g / S::SA) & 1u) ^ 1u, abort_flag);
             const uint32_t ta = tmem_a + sa * S::A_STAGE + kk * S::A_COLS + ((uint32_t)(q * 32) << 16);
             tc_tmem_st32(ta, hi);
             tc_tmem_st32(ta + TC_BK, lo);
