@@ -94,7 +94,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_cons
   __shared__ float s_max[2][PTC_TQ];                 // row maxima / sums of the two column halves
   __shared__ uint64_t qbar, kbar, vbar, sbar, pbar;
   __shared__ uint32_t tmem_slot;
-  __shared__ int abort_s;
+  __shared__ int abort_s, key_tiles;                 // key_tiles: of K, and of V, that are asked for; thread 0's
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ptc_raw) + 1023) & ~(uintptr_t)1023);
   unsigned char *Qs = smem, *Ks = smem + TILE, *Vs = smem + 2 * TILE;
 
@@ -147,6 +147,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_cons
     }
     tc_commit(&sbar);
   };
+  if (tid == 0) key_tiles = live_tile ? kmax / PTC_TK + 1 : 0;
   bool ok = true;
   if (warp == 0 && live_tile) {
     if (tc_elect()) {
@@ -265,10 +266,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_cons
       *reinterpret_cast<uint4*>(orow + c) = make_uint4(ptc_bf16x2(acc[c] * inv, acc[c + 1] * inv), ptc_bf16x2(acc[c + 2] * inv, acc[c + 3] * inv),
                                                        ptc_bf16x2(acc[c + 4] * inv, acc[c + 5] * inv), ptc_bf16x2(acc[c + 6] * inv, acc[c + 7] * inv));
   }
-  if (warp == 0 && live_tile && *((volatile int*)abort_flag) && tc_elect()) {   // a tile of K and of V for every tile of keys
+  if (tid == 0 && *((volatile int*)&abort_s) && key_tiles) {
     tc_drain(&qbar, 1, 1);
-    tc_drain(&kbar, 1, kmax / PTC_TK + 1);
-    tc_drain(&vbar, 1, kmax / PTC_TK + 1);
+    tc_drain(&kbar, 1, key_tiles);
+    tc_drain(&vbar, 1, key_tiles);
   }
   __syncthreads();
   if (warp == 0) {

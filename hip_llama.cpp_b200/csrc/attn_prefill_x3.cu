@@ -188,7 +188,7 @@ attn_prefill_x3_kernel(const __grid_constant__ CUtensorMap mqh, const __grid_con
   __shared__ float s_vp[2][AX_T], s_vm[2][4];        // largest of s_vs up to a key of the warp's 32, of all 32
   __shared__ uint64_t qbar, kbar, vbar, sbar, pbar;
   __shared__ uint32_t tmem_slot;
-  __shared__ int abort_s;
+  __shared__ int abort_s, key_tiles;                 // key_tiles: of K, and of V, that are asked for; thread 0's
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ax_raw) + 1023) & ~(uintptr_t)1023);
   unsigned char *Qs = smem, *Ks = smem + 2 * TILE, *Vs = smem + 4 * TILE;      // each hi | lo
 
@@ -245,6 +245,7 @@ attn_prefill_x3_kernel(const __grid_constant__ CUtensorMap mqh, const __grid_con
     }
     tc_commit(&sbar);
   };
+  if (tid == 0) key_tiles = live_tile ? kmax / AX_T + 1 : 0;
   bool ok = true;
   if (warp == 0 && live_tile) {
     if (tc_elect()) {
@@ -403,10 +404,10 @@ attn_prefill_x3_kernel(const __grid_constant__ CUtensorMap mqh, const __grid_con
 #pragma unroll
     for (int c = 0; c < HH; c += 4) *reinterpret_cast<float4*>(orow + c) = make_float4(acc[c] / l, acc[c + 1] / l, acc[c + 2] / l, acc[c + 3] / l);
   }
-  if (warp == 0 && live_tile && *((volatile int*)abort_flag) && tc_elect()) {   // a tile of K and of V for every tile of keys
+  if (tid == 0 && *((volatile int*)&abort_s) && key_tiles) {
     tc_drain(&qbar, 1, 1);
-    tc_drain(&kbar, 1, kmax / AX_T + 1);
-    tc_drain(&vbar, 1, kmax / AX_T + 1);
+    tc_drain(&kbar, 1, key_tiles);
+    tc_drain(&vbar, 1, key_tiles);
   }
   __syncthreads();
   if (warp == 0) {

@@ -216,10 +216,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) chain_tf32x3_kernel(const __gri
         for (int i = 0; i < w.nst; i++) {
           const int g = gb + i, s = g % S::SW;
           if (i == w.nst - 1) CH_TRACE(9, n_it);
-          if (g >= S::SW && !tc_mbar_wait(&wfree[s], ((g / S::SW) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+          if (g >= S::SW && !tc_mbar_wait(&wfree[s], ((g / S::SW) & 1u) ^ 1u, abort_flag)) { ok = false; sent = g; break; }
           const int nk = (w.nkb - i * S::KG) < S::KG ? (w.nkb - i * S::KG) : S::KG;
           tc_mbar_expect_tx(&wfull[s], nk * S::W_BYTES);
-          sent = g + 1;
           for (int kk = 0; kk < nk; kk++) {
             unsigned char* dst = wring + s * S::W_STAGE + kk * S::W_BYTES;
             const int kc = (w.kb0 + i * S::KG + kk) * TC_BK;
@@ -257,7 +256,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) chain_tf32x3_kernel(const __gri
             if (*((volatile int*)abort_flag)) { ok = false; break; }
             if (tc_clock() - t0 > CH_DEP_TIMEOUT) { *abort_flag = 1; ok = false; break; }
           }
-          if (!ok) break;
+          if (!ok) { sent = gb; break; }
           ch_fence_async_global();   // the rows were written with generic stores; TMA reads them through the async proxy
         }
         CH_TRACE(0, n_it);
@@ -265,10 +264,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) chain_tf32x3_kernel(const __gri
         const CUtensorMap* mxl = &P.maps[f.xmap + 1];
         for (int i = 0; i < w.nst; i++) {
           const int g = gb + i, s = g % S::SX;
-          if (g >= S::SX && !tc_mbar_wait(&aempty[s], ((g / S::SX) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+          if (g >= S::SX && !tc_mbar_wait(&aempty[s], ((g / S::SX) & 1u) ^ 1u, abort_flag)) { ok = false; sent = g; break; }
           const int nk = (w.nkb - i * S::KG) < S::KG ? (w.nkb - i * S::KG) : S::KG;
           tc_mbar_expect_tx(&ready[s], nk * S::XS_BYTES);
-          sent = g + 1;
           for (int kk = 0; kk < nk; kk++) {
             unsigned char* st = xring + s * S::XS_STAGE + kk * S::XS_BYTES;
             tc_tma_2d(st, mxh, (w.kb0 + i * S::KG + kk) * TC_BK, w.n0, &ready[s]);
@@ -369,7 +367,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) chain_tf32x3_kernel(const __gri
         pdl_trigger();
         pdl_wait();
       }
-      if (ok) ok = tc_mbar_wait_warp(accum, n_it & 1u, abort_flag);
+      if (ok) ok = tc_mbar_wait(accum, n_it & 1u, abort_flag);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (et == 0) CH_TRACE(4, n_it);
       const int mode = f.mode;

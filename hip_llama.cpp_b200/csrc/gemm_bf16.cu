@@ -184,16 +184,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant_
           pdl_wait();
           for (int j = 0; j < pre; j++) {
             tc_mbar_expect_tx(&full[j], S::STAGE);
-            sent = j + 1;
             tc_tma_2d(smem + j * S::STAGE + S::W_BYTES, &mx, (w.kb0 + j) * BF_BK, w.xrow, &full[j]);
           }
           first = false;
         }
         for (; i < w.nkb; i++) {
           const int g = gb + i, s = g % S::NST;
-          if (g >= S::NST && !tc_mbar_wait(&empty[s], ((g / S::NST) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+          if (g >= S::NST && !tc_mbar_wait(&empty[s], ((g / S::NST) & 1u) ^ 1u, abort_flag)) { ok = false; sent = g; break; }
           tc_mbar_expect_tx(&full[s], S::STAGE);
-          sent = g + 1;
           load_w(smem + s * S::STAGE, mw, (w.kb0 + i) * BF_BK, w.wrow, &full[s]);
           tc_tma_2d(smem + s * S::STAGE + S::W_BYTES, &mx, (w.kb0 + i) * BF_BK, w.xrow, &full[s]);
         }
@@ -439,17 +437,13 @@ gemm_bf16_cluster_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_c
         tc_mbar_expect_tx(&full[i], S::STAGE);
         tc_tma_2d(smem + i * S::STAGE + S::W_BYTES, &mx, (kb0 + i) * BF_BK, xrow, &full[i]);
       }
-      int sent = pre;
-      bool ok = true;
-      for (int i = pre; i < nkb && ok; i++) {
+      for (int i = pre; i < nkb; i++) {
         const int s = i % S::NST;
-        if (!tc_mbar_wait(&empty[s], ((i / S::NST) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+        if (!tc_mbar_wait(&empty[s], ((i / S::NST) & 1u) ^ 1u, abort_flag)) { tc_drain(full, S::NST, i); break; }
         tc_mbar_expect_tx(&full[s], S::STAGE);
         load_w(i, s);
         tc_tma_2d(smem + s * S::STAGE + S::W_BYTES, &mx, (kb0 + i) * BF_BK, xrow, &full[s]);
-        sent = i + 1;
       }
-      if (!ok) tc_drain(full, S::NST, sent);
     }
   } else if (warp == 1) {
     if (tc_elect()) {

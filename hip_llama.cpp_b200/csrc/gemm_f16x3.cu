@@ -162,7 +162,7 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
 
   int gb = 0, n_it = 0, n_run = 0;      // k-blocks, items and runs so far, of both passes
   bool ok = true;
-  int sent = 0;                         // stages that a producer has asked for
+  int sent = -1;                        // stages that a producer has asked for, where it has given up
   // The end of a pass: whether there is another one, the same answer in both CTAs.  Every thread comes here, whatever became of its waits, and each of these is
   // bounded: so are the two CTAs' waits for each other.
   auto again = [&]() -> bool {
@@ -186,12 +186,11 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
             const CUtensorMap* mw = w.mat == 0 ? &mw0 : (w.mat == 1 ? &mw1 : &mw2);
             for (int i = 0; i < w.nkb; i++) {
               const int g = gb + i, s = g % S::SW;
-              if (g >= S::SW && !tc_mbar_wait(&wfree[s], ((g / S::SW) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+              if (g >= S::SW && !tc_mbar_wait(&wfree[s], ((g / S::SW) & 1u) ^ 1u, abort_flag)) { ok = false; sent = g; break; }
               tc_mbar_expect_tx(&wfull[s], S::W_STAGE);
               unsigned char* dst = wring + s * S::W_STAGE;
               tc_tma_2d(dst, mw, (w.kb0 + i) * X3_BK, w.row0, &wfull[s]);
               tc_tma_2d(dst + TC_BM * 128, mw, (w.kb0 + i) * X3_BK + 32, w.row0, &wfull[s]);
-              sent = g + 1;
             }
             gb += w.nkb;
           }
@@ -203,12 +202,11 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
             const Item w = item_of(it);
             for (int i = 0; i < w.nkb; i++) {
               const int g = gb + i, s = g % S::SX;
-              if (g >= S::SX && !tc_mbar_wait(&xempty[s], ((g / S::SX) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+              if (g >= S::SX && !tc_mbar_wait(&xempty[s], ((g / S::SX) & 1u) ^ 1u, abort_flag)) { ok = false; sent = g; break; }
               tc_mbar_expect_tx(&xfull[s], S::X_STAGE);
               unsigned char* dst = xring + s * S::X_STAGE;
               tc_tma_2d(dst, &mxh, (w.kb0 + i) * X3_BK, w.n0 + rank * (X3_NT / 2), &xfull[s]);
               tc_tma_2d(dst + S::X_PLANE, &mxl, (w.kb0 + i) * X3_BK, w.n0 + rank * (X3_NT / 2), &xfull[s]);
-              sent = g + 1;
             }
             gb += w.nkb;
           }
@@ -257,8 +255,8 @@ gemm_f16x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant
       if (!again()) break;
     }
     if (*((volatile int*)abort_flag)) {                // copies and MMAs end ahead of the blocks
-      if (warp == 0 && tc_elect()) tc_drain(wfull, S::SW, sent);
-      if (warp == 3 && tc_elect()) tc_drain(xfull, S::SX, sent);
+      if (warp == 0 && tc_elect()) tc_drain(wfull, S::SW, sent < 0 ? gb : sent);
+      if (warp == 3 && tc_elect()) tc_drain(xfull, S::SX, sent < 0 ? gb : sent);
       if (warp == 1 && rank == 0 && tc_elect()) {
         x3_commit(mmadone);
         tc_drain(mmadone, 1, 1);

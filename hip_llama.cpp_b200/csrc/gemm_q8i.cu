@@ -211,7 +211,6 @@ gemm_q8i_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant__
           for (int g = 0; g < n; g++) q8i_bulk(xs_sm + ((xr << gps_sh) + g) * NT, src + (size_t)g * p.ldxs, xbytes, &xfull[xr]);
           if (++xr == nxs) xr = 0;
           if (++s == nring) s = 0;
-          sent++;
         };
         int j = 0;
         if (jb == 0) {
@@ -229,7 +228,7 @@ gemm_q8i_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant__
             // The slot use whose MMAs must have completed.  They began when the stage nacc uses earlier had been read out, and a warp has
             // read a stage out only behind its last use of the scales before it: with nring + nacc + 1 scale buffers the next is free too.
             const int st = jg - nring;
-            if (!tc_mbar_wait(&mdone[st % S::NMD], (st / S::NMD) & 1u, abort_flag)) { ok = false; break; }
+            if (!tc_mbar_wait(&mdone[st % S::NMD], (st / S::NMD) & 1u, abort_flag)) { ok = false; sent = jg; break; }
           }
           tc_tma_2d_hint(smem + s * S::SLOT, mw, (w.slot0 + j) * 32, w.row0, &full[s], pol_w);
           activations(j);

@@ -136,10 +136,9 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constan
         const CUtensorMap* mw = (w.mat == 0) ? &mw0 : (w.mat == 1 ? &mw1 : &mw2);
         for (int i = 0; i < w.nst; i++) {
           const int g = gb + i, s = g % S::SW;
-          if (g >= S::SW && !tc_mbar_wait(&wfree[s], ((g / S::SW) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+          if (g >= S::SW && !tc_mbar_wait(&wfree[s], ((g / S::SW) & 1u) ^ 1u, abort_flag)) { ok = false; sent = g; break; }
           const int nk = (w.nkb - i * S::KG) < S::KG ? (w.nkb - i * S::KG) : S::KG;
           tc_mbar_expect_tx(&wfull[s], nk * S::W_BYTES);
-          sent = g + 1;
           TC_TRACE(0, i);
           for (int kk = 0; kk < nk; kk++)
             tc_tma_2d_hint(wring + s * S::W_STAGE + kk * S::W_BYTES, mw, (w.kb0 + i * S::KG + kk) * TC_BK, w.row0, &wfull[s], pol_w);
@@ -160,11 +159,10 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constan
         const Item w = item_of(it);
         for (int i = 0; i < w.nst; i++) {
           const int g = gb + i, s = g % S::SX;
-          if (g >= S::SX && !tc_mbar_wait(&aempty[s], ((g / S::SX) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+          if (g >= S::SX && !tc_mbar_wait(&aempty[s], ((g / S::SX) & 1u) ^ 1u, abort_flag)) { ok = false; sent = g; break; }
           const int nk = (w.nkb - i * S::KG) < S::KG ? (w.nkb - i * S::KG) : S::KG;
           TC_TRACE(1, i);
           tc_mbar_expect_tx(&ready[s], nk * S::XS_BYTES);
-          sent = g + 1;
           for (int kk = 0; kk < nk; kk++) {
             unsigned char* st = xring + s * S::XS_STAGE + kk * S::XS_BYTES;
             tc_tma_2d(st, &mxh, (w.kb0 + i * S::KG + kk) * TC_BK, w.n0, &ready[s]);
@@ -271,7 +269,7 @@ gemm_tf32x3_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constan
         pdl_trigger();
         pdl_wait();   // returns at once (the X producer already waited); makes the predecessor's writes visible to these threads
       }
-      if (ok) ok = tc_mbar_wait_warp(accum, n_it & 1u, abort_flag);
+      if (ok) ok = tc_mbar_wait(accum, n_it & 1u, abort_flag);
       if (n_it == 0 && threadIdx.x == 128) kt_stamp(kt, 4);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int row = w.row0 + r;

@@ -367,12 +367,10 @@ __global__ void __launch_bounds__(AT_THREADS, 1) hyb_attn_tc_kernel(const __grid
     // ===== tiles: two halves of 32 keys, each a box of 64 channels at a time
     if (tc_elect()) {
       bool ok = true;
-      int sent = 0;
       for (int j = 0; j < n && ok; j++) {
         const int st = j % AT_STAGES;
-        if (j >= AT_STAGES && !tc_mbar_wait(&kv_empty[st], (unsigned)(j / AT_STAGES - 1) & 1u, abort_flag)) { ok = false; break; }
+        if (j >= AT_STAGES && !tc_mbar_wait(&kv_empty[st], (unsigned)(j / AT_STAGES - 1) & 1u, abort_flag)) { ok = false; tc_drain(kv_full, AT_STAGES, j); break; }
         tc_mbar_expect_tx(&kv_full[st], KV_STAGE);
-        sent = j + 1;
 #pragma unroll
         for (int hf = 0; hf < 2; hf++) {
           // behind the last half its own rows again: finite, and masked
@@ -385,7 +383,6 @@ __global__ void __launch_bounds__(AT_THREADS, 1) hyb_attn_tc_kernel(const __grid
           }
         }
       }
-      if (!ok) tc_drain(kv_full, AT_STAGES, sent);
     }
   } else if (tc_elect()) {
     // ===== products

@@ -39,9 +39,12 @@ __device__ __forceinline__ void split_f16x2(float2 v, float s, uint32_t& hi, uin
   const float up = s * SPLIT_UP;
   lo = f16x2_of(f32x2_fma(h, make_float2(-SPLIT_UP, -SPLIT_UP), f32x2_mul(v, make_float2(up, up))));   // every step of it is exact but the last rounding
 }
+// (row kernels, bound by memory: single operations leave them more registers for loads in flight)
 __device__ __forceinline__ void split_f16x4(float4 v, float s, uint2& hi, uint2& lo) {
-  split_f16x2(make_float2(v.x, v.y), s, hi.x, lo.x);
-  split_f16x2(make_float2(v.z, v.w), s, hi.y, lo.y);
+  v.x *= s; v.y *= s; v.z *= s; v.w *= s;
+  hi = make_uint2(f16x2_of(make_float2(v.x, v.y)), f16x2_of(make_float2(v.z, v.w)));
+  const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&hi.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&hi.y));
+  lo = make_uint2(f16x2_of(make_float2((v.x - a.x) * SPLIT_UP, (v.y - a.y) * SPLIT_UP)), f16x2_of(make_float2((v.z - b.x) * SPLIT_UP, (v.w - b.y) * SPLIT_UP)));
 }
 // The power of two, 2^MOST at most, that brings |v| to [2^e, 2^(e+1)), and its inverse
 template <int MOST>
