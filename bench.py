@@ -683,6 +683,10 @@ def tp_extra(args, rank, world, local_rank, B=64, W=3, K=10):
 
 
 # ------------------------------------------------------------------ the reference's CPU path ----
+class ReferenceMissing(RuntimeError):
+    """The reference's own sources were not there to be compiled."""
+
+
 def cpu_reference(args, cfg, host_w, n_seqs, n_threads, max_steps, warmup, budget_s):
     """Time oracle/_ref (run.cc / runq.c compiled unmodified; -O3 -mavx2 -mfma build) on the host.
     fp32: run.cc has no OpenMP pragma, so threads run independent sequences (one forward() each per
@@ -695,7 +699,7 @@ def cpu_reference(args, cfg, host_w, n_seqs, n_threads, max_steps, warmup, budge
     kindname = "q8" if q8 else "fp32"
     fast = cpu_has_avx2_fma() and ref_available(kindname, fast=True)
     if not ref_available(kindname, fast=fast):
-        raise RuntimeError("oracle/_ref is not built (run __graft_entry__.build() where the reference's sources are)")
+        raise ReferenceMissing("oracle/_ref is not built (run __graft_entry__.build() where the reference's sources are)")
     if host_w is None:
         host_w = ck.random_weights(cfg, seed=1337, std=0.02)
     with tempfile.TemporaryDirectory() as td:
@@ -785,7 +789,11 @@ def main():
         cores = host_cores()
         n_seqs = min(args.batch * max(world, 1), 2 * cores)
         threads = cores if args.quant == "q8" else min(cores, n_seqs)
-        v, done, kind, used, fast = cpu_reference(args, cfg, None, n_seqs, threads, args.steps, min(args.warmup, 2), 150.0)
+        try:
+            v, done, kind, used, fast = cpu_reference(args, cfg, None, n_seqs, threads, args.steps, min(args.warmup, 2), 150.0)
+        except ReferenceMissing as ex:
+            print(json.dumps({"impl": "reference", "unavailable": str(ex)}), flush=True)
+            return 0
         line = base_line(args, cfg, world)
         sample = (f"{n_seqs} sequences x {done} greedy decode positions from pos 0 through oracle/_ref "
                   f"({'runq.c' if args.quant == 'q8' else 'run.cc'} compiled unmodified, "
