@@ -57,20 +57,6 @@ __device__ __forceinline__ void ptc_tmem_ld32(uint32_t taddr, uint32_t (&v)[32])
 __host__ __device__ constexpr uint32_t ptc_idesc(int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
-__device__ __forceinline__ void ptc_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void ptc_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
 __device__ __forceinline__ void ptc_tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
@@ -143,7 +129,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_cons
     for (int kb = 0; kb < KBH; kb++) {
       const uint64_t a = tc_smem_desc(tc_smem_u32(Qs + kb * (128 * 128))), b = tc_smem_desc(tc_smem_u32(Ks + kb * (128 * 128)));
 #pragma unroll
-      for (int k = 0; k < 4; k++) ptc_mma(tmem_s, a + (uint64_t)(2 * k), b + (uint64_t)(2 * k), idesc, (uint32_t)((kb | k) != 0));
+      for (int k = 0; k < 4; k++) tc_mma_f16(tmem_s, a + (uint64_t)(2 * k), b + (uint64_t)(2 * k), idesc, (uint32_t)((kb | k) != 0));
     }
     tc_commit(&sbar);
   };
@@ -229,7 +215,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap mq, const __grid_cons
         const uint64_t b = ptc_desc_mn(tc_smem_u32(Vs), 128 * 128);
         const int groups = more ? PTC_TK / 16 : (kmax - t0 + 16) / 16;
         for (int x = 0; x < groups; x++)
-          ptc_mma_ts(tmem_pv, tmem_s + (uint32_t)(64 * (x >> 2) + 8 * (x & 3)), b + (uint64_t)(x * (2048 >> 4)), idesc, (uint32_t)(x != 0));
+          tc_mma_f16_ts(tmem_pv, tmem_s + (uint32_t)(64 * (x >> 2) + 8 * (x & 3)), b + (uint64_t)(x * (2048 >> 4)), idesc, (uint32_t)(x != 0));
         tc_commit(&pbar);
       }
       __syncwarp();

@@ -7,8 +7,9 @@
 // over times 2^-11 (the MMA's scale of its input D).
 //
 // CTA = 128 consecutive query rows of one (sequence, head), 256 threads, two a row (attn_prefill_tc.cu); tiles of 128 keys.  A chain
-// of S, softmax, P V and accumulator, in which the next tile's loads and its S run ahead; heads of 64 have two CTAs an SM (96 KB), of 128 one (192 KB).  Bound by the
-// softmax threads (some 20 instructions a score) and, at one CTA an SM, by the chain.
+// of S, softmax, P V and accumulator, in which the next tile's loads and its S run ahead; heads of 64 have two CTAs an SM (96 KB), of 128 one (192 KB).  Bound by that
+// chain: issue slots 29 and 32 % busy, the tensor pipe 23 and 10 % (heads of 128, one prompt of 1024; of 64, 16 of 9 .. 201).  A layer of these 333 -> 61 us and 38 -> 21
+// against attn_prefill.cu.
 #include <cuda.h>
 
 #include "common.cuh"
@@ -140,13 +141,6 @@ __device__ __forceinline__ void ax_tmem_st8(uint32_t taddr, const uint32_t (&v)[
 }
 // kind::f16, fp16 x fp16 -> fp32, M = 128, N = n, A and B K-major
 __host__ __device__ constexpr uint32_t ax_idesc(int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24); }
-__device__ __forceinline__ void ax_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
 // D = A B + D 2^-11
 __device__ __forceinline__ void ax_mma_over(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc) {
   asm volatile(
@@ -154,13 +148,6 @@ __device__ __forceinline__ void ax_mma_over(uint32_t tmem_d, uint64_t adesc, uin
       "setp.eq.b32 p, 0, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p, %4;\n\t}"
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "n"(SPLIT_LO) : "memory");
-}
-__device__ __forceinline__ void ax_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void ax_mma_ts_over(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc) {
   asm volatile(
@@ -239,7 +226,7 @@ attn_prefill_x3_kernel(const __grid_constant__ CUtensorMap mqh, const __grid_con
 #pragma unroll
         for (int k = 0; k < 4; k++) {
           if (part == 2 && (kb | k) == 0) ax_mma_over(tmem_s, a, b, idesc);
-          else ax_mma(tmem_s, a + (uint64_t)(2 * k), b + (uint64_t)(2 * k), idesc, (uint32_t)((part | kb | k) != 0));
+          else tc_mma_f16(tmem_s, a + (uint64_t)(2 * k), b + (uint64_t)(2 * k), idesc, (uint32_t)((part | kb | k) != 0));
         }
       }
     }
@@ -364,11 +351,11 @@ attn_prefill_x3_kernel(const __grid_constant__ CUtensorMap mqh, const __grid_con
         const int groups = more ? AX_T / 16 : (kmax - t0 + 16) / 16;
         for (int x = 0; x < groups; x++) {
           const uint32_t a = tmem_s + (uint32_t)(16 * x);
-          ax_mma_ts(tmem_pv, a + 8, vh + (uint64_t)(x * (2048 >> 4)), idesc, (uint32_t)(x != 0));
-          ax_mma_ts(tmem_pv, a, vl + (uint64_t)(x * (2048 >> 4)), idesc, 1u);
+          tc_mma_f16_ts(tmem_pv, a + 8, vh + (uint64_t)(x * (2048 >> 4)), idesc, (uint32_t)(x != 0));
+          tc_mma_f16_ts(tmem_pv, a, vl + (uint64_t)(x * (2048 >> 4)), idesc, 1u);
         }
         ax_mma_ts_over(tmem_pv, tmem_s, vh, idesc);
-        for (int x = 1; x < groups; x++) ax_mma_ts(tmem_pv, tmem_s + (uint32_t)(16 * x), vh + (uint64_t)(x * (2048 >> 4)), idesc, 1u);
+        for (int x = 1; x < groups; x++) tc_mma_f16_ts(tmem_pv, tmem_s + (uint32_t)(16 * x), vh + (uint64_t)(x * (2048 >> 4)), idesc, 1u);
         tc_commit(&pbar);
       }
       __syncwarp();

@@ -66,13 +66,6 @@ struct BfSmem {
 __host__ __device__ constexpr uint32_t bf_idesc(int nt) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(nt >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
 }
-__device__ __forceinline__ void bf_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
 
 // Sixteen columns of a row through an activation (THA_ACT_*) and out as bf16: the branch on the activation is taken once per sixteen.
 template <int ACT>
@@ -223,7 +216,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_constant_
           for (int k = 0; k < BF_BK / 16; k++)     // UMMA K = 16 bf16 = 32 bytes = 2 descriptor units
 #pragma unroll
             for (int m = 0; m < MT; m++)           // the m-th 128 rows of the W stage: 16 KB = 1024 descriptor units further
-              bf_mma(d + (uint32_t)(m * NT), adesc + (uint64_t)(1024 * m + 2 * k), bdesc + (uint64_t)(2 * k), idesc, (uint32_t)((i | k) != 0));
+              tc_mma_f16(d + (uint32_t)(m * NT), adesc + (uint64_t)(1024 * m + 2 * k), bdesc + (uint64_t)(2 * k), idesc, (uint32_t)((i | k) != 0));
           tc_commit(&empty[s]);
         }
         if (ok) tc_commit(&accum[buf]);
@@ -456,7 +449,7 @@ gemm_bf16_cluster_kernel(const __grid_constant__ CUtensorMap mw0, const __grid_c
         const uint64_t adesc = tc_smem_desc(tc_smem_u32(smem + s * S::STAGE));
         const uint64_t bdesc = tc_smem_desc(tc_smem_u32(smem + s * S::STAGE + S::W_BYTES));
 #pragma unroll
-        for (int k = 0; k < BF_BK / 16; k++) bf_mma(tmem_d, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, (uint32_t)((i | k) != 0));
+        for (int k = 0; k < BF_BK / 16; k++) tc_mma_f16(tmem_d, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, (uint32_t)((i | k) != 0));
         tc_commit(&empty[s]);
       }
       if (ok && nkb > 0) tc_commit(accum);

@@ -10,12 +10,12 @@
 // sum takes K / 16 additions (3xTF32: K / 8); the corrections join it in the read-out, times 2^-11.
 //
 // A pair of CTAs (cta_group::2) takes 256 weight rows x 128 activation rows: each has 128 of the weight rows, in TMEM, and 64 of the activation rows, in shared
-// memory, that both halves of the MMA read.  Bound by the tensor pipe under the power limit and by the last, partly filled round over the 74 pairs; the tf32 kernel was
-// bound by what reaches shared memory through L2: per 64 values of K a CTA loads 32 KB of weights and 16 KB of activations for 768 cycles of MMAs, there 32 + 64 KB for
-// 1536 (and took 2100).  1024 rows x 22016 x 4096: 800 us with 3xTF32, 460 with this, 400 for three products at the sustained cuBLAS bf16 rate;
-// 4096 x 11008: 480, 250 (200); 1936 rows of 768, 4096 outputs: 70, 52 (26).
+// memory, that both halves of the MMA read.  Bound by the tensor pipe under the power limit (73 % of its cycles active at 1024 rows x 12288 x 4096) and by the last, partly
+// filled round over the 74 pairs (51 % at 1936 rows of 768, 4096 outputs); the tf32 kernel was bound by what reaches shared memory through L2: per 64 values of K a CTA loads
+// 32 KB of weights and 16 KB of activations for 768 cycles of MMAs, there 32 + 64 KB for 1536 (and took 2100).  The kernel by itself, 1024 rows x 22016 x 4096: 675 us with
+// 3xTF32, 472 with this, 400 for three products at the sustained cuBLAS bf16 rate; 4096 x 11008: 364, 238 (200); 1936 rows of 768, 4096 outputs: 58, 43 (26).
 // The MMAs sum up runs of 1024 values of K, the read-out adds the runs in its registers: the tensor core's sum loses up to a unit in the last place with every
-// addition.  Relative error at K = 4096: 9.6e-6 with 3xTF32, 4.9e-6 with one run, 1.25e-6 with runs of 1024 (6.5e-7 of 512; 267, 275 and 285 us for 12288 x 4096).
+// addition.  Relative error at K = 4096: 9.6e-6 with 3xTF32, 4.9e-6 with one run, 1.25e-6 with runs of 1024 (6.5e-7 of 512; 3 and 7 % more time than one run).
 // Announcements across the pair carry no generic memory, so no fence: with release and acquire at cluster scope the same products took 418 us in place of 267.
 //   warp 0      TMA producer of W (weights: ahead of griddepcontrol.wait)
 //   warp 1      rank 0: MMA issuer of the pair; rank 1: tells it that a stage of X has landed

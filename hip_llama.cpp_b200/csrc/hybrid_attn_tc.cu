@@ -74,14 +74,6 @@ __host__ __device__ constexpr uint32_t at_idesc(int n, int b_mn) {
 __device__ __forceinline__ uint64_t at_desc_mn(uint32_t saddr, uint32_t block) {
   return (uint64_t)((saddr & 0x3FFFFu) >> 4) | (uint64_t)(block >> 4) << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;
 }
-__device__ __forceinline__ void at_mma_ss(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-               ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc) : "memory");
-}
-__device__ __forceinline__ void at_mma_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-               ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(acc) : "memory");
-}
 
 // Where the staged rows of sequence `seq` begin: behind those of the sequences ahead of it that have min_rows rows in the step, each up to a multiple of 32.
 __device__ __forceinline__ int at_stage_rows(const tha_rows_t& rows, int s, int min_rows) {
@@ -395,7 +387,7 @@ __global__ void __launch_bounds__(AT_THREADS, 1) hyb_attn_tc_kernel(const __grid
       for (int kb = 0; kb < KB; kb++) {
         const uint64_t ad = tc_smem_desc(q_addr + (uint32_t)(w * Q_GROUP + kb * AT_ROWS * 128)), bd = tc_smem_desc(k + (uint32_t)(kb * AT_KEYS * 128));
 #pragma unroll
-        for (int x = 0; x < 4; x++) at_mma_ss(d, ad + (uint64_t)(2 * x), bd + (uint64_t)(2 * x), id_s, (uint32_t)((kb | x) != 0));
+        for (int x = 0; x < 4; x++) tc_mma_f16(d, ad + (uint64_t)(2 * x), bd + (uint64_t)(2 * x), id_s, (uint32_t)((kb | x) != 0));
       }
       tc_commit(&s_full[w][j & 1]);
     };
@@ -419,8 +411,8 @@ __global__ void __launch_bounds__(AT_THREADS, 1) hyb_attn_tc_kernel(const __grid
         const uint64_t vd = at_desc_mn(kv_addr + (uint32_t)((j % AT_STAGES) * KV_STAGE + K_STAGE), AT_KEYS * 128);
 #pragma unroll
         for (int x = 0; x < AT_KEYS / 16; x++) {
-          at_mma_ts(d, p + (uint32_t)(8 * x), vd + (uint64_t)(x * (2048 >> 4)), id_o, (uint32_t)((j | x) != 0));
-          if (EXACT) at_mma_ts(d, p + (uint32_t)(32 + 8 * x), vd + (uint64_t)(x * (2048 >> 4)), id_o, 1u);
+          tc_mma_f16_ts(d, p + (uint32_t)(8 * x), vd + (uint64_t)(x * (2048 >> 4)), id_o, (uint32_t)((j | x) != 0));
+          if (EXACT) tc_mma_f16_ts(d, p + (uint32_t)(32 + 8 * x), vd + (uint64_t)(x * (2048 >> 4)), id_o, 1u);
         }
         tc_commit(&pv_done[w][j & 1]);
       }

@@ -132,7 +132,7 @@ __global__ void hyb_block_finish_kernel(float* __restrict__ x, const float* __re
 // ---- the same two passes with the row in registers: widths of up to 4096 that are a multiple of four, 16-byte aligned ----
 // P float4 a thread.  The kernels above write x and read it back for each sum; here all that a thread needs of the row and of the norm is asked
 // for at once.  Bound by the latency of one load, two block sums and a store where there are few rows (decoding: 20 to 100 such kernels a
-// step).  3 rows of 1024, behind the kernel ahead: 4.2 -> 1.5 us and 3.5 -> 1.4; 2000 rows: 13 -> 7.7.
+// step).  Launched plainly, 3 rows of 1024 (and once in nine their prompts): 4.6 -> 2.6 us and 4.1 -> 2.2.
 template <int P, typename T>
 __device__ __forceinline__ void row_norm(const HybRow<P>& x, const HybRow<P>& w, const HybRow<P>& b, const tha_norm_t& n, float eps, T* out, int width, HybRowSum<P>& sm) {
   HybRow<P> y;

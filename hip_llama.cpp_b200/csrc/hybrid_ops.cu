@@ -35,8 +35,8 @@ __global__ void hyb_rmsnorm_kernel(T* __restrict__ out, const float* __restrict_
   for (int i = threadIdx.x; i < width; i += blockDim.x) hyb_store(out + (size_t)r * width + i, xr[i] * inv * (w_offset + (w ? w[i] : 0.f)));
 }
 
-// the same with the row in registers: widths of up to 4096 that are a multiple of four, 16-byte aligned.  Bound by latency: 3 rows of 1024, behind the kernel
-// ahead, 2.9 -> 1.8 us
+// the same with the row in registers: widths of up to 4096 that are a multiple of four, 16-byte aligned.  Bound by latency: launched plainly, 3 rows of 1024
+// (and once in nine their prompts), 3.5 -> 1.95 us
 template <typename T, int P>
 __global__ void __launch_bounds__(ROW_THREADS) hyb_rmsnorm_row_kernel(T* out, const float* x, const float* w, float w_offset, float eps, int width, const int* rows_idx) {
   hyb_pdl_enter();
@@ -1370,7 +1370,7 @@ __global__ void hyb_head_gate_kernel(T* __restrict__ out, const float* __restric
 }
 
 // the same with a head's columns in registers, four of every 128 a lane: heads of up to 512 columns, a multiple of four, everything 16-byte aligned.  The squares
-// change hands to be added in the same order.  3 rows of 8 heads of 128, behind the kernel ahead: 4.5 -> 2.0 us
+// change hands to be added in the same order.  Launched plainly, 3 rows of 8 heads of 128 and 256 (and once in nine their prompts): 5.0 -> 3.0 us
 template <typename T, int P>
 __global__ void __launch_bounds__(128) hyb_head_gate4_kernel(T* out, const float* o_raw, int n_rows, int heads, int E, float eps, const float* norm, int norm_per_head,
                                                              const float* gate, long long ldg, int do_norm, int gate_act) {
@@ -1986,7 +1986,7 @@ extern "C" int tha_hyb_attn_prepare(void* stream, const tha_attn_t* a, const tha
       a->kv_heads / (a->v_share > 1 ? a->v_share : 1) * a->vdim > kv->kv_dim || (a->v_is_k && a->vdim != a->dim))
     return THA_STATUS_INVALID_ARG;
   if (hyb_attn_prepare_ok(a, kv, proj, ldp, rot_dims, q_out)) {
-    // a warp a head where rows are few (a decode step's 6.5 -> 2.2 us), blocks of eight warps for portions, several an SM (4000 rows of 3072 columns 46 -> 31 us)
+    // a warp a head where rows are few (launched plainly, a decode step's 6.8 -> 3.5 us), blocks of eight warps for portions, several an SM (4000 rows of 3072 columns 46 -> 36 us)
     const bool few = rows->n_rows <= 148;
     const int warps = a->heads + 2 * a->kv_heads, most = few ? 32 : 8;
     THA_CUDA_OK(launch(few ? hyb_attn_prepare4_kernel<1024> : hyb_attn_prepare4_kernel<256>, dim3(rows->n_rows), dim3(32 * (warps < most ? warps : most)), 0,

@@ -297,7 +297,8 @@ int tha_advance_slots(void* stream, int n_batches, int* token_d, int* pos_d, con
  * decode step (src/llama.cpp:1029-1030); this runs all prompt positions of n_seqs sequences through the tcgen05
  * matmuls in one pass.  HOST arrays: sequence i lives in cache slab slot_host[i]; its len_host[i] tokens (concatenated
  * in tokens_host, sequence after sequence) go to positions pos0_host[i] .. pos0_host[i]+len_host[i]-1.  Every row's K/V
- * is written to the cache exactly where the decode step would have put it.  logits_d (device, [n_seqs, vocab], nullable):
+ * is written to the cache exactly where the decode step would have put it; every portion sees the call's rows at the positions before
+ * its own, another portion of its slot (or of a slot whose block table shares the block) included, in whatever order they come.  logits_d (device, [n_seqs, vocab], nullable):
  * logits of the LAST position of each sequence; next_d (device, [n_seqs], nullable): their argmax.  With logits_d == NULL
  * the call only fills the cache.  Asynchronous on `stream`; the host arrays may be reused when it returns. */
 int tha_prefill_f32(void* stream, const tha_config_t* cfg, const tha_weights_f32_t* w, const tha_state_t* s, int n_seqs,

@@ -37,3 +37,27 @@ def test_portions_of_one_sequence(heads, hs, kv_heads, lens, how):
         want, _, _ = llama64.forward(cfg, w.t, lambda c, s, l, n: e.state.key_cache[:0].reshape(-1, kv_heads * hs)[:0], [(0, 0, toks[:at[i + 1]])])
         # products of up to 2048 terms at 1e-6 to 1e-5 each (test_gpu_prompt_rows.py), through two layers
         assert float((got[row].double() - want[0]).norm() / want.norm()) < 5e-5
+
+
+@pytest.mark.parametrize("kind", ["q8", "bf16"])
+@pytest.mark.parametrize("lens", [[20, 12], [200, 57], [300, 400]])
+@pytest.mark.parametrize("reverse", [False, True])
+def test_portions_of_the_other_formats(kind, lens, reverse):
+    """Against the whole sequence as one portion: the second layer's cache rows, a value in some hundred of which may fall on the other side of a quantiser's or a bf16 step."""
+    eng, ck = load_pkg("engine"), load_pkg("checkpoint")
+    cfg = ck.Config(1024, 1024, 2, 8, 8, 96, 768)
+    w = eng.DeviceWeightsBF16.random(cfg, seed=2) if kind == "bf16" else eng.device_random_weights(cfg, q8=True, seed=2, gs=64)
+    toks = np.random.default_rng(3).integers(0, 96, sum(lens)).astype(np.int32)
+    at = np.cumsum([0] + lens)
+    parts = [(0, int(at[i]), toks[at[i]:at[i + 1]]) for i in range(len(lens))]
+    rows = []
+    for seqs in (parts[::-1] if reverse else parts, [(0, 0, toks)]):
+        e = eng.Engine(w, 1, with_att=False)
+        e.state.key_cache.normal_(0.0, 1.0)
+        e.state.value_cache.normal_(0.0, 1.0)
+        out = torch.empty(len(seqs), 96, device="cuda")
+        torch.cuda.synchronize()
+        e.prefill(seqs, out)
+        torch.cuda.synchronize()
+        rows.append(torch.stack([e.state.key_cache[0, 1, :sum(lens)], e.state.value_cache[0, 1, :sum(lens)]]).double())
+    assert float((rows[0] - rows[1]).norm() / rows[1].norm()) < 2e-2
