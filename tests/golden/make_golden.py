@@ -1,6 +1,6 @@
 """Generate the committed golden fixtures from the REFERENCE ITSELF.
 
-Runs only in the build container (needs /root/reference and oracle/_ref); the
+Runs only in the build container (needs the reference sources and oracle/_ref); the
 GPU box never runs it -- tests read the files it leaves in tests/golden/.
 
 For each tiny architecture:
@@ -8,7 +8,7 @@ For each tiny architecture:
   2. export it with the reference's own `train/export.py` (`legacy_export`, `version2_export`),
   3. run the reference's compiled CPU code (run.cc / runq.c via oracle/_ref) token by token
      and record logits, the KV cache, and (Q8_0) the last quantised activation.
-Also: tokenizer known answers -- the vectors of /root/reference/test.c:49-75 are re-checked
+Also: tokenizer known answers -- the vectors of test.c:49-75 are re-checked
 against run.cc's encode(), and the encodings of the gen_in prompts are recorded.
 
 usage: python tests/golden/make_golden.py
@@ -160,7 +160,7 @@ def main():
             [1, 3439, 17632, 1925, 29892, 278, 6368, 310, 14215, 537, 5922, 393, 29871],
     }
     buf = (C.c_int * 4096)()
-    for text, want in kat.items():  # vectors of /root/reference/test.c:49-63
+    for text, want in kat.items():  # vectors of test.c:49-63
         n = l32.ref32_encode(tok, text.encode(), 1, 0, buf)
         assert list(buf[:n]) == want, (text, list(buf[:n]))
     with open(os.path.join(REF, "assets/in/gen_in_128.txt")) as f:

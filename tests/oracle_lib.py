@@ -213,7 +213,7 @@ def cpu_has_avx2_fma():
 
 
 class Ref32:
-    """/root/reference/run.cc compiled unmodified (oracle/ref_shim_fp32.cc)."""
+    """run.cc compiled unmodified (oracle/ref_shim_fp32.cc)."""
 
     def __init__(self, fast=False):
         lib = C.CDLL(os.path.join(ORACLE_DIR, "_ref", f"libref_fp32{'_fast' if fast else ''}.so"))
@@ -257,7 +257,7 @@ class Ref32:
 
 
 class RefQ8:
-    """/root/reference/runq.c compiled unmodified (oracle/ref_shim_q8.c)."""
+    """runq.c compiled unmodified (oracle/ref_shim_q8.c)."""
 
     def __init__(self, fast=False):
         lib = C.CDLL(os.path.join(ORACLE_DIR, "_ref", f"libref_q8{'_fast' if fast else ''}.so"))

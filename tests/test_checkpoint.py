@@ -33,7 +33,7 @@ def test_named_shapes():
     assert ck.hidden_dim_for(768, 32) == 2048
     assert ck.hidden_dim_for(4096, 256) == 11008
     n = sum(int(np.prod(s)) for s in ck.tensor_shapes(ck.STORIES110M).values())
-    assert n == 109_529_856
+    assert n == 109_529_856  # the published parameter count
     assert 28 + 4 * n + 2 * 4 * (1024 * 64 // 2) == 438_381_596
 
 

@@ -1,11 +1,11 @@
-"""Parity at the shapes BASELINE.json names, through the same entry points bench.py times.
+"""Parity at the shapes that are quoted, through the same entry points bench.py times.
 
-  * stories110M fp32 at 256 slots (configs[1], the headline line): the tensor-core row pipeline with two 128-column
+  * stories110M fp32 at 256 slots (the headline line): the tensor-core row pipeline with two 128-column
     tiles and the planner's split-K, teacher-forced from position 0 past position 64, sampled slots against the
     oracle at the reference's own 1e-4 (scripts/test/thaDNN.test.cpp:224, full-forward check :541-548);
-  * stories110M Q8_0 at 64 slots (configs[2]);
+  * stories110M Q8_0 at 64 slots;
   * a 2-layer truncation at Llama-2-7B widths (dim 4096, hidden 11008, 32 heads, vocab 32000), fp32 and Q8_0, at
-    1 / 8 / 64 slots (configs[3], configs[4]);
+    1 / 8 / 64 slots;
   * Q8_0 layer by layer with EXACT inputs: every layer of a model as its own 1-layer model whose embedding rows are
     realistic activations, so no rounding flip of an earlier layer reaches the comparison (runq.c:344-481).
 The oracle runs a handful of sampled slots only (it needs ~70 ms per stories110M position and core)."""

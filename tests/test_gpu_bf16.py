@@ -1,4 +1,4 @@
-"""The bf16 model path (csrc/step_bf16.cu, gemm_bf16.cu; BASELINE.json configs[3] "fp32/bf16") against the oracle's
+"""The bf16 model path (csrc/step_bf16.cu, gemm_bf16.cu) against the oracle's
 restatement of the same rule: bf16-rounded weights, every vector entering a weight matmul rounded to bf16 (nearest even),
 everything else fp32 as run.cc:244-374.  GPU and oracle then differ by fp32 accumulation order (~1e-7), plus -- now and
 then -- a value that sits on a bf16 rounding boundary and lands on the other side: that element moves by 2^-8 of its

@@ -2,7 +2,7 @@
 (thaDNN_s_forward_batch -> tha_forward_batch_*): logits and KV cache against the committed
 golden vectors (produced by the reference's run.cc / runq.c) and against the oracle on
 seeded models.  Tolerances: fp32 logits 1e-4 abs-or-rel (scripts/test/thaDNN.test.cpp:224);
-Q8_0 logits 1e-3 abs-or-rel (SURVEY.md 8d config 3)."""
+Q8_0 logits 1e-3 abs-or-rel."""
 import os
 
 import numpy as np
@@ -127,7 +127,7 @@ def test_fp32_tensor_core_step_vs_oracle(oracle, tmp_path, name, B):
     assert flips == 0
 
 
-# the attention shape of Llama-2-70B (SURVEY.md 8 f4: the reference's 70B drivers stream layers because the model does not fit
+# the attention shape of Llama-2-70B (the reference's 70B drivers stream layers because the model does not fit
 # its GPUs; on a B200 a 70B Q8_0 / bf16 model is resident and only the grouped-query attention differs from 7B): 8 query heads
 # of 128 on one K/V head -- a CTA covers the whole group (J = 8), RoPE stays its own kernel
 GQA70 = dict(dim=1024, hidden_dim=2816, n_layers=2, n_heads=8, n_kv_heads=1, vocab_size=512, seq_len=72)
@@ -447,7 +447,7 @@ def test_stories110m_shape_q8_vs_oracle(oracle, tmp_path):
     w = ck.random_weights(cfg, seed=1337, std=0.05)
     v2 = str(tmp_path / "s110m_v2.bin")
     ck.write_v2(v2, cfg, w)
-    assert os.path.getsize(v2) == 116_432_128
+    assert os.path.getsize(v2) == 116_432_128   # 109529856 parameters
     e = engine_from_v2(v2, 2)
     m = oracle.open(v2, quantized=True)
     run_ragged(e, m, 5, 2, np.random.default_rng(8), Q8_E2E_EPS, q8=True)

@@ -1,6 +1,6 @@
 """Per-op parity on the B200: every thaBLAS / thaDNN entry point, called through the C-ABI,
 against the oracle, with the shapes and tolerances of the reference's own comparers
-(scripts/test/thaBLAS.test.cpp, scripts/test/thaDNN.test.cpp; SURVEY.md section 4)."""
+(scripts/test/thaBLAS.test.cpp, scripts/test/thaDNN.test.cpp)."""
 import ctypes as C
 
 import numpy as np
@@ -128,7 +128,7 @@ def test_matmul_tensor_cores(L, m, n, k):
     assert_close_scaled(Cc.cpu().numpy(), want, 2e-5, f"matmul {m}x{n}x{k} on the tensor cores")
 
 
-# the weight matmul: stories110M and 7B shapes (SURVEY 7.2), odd shapes through the scalar path
+# the weight matmul: stories110M and 7B shapes, odd shapes through the scalar path
 @pytest.mark.parametrize("M,K", [(768, 768), (2048, 768), (768, 2048), (32000, 768), (4096, 11008), (100, 100), (3, 3), (31, 20)])
 @pytest.mark.parametrize("B", [1, 3, 8, 13])
 def test_matmul_batch(L, oracle, M, K, B):

@@ -1,4 +1,4 @@
-"""Paged KV cache (SURVEY.md 8(f) rank 3: what the reference's BatchManager stub -- include/BatchManager.hpp:11-52 --
+"""Paged KV cache (what the reference's BatchManager stub -- include/BatchManager.hpp:11-52 --
 gestures at): K/V rows in blocks of 16 positions, found through a per-slot block table by the attention, prefill-attention
 and RoPE/scatter kernels.  With a deliberately FRAGMENTED table (blocks of one slot scattered over the pool, interleaved
 with other slots', out of order) the results must be what the dense slab gives: logits against the oracle at the usual

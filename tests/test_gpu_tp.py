@@ -1,4 +1,4 @@
-"""Tensor-parallel step (tha_tp_*, SURVEY.md 8e "Optional TP") against the oracle of the UNSPLIT model.
+"""Tensor-parallel step (tha_tp_*) against the oracle of the UNSPLIT model.
 
 The ranks of one replica normally sit on different GPUs; the exchange only needs every rank to be able to address its
 peers' exchange blocks, so on a single-GPU box the same code runs with all ranks on cuda:0, one stream per rank (the

@@ -125,7 +125,7 @@ def test_batch_manager(built):
 
 
 def test_cpp_api_symbols(built):
-    """libthablas.so exports the reference's C++ names (SURVEY.md 8b) and needs no CUDA library itself."""
+    """libthablas.so exports the reference's C++ names and needs no CUDA library itself."""
     so = os.path.join(ROOT, "hip_llama.cpp_b200", "lib", "libthablas.so")
     syms = run(["nm", "-DC", "--defined-only", so])
     for name in ["thablasCreate(thablasHandle_t*)", "thablasDestroy(thablasHandle_t)", "thablas_Svds(", "thaBLAS_s_vecaddvec(",
@@ -234,7 +234,7 @@ def test_llama_app_tensor_parallel_matches_oracle(built, oracle, tmp_path, quant
 
 @pytest.mark.gpu
 def test_llama_app_config1_all_128_requests(built, oracle, tmp_path):
-    """the stories110M architecture (fp32, seeded random-init -- there is no checkpoint on the
+    """The stories110M architecture (fp32, seeded random-init -- there is no checkpoint on the
     box) greedy-decodes all 128 prompts of assets/in/gen_in_128.txt through the shipped driver; the first 24 generated
     ids of EVERY request against the oracle's greedy loop run in lock step (src/llama.cpp:1025-1050 semantics).  A
     request may only leave the oracle's stream where the oracle's own top-2 logit margin is inside the fp32 tolerance."""

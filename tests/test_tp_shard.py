@@ -68,7 +68,7 @@ def test_q8_shards_keep_groups():
 
 
 def _tp_forward_numpy(cfg, shards, tokens):
-    """The arithmetic of the tensor-parallel step (DESIGN.md section 5) in numpy float64: every rank works on its
+    """The arithmetic of the tensor-parallel step in numpy float64: every rank works on its
     shard with the LOCAL config, the wo / w2 partial products of all ranks are summed into one residual stream.
     Returns the logits after each token (run.cc:244-374 semantics)."""
     tp = len(shards)
