@@ -100,9 +100,9 @@ __global__ void __launch_bounds__(256) hyb_wkv_decay_kernel(float* __restrict__ 
   }
 }
 
-// The same for few rows: four threads share a channel, sixteen bytes of every 64 of its W2 row each, all asked for before the rows' tanh; R rows at a
-// time.  The tiles above take a barrier and a load latency for every 16 of the rank and fill 1/16 of themselves with 3 rows: rank 64, 1024 channels, 3
-// rows, behind the kernel ahead, 8.3 -> 2.7 us
+// The same for few rows: four threads share a channel and ask for its W2 row between them, all of it before the rows' tanh; then, 64 of the rank at a time, the weights change hands
+// through shared memory and each thread takes two of the rows, k ascending as above: the same bits.  The tiles above take a barrier and a load latency for every 16 of the rank
+// and fill 1/16 of themselves with 3 rows: rank 64, 1024 channels, 3 rows, launched plainly, 8.2 -> 2.9 us.
 constexpr int WD_FEW = 8, WD_RANK = 256;
 __device__ __forceinline__ void wd_load8(const float* p, float (&v)[8]) {
   const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
@@ -117,8 +117,9 @@ __device__ __forceinline__ void wd_load8(const __nv_bfloat16* p, float (&v)[8]) 
 template <typename T>
 __global__ void __launch_bounds__(256) hyb_wkv_decay_few_kernel(float* decay, const float* z, long long ldz, int rank, const T* w2, const float* w0, int n_rows, int n_ch) {
   hyb_pdl_enter();
-  __shared__ __align__(16) float t[WD_FEW][WD_RANK];
-  const int c = blockIdx.x * 64 + (threadIdx.x >> 2), part = threadIdx.x & 3;
+  __shared__ __align__(16) float t[WD_FEW][WD_RANK + 4];
+  __shared__ __align__(16) float ws[64][64 + 4];
+  const int ch = threadIdx.x >> 2, c = blockIdx.x * 64 + ch, part = threadIdx.x & 3;
   constexpr int NI = WD_RANK / 32;
   float w[NI][8];
 #pragma unroll
@@ -134,23 +135,32 @@ __global__ void __launch_bounds__(256) hyb_wkv_decay_few_kernel(float* decay, co
     const int r = i / rank;
     t[r][i - r * rank] = tanhf(z[(size_t)r * ldz + (i - r * rank)]);
   }
-  __syncthreads();
-  for (int r = 0; r < n_rows; r++) {
-    float acc = 0.f;
+  float acc0 = 0.f, acc1 = 0.f;                     // of rows part and part + 4
 #pragma unroll
-    for (int i = 0; i < NI; i++) {
-      const int k = 32 * i + 8 * part;
-      if (k < rank) {
-        float v[8];
-        wd_load8(&t[r][k], v);
+  for (int k0 = 0; k0 < WD_RANK; k0 += 64) {
+    if (k0 >= rank) break;
+    if (k0) __syncthreads();                        // the 64 before have been used
 #pragma unroll
-        for (int e = 0; e < 8; e++) acc = fmaf(v[e], w[i][e], acc);
-      }
+    for (int h = 0; h < 2; h++) {
+      float* d = &ws[ch][32 * h + 8 * part];
+      const float(&v)[8] = w[k0 / 32 + h];
+      *reinterpret_cast<float4*>(d) = make_float4(v[0], v[1], v[2], v[3]);
+      *reinterpret_cast<float4*>(d + 4) = make_float4(v[4], v[5], v[6], v[7]);
     }
-    acc += __shfl_xor_sync(THA_FULL_MASK, acc, 1);
-    acc += __shfl_xor_sync(THA_FULL_MASK, acc, 2);
-    if (part == 0 && c < n_ch) decay[(size_t)r * n_ch + c] = expf(-expf(acc + bias));
+    __syncthreads();
+    const int n = min(64, rank - k0);               // a multiple of 8
+    for (int k = 0; k < n; k += 4) {
+      const float4 x = *reinterpret_cast<const float4*>(&ws[ch][k]);
+      const float4 a = *reinterpret_cast<const float4*>(&t[part][k0 + k]), b = *reinterpret_cast<const float4*>(&t[part + 4][k0 + k]);
+      acc0 = fmaf(a.x, x.x, acc0); acc1 = fmaf(b.x, x.x, acc1);
+      acc0 = fmaf(a.y, x.y, acc0); acc1 = fmaf(b.y, x.y, acc1);
+      acc0 = fmaf(a.z, x.z, acc0); acc1 = fmaf(b.z, x.z, acc1);
+      acc0 = fmaf(a.w, x.w, acc0); acc1 = fmaf(b.w, x.w, acc1);
+    }
   }
+  if (c >= n_ch) return;
+  if (part < n_rows) decay[(size_t)part * n_ch + c] = expf(-expf(acc0 + bias));
+  if (part + 4 < n_rows) decay[(size_t)(part + 4) * n_ch + c] = expf(-expf(acc1 + bias));
 }
 
 }  // namespace tha

@@ -87,3 +87,33 @@ def test_head_gate(dtype, out_t, E, gated, act):
         return (out,)
 
     both(run, [torch.randn(R, heads * E, device="cuda", generator=g)])
+
+
+Wkv = H._struct("tha_wkv_t", [("heads dim rank", H.I), ("eps", H.F), ("mu", H.P), ("o_r o_k o_v o_g o_w1", H.I), ("w_w2 w0 u norm w_o", H.P), ("state_off shift_state_off", H.L)])
+
+
+@pytest.mark.parametrize("dtype,t", [(H.F32, torch.float32), (H.BF16, torch.bfloat16)])
+@pytest.mark.parametrize("rank", [8, 56, 64, 72, 128, 200, 256])
+@pytest.mark.parametrize("rows", [1, 3, 4, 5, 8])
+def test_decay_of_few_rows(dtype, t, rank, rows):
+    """Up to eight rows against the tiles, which take a W2 that does not start on 16 bytes."""
+    lib, heads, dim = H.lib(), 3, 26
+    HD = heads * dim
+    g = torch.Generator("cuda").manual_seed(rank + rows)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    ldp = 4 * HD + rank
+    proj, w0, u, norm = rnd(rows, ldp), rnd(HD), rnd(HD), rnd(HD)
+    w2 = (rnd(HD, rank) / rank ** 0.5).to(t)
+    r, keep = H.rows_of([(0, 0, rows)])
+    lib.c.tha_hyb_scan_state_floats.restype = L
+    floats = lib.c.tha_hyb_scan_state_floats(heads, dim, dim)
+
+    def run(m):
+        state = torch.zeros(1, floats, device="cuda")
+        decay, raw, out = torch.zeros(rows, HD, device="cuda"), torch.zeros(rows, HD, device="cuda"), torch.zeros(rows, HD, device="cuda", dtype=t)
+        k = Wkv(heads=heads, dim=dim, rank=rank, eps=1e-5, o_r=0, o_k=HD, o_v=2 * HD, o_g=3 * HD, o_w1=4 * HD, w_w2=H.ptr(m[0]), w0=H.ptr(w0), u=H.ptr(u), norm=H.ptr(norm))
+        st = H.States(H.ptr(state), state.shape[1])
+        lib.check(lib.c.tha_hyb_wkv_scan(None, dtype, C.byref(k), C.byref(r), C.byref(st), p(proj), L(ldp), p(decay), p(raw), p(out), None, C.c_size_t(0)))
+        return decay, raw, out
+
+    both(run, [w2])
