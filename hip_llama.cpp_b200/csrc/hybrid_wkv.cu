@@ -2,7 +2,7 @@
 //   hyb_token_shift_kernel   every row's mixes with its predecessor, h + (h' - h) * mu, n of them in one pass: the inputs of the grouped
 //                            product (tha_hyb_linear_groups).  The predecessor of a portion's first row is the slot's stored row.
 //   hyb_wkv_decay_kernel     the low-rank decay from end to end: tanh of the W_w1 columns on the way into shared memory, the product with
-//                            W_w2 (fp32 FMA), and exp(-exp(. + w0)) on the way out; hyb_wkv_decay_few_kernel for up to eight rows
+//                            W_w2 (fp32 FMA, k ascending), and exp(-exp(. + w0)) on the way out; hyb_wkv_decay_few_kernel for up to eight rows
 //   the recurrence           hybrid_gla.cu, SCAN_BONUS
 // Mixes are formed from the fp32 norm and rounded once, to the product's number format; decays, state and read-out are fp32 in both
 // number formats.  The head norm, its weight and the silu gate follow in tha_hyb_head_gate.

@@ -69,6 +69,15 @@ def test_rows_beyond_their_first_values(splits):
     check(W, X, splits)                             # every output against the sizes of its own row and column
 
 
+@pytest.mark.parametrize("splits", [1, 3])
+def test_second_pass_over_many_items(splits):
+    """Five and more items a pair of CTAs, gone over twice by the pairs that have a row beyond its first values."""
+    g = torch.Generator(device="cuda").manual_seed(6)
+    W, X = torch.randn(40000, 576, device="cuda", generator=g), torch.randn(300, 576, device="cuda", generator=g)
+    W[torch.arange(7, 40000, 3000, device="cuda"), 191] = 1e6
+    check(W, X, splits)
+
+
 @pytest.mark.parametrize("down", [2.0 ** -12, 2.0 ** -20, 1e-6])
 @pytest.mark.parametrize("splits", [1, 2])
 def test_rows_that_shrink_behind_their_first_values(splits, down):
